@@ -242,6 +242,11 @@ int npa_moment_matrix_backward(const npa_grid *g, const float *x_bin,
 int npa_safe_inv_sym_mat(int32_t dim, int64_t n, const float *m, float *m_inv,
                          float tol, void *stream);
 
+/* out[n,C,D] = raw[n,C,D] . inv(M[n,D,D]) with the inverse of npa_safe_inv_sym_mat: the value of
+ * gradient_hybrid (sphops/sph.py:474-484), whose gradient is that of the raw operator.  out may be raw. */
+int npa_corrected_gradient(int32_t dim, int64_t n, int32_t channels, const float *raw, const float *moment,
+                           float tol, float *out, void *stream);
+
 /* ---- neighbour list cache ---------------------------------------------------- *
  * All sweeps over one snapshot visit the same pairs.  The fused entry points
  * below take an optional cache  pair_cache [B*N, pair_stride] (int32,

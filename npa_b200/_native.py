@@ -66,6 +66,7 @@ SIGNATURES = {
     "npa_density_gradient_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P]),
     "npa_moment_matrix_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _P, _P, _P]),
     "npa_safe_inv_sym_mat": (ctypes.c_int, [_I32, _I64, _P, _P, ctypes.c_float, _P]),
+    "npa_corrected_gradient": (ctypes.c_int, [_I32, _I64, _I32, _P, _P, ctypes.c_float, _P, _P]),
     "npa_blur_gradient_forward": (ctypes.c_int, [_P, _I32] + [_P] * 9 + [_P, _I32, _I32, _P]),
     "npa_blur_gradient_backward": (ctypes.c_int, [_P, _I32] + [_P] * 11 + [_P, _I32, _P]),
     "npa_density_chain_backward": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _P, _I32, _P, _P, _P, _I32, _P]),
@@ -122,6 +123,23 @@ def _load() -> ctypes.CDLL:
 
 
 lib = _load()
+
+
+def _load_ops():
+    """The autograd binding (``csrc/torch_ops.cpp``), linked to the same library."""
+    import torch  # noqa: F401  (its libraries must be loaded first)
+
+    try:
+        from . import _torch_ops
+    except ImportError as e:
+        raise ImportError(f"{_PKG / '_torch_ops.so'} is missing or does not load ({e}): build it first "
+                          "(python -m npa_b200.build)") from e
+    if _torch_ops.abi_version != ABI_VERSION:
+        raise ImportError(f"_torch_ops.so was built for ABI version {_torch_ops.abi_version}, this binding expects {ABI_VERSION}")
+    return _torch_ops
+
+
+ops = _load_ops()
 
 
 def last_error() -> str:
@@ -182,4 +200,4 @@ def ptr(t):
 def current_stream():
     import torch
 
-    return ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)
+    return ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(torch.cuda.current_device()))

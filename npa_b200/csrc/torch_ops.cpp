@@ -1,0 +1,628 @@
+// The operators of npa_b200 as autograd nodes in C++, over the C ABI of libnpa_b200.so.
+//
+// What a training step of a small system waits for is the host: with torch.autograd.Function in
+// Python and ctypes underneath, one operator costs 30-50 us of argument conversion, checks,
+// allocation and node bookkeeping per direction, several times what its kernels take at 4,096
+// particles.  Here an operator is one call: checks, output allocation, launch and graph node
+// together are a few microseconds, and backward nodes run in the autograd engine without the
+// interpreter.  Semantics are those of the reference's Functions (sphops/sph.py:127-464): a
+// gradient is produced only for inputs that need it, mass receives one in the reorder only, and
+// kernels run on the current stream of the tensors' device.
+#include <torch/extension.h>
+#include <c10/cuda/CUDAGuard.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/autograd/function.h>
+#include <torch/csrc/autograd/functions/utils.h>
+#include <torch/csrc/autograd/saved_variable.h>
+
+#include "../../include/npa_b200.h"
+
+namespace {
+
+namespace py = pybind11;
+using at::Tensor;
+using torch::autograd::Node;
+using torch::autograd::SavedVariable;
+using torch::autograd::variable_list;
+using OptTensor = std::optional<Tensor>;
+
+// ---- status codes and argument checks --------------------------------------------------------
+void check_status(int rc) {
+    if (rc == NPA_OK) return;
+    const std::string text = npa_last_error();
+    if (rc == NPA_ERR_UNSUPPORTED) throw std::invalid_argument(text);  // ValueError
+    throw std::runtime_error(text);
+}
+
+std::string shape_text(at::IntArrayRef s) {
+    std::string t = "(";
+    for (size_t k = 0; k < s.size(); ++k) t += (k ? ", " : "") + std::to_string(s[k]);
+    return t + ")";
+}
+
+// The checks of the reference's binding: wrong dtype, device or layout is a TypeError (nanobind), a
+// wrong shape a RuntimeError with the reference's wording (sphops/utils.cuh:526-567).
+void require(const Tensor &t, at::IntArrayRef shape, const char *name, at::ScalarType dtype = at::kFloat) {
+    if (!t.is_cuda() || t.scalar_type() != dtype || !t.is_contiguous())
+        throw py::type_error(std::string(name) + ": incompatible function arguments; expected a contiguous CUDA tensor of dtype " +
+                             (dtype == at::kFloat ? "torch.float32" : "torch.int32") + ", got tensor(dtype=" + toString(t.scalar_type()) +
+                             ", device=" + t.device().str() + ", contiguous=" + (t.is_contiguous() ? "True" : "False") + ")");
+    if (t.dim() != (int64_t)shape.size())
+        throw std::runtime_error(std::string(name) + " must have " + std::to_string(shape.size()) + " dimensions, got " + std::to_string(t.dim()));
+    if (t.sizes() != shape)
+        throw std::runtime_error(std::string(name) + " must have shape " + shape_text(shape) + ", got " + shape_text(t.sizes()));
+}
+
+const float *fptr(const Tensor &t) { return t.defined() ? t.const_data_ptr<float>() : nullptr; }
+float *fmut(const Tensor &t) { return t.defined() ? t.mutable_data_ptr<float>() : nullptr; }
+const int32_t *iptr(const Tensor &t) { return t.defined() ? t.const_data_ptr<int32_t>() : nullptr; }
+int32_t *imut(const Tensor &t) { return t.defined() ? t.mutable_data_ptr<int32_t>() : nullptr; }
+Tensor or_none(const OptTensor &t) { return t.has_value() ? *t : Tensor(); }
+Tensor solid(const Tensor &t) { return t.defined() ? t.contiguous() : t; }
+void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
+Tensor floats(const Tensor &like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat).requires_grad(false)); }
+Tensor blank(const Tensor &like) { return floats(like, like.sizes()); }
+bool wants_grad(const Tensor &t) { return t.defined() && t.requires_grad(); }
+
+// ---- a grid and the snapshot of one binning pass -------------------------------------------------
+struct Grid {
+    npa_grid g;
+    int64_t cells, max_blocks, scratch_bytes, B, N, P, D;
+    Tensor scratch;  // work arrays of the binning, allocated once per device
+
+    explicit Grid(uintptr_t descriptor) : g(*reinterpret_cast<const npa_grid *>(descriptor)) {
+        cells = npa_grid_num_cells(&g);
+        if (cells < 0) check_status((int)cells);
+        max_blocks = npa_grid_max_blocks(&g);
+        scratch_bytes = npa_grid_scratch_bytes(&g);
+        B = g.batch; N = g.particles; D = g.dim; P = g.dim == 2 ? 2 : 4;
+    }
+    void positions(const Tensor &x, const char *name) const { require(x, {B, N, P}, name); }
+    void rows(const Tensor &t, const char *name) const { require(t, {B, N}, name); }
+    void rows(const Tensor &t, const char *name, int64_t c) const { require(t, {B, N, c}, name); }
+    void snapshot(const Tensor &offs, const Tensor &info) const {
+        require(offs, {B * cells + 1}, "bin_offsets", at::kInt);
+        require(info, {max_blocks, 4}, "block_info", at::kInt);
+    }
+    void features(const Tensor &s, const char *name) const { require(s, {B, N, s.dim() == 3 ? s.size(2) : -1}, name); }
+};
+using GridPtr = std::shared_ptr<Grid>;
+
+py::tuple instantiate(const GridPtr &grid, const Tensor &x) {
+    Grid &g = *grid;
+    g.positions(x, "positions");
+    c10::cuda::CUDAGuard guard(x.device());
+    const auto ints = at::TensorOptions().dtype(at::kInt).device(x.device());
+    Tensor perm = at::empty({g.B, g.N}, ints), offs = at::empty({g.B * g.cells + 1}, ints), info = at::empty({g.max_blocks, 4}, ints);
+    if (!g.scratch.defined() || g.scratch.device() != x.device())
+        g.scratch = at::empty({g.scratch_bytes}, at::TensorOptions().dtype(at::kByte).device(x.device()));
+    check_status(npa_grid_build(&g.g, fptr(x), imut(perm), imut(offs), imut(info), g.scratch.mutable_data_ptr(), g.scratch_bytes, stream_of(x)));
+    return py::make_tuple(offs, perm, info);
+}
+
+// ---- node plumbing ------------------------------------------------------------------------------
+template <typename T, typename... In>
+std::shared_ptr<T> node_for(const In &...inputs) {
+    std::shared_ptr<T> n(new T(), torch::autograd::deleteNode);
+    n->set_next_edges(torch::autograd::collect_next_edges(inputs...));
+    return n;
+}
+template <typename... In>
+bool recording(const In &...inputs) {
+    return at::GradMode::is_enabled() && (wants_grad(inputs) || ...);
+}
+
+// What every node of a neighbour sweep keeps: the grid, the snapshot arrays, the neighbour lists.
+struct SweepNode : Node {
+    GridPtr grid;
+    Tensor offs, info, pairs;
+    SavedVariable x_, mass_;
+    void keep(const GridPtr &g, const Tensor &o, const Tensor &i, const Tensor &p, const Tensor &x, const Tensor &mass) {
+        grid = g; offs = o; info = i; pairs = p;
+        x_ = SavedVariable(x, false);
+        mass_ = SavedVariable(mass, false);
+    }
+    void release_variables() override {
+        x_.reset_data(); mass_.reset_data();
+        pairs = Tensor();
+    }
+    int list_stride() const { return pairs.defined() ? (int)pairs.size(2) : 0; }
+};
+
+struct Snap {  // arguments every sweep shares, checked
+    GridPtr grid;
+    Tensor offs, info, mass, pairs;
+    Snap(const GridPtr &g, const Tensor &o, const Tensor &i, const OptTensor &m, const OptTensor &p)
+        : grid(g), offs(o), info(i), mass(or_none(m)), pairs(or_none(p)) {
+        grid->snapshot(offs, info);
+        if (mass.defined()) grid->rows(mass, "mass");
+        if (pairs.defined()) {
+            require(pairs, {grid->B, grid->N, pairs.dim() == 3 ? pairs.size(2) : -1}, "pair_cache", at::kInt);
+            if (pairs.size(2) < 2 || pairs.size(2) > 513)
+                throw std::runtime_error("pair_cache must have between 2 and 513 columns, got " + std::to_string(pairs.size(2)));
+        }
+    }
+    int stride() const { return pairs.defined() ? (int)pairs.size(2) : 0; }
+};
+
+Tensor new_lists(const Grid &g, const Tensor &like, int64_t columns) {
+    return columns ? at::empty({g.B, g.N, columns}, like.options().dtype(at::kInt).requires_grad(false)) : Tensor();
+}
+
+// ---- reorder into cell order (Permute, sph.py:127-184) ---------------------------------------------
+struct ReorderNode : Node {
+    GridPtr grid;
+    Tensor perm;
+    std::vector<int64_t> xs, ss, ms;
+    at::TensorOptions opt;
+    variable_list apply(variable_list &&g) override {
+        c10::cuda::CUDAGuard guard(perm.device());
+        auto upstream = [&](const Tensor &t, const std::vector<int64_t> &shape, bool need) {
+            if (!need) return Tensor();
+            return t.defined() ? t.contiguous() : at::zeros(shape, opt);
+        };
+        const bool nx = should_compute_output(0), ns = should_compute_output(1), nm = !ms.empty() && should_compute_output(2);
+        const Tensor gx = upstream(g[0], xs, nx), gs = upstream(g[1], ss, ns), gm = ms.empty() ? Tensor() : upstream(g[2], ms, nm);
+        Tensor ox = nx ? blank(gx) : Tensor(), os = ns ? blank(gs) : Tensor(), om = nm ? blank(gm) : Tensor();
+        const int C = (int)ss[2];
+        const bool feats = ns && C > 0;
+        if (nx || feats || nm)
+            check_status(npa_unbin_particles(&grid->g, C, fptr(gx), feats ? fptr(gs) : nullptr, fptr(gm), iptr(perm), fmut(ox),
+                                             feats ? fmut(os) : nullptr, fmut(om), stream_of(perm)));
+        return {ox, os, om};
+    }
+};
+
+py::tuple reorder(const GridPtr &grid, const Tensor &perm, const Tensor &x, const Tensor &s, const OptTensor &mass_) {
+    const Tensor mass = or_none(mass_);
+    Grid &g = *grid;
+    g.positions(x, "input_positions");
+    g.features(s, "input_state");
+    if (mass.defined()) g.rows(mass, "input_mass");
+    require(perm, {g.B, g.N}, "permutation", at::kInt);
+    c10::cuda::CUDAGuard guard(x.device());
+    const int C = (int)s.size(2);
+    Tensor xo = blank(x), so = blank(s), mo = mass.defined() ? blank(mass) : Tensor();
+    check_status(npa_bin_particles(&g.g, C, fptr(x), C ? fptr(s) : nullptr, fptr(mass), iptr(perm), fmut(xo), C ? fmut(so) : nullptr, fmut(mo),
+                                   stream_of(x)));
+    if (recording(x, s, mass)) {
+        auto n = node_for<ReorderNode>(x, s, mass);
+        n->grid = grid; n->perm = perm; n->opt = x.options().requires_grad(false);
+        n->xs = x.sizes().vec(); n->ss = s.sizes().vec();
+        if (mass.defined()) n->ms = mass.sizes().vec();
+        variable_list outs = {xo, so};
+        if (mass.defined()) outs.push_back(mo);
+        torch::autograd::set_history(outs, n);
+    }
+    return mass.defined() ? py::make_tuple(xo, so, mo) : py::make_tuple(xo, so);
+}
+
+py::tuple unreorder(const GridPtr &grid, const Tensor &perm, const Tensor &x, const Tensor &s, const OptTensor &mass_) {
+    const Tensor mass = or_none(mass_);
+    Grid &g = *grid;
+    g.positions(x, "grad_output_positions");
+    g.features(s, "grad_output_state");
+    if (mass.defined()) g.rows(mass, "grad_output_mass");
+    require(perm, {g.B, g.N}, "permutation", at::kInt);
+    c10::cuda::CUDAGuard guard(x.device());
+    const int C = (int)s.size(2);
+    Tensor xo = blank(x), so = blank(s), mo = mass.defined() ? blank(mass) : Tensor();
+    check_status(npa_unbin_particles(&g.g, C, fptr(x), C ? fptr(s) : nullptr, fptr(mass), iptr(perm), fmut(xo), C ? fmut(so) : nullptr, fmut(mo),
+                                     stream_of(x)));
+    return mass.defined() ? py::make_tuple(xo, so, mo) : py::make_tuple(xo, so);
+}
+
+// ---- density and density gradient -------------------------------------------------------------------
+struct DensityNode : SweepNode {
+    bool has_rho, has_dg;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), mass = mass_.unpack();
+        const Tensor g_rho = has_rho ? solid(g[0]) : Tensor(), g_dg = has_dg ? solid(g[has_rho ? 1 : 0]) : Tensor();
+        if (!g_rho.defined() && !g_dg.defined()) return {Tensor()};
+        c10::cuda::CUDAGuard guard(x.device());
+        Tensor gx = blank(x);
+        check_status(npa_density_chain_backward(&grid->g, fptr(x), fptr(mass), fptr(g_rho), nullptr, fptr(g_dg), fmut(gx), 0, iptr(offs),
+                                                iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+        return {gx};
+    }
+};
+
+// (rho, density gradient); either may be left out.  `pairs` holds lists of these positions to be used by the backward:
+// with `write` the forward records them first.
+py::tuple density(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const OptTensor &mass, const OptTensor &pairs,
+                  bool want_rho, bool want_dg, bool write) {
+    Snap sn(grid, offs, info, mass, pairs);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor rho = want_rho ? floats(x, {g.B, g.N}) : Tensor(), dg = want_dg ? floats(x, {g.B, g.N, g.D}) : Tensor();
+    if (want_rho)
+        check_status(npa_perception_forward(&g.g, 0, fptr(x), fptr(sn.mass), nullptr, fmut(rho), nullptr, fmut(dg), nullptr, nullptr, nullptr,
+                                            iptr(offs), iptr(info), write ? imut(sn.pairs) : nullptr, write ? sn.stride() : 0, stream_of(x)));
+    else
+        check_status(npa_density_gradient_forward(&g.g, fptr(x), fptr(sn.mass), fmut(dg), iptr(offs), iptr(info), stream_of(x)));
+    if (recording(x)) {
+        auto n = node_for<DensityNode>(x);
+        n->keep(grid, offs, info, sn.pairs, x, sn.mass);
+        n->has_rho = want_rho; n->has_dg = want_dg;
+        if (want_rho) torch::autograd::set_history(rho, n);
+        if (want_dg) torch::autograd::set_history(dg, n);
+    }
+    return py::make_tuple(want_rho ? py::cast(rho) : py::none(), want_dg ? py::cast(dg) : py::none());
+}
+
+// ---- blur and feature gradient ----------------------------------------------------------------------
+struct FeatureNode : SweepNode {
+    SavedVariable s_, rho_;
+    bool has_blur, has_grad;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(), mass = mass_.unpack();
+        const bool nx = should_compute_output(0), ns = should_compute_output(1), nr = should_compute_output(2);
+        const Tensor gb = has_blur ? solid(g[0]) : Tensor(), gg = has_grad ? solid(g[has_blur ? 1 : 0]) : Tensor();
+        if ((!gb.defined() && !gg.defined()) || !(nx || ns || nr)) return {Tensor(), Tensor(), Tensor()};
+        c10::cuda::CUDAGuard guard(x.device());
+        Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nr ? blank(rho) : Tensor();
+        if (s.size(2) > 0)
+            check_status(npa_blur_gradient_backward(&grid->g, (int)s.size(2), fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx),
+                                                    fmut(gs), fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+        return {gx, gs, gr};
+    }
+    void release_variables() override {
+        SweepNode::release_variables();
+        s_.reset_data(); rho_.reset_data();
+    }
+};
+
+// (blur, gradient, moment matrix) of the requested set; the moment matrix carries no gradient here.  `pairs`: neighbour
+// lists, valid when `have_lists`, otherwise recorded by this sweep.
+py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const Tensor &s,
+                        const OptTensor &mass, const OptTensor &pairs, bool have_lists, bool want_blur, bool want_grad, bool want_moment) {
+    Snap sn(grid, offs, info, mass, pairs);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    g.rows(rho, "rho");
+    g.features(s, "state_in");
+    const int64_t C = s.size(2);
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor blur = want_blur ? blank(s) : Tensor(), grad = want_grad ? floats(s, {g.B, g.N, C, g.D}) : Tensor();
+    Tensor moment = want_moment ? floats(s, {g.B, g.N, g.D, g.D}) : Tensor();
+    if (C > 0)
+        check_status(npa_blur_gradient_forward(&g.g, (int)C, fptr(x), fptr(rho), fptr(sn.mass), fptr(s), fmut(blur), fmut(grad), fmut(moment),
+                                               iptr(offs), iptr(info), imut(sn.pairs), sn.stride(), have_lists ? 1 : 0, stream_of(x)));
+    if (recording(x, s, rho)) {
+        auto n = node_for<FeatureNode>(x, s, rho);
+        n->keep(grid, offs, info, sn.pairs, x, sn.mass);
+        n->s_ = SavedVariable(s, false);
+        n->rho_ = SavedVariable(rho, false);
+        n->has_blur = want_blur; n->has_grad = want_grad;
+        if (want_blur) torch::autograd::set_history(blur, n);
+        if (want_grad) torch::autograd::set_history(grad, n);
+    }
+    auto cast = [](const Tensor &t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
+    return py::make_tuple(cast(blur), cast(grad), cast(moment));
+}
+
+// ---- moment matrix -----------------------------------------------------------------------------------
+struct MomentNode : SweepNode {
+    SavedVariable rho_;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), rho = rho_.unpack(), mass = mass_.unpack();
+        const bool nx = should_compute_output(0), nr = should_compute_output(1);
+        if (!g[0].defined() || !(nx || nr)) return {Tensor(), Tensor()};
+        c10::cuda::CUDAGuard guard(x.device());
+        Tensor gx = nx ? blank(x) : Tensor(), gr = nr ? blank(rho) : Tensor();
+        check_status(npa_moment_matrix_backward(&grid->g, fptr(x), fptr(rho), fptr(mass), fptr(solid(g[0])), fmut(gx), fmut(gr), iptr(offs),
+                                                iptr(info), stream_of(x)));
+        return {gx, gr};
+    }
+    void release_variables() override {
+        SweepNode::release_variables();
+        rho_.reset_data();
+    }
+};
+
+Tensor moment_matrix(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const OptTensor &mass) {
+    Snap sn(grid, offs, info, mass, std::nullopt);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    g.rows(rho, "rho");
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = floats(x, {g.B, g.N, g.D, g.D});
+    check_status(npa_moment_matrix_forward(&g.g, fptr(x), fptr(rho), fptr(sn.mass), fmut(out), iptr(offs), iptr(info), stream_of(x)));
+    if (recording(x, rho)) {
+        auto n = node_for<MomentNode>(x, rho);
+        n->keep(grid, offs, info, Tensor(), x, sn.mass);
+        n->rho_ = SavedVariable(rho, false);
+        torch::autograd::set_history(out, n);
+    }
+    return out;
+}
+
+// ---- moment-corrected gradient (sph.py:474-484): value raw @ inv(M), gradient of the raw operator ----------
+struct StraightThroughNode : Node {
+    variable_list apply(variable_list &&g) override { return {g[0]}; }
+};
+
+Tensor corrected_gradient(const Tensor &raw, const Tensor &moment, double rtol) {
+    const int64_t B = raw.size(0), N = raw.size(1), C = raw.size(2), D = raw.size(3);
+    require(raw, {B, N, C, D}, "gradient");
+    require(moment, {B, N, D, D}, "moment_matrix");
+    c10::cuda::CUDAGuard guard(raw.device());
+    Tensor out = blank(raw);
+    if (out.numel() > 0)
+        check_status(npa_corrected_gradient((int)D, B * N, (int)C, fptr(raw), fptr(moment), (float)rtol, fmut(out), stream_of(raw)));
+    if (recording(raw)) {
+        auto n = node_for<StraightThroughNode>(raw);
+        torch::autograd::set_history(out, n);
+    }
+    return out;
+}
+
+// ---- the fused perception step -------------------------------------------------------------------------
+struct PerceptionNode : SweepNode {
+    SavedVariable s_, rho_;
+    bool has_dg;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(shared_from_this()), mass = mass_.unpack();
+        const bool nx = should_compute_output(0), ns = should_compute_output(1);
+        if (!(nx || ns)) return {Tensor(), Tensor()};
+        const Tensor g_rho = nx ? solid(g[0]) : Tensor(), gb = solid(g[1]), gg = solid(g[2]), g_dg = nx && has_dg ? solid(g[3]) : Tensor();
+        c10::cuda::CUDAGuard guard(x.device());
+        Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nx ? blank(rho) : Tensor();
+        check_status(npa_perception_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(g_rho), fptr(gb), fptr(gg),
+                                             fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(),
+                                             stream_of(x)));
+        return {gx, gs};
+    }
+    void release_variables() override {
+        SweepNode::release_variables();
+        s_.reset_data(); rho_.reset_data();
+    }
+};
+
+py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &s, const OptTensor &mass,
+                     bool want_dg, int64_t columns) {
+    Snap sn(grid, offs, info, mass, std::nullopt);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    g.features(s, "state_in");
+    const int64_t C = s.size(2);
+    c10::cuda::CUDAGuard guard(x.device());
+    const bool record = recording(x, s);
+    Tensor rho = floats(x, {g.B, g.N}), blur = blank(s), grad = floats(s, {g.B, g.N, C, g.D});
+    Tensor dg = want_dg ? floats(x, {g.B, g.N, g.D}) : Tensor(), pairs = new_lists(g, x, columns);
+    check_status(npa_perception_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), fmut(rho), nullptr, fmut(dg), fmut(blur), fmut(grad), nullptr,
+                                        iptr(offs), iptr(info), imut(pairs), pairs.defined() ? (int)columns : 0, stream_of(x)));
+    if (record) {
+        auto n = node_for<PerceptionNode>(x, s);
+        n->keep(grid, offs, info, pairs, x, sn.mass);
+        n->s_ = SavedVariable(s, false);
+        n->has_dg = want_dg;
+        torch::autograd::set_history(rho, n);
+        torch::autograd::set_history(blur, n);
+        torch::autograd::set_history(grad, n);
+        if (want_dg) torch::autograd::set_history(dg, n);
+        n->rho_ = SavedVariable(rho, true);
+    }
+    return want_dg ? py::make_tuple(rho, blur, grad, dg) : py::make_tuple(rho, blur, grad);
+}
+
+// ---- the packed perception row ---------------------------------------------------------------------------
+struct PackedNode : SweepNode {
+    SavedVariable s_;
+    Tensor rho, rho_grad, vgrad;
+    float coef, dg_scale;
+    bool ln_grad, ln_dg;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), s = s_.unpack(), mass = mass_.unpack();
+        const bool nx = should_compute_output(0), ns = should_compute_output(1);
+        if (!g[0].defined() || !(nx || ns)) return {Tensor(), Tensor()};
+        c10::cuda::CUDAGuard guard(x.device());
+        const Tensor gz = g[0].contiguous();
+        const int64_t n = s.numel(), D = grid->D, rows = rho.numel();
+        // dL/dblur and dL/dgradient of the rows, and with position gradients the two per-particle upstreams, in one buffer
+        Tensor work = floats(s, {n * (1 + D) + (nx ? rows * (1 + D) : 0)});
+        float *gb = fmut(work), *gg = gb + n, *g_dg = nx ? gg + n * D : nullptr, *gr = nx ? g_dg + rows * D : nullptr;
+        Tensor gx = nx ? blank(x) : Tensor(), gs = blank(s);
+        check_status(npa_perceive_features_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad), fptr(vgrad),
+                                                    fptr(gz), coef, dg_scale, ln_grad, ln_dg, gb, gg, g_dg, gr, fmut(gx), fmut(gs), iptr(offs),
+                                                    iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+        return {gx, ns ? gs : Tensor()};
+    }
+    void release_variables() override {
+        SweepNode::release_variables();
+        s_.reset_data();
+        rho = rho_grad = vgrad = Tensor();
+    }
+};
+
+Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &s, const OptTensor &mass,
+                         double coef, double dg_scale, double inv_tol, bool ln_grad, bool ln_dg, int64_t columns) {
+    Snap sn(grid, offs, info, mass, std::nullopt);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    g.features(s, "state_in");
+    const int64_t C = s.size(2), D = g.D;
+    c10::cuda::CUDAGuard guard(x.device());
+    const bool record = recording(x, s);
+    Tensor rho = floats(x, {g.B, g.N}), rho_grad = floats(x, {g.B, g.N, D}), z = floats(s, {g.B, g.N, 2 * C + C * D + D});
+    Tensor vgrad = record ? floats(s, {g.B, g.N, C, D}) : Tensor(), pairs = new_lists(g, x, columns);
+    check_status(npa_perceive_features_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), (float)coef, (float)dg_scale, (float)inv_tol, ln_grad,
+                                               ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), iptr(offs), iptr(info), imut(pairs),
+                                               pairs.defined() ? (int)columns : 0, stream_of(x)));
+    if (record) {
+        auto n = node_for<PackedNode>(x, s);
+        n->keep(grid, offs, info, pairs, x, sn.mass);
+        n->s_ = SavedVariable(s, false);
+        n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad;
+        n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->ln_grad = ln_grad; n->ln_dg = ln_dg;
+        torch::autograd::set_history(z, n);
+    }
+    return z;
+}
+
+// ---- the Euler update --------------------------------------------------------------------------------------
+struct StepNode : Node {
+    GridPtr grid;
+    SavedVariable y_;
+    Tensor mask;
+    int C;
+    float alpha, dt;
+    variable_list apply(variable_list &&g) override {
+        const Tensor y = y_.unpack(), gx = solid(g[0]), gs = solid(g[1]);
+        Tensor gy;
+        if (should_compute_output(0) && (gx.defined() || gs.defined())) {
+            c10::cuda::CUDAGuard guard(y.device());
+            gy = blank(y);
+            check_status(npa_step_update_backward(&grid->g, fptr(y), fptr(mask), C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y)));
+        }
+        return {gy, should_compute_output(1) ? gx : Tensor(), should_compute_output(2) ? gs : Tensor()};
+    }
+    void release_variables() override {
+        y_.reset_data();
+        mask = Tensor();
+    }
+};
+
+py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, const Tensor &s, const OptTensor &mask_, double alpha, double dt, bool wrap) {
+    Grid &g = *grid;
+    const Tensor mask = or_none(mask_);
+    g.positions(x, "binned_positions");
+    g.features(s, "state_in");
+    g.rows(y, "y", g.D + s.size(2));
+    if (mask.defined()) g.rows(mask, "mask");
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor xo = blank(x), so = blank(s);
+    check_status(npa_step_update_forward(&g.g, fptr(y), fptr(x), fptr(s), fptr(mask), (int)s.size(2), (float)alpha, (float)dt, wrap, fmut(xo),
+                                         fmut(so), stream_of(x)));
+    if (recording(y, x, s)) {
+        auto n = node_for<StepNode>(y, x, s);
+        n->grid = grid; n->mask = mask; n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt;
+        n->y_ = SavedVariable(y, false);
+        torch::autograd::set_history(xo, n);
+        torch::autograd::set_history(so, n);
+    }
+    return py::make_tuple(xo, so);
+}
+
+// ---- the adaptation MLP on the tensor-memory kernels (mlp.py) -------------------------------------------------
+constexpr int kHidden = 128;
+
+struct MlpNode : Node {
+    SavedVariable z_, w1_, w2_;
+    Tensor h;
+    std::vector<int64_t> z_shape;
+    variable_list apply(variable_list &&g) override {
+        const Tensor z = z_.unpack(), w1 = w1_.unpack(), w2 = w2_.unpack();
+        if (!g[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
+        c10::cuda::CUDAGuard guard(z.device());
+        const Tensor dy = g[0].contiguous();
+        const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
+        void *st = stream_of(z);
+        Tensor dh = floats(z, {m, kHidden});
+        check_status(npa_mlp_hidden_grad(fptr(dy), fptr(w2), fptr(h), fmut(dh), m, kHidden, (int)o, w2.stride(0), w2.stride(1), st));
+        Tensor gz, gw1, gb1, gw2;
+        if (should_compute_output(0)) {
+            gz = floats(z, z_shape);
+            const int64_t bytes = npa_linear_tcgen05_scratch_bytes(kHidden, (int)k);
+            Tensor image = floats(z, {bytes / 4});
+            check_status(npa_linear_tcgen05(fptr(dh), fptr(w1), nullptr, nullptr, fmut(gz), m, kHidden, (int)k, w1.stride(1), w1.stride(0), 0,
+                                            image.mutable_data_ptr(), bytes, st));
+        }
+        const bool n1 = should_compute_output(1), nb = should_compute_output(2), n2 = should_compute_output(3);
+        if (n1 || nb || n2) {
+            gw1 = at::empty_strided(w1.sizes(), at::IntArrayRef({k, (int64_t)1}), w1.options().requires_grad(false));
+            gw2 = at::empty_strided(w2.sizes(), at::IntArrayRef({(int64_t)kHidden, (int64_t)1}), w2.options().requires_grad(false));
+            gb1 = floats(z, {kHidden});
+            // the tensor-memory kernel appends a column of ones to z, 176 columns in all
+            const bool tensor = k < 176;
+            const int64_t count = tensor ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o)
+                                         : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
+            Tensor scratch = floats(z, {count});
+            check_status((tensor ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(fptr(z), fptr(dh), fptr(h), fptr(dy), m, (int)k, kHidden, (int)o,
+                                                                                      fmut(scratch), count, fmut(gw1), fmut(gw2), fmut(gb1), st));
+        }
+        return {gz, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
+    }
+    void release_variables() override {
+        z_.reset_data(); w1_.reset_data(); w2_.reset_data();
+        h = Tensor();
+    }
+};
+
+// y = relu(z W1^T + b1) W2^T over the rows of z; the caller has checked the shapes (mlp.supported).
+Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2) {
+    c10::cuda::CUDAGuard guard(z.device());
+    const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
+    std::vector<int64_t> shape = z.sizes().vec();
+    shape.back() = o;
+    Tensor y = floats(z, shape), h = floats(z, {m, kHidden});
+    const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o);
+    Tensor image = floats(z, {bytes / 4});
+    check_status(npa_mlp_forward_tcgen05(fptr(z), fptr(w1), fptr(b1), fptr(w2), fmut(h), fmut(y), m, (int)k, (int)o, w1.stride(0), w1.stride(1),
+                                         w2.stride(0), w2.stride(1), image.mutable_data_ptr(), bytes, stream_of(z)));
+    if (recording(z, w1, b1, w2)) {
+        auto n = node_for<MlpNode>(z, w1, b1, w2);
+        n->z_ = SavedVariable(z, false); n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
+        n->h = h; n->z_shape = z.sizes().vec();
+        torch::autograd::set_history(y, n);
+    }
+    return y;
+}
+
+// ---- splat renderer ------------------------------------------------------------------------------------------
+struct SplatConsts {
+    int img, radius, y_up, normalize;
+    double sigma, lo, hi, scale;
+};
+
+struct SplatNode : Node {
+    SavedVariable x_, color_;
+    SplatConsts c;
+    variable_list apply(variable_list &&g) override {
+        const Tensor x = x_.unpack(), color = color_.unpack();
+        const bool nx = should_compute_output(0), nc = should_compute_output(1);
+        if (!g[0].defined() || !(nx || nc)) return {Tensor(), Tensor()};
+        c10::cuda::CUDAGuard guard(x.device());
+        const Tensor up = g[0].contiguous();
+        Tensor gx = nx ? blank(x) : Tensor(), gc = nc ? blank(color) : Tensor();
+        check_status(npa_splat_backward(fptr(x), fptr(color), fptr(up), (int)x.size(0), (int)x.size(1), c.img, c.sigma, c.radius, c.lo, c.hi, c.y_up,
+                                        c.normalize, c.scale, fmut(gx), fmut(gc), stream_of(x)));
+        return {gx, gc};
+    }
+    void release_variables() override { x_.reset_data(); color_.reset_data(); }
+};
+
+Tensor splat(const Tensor &x, const Tensor &color, int img, double sigma, int radius, double lo, double hi, bool y_up, bool normalize, double scale) {
+    c10::cuda::CUDAGuard guard(x.device());
+    const int64_t B = x.size(0), n = x.size(1);
+    Tensor out = floats(x, {B, img, img, 4}), scratch = normalize ? floats(x, {B, n}) : Tensor();
+    check_status(npa_splat_forward(fptr(x), fptr(color), (int)B, (int)n, img, sigma, radius, lo, hi, y_up, normalize, scale, fmut(scratch), fmut(out),
+                                   stream_of(x)));
+    if (recording(x, color)) {
+        auto node = node_for<SplatNode>(x, color);
+        node->x_ = SavedVariable(x, false); node->color_ = SavedVariable(color, false);
+        node->c = SplatConsts{img, radius, y_up ? 1 : 0, normalize ? 1 : 0, sigma, lo, hi, scale};
+        torch::autograd::set_history(out, node);
+    }
+    return out;
+}
+
+}  // namespace
+
+PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
+    m.attr("abi_version") = NPA_B200_ABI_VERSION;
+    py::class_<Grid, GridPtr>(m, "Grid").def(py::init<uintptr_t>());
+    m.def("instantiate", &instantiate);
+    m.def("reorder", &reorder);
+    m.def("unreorder", &unreorder);
+    m.def("density", &density);
+    m.def("blur_gradient", &blur_gradient);
+    m.def("moment_matrix", &moment_matrix);
+    m.def("corrected_gradient", &corrected_gradient);
+    m.def("perception", &perception);
+    m.def("packed_perception", &packed_perception);
+    m.def("step_update", &step_update);
+    m.def("mlp", &mlp);
+    m.def("splat", &splat);
+}

@@ -127,4 +127,6 @@ def apply_mlp(module, z):
     """``module(z)``; with the fused weight-gradient backward when ``supported(module)``."""
     if not (supported(module) and z.is_cuda and z.dtype == torch.float32):
         return module(z)
+    if TENSOR_ENGINE == "tcgen05" and FUSED_FORWARD and FUSED_HIDDEN_GRAD:
+        return N.ops.mlp(z.contiguous(), module[0].weight, module[0].bias, module[2].weight)
     return _AdaptationMLP.apply(z.contiguous(), module[0].weight, module[0].bias, module[2].weight)

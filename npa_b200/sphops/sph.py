@@ -23,15 +23,12 @@ from dataclasses import dataclass, field
 import torch
 
 from . import sph_cuda
+from .._native import ops as _ops
 
 
-def _default_mass(x, mass):
-    if mass is None:
-        B, N, _ = x.shape
-        return x.new_full((B, N), 1.0)
-    if mass.dim() == 3 and mass.shape[-1] == 1:
-        return mass.squeeze(-1)
-    return mass
+def _mass(mass):
+    """``[B, N]`` masses (a trailing axis of one is dropped), or None = 1.0 per particle."""
+    return mass.squeeze(-1) if mass is not None and mass.dim() == 3 and mass.shape[-1] == 1 else mass
 
 
 _GRID_CLASSES = {
@@ -62,6 +59,8 @@ class HashGridSnapshot:
     # outputs computed ahead of their call by a fused sweep (see enable_fusion); not part of the
     # reference's dataclass, defaulted so positional construction still works
     parked: dict = field(default_factory=dict, repr=False, compare=False)
+    # neighbour lists of the positions the first density sweep saw: (key, tensor), see _lists_of
+    lists: tuple = field(default=None, repr=False, compare=False)
 
 
 class HashGrid:
@@ -93,17 +92,13 @@ class HashGrid:
 
     def instantiate(self, x):
         """Bin positions ``x [B, N, P]`` and return the snapshot the operators take."""
-        B, N, _ = x.shape
-        dev = x.device if x.is_cuda else self.device
-        permutation = torch.empty(B, N, dtype=torch.int32, device=dev)
-        bin_offsets = torch.empty(B * self.num_cells + 1, dtype=torch.int32, device=dev)
-        block_info = torch.empty(self.hashgrid.max_blocks, 4, dtype=torch.int32, device=dev)
-        self.hashgrid.initialize(x, permutation, bin_offsets, block_info)
-        # outputs a fused sweep parked on the previous snapshot and nobody claimed are dropped now: they would
-        # otherwise live (with the autograd graph they hang on) for as long as that snapshot does
+        bin_offsets, permutation, block_info = _ops.instantiate(self.hashgrid.native, x)
+        # outputs a fused sweep parked on the previous snapshot and nobody claimed, and its neighbour lists, are
+        # dropped now: they would otherwise live (with the autograd graph they hang on) as long as that snapshot does
         previous = self._last_snapshot() if self._last_snapshot is not None else None
         if previous is not None:
             previous.parked.clear()
+            previous.lists = None
         snapshot = HashGridSnapshot(grid=self.hashgrid, bin_offsets=bin_offsets, permutation=permutation,
                                     block_info=block_info, dim=self.dim)
         self._last_snapshot = weakref.ref(snapshot)
@@ -133,26 +128,45 @@ class HashGrid:
 # is fused too.  Off by default: a caller that only wants blur would pay for the gradient.
 # ---------------------------------------------------------------------------------------------
 _FUSION = {"enabled": False}
-# Columns of the neighbour-list cache the fused forward passes write for their backward pass
-# (row = count, j_0, j_1, ...; particles with more neighbours are searched again); 0 = off.
-_PAIR_CACHE = {"columns": 128}
+# Columns of the neighbour lists the density sweep records for the other sweeps of its snapshot
+# (row = count, j_0, j_1, ...; particles with more neighbours are searched again); 0 = off, None = by the grid.
+_PAIR_CACHE = {"columns": None}
 
 
 def set_pair_cache(columns=128):
-    """Size of the per-particle neighbour list the fused forward sweeps keep for their backward
-    (4 * columns bytes per particle while the autograd graph is alive); 0 disables it."""
+    """Length of the per-particle neighbour lists that the sweeps of a snapshot share (4 * columns bytes
+    per particle while the snapshot or the autograd graph is alive); 0 disables them."""
     columns = int(columns)
     if columns != 0 and not 2 <= columns <= 513:
         raise ValueError("columns must be 0 or between 2 and 513")
     _PAIR_CACHE["columns"] = columns
 
 
-def _new_pair_cache(s_bin, wanted):
-    K = _PAIR_CACHE["columns"]
-    if not wanted or K == 0:
-        return None
-    B, N = s_bin.shape[:2]
-    return torch.empty(B, N, K, dtype=torch.int32, device=s_bin.device)
+def _columns(grid):
+    set_by_user = _PAIR_CACHE["columns"]
+    return grid.list_columns if set_by_user is None else set_by_user
+
+
+def _lists_of(snapshot, x_bin):
+    """Neighbour lists recorded on this snapshot for the very same positions object, or None."""
+    return snapshot.lists[1] if snapshot.lists is not None and _same(snapshot.lists[0], x_bin) else None
+
+
+def _lists_for(snapshot, x_bin):
+    """``(lists or None, whether the caller has to record them)``; new lists are left on the snapshot."""
+    pairs = _lists_of(snapshot, x_bin)
+    if pairs is not None:
+        return pairs, False
+    columns = _columns(snapshot.grid)
+    if columns == 0:
+        return None, False
+    pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device)
+    snapshot.lists = (_key(x_bin), pairs)
+    return pairs, True
+
+
+def _sweep_args(snapshot):
+    return snapshot.grid.native, snapshot.bin_offsets, snapshot.block_info
 
 
 def enable_fusion(flag=True):
@@ -188,280 +202,116 @@ def _claim(snapshot, name, *tensors):
     return entry[1]
 
 
-class DensityPair(torch.autograd.Function):
+class DensityPair:
     """density and density_gradient of the same positions in one sweep."""
 
     @staticmethod
-    def forward(ctx, x_bin, mass, snapshot, pairs=None):
-        B, N = x_bin.shape[:2]
-        rho = torch.empty(B, N, dtype=torch.float32, device=x_bin.device)
-        rho_grad = torch.empty(B, N, snapshot.dim, dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.perception_forward(x_bin, mass, None, rho, None, rho_grad, None, None, None,
-                                         snapshot.bin_offsets, snapshot.block_info, pair_cache=pairs)
-        ctx.save_for_backward(x_bin, *([] if mass is None else [mass]))
-        ctx.pairs = pairs
-        ctx.has_mass = mass is not None
-        ctx.snapshot = snapshot
-        ctx.dLdx = x_bin.requires_grad
-        return rho, rho_grad
-
-    @staticmethod
-    def backward(ctx, g_rho, g_rho_grad):
-        if not ctx.dLdx or (g_rho is None and g_rho_grad is None):
-            return None, None, None, None
-        saved = ctx.saved_tensors
-        x_bin, mass = saved[0], (saved[1] if ctx.has_mass else None)
-        snap = ctx.snapshot
-        grad_x = torch.empty_like(x_bin)
-        cont = lambda t: None if t is None else t.contiguous()
-        snap.grid.density_chain_backward(x_bin, mass, cont(g_rho), None, cont(g_rho_grad), grad_x, False,
-                                         snap.bin_offsets, snap.block_info, pair_cache=ctx.pairs)
-        return grad_x, None, None, None
+    def apply(x_bin, mass, snapshot):
+        pairs, record = _lists_for(snapshot, x_bin)
+        return _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, True, record)
 
 
-class BlurGradient(torch.autograd.Function):
+class BlurGradient:
     """blur, feature gradient and (not differentiated) moment matrix in one sweep."""
 
     @staticmethod
-    def forward(ctx, x_bin, s_bin, rho, mass, snapshot, pairs=None):
-        B, N, C = s_bin.shape
-        dev, dim = x_bin.device, snapshot.dim
-        s_blur = torch.empty_like(s_bin)
-        s_grad = torch.empty(B, N, C, dim, dtype=torch.float32, device=dev)
-        moment = torch.empty(B, N, dim, dim, dtype=torch.float32, device=dev)
-        valid = pairs is not None          # lists recorded by the density sweep of the same positions
-        if pairs is None:
-            pairs = _new_pair_cache(s_bin, x_bin.requires_grad or s_bin.requires_grad or rho.requires_grad)
-        snapshot.grid.blur_gradient_forward(x_bin, rho, mass, s_bin, s_blur, s_grad, snapshot.bin_offsets,
-                                            snapshot.block_info, moment, pair_cache=pairs, pair_cache_valid=valid)
-        ctx.save_for_backward(x_bin, s_bin, rho, *([] if mass is None else [mass]))
-        ctx.pairs = pairs
-        ctx.has_mass = mass is not None
-        ctx.snapshot = snapshot
-        ctx.needs = (x_bin.requires_grad, s_bin.requires_grad, rho.requires_grad)
-        ctx.mark_non_differentiable(moment)
-        return s_blur, s_grad, moment
+    def apply(x_bin, s_bin, rho, mass, snapshot):
+        pairs = _lists_of(snapshot, x_bin)
+        return _ops.blur_gradient(*_sweep_args(snapshot), x_bin, rho, s_bin, mass, pairs, pairs is not None, True, True, True)
+
+
+class Permute:
+    """Reorder into cell order (gradients: the inverse reorder)."""
 
     @staticmethod
-    def backward(ctx, g_blur, g_grad, _g_moment):
-        saved = ctx.saved_tensors
-        x_bin, s_bin, rho = saved[:3]
-        mass = saved[3] if ctx.has_mass else None
-        dLdx, dLds, dLdrho = ctx.needs
-        if (g_blur is None and g_grad is None) or not (dLdx or dLds or dLdrho):
-            return None, None, None, None, None, None
-        snap = ctx.snapshot
-        cont = lambda t: None if t is None else t.contiguous()
-        grad_x = torch.empty_like(x_bin) if dLdx else None
-        grad_s = torch.empty_like(s_bin) if dLds else None
-        grad_rho = torch.empty_like(rho) if dLdrho else None
-        snap.grid.blur_gradient_backward(x_bin, rho, mass, s_bin, cont(g_blur), cont(g_grad), grad_x, grad_s,
-                                         grad_rho, snap.bin_offsets, snap.block_info, pair_cache=ctx.pairs)
-        return grad_x, grad_s, grad_rho, None, None, None
-
-
-def _zeros_like_shape(shape, dtype, device):
-    return torch.zeros(shape, dtype=dtype, device=device)
-
-
-class Permute(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, s, mass, snapshot):
-        x_bin, s_bin, mass_bin = torch.empty_like(x), torch.empty_like(s), torch.empty_like(mass)
-        snapshot.grid.bin_particles(x, s, mass, snapshot.permutation, x_bin, s_bin, mass_bin)
-        ctx.snapshot = snapshot
-        ctx.meta = (x.shape, s.shape, mass.shape, x.dtype, x.device)
-        ctx.needs = (x.requires_grad, s.requires_grad, mass.requires_grad)
-        return x_bin, s_bin, mass_bin
-
-    @staticmethod
-    def backward(ctx, g_x, g_s, g_m):
-        xs, ss, ms, dtype, device = ctx.meta
-        g_x = _zeros_like_shape(xs, dtype, device) if g_x is None else g_x.contiguous()
-        g_s = _zeros_like_shape(ss, dtype, device) if g_s is None else g_s.contiguous()
-        g_m = _zeros_like_shape(ms, dtype, device) if g_m is None else g_m.contiguous()
-        o_x, o_s, o_m = torch.empty_like(g_x), torch.empty_like(g_s), torch.empty_like(g_m)
-        snap = ctx.snapshot
-        snap.grid.backward_bin_particles(g_x, g_s, g_m, snap.permutation, o_x, o_s, o_m)
-        nx, ns, nm = ctx.needs
-        return (o_x if nx else None, o_s if ns else None, o_m if nm else None, None)
+    def apply(x, s, mass, snapshot):
+        return _ops.reorder(snapshot.grid.native, snapshot.permutation, x, s, mass)
 
 
 def bin_particles(x, s, snapshot, mass=None):
-    no_mass = mass is None
-    out = Permute.apply(x, s, _default_mass(x, mass), snapshot)
-    return out[:2] if no_mass else out
+    return Permute.apply(x, s, _mass(mass), snapshot)
 
 
 def unbin_particles(x_bin, s_bin, snapshot, mass_bin=None):
-    no_mass = mass_bin is None
-    mass_bin = _default_mass(x_bin, mass_bin)
-    x, s, mass = torch.empty_like(x_bin), torch.empty_like(s_bin), torch.empty_like(mass_bin)
-    snapshot.grid.backward_bin_particles(x_bin, s_bin, mass_bin, snapshot.permutation, x, s, mass)
-    return (x, s) if no_mass else (x, s, mass)
+    return _ops.unreorder(snapshot.grid.native, snapshot.permutation, x_bin, s_bin, _mass(mass_bin))
 
 
-class Count(torch.autograd.Function):
+class Count:
     @staticmethod
-    def forward(ctx, x_bin, snapshot):
+    def apply(x_bin, snapshot):
+        # a neighbour count is piecewise constant in the positions: it takes no gradient
         out = torch.empty(x_bin.shape[:-1], dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.count_forward(x_bin, out, snapshot.bin_offsets, snapshot.block_info)
+        snapshot.grid.count_forward(x_bin.detach(), out, snapshot.bin_offsets, snapshot.block_info)
         return out
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        # a neighbour count is piecewise constant in the positions
-        return None, None
 
 
 def count(x_bin, snapshot):
     return Count.apply(x_bin, snapshot)
 
 
-class Density(torch.autograd.Function):
+class Density:
     @staticmethod
-    def forward(ctx, x_bin, mass, snapshot):
-        rho = torch.empty(x_bin.shape[:-1], dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.density_forward(x_bin, mass, rho, snapshot.bin_offsets, snapshot.block_info)
-        ctx.save_for_backward(x_bin, mass)
-        ctx.snapshot = snapshot
-        ctx.dLdx = x_bin.requires_grad
-        return rho
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        if not ctx.dLdx:
-            return None, None, None
-        x_bin, mass = ctx.saved_tensors
-        snap = ctx.snapshot
-        grad_x = torch.empty_like(x_bin)
-        snap.grid.density_backward(x_bin, mass, grad_output.contiguous(), grad_x, snap.bin_offsets,
-                                   snap.block_info, True)
-        return grad_x, None, None
+    def apply(x_bin, mass, snapshot):
+        # the lists recorded here serve every later operator on the same positions, and its own backward
+        pairs, record = _lists_for(snapshot, x_bin)
+        return _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, False, record)[0]
 
 
 def density(x_bin, snapshot, mass=None):
     if _FUSION["enabled"]:
-        pairs = _new_pair_cache(x_bin, True)
-        rho, rho_grad = DensityPair.apply(x_bin, None if mass is None else _default_mass(x_bin, mass), snapshot,
-                                          pairs)
+        rho, rho_grad = DensityPair.apply(x_bin, _mass(mass), snapshot)
         _park(snapshot, "density_gradient", _key(x_bin, mass), rho_grad)
-        if pairs is not None:
-            _park(snapshot, "pair_cache", _key(x_bin), pairs)   # the lists depend on the positions only
         return rho
-    return Density.apply(x_bin, _default_mass(x_bin, mass), snapshot)
+    return Density.apply(x_bin, _mass(mass), snapshot)
 
 
-class _FeatureOp(torch.autograd.Function):
-    """Shared autograd plumbing of Blur and Gradient (inputs x_bin, s_bin, rho, mass, snapshot)."""
-
+class Blur:
     @staticmethod
-    def _forward(ctx, fwd_name, out_tail, x_bin, s_bin, rho, mass, snapshot):
-        out = torch.empty(*s_bin.shape, *out_tail, dtype=torch.float32, device=x_bin.device)
-        getattr(snapshot.grid, fwd_name)(x_bin, rho, mass, s_bin, out, snapshot.bin_offsets, snapshot.block_info)
-        ctx.save_for_backward(x_bin, s_bin, rho, mass)
-        ctx.snapshot = snapshot
-        ctx.needs = (x_bin.requires_grad, s_bin.requires_grad, rho.requires_grad)
-        return out
-
-    @staticmethod
-    def _backward(ctx, bwd_name, grad_output):
-        x_bin, s_bin, rho, mass = ctx.saved_tensors
-        snap = ctx.snapshot
-        dLdx, dLds, dLdrho = ctx.needs
-        grad_x, grad_s, grad_rho = torch.empty_like(x_bin), torch.empty_like(s_bin), torch.empty_like(rho)
-        getattr(snap.grid, bwd_name)(x_bin, rho, mass, s_bin, grad_output.contiguous(), grad_x, grad_s, grad_rho,
-                                     snap.bin_offsets, snap.block_info, dLdx, dLds, dLdrho)
-        return (grad_x if dLdx else None, grad_s if dLds else None, grad_rho if dLdrho else None, None, None)
-
-
-class Blur(_FeatureOp):
-    @staticmethod
-    def forward(ctx, x_bin, s_bin, rho, mass, snapshot):
-        return _FeatureOp._forward(ctx, "blur_forward", (), x_bin, s_bin, rho, mass, snapshot)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        return _FeatureOp._backward(ctx, "blur_backward", grad_output)
+    def apply(x_bin, s_bin, rho, mass, snapshot):
+        pairs = _lists_of(snapshot, x_bin)
+        return _ops.blur_gradient(*_sweep_args(snapshot), x_bin, rho, s_bin, mass, pairs, pairs is not None, True, False, False)[0]
 
 
 def blur(x_bin, rho, s_bin, snapshot, mass=None):
     if _FUSION["enabled"]:
-        s_blur, s_grad, moment = BlurGradient.apply(
-            x_bin, s_bin, rho, None if mass is None else _default_mass(x_bin, mass), snapshot,
-            _claim(snapshot, "pair_cache", x_bin))
+        s_blur, s_grad, moment = BlurGradient.apply(x_bin, s_bin, rho, _mass(mass), snapshot)
         _park(snapshot, "gradient", _key(x_bin, rho, s_bin, mass), s_grad)
         _park(snapshot, "moment_matrix", _key(x_bin, rho, mass), moment)
         return s_blur
-    return Blur.apply(x_bin, s_bin, rho, _default_mass(x_bin, mass), snapshot)
+    return Blur.apply(x_bin, s_bin, rho, _mass(mass), snapshot)
 
 
-class Gradient(_FeatureOp):
+class Gradient:
     @staticmethod
-    def forward(ctx, x_bin, s_bin, rho, mass, snapshot):
-        return _FeatureOp._forward(ctx, "gradient_forward", (snapshot.dim,), x_bin, s_bin, rho, mass, snapshot)
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        return _FeatureOp._backward(ctx, "gradient_backward", grad_output)
+    def apply(x_bin, s_bin, rho, mass, snapshot):
+        pairs = _lists_of(snapshot, x_bin)
+        return _ops.blur_gradient(*_sweep_args(snapshot), x_bin, rho, s_bin, mass, pairs, pairs is not None, False, True, False)[1]
 
 
 def gradient(x_bin, rho, s_bin, snapshot, mass=None):
     parked = _claim(snapshot, "gradient", x_bin, rho, s_bin, mass)
     if parked is not None:
         return parked
-    return Gradient.apply(x_bin, s_bin, rho, _default_mass(x_bin, mass), snapshot)
+    return Gradient.apply(x_bin, s_bin, rho, _mass(mass), snapshot)
 
 
-class DensityGradient(torch.autograd.Function):
+class DensityGradient:
     @staticmethod
-    def forward(ctx, x_bin, mass, snapshot):
-        out = torch.empty(*x_bin.shape[:-1], snapshot.dim, dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.density_gradient_forward(x_bin, mass, out, snapshot.bin_offsets, snapshot.block_info)
-        ctx.save_for_backward(x_bin, mass)
-        ctx.snapshot = snapshot
-        ctx.dLdx = x_bin.requires_grad
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        if not ctx.dLdx:
-            return None, None, None
-        x_bin, mass = ctx.saved_tensors
-        snap = ctx.snapshot
-        grad_x = torch.empty_like(x_bin)
-        snap.grid.density_gradient_backward(x_bin, mass, grad_output.contiguous(), grad_x, snap.bin_offsets,
-                                            snap.block_info, True)
-        return grad_x, None, None
+    def apply(x_bin, mass, snapshot):
+        return _ops.density(*_sweep_args(snapshot), x_bin, mass, _lists_of(snapshot, x_bin), False, True, False)[1]
 
 
 def density_gradient(x_bin, snapshot, mass=None):
     parked = _claim(snapshot, "density_gradient", x_bin, mass)
     if parked is not None:
         return parked
-    return DensityGradient.apply(x_bin, _default_mass(x_bin, mass), snapshot)
+    return DensityGradient.apply(x_bin, _mass(mass), snapshot)
 
 
-class MomentMatrix(torch.autograd.Function):
+class MomentMatrix:
     @staticmethod
-    def forward(ctx, x_bin, rho, mass, snapshot):
-        dim = snapshot.dim
-        out = torch.empty(*x_bin.shape[:-1], dim, dim, dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.moment_matrix_forward(x_bin, rho, mass, out, snapshot.bin_offsets, snapshot.block_info)
-        ctx.save_for_backward(x_bin, rho, mass)
-        ctx.snapshot = snapshot
-        ctx.needs = (x_bin.requires_grad, rho.requires_grad)
-        return out
-
-    @staticmethod
-    def backward(ctx, grad_output):
-        x_bin, rho, mass = ctx.saved_tensors
-        snap = ctx.snapshot
-        dLdx, dLdrho = ctx.needs
-        grad_x, grad_rho = torch.empty_like(x_bin), torch.empty_like(rho)
-        snap.grid.moment_matrix_backward(x_bin, rho, mass, grad_output.contiguous(), grad_x, grad_rho,
-                                         snap.bin_offsets, snap.block_info, dLdx, dLdrho)
-        return (grad_x if dLdx else None, grad_rho if dLdrho else None, None, None)
+    def apply(x_bin, rho, mass, snapshot):
+        return _ops.moment_matrix(*_sweep_args(snapshot), x_bin, rho, mass)
 
 
 def moment_matrix(x_bin, rho, snapshot, mass=None):
@@ -470,7 +320,7 @@ def moment_matrix(x_bin, rho, snapshot, mass=None):
         parked = _claim(snapshot, "moment_matrix", x_bin, rho, mass)
         if parked is not None:
             return parked
-    return MomentMatrix.apply(x_bin, rho, _default_mass(x_bin, mass), snapshot)
+    return MomentMatrix.apply(x_bin, rho, _mass(mass), snapshot)
 
 
 @torch.no_grad()
@@ -484,18 +334,14 @@ def gradient_hybrid(x_bin, rho, s_bin, snapshot, mass=None):
     """Moment-corrected gradient: value ``raw @ inv(M)``, gradient of the raw SPH gradient."""
     with torch.no_grad():
         M = moment_matrix(x_bin, rho, snapshot, mass=mass)
-        if snapshot.dim in (2, 3):
-            L = safe_inv_sym_mat(M, rtol=1e-3)
-        else:
-            L = torch.linalg.pinv(M, hermitian=True, rtol=1e-3)
     raw = gradient(x_bin, rho, s_bin, snapshot, mass=mass)
-    return raw + (raw @ L - raw).detach()
+    return _ops.corrected_gradient(raw, M, 1e-3)
 
 
 # ---------------------------------------------------------------------------------------------
 # Fused perception step (extension; the reference issues one launch per operator).
 # ---------------------------------------------------------------------------------------------
-class Perception(torch.autograd.Function):
+class Perception:
     """rho = density(x); blur(x, rho, s); gradient(x, rho, s); density_gradient(x) as one node.
 
     Forward runs two sweeps over the neighbour cells instead of four launches; backward runs the
@@ -503,42 +349,8 @@ class Perception(torch.autograd.Function):
     """
 
     @staticmethod
-    def forward(ctx, x_bin, s_bin, mass, snapshot, want_density_gradient):
-        B, N, C = s_bin.shape
-        dev, dim = x_bin.device, snapshot.dim
-        rho = torch.empty(B, N, dtype=torch.float32, device=dev)
-        s_blur = torch.empty_like(s_bin)
-        s_grad = torch.empty(B, N, C, dim, dtype=torch.float32, device=dev)
-        rho_grad = torch.empty(B, N, dim, dtype=torch.float32, device=dev) if want_density_gradient else None
-        pairs = _new_pair_cache(s_bin, x_bin.requires_grad or s_bin.requires_grad)
-        snapshot.grid.perception_forward(x_bin, mass, s_bin, rho, None, rho_grad, s_blur, s_grad, None,
-                                         snapshot.bin_offsets, snapshot.block_info, pair_cache=pairs)
-        ctx.pairs = pairs
-        ctx.save_for_backward(x_bin, s_bin, rho, *([] if mass is None else [mass]))
-        ctx.has_mass = mass is not None
-        ctx.snapshot = snapshot
-        ctx.needs = (x_bin.requires_grad, s_bin.requires_grad)
-        ctx.want_dg = want_density_gradient
-        if want_density_gradient:
-            return rho, s_blur, s_grad, rho_grad
-        return rho, s_blur, s_grad
-
-    @staticmethod
-    def backward(ctx, g_rho, g_blur, g_grad, g_rho_grad=None):
-        saved = ctx.saved_tensors
-        x_bin, s_bin, rho = saved[:3]
-        mass = saved[3] if ctx.has_mass else None
-        dLdx, dLds = ctx.needs
-        snap = ctx.snapshot
-        cont = lambda t: None if t is None else t.contiguous()
-        grad_x = torch.empty_like(x_bin) if dLdx else None
-        grad_s = torch.empty_like(s_bin) if dLds else None
-        scratch = torch.empty_like(rho) if dLdx else None
-        if dLdx or dLds:
-            snap.grid.perception_backward(x_bin, mass, s_bin, rho, cont(g_rho) if dLdx else None, cont(g_blur),
-                                          cont(g_grad), cont(g_rho_grad) if dLdx else None, grad_x, grad_s,
-                                          scratch, snap.bin_offsets, snap.block_info, pair_cache=ctx.pairs)
-        return grad_x, grad_s, None, None, None
+    def apply(x_bin, s_bin, mass, snapshot, want_density_gradient):
+        return _ops.perception(*_sweep_args(snapshot), x_bin, s_bin, mass, want_density_gradient, _columns(snapshot.grid))
 
 
 def perceive(x_bin, s_bin, snapshot, mass=None, with_density_gradient=True):
@@ -548,57 +360,16 @@ def perceive(x_bin, s_bin, snapshot, mass=None, with_density_gradient=True):
     ``gradient(x_bin, rho, s_bin, ...)`` and ``density_gradient(x_bin, ...)`` with gradients
     flowing through ``rho`` into ``x_bin``.
     """
-    if mass is not None:
-        mass = _default_mass(x_bin, mass)
-    return Perception.apply(x_bin, s_bin, mass, snapshot, with_density_gradient)
+    return Perception.apply(x_bin, s_bin, _mass(mass), snapshot, with_density_gradient)
 
 
-class PerceiveFeatures(torch.autograd.Function):
+class PerceiveFeatures:
     """The packed perception row of NPA.perceive (models/npa.py:87-137) as one autograd node."""
 
     @staticmethod
-    def forward(ctx, x_bin, s_bin, mass, snapshot, coef, dg_scale, inv_tol, log_norm_grad, log_norm_dg):
-        B, N, C = s_bin.shape
-        dev, D = x_bin.device, snapshot.dim
-        f32 = dict(dtype=torch.float32, device=dev)
-        rho = torch.empty(B, N, **f32)
-        rho_grad = torch.empty(B, N, D, **f32)
-        z = torch.empty(B, N, 2 * C + C * D + D, **f32)
-        keep = x_bin.requires_grad or s_bin.requires_grad
-        vgrad = torch.empty(B, N, C, D, **f32) if keep else None
-        pairs = _new_pair_cache(s_bin, keep)
-        snapshot.grid.perceive_features_forward(x_bin, mass, s_bin, coef, dg_scale, inv_tol, log_norm_grad,
-                                                log_norm_dg, rho, rho_grad, z, vgrad, snapshot.bin_offsets,
-                                                snapshot.block_info, pair_cache=pairs)
-        ctx.pairs = pairs
-        if keep:
-            ctx.save_for_backward(x_bin, s_bin, rho, rho_grad, vgrad, *([] if mass is None else [mass]))
-        ctx.has_mass = mass is not None
-        ctx.snapshot = snapshot
-        ctx.consts = (coef, dg_scale, log_norm_grad, log_norm_dg)
-        ctx.needs = (x_bin.requires_grad, s_bin.requires_grad)
-        return z
-
-    @staticmethod
-    def backward(ctx, g_z):
-        dLdx, dLds = ctx.needs
-        if not (dLdx or dLds):
-            return (None,) * 9
-        saved = ctx.saved_tensors
-        x_bin, s_bin, rho, rho_grad, vgrad = saved[:5]
-        mass = saved[5] if ctx.has_mass else None
-        coef, dg_scale, ln_g, ln_dg = ctx.consts
-        snap = ctx.snapshot
-        g_blur = torch.empty_like(s_bin)
-        g_grad = torch.empty_like(vgrad)
-        grad_x = torch.empty_like(x_bin) if dLdx else None
-        grad_s = torch.empty_like(s_bin)
-        g_rho_grad = torch.empty_like(rho_grad) if dLdx else None
-        grad_rho = torch.empty_like(rho) if dLdx else None
-        snap.grid.perceive_features_backward(x_bin, mass, s_bin, rho, rho_grad, vgrad, g_z.contiguous(), coef,
-                                             dg_scale, ln_g, ln_dg, g_blur, g_grad, g_rho_grad, grad_rho, grad_x,
-                                             grad_s, snap.bin_offsets, snap.block_info, pair_cache=ctx.pairs)
-        return (grad_x, grad_s if dLds else None) + (None,) * 7
+    def apply(x_bin, s_bin, mass, snapshot, coef, dg_scale, inv_tol, log_norm_grad, log_norm_dg):
+        return _ops.packed_perception(*_sweep_args(snapshot), x_bin, s_bin, mass, coef, dg_scale, inv_tol, log_norm_grad, log_norm_dg,
+                                      _columns(snapshot.grid))
 
 
 def perceive_features(x_bin, s_bin, snapshot, eps0, mass=None, log_norm_grad=True, log_norm_density_grad=True,
@@ -610,8 +381,7 @@ def perceive_features(x_bin, s_bin, snapshot, eps0, mass=None, log_norm_grad=Tru
     with ``coef = eps / eps0`` and ``LN(w) = log(1+|w|) w/|w|`` (skipped when the flag is False).
     Pass ``x_bin.detach()`` to stop gradients into the positions, as NPA does by default.
     """
-    if mass is not None:
-        mass = _default_mass(x_bin, mass)
+    mass = _mass(mass)
     B, N, C = s_bin.shape
     coef = float(snapshot.grid.eps) / float(eps0)
     dg_scale = coef ** (1 + snapshot.dim) / N
@@ -635,34 +405,13 @@ def perceive_features(x_bin, s_bin, snapshot, eps0, mass=None, log_norm_grad=Tru
                                   bool(log_norm_grad), bool(log_norm_density_grad))
 
 
-class StepUpdate(torch.autograd.Function):
+class StepUpdate:
     """The Euler update of step_euler (models/npa.py:183-203) with the displacement limiter of
     NPA.forward (models/npa.py:145-153) as one elementwise kernel and one autograd node."""
 
     @staticmethod
-    def forward(ctx, y, x_bin, s_bin, mask, snapshot, alpha, dt, wrap):
-        x_out, s_out = torch.empty_like(x_bin), torch.empty_like(s_bin)
-        snapshot.grid.step_update_forward(y, x_bin, s_bin, mask, alpha, dt, wrap, x_out, s_out)
-        ctx.save_for_backward(y, *([] if mask is None else [mask]))
-        ctx.has_mask = mask is not None
-        ctx.snapshot = snapshot
-        ctx.consts = (s_bin.shape[2], alpha, dt)
-        ctx.needs = (y.requires_grad, x_bin.requires_grad, s_bin.requires_grad)
-        return x_out, s_out
-
-    @staticmethod
-    def backward(ctx, g_x, g_s):
-        y = ctx.saved_tensors[0]
-        mask = ctx.saved_tensors[1] if ctx.has_mask else None
-        need_y, need_x, need_s = ctx.needs
-        C, alpha, dt = ctx.consts
-        g_x = g_x.contiguous() if g_x is not None else None
-        g_s = g_s.contiguous() if g_s is not None else None
-        g_y = None
-        if need_y:
-            g_y = torch.empty_like(y)
-            ctx.snapshot.grid.step_update_backward(y, mask, C, alpha, dt, g_x, g_s, g_y)
-        return g_y, (g_x if need_x else None), (g_s if need_s else None), None, None, None, None, None
+    def apply(y, x_bin, s_bin, mask, snapshot, alpha, dt, wrap):
+        return _ops.step_update(snapshot.grid.native, y, x_bin, s_bin, mask, alpha, dt, wrap)
 
 
 def step_update(y, x_bin, s_bin, snapshot, alpha, dt=1.0, update_mask=None, wrap=False):

@@ -81,6 +81,13 @@ class _HashGridBase:
         self._B, self._N, self._P = batch_size, particle_count, (2 if dim == 2 else 4)
         self._eps = eps
         self._mpb = mpb
+        # Columns of a neighbour list (one count + the neighbours): room for 1.6 times the mean number of neighbours
+        # of particles that fill the grid evenly, at least 127 (a particle with more searches the cells again), so
+        # that long-range grids -- 128 neighbours in a 10 x 10 periodic box of 4,096 particles -- fit as well.
+        ball = 3.14159265 if dim == 2 else 4.18879020
+        mean = ball * particle_count / self._cells
+        self.list_columns = 128 if mean <= 79 else min(512, -(-int(1.6 * mean + 1) // 64) * 64)
+        self.native = N.ops.Grid(ctypes.addressof(self._desc))  # what the autograd nodes take (csrc/torch_ops.cpp)
 
     # ---- read-only properties of the nanobind classes ----------------------
     grid_size_x = property(lambda self: self._sizes[0])
@@ -123,7 +130,11 @@ class _HashGridBase:
 
     @staticmethod
     def _call(fn, tensor_for_device, *args):
-        with torch.cuda.device(tensor_for_device.device):
+        device = tensor_for_device.device.index
+        if device == torch.cuda.current_device():  # switching devices costs more than a launch
+            N.check(fn(*args, ctypes.c_void_p(torch._C._cuda_getCurrentRawStream(device))))
+            return
+        with torch.cuda.device(device):
             N.check(fn(*args, N.current_stream()))
 
     # ---- binning ---------------------------------------------------------------

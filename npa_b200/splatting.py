@@ -14,8 +14,6 @@ import torch
 
 from . import _native as N
 
-_lib = N.lib
-
 
 def _derived(img_size, sigma, lo, hi, normalize_color, pixel_size):
     """sigma in pixels, patch radius and colour scale exactly as utils/splatting.py:43-46,75-77."""
@@ -25,37 +23,6 @@ def _derived(img_size, sigma, lo, hi, normalize_color, pixel_size):
         scale = (img_size * pixel_size / (hi - lo)) ** 2.0
     radius = max(1, math.ceil(5 * float(sigma)))
     return float(sigma), int(radius), float(scale)
-
-
-class _Splat(torch.autograd.Function):
-    @staticmethod
-    def forward(ctx, x, color, img_size, sigma_pix, radius, lo, hi, y_up, normalize, scale):
-        B, n = x.shape[0], x.shape[1]
-        out = torch.empty(B, img_size, img_size, 4, dtype=torch.float32, device=x.device)
-        scratch = torch.empty(B, n, dtype=torch.float32, device=x.device) if normalize else None
-        with torch.cuda.device(x.device):
-            N.check(_lib.npa_splat_forward(N.ptr(x), N.ptr(color), B, n, img_size, sigma_pix, radius, lo, hi,
-                                           1 if y_up else 0, 1 if normalize else 0, scale, N.ptr(scratch), N.ptr(out),
-                                           N.current_stream()))
-        ctx.save_for_backward(x, color)
-        ctx.consts = (img_size, sigma_pix, radius, lo, hi, y_up, normalize, scale)
-        return out
-
-    @staticmethod
-    def backward(ctx, g_out):
-        x, color = ctx.saved_tensors
-        img_size, sigma_pix, radius, lo, hi, y_up, normalize, scale = ctx.consts
-        need_x, need_c = ctx.needs_input_grad[0], ctx.needs_input_grad[1]
-        if not (need_x or need_c):
-            return (None,) * 10
-        g_out = g_out.contiguous()
-        g_x = torch.empty_like(x) if need_x else None
-        g_c = torch.empty_like(color) if need_c else None
-        with torch.cuda.device(x.device):
-            N.check(_lib.npa_splat_backward(N.ptr(x), N.ptr(color), N.ptr(g_out), x.shape[0], x.shape[1], img_size,
-                                            sigma_pix, radius, lo, hi, 1 if y_up else 0, 1 if normalize else 0, scale,
-                                            N.ptr(g_x), N.ptr(g_c), N.current_stream()))
-        return (g_x, g_c) + (None,) * 8
 
 
 def _check(x, color):
@@ -73,8 +40,9 @@ def splat_particles_batch(x, color, img_size=256, sigma=2.0, lo=-1.0, hi=1.0, no
     ``[B, img_size, img_size, 4]`` with channels ``(r, g, b, density)``; one launch for the batch."""
     _check(x, color)
     sigma_pix, radius, scale = _derived(img_size, sigma, lo, hi, normalize_color, pixel_size)
-    return _Splat.apply(x.contiguous(), color[..., -3:].contiguous(), int(img_size), sigma_pix, radius, float(lo),
-                        float(hi), bool(y_up), bool(normalize_color), scale)
+    rgb = color if color.shape[-1] == 3 else color[..., -3:]
+    return N.ops.splat(x.contiguous(), rgb.contiguous(), int(img_size), sigma_pix, radius, float(lo), float(hi),
+                       bool(y_up), bool(normalize_color), scale)
 
 
 def splat_particles(x, color, img_size=256, sigma=2.0, lo=-1.0, hi=1.0, normalize_color=True, y_up=False,
