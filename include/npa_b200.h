@@ -370,6 +370,47 @@ int npa_perceive_features_backward(const npa_grid *g, int32_t channels, const fl
                                    const int32_t *bin_offsets, const int32_t *block_info,
                                    const int32_t *pair_cache, int32_t pair_stride, void *stream);
 
+/* ---- the same operators over neighbour lists, with work memory ------------------ *
+ * The calls above take the lists as an option; these need them (pair_cache [B*N, pair_stride] filled by the density
+ * sweep of the same positions) and use memory of the caller to move less:
+ *   packed   [B*N, 4] floats, 16-byte aligned: (x, y, z, m / rho) of every particle, written by the forward calls and
+ *            read by the sweeps after it; may be NULL;
+ *   scratch  npa_lists_backward_scratch_bytes(g, channels) bytes, 16-byte aligned, private to the call.
+ * No block_info is needed where it is not an argument.  Same results as the calls they stand for. */
+int64_t npa_lists_backward_scratch_bytes(const npa_grid *g, int32_t channels);
+int npa_perception_forward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass, const float *s_bin,
+                                 float *rho, float *rho_grad, float *s_blur, float *s_grad, float *packed,
+                                 const int32_t *bin_offsets, const int32_t *block_info, int32_t *pair_cache,
+                                 int32_t pair_stride, void *stream);
+int npa_perception_backward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
+                                  const float *s_bin, const float *rho, const float *packed, const float *dL_drho_out,
+                                  const float *dL_dblur, const float *dL_dgrad, const float *dL_drho_grad, float *grad_x,
+                                  float *grad_s, void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
+                                  const int32_t *pair_cache, int32_t pair_stride, void *stream);
+int npa_blur_gradient_backward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *rho,
+                                     const float *mass, const float *s_bin, const float *dL_dblur, const float *dL_dgrad,
+                                     float *grad_x, float *grad_s, float *grad_rho, void *scratch, int64_t scratch_bytes,
+                                     const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream);
+int npa_density_gradient_forward_lists(const npa_grid *g, const float *x_bin, const float *mass, float *rho_grad,
+                                       const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride,
+                                       void *stream);
+/* out[B,N,C,D] = gradient . inv(moment matrix), the value of gradient_hybrid (sphops/sph.py:474-484), in one sweep. */
+int npa_gradient_hybrid_forward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *rho,
+                                      const float *mass, const float *s_bin, float inv_tol, float *out,
+                                      const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride,
+                                      void *stream);
+int npa_perceive_features_forward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
+                                        const float *s_bin, float coef, float dg_scale, float inv_tol,
+                                        int32_t log_norm_grad, int32_t log_norm_dg, float *rho, float *rho_grad, float *z,
+                                        float *vgrad, float *packed, const int32_t *bin_offsets, const int32_t *block_info,
+                                        int32_t *pair_cache, int32_t pair_stride, void *stream);
+int npa_perceive_features_backward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
+                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                         const float *packed, const float *dL_dz, float coef, float dg_scale,
+                                         int32_t log_norm_grad, int32_t log_norm_dg, float *grad_x, float *grad_s,
+                                         void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
+                                         const int32_t *pair_cache, int32_t pair_stride, void *stream);
+
 /* ---- the Euler update after perception and the per-particle MLP ----------------- *
  * Replaces the elementwise torch code of NPA.forward (models/npa.py:145-153, the
  * displacement limiter) and of step_euler (models/npa.py:183-203) and, with

@@ -74,6 +74,16 @@ SIGNATURES = {
                                                      ctypes.c_float, _I32, _I32, _P, _P, _P, _P, _P, _P, _P, _I32, _P]),
     "npa_perceive_features_backward": (ctypes.c_int, [_P, _I32] + [_P] * 7 + [ctypes.c_float, ctypes.c_float, _I32, _I32]
                                        + [_P] * 8 + [_P, _I32, _P]),
+    "npa_lists_backward_scratch_bytes": (_I64, [_P, _I32]),
+    "npa_perception_forward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 11 + [_I32, _P]),
+    "npa_perception_backward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 11 + [_P, _I64, _P, _P, _I32, _P]),
+    "npa_blur_gradient_backward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 9 + [_P, _I64, _P, _P, _I32, _P]),
+    "npa_density_gradient_forward_lists": (ctypes.c_int, [_P] * 6 + [_I32, _P]),
+    "npa_gradient_hybrid_forward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 4 + [ctypes.c_float] + [_P] * 3 + [_I32, _P]),
+    "npa_perceive_features_forward_lists": (ctypes.c_int, [_P, _I32, _P, _P, _P, ctypes.c_float, ctypes.c_float, ctypes.c_float,
+                                                           _I32, _I32] + [_P] * 8 + [_I32, _P]),
+    "npa_perceive_features_backward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 8 + [ctypes.c_float, ctypes.c_float, _I32, _I32]
+                                             + [_P] * 3 + [_I64, _P, _P, _I32, _P]),
     "npa_perception_forward": (ctypes.c_int, [_P, _I32] + [_P] * 11 + [_P, _I32, _P]),
     "npa_perception_backward": (ctypes.c_int, [_P, _I32] + [_P] * 13 + [_P, _I32, _P]),
     "npa_step_update_forward": (ctypes.c_int, [_P] * 5 + [_I32, ctypes.c_float, ctypes.c_float, _I32, _P, _P, _P]),

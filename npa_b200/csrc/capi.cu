@@ -142,6 +142,16 @@ static int check_grad_x(const char *name, const Geom &g, const float *grad_x) {
     return NPA_OK;
 }
 
+// Checks of an operator over neighbour lists.
+static int begin_lists(const char *name, const npa_grid *gd, Geom *g, const float *x, const int32_t *bin_offsets, const void *lists, int stride) {
+    int rc = make_geom(gd, g);
+    if (rc != NPA_OK) return rc;
+    if (!x || !bin_offsets || !lists) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: binned_positions, bin_offsets or pair_cache is NULL", name);
+    if ((uintptr_t)x % (g->dim == 2 ? 8 : 16))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: binned_positions must be aligned to one position (%d bytes)", name, g->dim == 2 ? 8 : 16);
+    return check_pair_cache(name, lists, stride);
+}
+
 }  // namespace npa
 
 using namespace npa;
@@ -352,9 +362,166 @@ int npa_density_chain_backward(const npa_grid *gd, const float *x_bin, const flo
     const int mask = ((dL_drho_a || dL_drho_b) ? S_DENSITY : 0) | (dL_drho_grad ? S_DGRAD : 0);
     if (!mask) return fail(NPA_ERR_INVALID_ARGUMENT, "density_chain_backward: every upstream gradient is NULL");
     if ((rc = check_pair_cache("density_chain_backward", pair_cache, pair_stride)) != NPA_OK) return rc;
+    if (pair_cache) {
+        ScalarListArgs l = {};
+        l.x = x_bin; l.mass = mass; l.g_rho_a = dL_drho_a; l.g_rho_b = dL_drho_b; l.g_dg = dL_drho_grad; l.grad_x = grad_x;
+        l.accumulate_x = accumulate ? 1 : 0; l.bin_offsets = bin_offsets; l.pair_cache = pair_cache; l.pair_stride = pair_stride;
+        return launch_scalar_list_backward(g, l, (cudaStream_t)stream);
+    }
     ScalarBwdArgs a = {x_bin, mass, nullptr, dL_drho_a, dL_drho_b, dL_drho_grad, nullptr, grad_x, nullptr,
-                       accumulate ? 1 : 0, bin_offsets, block_info, pair_cache, pair_stride};
+                       accumulate ? 1 : 0, bin_offsets, block_info};
     return launch_scalar_backward(g, mask, a, (cudaStream_t)stream);
+}
+
+int npa_density_gradient_forward_lists(const npa_grid *gd, const float *x_bin, const float *mass, float *rho_grad, const int32_t *bin_offsets,
+                                       const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "density_gradient_forward_lists";
+    Geom g;
+    int rc = begin_lists(me, gd, &g, x_bin, bin_offsets, pair_cache, pair_stride);
+    if (rc != NPA_OK) return rc;
+    NPA_REQUIRE(rho_grad, me, "density_gradient_out");
+    ScalarListArgs l = {};
+    l.x = x_bin; l.mass = mass; l.rho_grad_out = rho_grad; l.bin_offsets = bin_offsets; l.pair_cache = pair_cache; l.pair_stride = pair_stride;
+    return launch_density_gradient_list(g, l, (cudaStream_t)stream);
+}
+
+int npa_gradient_hybrid_forward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *rho, const float *mass,
+                                      const float *s_bin, float inv_tol, float *out, const int32_t *bin_offsets,
+                                      const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "gradient_hybrid_forward_lists";
+    Geom g;
+    int rc = begin_lists(me, gd, &g, x_bin, bin_offsets, pair_cache, pair_stride);
+    if (rc != NPA_OK || (rc = check_channels(me, channels)) != NPA_OK) return rc;
+    NPA_REQUIRE(rho, me, "rho");
+    NPA_REQUIRE(s_bin, me, "state_in");
+    NPA_REQUIRE(out, me, "state_gradient_out");
+    FeatureFwdArgs a = {x_bin, mass, rho, s_bin, nullptr, out, channels, bin_offsets, nullptr, nullptr};
+    a.inv_tol = inv_tol;
+    a.pair_cache = const_cast<int32_t *>(pair_cache);
+    a.pair_stride = pair_stride;
+    a.pair_cache_valid = 1;
+    return launch_feature_list_forward(g, F_GRAD | F_MOMENT | F_CORRECTED, a, (cudaStream_t)stream);
+}
+
+int npa_perception_forward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass, const float *s_bin, float *rho,
+                                 float *rho_grad, float *s_blur, float *s_grad, float *packed, const int32_t *bin_offsets,
+                                 const int32_t *block_info, int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "perception_forward_lists";
+    Geom g;
+    int rc = begin_lists(me, gd, &g, x_bin, bin_offsets, pair_cache, pair_stride);
+    if (rc != NPA_OK || (rc = check_channels(me, channels)) != NPA_OK) return rc;
+    NPA_REQUIRE(block_info, me, "block_info");
+    NPA_REQUIRE(rho, me, "rho");
+    NPA_REQUIRE(s_bin, me, "state_in");
+    NPA_REQUIRE(s_blur, me, "state_out");
+    NPA_REQUIRE(s_grad, me, "state_gradient_out");
+    if ((uintptr_t)packed % 16 || (uintptr_t)block_info % 16)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: packed and block_info must be 16-byte aligned", me);
+    cudaStream_t st = (cudaStream_t)stream;
+    ScalarFwdArgs sa = {x_bin, mass, nullptr, nullptr, rho, nullptr, nullptr, bin_offsets, block_info, pair_cache, pair_stride};
+    sa.pv = reinterpret_cast<float4 *>(packed);
+    if ((rc = launch_scalar_forward(g, S_DENSITY, sa, st)) != NPA_OK) return rc;
+    // the feature sweep meets every pair with its spiky kernel value in hand: the density gradient rides along
+    FeatureFwdArgs fa = {x_bin, mass, rho, s_bin, s_blur, s_grad, channels, bin_offsets, block_info, nullptr};
+    fa.pv = sa.pv;
+    fa.rho_grad_out = rho_grad;
+    fa.pair_cache = pair_cache;
+    fa.pair_stride = pair_stride;
+    fa.pair_cache_valid = 1;
+    return launch_feature_list_forward(g, F_BLUR | F_GRAD | (rho_grad ? F_DGRAD : 0), fa, st);
+}
+
+// Upstream gradients in the layout the list kernels read: the gradient's are laid out anew in `rows`, the blur's are
+// read where they are when their rows are 16-byte addressable.
+static int lay_out_upstreams(const Geom &g, int C, const float *g_blur, const float *g_grad, float *rows, FeatureListBwdArgs &a, cudaStream_t st) {
+    const int cp = (C + 3) & ~3;
+    const bool copy_blur = g_blur && (C % 4 != 0 || (uintptr_t)g_blur % 16 != 0);
+    a.cp = cp;
+    a.gb = copy_blur ? rows : g_blur;
+    a.gb_pitch = copy_blur ? (1 + (g_grad ? g.dim : 0)) * cp : C;
+    a.gg = g_grad ? rows + (copy_blur ? cp : 0) : nullptr;
+    a.gg_pitch = ((copy_blur ? 1 : 0) + g.dim) * cp;
+    if (!copy_blur && !g_grad) return NPA_OK;
+    return launch_upstream_rows(g, C, g_blur, g_grad, copy_blur, rows, st);
+}
+
+static int check_scratch(const char *me, const npa_grid *gd, int C, const void *scratch, int64_t bytes) {
+    if (!scratch || (uintptr_t)scratch % 16) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: scratch must be non-NULL and 16-byte aligned", me);
+    const int64_t need = npa_lists_backward_scratch_bytes(gd, C);
+    if (bytes < need) return fail(NPA_ERR_SCRATCH_TOO_SMALL, "%s: scratch holds %lld bytes, %lld needed", me, (long long)bytes, (long long)need);
+    return NPA_OK;
+}
+
+int npa_blur_gradient_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *rho, const float *mass,
+                                     const float *s_bin, const float *dL_dblur, const float *dL_dgrad, float *grad_x, float *grad_s,
+                                     float *grad_rho, void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
+                                     const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "blur_gradient_backward_lists";
+    Geom g;
+    int rc = begin_lists(me, gd, &g, x_bin, bin_offsets, pair_cache, pair_stride);
+    if (rc != NPA_OK || (rc = check_channels(me, channels)) != NPA_OK || (rc = check_grad_x(me, g, grad_x)) != NPA_OK) return rc;
+    if (!grad_x && !grad_s && !grad_rho) return NPA_OK;
+    NPA_REQUIRE(rho, me, "rho");
+    NPA_REQUIRE(s_bin, me, "state_in");
+    const int mask = (dL_dblur ? F_BLUR : 0) | (dL_dgrad ? F_GRAD : 0);
+    if (!mask) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: both upstream gradients are NULL", me);
+    if ((rc = check_scratch(me, gd, channels, scratch, scratch_bytes)) != NPA_OK) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    FeatureListBwdArgs a = {};
+    a.x = x_bin; a.mass = mass; a.rho = rho; a.s = s_bin; a.grad_x = grad_x; a.grad_s = grad_s; a.grad_rho = grad_rho; a.C = channels;
+    a.bin_offsets = bin_offsets; a.pair_cache = pair_cache; a.pair_stride = pair_stride;
+    if ((rc = lay_out_upstreams(g, channels, dL_dblur, dL_dgrad, static_cast<float *>(scratch), a, st)) != NPA_OK) return rc;
+    return launch_feature_list_backward(g, mask, grad_x || grad_rho, a, st);
+}
+
+int npa_perception_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass, const float *s_bin,
+                                  const float *rho, const float *packed, const float *dL_drho_out, const float *dL_dblur,
+                                  const float *dL_dgrad, const float *dL_drho_grad, float *grad_x, float *grad_s, void *scratch,
+                                  int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride,
+                                  void *stream) {
+    const char *me = "perception_backward_lists";
+    Geom g;
+    int rc = begin_lists(me, gd, &g, x_bin, bin_offsets, pair_cache, pair_stride);
+    if (rc != NPA_OK || (rc = check_channels(me, channels)) != NPA_OK || (rc = check_grad_x(me, g, grad_x)) != NPA_OK) return rc;
+    if ((uintptr_t)packed % 16) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: packed must be 16-byte aligned", me);
+    if ((rc = check_scratch(me, gd, channels, scratch, scratch_bytes)) != NPA_OK) return rc;
+    cudaStream_t st = (cudaStream_t)stream;
+    const int mask = (dL_dblur ? F_BLUR : 0) | (dL_dgrad ? F_GRAD : 0);
+    const long long n = (long long)g.B * g.N;
+    ScalarListArgs d = {};
+    d.x = x_bin; d.mass = mass; d.grad_x = grad_x; d.bin_offsets = bin_offsets; d.pair_cache = pair_cache; d.pair_stride = pair_stride;
+    if (mask && (grad_s || grad_x)) {
+        NPA_REQUIRE(s_bin, me, "state_in");
+        NPA_REQUIRE(rho, me, "rho");
+        float *rows = static_cast<float *>(scratch);
+        FeatureListBwdArgs a = {};
+        a.x = x_bin; a.mass = mass; a.rho = rho; a.s = s_bin; a.pv = reinterpret_cast<const float4 *>(packed);
+        a.grad_x = grad_x; a.grad_s = grad_s; a.C = channels;
+        a.bin_offsets = bin_offsets; a.pair_cache = pair_cache; a.pair_stride = pair_stride;
+        if (grad_x) {
+            a.g_dg = dL_drho_grad;
+            a.g_rho = dL_drho_out;
+            a.pg = reinterpret_cast<float4 *>(rows + n * (1 + g.dim) * ((channels + 3) & ~3));
+        }
+        if ((rc = lay_out_upstreams(g, channels, dL_dblur, dL_dgrad, rows, a, st)) != NPA_OK) return rc;
+        if ((rc = launch_feature_list_backward(g, mask, grad_x != nullptr, a, st)) != NPA_OK || !grad_x) return rc;
+        d.pg = a.pg;
+        d.accumulate_x = 1;
+        return launch_scalar_list_backward(g, d, st);
+    }
+    if (grad_s) {
+        cudaError_t e = cudaMemsetAsync(grad_s, 0, sizeof(float) * (size_t)n * channels, st);
+        if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "cudaMemsetAsync(grad_s): %s", cudaGetErrorString(e));
+    }
+    if (!grad_x) return NPA_OK;
+    if (!dL_drho_out && !dL_drho_grad) {
+        cudaError_t e = cudaMemsetAsync(grad_x, 0, sizeof(float) * (size_t)n * (g.dim == 2 ? 2 : 4), st);
+        if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "cudaMemsetAsync(grad_x): %s", cudaGetErrorString(e));
+        return NPA_OK;
+    }
+    d.g_rho_a = dL_drho_out;
+    d.g_dg = dL_drho_grad;
+    return launch_scalar_list_backward(g, d, st);
 }
 
 int npa_perception_forward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
@@ -434,9 +601,9 @@ int npa_perception_backward(const npa_grid *gd, int32_t channels, const float *x
         const float *gb = x_written ? grad_rho_scratch : nullptr;
         const int smask = ((ga || gb) ? S_DENSITY : 0) | (dL_drho_grad ? S_DGRAD : 0);
         if (smask) {
-            ScalarBwdArgs sa = {x_bin, mass, nullptr, ga, gb, dL_drho_grad, nullptr, grad_x, nullptr,
-                                x_written ? 1 : 0, bin_offsets, block_info, pair_cache, pair_stride};
-            if ((rc = launch_scalar_backward(g, smask, sa, st)) != NPA_OK) return rc;
+            rc = npa_density_chain_backward(gd, x_bin, mass, ga, gb, dL_drho_grad, grad_x, x_written ? 1 : 0, bin_offsets, block_info, pair_cache,
+                                            pair_stride, stream);
+            if (rc != NPA_OK) return rc;
         } else if (!x_written) {
             cudaError_t e = cudaMemsetAsync(grad_x, 0, sizeof(float) * (size_t)g.B * g.N * (g.dim == 2 ? 2 : 4), st);
             if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "cudaMemsetAsync(grad_x): %s", cudaGetErrorString(e));

@@ -117,11 +117,6 @@ __device__ inline void collect_pairs(const Geom &g, const float *__restrict__ x,
     flush(n);
 }
 
-// Stage 1 from a cached neighbour list (written by the forward sweep of the same snapshot): the
-// lanes fetch the listed positions and rebuild the displacements; no candidate is tested.  On a
-// periodic grid the image of each pair is recovered from the raw difference (x_j - x_i is within half
-// a box of a multiple of the box length) and applied with the same error-free shifted origin as the
-// cell walk uses.
 // Starts `width` floats at `row` on their way into L1 (one or two lines; rows are read in pieces of at
 // most 128 bytes).
 __device__ inline void prefetch_row(const float *row, int width) {
@@ -129,16 +124,17 @@ __device__ inline void prefetch_row(const float *row, int width) {
     if ((reinterpret_cast<uintptr_t>(row) & 127) != 0 && width > 4) asm volatile("prefetch.global.L1 [%0];" ::"l"(row + width - 1));
 }
 
-// `rows` (optional): feature rows of `pitch` floats of which stage 3 will read `width` floats per neighbour;
-// they are prefetched as soon as the index is known.
+// Stage 1 of the backward from a cached neighbour list (written by the forward sweep of the same
+// snapshot): the lanes fetch the listed positions and rebuild the displacements; no candidate is tested.
+// On a periodic grid the image of each pair is recovered from the raw difference (x_j - x_i is within half
+// a box of a multiple of the box length) and applied with the same error-free shifted origin as the
+// cell walk uses.
 template <int D, bool PER>
 __device__ inline void expand_pairs(const Geom &g, const float *__restrict__ x, const Pos<D> &pi,
-                                    const int32_t *__restrict__ list, int count, float4 *geo,
-                                    const float *__restrict__ rows = nullptr, int pitch = 0, int width = 0) {
+                                    const int32_t *__restrict__ list, int count, float4 *geo) {
     const int lane = threadIdx.x & 31;
     for (int e = lane; e < count; e += 32) {
         const int j = __ldg(list + e);
-        if (rows) prefetch_row(rows + (long long)j * pitch, width);
         const Pos<D> pj = load_pos<D>(x, j);
         float rx, ry, rz;
         listed_displacement<D, PER>(g, pi, pj, rx, ry, rz);
@@ -175,10 +171,6 @@ feature_forward_kernel(FeatureFwdArgs a, Geom g) {
     for (int k = part; k < it.count; k += g.split) {
         const long long i = it.first + k;
         const Pos<D> pi = load_pos<D>(a.x, i);
-        if (a.pair_cache && a.pair_cache_valid && k + g.split < it.count && lane * 32 < a.pair_stride && lane < 4) {
-            // the head of the next particle's neighbour list (the first 512 bytes) on its way into L1
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(a.pair_cache + (i + g.split) * a.pair_stride + lane * 32));
-        }
         float mom[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // F_MOMENT: upper triangle, lane-partial over pairs
         float dgs[3] = {0.f, 0.f, 0.f};                   // F_PACK with rho_grad_out: density gradient, lane-partial over pairs
         for (int fbase = 0; fbase < C; fbase += LPP * VW) {
@@ -198,18 +190,16 @@ feature_forward_kernel(FeatureFwdArgs a, Geom g) {
             const unsigned long long nsi01 = pack2(-si[0], -si[VW == 4 ? 1 : 0]), nsi23 = pack2(-si[VW == 4 ? 2 : 0], -si[VW == 4 ? 3 : 0]);
 
             int cached = 0;  // pairs of this particle already written to the neighbour list cache
-            bool from_list = false;
             const int chunk_w = C - fbase < LPP * VW ? C - fbase : LPP * VW;  // floats of a row read in this chunk
             auto flush = [&](int n) {
                 __syncwarp();
                 for (int e = lane; e < n; e += 32) {  // stage 2: pair scalars, one entry per lane
                     const float4 ge = geo[e];
                     const int j = __float_as_int(ge.w);
-                    if (a.pair_cache && !a.pair_cache_valid && fbase == 0 && cached + e < a.pair_stride - 1)
+                    if (a.pair_cache && fbase == 0 && cached + e < a.pair_stride - 1)
                         a.pair_cache[i * a.pair_stride + 1 + cached + e] = j;
-                    // the neighbour's feature row is wanted in stage 3: start it on its way into L1 (the list path
-                    // has done so already, in expand_pairs)
-                    if (!from_list) prefetch_row(a.s + ((long long)j * C + fbase), chunk_w);
+                    // the neighbour's feature row is wanted in stage 3: start it on its way into L1
+                    prefetch_row(a.s + ((long long)j * C + fbase), chunk_w);
                     const float q = sq_norm_fast<D>(ge.x, ge.y, ge.z);
                     const float mj = a.mass ? __ldg(a.mass + j) : 1.0f;
                     const float vj = mj / __ldg(a.rho + j);
@@ -311,27 +301,9 @@ feature_forward_kernel(FeatureFwdArgs a, Geom g) {
                 cached += n;
                 __syncwarp();
             };
-            int listed = -1;
-            if (a.pair_cache && a.pair_cache_valid) listed = __ldg(a.pair_cache + i * a.pair_stride);
-            from_list = listed >= 0;
-            if (listed >= 0 && listed <= kListPerWarp) {
-                expand_pairs<D, PER>(g, a.x, pi, a.pair_cache + i * a.pair_stride + 1, listed, geo, a.s + fbase, C, chunk_w);
-                flush(listed);
-            } else if (listed > kListPerWarp) {
-                // a list longer than the warp's pair slots goes through in pieces (the sums carry over); kept apart
-                // from the common case above, which a loop around it was measured to slow down by 4 %
-                const int32_t *list = a.pair_cache + i * a.pair_stride + 1;
-#pragma unroll 1
-                for (int off = 0; off < listed; off += kListPerWarp) {
-                    const int n = listed - off < kListPerWarp ? listed - off : kListPerWarp;
-                    expand_pairs<D, PER>(g, a.x, pi, list + off, n, geo, a.s + fbase, C, chunk_w);
-                    flush(n);
-                }
-            } else {
-                collect_pairs<D, PER>(g, a.x, pi, rng, nr, geo, flush);
-                if (a.pair_cache && !a.pair_cache_valid && fbase == 0 && lane == 0)
-                    a.pair_cache[i * a.pair_stride] = cached <= a.pair_stride - 1 ? cached : -1;
-            }
+            collect_pairs<D, PER>(g, a.x, pi, rng, nr, geo, flush);
+            if (a.pair_cache && fbase == 0 && lane == 0)
+                a.pair_cache[i * a.pair_stride] = cached <= a.pair_stride - 1 ? cached : -1;
 
             if (VW == 4) {
                 unpack2(pacc[0], blur[0], blur[VW == 4 ? 1 : 0]);
@@ -778,6 +750,7 @@ int launch_feature_forward_geom(const Geom &g, int mask, const FeatureFwdArgs &a
         const int rc = launch_feature_tile_forward<D, PER>(g, mask, a, st, &taken);
         if (rc != NPA_OK || taken) return rc;
     }
+    if (a.pair_cache && a.pair_cache_valid) return launch_feature_list_forward(g, mask, a, st);
     if (feature_rows_vectorisable(a.C, a.s, a.blur, a.grad, nullptr, nullptr)) {
         const int need = a.C / 4;
         if (need <= 4) return launch_feature_forward_shape<D, PER, 4, 4>(g, mask, a, st);

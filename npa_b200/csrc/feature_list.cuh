@@ -1,0 +1,819 @@
+// Blur and feature gradient, forward and backward, over recorded neighbour lists.
+//
+// The kernels of feature_kernels.cuh give a particle the whole warp: its pairs are dealt to 32 / LPP
+// sub-groups and the sub-groups' partial sums are combined by shuffles once per particle.  At ~41 pairs
+// per particle that combination, the half-empty last round of pair scalars and the walk over work-list
+// rows are two thirds of the instructions (25 warp instructions per pair measured where the arithmetic
+// needs 4).  With a list nothing ties a particle to a work item, so here a sub-group of LPP lanes owns a
+// whole particle: lanes cover the features (4 each), every lane ends with the complete sum of its
+// features and nothing is combined.  32 / LPP particles advance together through chunks of CH list
+// entries:
+//   stage B  every lane turns one (LPP = 4: two) list entries of its particle into pair scalars and leaves
+//            them in the warp's shared memory, already duplicated for the packed arithmetic; the entries of
+//            the next chunk are on their way meanwhile;
+//   stage C  the lanes of a sub-group walk the chunk's entries: four neighbour rows are fetched at a time
+//            (128-bit loads, one line per sub-group) and multiplied in with fma.rn.f32x2.
+// The price is imbalance: a warp runs as long as the longest of its lists (neighbouring particles, ~16 %
+// over the mean for four lists of ~41).  Work items, tickets and cell ranges are not needed; blocks are
+// plain blocks over consecutive particles, which lie in consecutive cells.
+// A particle whose list overflowed (count -1) is searched by its sub-group's lanes over the cells around
+// its position, LPP candidates a round, in the same warp.
+//
+// What bounds them: instruction issue and the L1 data path (one 128-byte line per pair and row).  Measured,
+// B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us before -> now: blur + gradient 328 -> FWD_PLAIN,
+// packed perception 495 -> FWD_PACK, features-only backward 499 -> BWD_FEAT, full backward 902 -> BWD_FULL.
+#pragma once
+#include "neighbors.cuh"
+#include "ops.cuh"
+
+namespace npa {
+
+constexpr int kListWarps = 8;  // warps per CTA
+
+// (x, y, z, m_j / rho_j) of particle j: one 16-byte gather when the density sweep left it packed.
+template <int D>
+__device__ inline float4 fetch_particle(const float *__restrict__ x, const float4 *__restrict__ pv, const float *__restrict__ rho,
+                                        const float *__restrict__ mass, int j) {
+    if (pv) return __ldg(pv + j);
+    const Pos<D> p = load_pos<D>(x, j);
+    const float m = mass ? __ldg(mass + j) : 1.0f;
+    return make_float4(p.x, p.y, p.z, m / __ldg(rho + j));
+}
+
+// Four features f0..f0+3 of a row; lanes beyond the last feature read valid neighbours of it (unused).
+template <bool VEC>
+__device__ inline void load_row4(const float *__restrict__ row, int f0, int C, float (&v)[4]) {
+    if (VEC) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(row + min(f0, C - 4)));
+        v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q) v[q] = __ldg(row + min(f0 + q, C - 1));
+    }
+}
+
+template <bool VEC>
+__device__ inline void store_row4(float *__restrict__ row, int f0, int C, const float (&v)[4]) {
+    if (VEC) {
+        if (f0 < C) *reinterpret_cast<float4 *>(row + f0) = make_float4(v[0], v[1], v[2], v[3]);
+    } else {
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+            if (f0 + q < C) row[f0 + q] = v[q];
+    }
+}
+
+// Search of the cells around one particle by the LPP lanes of its sub-group: candidate ranges in the order of
+// the cell walk, LPP candidates per round.
+template <int D, bool PER, int LPP>
+struct SubgroupSearch {
+    int cx, cy, cz, piece, j, end;
+    const int32_t *off;
+    Origin<D, PER> org;
+
+    __device__ inline void begin(const Geom &g, const int32_t *bin_offsets, long long i, const Pos<D> &pi) {
+        cx = axis_cell(pi.x, g, 0);
+        cy = axis_cell(pi.y, g, 1);
+        cz = D == 3 ? axis_cell(pi.z, g, 2) : 0;
+        off = bin_offsets + (i / g.N) * (long long)g.cells;
+        piece = -1;
+        j = end = 0;
+    }
+    // Moves on to the next non-empty range when the current one is used up; false at the end.
+    __device__ inline bool more(const Geom &g, const Pos<D> &pi) {
+        while (j >= end) {
+            if (++piece >= range_pieces<D>(g)) return false;
+            int code;
+            range_piece<D>(g, off, cx, cy, cz, piece, j, end, code);
+            if (j < end) org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, code);
+        }
+        return true;
+    }
+};
+
+// Slot of this lane's entry when the accepted entries of its sub-group come first, in lane order, and the
+// others fill the slots behind them; m = number of accepted entries of the sub-group.
+template <int LPP>
+__device__ inline int compact_slot(bool acc, int sg, int sl, int &m) {
+    const unsigned all = LPP == 32 ? 0xffffffffu : ((1u << (LPP & 31)) - 1u);
+    const unsigned bits = (__ballot_sync(kFull, acc) >> (sg * LPP)) & all;
+    const unsigned below = (1u << sl) - 1u;
+    m = __popc(bits);
+    return acc ? __popc(bits & below) : m + __popc(~bits & below);
+}
+
+template <int D> struct TailWeights { using type = float4; };  // (Kz, Kz, W, W)
+template <> struct TailWeights<2> { using type = float2; };    // (W, W)
+
+template <int D, bool PER, int LPP, bool VEC, int MASK>
+__global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 3)
+feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
+    constexpr int EPL = LPP == 4 ? 2 : 1;  // list entries per lane and chunk
+    constexpr int CH = LPP * EPL, PP = 32 / LPP;
+    using KB = typename TailWeights<D>::type;
+    // one entry of padding per sub-group keeps the sub-groups' broadcasts on different banks
+    __shared__ float4 s_ka[kListWarps][2][PP * (CH + 1)];  // K.x K.x K.y K.y, all times v_j
+    __shared__ KB s_kb[kListWarps][2][PP * (CH + 1)];      // [K.z K.z] W W
+    __shared__ int4 s_j[kListWarps][2][PP * (CH / 4 + 1)];
+    extern __shared__ float4 s_dyn[];                      // F_PACK: the rows of z of a warp's particles
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
+    const int total = g.B * g.N, C = a.C;
+    const int first = (blockIdx.x * kListWarps + warp) * PP;
+    if (first >= total) return;
+    const bool ivalid = first + sg < total;
+    const int i = ivalid ? first + sg : total - 1;
+    const Pos<D> pi = load_pos<D>(a.x, i);
+    const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
+    const int count = ivalid ? __ldg(list) : 0;
+    ++list;
+    const int n = max(count, 0);
+    const int nmax = __reduce_max_sync(kFull, n);
+    const unsigned pitch = (unsigned)C * 4u;
+    constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
+    constexpr bool kMoment = (MASK & F_MOMENT) != 0;
+    constexpr bool kDg = (MASK & F_DGRAD) != 0;
+
+    for (int fbase = 0; fbase < C; fbase += LPP * 4) {
+        __syncwarp();  // the slice before has drained its buffers
+        const int f0 = fbase + sl * 4;
+        float si[4];
+        load_row4<VEC>(a.s + (long long)i * C, f0, C, si);
+        const unsigned long long nsi01 = pack2(-si[0], -si[1]), nsi23 = pack2(-si[2], -si[3]);
+        // packed sums of the features (0, 1) and (2, 3): blur, then the gradient axis by axis
+        unsigned long long acc[2 + 2 * D];
+#pragma unroll
+        for (int q = 0; q < 2 + 2 * D; ++q) acc[q] = 0ull;
+        float mom[D * (D + 1) / 2], dgs[EPL][3];  // lane-partial over the pairs
+#pragma unroll
+        for (int q = 0; q < D * (D + 1) / 2; ++q) mom[q] = 0.f;
+#pragma unroll
+        for (int k = 0; k < EPL; ++k) dgs[k][0] = dgs[k][1] = dgs[k][2] = 0.f;
+
+        // pair scalars of one entry (zero volume: no pair) into slot `slot` of buffer `buf`
+        auto put = [&](int buf, int slot, int k, float rx, float ry, float rz, float vj, float mj, int j) {
+            const float q = sq_norm_fast<D>(rx, ry, rz);
+            float w = 0.f, kv = 0.f;
+            if (kBlur) {
+                const float t = fmaxf(g.h2 - q, 0.f);
+                w = vj * (t * t * t);
+            }
+            if ((kGrad || kMoment || kDg) && q > 0.f) {
+                float dist;
+                const float phi = spiky_phi(q, g.h, dist);
+                kv = vj * phi;
+                if (kDg) {
+                    const float md = mj * phi;
+                    dgs[k][0] = fmaf(md, rx, dgs[k][0]);
+                    dgs[k][1] = fmaf(md, ry, dgs[k][1]);
+                    if (D == 3) dgs[k][2] = fmaf(md, rz, dgs[k][2]);
+                }
+            }
+            if (kMoment) {
+                mom[0] = fmaf(kv * rx, rx, mom[0]);
+                mom[1] = fmaf(kv * rx, ry, mom[1]);
+                if (D == 2) {
+                    mom[2] = fmaf(kv * ry, ry, mom[2]);
+                } else {
+                    mom[2] = fmaf(kv * rx, rz, mom[2]);
+                    mom[3] = fmaf(kv * ry, ry, mom[3]);
+                    mom[D == 3 ? 4 : 0] = fmaf(kv * ry, rz, mom[D == 3 ? 4 : 0]);
+                    mom[D == 3 ? 5 : 0] = fmaf(kv * rz, rz, mom[D == 3 ? 5 : 0]);
+                }
+            }
+            const float kx = kv * rx, ky = kv * ry, kz = kv * rz;
+            if (kGrad) s_ka[warp][buf][sg * (CH + 1) + slot] = make_float4(kx, kx, ky, ky);
+            if constexpr (D == 3) s_kb[warp][buf][sg * (CH + 1) + slot] = make_float4(kz, kz, w, w);
+            else s_kb[warp][buf][sg * (CH + 1) + slot] = make_float2(w, w);
+            reinterpret_cast<int *>(&s_j[warp][buf][sg * (CH / 4 + 1)])[slot] = j;
+        };
+        // the first m entries of a buffer (m uniform; slots up to the next multiple of four are filled)
+        auto drain = [&](int buf, int m) {
+            const float4 *ka = &s_ka[warp][buf][sg * (CH + 1)];
+            const KB *kb = &s_kb[warp][buf][sg * (CH + 1)];
+            const int4 *jj = &s_j[warp][buf][sg * (CH / 4 + 1)];
+#pragma unroll
+            for (int e0 = 0; e0 < CH; e0 += 4) {
+                if (e0 >= m) break;
+                const int4 j4 = jj[e0 / 4];
+                const int js[4] = {j4.x, j4.y, j4.z, j4.w};
+                float r[4][4];
+#pragma unroll
+                for (int u = 0; u < 4; ++u)
+                    load_row4<VEC>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + (unsigned long long)(unsigned)js[u] * pitch),
+                                   f0, C, r[u]);
+#pragma unroll
+                for (int u = 0; u < 4; ++u) {
+                    const unsigned long long s01 = pack2(r[u][0], r[u][1]), s23 = pack2(r[u][2], r[u][3]);
+                    const KB b = kb[e0 + u];
+                    if (kBlur) {
+                        unsigned long long ww;
+                        if constexpr (D == 3) ww = pack2(b.z, b.w);
+                        else ww = pack2(b.x, b.y);
+                        acc[0] = fma2(ww, s01, acc[0]);
+                        acc[1] = fma2(ww, s23, acc[1]);
+                    }
+                    if (kGrad) {
+                        const float4 k4 = ka[e0 + u];
+                        const unsigned long long d01 = add2(s01, nsi01), d23 = add2(s23, nsi23);  // s_j - s_i
+                        const unsigned long long kx = pack2(k4.x, k4.y), ky = pack2(k4.z, k4.w);
+                        acc[2] = fma2(d01, kx, acc[2]);
+                        acc[3] = fma2(d23, kx, acc[3]);
+                        acc[4] = fma2(d01, ky, acc[4]);
+                        acc[5] = fma2(d23, ky, acc[5]);
+                        if constexpr (D == 3) {
+                            const unsigned long long kz = pack2(b.x, b.y);
+                            acc[6] = fma2(d01, kz, acc[6]);
+                            acc[7] = fma2(d23, kz, acc[7]);
+                        }
+                    }
+                }
+            }
+        };
+
+        // ---- the listed pairs
+        int jn[EPL];
+        float4 pj[EPL];
+        float mj[EPL];
+        auto indices = [&](int c) {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                const int e = c + k * LPP + sl;
+                jn[k] = e < n ? __ldg(list + e) : -1;
+            }
+        };
+        auto particles = [&]() {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                const int j = jn[k] >= 0 ? jn[k] : i;
+                pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, j);
+                mj[k] = kDg ? (a.mass ? __ldg(a.mass + j) : 1.0f) : 0.f;
+                if (jn[k] < 0) { pj[k].w = 0.f; mj[k] = 0.f; }
+            }
+        };
+        int buf = 0;
+        indices(0);
+        particles();
+        for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                float rx, ry, rz;
+                listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
+                put(buf, k * LPP + sl, k, rx, ry, rz, pj[k].w, mj[k], jn[k] >= 0 ? jn[k] : i);
+            }
+            indices(c + CH);
+            __syncwarp();
+            particles();
+            drain(buf, nmax - c);
+        }
+
+        // ---- particles without a list
+        bool over = count < 0;
+        if (__any_sync(kFull, over)) {
+            SubgroupSearch<D, PER, LPP> search;
+            if (over) search.begin(g, a.bin_offsets, i, pi);
+            while (true) {
+                over = over && search.more(g, pi);
+                if (!__any_sync(kFull, over)) break;
+                float rx = 0.f, ry = 0.f, rz = 0.f;
+                bool hit = false;
+                const int j = over ? search.j + sl : i;
+                if (over) {
+                    if (j < search.end) {
+                        const Pos<D> p = load_pos<D>(a.x, j);
+                        hit = displacement<D, PER, false>(g, search.org, p.x, p.y, p.z, rx, ry, rz) < g.h2;
+                    }
+                    search.j += LPP;
+                }
+                int m;
+                const int slot = compact_slot<LPP>(hit, sg, sl, m);
+                const int most = __reduce_max_sync(kFull, m);
+                if (most == 0) continue;
+                const float m_j = hit && a.mass ? __ldg(a.mass + j) : 1.0f;
+                put(buf, slot, 0, rx, ry, rz, hit ? m_j / __ldg(a.rho + j) : 0.f, hit ? m_j : 0.f, hit ? j : i);
+                __syncwarp();
+                drain(buf, most);
+                buf ^= 1;
+            }
+        }
+
+        float blur[4], gr[4][D];
+        unpack2(acc[0], blur[0], blur[1]);
+        unpack2(acc[1], blur[2], blur[3]);
+#pragma unroll
+        for (int d = 0; d < D; ++d) {
+            unpack2(acc[2 + 2 * d], gr[0][d], gr[1][d]);
+            unpack2(acc[3 + 2 * d], gr[2][d], gr[3][d]);
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            blur[q] *= g.c_s;
+#pragma unroll
+            for (int d = 0; d < D; ++d) gr[q][d] *= g.c_g;
+        }
+        float dg[3] = {0.f, 0.f, 0.f};
+        if (kDg && fbase == 0) {
+            // partial sums over the entries with equal (entry mod 8) meet in the same order for LPP = 4 and 8
+#pragma unroll
+            for (int d = 0; d < D; ++d) dg[d] = g.c_g * subgroup_sum<LPP>(EPL == 2 ? dgs[0][d] + dgs[EPL - 1][d] : dgs[0][d]);
+        }
+        if (kMoment) {
+#pragma unroll
+            for (int q = 0; q < D * (D + 1) / 2; ++q) mom[q] = g.c_g * subgroup_sum<LPP>(mom[q]);
+        }
+        if (kBlur && a.blur && ivalid) store_row4<VEC>(a.blur + (long long)i * C, f0, C, blur);
+        float L[D * D];
+        if (MASK & (F_PACK | F_CORRECTED)) {
+            safe_inverse_sym<D>(mom, a.inv_tol, L);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {  // gradient . inv(M)
+                float v[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    float s = 0.f;
+#pragma unroll
+                    for (int k = 0; k < D; ++k) s = fmaf(gr[q][k], L[k * D + d], s);
+                    v[d] = s;
+                }
+#pragma unroll
+                for (int d = 0; d < D; ++d) gr[q][d] = v[d];
+            }
+        }
+        float *gout = (MASK & F_PACK) ? a.vgrad : a.grad;
+        if (kGrad && gout && ivalid) {
+            float *o = gout + ((long long)i * C + f0) * D;
+            if (VEC) {
+                if (f0 < C) {
+                    const float *v = &gr[0][0];
+#pragma unroll
+                    for (int k = 0; k < D; ++k) reinterpret_cast<float4 *>(o)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
+                }
+            } else {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (f0 + q < C) {
+#pragma unroll
+                        for (int d = 0; d < D; ++d) o[q * D + d] = gr[q][d];
+                    }
+            }
+        }
+        if (kDg && fbase == 0 && a.rho_grad_out && ivalid && sl == 0) {
+#pragma unroll
+            for (int d = 0; d < D; ++d) a.rho_grad_out[(long long)i * D + d] = dg[d];
+        }
+        if (kMoment && fbase == 0 && a.moment && ivalid && sl == 0) {
+            float *o = a.moment + (long long)i * (D * D);
+            int k = 0;
+#pragma unroll
+            for (int p = 0; p < D; ++p)
+#pragma unroll
+                for (int q = p; q < D; ++q, ++k) {
+                    o[p * D + q] = mom[k];
+                    o[q * D + p] = mom[k];
+                }
+        }
+        if (MASK & F_PACK) {
+            // the rows of z of the warp's particles are contiguous: assembled in shared memory, written as one run
+            const int Z = a.zstride;
+            float *stage = reinterpret_cast<float *>(s_dyn) + (size_t)warp * ((PP * Z + 3) & ~3);
+            float *zs = stage + sg * Z;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int f = f0 + q;
+                float v[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) v[d] = a.coef * gr[q][d];
+                if (a.log_norm_grad) log_normalize<D>(v);
+                if (f < C) {
+                    zs[f] = si[q];
+                    zs[C + f] = blur[q];
+#pragma unroll
+                    for (int d = 0; d < D; ++d) zs[2 * C + f * D + d] = v[d];
+                }
+            }
+            if (sl == 0) {
+                float w[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) w[d] = a.dg_scale * dg[d];
+                if (a.log_norm_dg) log_normalize<D>(w);
+#pragma unroll
+                for (int d = 0; d < D; ++d) zs[2 * C + C * D + d] = w[d];
+            }
+            __syncwarp();
+            const int floats = min(PP, total - first) * Z;
+            float *out = a.z + (long long)first * Z;
+            if (PP % 4 == 0) {  // first is a multiple of four rows: 16-byte aligned
+                const int quads = floats / 4;
+                for (int q = lane; q < quads; q += 32) reinterpret_cast<float4 *>(out)[q] = reinterpret_cast<const float4 *>(stage)[q];
+                for (int q = quads * 4 + lane; q < floats; q += 32) out[q] = stage[q];
+            } else {
+                for (int q = lane; q < floats; q += 32) out[q] = stage[q];
+            }
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// Backward.  The upstream of the gradient comes with the axis in front of the features ([N, D, C], rows
+// padded to a multiple of four; upstream_rows_kernel or the packed perception's own epilogue write it so),
+// so that the lanes of a sub-group read one line per axis instead of runs 48 bytes apart.
+//   ds_i   = v_i sum_j [ c_s W gB_j - sum_d K_d gG_j[d] ] - gG_i . T,        K = c_g phi r, T = sum_j v_j K
+//   u_d    = v_j (s_i - s_j).gG_i[d] + v_i (s_i - s_j).gG_j[d],   t = v_j gB_i.s_j + v_i gB_j.s_i
+//   dx_i   = sum_j (E t - psi r.u) r + phi u      (E, phi, psi with their constants)
+//   drho_i = (v_i / m_i) v_i sum_j [ phi r.((s_i - s_j) gG_j) - c_s W gB_j.s_i ]
+// Sums over features stay lane-partial (packed pairs) until the particle is done.  The density gradient's own
+// backward, dx_i += sum_j J (m_i g_j - m_j g_i), uses the same pair scalars and rides stage B.
+// ---------------------------------------------------------------------------------------------------------
+template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
+__global__ void __launch_bounds__(FULL ? 128 : kListWarps * 32, FULL ? 4 : 3)
+feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
+    constexpr int EPL = LPP == 4 ? 2 : 1;
+    constexpr int CH = LPP * EPL, PP = 32 / LPP, WARPS = FULL ? 4 : kListWarps;
+    __shared__ float4 s_ka[WARPS][2][PP * (CH + 1)];                // -K.x -K.x -K.y -K.y
+    __shared__ float4 s_kb[WARPS][2][PP * (CH + 1)];                // -K.z -K.z W W
+    __shared__ float4 s_kc[FULL ? WARPS : 1][2][PP * (CH + 1)];     // r.x r.y r.z phi
+    __shared__ float4 s_kd[FULL ? WARPS : 1][2][PP * (CH + 1)];     // v_j v_j E psi
+    __shared__ int4 s_j[WARPS][2][PP * (CH / 4 + 1)];
+    constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
+
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
+    const int total = g.B * g.N, C = a.C;
+    const int first = (blockIdx.x * WARPS + warp) * PP;
+    if (first >= total) return;
+    const bool ivalid = first + sg < total;
+    const int i = ivalid ? first + sg : total - 1;
+    const Pos<D> pi = load_pos<D>(a.x, i);
+    const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
+    const int count = ivalid ? __ldg(list) : 0;
+    ++list;
+    const int n = max(count, 0);
+    const int nmax = __reduce_max_sync(kFull, n);
+    const float mi = a.mass ? __ldg(a.mass + i) : 1.0f;
+    const float rhoi = __ldg(a.rho + i);
+    const float vi = mi / rhoi;
+    const unsigned spitch = (unsigned)C * 4u, bpitch = (unsigned)a.gb_pitch * 4u, gpitch = (unsigned)a.gg_pitch * 4u;
+    const int Cp = a.cp;
+    float dx[3] = {0.f, 0.f, 0.f};           // lane-partial over features and pairs
+    float dxd[3] = {0.f, 0.f, 0.f};          // density-gradient part, lane-partial over pairs
+    unsigned long long drp = 0ull;           // minus the sum in drho, lane-partial
+    float gdi[3] = {0.f, 0.f, 0.f};
+    if (FULL && a.g_dg) {
+#pragma unroll
+        for (int d = 0; d < D; ++d) gdi[d] = __ldg(a.g_dg + (long long)i * D + d);
+    }
+
+    for (int fbase = 0; fbase < C; fbase += LPP * 4) {
+        __syncwarp();
+        const int f0 = fbase + sl * 4, fv = min(f0, Cp - 4);
+        // the i side: s_i, v_i s_i, gB_i, gG_i and v_i in packed pairs; a lane beyond the last feature contributes zeros
+        unsigned long long si[2] = {0ull, 0ull}, svi[2] = {0ull, 0ull}, gbi[2] = {0ull, 0ull}, vi2[2] = {0ull, 0ull}, ggi[2 * D];
+#pragma unroll
+        for (int q = 0; q < 2 * D; ++q) ggi[q] = 0ull;
+        if (FULL) {
+            float t[4];
+            load_row4<VEC>(a.s + (long long)i * C, f0, C, t);
+            const bool live[4] = {f0 < C, f0 + 1 < C, f0 + 2 < C, f0 + 3 < C};
+#pragma unroll
+            for (int q = 0; q < 4; ++q) t[q] = live[q] ? t[q] : 0.f;
+            si[0] = pack2(t[0], t[1]); si[1] = pack2(t[2], t[3]);
+            vi2[0] = pack2(live[0] ? vi : 0.f, live[1] ? vi : 0.f); vi2[1] = pack2(live[2] ? vi : 0.f, live[3] ? vi : 0.f);
+            svi[0] = pack2(vi * t[0], vi * t[1]); svi[1] = pack2(vi * t[2], vi * t[3]);
+            if (kBlur && f0 < C) {
+                const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gb + (long long)i * a.gb_pitch + f0));
+                gbi[0] = pack2(b.x, live[1] ? b.y : 0.f);
+                gbi[1] = pack2(live[2] ? b.z : 0.f, live[3] ? b.w : 0.f);
+            }
+            if (kGrad && f0 < C) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gg + (long long)i * a.gg_pitch + d * Cp + f0));
+                    ggi[2 * d] = pack2(b.x, live[1] ? b.y : 0.f);
+                    ggi[2 * d + 1] = pack2(live[2] ? b.z : 0.f, live[3] ? b.w : 0.f);
+                }
+            }
+        }
+        const unsigned long long minus1 = pack2(-1.f, -1.f);
+        unsigned long long ds[2] = {0ull, 0ull};
+        float tsum[3] = {0.f, 0.f, 0.f};  // T, lane-partial over the pairs
+
+        auto put = [&](int buf, int slot, float rx, float ry, float rz, float vj, int j) {
+            const float q = sq_norm_fast<D>(rx, ry, rz);
+            const float t = fmaxf(g.h2 - q, 0.f);
+            const bool pair = vj != 0.f || j != i;  // a filled-up slot is (self, zero volume)
+            const float w = pair ? g.c_s * (t * t * t) : 0.f;
+            float phi = 0.f, psi = 0.f;
+            if ((kGrad || (FULL && a.g_dg)) && q > 0.f) {
+                float dist;
+                phi = g.c_g * spiky_phi(q, g.h, dist);
+                if (FULL) psi = g.c_g * spiky_psi(dist, g.h);
+            }
+            const float kx = phi * rx, ky = phi * ry, kz = phi * rz;
+            tsum[0] = fmaf(vj, kx, tsum[0]);
+            tsum[1] = fmaf(vj, ky, tsum[1]);
+            if (D == 3) tsum[2] = fmaf(vj, kz, tsum[2]);
+            const int at = sg * (CH + 1) + slot;
+            if (kGrad) s_ka[warp][buf][at] = make_float4(-kx, -kx, -ky, -ky);
+            s_kb[warp][buf][at] = make_float4(-kz, -kz, w, w);
+            if (FULL) {
+                s_kc[warp][buf][at] = make_float4(rx, ry, rz, phi);
+                s_kd[warp][buf][at] = make_float4(vj, vj, pair ? g.c_s * 6.0f * t * t : 0.f, psi);
+                if (a.g_dg && fbase == 0 && q > 0.f) {
+                    const float mj = a.mass ? __ldg(a.mass + j) : 1.0f;
+                    const float rv[3] = {rx, ry, rz};
+                    float u[3] = {0.f, 0.f, 0.f}, ru = 0.f;
+#pragma unroll
+                    for (int d = 0; d < D; ++d) {
+                        u[d] = mi * __ldg(a.g_dg + (long long)j * D + d) - mj * gdi[d];
+                        ru = fmaf(rv[d], u[d], ru);
+                    }
+                    const float sc = psi * ru;
+#pragma unroll
+                    for (int d = 0; d < D; ++d) dxd[d] += phi * u[d] - sc * rv[d];
+                }
+            }
+            reinterpret_cast<int *>(&s_j[warp][buf][sg * (CH / 4 + 1)])[slot] = j;
+        };
+
+        struct Rows { float s[4], b[4], g[D][4]; };
+        auto load = [&](int j, Rows &r) {
+            const unsigned long long u = (unsigned)j;
+            if (FULL) load_row4<VEC>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + u * spitch), f0, C, r.s);
+            if (kBlur) {
+                const float4 t = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(a.gb + fv) + u * bpitch));
+                r.b[0] = t.x; r.b[1] = t.y; r.b[2] = t.z; r.b[3] = t.w;
+            }
+            if (kGrad) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const float4 t = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(a.gg + fv + d * Cp) + u * gpitch));
+                    r.g[d][0] = t.x; r.g[d][1] = t.y; r.g[d][2] = t.z; r.g[d][3] = t.w;
+                }
+            }
+        };
+        auto add = [&](int buf, int e, const Rows &r) {
+            const int at = sg * (CH + 1) + e;
+            const float4 kb = s_kb[warp][buf][at];
+            unsigned long long b01, b23, k[D];
+            if (kBlur) {
+                b01 = pack2(r.b[0], r.b[1]); b23 = pack2(r.b[2], r.b[3]);
+                const unsigned long long w = pack2(kb.z, kb.w);
+                ds[0] = fma2(w, b01, ds[0]);
+                ds[1] = fma2(w, b23, ds[1]);
+            }
+            if (kGrad) {
+                const float4 ka = s_ka[warp][buf][at];
+                k[0] = pack2(ka.x, ka.y);
+                k[1] = pack2(ka.z, ka.w);
+                if (D == 3) k[D - 1] = pack2(kb.x, kb.y);
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    ds[0] = fma2(k[d], pack2(r.g[d][0], r.g[d][1]), ds[0]);
+                    ds[1] = fma2(k[d], pack2(r.g[d][2], r.g[d][3]), ds[1]);
+                }
+            }
+            if (FULL) {
+                const float4 kc = s_kc[warp][buf][at], kd = s_kd[warp][buf][at];
+                const unsigned long long s01 = pack2(r.s[0], r.s[1]), s23 = pack2(r.s[2], r.s[3]), vj = pack2(kd.x, kd.y);
+                const float rv[3] = {kc.x, kc.y, kc.z};
+                float coef = 0.f;
+                if (kBlur) {
+                    const unsigned long long A = fma2(gbi[1], s23, mul2(gbi[0], s01));
+                    const unsigned long long Bp = fma2(svi[1], b23, mul2(svi[0], b01));
+                    float lo, hi;
+                    unpack2(fma2(vj, A, Bp), lo, hi);
+                    coef = kd.z * (lo + hi);
+                    drp = fma2(pack2(kb.z, kb.w), Bp, drp);
+                }
+                if (kGrad) {
+                    const unsigned long long e01 = fma2(s01, minus1, si[0]), e23 = fma2(s23, minus1, si[1]);  // s_i - s_j
+                    const unsigned long long f01 = mul2(vi2[0], e01), f23 = mul2(vi2[1], e23);
+                    float u[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+                    for (int d = 0; d < D; ++d) {
+                        const unsigned long long A = fma2(ggi[2 * d + 1], e23, mul2(ggi[2 * d], e01));
+                        const unsigned long long Bv = fma2(pack2(r.g[d][2], r.g[d][3]), f23, mul2(pack2(r.g[d][0], r.g[d][1]), f01));
+                        drp = fma2(k[d], Bv, drp);
+                        float lo, hi;
+                        unpack2(fma2(vj, A, Bv), lo, hi);
+                        u[d] = lo + hi;
+                    }
+                    float ru = rv[0] * u[0] + rv[1] * u[1];
+                    if (D == 3) ru = fmaf(rv[2], u[2], ru);
+                    coef = fmaf(-kd.w, ru, coef);
+#pragma unroll
+                    for (int d = 0; d < D; ++d) dx[d] = fmaf(kc.w, u[d], dx[d]);
+                }
+#pragma unroll
+                for (int d = 0; d < D; ++d) dx[d] = fmaf(coef, rv[d], dx[d]);
+            }
+        };
+        auto drain = [&](int buf, int m) {
+            const int4 *jj = &s_j[warp][buf][sg * (CH / 4 + 1)];
+#pragma unroll
+            for (int e0 = 0; e0 < CH; e0 += 4) {
+                if (e0 >= m) break;
+                const int4 j4 = jj[e0 / 4];
+                // two pairs in flight
+                Rows r0, r1;
+                load(j4.x, r0);
+                load(j4.y, r1);
+                add(buf, e0, r0);
+                load(j4.z, r0);
+                add(buf, e0 + 1, r1);
+                load(j4.w, r1);
+                add(buf, e0 + 2, r0);
+                add(buf, e0 + 3, r1);
+            }
+        };
+
+        int jn[EPL];
+        float4 pj[EPL];
+        auto indices = [&](int c) {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                const int e = c + k * LPP + sl;
+                jn[k] = e < n ? __ldg(list + e) : -1;
+            }
+        };
+        auto particles = [&]() {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, jn[k] >= 0 ? jn[k] : i);
+                if (jn[k] < 0) pj[k].w = 0.f;
+            }
+        };
+        int buf = 0;
+        indices(0);
+        particles();
+        for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+#pragma unroll
+            for (int k = 0; k < EPL; ++k) {
+                float rx, ry, rz;
+                listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
+                put(buf, k * LPP + sl, rx, ry, rz, pj[k].w, jn[k] >= 0 ? jn[k] : i);
+            }
+            indices(c + CH);
+            __syncwarp();
+            particles();
+            drain(buf, nmax - c);
+        }
+
+        bool over = count < 0;
+        if (__any_sync(kFull, over)) {
+            SubgroupSearch<D, PER, LPP> search;
+            if (over) search.begin(g, a.bin_offsets, i, pi);
+            while (true) {
+                over = over && search.more(g, pi);
+                if (!__any_sync(kFull, over)) break;
+                float rx = 0.f, ry = 0.f, rz = 0.f;
+                bool hit = false;
+                const int j = over ? search.j + sl : i;
+                if (over) {
+                    if (j < search.end) {
+                        const Pos<D> p = load_pos<D>(a.x, j);
+                        hit = displacement<D, PER, false>(g, search.org, p.x, p.y, p.z, rx, ry, rz) < g.h2;
+                    }
+                    search.j += LPP;
+                }
+                int m;
+                const int slot = compact_slot<LPP>(hit, sg, sl, m);
+                const int most = __reduce_max_sync(kFull, m);
+                if (most == 0) continue;
+                if (!hit) rx = ry = rz = 0.f;
+                const float m_j = hit && a.mass ? __ldg(a.mass + j) : 1.0f;
+                put(buf, slot, rx, ry, rz, hit ? m_j / __ldg(a.rho + j) : 0.f, hit ? j : i);
+                __syncwarp();
+                drain(buf, most);
+                buf ^= 1;
+            }
+        }
+
+        if (a.grad_s) {
+            float o[4];
+            unpack2(ds[0], o[0], o[1]);
+            unpack2(ds[1], o[2], o[3]);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) o[q] *= vi;
+            if (kGrad) {
+#pragma unroll
+                for (int d = 0; d < D; ++d) {
+                    const float T = subgroup_sum<LPP>(tsum[d]);
+                    const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gg + (long long)i * a.gg_pitch + d * Cp + fv));
+                    o[0] = fmaf(-T, b.x, o[0]); o[1] = fmaf(-T, b.y, o[1]);
+                    o[2] = fmaf(-T, b.z, o[2]); o[3] = fmaf(-T, b.w, o[3]);
+                }
+            }
+            if (a.direct && ivalid) {  // upstream that reaches the features unchanged
+                const float *z = a.direct + (long long)i * a.direct_pitch;
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (f0 + q < C) o[q] += __ldg(z + f0 + q);
+            }
+            if (ivalid) store_row4<VEC>(a.grad_s + (long long)i * C, f0, C, o);
+        }
+    }
+    if (FULL) {
+        float lo, hi;
+        unpack2(drp, lo, hi);
+        const float dr = -subgroup_sum<LPP>(lo + hi) / rhoi;
+        float out[3] = {0.f, 0.f, 0.f};
+#pragma unroll
+        for (int d = 0; d < D; ++d) out[d] = subgroup_sum<LPP>(dx[d] + dxd[d]);
+        if (ivalid && sl == 0) {
+            if (a.grad_x) {
+                if (D == 2) reinterpret_cast<float2 *>(a.grad_x)[i] = make_float2(out[0], out[1]);
+                else reinterpret_cast<float4 *>(a.grad_x)[i] = make_float4(out[0], out[1], out[2], 0.f);
+            }
+            if (a.grad_rho) a.grad_rho[i] = dr;
+            // what the density backward gathers per neighbour: position and total upstream of the density
+            if (a.pg) a.pg[i] = make_float4(pi.x, pi.y, pi.z, dr + (a.g_rho ? __ldg(a.g_rho + i) : 0.f));
+        }
+    }
+}
+
+// ---------------------------------------------------------------------------------------------------------
+// dispatch
+// ---------------------------------------------------------------------------------------------------------
+template <int D, bool PER, int LPP, bool VEC, int MASK>
+int launch_list_forward(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
+    constexpr int PP = 32 / LPP;
+    const auto kernel = feature_list_forward_kernel<D, PER, LPP, VEC, MASK>;
+    const size_t dyn = (MASK & F_PACK) ? (size_t)kListWarps * ((PP * a.zstride + 3) & ~3) * sizeof(float) : 0;
+    if (dyn > 0) {
+        int rc, unused = 0;
+        if ((rc = persistent_ctas(kernel, kListWarps * 32, dyn, &unused)) != NPA_OK) return rc;  // raises the shared-memory limit once
+    }
+    const long long particles = (long long)g.B * g.N, per_cta = (long long)kListWarps * PP;
+    kernel<<<(unsigned)((particles + per_cta - 1) / per_cta), kListWarps * 32, dyn, st>>>(a, g);
+    return check_launch("feature_list_forward_kernel");
+}
+
+template <int D, bool PER, int LPP, bool VEC>
+int launch_list_forward_mask(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st) {
+    switch (mask) {
+        case F_BLUR: return launch_list_forward<D, PER, LPP, VEC, F_BLUR>(g, a, st);
+        case F_GRAD: return launch_list_forward<D, PER, LPP, VEC, F_GRAD>(g, a, st);
+        case F_BLUR | F_GRAD: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD>(g, a, st);
+        case F_BLUR | F_GRAD | F_DGRAD: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_DGRAD>(g, a, st);
+        case F_BLUR | F_GRAD | F_MOMENT: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_MOMENT>(g, a, st);
+        case F_GRAD | F_MOMENT | F_CORRECTED: return launch_list_forward<D, PER, LPP, VEC, F_GRAD | F_MOMENT | F_CORRECTED>(g, a, st);
+        case F_BLUR | F_GRAD | F_MOMENT | F_PACK:
+            if (a.C > LPP * 4) return fail(NPA_ERR_UNSUPPORTED, "the packed perception sweep supports up to %d features here", LPP * 4);
+            return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_MOMENT | F_PACK | F_DGRAD>(g, a, st);
+        default: return fail(NPA_ERR_INVALID_ARGUMENT, "unsupported feature forward mask %d", mask);
+    }
+}
+
+// Lanes per particle: the smallest supported power of two whose lanes cover the features four at a time; wider rows
+// (more than 128 features) are walked in slices of 128.
+#define NPA_LIST_LPP(C, CALL)                                 \
+    do {                                                      \
+        if ((C) <= 16) return CALL(4);                        \
+        if ((C) <= 32) return CALL(8);                        \
+        if ((C) <= 64) return CALL(16);                       \
+        return CALL(32);                                      \
+    } while (0)
+
+template <int D, bool PER>
+int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st) {
+    const uintptr_t bits = (uintptr_t)a.s | (uintptr_t)a.blur | (uintptr_t)a.grad | (uintptr_t)a.vgrad;
+    if ((mask & F_PACK) && ((uintptr_t)a.z % 16)) return fail(NPA_ERR_INVALID_ARGUMENT, "the packed row tensor must be 16-byte aligned");
+    if (a.C % 4 == 0 && bits % 16 == 0) {
+#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, true>(g, mask, a, st)
+        NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+    }
+#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, false>(g, mask, a, st)
+    NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+}
+
+template <int D, bool PER, int LPP, bool VEC, bool FULL>
+int launch_list_backward_mask(const Geom &g, int mask, const FeatureListBwdArgs &a, cudaStream_t st) {
+    constexpr int PP = 32 / LPP, WARPS = FULL ? 4 : kListWarps;
+    const long long particles = (long long)g.B * g.N, per_cta = (long long)WARPS * PP;
+    const unsigned blocks = (unsigned)((particles + per_cta - 1) / per_cta);
+    switch (mask) {
+        case F_BLUR: feature_list_backward_kernel<D, PER, LPP, VEC, F_BLUR, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        case F_GRAD: feature_list_backward_kernel<D, PER, LPP, VEC, F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        case F_BLUR | F_GRAD: feature_list_backward_kernel<D, PER, LPP, VEC, F_BLUR | F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        default: return fail(NPA_ERR_INVALID_ARGUMENT, "unsupported feature backward mask %d", mask);
+    }
+    return check_launch("feature_list_backward_kernel");
+}
+
+template <int D, bool PER, bool FULL>
+int launch_feature_list_backward_geom(const Geom &g, int mask, const FeatureListBwdArgs &a, cudaStream_t st) {
+    // the features-only pass reads no feature row, only its output has the caller's layout
+    const uintptr_t bits = (FULL ? (uintptr_t)a.s : 0) | (uintptr_t)a.grad_s;
+    if (a.C % 4 == 0 && bits % 16 == 0) {
+#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, true, FULL>(g, mask, a, st)
+        NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+    }
+#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, false, FULL>(g, mask, a, st)
+    NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+}
+
+}  // namespace npa

@@ -1,0 +1,7 @@
+// Instantiates the backward feature kernels over neighbour lists for dim 3, clamped boundary.
+#include "feature_list.cuh"
+
+namespace npa {
+template int launch_feature_list_backward_geom<3, false, true>(const Geom &, int, const FeatureListBwdArgs &, cudaStream_t);
+template int launch_feature_list_backward_geom<3, false, false>(const Geom &, int, const FeatureListBwdArgs &, cudaStream_t);
+}  // namespace npa

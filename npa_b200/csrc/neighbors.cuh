@@ -122,19 +122,20 @@ __device__ inline Origin<D, PER> make_origin(const Geom &g, float px, float py, 
     return o;
 }
 
-// Fills rng[0..n) with the non-empty candidate ranges [start, end) of global
-// particle indices for the cell of `it`; returns n.  Must be called by all 32
-// lanes; rng is per-warp shared memory of kMaxRanges entries.
+// Number of candidate ranges of a cell: two per neighbour row with the linear hash (the second is the
+// wrapped cell of a periodic row), one per neighbour cell with the Morton hash.
 template <int D>
-__device__ inline int build_ranges(const Geom &g, const int32_t *__restrict__ bin_offsets,
-                                   const WorkItem &it, int4 *rng) {
-    const int lane = threadIdx.x & 31;
-    int cx, cy, cz;
-    hash_to_cell<D>(g, (uint32_t)(it.cell - it.sys * g.cells), cx, cy, cz);
-    const int32_t *off = bin_offsets + (size_t)it.sys * g.cells;
-    int start = 0, end = 0, sx = 0, sy = 0, sz = 0;
+__device__ inline int range_pieces(const Geom &g) { return g.morton ? (D == 2 ? 9 : 27) : (D == 2 ? 6 : 18); }
+
+// The k-th candidate range [start, end) of global particle indices around cell (cx, cy, cz) and its image
+// shift; empty (start == end) where the grid ends or nothing wraps.  `off`: bin_offsets of the system.
+template <int D>
+__device__ inline void range_piece(const Geom &g, const int32_t *__restrict__ off, int cx, int cy, int cz, int k, int &start,
+                                   int &end, int &code) {
+    start = end = 0;
+    int sx = 0, sy = 0, sz = 0;
     if (!g.morton) {
-        const int row = lane >> 1, piece = lane & 1;
+        const int row = k >> 1, piece = k & 1;
         if (row < (D == 2 ? 3 : 9)) {
             int ny = 0, nz = 0;
             bool ok = neighbor_axis(cy, row % 3 - 1, g.g[1], g.periodic, ny, sy);
@@ -157,22 +158,33 @@ __device__ inline int build_ranges(const Geom &g, const int32_t *__restrict__ bi
                 end = __ldg(off + cell_hash<D>(g, xhi, ny, nz) + 1);
             }
         }
-    } else {
-        if (lane < (D == 2 ? 9 : 27)) {
-            int nx = 0, ny = 0, nz = 0;
-            bool ok = neighbor_axis(cx, lane % 3 - 1, g.g[0], g.periodic, nx, sx);
-            ok = neighbor_axis(cy, (lane / 3) % 3 - 1, g.g[1], g.periodic, ny, sy) && ok;
-            if (D == 3) ok = neighbor_axis(cz, lane / 9 - 1, g.g[2], g.periodic, nz, sz) && ok;
-            if (ok) {
-                const uint32_t hsh = cell_hash<D>(g, nx, ny, nz);
-                start = __ldg(off + hsh);
-                end = __ldg(off + hsh + 1);
-            }
+    } else if (k < (D == 2 ? 9 : 27)) {
+        int nx = 0, ny = 0, nz = 0;
+        bool ok = neighbor_axis(cx, k % 3 - 1, g.g[0], g.periodic, nx, sx);
+        ok = neighbor_axis(cy, (k / 3) % 3 - 1, g.g[1], g.periodic, ny, sy) && ok;
+        if (D == 3) ok = neighbor_axis(cz, k / 9 - 1, g.g[2], g.periodic, nz, sz) && ok;
+        if (ok) {
+            const uint32_t hsh = cell_hash<D>(g, nx, ny, nz);
+            start = __ldg(off + hsh);
+            end = __ldg(off + hsh + 1);
         }
     }
+    code = shift_code(sx, sy, sz);
+}
+
+// Fills rng[0..n) with the non-empty candidate ranges [start, end) of global
+// particle indices for the cell of `it`; returns n.  Must be called by all 32
+// lanes; rng is per-warp shared memory of kMaxRanges entries.
+template <int D>
+__device__ inline int build_ranges(const Geom &g, const int32_t *__restrict__ bin_offsets,
+                                   const WorkItem &it, int4 *rng) {
+    const int lane = threadIdx.x & 31;
+    int cx, cy, cz, start, end, code;
+    hash_to_cell<D>(g, (uint32_t)(it.cell - it.sys * g.cells), cx, cy, cz);
+    range_piece<D>(g, bin_offsets + (size_t)it.sys * g.cells, cx, cy, cz, lane, start, end, code);
     const bool nonempty = end > start;
     const unsigned m = __ballot_sync(kFull, nonempty);
-    if (nonempty) rng[__popc(m & ((1u << lane) - 1))] = make_int4(start, end, shift_code(sx, sy, sz), 0);
+    if (nonempty) rng[__popc(m & ((1u << lane) - 1))] = make_int4(start, end, code, 0);
     __syncwarp();
     return __popc(m);
 }

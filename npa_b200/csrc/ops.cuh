@@ -11,7 +11,9 @@ enum { S_COUNT = 1, S_DENSITY = 2, S_DGRAD = 4, S_MOMENT = 8 };
 // F_MOMENT (forward only) adds the moment matrix to a blur + gradient sweep.
 // F_PACK (forward only, with all three others) applies the perception epilogue per particle and
 // writes the packed perception vector instead of the separate tensors.
-enum { F_BLUR = 1, F_GRAD = 2, F_MOMENT = 4, F_PACK = 8 };
+// Over neighbour lists also: F_DGRAD sums the density gradient (rho_grad_out) and F_CORRECTED (with F_GRAD |
+// F_MOMENT) writes gradient . safe_inv(moment) in place of the gradient.
+enum { F_BLUR = 1, F_GRAD = 2, F_MOMENT = 4, F_PACK = 8, F_DGRAD = 16, F_CORRECTED = 32 };
 bool tile_forward_enabled();  // tile_host.cu: the cell-tile streaming engine is switched on for forward sweeps
 
 struct ScalarFwdArgs {
@@ -27,6 +29,7 @@ struct ScalarFwdArgs {
     int32_t *pair_cache;  // neighbour lists to write ([B*N, pair_stride]) or NULL
     int pair_stride;
     unsigned int *tickets;  // row tickets of this launch (set by the launcher)
+    float4 *pv;             // [B*N] out: (x, y, z, m / rho), or NULL (S_DENSITY)
 };
 
 struct ScalarBwdArgs {
@@ -42,8 +45,6 @@ struct ScalarBwdArgs {
     int accumulate_x;         // add into grad_x instead of overwriting
     const int32_t *bin_offsets;
     const int32_t *block_info;
-    const int32_t *pair_cache;  // neighbour lists of this snapshot to read, or NULL
-    int pair_stride;
     unsigned int *tickets;  // row tickets of this launch (set by the launcher)
 };
 
@@ -72,6 +73,7 @@ struct FeatureFwdArgs {
     int pair_stride;
     int pair_cache_valid;    // 0: this sweep writes the lists; 1: they are valid, read them instead of searching
     unsigned int *tickets;  // row tickets of this launch (set by the launcher)
+    const float4 *pv;        // [B*N] (x, y, z, m / rho) written by the density sweep, or NULL (lists only)
 };
 
 struct FeatureBwdArgs {
@@ -91,6 +93,43 @@ struct FeatureBwdArgs {
     int pair_stride;
     unsigned int *tickets;  // row tickets of this launch (set by the launcher)
 };
+
+// Backward of blur and / or gradient over neighbour lists (feature_list.cuh).
+struct FeatureListBwdArgs {
+    const float *x, *mass, *rho, *s;
+    const float4 *pv;         // as above, or NULL
+    const float *gb;          // dL/dblur, rows of gb_pitch floats, 16-byte aligned, padded to cp features
+    const float *gg;          // dL/dgradient as [N, D, cp] inside rows of gg_pitch floats, 16-byte aligned
+    int gb_pitch, gg_pitch, cp;
+    const float *direct;      // rows of direct_pitch floats added to grad_s, or NULL
+    int direct_pitch;
+    const float *g_dg;        // upstream of the density gradient [B,N,D] (its part of grad_x is added), or NULL
+    const float *g_rho;       // upstream of the density [B,N], or NULL: only goes into pg
+    float *grad_x, *grad_s, *grad_rho;
+    float4 *pg;               // [B*N] (x, y, z, g_rho + drho) for the density backward, or NULL
+    int C;
+    const int32_t *bin_offsets;
+    const int32_t *pair_cache;
+    int pair_stride;
+};
+
+// Backward of density (upstream g_rho_a + g_rho_b, or packed in pg) and density gradient over neighbour lists, and the
+// density gradient itself over lists (scalar_list.cu).
+struct ScalarListArgs {
+    const float *x, *mass, *g_rho_a, *g_rho_b, *g_dg;
+    const float4 *pg;
+    float *grad_x;
+    int accumulate_x;
+    float *rho_grad_out;
+    const int32_t *bin_offsets, *pair_cache;
+    int pair_stride;
+};
+int launch_scalar_list_backward(const Geom &g, const ScalarListArgs &a, cudaStream_t st);
+int launch_density_gradient_list(const Geom &g, const ScalarListArgs &a, cudaStream_t st);
+int launch_feature_list_forward(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st);
+int launch_feature_list_backward(const Geom &g, int mask, bool full, const FeatureListBwdArgs &a, cudaStream_t st);
+// [N, C(, D)] upstreams -> rows [N, (1 +) D, cp] of `rows` (blur part only when with_blur).
+int launch_upstream_rows(const Geom &g, int C, const float *g_blur, const float *g_grad, bool with_blur, float *rows, cudaStream_t st);
 
 // Number of CTAs of a persistent launch of `kernel`: every SM filled to the kernel's occupancy.
 // Cached per (device, kernel); the first call also raises the kernel's dynamic shared-memory

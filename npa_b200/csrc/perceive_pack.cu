@@ -34,28 +34,41 @@ __device__ inline void log_normalize_backward(const float *w, const float *gin, 
 }
 
 // One thread per (particle, feature): dL/dz -> dL/dblur, dL/dgrad; the thread of feature 0 also
-// handles the density-gradient part.
-template <int D>
+// handles the density-gradient part.  ROWS: the rows the backward over neighbour lists reads, blur and the D
+// axes of the gradient as cp floats each (g_blur = the rows, g_grad unused, columns C..cp-1 zero); otherwise the
+// operators' own layouts.
+template <int D, bool ROWS>
 __global__ void __launch_bounds__(256)
 pack_backward_kernel(const float *__restrict__ gz, const float *__restrict__ vgrad, const float *__restrict__ rho_grad,
                      float *__restrict__ g_blur, float *__restrict__ g_grad, float *__restrict__ g_rho_grad,
                      long long particles, int C, float coef, float dg_scale, int log_norm_grad, int log_norm_dg) {
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
-    if (t >= particles * C) return;
-    const long long i = t / C;
-    const int f = (int)(t - i * C);
+    const int cp = ROWS ? (C + 3) & ~3 : C;
+    if (t >= particles * cp) return;
+    const long long i = t / cp;
+    const int f = (int)(t - i * cp);
     const int Z = 2 * C + C * D + D;
     const float *gr = gz + i * Z;
-    g_blur[t] = gr[C + f];
+    float *row = ROWS ? g_blur + i * ((1 + D) * cp) + f : nullptr;
+    if (ROWS && f >= C) {
+#pragma unroll
+        for (int d = 0; d <= D; ++d) row[d * cp] = 0.f;
+        return;
+    }
+    if (ROWS) row[0] = gr[C + f];
+    else g_blur[t] = gr[C + f];
     float w[D], gin[D], gout[D];
 #pragma unroll
     for (int d = 0; d < D; ++d) {
-        w[d] = vgrad[t * D + d] * coef;
+        w[d] = vgrad[(i * C + f) * D + d] * coef;
         gin[d] = gr[2 * C + f * D + d];
     }
     log_normalize_backward<D>(w, gin, log_norm_grad, coef, gout);
 #pragma unroll
-    for (int d = 0; d < D; ++d) g_grad[t * D + d] = gout[d];
+    for (int d = 0; d < D; ++d) {
+        if (ROWS) row[(1 + d) * cp] = gout[d];
+        else g_grad[t * D + d] = gout[d];
+    }
     if (f == 0 && g_rho_grad) {
 #pragma unroll
         for (int d = 0; d < D; ++d) {
@@ -83,11 +96,11 @@ using namespace npa;
 
 extern "C" {
 
-int npa_perceive_features_forward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
-                                  const float *s_bin, float coef, float dg_scale, float inv_tol,
-                                  int32_t log_norm_grad, int32_t log_norm_dg, float *rho, float *rho_grad,
-                                  float *z, float *vgrad, const int32_t *bin_offsets, const int32_t *block_info,
-                                  int32_t *pair_cache, int32_t pair_stride, void *stream) {
+int npa_perceive_features_forward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                        const float *s_bin, float coef, float dg_scale, float inv_tol,
+                                        int32_t log_norm_grad, int32_t log_norm_dg, float *rho, float *rho_grad,
+                                        float *z, float *vgrad, float *packed, const int32_t *bin_offsets, const int32_t *block_info,
+                                        int32_t *pair_cache, int32_t pair_stride, void *stream) {
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
@@ -103,8 +116,11 @@ int npa_perceive_features_forward(const npa_grid *gd, int32_t channels, const fl
     // gradient; the first sweep is then the density alone (and the neighbour lists), which the shared-
     // candidate kernel runs in about half the time of the density + density-gradient sweep.  With the
     // cell-tile engine switched on (it has no such sum) the first sweep computes both as before.
+    if (packed && ((uintptr_t)packed % 16 || !pair_cache))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "perceive_features_forward: packed must be 16-byte aligned and needs neighbour lists");
     const bool in_sweep = !tile_forward_enabled();
     ScalarFwdArgs sa = {x_bin, mass, nullptr, nullptr, rho, in_sweep ? nullptr : rho_grad, nullptr, bin_offsets, block_info, pair_cache, pair_stride};
+    sa.pv = reinterpret_cast<float4 *>(packed);
     if ((rc = launch_scalar_forward(g, in_sweep ? S_DENSITY : (S_DENSITY | S_DGRAD), sa, st)) != NPA_OK) return rc;
     FeatureFwdArgs fa = {x_bin, mass, rho, s_bin, nullptr, nullptr, channels, bin_offsets, block_info, nullptr};
     fa.z = z;
@@ -117,12 +133,76 @@ int npa_perceive_features_forward(const npa_grid *gd, int32_t channels, const fl
     fa.inv_tol = inv_tol;
     fa.log_norm_grad = log_norm_grad;
     fa.log_norm_dg = log_norm_dg;
-    if (pair_cache && (pair_stride < 2 || pair_stride > 513))
-        return fail(NPA_ERR_INVALID_ARGUMENT, "perceive_features_forward: pair_stride must be in [2, 513]");
+    fa.pv = sa.pv;
     fa.pair_cache = pair_cache;
     fa.pair_stride = pair_stride;
     fa.pair_cache_valid = pair_cache != nullptr;  // written by the density sweep above
     return launch_feature_forward(g, F_BLUR | F_GRAD | F_MOMENT | F_PACK, fa, st);
+}
+
+int npa_perceive_features_forward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                  const float *s_bin, float coef, float dg_scale, float inv_tol,
+                                  int32_t log_norm_grad, int32_t log_norm_dg, float *rho, float *rho_grad,
+                                  float *z, float *vgrad, const int32_t *bin_offsets, const int32_t *block_info,
+                                  int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    return npa_perceive_features_forward_lists(gd, channels, x_bin, mass, s_bin, coef, dg_scale, inv_tol, log_norm_grad, log_norm_dg, rho,
+                                               rho_grad, z, vgrad, nullptr, bin_offsets, block_info, pair_cache, pair_stride, stream);
+}
+
+int64_t npa_lists_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
+    Geom g;
+    const int rc = make_geom(gd, &g);
+    if (rc != NPA_OK) return rc;
+    if (channels < 0) return fail(NPA_ERR_INVALID_ARGUMENT, "lists_backward_scratch_bytes: channels must not be negative");
+    // upstream rows, the density gradient's upstream (rounded up to whole 16-byte records), position + upstream records
+    const int64_t n = (int64_t)g.B * g.N, cp = (channels + 3) & ~3;
+    return n * (1 + g.dim) * cp * 4 + n * 16 + n * 16;
+}
+
+int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                         const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
+                                         int32_t log_norm_dg, float *grad_x, float *grad_s, void *scratch, int64_t scratch_bytes,
+                                         const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "perceive_features_backward_lists";
+    Geom g;
+    int rc = make_geom(gd, &g);
+    if (rc != NPA_OK) return rc;
+    if (!x_bin || !s_bin || !rho || !rho_grad || !vgrad || !dL_dz || !scratch || !bin_offsets || !pair_cache)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: a required pointer is NULL", me);
+    if (channels <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: channels must be positive", me);
+    if (((uintptr_t)x_bin | (uintptr_t)grad_x) % (g.dim == 2 ? 8 : 16) || ((uintptr_t)scratch | (uintptr_t)packed) % 16)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: positions, packed or scratch are misaligned", me);
+    if (pair_stride < 2 || pair_stride > 513) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: pair_stride must be in [2, 513]", me);
+    if (scratch_bytes < npa_lists_backward_scratch_bytes(gd, channels))
+        return fail(NPA_ERR_SCRATCH_TOO_SMALL, "%s: scratch holds %lld bytes, %lld needed", me, (long long)scratch_bytes,
+                    (long long)npa_lists_backward_scratch_bytes(gd, channels));
+    if (!grad_x && !grad_s) return NPA_OK;
+    cudaStream_t st = (cudaStream_t)stream;
+    const long long n = (long long)g.B * g.N;
+    const int cp = (channels + 3) & ~3, pitch = (1 + g.dim) * cp;
+    float *rows = static_cast<float *>(scratch), *g_dg = rows + n * pitch;
+    float4 *pg = reinterpret_cast<float4 *>(g_dg + n * 4);
+    const unsigned blocks = (unsigned)((n * cp + 255) / 256);
+    if (g.dim == 2)
+        pack_backward_kernel<2, true><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+                                                              dg_scale, log_norm_grad, log_norm_dg);
+    else
+        pack_backward_kernel<3, true><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+                                                              dg_scale, log_norm_grad, log_norm_dg);
+    if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
+    FeatureListBwdArgs a = {};
+    a.x = x_bin; a.mass = mass; a.rho = rho; a.s = s_bin; a.pv = reinterpret_cast<const float4 *>(packed);
+    a.gb = rows; a.gg = rows + cp; a.gb_pitch = a.gg_pitch = pitch; a.cp = cp;
+    a.direct = dL_dz; a.direct_pitch = 2 * channels + channels * g.dim + g.dim;  // the features enter z unchanged as its first columns
+    a.g_dg = grad_x ? g_dg : nullptr;
+    a.grad_x = grad_x; a.grad_s = grad_s; a.pg = grad_x ? pg : nullptr; a.C = channels;
+    a.bin_offsets = bin_offsets; a.pair_cache = pair_cache; a.pair_stride = pair_stride;
+    if ((rc = launch_feature_list_backward(g, F_BLUR | F_GRAD, grad_x != nullptr, a, st)) != NPA_OK || !grad_x) return rc;
+    ScalarListArgs d = {};
+    d.x = x_bin; d.mass = mass; d.pg = pg; d.grad_x = grad_x; d.accumulate_x = 1;
+    d.bin_offsets = bin_offsets; d.pair_cache = pair_cache; d.pair_stride = pair_stride;
+    return launch_scalar_list_backward(g, d, st);
 }
 
 int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
@@ -147,10 +227,10 @@ int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const f
     const unsigned blocks = (unsigned)((particles * channels + 255) / 256);
     float *grg = grad_x ? g_rho_grad_scratch : nullptr;
     if (g.dim == 2)
-        pack_backward_kernel<2><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
+        pack_backward_kernel<2, false><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
                                                         particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
     else
-        pack_backward_kernel<3><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
+        pack_backward_kernel<3, false><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
                                                         particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
     if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
     rc = npa_perception_backward(gd, channels, x_bin, mass, s_bin, rho, nullptr, g_blur_scratch, g_grad_scratch, grg,

@@ -128,7 +128,11 @@ scalar_forward_kernel(ScalarFwdArgs a, Geom g) {
             if (ivalid && sl == 0) {
                 if (list) list[-1] = listed <= K - 1 ? listed : -1;
                 if ((MASK & S_COUNT) && a.count) a.count[i] = cnt;
-                if (kPoly && a.rho_out) a.rho_out[i] = g.c_s * rho;
+                if (kPoly && a.rho_out) {
+                    const float r = g.c_s * rho;
+                    a.rho_out[i] = r;
+                    if (a.pv) a.pv[i] = make_float4(pi.x, pi.y, pi.z, (a.mass ? __ldg(a.mass + i) : 1.0f) / r);
+                }
                 if ((MASK & S_DGRAD) && a.rho_grad) {
 #pragma unroll
                     for (int d = 0; d < D; ++d) a.rho_grad[i * D + d] = g.c_g * dg[d];
@@ -349,7 +353,11 @@ scalar_forward_shared_kernel(ScalarFwdArgs a, Geom g, int span, int batch) {
                 if (ivalid) {
                     if (list) list[-1] = listed <= K - 1 ? listed : -1;
                     if ((MASK & S_COUNT) && a.count) a.count[i] = cnt;
-                    if (kPoly && a.rho_out) a.rho_out[i] = g.c_s * rho;
+                    if (kPoly && a.rho_out) {
+                    const float r = g.c_s * rho;
+                    a.rho_out[i] = r;
+                    if (a.pv) a.pv[i] = make_float4(pi.x, pi.y, pi.z, (a.mass ? __ldg(a.mass + i) : 1.0f) / r);
+                }
                     if ((MASK & S_DGRAD) && a.rho_grad) {
 #pragma unroll
                         for (int d = 0; d < D; ++d) a.rho_grad[i * D + d] = g.c_g * dg[d];
@@ -372,10 +380,8 @@ scalar_forward_shared_kernel(ScalarFwdArgs a, Geom g, int span, int batch) {
     release_rows(a.tickets);
 }
 
-// Gather backward of density / density gradient / moment matrix, same layout (8 particles per warp
-// pass, 4 lanes each).  With a neighbour-list cache of the snapshot the lanes of a sub-group walk
-// the list of their particle; particles without a list (cache off, or more neighbours than the
-// list holds) test the candidates of the cells.
+// Gather backward of density / density gradient / moment matrix by the cell search, same layout (8
+// particles per warp pass, 4 lanes each); over neighbour lists it is scalar_list.cu.
 template <int D, bool PER, int MASK>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 scalar_backward_kernel(ScalarBwdArgs a, Geom g) {
@@ -385,7 +391,6 @@ scalar_backward_kernel(ScalarBwdArgs a, Geom g) {
     const int sub = lane / kScalarLpp, sl = lane % kScalarLpp;
     constexpr bool kSpiky = (MASK & (S_DGRAD | S_MOMENT)) != 0;
     constexpr int DD = D * D;
-    const int K = a.pair_stride;
 
     const int vrows = g.max_blocks * g.split;
     for (int vrow = next_row(a.tickets); vrow < vrows; vrow = next_row(a.tickets)) {
@@ -471,30 +476,16 @@ scalar_backward_kernel(ScalarBwdArgs a, Geom g) {
                 }
             };
 
-            int listed = -1;  // the same in the four lanes of a sub-group
-            if (a.pair_cache && ivalid) listed = __ldg(a.pair_cache + i * K);
-            if (listed >= 0) {
-                const int32_t *list = a.pair_cache + i * K + 1;
-                for (int e = sl; e < listed; e += kScalarLpp) {
-                    const int j = __ldg(list + e);
+            for (int r = 0; r < nr; ++r) {
+                const int4 rg = rng[r];
+                const Origin<D, PER> org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, rg.z);
+                for (int j0 = rg.x; j0 < rg.y; j0 += kScalarLpp) {
+                    const int j = j0 + sl;
+                    if (!(ivalid && j < rg.y)) continue;
                     const Pos<D> pj = load_pos<D>(a.x, j);
                     float rx, ry, rz;
-                    listed_displacement<D, PER>(g, pi, pj, rx, ry, rz);
-                    visit(j, rx, ry, rz, sq_norm_fast<D>(rx, ry, rz));
-                }
-            }
-            if (__any_sync(kFull, ivalid && listed < 0)) {
-                for (int r = 0; r < nr; ++r) {
-                    const int4 rg = rng[r];
-                    const Origin<D, PER> org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, rg.z);
-                    for (int j0 = rg.x; j0 < rg.y; j0 += kScalarLpp) {
-                        const int j = j0 + sl;
-                        if (!(ivalid && listed < 0 && j < rg.y)) continue;
-                        const Pos<D> pj = load_pos<D>(a.x, j);
-                        float rx, ry, rz;
-                        const float q = displacement<D, PER, false>(g, org, pj.x, pj.y, pj.z, rx, ry, rz);
-                        if (q < g.h2) visit(j, rx, ry, rz, q);
-                    }
+                    const float q = displacement<D, PER, false>(g, org, pj.x, pj.y, pj.z, rx, ry, rz);
+                    if (q < g.h2) visit(j, rx, ry, rz, q);
                 }
             }
 

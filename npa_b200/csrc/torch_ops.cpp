@@ -149,6 +149,13 @@ Tensor new_lists(const Grid &g, const Tensor &like, int64_t columns) {
     return columns ? at::empty({g.B, g.N, columns}, like.options().dtype(at::kInt).requires_grad(false)) : Tensor();
 }
 
+// Work memory of a backward over lists.
+Tensor list_scratch(const Grid &g, const Tensor &like, int64_t channels) {
+    const int64_t bytes = npa_lists_backward_scratch_bytes(&g.g, (int)channels);
+    if (bytes < 0) check_status((int)bytes);
+    return floats(like, {bytes / 4});
+}
+
 // ---- reorder into cell order (Permute, sph.py:127-184) ---------------------------------------------
 struct ReorderNode : Node {
     GridPtr grid;
@@ -239,6 +246,8 @@ py::tuple density(const GridPtr &grid, const Tensor &offs, const Tensor &info, c
     if (want_rho)
         check_status(npa_perception_forward(&g.g, 0, fptr(x), fptr(sn.mass), nullptr, fmut(rho), nullptr, fmut(dg), nullptr, nullptr, nullptr,
                                             iptr(offs), iptr(info), write ? imut(sn.pairs) : nullptr, write ? sn.stride() : 0, stream_of(x)));
+    else if (sn.pairs.defined())
+        check_status(npa_density_gradient_forward_lists(&g.g, fptr(x), fptr(sn.mass), fmut(dg), iptr(offs), iptr(sn.pairs), sn.stride(), stream_of(x)));
     else
         check_status(npa_density_gradient_forward(&g.g, fptr(x), fptr(sn.mass), fmut(dg), iptr(offs), iptr(info), stream_of(x)));
     if (recording(x)) {
@@ -262,9 +271,16 @@ struct FeatureNode : SweepNode {
         if ((!gb.defined() && !gg.defined()) || !(nx || ns || nr)) return {Tensor(), Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nr ? blank(rho) : Tensor();
-        if (s.size(2) > 0)
-            check_status(npa_blur_gradient_backward(&grid->g, (int)s.size(2), fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx),
-                                                    fmut(gs), fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+        const int C = (int)s.size(2);
+        if (C > 0 && pairs.defined()) {
+            Tensor work = list_scratch(*grid, s, C);
+            check_status(npa_blur_gradient_backward_lists(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
+                                                          fmut(gr), work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
+                                                          stream_of(x)));
+        } else if (C > 0) {
+            check_status(npa_blur_gradient_backward(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
+                                                    fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
+        }
         return {gx, gs, gr};
     }
     void release_variables() override {
@@ -300,6 +316,32 @@ py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &i
     }
     auto cast = [](const Tensor &t) -> py::object { return t.defined() ? py::cast(t) : py::none(); };
     return py::make_tuple(cast(blur), cast(grad), cast(moment));
+}
+
+// gradient_hybrid (sph.py:474-484) over neighbour lists: the value is gradient . inv(moment), the gradient that of the
+// raw operator.
+Tensor gradient_hybrid(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const Tensor &s,
+                       const OptTensor &mass, const Tensor &pairs, double rtol) {
+    Snap sn(grid, offs, info, mass, pairs);
+    Grid &g = *grid;
+    g.positions(x, "binned_positions");
+    g.rows(rho, "rho");
+    g.features(s, "state_in");
+    const int64_t C = s.size(2);
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = floats(s, {g.B, g.N, C, g.D});
+    if (C > 0)
+        check_status(npa_gradient_hybrid_forward_lists(&g.g, (int)C, fptr(x), fptr(rho), fptr(sn.mass), fptr(s), (float)rtol, fmut(out), iptr(offs),
+                                                       iptr(sn.pairs), sn.stride(), stream_of(x)));
+    if (recording(x, s, rho)) {
+        auto n = node_for<FeatureNode>(x, s, rho);
+        n->keep(grid, offs, info, sn.pairs, x, sn.mass);
+        n->s_ = SavedVariable(s, false);
+        n->rho_ = SavedVariable(rho, false);
+        n->has_blur = false; n->has_grad = true;
+        torch::autograd::set_history(out, n);
+    }
+    return out;
 }
 
 // ---- moment matrix -----------------------------------------------------------------------------------
@@ -338,7 +380,7 @@ Tensor moment_matrix(const GridPtr &grid, const Tensor &offs, const Tensor &info
     return out;
 }
 
-// ---- moment-corrected gradient (sph.py:474-484): value raw @ inv(M), gradient of the raw operator ----------
+// ---- the same from a gradient and a moment matrix that are there already ------------------------------------
 struct StraightThroughNode : Node {
     variable_list apply(variable_list &&g) override { return {g[0]}; }
 };
@@ -361,6 +403,7 @@ Tensor corrected_gradient(const Tensor &raw, const Tensor &moment, double rtol) 
 // ---- the fused perception step -------------------------------------------------------------------------
 struct PerceptionNode : SweepNode {
     SavedVariable s_, rho_;
+    Tensor packed;  // (x, y, z, m / rho) records of the density sweep
     bool has_dg;
     variable_list apply(variable_list &&g) override {
         const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(shared_from_this()), mass = mass_.unpack();
@@ -368,15 +411,23 @@ struct PerceptionNode : SweepNode {
         if (!(nx || ns)) return {Tensor(), Tensor()};
         const Tensor g_rho = nx ? solid(g[0]) : Tensor(), gb = solid(g[1]), gg = solid(g[2]), g_dg = nx && has_dg ? solid(g[3]) : Tensor();
         c10::cuda::CUDAGuard guard(x.device());
-        Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nx ? blank(rho) : Tensor();
+        Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
+        if (pairs.defined()) {
+            Tensor work = list_scratch(*grid, s, s.size(2));
+            check_status(npa_perception_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(packed), fptr(g_rho),
+                                                       fptr(gb), fptr(gg), fptr(g_dg), fmut(gx), fmut(gs), work.mutable_data_ptr(), work.numel() * 4,
+                                                       iptr(offs), iptr(pairs), list_stride(), stream_of(x)));
+            return {gx, gs};
+        }
+        Tensor gr = nx ? blank(rho) : Tensor();
         check_status(npa_perception_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(g_rho), fptr(gb), fptr(gg),
-                                             fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(),
-                                             stream_of(x)));
+                                             fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
         return {gx, gs};
     }
     void release_variables() override {
         SweepNode::release_variables();
         s_.reset_data(); rho_.reset_data();
+        packed = Tensor();
     }
 };
 
@@ -391,13 +442,19 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
     const bool record = recording(x, s);
     Tensor rho = floats(x, {g.B, g.N}), blur = blank(s), grad = floats(s, {g.B, g.N, C, g.D});
     Tensor dg = want_dg ? floats(x, {g.B, g.N, g.D}) : Tensor(), pairs = new_lists(g, x, columns);
-    check_status(npa_perception_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), fmut(rho), nullptr, fmut(dg), fmut(blur), fmut(grad), nullptr,
-                                        iptr(offs), iptr(info), imut(pairs), pairs.defined() ? (int)columns : 0, stream_of(x)));
+    Tensor packed = columns ? floats(x, {g.B, g.N, 4}) : Tensor();
+    if (columns)
+        check_status(npa_perception_forward_lists(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), fmut(rho), fmut(dg), fmut(blur), fmut(grad),
+                                                  fmut(packed), iptr(offs), iptr(info), imut(pairs), (int)columns, stream_of(x)));
+    else
+        check_status(npa_perception_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), fmut(rho), nullptr, fmut(dg), fmut(blur), fmut(grad),
+                                            nullptr, iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
     if (record) {
         auto n = node_for<PerceptionNode>(x, s);
         n->keep(grid, offs, info, pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
         n->has_dg = want_dg;
+        n->packed = packed;
         torch::autograd::set_history(rho, n);
         torch::autograd::set_history(blur, n);
         torch::autograd::set_history(grad, n);
@@ -410,7 +467,7 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
 // ---- the packed perception row ---------------------------------------------------------------------------
 struct PackedNode : SweepNode {
     SavedVariable s_;
-    Tensor rho, rho_grad, vgrad;
+    Tensor rho, rho_grad, vgrad, packed;
     float coef, dg_scale;
     bool ln_grad, ln_dg;
     variable_list apply(variable_list &&g) override {
@@ -419,6 +476,14 @@ struct PackedNode : SweepNode {
         if (!g[0].defined() || !(nx || ns)) return {Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(x.device());
         const Tensor gz = g[0].contiguous();
+        if (pairs.defined()) {
+            Tensor work = list_scratch(*grid, s, s.size(2)), gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
+            check_status(npa_perceive_features_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad),
+                                                              fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, fmut(gx), fmut(gs),
+                                                              work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
+                                                              stream_of(x)));
+            return {gx, gs};
+        }
         const int64_t n = s.numel(), D = grid->D, rows = rho.numel();
         // dL/dblur and dL/dgradient of the rows, and with position gradients the two per-particle upstreams, in one buffer
         Tensor work = floats(s, {n * (1 + D) + (nx ? rows * (1 + D) : 0)});
@@ -426,13 +491,13 @@ struct PackedNode : SweepNode {
         Tensor gx = nx ? blank(x) : Tensor(), gs = blank(s);
         check_status(npa_perceive_features_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad), fptr(vgrad),
                                                     fptr(gz), coef, dg_scale, ln_grad, ln_dg, gb, gg, g_dg, gr, fmut(gx), fmut(gs), iptr(offs),
-                                                    iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+                                                    iptr(info), nullptr, 0, stream_of(x)));
         return {gx, ns ? gs : Tensor()};
     }
     void release_variables() override {
         SweepNode::release_variables();
         s_.reset_data();
-        rho = rho_grad = vgrad = Tensor();
+        rho = rho_grad = vgrad = packed = Tensor();
     }
 };
 
@@ -447,14 +512,15 @@ Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &
     const bool record = recording(x, s);
     Tensor rho = floats(x, {g.B, g.N}), rho_grad = floats(x, {g.B, g.N, D}), z = floats(s, {g.B, g.N, 2 * C + C * D + D});
     Tensor vgrad = record ? floats(s, {g.B, g.N, C, D}) : Tensor(), pairs = new_lists(g, x, columns);
-    check_status(npa_perceive_features_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), (float)coef, (float)dg_scale, (float)inv_tol, ln_grad,
-                                               ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), iptr(offs), iptr(info), imut(pairs),
-                                               pairs.defined() ? (int)columns : 0, stream_of(x)));
+    Tensor packed = columns ? floats(x, {g.B, g.N, 4}) : Tensor();
+    check_status(npa_perceive_features_forward_lists(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), (float)coef, (float)dg_scale, (float)inv_tol,
+                                                     ln_grad, ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), fmut(packed), iptr(offs),
+                                                     iptr(info), imut(pairs), pairs.defined() ? (int)columns : 0, stream_of(x)));
     if (record) {
         auto n = node_for<PackedNode>(x, s);
         n->keep(grid, offs, info, pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
-        n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad;
+        n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad; n->packed = packed;
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->ln_grad = ln_grad; n->ln_dg = ln_dg;
         torch::autograd::set_history(z, n);
     }
@@ -618,6 +684,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("unreorder", &unreorder);
     m.def("density", &density);
     m.def("blur_gradient", &blur_gradient);
+    m.def("gradient_hybrid", &gradient_hybrid);
     m.def("moment_matrix", &moment_matrix);
     m.def("corrected_gradient", &corrected_gradient);
     m.def("perception", &perception);

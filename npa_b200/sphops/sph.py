@@ -332,6 +332,9 @@ def safe_inv_sym_mat(M, rtol=1e-6):
 
 def gradient_hybrid(x_bin, rho, s_bin, snapshot, mass=None):
     """Moment-corrected gradient: value ``raw @ inv(M)``, gradient of the raw SPH gradient."""
+    pairs = _lists_of(snapshot, x_bin)
+    if pairs is not None and "gradient" not in snapshot.parked:
+        return _ops.gradient_hybrid(*_sweep_args(snapshot), x_bin, rho, s_bin, _mass(mass), pairs, 1e-3)
     with torch.no_grad():
         M = moment_matrix(x_bin, rho, snapshot, mass=mass)
     raw = gradient(x_bin, rho, s_bin, snapshot, mass=mass)

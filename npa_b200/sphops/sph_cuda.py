@@ -128,6 +128,12 @@ class _HashGridBase:
             raise RuntimeError(f"pair_cache must have between 2 and 513 columns, got {K}")
         return N.ptr(pair_cache), K
 
+    def _list_scratch(self, channels, device):
+        """Work memory of a backward over neighbour lists, private to the call."""
+        n = _lib.npa_lists_backward_scratch_bytes(self._ref(), channels)
+        N.check(int(n) if n < 0 else 0)
+        return torch.empty(int(n), dtype=torch.uint8, device=device), int(n)
+
     @staticmethod
     def _call(fn, tensor_for_device, *args):
         device = tensor_for_device.device.index
@@ -366,6 +372,12 @@ class _HashGridBase:
         self._snap(bin_offsets, block_info)
         if C == 0:
             return
+        if pair_cache is not None:
+            pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
+            self._call(_lib.npa_blur_gradient_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
+                       N.ptr(rho), N.ptr(mass), N.ptr(state_in), N.ptr(dL_blur_state_out), N.ptr(dL_grad_state_out),
+                       N.ptr(grad_x), N.ptr(grad_s), N.ptr(grad_rho), N.ptr(scratch[0]), scratch[1], N.ptr(bin_offsets), *pairs)
+            return
         self._call(_lib.npa_blur_gradient_backward, binned_positions, self._ref(), C, N.ptr(binned_positions),
                    N.ptr(rho), N.ptr(mass), N.ptr(state_in), N.ptr(dL_blur_state_out), N.ptr(dL_grad_state_out),
                    N.ptr(grad_x), N.ptr(grad_s), N.ptr(grad_rho), N.ptr(bin_offsets), N.ptr(block_info),
@@ -435,6 +447,13 @@ class _HashGridBase:
         if grad_s is not None:
             self._bn(grad_s, "grad_s", C)
         self._snap(bin_offsets, block_info)
+        if pair_cache is not None:
+            pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
+            self._call(_lib.npa_perceive_features_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
+                       N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(density_gradient), N.ptr(corrected_gradient), None,
+                       N.ptr(dL_dz), float(coef), float(dg_scale), 1 if log_norm_grad else 0, 1 if log_norm_dg else 0,
+                       N.ptr(grad_x), N.ptr(grad_s), N.ptr(scratch[0]), scratch[1], N.ptr(bin_offsets), *pairs)
+            return
         self._call(_lib.npa_perceive_features_backward, binned_positions, self._ref(), C, N.ptr(binned_positions),
                    N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(density_gradient), N.ptr(corrected_gradient),
                    N.ptr(dL_dz), float(coef), float(dg_scale), 1 if log_norm_grad else 0, 1 if log_norm_dg else 0,
@@ -523,6 +542,13 @@ class _HashGridBase:
             self._bn(grad_s, "grad_s", C)
         if grad_rho_scratch is not None:
             self._bn(grad_rho_scratch, "grad_rho_scratch")
+        if pair_cache is not None and C > 0:
+            pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
+            self._call(_lib.npa_perception_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
+                       N.ptr(mass), N.ptr(state_in), N.ptr(rho), None, N.ptr(dL_rho_out), N.ptr(dL_blur_state_out),
+                       N.ptr(dL_grad_state_out), N.ptr(dL_density_gradient_out), N.ptr(grad_x), N.ptr(grad_s),
+                       N.ptr(scratch[0]), scratch[1], N.ptr(bin_offsets), *pairs)
+            return
         self._call(_lib.npa_perception_backward, binned_positions, self._ref(), C, N.ptr(binned_positions),
                    N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(dL_rho_out), N.ptr(dL_blur_state_out),
                    N.ptr(dL_grad_state_out), N.ptr(dL_density_gradient_out), N.ptr(grad_x), N.ptr(grad_s),
