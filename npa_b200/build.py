@@ -30,6 +30,7 @@ NVCC_FLAGS = [
     "-O3", "-lineinfo", "-std=c++17",
     "-Xcompiler", "-fPIC",
     "--expt-relaxed-constexpr",
+    "--compress-mode=size",  # the library is a hundred megabytes of sparse device code otherwise
 ]
 
 

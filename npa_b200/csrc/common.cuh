@@ -186,18 +186,28 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
 // Spiky pair factors for 0 < q < h2: phi = 3 (h - d)^2 / d with
 // d = sqrt(q + 1e-12), so that K(r) = phi * r; psi = 3 (h^2 - d^2) / d^3 so that
 // dK/dr = phi * I - psi * r r^T.
-__device__ inline float spiky_phi(float q, float h, float &d_out) {
-    float d = sqrtf(q + 1e-12f);
-    float t = fmaxf(h - d, 0.0f);
-    d_out = d;
-    return 3.0f * t * t / d;
+// d and 1 / d come from one reciprocal square root with a Newton step each (tests/test_gpu_neighbour_lists.py holds
+// the kernel values of single pairs to the fp64 formula): an IEEE square root and a division or two were half of the
+// instructions of the pair-scalar stage of the sweeps over neighbour lists.
+struct Spiky {
+    float d, inv;  // distance and its reciprocal
+};
+__device__ inline Spiky spiky_distance(float q) {
+    const float Q = q + 1e-12f;
+    float y = rsqrtf(Q);
+    y = fmaf(0.5f * y, fmaf(-(Q * y), y, 1.0f), y);
+    const float d = Q * y;
+    return Spiky{fmaf(0.5f * y, fmaf(-d, d, Q), d), y};
 }
-__device__ inline float spiky_psi(float d, float h) {
+__device__ inline float spiky_phi(const Spiky &s, float h) {
+    const float t = fmaxf(h - s.d, 0.0f);
+    return 3.0f * t * t * s.inv;
+}
+__device__ inline float spiky_psi(const Spiky &s, float h) {
     // d(phi)/dd / d with phi = 3 max(h-d,0)^2 / d  ==  -3 (h - d)(h + d) / d^3
-    float t = fmaxf(h - d, 0.0f);
-    return 3.0f * t * (h + d) / (d * d * d);
+    const float t = fmaxf(h - s.d, 0.0f);
+    return 3.0f * t * (h + s.d) * (s.inv * s.inv * s.inv);
 }
-
 
 // Inverse of a symmetric DxD matrix given by its upper triangle m (row-major order of the
 // triangle), identity when |det| < tol: the rule of the reference's safe_inv_sym_mat

@@ -209,8 +209,8 @@ feature_forward_kernel(FeatureFwdArgs a, Geom g) {
                         wv = vj * (t * t * t);
                     }
                     if ((MASK & (F_GRAD | F_MOMENT)) && q > 0.f) {
-                        float dist;
-                        const float phi = spiky_phi(q, g.h, dist);
+                        const Spiky sp = spiky_distance(q);
+                        const float phi = spiky_phi(sp, g.h);
                         kv = vj * phi;
                         if ((MASK & F_PACK) && a.rho_grad_out && fbase == 0) {  // the density gradient's pair term: m_j phi r
                             const float w = mj * phi;
@@ -509,9 +509,9 @@ feature_backward_kernel(FeatureBwdArgs a, Geom g) {
                     const float t = fmaxf(g.h2 - q, 0.f);
                     float phi = 0.f, psi = 0.f;
                     if ((MASK & F_GRAD) && q > 0.f) {
-                        float dist;
-                        phi = spiky_phi(q, g.h, dist);
-                        if (FULL) psi = spiky_psi(dist, g.h);
+                        const Spiky sp = spiky_distance(q);
+                        phi = spiky_phi(sp, g.h);
+                        if (FULL) psi = spiky_psi(sp, g.h);
                     }
                     ker[e] = make_float4(t * t * t, 6.0f * t * t, phi, psi);
                     vol[e] = mj / __ldg(a.rho + j);

@@ -9,26 +9,31 @@
 // features and nothing is combined.  32 / LPP particles advance together through chunks of CH list
 // entries:
 //   stage B  every lane turns one (LPP = 4: two) list entries of its particle into pair scalars and leaves
-//            them in the warp's shared memory, already duplicated for the packed arithmetic; the entries of
-//            the next chunk are on their way meanwhile;
-//   stage C  the lanes of a sub-group walk the chunk's entries: four neighbour rows are fetched at a time
+//            them in the warp's shared memory; list entries are loaded two chunks ahead, particles one;
+//   stage C  the lanes of a sub-group walk the chunk's entries: neighbour rows are fetched a few at a time
 //            (128-bit loads, one line per sub-group) and multiplied in with fma.rn.f32x2.
 // The price is imbalance: a warp runs as long as the longest of its lists (neighbouring particles, ~16 %
 // over the mean for four lists of ~41).  Work items, tickets and cell ranges are not needed; blocks are
 // plain blocks over consecutive particles, which lie in consecutive cells.
 // A particle whose list overflowed (count -1) is searched by its sub-group's lanes over the cells around
-// its position, LPP candidates a round, in the same warp.
+// its position, LPP candidates a round, out of line so that the walk over lists keeps its registers.
 //
-// What bounds them: instruction issue and the L1 data path (one 128-byte line per pair and row).  Measured,
-// B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us before -> now: blur + gradient 328 -> FWD_PLAIN,
-// packed perception 495 -> FWD_PACK, features-only backward 499 -> BWD_FEAT, full backward 902 -> BWD_FULL.
+// What bounds them: the L1 data path.  A 128-byte row of a neighbour is one wavefront, but so are every four
+// bytes per lane of shared memory, broadcast or not: with the scalars stored twice for the packed arithmetic
+// (32 bytes per pair) the forward took 231 us instead of 194.  Then latency: 16-24 warps per SM are resident, a third
+// of the row sectors come from L2 (prefetching rows into L1 a chunk ahead was slower, 330 -> 340 us; one register
+// set per row refilled early cost spills, 194 -> 234 us; five CTAs of the full backward instead of four 664 -> 758 us).
+// Measured, B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us, kernel with the whole warp per particle
+// -> this one: blur + gradient 328 -> 182 (with the density gradient), packed perception 495 -> 275,
+// features-only backward 499 -> 396, full backward 902 -> 664.
 #pragma once
 #include "neighbors.cuh"
 #include "ops.cuh"
 
 namespace npa {
 
-constexpr int kListWarps = 8;  // warps per CTA
+constexpr int kListWarps = 8;      // warps per CTA
+constexpr int kListFullWarps = 4;  // same, backward with position gradients
 
 // (x, y, z, m_j / rho_j) of particle j: one 16-byte gather when the density sweep left it packed.
 template <int D>
@@ -102,33 +107,40 @@ __device__ inline int compact_slot(bool acc, int sg, int sl, int &m) {
     return acc ? __popc(bits & below) : m + __popc(~bits & below);
 }
 
-template <int D> struct TailWeights { using type = float4; };  // (Kz, Kz, W, W)
-template <> struct TailWeights<2> { using type = float2; };    // (W, W)
+// Shared memory of one warp: the entries of two chunks per sub-group (one entry of padding keeps the sub-groups'
+// broadcasts on different banks).
+template <int LPP>
+struct ListShape {
+    static constexpr int EPL = LPP == 4 ? 2 : 1;  // list entries per lane and chunk
+    static constexpr int CH = LPP * EPL, PP = 32 / LPP;
+    static constexpr int kSlots = PP * (CH + 1), kIndexQuads = PP * (CH / 4 + 1);
+};
 
-template <int D, bool PER, int LPP, bool VEC, int MASK>
-__global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 3)
-feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
-    constexpr int EPL = LPP == 4 ? 2 : 1;  // list entries per lane and chunk
-    constexpr int CH = LPP * EPL, PP = 32 / LPP;
-    using KB = typename TailWeights<D>::type;
-    // one entry of padding per sub-group keeps the sub-groups' broadcasts on different banks
-    __shared__ float4 s_ka[kListWarps][2][PP * (CH + 1)];  // K.x K.x K.y K.y, all times v_j
-    __shared__ KB s_kb[kListWarps][2][PP * (CH + 1)];      // [K.z K.z] W W
-    __shared__ int4 s_j[kListWarps][2][PP * (CH / 4 + 1)];
-    extern __shared__ float4 s_dyn[];                      // F_PACK: the rows of z of a warp's particles
+// Starts the head of a particle's list (256 bytes) on its way into L1 while its count is still awaited.
+template <int LPP>
+__device__ inline int list_count(const int32_t *list, int stride, bool valid, int sl) {
+    for (int q = sl; q < 8; q += LPP)
+        if (q * 8 < stride) asm volatile("prefetch.global.L1 [%0];" ::"l"(list + q * 8));
+    return valid ? __ldg(list) : 0;
+}
 
+// The particles first .. first + PP - 1 of a warp: those with a list (SEARCH false) or those whose list overflowed.
+template <int D, bool PER, int LPP, bool VEC, int MASK, bool SEARCH>
+__device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
+                                             int4 (*s_j)[ListShape<LPP>::kIndexQuads], float *stage) {
+    constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
     const int first = (blockIdx.x * kListWarps + warp) * PP;
-    if (first >= total) return;
-    const bool ivalid = first + sg < total;
+    bool ivalid = first + sg < total;
     const int i = ivalid ? first + sg : total - 1;
-    const Pos<D> pi = load_pos<D>(a.x, i);
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
-    const int count = ivalid ? __ldg(list) : 0;
+    const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
+    const Pos<D> pi = load_pos<D>(a.x, i);
     ++list;
-    const int n = max(count, 0);
-    const int nmax = __reduce_max_sync(kFull, n);
+    const int n = SEARCH ? 0 : max(count, 0);
+    const int nmax = SEARCH ? 0 : __reduce_max_sync(kFull, n);
+    ivalid = ivalid && (count < 0) == SEARCH;
     const unsigned pitch = (unsigned)C * 4u;
     constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
     constexpr bool kMoment = (MASK & F_MOMENT) != 0;
@@ -159,8 +171,8 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
                 w = vj * (t * t * t);
             }
             if ((kGrad || kMoment || kDg) && q > 0.f) {
-                float dist;
-                const float phi = spiky_phi(q, g.h, dist);
+                const Spiky sp = spiky_distance(q);
+                const float phi = spiky_phi(sp, g.h);
                 kv = vj * phi;
                 if (kDg) {
                     const float md = mj * phi;
@@ -182,16 +194,13 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
                 }
             }
             const float kx = kv * rx, ky = kv * ry, kz = kv * rz;
-            if (kGrad) s_ka[warp][buf][sg * (CH + 1) + slot] = make_float4(kx, kx, ky, ky);
-            if constexpr (D == 3) s_kb[warp][buf][sg * (CH + 1) + slot] = make_float4(kz, kz, w, w);
-            else s_kb[warp][buf][sg * (CH + 1) + slot] = make_float2(w, w);
-            reinterpret_cast<int *>(&s_j[warp][buf][sg * (CH / 4 + 1)])[slot] = j;
+            s_k[buf][sg * (CH + 1) + slot] = make_float4(kx, ky, kz, w);
+            reinterpret_cast<int *>(&s_j[buf][sg * (CH / 4 + 1)])[slot] = j;
         };
         // the first m entries of a buffer (m uniform; slots up to the next multiple of four are filled)
         auto drain = [&](int buf, int m) {
-            const float4 *ka = &s_ka[warp][buf][sg * (CH + 1)];
-            const KB *kb = &s_kb[warp][buf][sg * (CH + 1)];
-            const int4 *jj = &s_j[warp][buf][sg * (CH / 4 + 1)];
+            const float4 *ks = &s_k[buf][sg * (CH + 1)];
+            const int4 *jj = &s_j[buf][sg * (CH / 4 + 1)];
 #pragma unroll
             for (int e0 = 0; e0 < CH; e0 += 4) {
                 if (e0 >= m) break;
@@ -205,71 +214,70 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
                     const unsigned long long s01 = pack2(r[u][0], r[u][1]), s23 = pack2(r[u][2], r[u][3]);
-                    const KB b = kb[e0 + u];
+                    const float4 k4 = ks[e0 + u];
                     if (kBlur) {
-                        unsigned long long ww;
-                        if constexpr (D == 3) ww = pack2(b.z, b.w);
-                        else ww = pack2(b.x, b.y);
+                        const unsigned long long ww = pack2(k4.w, k4.w);
                         acc[0] = fma2(ww, s01, acc[0]);
                         acc[1] = fma2(ww, s23, acc[1]);
                     }
                     if (kGrad) {
-                        const float4 k4 = ka[e0 + u];
                         const unsigned long long d01 = add2(s01, nsi01), d23 = add2(s23, nsi23);  // s_j - s_i
-                        const unsigned long long kx = pack2(k4.x, k4.y), ky = pack2(k4.z, k4.w);
-                        acc[2] = fma2(d01, kx, acc[2]);
-                        acc[3] = fma2(d23, kx, acc[3]);
-                        acc[4] = fma2(d01, ky, acc[4]);
-                        acc[5] = fma2(d23, ky, acc[5]);
-                        if constexpr (D == 3) {
-                            const unsigned long long kz = pack2(b.x, b.y);
-                            acc[6] = fma2(d01, kz, acc[6]);
-                            acc[7] = fma2(d23, kz, acc[7]);
+                        const float kd[3] = {k4.x, k4.y, k4.z};
+#pragma unroll
+                        for (int d = 0; d < D; ++d) {
+                            const unsigned long long kk = pack2(kd[d], kd[d]);
+                            acc[2 + 2 * d] = fma2(d01, kk, acc[2 + 2 * d]);
+                            acc[3 + 2 * d] = fma2(d23, kk, acc[3 + 2 * d]);
                         }
                     }
                 }
             }
         };
 
-        // ---- the listed pairs
-        int jn[EPL];
-        float4 pj[EPL];
-        float mj[EPL];
-        auto indices = [&](int c) {
-#pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                const int e = c + k * LPP + sl;
-                jn[k] = e < n ? __ldg(list + e) : -1;
-            }
-        };
-        auto particles = [&]() {
-#pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                const int j = jn[k] >= 0 ? jn[k] : i;
-                pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, j);
-                mj[k] = kDg ? (a.mass ? __ldg(a.mass + j) : 1.0f) : 0.f;
-                if (jn[k] < 0) { pj[k].w = 0.f; mj[k] = 0.f; }
-            }
-        };
         int buf = 0;
-        indices(0);
-        particles();
-        for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+        if constexpr (!SEARCH) {
+            // indices are loaded two chunks ahead and particles one, so that neither waits for the other's latency
+            int jn[EPL], ja[EPL];
+            float4 pj[EPL];
+            float mj[EPL];
+            auto indices = [&](int c) {
 #pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                float rx, ry, rz;
-                listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
-                put(buf, k * LPP + sl, k, rx, ry, rz, pj[k].w, mj[k], jn[k] >= 0 ? jn[k] : i);
+                for (int k = 0; k < EPL; ++k) {
+                    const int e = c + k * LPP + sl;
+                    ja[k] = e < n ? __ldg(list + e) : -1;
+                }
+            };
+            auto particles = [&]() {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) {
+                    const int j = jn[k] >= 0 ? jn[k] : i;
+                    pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, j);
+                    mj[k] = kDg ? (a.mass ? __ldg(a.mass + j) : 1.0f) : 0.f;
+                    if (jn[k] < 0) { pj[k].w = 0.f; mj[k] = 0.f; }
+                }
+            };
+            auto advance = [&](int c) {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) jn[k] = ja[k];
+                indices(c);
+                particles();
+            };
+            indices(0);
+            advance(CH);
+            for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) {
+                    float rx, ry, rz;
+                    listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
+                    put(buf, k * LPP + sl, k, rx, ry, rz, pj[k].w, mj[k], jn[k] >= 0 ? jn[k] : i);
+                }
+                __syncwarp();
+                advance(c + 2 * CH);
+                drain(buf, nmax - c);
             }
-            indices(c + CH);
-            __syncwarp();
-            particles();
-            drain(buf, nmax - c);
         }
-
-        // ---- particles without a list
-        bool over = count < 0;
-        if (__any_sync(kFull, over)) {
+        if constexpr (SEARCH) {
+            bool over = ivalid;
             SubgroupSearch<D, PER, LPP> search;
             if (over) search.begin(g, a.bin_offsets, i, pi);
             while (true) {
@@ -375,7 +383,6 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
         if (MASK & F_PACK) {
             // the rows of z of the warp's particles are contiguous: assembled in shared memory, written as one run
             const int Z = a.zstride;
-            float *stage = reinterpret_cast<float *>(s_dyn) + (size_t)warp * ((PP * Z + 3) & ~3);
             float *zs = stage + sg * Z;
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
@@ -400,6 +407,12 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
                 for (int d = 0; d < D; ++d) zs[2 * C + C * D + d] = w[d];
             }
             __syncwarp();
+            if (SEARCH) {
+                if (ivalid)
+                    for (int q = sl; q < Z; q += LPP) a.z[(long long)i * Z + q] = zs[q];
+                return;
+            }
+            // (rows of particles without a list are written again by the search that follows)
             const int floats = min(PP, total - first) * Z;
             float *out = a.z + (long long)first * Z;
             if (PP % 4 == 0) {  // first is a multiple of four rows: 16-byte aligned
@@ -413,6 +426,30 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
     }
 }
 
+// Out of line, so that the search does not cost the walk over lists registers.
+template <int D, bool PER, int LPP, bool VEC, int MASK>
+__device__ __noinline__ void list_forward_search(const FeatureFwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
+                                                 int4 (*s_j)[ListShape<LPP>::kIndexQuads], float *stage) {
+    list_forward<D, PER, LPP, VEC, MASK, true>(a, g, s_k, s_j, stage);
+}
+
+template <int D, bool PER, int LPP, bool VEC, int MASK>
+__global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 3)
+feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
+    using S = ListShape<LPP>;
+    __shared__ float4 s_k[kListWarps][2][S::kSlots];  // v_j (K.x, K.y, K.z, W)
+    __shared__ int4 s_j[kListWarps][2][S::kIndexQuads];
+    extern __shared__ float4 s_dyn[];                 // F_PACK: the rows of z of a warp's particles
+    const int warp = threadIdx.x >> 5, total = g.B * g.N, first = (blockIdx.x * kListWarps + warp) * S::PP;
+    if (first >= total) return;
+    float *stage = reinterpret_cast<float *>(s_dyn) + ((MASK & F_PACK) ? (size_t)warp * ((S::PP * a.zstride + 3) & ~3) : 0);
+    list_forward<D, PER, LPP, VEC, MASK, false>(a, g, s_k[warp], s_j[warp], stage);
+    __syncwarp();
+    const int i = min(first + (int)(threadIdx.x & 31) / LPP, total - 1);
+    if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
+        list_forward_search<D, PER, LPP, VEC, MASK>(a, g, s_k[warp], s_j[warp], stage);
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // Backward.  The upstream of the gradient comes with the axis in front of the features ([N, D, C], rows
 // padded to a multiple of four; upstream_rows_kernel or the packed perception's own epilogue write it so),
@@ -424,30 +461,23 @@ feature_list_forward_kernel(FeatureFwdArgs a, Geom g) {
 // Sums over features stay lane-partial (packed pairs) until the particle is done.  The density gradient's own
 // backward, dx_i += sum_j J (m_i g_j - m_j g_i), uses the same pair scalars and rides stage B.
 // ---------------------------------------------------------------------------------------------------------
-template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
-__global__ void __launch_bounds__(FULL ? 128 : kListWarps * 32, FULL ? 4 : 3)
-feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
-    constexpr int EPL = LPP == 4 ? 2 : 1;
-    constexpr int CH = LPP * EPL, PP = 32 / LPP, WARPS = FULL ? 4 : kListWarps;
-    __shared__ float4 s_ka[WARPS][2][PP * (CH + 1)];                // -K.x -K.x -K.y -K.y
-    __shared__ float4 s_kb[WARPS][2][PP * (CH + 1)];                // -K.z -K.z W W
-    __shared__ float4 s_kc[FULL ? WARPS : 1][2][PP * (CH + 1)];     // r.x r.y r.z phi
-    __shared__ float4 s_kd[FULL ? WARPS : 1][2][PP * (CH + 1)];     // v_j v_j E psi
-    __shared__ int4 s_j[WARPS][2][PP * (CH / 4 + 1)];
+template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL, bool SEARCH>
+__device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
+                                              float4 (*s_e)[ListShape<LPP>::kSlots], int4 (*s_j)[ListShape<LPP>::kIndexQuads]) {
+    constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP, WARPS = FULL ? kListFullWarps : kListWarps;
     constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
-
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
     const int first = (blockIdx.x * WARPS + warp) * PP;
-    if (first >= total) return;
-    const bool ivalid = first + sg < total;
+    bool ivalid = first + sg < total;
     const int i = ivalid ? first + sg : total - 1;
-    const Pos<D> pi = load_pos<D>(a.x, i);
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
-    const int count = ivalid ? __ldg(list) : 0;
+    const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
+    const Pos<D> pi = load_pos<D>(a.x, i);
     ++list;
-    const int n = max(count, 0);
-    const int nmax = __reduce_max_sync(kFull, n);
+    const int n = SEARCH ? 0 : max(count, 0);
+    const int nmax = SEARCH ? 0 : __reduce_max_sync(kFull, n);
+    ivalid = ivalid && (count < 0) == SEARCH;
     const float mi = a.mass ? __ldg(a.mass + i) : 1.0f;
     const float rhoi = __ldg(a.rho + i);
     const float vi = mi / rhoi;
@@ -503,20 +533,18 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
             const float w = pair ? g.c_s * (t * t * t) : 0.f;
             float phi = 0.f, psi = 0.f;
             if ((kGrad || (FULL && a.g_dg)) && q > 0.f) {
-                float dist;
-                phi = g.c_g * spiky_phi(q, g.h, dist);
-                if (FULL) psi = g.c_g * spiky_psi(dist, g.h);
+                const Spiky sp = spiky_distance(q);
+                phi = g.c_g * spiky_phi(sp, g.h);
+                if (FULL) psi = g.c_g * spiky_psi(sp, g.h);
             }
             const float kx = phi * rx, ky = phi * ry, kz = phi * rz;
             tsum[0] = fmaf(vj, kx, tsum[0]);
             tsum[1] = fmaf(vj, ky, tsum[1]);
             if (D == 3) tsum[2] = fmaf(vj, kz, tsum[2]);
             const int at = sg * (CH + 1) + slot;
-            if (kGrad) s_ka[warp][buf][at] = make_float4(-kx, -kx, -ky, -ky);
-            s_kb[warp][buf][at] = make_float4(-kz, -kz, w, w);
+            s_k[buf][at] = FULL ? make_float4(rx, ry, rz, w) : make_float4(-kx, -ky, -kz, w);
             if (FULL) {
-                s_kc[warp][buf][at] = make_float4(rx, ry, rz, phi);
-                s_kd[warp][buf][at] = make_float4(vj, vj, pair ? g.c_s * 6.0f * t * t : 0.f, psi);
+                s_e[buf][at] = make_float4(phi, psi, vj, pair ? g.c_s * 6.0f * t * t : 0.f);
                 if (a.g_dg && fbase == 0 && q > 0.f) {
                     const float mj = a.mass ? __ldg(a.mass + j) : 1.0f;
                     const float rv[3] = {rx, ry, rz};
@@ -531,7 +559,7 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
                     for (int d = 0; d < D; ++d) dxd[d] += phi * u[d] - sc * rv[d];
                 }
             }
-            reinterpret_cast<int *>(&s_j[warp][buf][sg * (CH / 4 + 1)])[slot] = j;
+            reinterpret_cast<int *>(&s_j[buf][sg * (CH / 4 + 1)])[slot] = j;
         };
 
         struct Rows { float s[4], b[4], g[D][4]; };
@@ -552,37 +580,36 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
         };
         auto add = [&](int buf, int e, const Rows &r) {
             const int at = sg * (CH + 1) + e;
-            const float4 kb = s_kb[warp][buf][at];
+            const float4 ke = s_k[buf][at];
+            const float4 ex = FULL ? s_e[buf][at] : make_float4(-1.f, 0.f, 0.f, 0.f);
+            const unsigned long long w = pack2(ke.w, ke.w);
             unsigned long long b01, b23, k[D];
             if (kBlur) {
                 b01 = pack2(r.b[0], r.b[1]); b23 = pack2(r.b[2], r.b[3]);
-                const unsigned long long w = pack2(kb.z, kb.w);
                 ds[0] = fma2(w, b01, ds[0]);
                 ds[1] = fma2(w, b23, ds[1]);
             }
             if (kGrad) {
-                const float4 ka = s_ka[warp][buf][at];
-                k[0] = pack2(ka.x, ka.y);
-                k[1] = pack2(ka.z, ka.w);
-                if (D == 3) k[D - 1] = pack2(kb.x, kb.y);
+                const float kv[3] = {ke.x, ke.y, ke.z};
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
+                    const float m = FULL ? -(ex.x * kv[d]) : kv[d];  // -K
+                    k[d] = pack2(m, m);
                     ds[0] = fma2(k[d], pack2(r.g[d][0], r.g[d][1]), ds[0]);
                     ds[1] = fma2(k[d], pack2(r.g[d][2], r.g[d][3]), ds[1]);
                 }
             }
             if (FULL) {
-                const float4 kc = s_kc[warp][buf][at], kd = s_kd[warp][buf][at];
-                const unsigned long long s01 = pack2(r.s[0], r.s[1]), s23 = pack2(r.s[2], r.s[3]), vj = pack2(kd.x, kd.y);
-                const float rv[3] = {kc.x, kc.y, kc.z};
+                const unsigned long long s01 = pack2(r.s[0], r.s[1]), s23 = pack2(r.s[2], r.s[3]), vj = pack2(ex.z, ex.z);
+                const float rv[3] = {ke.x, ke.y, ke.z};
                 float coef = 0.f;
                 if (kBlur) {
                     const unsigned long long A = fma2(gbi[1], s23, mul2(gbi[0], s01));
                     const unsigned long long Bp = fma2(svi[1], b23, mul2(svi[0], b01));
                     float lo, hi;
                     unpack2(fma2(vj, A, Bp), lo, hi);
-                    coef = kd.z * (lo + hi);
-                    drp = fma2(pack2(kb.z, kb.w), Bp, drp);
+                    coef = ex.w * (lo + hi);
+                    drp = fma2(w, Bp, drp);
                 }
                 if (kGrad) {
                     const unsigned long long e01 = fma2(s01, minus1, si[0]), e23 = fma2(s23, minus1, si[1]);  // s_i - s_j
@@ -599,22 +626,21 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
                     }
                     float ru = rv[0] * u[0] + rv[1] * u[1];
                     if (D == 3) ru = fmaf(rv[2], u[2], ru);
-                    coef = fmaf(-kd.w, ru, coef);
+                    coef = fmaf(-ex.y, ru, coef);
 #pragma unroll
-                    for (int d = 0; d < D; ++d) dx[d] = fmaf(kc.w, u[d], dx[d]);
+                    for (int d = 0; d < D; ++d) dx[d] = fmaf(ex.x, u[d], dx[d]);
                 }
 #pragma unroll
                 for (int d = 0; d < D; ++d) dx[d] = fmaf(coef, rv[d], dx[d]);
             }
         };
         auto drain = [&](int buf, int m) {
-            const int4 *jj = &s_j[warp][buf][sg * (CH / 4 + 1)];
+            const int4 *jj = &s_j[buf][sg * (CH / 4 + 1)];
 #pragma unroll
             for (int e0 = 0; e0 < CH; e0 += 4) {
                 if (e0 >= m) break;
                 const int4 j4 = jj[e0 / 4];
-                // two pairs in flight
-                Rows r0, r1;
+                Rows r0, r1;  // two pairs in flight
                 load(j4.x, r0);
                 load(j4.y, r1);
                 add(buf, e0, r0);
@@ -626,40 +652,47 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
             }
         };
 
-        int jn[EPL];
-        float4 pj[EPL];
-        auto indices = [&](int c) {
-#pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                const int e = c + k * LPP + sl;
-                jn[k] = e < n ? __ldg(list + e) : -1;
-            }
-        };
-        auto particles = [&]() {
-#pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, jn[k] >= 0 ? jn[k] : i);
-                if (jn[k] < 0) pj[k].w = 0.f;
-            }
-        };
         int buf = 0;
-        indices(0);
-        particles();
-        for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+        if constexpr (!SEARCH) {
+            // indices are loaded two chunks ahead and particles one, so that neither waits for the other's latency
+            int jn[EPL], ja[EPL];
+            float4 pj[EPL];
+            auto indices = [&](int c) {
 #pragma unroll
-            for (int k = 0; k < EPL; ++k) {
-                float rx, ry, rz;
-                listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
-                put(buf, k * LPP + sl, rx, ry, rz, pj[k].w, jn[k] >= 0 ? jn[k] : i);
+                for (int k = 0; k < EPL; ++k) {
+                    const int e = c + k * LPP + sl;
+                    ja[k] = e < n ? __ldg(list + e) : -1;
+                }
+            };
+            auto particles = [&]() {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) {
+                    pj[k] = fetch_particle<D>(a.x, a.pv, a.rho, a.mass, jn[k] >= 0 ? jn[k] : i);
+                    if (jn[k] < 0) pj[k].w = 0.f;
+                }
+            };
+            auto advance = [&](int c) {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) jn[k] = ja[k];
+                indices(c);
+                particles();
+            };
+            indices(0);
+            advance(CH);
+            for (int c = 0; c < nmax; c += CH, buf ^= 1) {
+#pragma unroll
+                for (int k = 0; k < EPL; ++k) {
+                    float rx, ry, rz;
+                    listed_displacement<D, PER>(g, pi, Pos<D>{pj[k].x, pj[k].y, pj[k].z}, rx, ry, rz);
+                    put(buf, k * LPP + sl, rx, ry, rz, pj[k].w, jn[k] >= 0 ? jn[k] : i);
+                }
+                __syncwarp();
+                advance(c + 2 * CH);
+                drain(buf, nmax - c);
             }
-            indices(c + CH);
-            __syncwarp();
-            particles();
-            drain(buf, nmax - c);
         }
-
-        bool over = count < 0;
-        if (__any_sync(kFull, over)) {
+        if constexpr (SEARCH) {
+            bool over = ivalid;
             SubgroupSearch<D, PER, LPP> search;
             if (over) search.begin(g, a.bin_offsets, i, pi);
             while (true) {
@@ -731,6 +764,29 @@ feature_list_backward_kernel(FeatureListBwdArgs a, Geom g) {
     }
 }
 
+template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
+__device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
+                                                  float4 (*s_e)[ListShape<LPP>::kSlots], int4 (*s_j)[ListShape<LPP>::kIndexQuads]) {
+    list_backward<D, PER, LPP, VEC, MASK, FULL, true>(a, g, s_k, s_e, s_j);
+}
+
+template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
+__global__ void __launch_bounds__(FULL ? kListFullWarps * 32 : kListWarps * 32, FULL ? 4 : 3)
+feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
+    using S = ListShape<LPP>;
+    constexpr int WARPS = FULL ? kListFullWarps : kListWarps;
+    __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z W
+    __shared__ float4 s_e[FULL ? WARPS : 1][2][S::kSlots];  // FULL: phi psi v_j E
+    __shared__ int4 s_j[WARPS][2][S::kIndexQuads];
+    const int warp = threadIdx.x >> 5, total = g.B * g.N, first = (blockIdx.x * WARPS + warp) * S::PP;
+    if (first >= total) return;
+    list_backward<D, PER, LPP, VEC, MASK, FULL, false>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
+    __syncwarp();
+    const int i = min(first + (int)(threadIdx.x & 31) / LPP, total - 1);
+    if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
+        list_backward_search<D, PER, LPP, VEC, MASK, FULL>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
+}
+
 // ---------------------------------------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------------------------------------
@@ -790,7 +846,7 @@ int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdAr
 
 template <int D, bool PER, int LPP, bool VEC, bool FULL>
 int launch_list_backward_mask(const Geom &g, int mask, const FeatureListBwdArgs &a, cudaStream_t st) {
-    constexpr int PP = 32 / LPP, WARPS = FULL ? 4 : kListWarps;
+    constexpr int PP = 32 / LPP, WARPS = FULL ? kListFullWarps : kListWarps;
     const long long particles = (long long)g.B * g.N, per_cta = (long long)WARPS * PP;
     const unsigned blocks = (unsigned)((particles + per_cta - 1) / per_cta);
     switch (mask) {

@@ -175,8 +175,8 @@ feature_tile_forward_kernel(FeatureFwdArgs a, Geom g, TileLayout L, unsigned int
                             wv = vj * (t * t * t);
                         }
                         if ((MASK & (F_GRAD | F_MOMENT)) && q > 0.f) {
-                            float dist;
-                            kv = vj * spiky_phi(q, g.h, dist);
+                            const Spiky sp = spiky_distance(q);
+                            kv = vj * spiky_phi(sp, g.h);
                         }
                         if (MASK & F_MOMENT) {
                             mom[0] = fmaf(kv * ge.x, ge.x, mom[0]);
@@ -459,9 +459,9 @@ feature_tile_backward_kernel(FeatureBwdArgs a, Geom g, TileLayout L, unsigned in
                         const float t = fmaxf(g.h2 - q, 0.f);
                         float phi = 0.f, psi = 0.f;
                         if ((MASK & F_GRAD) && q > 0.f) {
-                            float dist;
-                            phi = spiky_phi(q, g.h, dist);
-                            if (FULL) psi = spiky_psi(dist, g.h);
+                            const Spiky sp = spiky_distance(q);
+                            phi = spiky_phi(sp, g.h);
+                            if (FULL) psi = spiky_psi(sp, g.h);
                         }
                         const float t2 = ratio * t * t;
                         ker[e] = make_float4(t2 * t, 6.0f * t2, phi, psi);

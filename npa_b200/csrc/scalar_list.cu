@@ -51,8 +51,8 @@ scalar_list_backward_kernel(ScalarListArgs a, Geom g) {
             for (int d = 0; d < D; ++d) dxs[d] = fmaf(w, rv[d], dxs[d]);
         }
         if (MASK & S_DGRAD) {
-            float dist;
-            const float phi = spiky_phi(q, g.h, dist), psi = spiky_psi(dist, g.h);
+            const Spiky sp = spiky_distance(q);
+            const float phi = spiky_phi(sp, g.h), psi = spiky_psi(sp, g.h);
             float u[3] = {0.f, 0.f, 0.f}, ru = 0.f;
 #pragma unroll
             for (int d = 0; d < D; ++d) {
@@ -161,8 +161,8 @@ density_gradient_list_kernel(ScalarListArgs a, Geom g) {
     auto visit = [&](int j, float rx, float ry, float rz) {
         const float q = sq_norm_fast<D>(rx, ry, rz);
         if (!(q > 0.f)) return;
-        float dist;
-        const float md = (a.mass ? __ldg(a.mass + j) : 1.0f) * spiky_phi(q, g.h, dist);
+        const Spiky sp = spiky_distance(q);
+        const float md = (a.mass ? __ldg(a.mass + j) : 1.0f) * spiky_phi(sp, g.h);
         dg[0] = fmaf(md, rx, dg[0]);
         dg[1] = fmaf(md, ry, dg[1]);
         if (D == 3) dg[2] = fmaf(md, rz, dg[2]);

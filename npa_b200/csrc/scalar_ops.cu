@@ -91,8 +91,8 @@ scalar_forward_kernel(ScalarFwdArgs a, Geom g) {
                         rho = fmaf(mj, t * t * t, rho);
                     }
                     if (kSpiky && q > 0.f) {
-                        float d;
-                        const float phi = spiky_phi(q, g.h, d);
+                        const Spiky sp = spiky_distance(q);
+                        const float phi = spiky_phi(sp, g.h);
                         if (MASK & S_DGRAD) {
                             const float w = mj * phi;
                             dg[0] = fmaf(w, rx, dg[0]);
@@ -316,8 +316,8 @@ scalar_forward_shared_kernel(ScalarFwdArgs a, Geom g, int span, int batch) {
                                 rho = fmaf(c.w, t * t * t, rho);
                             }
                             if (kSpiky) {
-                                float d;
-                                const float phi = acc ? spiky_phi(q, g.h, d) : 0.f;  // phi r = 0 for the self pair
+                                const Spiky sp = spiky_distance(q);
+                                const float phi = acc ? spiky_phi(sp, g.h) : 0.f;  // phi r = 0 for the self pair
                                 if (MASK & S_DGRAD) {
                                     const float w = c.w * phi;
                                     dg[0] = fmaf(w, rx, dg[0]);
@@ -440,9 +440,9 @@ scalar_backward_kernel(ScalarBwdArgs a, Geom g) {
                     for (int d = 0; d < D; ++d) dxs[d] = fmaf(w, rv[d], dxs[d]);
                 }
                 if (kSpiky) {
-                    float dist;
-                    const float phi = spiky_phi(q, g.h, dist);
-                    const float psi = spiky_psi(dist, g.h);
+                    const Spiky sp = spiky_distance(q);
+                    const float phi = spiky_phi(sp, g.h);
+                    const float psi = spiky_psi(sp, g.h);
                     if (MASK & S_DGRAD) {
                         float u[3] = {0.f, 0.f, 0.f}, o[3];
 #pragma unroll
