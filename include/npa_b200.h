@@ -425,6 +425,15 @@ int npa_step_update_forward(const npa_grid *g, const float *y, const float *x_bi
                             const float *mask, int32_t channels, float alpha, float dt, int32_t wrap,
                             float *x_out, float *s_out, void *stream);
 
+/* The same with the update mask given as uniforms: a particle is updated where mask[i] < update_below (models/npa.py:189-191
+ * draws the uniforms and compares); likewise the backward. */
+int npa_step_update_forward_masked(const npa_grid *g, const float *y, const float *x_bin, const float *s_bin,
+                                   const float *uniforms, float update_below, int32_t channels, float alpha, float dt,
+                                   int32_t wrap, float *x_out, float *s_out, void *stream);
+int npa_step_update_backward_masked(const npa_grid *g, const float *y, const float *uniforms, float update_below,
+                                    int32_t channels, float alpha, float dt, const float *g_x_out, const float *g_s_out,
+                                    float *g_y, void *stream);
+
 /* dL/dy [B,N,D+C] from the upstream gradients of x_out [B,N,P] and s_out [B,N,C] (either
  * may be NULL = zero).  The gradients with respect to x_bin and s_bin are the upstream
  * gradients themselves and need no kernel. */
@@ -530,6 +539,15 @@ int npa_mlp_forward_tcgen05(const float *z, const float *W1, const float *b1, co
                             int64_t rows, int32_t in_dim, int32_t out_dim, int64_t w1_stride_out,
                             int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,
                             int64_t scratch_bytes, void *stream);
+/* The same with h == NULL allowed (the hidden layer is not stored: inference), and with the image of W1 that the
+ * backward's dz = dh W1 wants made in the same launch: dz_image holds npa_linear_tcgen05_scratch_bytes(128, in_dim)
+ * bytes, 16-byte aligned, or is NULL.  npa_linear_tcgen05_prepared is npa_linear_tcgen05 on such an image, without bias. */
+int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float *b1, const float *W2, float *h, float *y,
+                                   int64_t rows, int32_t in_dim, int32_t out_dim, int64_t w1_stride_out,
+                                   int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,
+                                   int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, void *stream);
+int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image_bytes, float *C, int64_t rows,
+                                int32_t in_dim, int32_t out_dim, void *stream);
 /* Self-test of those bounded waits: a two-warp kernel in which warp 0 waits `limit_us` (1..1,000,000)
  * on an mbarrier that nothing completes, gives up and raises the kernel's leave flag, and warp 1,
  * waiting on a second such mbarrier with the full limit, leaves through the flag.  device_result[0]

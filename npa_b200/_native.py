@@ -103,6 +103,11 @@ SIGNATURES = {
     "npa_linear_tcgen05": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_int64, _I32, _I32, ctypes.c_int64, ctypes.c_int64,
                                           _I32, _P, ctypes.c_int64, _P]),
     "npa_mlp_forward_tcgen05": (ctypes.c_int, [_P] * 6 + [ctypes.c_int64, _I32, _I32] + [ctypes.c_int64] * 4 + [_P, ctypes.c_int64, _P]),
+    "npa_mlp_forward_tcgen05_images": (ctypes.c_int, [_P] * 6 + [ctypes.c_int64, _I32, _I32] + [ctypes.c_int64] * 4
+                                       + [_P, ctypes.c_int64, _P, ctypes.c_int64, _P]),
+    "npa_linear_tcgen05_prepared": (ctypes.c_int, [_P, _P, ctypes.c_int64, _P, ctypes.c_int64, _I32, _I32, _P]),
+    "npa_step_update_forward_masked": (ctypes.c_int, [_P] * 5 + [ctypes.c_float, _I32, ctypes.c_float, ctypes.c_float, _I32, _P, _P, _P]),
+    "npa_step_update_backward_masked": (ctypes.c_int, [_P] * 3 + [ctypes.c_float, _I32, ctypes.c_float, ctypes.c_float, _P, _P, _P, _P]),
     "npa_mlp_forward_tcgen05_scratch_bytes": (ctypes.c_int64, [_I32, _I32]),
     "npa_linear_tcgen05_scratch_bytes": (ctypes.c_int64, [_I32, _I32]),
     "npa_linear_tcgen05_status": (ctypes.c_int, [_P, _I32]),

@@ -13,7 +13,7 @@
 // All kernels are HBM-bound integer work; nothing here is GEMM shaped.
 #include <mutex>
 
-#include "common.cuh"
+#include "ops.cuh"
 
 namespace npa {
 
@@ -277,32 +277,14 @@ scatter_kernel(const uint32_t *__restrict__ cellid, const uint32_t *__restrict__
     order[(uint32_t)bin_offsets[cell] + arrive[idx]] = (uint32_t)i;  // no atomics: the slot was drawn in pass 1
 }
 
-__global__ void __launch_bounds__(kBinThreads)
-rank_kernel(const uint32_t *__restrict__ cellid, const int32_t *__restrict__ bin_offsets,
-            const uint32_t *__restrict__ order, int32_t *__restrict__ permutation, Geom g) {
-    const int b = blockIdx.y;
-    const int p = blockIdx.x * kBinThreads + threadIdx.x;
-    if (p >= g.N) return;
-    const size_t sys = (size_t)b * g.N;
-    const uint32_t i = order[sys + p];
-    const uint32_t key = cellid[sys + i];
-    const size_t cell = (size_t)b * g.cells + key;
-    const uint32_t s = (uint32_t)bin_offsets[cell], e = (uint32_t)bin_offsets[cell + 1];
-    if (e - s > (uint32_t)kCrowdedCell) return;  // ranked by rank_crowded_kernel
-    uint32_t rank = 0;
-    for (uint32_t q = s; q < e; ++q) rank += order[q] < i ? 1u : 0u;
-    permutation[sys + i] = (int32_t)(s - (uint32_t)sys + rank);
-}
-
 // Stable ranks inside crowded cells (a collapsed system, or particles clamped into an edge cell): a
 // CTA takes one crowded cell at a time, marks the original indices of its particles in a bitmap over
 // the system's particle indices (in windows of kRankWindow indices), turns the bitmap into prefix
 // popcounts, and a particle's rank is the number of marked indices below its own.  Linear in the
 // population plus N / 32 words per window; no sort, no atomics in global memory.
-__global__ void __launch_bounds__(256)
-rank_crowded_kernel(const int32_t *__restrict__ bin_offsets, const uint32_t *__restrict__ order,
-                    int32_t *__restrict__ permutation, const uint32_t *__restrict__ crowded,
-                    const uint32_t *__restrict__ crowded_count, Geom g) {
+__device__ inline void rank_crowded(const int32_t *__restrict__ bin_offsets, const uint32_t *__restrict__ order,
+                                    int32_t *__restrict__ permutation, const uint32_t *__restrict__ crowded,
+                                    const uint32_t *__restrict__ crowded_count, const Geom &g, uint32_t first, uint32_t stride) {
     extern __shared__ uint32_t rank_smem[];
     __shared__ uint32_t warp_tot[8];
     __shared__ uint32_t carry;
@@ -311,7 +293,7 @@ rank_crowded_kernel(const int32_t *__restrict__ bin_offsets, const uint32_t *__r
     uint32_t *bits = rank_smem, *pre = rank_smem + words;
     const uint32_t n = *crowded_count;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    for (uint32_t entry = blockIdx.x; entry < n; entry += gridDim.x) {
+    for (uint32_t entry = first; entry < n; entry += stride) {
         const uint32_t cell = crowded[entry];
         const uint32_t sys = (cell / (uint32_t)g.cells) * (uint32_t)g.N;
         const uint32_t s = (uint32_t)bin_offsets[cell], e = (uint32_t)bin_offsets[cell + 1];
@@ -356,6 +338,162 @@ rank_crowded_kernel(const int32_t *__restrict__ bin_offsets, const uint32_t *__r
             __syncthreads();
         }
     }
+}
+
+// The last kRankCtas columns of the grid take the crowded cells, the others a particle slot per thread.
+__global__ void __launch_bounds__(kBinThreads)
+rank_kernel(const uint32_t *__restrict__ cellid, const int32_t *__restrict__ bin_offsets, const uint32_t *__restrict__ order,
+            int32_t *__restrict__ permutation, const uint32_t *__restrict__ crowded, const uint32_t *__restrict__ crowded_count, Geom g,
+            int rank_columns) {
+    if ((int)blockIdx.x >= rank_columns) {
+        if (blockIdx.y == 0)
+            rank_crowded(bin_offsets, order, permutation, crowded, crowded_count, g, blockIdx.x - rank_columns, gridDim.x - rank_columns);
+        return;
+    }
+    const int b = blockIdx.y;
+    const int p = blockIdx.x * kBinThreads + threadIdx.x;
+    if (p >= g.N) return;
+    const size_t sys = (size_t)b * g.N;
+    const uint32_t i = order[sys + p];
+    const uint32_t key = cellid[sys + i];
+    const size_t cell = (size_t)b * g.cells + key;
+    const uint32_t s = (uint32_t)bin_offsets[cell], e = (uint32_t)bin_offsets[cell + 1];
+    if (e - s > (uint32_t)kCrowdedCell) return;  // ranked by the crowded-cell blocks
+    uint32_t rank = 0;
+    for (uint32_t q = s; q < e; ++q) rank += order[q] < i ? 1u : 0u;
+    permutation[sys + i] = (int32_t)(s - (uint32_t)sys + rank);
+}
+
+// ---------------------------------------------------------------------------
+// Small systems: everything but the work list in one launch, a CTA per system with the cell table, the cell ids and the
+// slots in shared memory.  The general path is seven dependent launches of 1.5-11 us each for 8 x 4,096 particles
+// (31 us, and a host that needs 35-40 us to issue them): what bounds it there is launch latency and the serial atomics
+// of few CTAs, not memory.  Measured with the work list's launch: BIN_SMALL.
+// ---------------------------------------------------------------------------
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallParticles = 16384;
+constexpr size_t kSmallSmem = 200 * 1024;
+
+// Place of a cell in the shared table: one word of padding per 32, so that threads that walk consecutive cells each do not
+// meet on one bank.
+__host__ __device__ inline int table_at(int c) { return c + (c >> 5); }
+
+static size_t small_smem(const Geom &g) {
+    return (size_t)(table_at(g.cells) + 1) * 4 + (size_t)((g.N + 1) & ~1) * 4 + (size_t)((g.N + 31) / 32) * 8;
+}
+static bool small_system(const Geom &g) { return g.N <= kSmallParticles && g.cells < 65536 && small_smem(g) <= kSmallSmem; }
+
+// Exclusive scan over the CTA's cell table: every thread takes `per` consecutive cells.  Calls emit(cell, count, prefix)
+// in cell order; returns the grand total.  prefix and total count (work items << 32 | particles).
+template <typename Count, typename Emit>
+__device__ inline unsigned long long scan_cells(const Geom &g, Count &&count, Emit &&emit) {
+    __shared__ unsigned long long tot;
+    const int per = (g.cells + kSmallThreads - 1) / kSmallThreads, c0 = threadIdx.x * per, c1 = min(c0 + per, g.cells);
+    unsigned long long v = 0;
+    for (int c = c0; c < c1; ++c) v += pack_cell(count(c), g.mpb);
+    unsigned long long run = block_exclusive<kSmallThreads>(v, tot);
+    for (int c = c0; c < c1; ++c) {
+        const uint32_t n = count(c);
+        emit(c, n, run);
+        run += pack_cell(n, g.mpb);
+    }
+    __syncthreads();
+    return tot;
+}
+
+// Rows of one system from its cell starts; row0 = rows of the systems before it.
+__device__ inline void write_rows(int4 *__restrict__ block_info, const Geom &g, int b, int cell, uint32_t n, uint32_t row) {
+    for (uint32_t off = 0; off < n; off += (uint32_t)g.mpb, ++row)
+        block_info[row] = make_int4(b * g.cells + cell, (int)off, (int)min((uint32_t)g.mpb, n - off), b);
+}
+
+template <int D>
+__global__ void __launch_bounds__(kSmallThreads)
+bin_small_kernel(const float *__restrict__ x, int32_t *__restrict__ permutation, int32_t *__restrict__ bin_offsets,
+                 int4 *__restrict__ block_info, uint32_t *__restrict__ rows_of_system, Geom g) {
+    extern __shared__ uint32_t small_mem[];
+    __shared__ uint32_t crowded_n, s_crowded[kSmallParticles / kCrowdedCell];
+    uint32_t *table = small_mem;                                     // per cell: count, then next free slot, then end
+    uint16_t *key = reinterpret_cast<uint16_t *>(table + table_at(g.cells) + 1);  // [N] cell of the particle
+    uint16_t *order = key + ((g.N + 1) & ~1);                        // [N] particle of the slot, any order in a cell
+    const int words = (g.N + 31) / 32;
+    uint32_t *bits = reinterpret_cast<uint32_t *>(order + ((g.N + 1) & ~1)), *pre = bits + words;  // crowded cells only
+    const int b = blockIdx.x, tid = threadIdx.x;
+    const size_t sys = (size_t)b * g.N;
+    for (int c = tid; c <= table_at(g.cells); c += kSmallThreads) table[c] = 0u;
+    if (tid == 0) crowded_n = 0u;
+    __syncthreads();
+    for (int i = tid; i < g.N; i += kSmallThreads) {
+        const uint32_t k = particle_cell<D>(x, sys + i, g);
+        key[i] = (uint16_t)k;
+        atomicAdd(&table[table_at((int)k)], 1u);
+    }
+    __syncthreads();
+    const unsigned long long total = scan_cells(
+        g, [&](int c) { return table[table_at(c)]; },
+        [&](int c, uint32_t n, unsigned long long run) {
+            if (g.B == 1) write_rows(block_info, g, 0, c, n, (uint32_t)(run >> 32));
+            if (n > (uint32_t)kCrowdedCell) s_crowded[atomicAdd(&crowded_n, 1u)] = (uint32_t)c;
+            table[table_at(c)] = (uint32_t)run;
+        });
+    for (int c = tid; c < g.cells; c += kSmallThreads) bin_offsets[(size_t)b * g.cells + c] = (int32_t)((uint32_t)sys + table[table_at(c)]);
+    if (tid == 0) {
+        rows_of_system[b] = (uint32_t)(total >> 32);
+        if (b == g.B - 1) bin_offsets[(size_t)g.B * g.cells] = (int32_t)((size_t)g.B * g.N);
+    }
+    if (g.B == 1)
+        for (int r = (int)(total >> 32) + tid; r < g.max_blocks; r += kSmallThreads) block_info[r] = make_int4(0, 0, 0, 0);
+    __syncthreads();
+    for (int i = tid; i < g.N; i += kSmallThreads) order[atomicAdd(&table[table_at(key[i])], 1u)] = (uint16_t)i;
+    __syncthreads();
+    // every slot of a cell is taken: its entry is now its end, the entry before it its start
+    auto cell_start = [&](uint32_t c) { return c ? table[table_at((int)c - 1)] : 0u; };
+    for (int p = tid; p < g.N; p += kSmallThreads) {
+        const uint32_t i = order[p], c = key[i], s = cell_start(c), e = table[table_at((int)c)];
+        if (e - s > (uint32_t)kCrowdedCell) continue;
+        uint32_t rank = 0;
+        for (uint32_t q = s; q < e; ++q) rank += order[q] < i ? 1u : 0u;
+        permutation[sys + i] = (int32_t)(s + rank);
+    }
+    // crowded cells: a bitmap over the particle indices and its prefix popcounts, as in rank_crowded
+    for (uint32_t k = 0; k < crowded_n; ++k) {
+        const uint32_t s = cell_start(s_crowded[k]), e = table[table_at((int)s_crowded[k])];
+        __syncthreads();
+        for (int w = tid; w < words; w += kSmallThreads) bits[w] = 0u;
+        __syncthreads();
+        for (uint32_t q = s + tid; q < e; q += kSmallThreads) atomicOr(&bits[order[q] >> 5], 1u << (order[q] & 31));
+        __syncthreads();
+        __shared__ unsigned long long marked;
+        const unsigned long long mine = tid < words ? (unsigned long long)__popc(bits[tid]) : 0ull;  // words <= 512
+        const unsigned long long before = block_exclusive<kSmallThreads>(mine, marked);
+        if (tid < words) pre[tid] = (uint32_t)before;
+        __syncthreads();
+        for (uint32_t q = s + tid; q < e; q += kSmallThreads) {
+            const uint32_t i = order[q];
+            permutation[sys + i] = (int32_t)(s + pre[i >> 5] + (uint32_t)__popc(bits[i >> 5] & ((1u << (i & 31)) - 1u)));
+        }
+    }
+}
+
+// Work list of several small systems: the rows of a system start behind those of the systems before it.
+__global__ void __launch_bounds__(kSmallThreads)
+rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, const uint32_t *__restrict__ rows_of_system, Geom g) {
+    __shared__ unsigned long long before_s;
+    const int b = blockIdx.x, tid = threadIdx.x;
+    unsigned long long before = 0, all = 0;  // rows of the systems before this one, rows in all
+    for (int k = tid; k < g.B; k += kSmallThreads) {
+        const uint32_t r = rows_of_system[k];
+        all += r;
+        if (k < b) before += r;
+    }
+    block_exclusive<kSmallThreads>(before | (all << 32), before_s);  // both totals below 2^29
+    __syncthreads();
+    const uint32_t row0 = (uint32_t)before_s, grand = (uint32_t)(before_s >> 32);
+    const int32_t *off = bin_offsets + (size_t)b * g.cells;
+    scan_cells(g, [&](int c) { return (uint32_t)(off[c + 1] - off[c]); },
+               [&](int c, uint32_t n, unsigned long long run) { write_rows(block_info, g, b, c, n, row0 + (uint32_t)(run >> 32)); });
+    for (long long r = (long long)grand + (long long)b * kSmallThreads + tid; r < g.max_blocks; r += (long long)g.B * kSmallThreads)
+        block_info[r] = make_int4(0, 0, 0, 0);
 }
 
 // ---------------------------------------------------------------------------
@@ -509,6 +647,20 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     if (scratch_bytes < (int64_t)need)
         return fail(NPA_ERR_SCRATCH_TOO_SMALL, "npa_grid_build: scratch has %lld bytes, %zu needed", (long long)scratch_bytes, need);
     cudaStream_t st = (cudaStream_t)stream;
+    if (small_system(g)) {
+        const size_t bytes = small_smem(g);
+        int unused = 0;
+        if (g.dim == 2) {
+            if ((rc = persistent_ctas(bin_small_kernel<2>, kSmallThreads, bytes, &unused)) != NPA_OK) return rc;  // shared-memory limit
+            bin_small_kernel<2><<<g.B, kSmallThreads, bytes, st>>>(x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        } else {
+            if ((rc = persistent_ctas(bin_small_kernel<3>, kSmallThreads, bytes, &unused)) != NPA_OK) return rc;
+            bin_small_kernel<3><<<g.B, kSmallThreads, bytes, st>>>(x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        }
+        if ((rc = check_launch("bin_small_kernel")) != NPA_OK || g.B == 1) return rc;
+        rows_small_kernel<<<g.B, kSmallThreads, 0, st>>>(bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        return check_launch("rows_small_kernel");
+    }
     cudaError_t e = cudaMemsetAsync(s.counts, 0, s.zero_bytes, st);
     if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "cudaMemsetAsync(scratch): %s", cudaGetErrorString(e));
 
@@ -537,12 +689,11 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     const dim3 tgrid((g.N + kBinThreads - 1) / kBinThreads, g.B);
     scatter_kernel<<<tgrid, kBinThreads, 0, st>>>(s.cellid, s.arrive, bin_offsets, s.order, g);
     if ((rc = check_launch("scatter_kernel")) != NPA_OK) return rc;
-    rank_kernel<<<tgrid, kBinThreads, 0, st>>>(s.cellid, bin_offsets, s.order, permutation, g);
-    if ((rc = check_launch("rank_kernel")) != NPA_OK) return rc;
     const int win = g.N < kRankWindow ? g.N : kRankWindow;
-    rank_crowded_kernel<<<kRankCtas, 256, (size_t)((win + 31) / 32) * 8, st>>>(bin_offsets, s.order, permutation, s.crowded,
-                                                                             crowded_count, g);
-    return check_launch("rank_crowded_kernel");
+    const dim3 rgrid(tgrid.x + kRankCtas, g.B);
+    rank_kernel<<<rgrid, kBinThreads, (size_t)((win + 31) / 32) * 8, st>>>(s.cellid, bin_offsets, s.order, permutation, s.crowded, crowded_count, g,
+                                                                         (int)tgrid.x);
+    return check_launch("rank_kernel");
 }
 
 }  // extern "C"

@@ -83,20 +83,39 @@ struct UmmaArgs {
 
 __device__ unsigned g_umma_status;
 
-// Head and tail images of the weights, chunk by chunk, in the layout the MMA reads.
-__global__ void weight_image_kernel(const float *W, long long stride_n, long long stride_k, int K, int N, int Np, int nchunks,
-                                    float *img) {
-    const int total = nchunks * Np * kUmmaChunk;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < total; e += gridDim.x * blockDim.x) {
-        const int c = e / (Np * kUmmaChunk), rem = e - c * Np * kUmmaChunk;
-        const int n = rem / kUmmaChunk, kk = rem - n * kUmmaChunk;
-        const int k = c * kUmmaChunk + kk;
-        const float v = (n < N && k < K) ? __ldg(W + n * stride_n + k * stride_k) : 0.f;
-        const float head = __uint_as_float(tf32_head_bits(v));
-        float *chunk = img + (size_t)c * 2 * Np * kUmmaChunk;
-        const int at = umma_swizzled(n, kk);
-        chunk[at] = head;
-        chunk[Np * kUmmaChunk + at] = v - head;
+// Head and tail images of one or more weight matrices, chunk by chunk, in the layout the MMA reads.  The jobs share one
+// launch: a step of a small system waits for its launches, and both layers' images (and the one the backward will
+// want) are a few microseconds of work together.
+struct ImageJob {
+    const float *W;
+    long long stride_n, stride_k;
+    int K, N, Np, nchunks;
+    float *img;
+    __host__ __device__ int total() const { return nchunks * Np * kUmmaChunk; }
+};
+constexpr int kImageJobs = 3;
+struct ImageJobs {
+    ImageJob job[kImageJobs];
+    int count;
+};
+__global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
+    int at = blockIdx.x * blockDim.x + threadIdx.x;
+    for (int q = 0; q < jobs.count; ++q) {
+        const ImageJob &j = jobs.job[q];
+        const int total = j.total();
+        if (at < total) {
+            const int Np = j.Np, c = at / (Np * kUmmaChunk), rem = at - c * Np * kUmmaChunk;
+            const int n = rem / kUmmaChunk, kk = rem - n * kUmmaChunk;
+            const int k = c * kUmmaChunk + kk;
+            const float v = (n < j.N && k < j.K) ? __ldg(j.W + n * j.stride_n + k * j.stride_k) : 0.f;
+            const float head = __uint_as_float(tf32_head_bits(v));
+            float *chunk = j.img + (size_t)c * 2 * Np * kUmmaChunk;
+            const int to = umma_swizzled(n, kk);
+            chunk[to] = head;
+            chunk[Np * kUmmaChunk + to] = v - head;
+            return;
+        }
+        at -= total;
     }
 }
 
@@ -339,6 +358,12 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
                 const float lo = (post && relu) ? 0.f : neg_inf;
                 const float *gt0 = (post && gate) ? gate : nullptr;
                 const bool vec4 = (ncol & 3) == 0 && ((uintptr_t)out & 15) == 0 && (!gt0 || ((uintptr_t)gt0 & 15) == 0);
+                if (fuse && pass == 1 && !C) {  // nobody wants the hidden layer: hand the accumulator back
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
+                    continue;
+                }
                 if (pass != 1 || !fuse) {  // pass 1 of the two-layer mode reads what pass 0 of the same thread wrote
                     if (!(ok = umma_wait(pass == 2 ? &sh->y_full : &sh->acc_full[acc], pass == 2 ? it & 1 : (it >> 1) & 1, &sh->abort))) break;
                     tc_fence_after();
@@ -535,6 +560,16 @@ unsigned *umma_status_word() {
 static int umma_round16(int v) { return (v + 15) / 16 * 16; }
 static int umma_chunks(int k) { return (k + kUmmaChunk - 1) / kUmmaChunk; }
 
+static ImageJob image_job(const float *W, int64_t stride_out, int64_t stride_in, int in_dim, int out_dim, void *img) {
+    return ImageJob{W, stride_out, stride_in, in_dim, out_dim, umma_round16(out_dim), umma_chunks(in_dim), static_cast<float *>(img)};
+}
+static int launch_images(const ImageJobs &jobs, cudaStream_t st) {
+    int total = 0;
+    for (int q = 0; q < jobs.count; ++q) total += jobs.job[q].total();
+    weight_image_kernel<<<(total + 255) / 256, 256, 0, st>>>(jobs);
+    return check_launch("weight_image_kernel");
+}
+
 }  // namespace npa
 
 using namespace npa;
@@ -546,14 +581,15 @@ int64_t npa_linear_tcgen05_scratch_bytes(int32_t in_dim, int32_t out_dim) {
     return (int64_t)umma_chunks(in_dim) * 2 * umma_round16(out_dim) * kUmmaChunk * (int64_t)sizeof(float);
 }
 
-int npa_linear_tcgen05(const float *A, const float *W, const float *bias, const float *gate, float *C, int64_t rows,
-                       int32_t in_dim, int32_t out_dim, int64_t w_stride_out, int64_t w_stride_in, int32_t relu, void *scratch,
-                       int64_t scratch_bytes, void *stream) {
+// W == NULL: scratch holds the image already (npa_mlp_forward_tcgen05_images made it).
+static int linear_tcgen05(const float *A, const float *W, const float *bias, const float *gate, float *C, int64_t rows,
+                          int32_t in_dim, int32_t out_dim, int64_t w_stride_out, int64_t w_stride_in, int32_t relu, void *scratch,
+                          int64_t scratch_bytes, void *stream) {
     if (rows <= 0 || in_dim <= 0 || out_dim <= 0)
         return fail(NPA_ERR_INVALID_ARGUMENT, "npa_linear_tcgen05: rows, in_dim and out_dim must be positive");
     if (out_dim > 256 || in_dim > 1024)
         return fail(NPA_ERR_UNSUPPORTED, "npa_linear_tcgen05: supports in_dim <= 1024 and out_dim <= 256, got %d and %d", in_dim, out_dim);
-    if (!A || !W || !C || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_linear_tcgen05: A, W, C and scratch must be non-NULL");
+    if (!A || !C || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_linear_tcgen05: A, W, C and scratch must be non-NULL");
     if ((uintptr_t)A % 4 || (uintptr_t)C % 4 || (uintptr_t)scratch % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "npa_linear_tcgen05: A and C must be float aligned, scratch 16-byte aligned");
     if (scratch_bytes < npa_linear_tcgen05_scratch_bytes(in_dim, out_dim))
@@ -573,15 +609,26 @@ int npa_linear_tcgen05(const float *A, const float *W, const float *bias, const 
     const size_t smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
     int rc = umma_device_setup((int)smem, false, &a.status);
     if (rc != NPA_OK) return rc;
-    const int total = a.nchunks * a.Np * kUmmaChunk;
-    weight_image_kernel<<<(total + 255) / 256, 256, 0, (cudaStream_t)stream>>>(W, w_stride_out, w_stride_in, in_dim, out_dim, a.Np,
-                                                                                 a.nchunks, (float *)scratch);
-    rc = check_launch("weight_image_kernel");
-    if (rc != NPA_OK) return rc;
+    if (W) {
+        ImageJobs jobs = {{image_job(W, w_stride_out, w_stride_in, in_dim, out_dim, scratch)}, 1};
+        if ((rc = launch_images(jobs, (cudaStream_t)stream)) != NPA_OK) return rc;
+    }
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
     linear_umma_kernel<false><<<ctas, kUmmaThreads, smem, (cudaStream_t)stream>>>(a);
     return check_launch("linear_umma_kernel");
+}
+
+int npa_linear_tcgen05(const float *A, const float *W, const float *bias, const float *gate, float *C, int64_t rows,
+                       int32_t in_dim, int32_t out_dim, int64_t w_stride_out, int64_t w_stride_in, int32_t relu, void *scratch,
+                       int64_t scratch_bytes, void *stream) {
+    if (!W) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_linear_tcgen05: A, W, C and scratch must be non-NULL");
+    return linear_tcgen05(A, W, bias, gate, C, rows, in_dim, out_dim, w_stride_out, w_stride_in, relu, scratch, scratch_bytes, stream);
+}
+
+int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image_bytes, float *C, int64_t rows, int32_t in_dim, int32_t out_dim,
+                                void *stream) {
+    return linear_tcgen05(A, nullptr, nullptr, nullptr, C, rows, in_dim, out_dim, 0, 0, 0, const_cast<void *>(image), image_bytes, stream);
 }
 
 int64_t npa_mlp_forward_tcgen05_scratch_bytes(int32_t in_dim, int32_t out_dim) {
@@ -589,14 +636,18 @@ int64_t npa_mlp_forward_tcgen05_scratch_bytes(int32_t in_dim, int32_t out_dim) {
     return npa_linear_tcgen05_scratch_bytes(in_dim, kUmmaRows) + (int64_t)4 * 2 * umma_round16(out_dim) * kUmmaChunk * (int64_t)sizeof(float);
 }
 
-int npa_mlp_forward_tcgen05(const float *z, const float *W1, const float *b1, const float *W2, float *h, float *y, int64_t rows,
-                            int32_t in_dim, int32_t out_dim, int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out,
-                            int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *stream) {
+int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float *b1, const float *W2, float *h, float *y, int64_t rows,
+                                   int32_t in_dim, int32_t out_dim, int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out,
+                                   int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes,
+                                   void *stream) {
     const char *me = "npa_mlp_forward_tcgen05";
+    if (dz_image && ((uintptr_t)dz_image % 16 || dz_image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim)))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: dz_image must be 16-byte aligned and hold %lld bytes", me,
+                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim));
     if (rows <= 0 || in_dim <= 0 || out_dim <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
     if (in_dim > 1024 || out_dim > 64)
         return fail(NPA_ERR_UNSUPPORTED, "%s: supports in_dim <= 1024 and out_dim <= 64 (hidden width 128), got %d and %d", me, in_dim, out_dim);
-    if (!z || !W1 || !W2 || !h || !y || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, h, y and scratch must be non-NULL", me);
+    if (!z || !W1 || !W2 || !y || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
     if ((uintptr_t)z % 4 || (uintptr_t)h % 4 || (uintptr_t)y % 4 || (uintptr_t)scratch % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, h and y must be float aligned, scratch 16-byte aligned", me);
     if (scratch_bytes < npa_mlp_forward_tcgen05_scratch_bytes(in_dim, out_dim))
@@ -620,15 +671,22 @@ int npa_mlp_forward_tcgen05(const float *z, const float *W1, const float *b1, co
     int rc = umma_device_setup((int)smem, true, &a.status);
     if (rc != NPA_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    const int total1 = a.nchunks * a.Np * kUmmaChunk, total2 = 4 * a.N2p * kUmmaChunk;
-    weight_image_kernel<<<(total1 + 255) / 256, 256, 0, st>>>(W1, w1_stride_out, w1_stride_in, in_dim, kUmmaRows, a.Np, a.nchunks, (float *)scratch);
-    if ((rc = check_launch("weight_image_kernel")) != NPA_OK) return rc;
-    weight_image_kernel<<<(total2 + 255) / 256, 256, 0, st>>>(W2, w2_stride_out, w2_stride_in, kUmmaRows, out_dim, a.N2p, 4, (float *)a.W2img);
-    if ((rc = check_launch("weight_image_kernel")) != NPA_OK) return rc;
+    ImageJobs jobs = {{image_job(W1, w1_stride_out, w1_stride_in, in_dim, kUmmaRows, scratch),
+                       image_job(W2, w2_stride_out, w2_stride_in, kUmmaRows, out_dim, (void *)a.W2img)}, 2};
+    if (dz_image) jobs.job[jobs.count++] = image_job(W1, w1_stride_in, w1_stride_out, kUmmaRows, in_dim, dz_image);
+    if ((rc = launch_images(jobs, st)) != NPA_OK) return rc;
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
     linear_umma_kernel<true><<<ctas, kUmmaThreads, smem, st>>>(a);
     return check_launch("linear_umma_kernel (two layers)");
+}
+
+int npa_mlp_forward_tcgen05(const float *z, const float *W1, const float *b1, const float *W2, float *h, float *y, int64_t rows,
+                            int32_t in_dim, int32_t out_dim, int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out,
+                            int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *stream) {
+    if (!h) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_mlp_forward_tcgen05: h must be non-NULL");
+    return npa_mlp_forward_tcgen05_images(z, W1, b1, W2, h, y, rows, in_dim, out_dim, w1_stride_out, w1_stride_in, w2_stride_out, w2_stride_in,
+                                          scratch, scratch_bytes, nullptr, 0, stream);
 }
 
 int npa_linear_tcgen05_wait_selftest(int32_t limit_us, int32_t *device_result, void *stream) {

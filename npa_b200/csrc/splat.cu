@@ -4,9 +4,8 @@
 // renderer of its splat loss (losses/splat_loss.py:71-86).  The reference materialises the
 // (2r+1)^2 patch of every particle as [N, (2r+1)^2] index / weight tensors and scatter-adds them
 // (atomics, run-to-run different sums).  Here both directions are gathers:
-//   forward  : a CTA owns a 16x16 pixel tile.  The particles of the system are culled against the
-//              tile 256 at a time (ordered ballot compaction into shared memory), then every pixel
-//              thread adds the listed particles in particle order -- no atomics, deterministic;
+//   forward  : a CTA owns a 16x16 pixel tile and multiplies the separable weights of the particles that
+//              touch it into it -- no atomics, fixed order of sums, deterministic;
 //   backward : a warp owns a particle and walks its patch, reading the upstream image gradient
 //              (L2 resident) and reducing the colour and position gradients with shuffles.
 // Pixel of a particle: p = (x - lo) / (hi - lo) * (img - 1) (y flipped when y_up), base = floor(p),
@@ -78,61 +77,165 @@ __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
     a.wscale[n] = a.norm_scale / (1e-8f + sx * sy);
 }
 
-__global__ void __launch_bounds__(kSplatTile *kSplatTile) splat_forward_kernel(SplatArgs a) {
-    constexpr int T = kSplatTile * kSplatTile;
-    __shared__ int s_cx[T], s_cy[T];
-    __shared__ float s_fx[T], s_fy[T], s_w[T], s_r[T], s_g[T], s_b[T];
-    __shared__ int s_warp_count[T / 32];
+// A CTA per 16 x 16 pixel tile.  The weight of a particle is a product of a row and a column factor, so a tile's image is
+// a product of small matrices over the particles that touch it: sum_n wx_n[px] (wy_n[py] c_n).  1,024 particles at a time
+// are culled with a pixel to spare (ordered compaction); 64 at a time get their 16 + 16 factors in shared memory (32
+// exponentials per particle and tile instead of 256), eight per thread; every half warp multiplies every 16th particle
+// into 8 x 2 pixels x 4 channels per thread in packed fp32x2; the 16 partial images are added in a fixed order.  Bound
+// by instruction issue (culling, factors and products about a third each).  8 systems of 4,096 particles, 256 x 256,
+// patches of 41 x 41: 201 -> SPLAT_FWD us.
+constexpr int kSplatThreads = 256, kSplatCull = 4, kSplatChunk = 64, kSplatParts = 16, kSplatWarps = kSplatThreads / 32;
+
+struct SplatLists {
+    int n[kSplatThreads * kSplatCull + kSplatChunk];
+    float wx[kSplatChunk][kSplatTile];
+    float4 wy[kSplatChunk][kSplatTile];  // row factor times scale times (r, g, b, 1)
+};
+union SplatShared {
+    SplatLists lists;
+    float4 part[kSplatWarps][kSplatTile * kSplatTile];
+};
+
+__global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatArgs a) {
+    __shared__ SplatShared sh;
+    __shared__ int s_count[kSplatCull * kSplatWarps];
     const int tiles = (a.img + kSplatTile - 1) / kSplatTile;
     const int tx0 = (blockIdx.x % tiles) * kSplatTile, ty0 = (blockIdx.x / tiles) * kSplatTile;
-    const int b = blockIdx.y;
+    const int b = blockIdx.y, r = a.radius;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int px = tx0 + (tid % kSplatTile), py = ty0 + (tid / kSplatTile);
-    const int r = a.radius;
+    const int part = tid >> 4, cell = tid & 15, px = (cell & 1) * 8, py = (cell >> 1) * 2;  // pixels px..px+7, py..py+1
     const float inv2s2 = 1.0f / (2.0f * a.sigma * a.sigma);
-    float acc[4] = {0.f, 0.f, 0.f, 0.f};
+    unsigned long long acc[2][8][2];  // [row][pixel][(r, g), (b, density)]
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int x = 0; x < 8; ++x) acc[y][x][0] = acc[y][x][1] = 0ull;
 
-    for (int n0 = 0; n0 < a.N; n0 += T) {
-        const int n = n0 + tid;
-        bool hit = false;
-        SplatPoint p = {0, 0, 0.f, 0.f};
-        if (n < a.N) {
-            p = splat_point(a, (long long)b * a.N + n);
-            hit = p.cx + r >= tx0 && p.cx - r < tx0 + kSplatTile && p.cy + r >= ty0 && p.cy - r < ty0 + kSplatTile;
+    // particles off .. off + count - 1 of the list
+    auto multiply = [&](int off, int count) {
+        const int padded = (count + kSplatParts - 1) / kSplatParts * kSplatParts;
+        const int p = tid >> 2, axis = (tid >> 1) & 1, o0 = (tid & 1) * 8;
+        if (p < padded) {
+            float w[8];
+            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            int at = 0, lo = 1, hi = 0;
+            float frac = 0.f;
+            if (p < count) {
+                const long long n = (long long)b * a.N + sh.lists.n[off + p];
+                const SplatPoint pt = splat_point(a, n);
+                at = (axis ? ty0 - pt.cy : tx0 - pt.cx) + o0;  // offset of the first of the eight from the particle's pixel
+                frac = axis ? pt.fy : pt.fx;
+                lo = -r; hi = r;
+                if (axis) {
+                    const float scale = a.normalize ? __ldg(a.wscale + n) : 1.0f;
+                    const float *col = a.color + n * 3;
+                    c = make_float4(scale * __ldg(col), scale * __ldg(col + 1), scale * __ldg(col + 2), scale);
+                }
+            }
+#pragma unroll
+            for (int k = 0; k < 8; ++k) {
+                const int d = at + k;
+                const float t = (float)d - frac;
+                w[k] = d >= lo && d <= hi ? expf(-(t * t) * inv2s2) : 0.f;
+            }
+            if (!axis) {
+                float4 *o = reinterpret_cast<float4 *>(&sh.lists.wx[p][o0]);
+                o[0] = make_float4(w[0], w[1], w[2], w[3]);
+                o[1] = make_float4(w[4], w[5], w[6], w[7]);
+            } else {
+#pragma unroll
+                for (int k = 0; k < 8; ++k) sh.lists.wy[p][o0 + k] = make_float4(w[k] * c.x, w[k] * c.y, w[k] * c.z, w[k] * c.w);
+            }
         }
-        // ordered compaction: particles keep their index order in the list
-        const unsigned bal = __ballot_sync(0xffffffffu, hit);
-        if (lane == 0) s_warp_count[warp] = __popc(bal);
         __syncthreads();
-        int base = 0, total = 0;
-        for (int w = 0; w < T / 32; ++w) {
-            const int c = s_warp_count[w];
-            if (w < warp) base += c;
-            total += c;
-        }
-        if (hit) {
-            const int slot = base + __popc(bal & ((1u << lane) - 1u));
-            const float scale = a.normalize ? __ldg(a.wscale + (long long)b * a.N + n) : 1.0f;
-            const float *c = a.color + ((long long)b * a.N + n) * 3;
-            s_cx[slot] = p.cx; s_cy[slot] = p.cy; s_fx[slot] = p.fx; s_fy[slot] = p.fy; s_w[slot] = scale;
-            s_r[slot] = __ldg(c); s_g[slot] = __ldg(c + 1); s_b[slot] = __ldg(c + 2);
-        }
-        __syncthreads();
-        for (int e = 0; e < total; ++e) {
-            const int dx = px - s_cx[e], dy = py - s_cy[e];
-            if (dx < -r || dx > r || dy < -r || dy > r) continue;
-            const float tx = (float)dx - s_fx[e], ty = (float)dy - s_fy[e];
-            const float w = expf(-(tx * tx + ty * ty) * inv2s2) * s_w[e];
-            acc[0] = fmaf(s_r[e], w, acc[0]);
-            acc[1] = fmaf(s_g[e], w, acc[1]);
-            acc[2] = fmaf(s_b[e], w, acc[2]);
-            acc[3] += w;
+        for (int q = part; q < padded; q += kSplatParts) {
+            const float4 x0 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px]), x1 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px + 4]);
+            const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+#pragma unroll
+            for (int y = 0; y < 2; ++y) {
+                const float4 w = sh.lists.wy[q][py + y];
+                const unsigned long long rg = pack2(w.x, w.y), bd = pack2(w.z, w.w);
+#pragma unroll
+                for (int x = 0; x < 8; ++x) {
+                    const unsigned long long xx = pack2(xs[x], xs[x]);
+                    acc[y][x][0] = fma2(xx, rg, acc[y][x][0]);
+                    acc[y][x][1] = fma2(xx, bd, acc[y][x][1]);
+                }
+            }
         }
         __syncthreads();
+    };
+
+    const float top = (float)(a.img - 1), per = top / a.span, reach = (float)r + 9.25f;  // patch radius, half a tile, a pixel, rounding
+    const float mx = (float)tx0 + 7.5f, my = (float)ty0 + 7.5f;
+    int pending = 0;
+    for (int n0 = 0; n0 < a.N; n0 += kSplatThreads * kSplatCull) {
+        unsigned ballots[kSplatCull];
+#pragma unroll
+        for (int q = 0; q < kSplatCull; ++q) {
+            const int n = n0 + q * kSplatThreads + tid;
+            bool hit = false;
+            if (n < a.N) {
+                const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + (long long)b * a.N + n);
+                const float x = (v.x - a.lo) * per;
+                float y = (v.y - a.lo) * per;
+                if (a.y_up) y = top - y;
+                hit = fabsf(x - mx) <= reach && fabsf(y - my) <= reach;
+            }
+            ballots[q] = __ballot_sync(0xffffffffu, hit);
+            if (lane == 0) s_count[q * kSplatWarps + warp] = __popc(ballots[q]);
+        }
+        __syncthreads();
+        int incl = s_count[lane];  // kSplatCull * kSplatWarps == 32 counts in list order
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int total = pending + __shfl_sync(0xffffffffu, incl, 31);
+#pragma unroll
+        for (int q = 0; q < kSplatCull; ++q) {
+            const int before = q * kSplatWarps + warp - 1;
+            const int base = __shfl_sync(0xffffffffu, incl, before & 31);
+            if ((ballots[q] >> lane) & 1u)
+                sh.lists.n[pending + (before < 0 ? 0 : base) + __popc(ballots[q] & ((1u << lane) - 1u))] = n0 + q * kSplatThreads + tid;
+        }
+        __syncthreads();
+        pending = total;
+        int done = 0;
+        for (; pending - done >= kSplatChunk; done += kSplatChunk) multiply(done, kSplatChunk);
+        // the rest of the list moves to its front
+        const int keep = tid < pending - done ? sh.lists.n[done + tid] : 0;
+        __syncthreads();
+        if (tid < pending - done) sh.lists.n[tid] = keep;
+        __syncthreads();
+        pending -= done;
     }
-    if (px < a.img && py < a.img)
-        reinterpret_cast<float4 *>(a.out)[((long long)b * a.img + py) * a.img + px] =
-            make_float4(acc[0], acc[1], acc[2], acc[3]);
+    if (pending > 0) multiply(0, pending);
+    __syncthreads();
+    // the two halves of a warp meet by shuffles, the eight warps in shared memory
+#pragma unroll
+    for (int y = 0; y < 2; ++y)
+#pragma unroll
+        for (int x = 0; x < 8; ++x) {
+            float4 v;
+            unpack2(acc[y][x][0], v.x, v.y);
+            unpack2(acc[y][x][1], v.z, v.w);
+            v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
+            v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
+            v.z += __shfl_xor_sync(0xffffffffu, v.z, 16);
+            v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
+            if (lane < 16) sh.part[warp][(py + y) * kSplatTile + px + x] = v;
+        }
+    __syncthreads();
+    const int ox = tx0 + (tid % kSplatTile), oy = ty0 + (tid / kSplatTile);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int w = 0; w < kSplatWarps; ++w) {
+        const float4 q = sh.part[w][tid];
+        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+    }
+    if (ox < a.img && oy < a.img) reinterpret_cast<float4 *>(a.out)[((long long)b * a.img + oy) * a.img + ox] = v;
 }
 
 __device__ inline float warp_sum(float v) {
@@ -147,8 +250,14 @@ __device__ inline float warp_sum(float v) {
 //              =         1 / sigma^2 * sum A g t_x                                         (plain)
 // sums over the pixels of the patch that lie inside the image; S = S_x S_y and T_x = sum g_x t_x over
 // the whole patch axis; t_x = dx - frac_x.  floor() passes no gradient, so dL/dp = dL/dfrac.
+// The weight is separable: a lane keeps one column of the patch, runs down its rows with the row factors from shared
+// memory and applies the column factor once at the end (2 (2r+1) exponentials per particle instead of (2r+1)^2).  The
+// last, narrow group of columns is dealt to the lanes several rows at a time.  Bound by the reads of the upstream image
+// (16 bytes per pixel of the patch, from L1 and L2).  8 x 4,096 particles, patches of 41 x 41: 158 -> SPLAT_BWD us.
 __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
-    const int lane = threadIdx.x & 31;
+    constexpr int kMost = 2 * kSplatMaxRadius + 1;
+    __shared__ float2 s_y[8][kMost];  // row factor, row factor times t_y
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const long long warp = (blockIdx.x * (long long)blockDim.x + threadIdx.x) >> 5;
     const long long total = (long long)a.B * a.N;
     if (warp >= total) return;
@@ -158,34 +267,44 @@ __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
     const float inv2s2 = 1.0f / (2.0f * a.sigma * a.sigma);
     const float *c = a.color + warp * 3;
     const float cr = __ldg(c), cg = __ldg(c + 1), cb = __ldg(c + 2);
-    float gr = 0.f, gg = 0.f, gb = 0.f, a0 = 0.f, ax = 0.f, ay = 0.f;
     const float4 *img = reinterpret_cast<const float4 *>(a.g_out) + (long long)b * a.img * a.img;
-    for (int k = lane; k < P * P; k += 32) {
-        const int dy = k / P - r, dx = k - (k / P) * P - r;
-        const int px = p.cx + dx, py = p.cy + dy;
-        if (px < 0 || px >= a.img || py < 0 || py >= a.img) continue;
-        const float tx = (float)dx - p.fx, ty = (float)dy - p.fy;
-        const float g = expf(-(tx * tx + ty * ty) * inv2s2);
-        const float4 d = __ldg(img + (long long)py * a.img + px);
-        const float A = fmaf(cr, d.x, fmaf(cg, d.y, fmaf(cb, d.z, d.w)));
-        gr = fmaf(g, d.x, gr); gg = fmaf(g, d.y, gg); gb = fmaf(g, d.z, gb);
-        const float Ag = A * g;
-        a0 += Ag;
-        ax = fmaf(Ag, tx, ax);
-        ay = fmaf(Ag, ty, ay);
+    float sx = 0.f, sy = 0.f, t_x = 0.f, t_y = 0.f;  // the axis sums, spread over the lanes
+    for (int k = lane; k < P; k += 32) {
+        const float ux = (float)(k - r) - p.fx, uy = (float)(k - r) - p.fy;
+        const float ex = expf(-(ux * ux) * inv2s2), ey = expf(-(uy * uy) * inv2s2);
+        sx += ex; sy += ey;
+        t_x = fmaf(ex, ux, t_x); t_y = fmaf(ey, uy, t_y);
+        s_y[w][k] = make_float2(ey, ey * uy);
+    }
+    __syncwarp();
+    // rows of the patch inside the image
+    const int k0 = max(0, r - p.cy), k1 = min(P, a.img - p.cy + r);
+    float gr = 0.f, gg = 0.f, gb = 0.f, a0 = 0.f, ax = 0.f, ay = 0.f;
+    for (int c0 = 0; c0 < P; c0 += 32) {
+        const int width = min(32, P - c0), steps = 32 / width;  // lanes: `width` columns x `steps` rows
+        const int col = lane % width, row0 = lane / width;
+        const int k = c0 + col, x = p.cx + k - r;
+        if (row0 >= steps || x < 0 || x >= a.img) continue;
+        float sr = 0.f, sg = 0.f, sb = 0.f, sA = 0.f, tA = 0.f;
+        const float4 *at = img + (long long)(p.cy - r + k0 + row0) * a.img + x;
+#pragma unroll 4
+        for (int y = k0 + row0; y < k1; y += steps, at += (long long)steps * a.img) {
+            const float4 d = __ldg(at);
+            const float2 f = s_y[w][y];
+            const float A = fmaf(cr, d.x, fmaf(cg, d.y, fmaf(cb, d.z, d.w)));
+            sr = fmaf(f.x, d.x, sr); sg = fmaf(f.x, d.y, sg); sb = fmaf(f.x, d.z, sb);
+            sA = fmaf(f.x, A, sA);
+            tA = fmaf(f.y, A, tA);
+        }
+        const float ux = (float)(k - r) - p.fx, ex = expf(-(ux * ux) * inv2s2);
+        gr = fmaf(ex, sr, gr); gg = fmaf(ex, sg, gg); gb = fmaf(ex, sb, gb);
+        a0 = fmaf(ex, sA, a0);
+        ax = fmaf(ex * ux, sA, ax);
+        ay = fmaf(ex, tA, ay);
     }
     gr = warp_sum(gr); gg = warp_sum(gg); gb = warp_sum(gb);
     a0 = warp_sum(a0); ax = warp_sum(ax); ay = warp_sum(ay);
-    float sx = 0.f, sy = 0.f, t_x = 0.f, t_y = 0.f;
-    if (a.normalize) {  // the axis sums, spread over the lanes
-        for (int d = -r + lane; d <= r; d += 32) {
-            const float ux = (float)d - p.fx, uy = (float)d - p.fy;
-            const float ex = expf(-(ux * ux) * inv2s2), ey = expf(-(uy * uy) * inv2s2);
-            sx += ex; sy += ey;
-            t_x = fmaf(ex, ux, t_x); t_y = fmaf(ey, uy, t_y);
-        }
-        sx = warp_sum(sx); sy = warp_sum(sy); t_x = warp_sum(t_x); t_y = warp_sum(t_y);
-    }
+    if (a.normalize) { sx = warp_sum(sx); sy = warp_sum(sy); t_x = warp_sum(t_x); t_y = warp_sum(t_y); }
     if (lane != 0) return;
     float scale = 1.0f, gfx = ax, gfy = ay;
     if (a.normalize) {
@@ -241,7 +360,7 @@ int npa_splat_forward(const float *x, const float *color, int32_t batch, int32_t
         if ((rc = check_launch("splat_scale_kernel")) != NPA_OK) return rc;
     }
     const int tiles = (img_size + kSplatTile - 1) / kSplatTile;
-    splat_forward_kernel<<<dim3(tiles * tiles, batch), kSplatTile * kSplatTile, 0, st>>>(a);
+    splat_forward_kernel<<<dim3(tiles * tiles, batch), kSplatThreads, 0, st>>>(a);
     return check_launch("splat_forward_kernel");
 }
 

@@ -15,7 +15,9 @@ struct StepArgs {
     const float *y;       // [BN, D + C]
     const float *x_bin;   // [BN, P]
     const float *s_bin;   // [BN, C]
-    const float *mask;    // [BN] (0 / 1) or NULL = every particle updates
+    const float *mask;    // [BN] (0 / 1, or uniforms) or NULL = every particle updates
+    int uniforms;         // mask holds uniforms: a particle updates where its value is below `below`
+    float below;
     float *x_out;         // [BN, P]
     float *s_out;         // [BN, C]
     const float *g_x_out; // backward: upstream of x_out [BN, P]
@@ -26,6 +28,12 @@ struct StepArgs {
     float alpha, eps, dt;
     int wrap;
 };
+
+__device__ inline float mask_of(const StepArgs &a, long long i) {
+    if (!a.mask) return 1.0f;
+    const float m = __ldg(a.mask + i);
+    return a.uniforms ? (m < a.below ? 1.0f : 0.0f) : m;
+}
 
 // remainder(x + L/2, L) - L/2 with torch's sign convention (result of remainder in [0, L)).
 __device__ inline float wrap_axis(float x, float L) {
@@ -39,7 +47,7 @@ __device__ inline float wrap_axis(float x, float L) {
 template <int D>
 __device__ inline void step_forward_element(const StepArgs &a, const Geom &g, long long i, int c, float v) {
     constexpr int P = D == 2 ? 2 : 4;
-    const float m = a.mask ? __ldg(a.mask + i) : 1.0f;
+    const float m = mask_of(a, i);
     if (c >= D) {
         const long long o = i * a.C + (c - D);
         a.s_out[o] = __ldg(a.s_bin + o) + (a.dt * v) * m;
@@ -66,7 +74,7 @@ __device__ inline void step_forward_element(const StepArgs &a, const Geom &g, lo
 template <int D>
 __device__ inline float step_backward_element(const StepArgs &a, long long i, int c) {
     constexpr int P = D == 2 ? 2 : 4;
-    const float m = a.mask ? __ldg(a.mask + i) : 1.0f;
+    const float m = mask_of(a, i);
     if (c >= D) return a.g_s_out ? (a.dt * m) * __ldg(a.g_s_out + i * a.C + (c - D)) : 0.f;
     if (!a.g_x_out) return 0.f;
     const float *row = a.y + i * (D + a.C);
@@ -167,7 +175,7 @@ __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom
             for (int f = threadIdx.x; f < rows * C4; f += blockDim.x) {
                 const int row = f / C4, c4 = f - row * C4;
                 const long long i = r0 + row;
-                const float m = a.mask ? __ldg(a.mask + i) : 1.0f;
+                const float m = mask_of(a, i);
                 const float4 sv = __ldg(reinterpret_cast<const float4 *>(a.s_bin) + i * C4 + c4);
                 const float *yr = tile + row * W + D + 4 * c4;
                 reinterpret_cast<float4 *>(a.s_out)[i * C4 + c4] =
@@ -176,7 +184,7 @@ __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom
             }
             for (int row = threadIdx.x; row < rows; row += blockDim.x) {
                 const long long i = r0 + row;
-                const float m = a.mask ? __ldg(a.mask + i) : 1.0f;
+                const float m = mask_of(a, i);
                 const float *yr = tile + row * W;
                 float n2 = 0.f;
 #pragma unroll
@@ -212,7 +220,7 @@ __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom
             for (int f = threadIdx.x; f < rows * C4; f += blockDim.x) {
                 const int row = f / C4, c4 = f - row * C4;
                 const long long i = r0 + row;
-                const float k = a.dt * (a.mask ? __ldg(a.mask + i) : 1.0f);
+                const float k = a.dt * (mask_of(a, i));
                 float4 gs = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (a.g_s_out) gs = __ldg(reinterpret_cast<const float4 *>(a.g_s_out) + i * C4 + c4);
                 float *o = tile + row * W + D + 4 * c4;
@@ -276,9 +284,8 @@ using namespace npa;
 
 extern "C" {
 
-int npa_step_update_forward(const npa_grid *gd, const float *y, const float *x_bin, const float *s_bin,
-                            const float *mask, int32_t channels, float alpha, float dt, int32_t wrap, float *x_out,
-                            float *s_out, void *stream) {
+static int step_forward(const npa_grid *gd, const float *y, const float *x_bin, const float *s_bin, const float *mask, int uniforms, float below,
+                        int32_t channels, float alpha, float dt, int32_t wrap, float *x_out, float *s_out, void *stream) {
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
@@ -286,24 +293,48 @@ int npa_step_update_forward(const npa_grid *gd, const float *y, const float *x_b
     if (!y || !x_bin || !s_bin || !x_out || !s_out)
         return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_forward: y, x_bin, s_bin, x_out and s_out must be non-NULL");
     StepArgs a = {};
-    a.y = y; a.x_bin = x_bin; a.s_bin = s_bin; a.mask = mask; a.x_out = x_out; a.s_out = s_out;
+    a.y = y; a.x_bin = x_bin; a.s_bin = s_bin; a.mask = mask; a.uniforms = uniforms; a.below = below; a.x_out = x_out; a.s_out = s_out;
     a.particles = (long long)g.B * g.N; a.C = channels; a.alpha = alpha; a.eps = g.h; a.dt = dt; a.wrap = wrap;
     if (((uintptr_t)y % 16)) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_forward: y must be 16-byte aligned");
     return launch_step<false>(g, a, (cudaStream_t)stream);
 }
 
-int npa_step_update_backward(const npa_grid *gd, const float *y, const float *mask, int32_t channels, float alpha,
-                             float dt, const float *g_x_out, const float *g_s_out, float *g_y, void *stream) {
+int npa_step_update_forward(const npa_grid *gd, const float *y, const float *x_bin, const float *s_bin,
+                            const float *mask, int32_t channels, float alpha, float dt, int32_t wrap, float *x_out,
+                            float *s_out, void *stream) {
+    return step_forward(gd, y, x_bin, s_bin, mask, 0, 0.f, channels, alpha, dt, wrap, x_out, s_out, stream);
+}
+
+int npa_step_update_forward_masked(const npa_grid *gd, const float *y, const float *x_bin, const float *s_bin, const float *uniforms,
+                                   float update_below, int32_t channels, float alpha, float dt, int32_t wrap, float *x_out, float *s_out,
+                                   void *stream) {
+    if (!uniforms) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_forward_masked: uniforms must be non-NULL");
+    return step_forward(gd, y, x_bin, s_bin, uniforms, 1, update_below, channels, alpha, dt, wrap, x_out, s_out, stream);
+}
+
+static int step_backward(const npa_grid *gd, const float *y, const float *mask, int uniforms, float below, int32_t channels, float alpha,
+                         float dt, const float *g_x_out, const float *g_s_out, float *g_y, void *stream) {
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
     if (channels <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_backward: channels must be positive, got %d", channels);
     if (!y || !g_y) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_backward: y and g_y must be non-NULL");
     StepArgs a = {};
-    a.y = y; a.mask = mask; a.g_x_out = g_x_out; a.g_s_out = g_s_out; a.g_y = g_y;
+    a.y = y; a.mask = mask; a.uniforms = uniforms; a.below = below; a.g_x_out = g_x_out; a.g_s_out = g_s_out; a.g_y = g_y;
     a.particles = (long long)g.B * g.N; a.C = channels; a.alpha = alpha; a.eps = g.h; a.dt = dt;
     if (((uintptr_t)g_y % 16)) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_backward: g_y must be 16-byte aligned");
     return launch_step<true>(g, a, (cudaStream_t)stream);
+}
+
+int npa_step_update_backward(const npa_grid *gd, const float *y, const float *mask, int32_t channels, float alpha,
+                             float dt, const float *g_x_out, const float *g_s_out, float *g_y, void *stream) {
+    return step_backward(gd, y, mask, 0, 0.f, channels, alpha, dt, g_x_out, g_s_out, g_y, stream);
+}
+
+int npa_step_update_backward_masked(const npa_grid *gd, const float *y, const float *uniforms, float update_below, int32_t channels, float alpha,
+                                    float dt, const float *g_x_out, const float *g_s_out, float *g_y, void *stream) {
+    if (!uniforms) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_step_update_backward_masked: uniforms must be non-NULL");
+    return step_backward(gd, y, uniforms, 1, update_below, channels, alpha, dt, g_x_out, g_s_out, g_y, stream);
 }
 
 }  // extern "C"

@@ -533,14 +533,16 @@ struct StepNode : Node {
     SavedVariable y_;
     Tensor mask;
     int C;
-    float alpha, dt;
+    float alpha, dt, below;  // below >= 0: the mask is uniforms, a particle updates where its value is below it
     variable_list apply(variable_list &&g) override {
         const Tensor y = y_.unpack(), gx = solid(g[0]), gs = solid(g[1]);
         Tensor gy;
         if (should_compute_output(0) && (gx.defined() || gs.defined())) {
             c10::cuda::CUDAGuard guard(y.device());
             gy = blank(y);
-            check_status(npa_step_update_backward(&grid->g, fptr(y), fptr(mask), C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y)));
+            check_status(mask.defined() && below >= 0.f
+                             ? npa_step_update_backward_masked(&grid->g, fptr(y), fptr(mask), below, C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y))
+                             : npa_step_update_backward(&grid->g, fptr(y), fptr(mask), C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y)));
         }
         return {gy, should_compute_output(1) ? gx : Tensor(), should_compute_output(2) ? gs : Tensor()};
     }
@@ -550,7 +552,8 @@ struct StepNode : Node {
     }
 };
 
-py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, const Tensor &s, const OptTensor &mask_, double alpha, double dt, bool wrap) {
+py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, const Tensor &s, const OptTensor &mask_, double alpha, double dt, bool wrap,
+                      double below) {
     Grid &g = *grid;
     const Tensor mask = or_none(mask_);
     g.positions(x, "binned_positions");
@@ -559,11 +562,14 @@ py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, con
     if (mask.defined()) g.rows(mask, "mask");
     c10::cuda::CUDAGuard guard(x.device());
     Tensor xo = blank(x), so = blank(s);
-    check_status(npa_step_update_forward(&g.g, fptr(y), fptr(x), fptr(s), fptr(mask), (int)s.size(2), (float)alpha, (float)dt, wrap, fmut(xo),
-                                         fmut(so), stream_of(x)));
+    check_status(mask.defined() && below >= 0.0
+                     ? npa_step_update_forward_masked(&g.g, fptr(y), fptr(x), fptr(s), fptr(mask), (float)below, (int)s.size(2), (float)alpha, (float)dt,
+                                                      wrap, fmut(xo), fmut(so), stream_of(x))
+                     : npa_step_update_forward(&g.g, fptr(y), fptr(x), fptr(s), fptr(mask), (int)s.size(2), (float)alpha, (float)dt, wrap, fmut(xo),
+                                               fmut(so), stream_of(x)));
     if (recording(y, x, s)) {
         auto n = node_for<StepNode>(y, x, s);
-        n->grid = grid; n->mask = mask; n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt;
+        n->grid = grid; n->mask = mask; n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)below;
         n->y_ = SavedVariable(y, false);
         torch::autograd::set_history(xo, n);
         torch::autograd::set_history(so, n);
@@ -576,7 +582,7 @@ constexpr int kHidden = 128;
 
 struct MlpNode : Node {
     SavedVariable z_, w1_, w2_;
-    Tensor h;
+    Tensor h, dz_image;  // hidden layer; W1 as the tensor cores read it for dz = dh W1
     std::vector<int64_t> z_shape;
     variable_list apply(variable_list &&g) override {
         const Tensor z = z_.unpack(), w1 = w1_.unpack(), w2 = w2_.unpack();
@@ -590,10 +596,7 @@ struct MlpNode : Node {
         Tensor gz, gw1, gb1, gw2;
         if (should_compute_output(0)) {
             gz = floats(z, z_shape);
-            const int64_t bytes = npa_linear_tcgen05_scratch_bytes(kHidden, (int)k);
-            Tensor image = floats(z, {bytes / 4});
-            check_status(npa_linear_tcgen05(fptr(dh), fptr(w1), nullptr, nullptr, fmut(gz), m, kHidden, (int)k, w1.stride(1), w1.stride(0), 0,
-                                            image.mutable_data_ptr(), bytes, st));
+            check_status(npa_linear_tcgen05_prepared(fptr(dh), dz_image.const_data_ptr(), dz_image.numel() * 4, fmut(gz), m, kHidden, (int)k, st));
         }
         const bool n1 = should_compute_output(1), nb = should_compute_output(2), n2 = should_compute_output(3);
         if (n1 || nb || n2) {
@@ -612,7 +615,7 @@ struct MlpNode : Node {
     }
     void release_variables() override {
         z_.reset_data(); w1_.reset_data(); w2_.reset_data();
-        h = Tensor();
+        h = dz_image = Tensor();
     }
 };
 
@@ -622,15 +625,19 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
     const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
     std::vector<int64_t> shape = z.sizes().vec();
     shape.back() = o;
-    Tensor y = floats(z, shape), h = floats(z, {m, kHidden});
+    const bool record = recording(z, w1, b1, w2);
     const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o);
-    Tensor image = floats(z, {bytes / 4});
-    check_status(npa_mlp_forward_tcgen05(fptr(z), fptr(w1), fptr(b1), fptr(w2), fmut(h), fmut(y), m, (int)k, (int)o, w1.stride(0), w1.stride(1),
-                                         w2.stride(0), w2.stride(1), image.mutable_data_ptr(), bytes, stream_of(z)));
-    if (recording(z, w1, b1, w2)) {
+    const int64_t dz_bytes = record && wants_grad(z) ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
+    // without a backward the hidden layer stays in tensor memory
+    Tensor y = floats(z, shape), h = record ? floats(z, {m, kHidden}) : Tensor(), image = floats(z, {bytes / 4});
+    Tensor dz_image = dz_bytes ? floats(z, {dz_bytes / 4}) : Tensor();
+    check_status(npa_mlp_forward_tcgen05_images(fptr(z), fptr(w1), fptr(b1), fptr(w2), fmut(h), fmut(y), m, (int)k, (int)o, w1.stride(0), w1.stride(1),
+                                                w2.stride(0), w2.stride(1), image.mutable_data_ptr(), bytes, fmut(dz_image), dz_bytes,
+                                                stream_of(z)));
+    if (record) {
         auto n = node_for<MlpNode>(z, w1, b1, w2);
         n->z_ = SavedVariable(z, false); n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
-        n->h = h; n->z_shape = z.sizes().vec();
+        n->h = h; n->dz_image = dz_image; n->z_shape = z.sizes().vec();
         torch::autograd::set_history(y, n);
     }
     return y;

@@ -414,7 +414,7 @@ class StepUpdate:
 
     @staticmethod
     def apply(y, x_bin, s_bin, mask, snapshot, alpha, dt, wrap):
-        return _ops.step_update(snapshot.grid.native, y, x_bin, s_bin, mask, alpha, dt, wrap)
+        return _ops.step_update(snapshot.grid.native, y, x_bin, s_bin, mask, alpha, dt, wrap, -1.0)
 
 
 def step_update(y, x_bin, s_bin, snapshot, alpha, dt=1.0, update_mask=None, wrap=False):
@@ -429,3 +429,9 @@ def step_update(y, x_bin, s_bin, snapshot, alpha, dt=1.0, update_mask=None, wrap
         update_mask = update_mask.reshape(y.shape[0], y.shape[1]).to(torch.float32).contiguous()
     return StepUpdate.apply(y.contiguous(), x_bin.contiguous(), s_bin.contiguous(), update_mask, snapshot,
                             float(alpha), float(dt), bool(wrap))
+
+
+def step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_prob, wrap=False):
+    """``step_update`` with ``update_mask = (uniforms < update_prob).float()``, the comparison made in the kernel."""
+    return _ops.step_update(snapshot.grid.native, y.contiguous(), x_bin.contiguous(), s_bin.contiguous(),
+                            uniforms.reshape(y.shape[0], y.shape[1]), float(alpha), float(dt), bool(wrap), float(update_prob))

@@ -18,6 +18,7 @@ import math
 import torch
 
 from . import sphops as sph
+from .sphops import sph as sph_ops
 from .mlp import apply_mlp
 
 
@@ -94,11 +95,13 @@ def step_euler(model, x, s, grid, dt=1.0, update_prob=0.5, intermediate=False, n
         dx = _buffer_scalar(model, "alpha") * d * grid.eps / (1.0 + d.norm(dim=-1, keepdim=True))
         stats = {"dx_norm": dx.norm(dim=-1).mean()}
 
-    update_mask = None
-    if update_prob < 1.0:
-        update_mask = (torch.rand(B, N, 1, device=x.device) < update_prob).float()
-    x_new, s_new = sph.step_update(y, x_bin, s_bin, snapshot, _buffer_scalar(model, "alpha"), dt, update_mask, wrap)
+    alpha = _buffer_scalar(model, "alpha")
+    uniforms = torch.rand(B, N, 1, device=x.device) if update_prob < 1.0 else None
+    if uniforms is None:
+        x_new, s_new = sph.step_update(y, x_bin, s_bin, snapshot, alpha, dt, None, wrap)
+    else:
+        x_new, s_new = sph_ops.step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_prob, wrap)
     if noise_std > 0:
         noise = torch.randn_like(x_new) * noise_std * math.sqrt(dt)
-        x_new = x_new + (noise * update_mask if update_mask is not None else noise)
+        x_new = x_new + (noise if uniforms is None else noise * (uniforms < update_prob).float())
     return x_new, s_new, stats
