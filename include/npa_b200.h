@@ -376,7 +376,8 @@ int npa_perceive_features_backward(const npa_grid *g, int32_t channels, const fl
  *   packed   [B*N, 4] floats, 16-byte aligned: (x, y, z, m / rho) of every particle, written by the forward calls and
  *            read by the sweeps after it; may be NULL;
  *   scratch  npa_lists_backward_scratch_bytes(g, channels) bytes, 16-byte aligned, private to the call.
- * No block_info is needed where it is not an argument.  Same results as the calls they stand for. */
+ * No block_info is needed where it is not an argument.  Same results as the calls they stand for; grad_s_add [B,N,C]
+ * (or NULL) is added to grad_s. */
 int64_t npa_lists_backward_scratch_bytes(const npa_grid *g, int32_t channels);
 int npa_perception_forward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass, const float *s_bin,
                                  float *rho, float *rho_grad, float *s_blur, float *s_grad, float *packed,
@@ -407,7 +408,8 @@ int npa_perceive_features_forward_lists(const npa_grid *g, int32_t channels, con
 int npa_perceive_features_backward_lists(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
                                          const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
                                          const float *packed, const float *dL_dz, float coef, float dg_scale,
-                                         int32_t log_norm_grad, int32_t log_norm_dg, float *grad_x, float *grad_s,
+                                         int32_t log_norm_grad, int32_t log_norm_dg, const float *grad_s_add,
+                                         float *grad_x, float *grad_s,
                                          void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
                                          const int32_t *pair_cache, int32_t pair_stride, void *stream);
 

@@ -742,6 +742,11 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
                 for (int q = 0; q < 4; ++q)
                     if (f0 + q < C) o[q] += __ldg(z + f0 + q);
             }
+            if (a.add && ivalid) {
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (f0 + q < C) o[q] += __ldg(a.add + (long long)i * C + f0 + q);
+            }
             if (ivalid) store_row4<VEC>(a.grad_s + (long long)i * C, f0, C, o);
         }
     }

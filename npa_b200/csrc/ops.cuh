@@ -103,6 +103,7 @@ struct FeatureListBwdArgs {
     int gb_pitch, gg_pitch, cp;
     const float *direct;      // rows of direct_pitch floats added to grad_s, or NULL
     int direct_pitch;
+    const float *add;         // [B,N,C] added to grad_s, or NULL
     const float *g_dg;        // upstream of the density gradient [B,N,D] (its part of grad_x is added), or NULL
     const float *g_rho;       // upstream of the density [B,N], or NULL: only goes into pg
     float *grad_x, *grad_s, *grad_rho;

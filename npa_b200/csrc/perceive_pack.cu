@@ -162,8 +162,8 @@ int64_t npa_lists_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
 int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
                                          const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
                                          const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
-                                         int32_t log_norm_dg, float *grad_x, float *grad_s, void *scratch, int64_t scratch_bytes,
-                                         const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+                                         int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
+                                         int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
     const char *me = "perceive_features_backward_lists";
     Geom g;
     int rc = make_geom(gd, &g);
@@ -195,6 +195,7 @@ int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, c
     a.x = x_bin; a.mass = mass; a.rho = rho; a.s = s_bin; a.pv = reinterpret_cast<const float4 *>(packed);
     a.gb = rows; a.gg = rows + cp; a.gb_pitch = a.gg_pitch = pitch; a.cp = cp;
     a.direct = dL_dz; a.direct_pitch = 2 * channels + channels * g.dim + g.dim;  // the features enter z unchanged as its first columns
+    a.add = grad_s_add;
     a.g_dg = grad_x ? g_dg : nullptr;
     a.grad_x = grad_x; a.grad_s = grad_s; a.pg = grad_x ? pg : nullptr; a.C = channels;
     a.bin_offsets = bin_offsets; a.pair_cache = pair_cache; a.pair_stride = pair_stride;

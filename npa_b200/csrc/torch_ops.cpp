@@ -84,6 +84,11 @@ struct Grid {
         require(offs, {B * cells + 1}, "bin_offsets", at::kInt);
         require(info, {max_blocks, 4}, "block_info", at::kInt);
     }
+    void bin(const Tensor &x, const Tensor &perm, const Tensor &offs, const Tensor &info, void *st) {
+        if (!scratch.defined() || scratch.device() != x.device())
+            scratch = at::empty({scratch_bytes}, at::TensorOptions().dtype(at::kByte).device(x.device()));
+        check_status(npa_grid_build(&g, fptr(x), imut(perm), imut(offs), imut(info), scratch.mutable_data_ptr(), scratch_bytes, st));
+    }
     void features(const Tensor &s, const char *name) const { require(s, {B, N, s.dim() == 3 ? s.size(2) : -1}, name); }
 };
 using GridPtr = std::shared_ptr<Grid>;
@@ -94,9 +99,7 @@ py::tuple instantiate(const GridPtr &grid, const Tensor &x) {
     c10::cuda::CUDAGuard guard(x.device());
     const auto ints = at::TensorOptions().dtype(at::kInt).device(x.device());
     Tensor perm = at::empty({g.B, g.N}, ints), offs = at::empty({g.B * g.cells + 1}, ints), info = at::empty({g.max_blocks, 4}, ints);
-    if (!g.scratch.defined() || g.scratch.device() != x.device())
-        g.scratch = at::empty({g.scratch_bytes}, at::TensorOptions().dtype(at::kByte).device(x.device()));
-    check_status(npa_grid_build(&g.g, fptr(x), imut(perm), imut(offs), imut(info), g.scratch.mutable_data_ptr(), g.scratch_bytes, stream_of(x)));
+    g.bin(x, perm, offs, info, stream_of(x));
     return py::make_tuple(offs, perm, info);
 }
 
@@ -479,7 +482,7 @@ struct PackedNode : SweepNode {
         if (pairs.defined()) {
             Tensor work = list_scratch(*grid, s, s.size(2)), gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
             check_status(npa_perceive_features_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad),
-                                                              fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, fmut(gx), fmut(gs),
+                                                              fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, nullptr, fmut(gx), fmut(gs),
                                                               work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
                                                               stream_of(x)));
             return {gx, gs};
@@ -580,6 +583,22 @@ py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, con
 // ---- the adaptation MLP on the tensor-memory kernels (mlp.py) -------------------------------------------------
 constexpr int kHidden = 128;
 
+// Gradients of the MLP's weights and bias from one kernel over the rows.
+void mlp_weight_grads(const Tensor &z, const Tensor &dh, const Tensor &h, const Tensor &dy, const Tensor &w1, const Tensor &w2, Tensor &gw1,
+                      Tensor &gb1, Tensor &gw2, void *st) {
+    const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
+    gw1 = at::empty_strided(w1.sizes(), at::IntArrayRef({k, (int64_t)1}), w1.options().requires_grad(false));
+    gw2 = at::empty_strided(w2.sizes(), at::IntArrayRef({(int64_t)kHidden, (int64_t)1}), w2.options().requires_grad(false));
+    gb1 = floats(z, {kHidden});
+    // the tensor-memory kernel appends a column of ones to z, 176 columns in all
+    const bool tensor = k < 176;
+    const int64_t count = tensor ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o)
+                                 : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
+    Tensor scratch = floats(z, {count});
+    check_status((tensor ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(fptr(z), fptr(dh), fptr(h), fptr(dy), m, (int)k, kHidden, (int)o,
+                                                                              fmut(scratch), count, fmut(gw1), fmut(gw2), fmut(gb1), st));
+}
+
 struct MlpNode : Node {
     SavedVariable z_, w1_, w2_;
     Tensor h, dz_image;  // hidden layer; W1 as the tensor cores read it for dz = dh W1
@@ -600,16 +619,7 @@ struct MlpNode : Node {
         }
         const bool n1 = should_compute_output(1), nb = should_compute_output(2), n2 = should_compute_output(3);
         if (n1 || nb || n2) {
-            gw1 = at::empty_strided(w1.sizes(), at::IntArrayRef({k, (int64_t)1}), w1.options().requires_grad(false));
-            gw2 = at::empty_strided(w2.sizes(), at::IntArrayRef({(int64_t)kHidden, (int64_t)1}), w2.options().requires_grad(false));
-            gb1 = floats(z, {kHidden});
-            // the tensor-memory kernel appends a column of ones to z, 176 columns in all
-            const bool tensor = k < 176;
-            const int64_t count = tensor ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o)
-                                         : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
-            Tensor scratch = floats(z, {count});
-            check_status((tensor ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(fptr(z), fptr(dh), fptr(h), fptr(dy), m, (int)k, kHidden, (int)o,
-                                                                                      fmut(scratch), count, fmut(gw1), fmut(gw2), fmut(gb1), st));
+            mlp_weight_grads(z, dh, h, dy, w1, w2, gw1, gb1, gw2, st);
         }
         return {gz, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
     }
@@ -641,6 +651,115 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
         torch::autograd::set_history(y, n);
     }
     return y;
+}
+
+// ---- a whole Euler step as one node ------------------------------------------------------------------------------
+// Binning, reorder, packed perception, MLP and update of stepping.step_euler: the same kernels as the operators above, but
+// one crossing from Python and one node.  Four nodes cost ~60 us of host time more per training step (graph bookkeeping,
+// the engine's hand-over between nodes, and the addition of the two gradients of the reordered states, which here rides
+// the perception's backward).
+struct EulerNode : Node {
+    GridPtr grid;
+    SavedVariable w1_, w2_;
+    Tensor offs, perm, pairs, x_bin, s_bin, rho, rho_grad, vgrad, packed, z, h, y, dz_image, mask;
+    float coef, dg_scale, alpha, dt, below;
+    bool ln_grad, ln_dg, stop_pos, stop_state;
+
+    variable_list apply(variable_list &&g) override {
+        const Tensor w1 = w1_.unpack(), w2 = w2_.unpack();  // raise when the graph was released
+        const Tensor gx_new = solid(g[0]), gs_new = solid(g[1]);
+        if (!gx_new.defined() && !gs_new.defined()) return variable_list(5);
+        c10::cuda::CUDAGuard guard(x_bin.device());
+        void *st = stream_of(x_bin);
+        npa_grid *gd = &grid->g;
+        const int64_t C = s_bin.size(2), k = z.size(-1), m = z.numel() / k, o = w2.size(0);
+        const bool nx = should_compute_output(0), ns = should_compute_output(1);
+        const bool n1 = should_compute_output(2), nb = should_compute_output(3), n2 = should_compute_output(4);
+        const bool back_x = nx && !stop_pos, back_s = ns && !stop_state;
+        // update
+        Tensor gy = blank(y);
+        check_status(mask.defined() ? npa_step_update_backward_masked(gd, fptr(y), fptr(mask), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fmut(gy), st)
+                                    : npa_step_update_backward(gd, fptr(y), nullptr, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fmut(gy), st));
+        // MLP
+        Tensor dh, gw1, gb1, gw2;
+        if (back_x || back_s || n1 || nb || n2) {
+            dh = floats(z, {m, kHidden});
+            check_status(npa_mlp_hidden_grad(fptr(gy), fptr(w2), fptr(h), fmut(dh), m, kHidden, (int)o, w2.stride(0), w2.stride(1), st));
+        }
+        if (n1 || nb || n2) mlp_weight_grads(z, dh, h, gy, w1, w2, gw1, gb1, gw2, st);
+        // perception, with the update's own gradient of the states added
+        Tensor gx_bin = gx_new, gs_bin = gs_new;
+        if (back_x || back_s) {
+            Tensor gz = blank(z);
+            check_status(npa_linear_tcgen05_prepared(fptr(dh), dz_image.const_data_ptr(), dz_image.numel() * 4, fmut(gz), m, kHidden, (int)k, st));
+            Tensor work = list_scratch(*grid, s_bin, C), gxp = back_x ? blank(x_bin) : Tensor(), gsp = back_s ? blank(s_bin) : Tensor();
+            check_status(npa_perceive_features_backward_lists(gd, (int)C, fptr(x_bin), nullptr, fptr(s_bin), fptr(rho), fptr(rho_grad), fptr(vgrad),
+                                                              fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, fptr(gs_new), fmut(gxp), fmut(gsp),
+                                                              work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs),
+                                                              (int)pairs.size(2), st));
+            if (back_s) gs_bin = gsp;
+            if (back_x) gx_bin = gx_bin.defined() ? gxp.add_(gx_bin) : gxp;
+        }
+        // back into the order of the inputs
+        Tensor gx, gs;
+        if (nx && !gx_bin.defined()) gx_bin = at::zeros_like(x_bin);
+        if (ns && !gs_bin.defined()) gs_bin = at::zeros_like(s_bin);
+        if (nx) gx = blank(x_bin);
+        if (ns) gs = blank(s_bin);
+        if (nx || ns)
+            check_status(npa_unbin_particles(gd, (int)C, nx ? fptr(gx_bin) : nullptr, ns ? fptr(gs_bin) : nullptr, nullptr, iptr(perm), fmut(gx), fmut(gs),
+                                             nullptr, st));
+        return {gx, gs, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
+    }
+    void release_variables() override {
+        w1_.reset_data(); w2_.reset_data();
+        pairs = x_bin = s_bin = rho = rho_grad = vgrad = packed = z = h = y = dz_image = mask = Tensor();
+    }
+};
+
+// (x_new, s_new, bin_offsets, permutation, block_info, uniforms or None)
+py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, const Tensor &w1, const Tensor &b1, const Tensor &w2, double coef,
+                     double dg_scale, double inv_tol, bool ln_grad, bool ln_dg, bool stop_pos, bool stop_state, double alpha, double dt,
+                     double update_prob, bool wrap, int64_t columns) {
+    Grid &g = *grid;
+    g.positions(x, "positions");
+    g.features(s, "input_state");
+    c10::cuda::CUDAGuard guard(x.device());
+    void *st = stream_of(x);
+    const int64_t C = s.size(2), D = g.D, k = 2 * C + C * D + D, o = D + C, m = g.B * g.N;
+    const bool record = recording(x, s, w1, b1, w2);
+    const bool back = record && ((wants_grad(x) && !stop_pos) || (wants_grad(s) && !stop_state));  // a backward reaches the perception
+    const auto ints = at::TensorOptions().dtype(at::kInt).device(x.device());
+    Tensor perm = at::empty({g.B, g.N}, ints), offs = at::empty({g.B * g.cells + 1}, ints), info = at::empty({g.max_blocks, 4}, ints);
+    Tensor x_bin = blank(x), s_bin = blank(s), rho = floats(x, {g.B, g.N}), rho_grad = floats(x, {g.B, g.N, D}), z = floats(s, {g.B, g.N, k});
+    Tensor vgrad = back ? floats(s, {g.B, g.N, C, D}) : Tensor(), pairs = new_lists(g, x, columns), packed = floats(x, {g.B, g.N, 4});
+    grid->bin(x, perm, offs, info, st);
+    check_status(npa_bin_particles(&g.g, (int)C, fptr(x), fptr(s), nullptr, iptr(perm), fmut(x_bin), fmut(s_bin), nullptr, st));
+    check_status(npa_perceive_features_forward_lists(&g.g, (int)C, fptr(x_bin), nullptr, fptr(s_bin), (float)coef, (float)dg_scale, (float)inv_tol,
+                                                     ln_grad, ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), fmut(packed), iptr(offs),
+                                                     iptr(info), imut(pairs), (int)columns, st));
+    const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), dz_bytes = back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
+    Tensor y = floats(s, {g.B, g.N, o}), h = record ? floats(s, {m, kHidden}) : Tensor(), image = floats(s, {bytes / 4});
+    Tensor dz_image = dz_bytes ? floats(s, {dz_bytes / 4}) : Tensor();
+    check_status(npa_mlp_forward_tcgen05_images(fptr(z), fptr(w1), fptr(b1), fptr(w2), fmut(h), fmut(y), m, (int)k, (int)o, w1.stride(0), w1.stride(1),
+                                                w2.stride(0), w2.stride(1), image.mutable_data_ptr(), bytes, fmut(dz_image), dz_bytes, st));
+    Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();
+    Tensor xo = blank(x), so = blank(s);
+    check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, fptr(y), fptr(x_bin), fptr(s_bin), fptr(mask), (float)update_prob, (int)C,
+                                                                 (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st)
+                                : npa_step_update_forward(&g.g, fptr(y), fptr(x_bin), fptr(s_bin), nullptr, (int)C, (float)alpha, (float)dt, wrap,
+                                                          fmut(xo), fmut(so), st));
+    if (record) {
+        auto n = node_for<EulerNode>(x, s, w1, b1, w2);
+        n->grid = grid; n->offs = offs; n->perm = perm; n->pairs = pairs; n->x_bin = x_bin; n->s_bin = s_bin; n->rho = rho; n->rho_grad = rho_grad;
+        n->vgrad = vgrad; n->packed = packed; n->z = z; n->h = h; n->y = y; n->dz_image = dz_image; n->mask = mask;
+        n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
+        n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
+        n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;
+        torch::autograd::set_history(xo, n);
+        torch::autograd::set_history(so, n);
+    }
+    return py::make_tuple(xo, so, offs, perm, info, mask.defined() ? py::cast(mask) : py::none());
 }
 
 // ---- splat renderer ------------------------------------------------------------------------------------------
@@ -698,5 +817,6 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("packed_perception", &packed_perception);
     m.def("step_update", &step_update);
     m.def("mlp", &mlp);
+    m.def("euler_step", &euler_step);
     m.def("splat", &splat);
 }

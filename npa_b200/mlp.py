@@ -123,6 +123,11 @@ def supported(module) -> bool:
     return l1.weight.is_cuda and l1.weight.dtype == torch.float32 and l2.weight.dtype == torch.float32
 
 
+def on_tensor_memory(module) -> bool:
+    """Whether ``apply_mlp(module, z)`` runs on the tensor-memory kernels end to end (the default engine)."""
+    return TENSOR_ENGINE == "tcgen05" and FUSED_FORWARD and FUSED_HIDDEN_GRAD and supported(module)
+
+
 def apply_mlp(module, z):
     """``module(z)``; with the fused weight-gradient backward when ``supported(module)``."""
     if not (supported(module) and z.is_cuda and z.dtype == torch.float32):

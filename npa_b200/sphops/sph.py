@@ -92,7 +92,10 @@ class HashGrid:
 
     def instantiate(self, x):
         """Bin positions ``x [B, N, P]`` and return the snapshot the operators take."""
-        bin_offsets, permutation, block_info = _ops.instantiate(self.hashgrid.native, x)
+        return self.adopt(*_ops.instantiate(self.hashgrid.native, x))
+
+    def adopt(self, bin_offsets, permutation, block_info):
+        """The snapshot of a binning pass whose arrays are there already."""
         # outputs a fused sweep parked on the previous snapshot and nobody claimed, and its neighbour lists, are
         # dropped now: they would otherwise live (with the autograd graph they hang on) as long as that snapshot does
         previous = self._last_snapshot() if self._last_snapshot is not None else None
@@ -375,6 +378,11 @@ class PerceiveFeatures:
                                       _columns(snapshot.grid))
 
 
+def packable(C):
+    """Whether one warp pass of the packed sweep covers rows of ``C`` features."""
+    return (C % 4 == 0 and C <= 128) or C <= 32
+
+
 def perceive_features(x_bin, s_bin, snapshot, eps0, mass=None, log_norm_grad=True, log_norm_density_grad=True,
                       inv_rtol=1e-3):
     """The perception vector ``z [B, N, 2C + C*dim + dim]`` an NPA model feeds its MLP, in two sweeps.
@@ -388,7 +396,7 @@ def perceive_features(x_bin, s_bin, snapshot, eps0, mass=None, log_norm_grad=Tru
     B, N, C = s_bin.shape
     coef = float(snapshot.grid.eps) / float(eps0)
     dg_scale = coef ** (1 + snapshot.dim) / N
-    if not ((C % 4 == 0 and C <= 128) or C <= 32):
+    if not packable(C):
         # wider feature rows than one warp pass covers: same result from the separate operators
         def _ln(v):
             return torch.log(1.0 + v.norm(dim=-1, keepdim=True)) * torch.nn.functional.normalize(v, dim=-1)
@@ -435,3 +443,15 @@ def step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_pro
     """``step_update`` with ``update_mask = (uniforms < update_prob).float()``, the comparison made in the kernel."""
     return _ops.step_update(snapshot.grid.native, y.contiguous(), x_bin.contiguous(), s_bin.contiguous(),
                             uniforms.reshape(y.shape[0], y.shape[1]), float(alpha), float(dt), bool(wrap), float(update_prob))
+
+
+def euler_step(grid, x, s, weights, eps0, alpha, dt, update_prob, wrap, log_norm_grad, log_norm_density_grad, stopgrad_pos,
+               stopgrad_state, inv_rtol=1e-3):
+    """``instantiate``, ``bin_particles``, ``perceive_features``, the MLP ``weights`` = (W1, b1, W2) and ``step_update`` as
+    one call and one autograd node: ``(x_new, s_new, snapshot, uniforms of the update mask or None)``."""
+    coef = float(grid.eps) / float(eps0)
+    x_new, s_new, bin_offsets, permutation, block_info, uniforms = _ops.euler_step(
+        grid.hashgrid.native, x, s, *weights, coef, coef ** (1 + grid.dim) / x.shape[1], float(inv_rtol), bool(log_norm_grad),
+        bool(log_norm_density_grad), bool(stopgrad_pos), bool(stopgrad_state), float(alpha), float(dt), float(update_prob), bool(wrap),
+        _columns(grid.hashgrid))
+    return x_new, s_new, grid.adopt(bin_offsets, permutation, block_info), uniforms

@@ -452,7 +452,7 @@ class _HashGridBase:
             self._call(_lib.npa_perceive_features_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
                        N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(density_gradient), N.ptr(corrected_gradient), None,
                        N.ptr(dL_dz), float(coef), float(dg_scale), 1 if log_norm_grad else 0, 1 if log_norm_dg else 0,
-                       N.ptr(grad_x), N.ptr(grad_s), N.ptr(scratch[0]), scratch[1], N.ptr(bin_offsets), *pairs)
+                       None, N.ptr(grad_x), N.ptr(grad_s), N.ptr(scratch[0]), scratch[1], N.ptr(bin_offsets), *pairs)
             return
         self._call(_lib.npa_perceive_features_backward, binned_positions, self._ref(), C, N.ptr(binned_positions),
                    N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(density_gradient), N.ptr(corrected_gradient),

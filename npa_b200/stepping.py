@@ -19,7 +19,7 @@ import torch
 
 from . import sphops as sph
 from .sphops import sph as sph_ops
-from .mlp import apply_mlp
+from .mlp import apply_mlp, on_tensor_memory
 
 
 def _scalar(v) -> float:
@@ -78,6 +78,16 @@ def perceive(model, x, s, grid):
     return z, x_bin, s_bin, snapshot
 
 
+def _one_node(model, x, s, grid) -> bool:
+    """Whether a step of this model is covered by the single autograd node: the adaptation MLP on the default
+    engine, gradient features on, rows one warp pass covers, neighbour lists on."""
+    C, module = s.shape[-1], model.model
+    return (getattr(model, "state_grad", True) and getattr(model, "density_grad", True) and sph_ops.packable(C)
+            and sph_ops._columns(grid.hashgrid) > 0 and on_tensor_memory(module)
+            and module[0].weight.device == x.device and module[0].in_features == 2 * C + C * grid.dim + grid.dim
+            and module[2].out_features == grid.dim + C)
+
+
 def step_euler(model, x, s, grid, dt=1.0, update_prob=0.5, intermediate=False, noise_std=0.0, wrap=False):
     """``x, s, stats`` after one step; the particles come back in cell order, as in the reference.
 
@@ -85,22 +95,27 @@ def step_euler(model, x, s, grid, dt=1.0, update_prob=0.5, intermediate=False, n
     after the rollout, train.py:238); the 3D padding column is kept either way.
     """
     B, N, C = s.shape
-    z, x_bin, s_bin, snapshot = perceive(model, x, s, grid)
-    model.last_snapshot = snapshot
-    y = apply_mlp(model.model, z)  # (B, N, dim + C); torch GEMMs, fused weight-gradient kernel in the backward
-
-    stats = None
-    if intermediate:
-        d = y[..., : model.spatial_dims]
-        dx = _buffer_scalar(model, "alpha") * d * grid.eps / (1.0 + d.norm(dim=-1, keepdim=True))
-        stats = {"dx_norm": dx.norm(dim=-1).mean()}
-
     alpha = _buffer_scalar(model, "alpha")
-    uniforms = torch.rand(B, N, 1, device=x.device) if update_prob < 1.0 else None
-    if uniforms is None:
-        x_new, s_new = sph.step_update(y, x_bin, s_bin, snapshot, alpha, dt, None, wrap)
+    stats = None
+    if not intermediate and _one_node(model, x, s, grid):
+        mlp = model.model
+        x_new, s_new, model.last_snapshot, uniforms = sph_ops.euler_step(
+            grid, x, s, (mlp[0].weight, mlp[0].bias, mlp[2].weight), _buffer_scalar(model, "eps0"), alpha, dt, update_prob, wrap,
+            getattr(model, "log_norm_grad", True), getattr(model, "log_norm_density_grad", True),
+            getattr(model, "stopgrad_pos", True), getattr(model, "stopgrad_state", False))
     else:
-        x_new, s_new = sph_ops.step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_prob, wrap)
+        z, x_bin, s_bin, snapshot = perceive(model, x, s, grid)
+        model.last_snapshot = snapshot
+        y = apply_mlp(model.model, z)  # (B, N, dim + C)
+        if intermediate:
+            d = y[..., : model.spatial_dims]
+            dx = alpha * d * grid.eps / (1.0 + d.norm(dim=-1, keepdim=True))
+            stats = {"dx_norm": dx.norm(dim=-1).mean()}
+        uniforms = torch.rand(B, N, 1, device=x.device) if update_prob < 1.0 else None
+        if uniforms is None:
+            x_new, s_new = sph.step_update(y, x_bin, s_bin, snapshot, alpha, dt, None, wrap)
+        else:
+            x_new, s_new = sph_ops.step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_prob, wrap)
     if noise_std > 0:
         noise = torch.randn_like(x_new) * noise_std * math.sqrt(dt)
         x_new = x_new + (noise if uniforms is None else noise * (uniforms < update_prob).float())
