@@ -591,13 +591,10 @@ int npa_tile_status(int32_t *host_status, int32_t reset);
  * != 0, clears them.  Synchronises the device: call it after an error status, never in the timed path
  * or during stream capture. */
 int npa_row_tickets_status(int32_t *host_nonzero_words, int32_t reset);
-/* The forward sweeps of the scalar operators (count, density, density gradient, moment matrix) on a
- * linear-hash grid let the particles of a tile -- work items of up to cells_per_tile x-adjacent
- * cells, at most 32 particles -- share the candidates they test (the sharing of a staged cell among
- * the threads of a block in sphops/sph_cuda.cu:1664-1690).  Used for the poly6 operators (count,
- * density) on clamped grids and 2D periodic grids, where it is measured faster; adding 100 forces it
- * on 3D periodic grids too.  cells_per_tile = 0 switches back to the per-particle candidate walk;
- * default 3.  Process-wide. */
+/* The count and density forward sweeps let the particles of a work item share the candidates they test (the
+ * sharing of a staged cell among the threads of a block in sphops/sph_cuda.cu:1664-1690).  cells_per_tile = 0
+ * switches to the per-particle candidate walk, any other accepted value (1..8, 101..108) back; default 3.
+ * Process-wide. */
 int npa_scalar_sweep_tuning(int32_t cells_per_tile);
 /* Self-test of the bounded waits: one CTA waits for an mbarrier phase that is never completed and
  * writes to *device_result (int32, device memory) 1 when the wait gave up after limit_us

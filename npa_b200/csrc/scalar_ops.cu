@@ -154,232 +154,6 @@ scalar_forward_kernel(ScalarFwdArgs a, Geom g) {
     release_rows(a.tickets);
 }
 
-// ---------------------------------------------------------------------------
-// Forward sweep with the candidates shared by the particles of a tile.
-//
-// The particles of one cell (and of its x-neighbours) test the same candidates, so a warp takes a
-// tile of up to 32 particles -- consecutive work-list rows of one x-row of cells, at most `span`
-// cells apart (sphops/sph_cuda.cu:1664-1690 shares a staged cell among the threads of a block in the
-// same way) -- gives every particle one lane, loads 32 candidates at a time into shared memory and
-// lets every lane test each of them against its own particle: a candidate position is loaded once
-// per tile instead of once per particle, every lane accumulates its own sums (no reductions), and
-// the test costs ~a dozen instructions per candidate for all particles of the tile together.
-// Linear hash only (the cells of an x-row must be contiguous); same outputs, same neighbour lists
-// (candidate order) as scalar_forward_kernel.
-// ---------------------------------------------------------------------------
-constexpr int kSharedBatch = 8;  // most work-list rows a warp draws per ticket
-
-template <int D, bool PER, int MASK>
-__global__ void __launch_bounds__(kWarpsPerCta * 32)
-scalar_forward_shared_kernel(ScalarFwdArgs a, Geom g, int span, int batch) {
-    __shared__ int4 s_ranges[kWarpsPerCta][kMaxRanges];
-    __shared__ float4 s_cand[kWarpsPerCta][2][32];  // x, y, z, mass of the staged candidates (two batches)
-    __shared__ float s_vol[kWarpsPerCta][2][32];    // m / rho of the staged candidates (moment matrix only)
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    int4 *rng = s_ranges[warp];
-    constexpr bool kSpiky = (MASK & (S_DGRAD | S_MOMENT)) != 0;
-    constexpr bool kPoly = (MASK & S_DENSITY) != 0;
-    // the neighbour count must agree bit for bit with the fp32 oracle on borderline pairs (r^2 without
-    // fused multiply-adds); every other output is continuous at the cut-off
-    constexpr bool kExact = (MASK & S_COUNT) != 0;
-    // density alone on a clamped grid: two candidates per step in packed fp32x2 arithmetic (the staged
-    // candidates are kept as four arrays x[32] y[32] z[32] m[32], so that a pair is one 8-byte broadcast)
-    constexpr bool kPacked = !PER && MASK == S_DENSITY;
-    const int K = a.pair_stride;
-
-    bool finished = false;
-    while (!finished) {
-        int row = 0;
-        if (lane == 0) row = (int)atomicAdd(a.tickets, (unsigned)batch);
-        row = __shfl_sync(kFull, row, 0) + lane;
-        WorkItem mine = {0, 0, 0, 0};
-        int mcx = 0, mcy = 0, mcz = 0;
-        if (lane < batch && row < g.max_blocks) mine = load_item(a.block_info, a.bin_offsets, row);
-        if (mine.count > 0) hash_to_cell<D>(g, (uint32_t)(mine.cell - mine.sys * g.cells), mcx, mcy, mcz);
-        int next = 0;
-        while (next < batch) {
-            const int h = next;
-            const int hcount = __shfl_sync(kFull, mine.count, h);
-            if (hcount <= 0) {  // rows after the last work item are zero
-                finished = true;
-                break;
-            }
-            const int hfirst = __shfl_sync(kFull, mine.first, h);
-            const int hsys = __shfl_sync(kFull, mine.sys, h);
-            const int hcx = __shfl_sync(kFull, mcx, h), hcy = __shfl_sync(kFull, mcy, h), hcz = __shfl_sync(kFull, mcz, h);
-            // rows h, h+1, ... join the tile while they lie in the same x-row, within `span` cells, and the
-            // tile holds at most 32 particles (rows of one x-row are contiguous in memory)
-            const bool in_batch = lane >= h && lane < batch && mine.count > 0;
-            const int upto = in_batch ? mine.first + mine.count - hfirst : 0;
-            const bool wide = g.periodic && (mcx - hcx + 3 >= g.g[0]);
-            const bool okrow = in_batch && mine.sys == hsys && mcy == hcy && mcz == hcz && mcx >= hcx &&
-                               mcx - hcx < span && upto <= 32 && upto > 0 && (lane == h || !wide);
-            const unsigned okm = __ballot_sync(kFull, okrow || lane == h);
-            const unsigned run = ~okm & ~((1u << h) - 1u);
-            const int stop = run ? __ffs(run) - 1 : 32;
-            const int last = stop - 1;
-            const int lcx = __shfl_sync(kFull, mcx, last);
-            const int tile_count = __shfl_sync(kFull, mine.first + mine.count, last) - hfirst;
-            next = stop;
-            __syncwarp();
-            const int nr = build_ranges_span<D>(g, a.bin_offsets, hsys, hcx, lcx, hcy, hcz, rng);
-
-            for (int p0 = 0; p0 < tile_count; p0 += 32) {  // a lone row of more than 32 particles: passes of 32
-                const bool ivalid = p0 + lane < tile_count;
-                const long long i = hfirst + p0 + (ivalid ? lane : 0);
-                const Pos<D> pi = load_pos<D>(a.x, i);
-                int32_t *list = a.pair_cache ? a.pair_cache + i * K + 1 : nullptr;
-                float cnt = 0.f, rho = 0.f, dg[3] = {0.f, 0.f, 0.f}, mom[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-                unsigned long long rho2 = 0ull;  // kPacked: sums over the even and the odd candidates of the batches
-                int listed = 0;
-
-                // candidates are staged 32 at a time; the next batch is fetched from global memory while the
-                // current one is tested.  A batch is (range r, first candidate j0); this walks them in order.
-                auto fetch = [&](int r, int j0, float4 &c, float &v) {
-                    c = make_float4(0.f, 0.f, 0.f, 0.f);
-                    v = 0.f;
-                    if (r < nr) {
-                        const int j = j0 + lane;
-                        if (j < rng[r].y) {
-                            const Pos<D> pj = load_pos<D>(a.x, j);
-                            const float mj = a.mass ? __ldg(a.mass + j) : 1.0f;
-                            c = make_float4(pj.x, pj.y, pj.z, mj);
-                            if (MASK & S_MOMENT) v = mj / __ldg(a.rho_in + j);
-                        }
-                    }
-                };
-                int r = 0, j0 = nr > 0 ? rng[0].x : 0, buf = 0;
-                float4 c_next;
-                float v_next;
-                fetch(r, j0, c_next, v_next);
-                while (r < nr) {
-                    const int4 rg = rng[r];
-                    float4 *cand = s_cand[warp][buf];
-                    float *cvol = s_vol[warp][buf];
-                    if (kPacked) {
-                        float *cs = reinterpret_cast<float *>(cand);
-                        cs[lane] = c_next.x; cs[32 + lane] = c_next.y; cs[64 + lane] = c_next.z; cs[96 + lane] = c_next.w;
-                    } else {
-                        cand[lane] = c_next;
-                    }
-                    if (MASK & S_MOMENT) cvol[lane] = v_next;
-                    __syncwarp();
-                    // the batch after this one
-                    int rn = r, jn0 = j0 + 32;
-                    if (jn0 >= rg.y) {
-                        rn = r + 1;
-                        jn0 = rn < nr ? rng[rn].x : 0;
-                    }
-                    fetch(rn, jn0, c_next, v_next);
-                    if (kPacked && ivalid) {
-                        const unsigned long long *cs = reinterpret_cast<const unsigned long long *>(cand);
-                        const unsigned long long nox = pack2(-pi.x, -pi.x), noy = pack2(-pi.y, -pi.y), noz = pack2(-pi.z, -pi.z);
-                        const int jn = min(32, rg.y - j0);
-#pragma unroll 2
-                        for (int k = 0; k < jn; k += 2) {
-                            // candidates k and k + 1 (a batch that ends on an odd count is followed by a zero-mass entry)
-                            const unsigned long long rx = add2(cs[k >> 1], nox), ry = add2(cs[16 + (k >> 1)], noy);
-                            unsigned long long q = fma2(ry, ry, mul2(rx, rx));
-                            if (D == 3) {
-                                const unsigned long long rz = add2(cs[32 + (k >> 1)], noz);
-                                q = fma2(rz, rz, q);
-                            }
-                            float q0, q1;
-                            unpack2(q, q0, q1);
-                            const bool acc0 = q0 < g.h2, acc1 = q1 < g.h2 && k + 1 < jn;
-                            if (list) {
-                                if (acc0 && listed < K - 1) list[listed] = j0 + k;
-                                listed += acc0 ? 1 : 0;
-                                if (acc1 && listed < K - 1) list[listed] = j0 + k + 1;
-                                listed += acc1 ? 1 : 0;
-                            }
-                            const unsigned long long t = pack2(fmaxf(g.h2 - q0, 0.f), fmaxf(g.h2 - q1, 0.f));
-                            rho2 = fma2(cs[48 + (k >> 1)], mul2(mul2(t, t), t), rho2);
-                        }
-                    } else if (ivalid) {
-                        const Origin<D, PER> org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, rg.z);
-                        const int jn = min(32, rg.y - j0);
-#pragma unroll 4
-                        for (int k = 0; k < jn; ++k) {
-                            const float4 c = cand[k];  // same address in every lane: one broadcast
-                            float rx, ry, rz;
-                            const float q = displacement<D, PER, kExact>(g, org, c.x, c.y, c.z, rx, ry, rz);
-                            const bool acc = q < g.h2;
-                            if (list) {
-                                if (acc && listed < K - 1) list[listed] = j0 + k;
-                                listed += acc ? 1 : 0;
-                            }
-                            if (MASK & S_COUNT) cnt += acc ? 1.0f : 0.f;
-                            // both kernels vanish at the cut-off: no branch on `acc` is needed
-                            if (kPoly) {
-                                const float t = fmaxf(g.h2 - q, 0.f);
-                                rho = fmaf(c.w, t * t * t, rho);
-                            }
-                            if (kSpiky) {
-                                const Spiky sp = spiky_distance(q);
-                                const float phi = acc ? spiky_phi(sp, g.h) : 0.f;  // phi r = 0 for the self pair
-                                if (MASK & S_DGRAD) {
-                                    const float w = c.w * phi;
-                                    dg[0] = fmaf(w, rx, dg[0]);
-                                    dg[1] = fmaf(w, ry, dg[1]);
-                                    if (D == 3) dg[2] = fmaf(w, rz, dg[2]);
-                                }
-                                if (MASK & S_MOMENT) {
-                                    const float w = phi * cvol[k];
-                                    mom[0] = fmaf(w * rx, rx, mom[0]);
-                                    mom[1] = fmaf(w * rx, ry, mom[1]);
-                                    if (D == 2) {
-                                        mom[2] = fmaf(w * ry, ry, mom[2]);
-                                    } else {
-                                        mom[2] = fmaf(w * rx, rz, mom[2]);
-                                        mom[3] = fmaf(w * ry, ry, mom[3]);
-                                        mom[4] = fmaf(w * ry, rz, mom[4]);
-                                        mom[5] = fmaf(w * rz, rz, mom[5]);
-                                    }
-                                }
-                            }
-                        }
-                    }
-                    r = rn;
-                    j0 = jn0;
-                    buf ^= 1;
-                }
-                __syncwarp();
-                if (kPacked) {
-                    float lo, hi;
-                    unpack2(rho2, lo, hi);
-                    rho = lo + hi;
-                }
-                if (ivalid) {
-                    if (list) list[-1] = listed <= K - 1 ? listed : -1;
-                    if ((MASK & S_COUNT) && a.count) a.count[i] = cnt;
-                    if (kPoly && a.rho_out) {
-                    const float r = g.c_s * rho;
-                    a.rho_out[i] = r;
-                    if (a.pv) a.pv[i] = make_float4(pi.x, pi.y, pi.z, (a.mass ? __ldg(a.mass + i) : 1.0f) / r);
-                }
-                    if ((MASK & S_DGRAD) && a.rho_grad) {
-#pragma unroll
-                        for (int d = 0; d < D; ++d) a.rho_grad[i * D + d] = g.c_g * dg[d];
-                    }
-                    if ((MASK & S_MOMENT) && a.moment) {
-                        float *o = a.moment + i * (D * D);
-                        if (D == 2) {
-                            reinterpret_cast<float4 *>(o)[0] =
-                                make_float4(g.c_g * mom[0], g.c_g * mom[1], g.c_g * mom[1], g.c_g * mom[2]);
-                        } else {
-                            o[0] = g.c_g * mom[0]; o[1] = g.c_g * mom[1]; o[2] = g.c_g * mom[2];
-                            o[3] = g.c_g * mom[1]; o[4] = g.c_g * mom[3]; o[5] = g.c_g * mom[4];
-                            o[6] = g.c_g * mom[2]; o[7] = g.c_g * mom[4]; o[8] = g.c_g * mom[5];
-                        }
-                    }
-                }
-            }
-        }
-    }
-    release_rows(a.tickets);
-}
-
 // Gather backward of density / density gradient / moment matrix by the cell search, same layout (8
 // particles per warp pass, 4 lanes each); over neighbour lists it is scalar_list.cu.
 template <int D, bool PER, int MASK>
@@ -530,41 +304,14 @@ static int launch_persistent(const Geom &g, Kernel kernel, const Args &a, cudaSt
     return check_launch(what);
 }
 
-// Cells per tile of the shared-candidate forward sweep (0 = keep the per-particle kernel).
-static int g_shared_span = 3;
-void set_scalar_shared_span(int span) { g_shared_span = span; }
-
-template <typename Kernel>
-static int launch_shared(const Geom &g, Kernel kernel, const ScalarFwdArgs &a, cudaStream_t st) {
-    const int threads = kWarpsPerCta * 32;
-    int ctas = 0;
-    int rc = persistent_ctas(kernel, threads, 0, &ctas);
-    if (rc != NPA_OK) return rc;
-    // rows a warp draws per ticket: enough tickets for two rounds over the resident warps, at most kSharedBatch
-    // (consecutive rows of one ticket can merge into a tile; a single row cannot)
-    int batch = g.max_blocks / (2 * ctas * kWarpsPerCta);
-    batch = batch < 1 ? 1 : (batch > kSharedBatch ? kSharedBatch : batch);
-    const int needed = (g.max_blocks + batch * kWarpsPerCta - 1) / (batch * kWarpsPerCta);
-    ScalarFwdArgs b = a;
-    if ((rc = acquire_row_tickets(st, &b.tickets)) != NPA_OK) return rc;
-    kernel<<<needed < ctas ? (needed > 0 ? needed : 1) : ctas, threads, 0, st>>>(b, g, g_shared_span % 100, batch);
-    return check_launch("scalar_forward_shared_kernel");
-}
+static bool g_shared_search = true;  // count / density by density_search.cu
+void set_scalar_shared_search(bool on) { g_shared_search = on; }
+bool scalar_shared_search() { return g_shared_search; }
 
 template <int MASK>
 static int launch_scalar_fwd_mask(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
-    // Shared candidates need the cells of an x-row contiguous (linear hash).  Measured: the sweep of the
-    // poly6 operators (count, density) gains 30-40 % on clamped grids in 2D and 3D; with the spiky operators
-    // in the mask, and on 3D periodic grids, the per-particle walk is as fast or faster and stays.
-    constexpr bool kSpikyMask = (MASK & (S_DGRAD | S_MOMENT)) != 0;
-    if (!g.morton && g_shared_span > 0 && !kSpikyMask && (!g.periodic || g.dim == 2 || g_shared_span >= 100)) {
-        if (g.dim == 2) {
-            if (g.periodic) return launch_shared(g, scalar_forward_shared_kernel<2, true, MASK>, a, st);
-            return launch_shared(g, scalar_forward_shared_kernel<2, false, MASK>, a, st);
-        }
-        if (g.periodic) return launch_shared(g, scalar_forward_shared_kernel<3, true, MASK>, a, st);
-        return launch_shared(g, scalar_forward_shared_kernel<3, false, MASK>, a, st);
-    }
+    // the count or the density alone: the search that shares its candidates between particles
+    if ((MASK == S_DENSITY || (MASK == S_COUNT && !g.morton)) && g_shared_search) return launch_density_search(g, MASK == S_COUNT, a, st);
     const char *what = "scalar_forward_kernel";
     if (g.dim == 2) {
         if (g.periodic) return launch_persistent(g, scalar_forward_kernel<2, true, MASK>, a, st, what);

@@ -6,7 +6,7 @@
 
 namespace npa {
 
-void set_scalar_shared_span(int span);  // scalar_ops.cu
+void set_scalar_shared_search(bool on);  // scalar_ops.cu
 
 static int align_up(int v, int a) { return (v + a - 1) / a * a; }
 
@@ -128,8 +128,8 @@ int npa_tile_tuning(int32_t backward, int32_t enabled, int32_t rows_per_stage, i
 
 int npa_scalar_sweep_tuning(int32_t cells_per_tile) {
     if (cells_per_tile < 0 || (cells_per_tile > 8 && (cells_per_tile < 101 || cells_per_tile > 108)))
-        return fail(NPA_ERR_INVALID_ARGUMENT, "scalar_sweep_tuning: cells_per_tile must be in [0, 8] (+100: also on 3D periodic grids)");
-    set_scalar_shared_span(cells_per_tile);
+        return fail(NPA_ERR_INVALID_ARGUMENT, "scalar_sweep_tuning: cells_per_tile must be in [0, 8] or [101, 108]");
+    set_scalar_shared_search(cells_per_tile != 0);
     return NPA_OK;
 }
 
