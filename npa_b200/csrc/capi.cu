@@ -543,7 +543,7 @@ int npa_perception_forward(const npa_grid *gd, int32_t channels, const float *x_
     if (moment && g.dim == 2 && (uintptr_t)moment % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "perception_forward: moment must be 16-byte aligned");
     // with lists to record, the density alone takes the search and the density gradient walks the lists: less than half
-    // of the sweep that sums both while it searches (15,003 particles in 2D, ~32 neighbours: FUSED_ODD)
+    // of the sweep that sums both while it searches (15,003 particles in 2D, ~32 neighbours: 28 us against 15 + 5)
     const bool apart = pair_cache && rho_grad && !count && scalar_shared_search();
     ScalarFwdArgs sa = {x_bin, mass, nullptr, count, rho, apart ? nullptr : rho_grad, nullptr, bin_offsets, block_info, pair_cache, pair_stride};
     if ((rc = launch_scalar_forward(g, apart ? S_DENSITY : smask, sa, st)) != NPA_OK) return rc;

@@ -14,9 +14,9 @@
 // Both are bound by instruction issue: about 8 warp instructions per 32 tests in the first, 11 in the second, which
 // also spends as much again on its lists and on setting up an item.
 // Measured, B200, density + lists, us (before: a lane per particle with every list entry written as a word of its own,
-// and a walk per particle on Morton and 3D periodic grids): 262,144 particles 3D, ~240 candidates 140 -> SEARCH_A;
-// 524,288 particles 3D periodic 542 -> SEARCH_B; 65,536 particles 3D Morton, thin cells 61 -> SEARCH_C; 4,096 particles 2D
-// periodic, 370 candidates 45 -> SEARCH_D; 32,768 particles in 2D 20 -> SEARCH_E.
+// and a walk per particle on Morton and 3D periodic grids): 262,144 particles 3D, ~240 candidates 140 -> 98;
+// 524,288 particles 3D periodic 542 -> 311; 65,536 particles 3D Morton, thin cells 61 -> 45; 4,096 particles 2D
+// periodic, 370 candidates 45 -> 17; 32,768 particles in 2D 20 -> 14.
 #include "neighbors.cuh"
 #include "ops.cuh"
 
@@ -55,8 +55,9 @@ __device__ inline void item_cell(const Geom &g, uint32_t hsh, int &cx, int &cy, 
 // ---------------------------------------------------------------------------------------------------------
 // Linear hash: a lane per particle.
 // ---------------------------------------------------------------------------------------------------------
-constexpr int kTileWarps = 4;
+constexpr int kTileWarps = 2;
 constexpr int kTileSlots = 256;  // candidates staged at a time per warp; a slot number is a byte
+constexpr int Q = 2;             // lanes per particle, below
 constexpr int kTileRun = 132;    // bytes per lane for the slots accepted since the last flush (33 words: spread over the banks)
 
 // Signs of two differences r^2 - h^2 shifted into a word, the first candidate's bit ending up highest: the bit is set
@@ -74,9 +75,11 @@ template <bool MASS> struct TileStage {
     unsigned char run[32 * kTileRun];
 };
 
-// Q lanes share a particle (each takes every Q-th batch of 32 candidates): 32 / Q consecutive particles per warp.
-template <int D, bool PER, bool COUNT, bool MASS, int Q>
-__global__ void __launch_bounds__(kTileWarps * 32, 6)
+// Q lanes share a particle (each takes every Q-th batch of 32 candidates): 32 / Q consecutive particles per warp.  Fewer
+// particles span fewer cells and meet fewer candidates that none of them accepts, but set up more often: 262,144
+// particles in 3D took 105 / 98 / 126 us with Q = 1 / 2 / 4, 524,288 periodic 340 / 321 / 403, 32,768 in 2D 15.1 / 13.6 / 16.2.
+template <int D, bool PER, bool COUNT, bool MASS>
+__global__ void __launch_bounds__(kTileWarps * 32, 12)
 density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g) {
     constexpr int PT = 32 / Q;
     extern __shared__ __align__(16) unsigned char s_tile[];
@@ -121,7 +124,8 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
             if (lane >= o) incl += v;
         }
         const int total = __shfl_sync(kFull, incl, 31);
-        if (lane < nr) rng[lane].w = incl - (own.y - own.x);
+        const int ordinal = incl - (own.y - own.x);
+        if (lane < nr) rng[lane] = make_int4(own.x - ordinal, ordinal, own.z, own.y - own.x);
         const bool wrapped = PER && __any_sync(kFull, own.z != shift_code(0, 0, 0));
         // an axis too short to know the image of a cell: the half-box test decides pair by pair
         bool check = PER && (g.g[0] <= 3 || g.g[1] <= 2 || (D == 3 && g.g[2] <= 2) || cx1 - cx0 + 3 >= g.g[0]);
@@ -135,45 +139,80 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
             const int count = min(cap, total - c0), padded = (count + 32 * Q - 1) / (32 * Q) * (32 * Q);
             __syncwarp();
             bool outside = false;
-            auto stage = [&](int group) {  // `group` lanes per range
-                for (int r = lane / group; r < nr; r += 32 / group) {
-                    const int4 R = rng[r];
-                    const int e = min(R.y - R.x, c0 + count - R.w);
+            if (!PER) {
+                // every lane stages its slots of the chunk: the range of a slot is the last one that starts at or before it;
+                // all loads are in flight together (range by range the gather was a chain of round trips, a third of the time)
+                constexpr int kPer = kTileSlots / 32;
+                int from[kPer];
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) from[u] = 0;
+                for (int r = 0; r < nr; ++r) {
+                    const int4 R = rng[r];  // particle of ordinal 0 as if the range began there, ordinal of the first candidate
+#pragma unroll
+                    for (int u = 0; u < kPer; ++u) {
+                        from[u] = c0 + u * 32 + lane >= R.y ? R.x : from[u];
+                    }
+                }
+                Pos<D> p[kPer];
+                float mass[kPer];
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    const int k = u * 32 + lane, j = from[u] + c0 + k;
+                    const bool real = k < count;
+                    p[u] = Pos<D>{kFarAway, kFarAway, kFarAway};
+                    mass[u] = 0.f;
+                    from[u] = real ? j : 0;
+                    if (real) p[u] = load_pos<D>(a.x, j);
+                    if (MASS && real) mass[u] = __ldg(a.mass + j);
+                }
+#pragma unroll
+                for (int u = 0; u < kPer; ++u) {
+                    const int k = u * 32 + lane;
+                    if (k >= padded) break;
+                    S.x[k] = p[u].x; S.y[k] = p[u].y;
+                    if (D == 3) S.z[k] = p[u].z;
+                    S.j[k] = COUNT ? shift_code(0, 0, 0) : from[u];
+                    if (MASS) S.m[k] = mass[u];
+                }
+            } else {  // up to 27 ranges, with image shifts: range by range, `group` lanes each
+                auto stage = [&](int group) {
+                    for (int r = lane / group; r < nr; r += 32 / group) {
+                        const int4 R = rng[r];
+                        const int e = min(R.w, c0 + count - R.y);
 #pragma unroll 2
-                    for (int k = max(0, c0 - R.w) + lane % group; k < e; k += group) {
-                        const int j = R.x + k, slot = R.w + k - c0;
-                        Pos<D> p = load_pos<D>(a.x, j);
-                        if (PER) {
+                        for (int k = max(0, c0 - R.y) + lane % group; k < e; k += group) {
+                            const int j = R.x + R.y + k, slot = R.y + k - c0;
+                            Pos<D> p = load_pos<D>(a.x, j);
                             const float v[3] = {p.x, p.y, p.z};
 #pragma unroll
                             for (int d = 0; d < D; ++d) outside |= !(v[d] > box_lo[d] && v[d] < box_hi[d]);
+                            if (wrapped && !COUNT) {
+                                float lx, ly, lz = 0.f, hx, hy, hz = 0.f;
+                                shifted(g, 0, p.x, (R.z & 3) - 1, hx, lx);
+                                shifted(g, 1, p.y, ((R.z >> 2) & 3) - 1, hy, ly);
+                                if (D == 3) shifted(g, 2, p.z, ((R.z >> 4) & 3) - 1, hz, lz);
+                                p = Pos<D>{hx, hy, hz};
+                                S.x[kTileSlots / 2 + slot] = lx; S.y[kTileSlots / 2 + slot] = ly;
+                                if (D == 3) S.z[kTileSlots / 2 + slot] = lz;
+                            }
+                            S.x[slot] = p.x; S.y[slot] = p.y;
+                            if (D == 3) S.z[slot] = p.z;
+                            S.j[slot] = COUNT ? R.z : j;
+                            if (MASS) S.m[slot] = __ldg(a.mass + j);
                         }
-                        if (PER && wrapped && !COUNT) {
-                            float lx, ly, lz = 0.f, hx, hy, hz = 0.f;
-                            shifted(g, 0, p.x, (R.z & 3) - 1, hx, lx);
-                            shifted(g, 1, p.y, ((R.z >> 2) & 3) - 1, hy, ly);
-                            if (D == 3) shifted(g, 2, p.z, ((R.z >> 4) & 3) - 1, hz, lz);
-                            p = Pos<D>{hx, hy, hz};
-                            S.x[kTileSlots / 2 + slot] = lx; S.y[kTileSlots / 2 + slot] = ly;
-                            if (D == 3) S.z[kTileSlots / 2 + slot] = lz;
-                        }
-                        S.x[slot] = p.x; S.y[slot] = p.y;
-                        if (D == 3) S.z[slot] = p.z;
-                        S.j[slot] = COUNT ? R.z : j;
-                        if (MASS) S.m[slot] = __ldg(a.mass + j);
                     }
-                }
-            };
-            if (total > 20 * nr) stage(32);  // lanes per range by the mean length of the ranges
-            else stage(8);
-            for (int k = count + lane; k < padded; k += 32) {
-                S.x[k] = S.y[k] = kFarAway;
-                if (D == 3) S.z[k] = kFarAway;
-                S.j[k] = COUNT ? shift_code(0, 0, 0) : 0;
-                if (MASS) S.m[k] = 0.f;
-                if (PER && wrapped && !COUNT) {
-                    S.x[kTileSlots / 2 + k] = S.y[kTileSlots / 2 + k] = 0.f;
-                    if (D == 3) S.z[kTileSlots / 2 + k] = 0.f;
+                };
+                if (total > 20 * nr) stage(32);  // by the mean length of the ranges
+                else stage(8);
+                for (int k = count + lane; k < padded; k += 32) {
+                    S.x[k] = S.y[k] = kFarAway;
+                    if (D == 3) S.z[k] = kFarAway;
+                    S.j[k] = COUNT ? shift_code(0, 0, 0) : 0;
+                    if (MASS) S.m[k] = 0.f;
+                    if (wrapped && !COUNT) {
+                        S.x[kTileSlots / 2 + k] = S.y[kTileSlots / 2 + k] = 0.f;
+                        if (D == 3) S.z[kTileSlots / 2 + k] = 0.f;
+                    }
                 }
             }
             if (PER) check = check || __any_sync(kFull, outside);
@@ -234,7 +273,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                             }
                         }
                     } else {
-#pragma unroll
+#pragma unroll 4
                         for (int k = 0; k < 32; k += 4) {
                             const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(S.x + s0 + k), Y = *reinterpret_cast<const ulonglong2 *>(S.y + s0 + k);
                             ulonglong2 Z = make_ulonglong2(0ull, 0ull), LX = Z, LY = Z, LZ = Z, M = Z;
@@ -277,10 +316,12 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                     if (COUNT) {
                         found += __popc(m);
                     } else if (lists) {
-                        while (m) {
+                        // as many rounds as the fullest lane has neighbours here: no divergence
+                        for (int left_over = __reduce_max_sync(kFull, __popc(m)); left_over > 0; --left_over) {
                             const int b = __clz(m);
-                            m ^= 0x80000000u >> b;
-                            run[held++] = (unsigned char)(s0 + b);
+                            if (m) run[held] = (unsigned char)(s0 + b);
+                            held += m != 0u;
+                            m &= ~(0x80000000u >> (b & 31));
                         }
                         if (__any_sync(kFull, held > kTileRun - 4 - 32)) flush();
                     }
@@ -312,9 +353,9 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     }
 }
 
-template <int D, bool PER, bool COUNT, bool MASS, int Q>
+template <int D, bool PER, bool COUNT, bool MASS>
 static int launch_tile(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
-    const auto kernel = density_tile_kernel<D, PER, COUNT, MASS, Q>;
+    const auto kernel = density_tile_kernel<D, PER, COUNT, MASS>;
     const size_t dyn = sizeof(TileStage<MASS>) * kTileWarps;
     int unused = 0;
     const int rc = persistent_ctas(kernel, kTileWarps * 32, dyn, &unused);  // raises the shared-memory limit once
@@ -322,15 +363,6 @@ static int launch_tile(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     const long long per_cta = (long long)kTileWarps * (32 / Q), particles = (long long)g.B * g.N;
     kernel<<<(unsigned)((particles + per_cta - 1) / per_cta), kTileWarps * 32, dyn, st>>>(a, g);
     return check_launch("density_tile_kernel");
-}
-
-template <int D, bool PER, bool COUNT, bool MASS>
-static int launch_tile_split(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
-    // lanes per particle: enough warps to give every scheduler TILE_WANT of them while particles are scarce
-    const long long particles = (long long)g.B * g.N, want = 148ll * 4 * 3 * 32;
-    if (particles >= want) return launch_tile<D, PER, COUNT, MASS, 1>(g, a, st);
-    if (2 * particles >= want) return launch_tile<D, PER, COUNT, MASS, 2>(g, a, st);
-    return launch_tile<D, PER, COUNT, MASS, 4>(g, a, st);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -591,8 +623,8 @@ static int launch_search(const Geom &g, bool count, const ScalarFwdArgs &a, cuda
     // few particles: the item kernel's warps are shorter (2,500 particles in 2D 5.3 us against 8.4, 4,096 with 128
     // neighbours 17.5 against 27; 15,003 about equal, 32,768 18 against 15)
     if (g.morton || (!count && (long long)g.B * g.N < 16384)) return launch_item<D, PER>(g, a, st);
-    if (count) return launch_tile_split<D, PER, true, false>(g, a, st);
-    return a.mass ? launch_tile_split<D, PER, false, true>(g, a, st) : launch_tile_split<D, PER, false, false>(g, a, st);
+    if (count) return launch_tile<D, PER, true, false>(g, a, st);
+    return a.mass ? launch_tile<D, PER, false, true>(g, a, st) : launch_tile<D, PER, false, false>(g, a, st);
 }
 
 int launch_density_search(const Geom &g, bool count, const ScalarFwdArgs &a, cudaStream_t st) {

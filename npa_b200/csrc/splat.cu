@@ -83,7 +83,7 @@ __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
 // exponentials per particle and tile instead of 256), eight per thread; every half warp multiplies every 16th particle
 // into 8 x 2 pixels x 4 channels per thread in packed fp32x2; the 16 partial images are added in a fixed order.  Bound
 // by instruction issue (culling, factors and products about a third each).  8 systems of 4,096 particles, 256 x 256,
-// patches of 41 x 41: 201 -> SPLAT_FWD us.
+// patches of 41 x 41: 201 -> 123 us.
 constexpr int kSplatThreads = 256, kSplatCull = 4, kSplatChunk = 64, kSplatParts = 16, kSplatWarps = kSplatThreads / 32;
 
 struct SplatLists {
@@ -253,7 +253,7 @@ __device__ inline float warp_sum(float v) {
 // The weight is separable: a lane keeps one column of the patch, runs down its rows with the row factors from shared
 // memory and applies the column factor once at the end (2 (2r+1) exponentials per particle instead of (2r+1)^2).  The
 // last, narrow group of columns is dealt to the lanes several rows at a time.  Bound by the reads of the upstream image
-// (16 bytes per pixel of the patch, from L1 and L2).  8 x 4,096 particles, patches of 41 x 41: 158 -> SPLAT_BWD us.
+// (16 bytes per pixel of the patch, from L1 and L2).  8 x 4,096 particles, patches of 41 x 41: 158 -> 75 us.
 __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
     constexpr int kMost = 2 * kSplatMaxRadius + 1;
     __shared__ float2 s_y[8][kMost];  // row factor, row factor times t_y
