@@ -439,10 +439,10 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
     using S = ListShape<LPP>;
     __shared__ float4 s_k[kListWarps][2][S::kSlots];  // v_j (K.x, K.y, K.z, W)
     __shared__ int4 s_j[kListWarps][2][S::kIndexQuads];
-    extern __shared__ float4 s_dyn[];                 // F_PACK: the rows of z of a warp's particles
+    extern __shared__ float4 s_rows[];                 // F_PACK: the rows of z of a warp's particles
     const int warp = threadIdx.x >> 5, total = g.B * g.N, first = (blockIdx.x * kListWarps + warp) * S::PP;
     if (first >= total) return;
-    float *stage = reinterpret_cast<float *>(s_dyn) + ((MASK & F_PACK) ? (size_t)warp * ((S::PP * a.zstride + 3) & ~3) : 0);
+    float *stage = reinterpret_cast<float *>(s_rows) + ((MASK & F_PACK) ? (size_t)warp * ((S::PP * a.zstride + 3) & ~3) : 0);
     list_forward<D, PER, LPP, VEC, MASK, false>(a, g, s_k[warp], s_j[warp], stage);
     __syncwarp();
     const int i = min(first + (int)(threadIdx.x & 31) / LPP, total - 1);

@@ -1,0 +1,6 @@
+// Instantiates the packed perception sweep of recorded steps for dim 3, periodic boundary.
+#include "packed_ordered.cuh"
+
+namespace npa {
+template int launch_packed_ordered_geom<3, true>(const Geom &, const FeatureFwdArgs &, cudaStream_t);
+}  // namespace npa

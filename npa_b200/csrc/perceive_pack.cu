@@ -94,6 +94,20 @@ add_direct_kernel(const float *__restrict__ gz, float *__restrict__ grad_s, long
 
 using namespace npa;
 
+namespace npa {
+template <int D, bool PER>
+int launch_packed_ordered_geom(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st);
+extern template int launch_packed_ordered_geom<2, false>(const Geom &, const FeatureFwdArgs &, cudaStream_t);
+extern template int launch_packed_ordered_geom<2, true>(const Geom &, const FeatureFwdArgs &, cudaStream_t);
+extern template int launch_packed_ordered_geom<3, false>(const Geom &, const FeatureFwdArgs &, cudaStream_t);
+extern template int launch_packed_ordered_geom<3, true>(const Geom &, const FeatureFwdArgs &, cudaStream_t);
+
+static int launch_packed_ordered(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
+    if (g.dim == 2) return g.periodic ? launch_packed_ordered_geom<2, true>(g, a, st) : launch_packed_ordered_geom<2, false>(g, a, st);
+    return g.periodic ? launch_packed_ordered_geom<3, true>(g, a, st) : launch_packed_ordered_geom<3, false>(g, a, st);
+}
+}  // namespace npa
+
 extern "C" {
 
 int npa_perceive_features_forward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
@@ -119,9 +133,12 @@ int npa_perceive_features_forward_lists(const npa_grid *gd, int32_t channels, co
     if (packed && ((uintptr_t)packed % 16 || !pair_cache))
         return fail(NPA_ERR_INVALID_ARGUMENT, "perceive_features_forward: packed must be 16-byte aligned and needs neighbour lists");
     const bool in_sweep = !tile_forward_enabled();
+    // Over lists the sums have one fixed order, recorded for a backward or not: see density_ordered.cu.
+    const bool ordered = pair_cache && in_sweep && channels <= 32;
     ScalarFwdArgs sa = {x_bin, mass, nullptr, nullptr, rho, in_sweep ? nullptr : rho_grad, nullptr, bin_offsets, block_info, pair_cache, pair_stride};
     sa.pv = reinterpret_cast<float4 *>(packed);
-    if ((rc = launch_scalar_forward(g, in_sweep ? S_DENSITY : (S_DENSITY | S_DGRAD), sa, st)) != NPA_OK) return rc;
+    rc = ordered ? launch_density_ordered(g, sa, st) : launch_scalar_forward(g, in_sweep ? S_DENSITY : (S_DENSITY | S_DGRAD), sa, st);
+    if (rc != NPA_OK) return rc;
     FeatureFwdArgs fa = {x_bin, mass, rho, s_bin, nullptr, nullptr, channels, bin_offsets, block_info, nullptr};
     fa.z = z;
     fa.zstride = 2 * channels + channels * g.dim + g.dim;
@@ -137,6 +154,7 @@ int npa_perceive_features_forward_lists(const npa_grid *gd, int32_t channels, co
     fa.pair_cache = pair_cache;
     fa.pair_stride = pair_stride;
     fa.pair_cache_valid = pair_cache != nullptr;  // written by the density sweep above
+    if (ordered) return launch_packed_ordered(g, fa, st);
     return launch_feature_forward(g, F_BLUR | F_GRAD | F_MOMENT | F_PACK, fa, st);
 }
 
