@@ -199,6 +199,23 @@ __device__ inline Spiky spiky_distance(float q) {
     const float d = Q * y;
     return Spiky{fmaf(0.5f * y, fmaf(-d, d, Q), d), y};
 }
+// Square root and quotient as IEEE rounds them, without the range checks and branches of the general routines: Newton steps
+// whose residuals are exact by fused multiply-add (P. Markstein, IA-64 and Elementary Functions, ch. 8-9).  Q normal,
+// 2^-66 <= Q < 2^66: over all of them the root equals __fsqrt_rn, and 6e9 quotients of them equal __fdiv_rn.
+struct Root {
+    float d, inv;  // sqrt(Q), and 1 / d to within an ulp
+};
+__device__ inline Root root_rounded(float Q) {
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Q));
+    const float s = __fmul_rn(Q, y);
+    const float d = fmaf(fmaf(-s, s, Q), __fmul_rn(0.5f, y), s);
+    return Root{d, fmaf(fmaf(-d, y, 1.0f), y, y)};
+}
+__device__ inline float quotient_rounded(float n, const Root &r) {  // n / r.d
+    const float q = __fmul_rn(n, r.inv);
+    return fmaf(fmaf(-r.d, q, n), r.inv, q);
+}
 __device__ inline float spiky_phi(const Spiky &s, float h) {
     const float t = fmaxf(h - s.d, 0.0f);
     return 3.0f * t * t * s.inv;
@@ -244,8 +261,14 @@ template <int D>
 __device__ inline void log_normalize(float *w) {
     float n2 = w[0] * w[0] + w[1] * w[1];
     if (D == 3) n2 += w[2] * w[2];
-    const float n = sqrtf(n2);
-    const float sc = logf(1.0f + n) / fmaxf(n, 1e-12f);
+    float sc;
+    if (n2 > 1e-18f && n2 < 1e18f) {
+        const Root r = root_rounded(n2);
+        sc = quotient_rounded(logf(1.0f + r.d), r);
+    } else {
+        const float n = sqrtf(n2);
+        sc = logf(1.0f + n) / fmaxf(n, 1e-12f);
+    }
 #pragma unroll
     for (int d = 0; d < D; ++d) w[d] *= sc;
 }

@@ -10,7 +10,7 @@
 // kTileSpan cells apart -- gives every particle a lane, loads 32 candidates at a time into shared memory and lets every lane test
 // each of them.  Bound by instruction issue (about a dozen instructions per candidate and tile) and by the list entries,
 // written a word at a time.  Measured, B200, us: 262,144 particles 3D, ~240 candidates 140; 32,768 particles 2D 20.
-// Morton and 3D periodic grids: the walk per particle of scalar_ops.cu.
+// Few particles, Morton and 3D periodic grids: a lane per candidate, below.
 #include "neighbors.cuh"
 #include "ops.cuh"
 
@@ -165,16 +165,20 @@ density_ordered_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_con
     release_rows(a.tickets);
 }
 
+// Rows a warp draws per ticket: two tickets for each of 32 warps on 148 SMs, at most kTicketRows rows (consecutive rows
+// of one ticket can merge into a tile; a single row cannot).  The tiles decide which candidates are even, so the rule
+// depends on nothing but the size of the work list.
+static int ticket_rows(const Geom &g) {
+    const int batch = g.max_blocks / (2 * 32 * 148);
+    return batch < 1 ? 1 : (batch > kTicketRows ? kTicketRows : batch);
+}
+
 template <int D, bool PER>
 static int launch_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     int ctas = 0;
     int rc = persistent_ctas(density_ordered_kernel<D, PER>, kWarpsPerCta * 32, 0, &ctas);
     if (rc != NPA_OK) return rc;
-    // rows a warp draws per ticket: two tickets for each of 32 warps on 148 SMs, at most kTicketRows rows (consecutive rows
-    // of one ticket can merge into a tile; a single row cannot).  The tiles decide which candidates are even, so the rule
-    // depends on nothing but the size of the work list.
-    int batch = g.max_blocks / (2 * 32 * 148);
-    batch = batch < 1 ? 1 : (batch > kTicketRows ? kTicketRows : batch);
+    const int batch = ticket_rows(g);
     const int needed = (g.max_blocks + batch * kWarpsPerCta - 1) / (batch * kWarpsPerCta);
     ScalarFwdArgs b = a;
     if ((rc = acquire_row_tickets(st, &b.tickets)) != NPA_OK) return rc;
@@ -182,8 +186,230 @@ static int launch_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st
     return check_launch("density_ordered_kernel");
 }
 
+// ---------------------------------------------------------------------------------------------------------
+// The same sums with a lane per candidate: a warp takes up to eight particles of an item, tests 32 candidates at a time
+// against four of them and appends the accepted ones (kernel value, index and class) to the particle's run in shared
+// memory by their rank in the ballot, that is in candidate order.  Afterwards a lane per particle and class walks
+// the run.  CLS classes by the position in the range: 1 on the 2D periodic grid, 2 on the clamped one, 4 (the lanes of the
+// walk per particle) with Morton order and on the 3D periodic grid.  Bound by instruction issue (~56 % of the slots, at 10 warps
+// per SM; 4,096 particles in 2D with 370 candidates took the tile 43 us, this 18).
+// ---------------------------------------------------------------------------------------------------------
+constexpr int kItemWarps = 4;
+constexpr int kItemSlots = 320;  // candidates staged at a time per warp
+constexpr int kItemRun = 96;     // accepted neighbours of a particle between two flushes
+
+struct ItemMem {
+    float4 cand[kItemSlots];            // x, y, z, (index << 2) | class
+    unsigned char code[kItemSlots];     // image shift
+    float value[8][kItemRun + 1];       // (one more: the rows start on different banks)
+    unsigned index[8][kItemRun + 1];
+    int4 rng[32];
+};
+
+template <int D, bool PER, int CLS>
+__global__ void __launch_bounds__(kItemWarps * 32, 4)
+density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g, int split) {
+    extern __shared__ __align__(16) unsigned char s_item[];
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = a.pair_stride;
+    ItemMem &S = reinterpret_cast<ItemMem *>(s_item)[warp];
+    const unsigned below = (1u << lane) - 1u;
+    const int pl = lane >> 2, cls = lane & 3;  // the particle and the class this lane sums
+
+    const int vrows = g.max_blocks * split;
+    for (int vrow = blockIdx.x * kItemWarps + warp; vrow < vrows; vrow += gridDim.x * kItemWarps) {
+        const int row = split == 1 ? vrow : vrow / split, part = vrow - row * split;
+        const WorkItem it = load_item(a.block_info, a.bin_offsets, row);
+        if (it.count <= 0) break;  // rows after the last work item are zero
+        const int share = split == 1 ? it.count : ((it.count + split - 1) / split + 3) & ~3;
+        const int k0 = part * share, k1 = min(k0 + share, it.count);
+        if (k0 >= k1) continue;
+
+        // the non-empty candidate ranges: start, length, image shift, ordinal of the first candidate
+        int cx, cy, cz, start, end, code;
+        hash_to_cell<D>(g, (uint32_t)(it.cell - it.sys * g.cells), cx, cy, cz);
+        range_piece<D>(g, a.bin_offsets + (size_t)it.sys * g.cells, cx, cy, cz, lane, start, end, code);
+        const int len = max(end - start, 0);
+        int incl = len;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int v = __shfl_up_sync(kFull, incl, o);
+            if (lane >= o) incl += v;
+        }
+        const int total = __shfl_sync(kFull, incl, 31);
+        const unsigned some = __ballot_sync(kFull, len > 0);
+        const int nr = __popc(some);
+        __syncwarp();
+        if (len > 0) S.rng[__popc(some & below)] = make_int4(start, len, code, incl - len);
+        __syncwarp();
+        const bool wrapped = PER && __any_sync(kFull, len > 0 && code != shift_code(0, 0, 0));
+        // an axis too short to know the image of a cell, or a position outside the box: the half-box test decides pair by pair
+        bool check = PER && (g.g[0] <= 4 || g.g[1] <= 4 || (D == 3 && g.g[2] <= 4));
+
+        for (int kb = k0; kb < k1; kb += 8) {
+            const int nb = min(8, k1 - kb);
+            float rho = 0.f;       // of particle kb + pl, the pairs of class cls
+            int found = 0, held = 0;  // of particle kb + lane: entries in its list, and in its run
+            auto flush = [&]() {
+                __syncwarp();
+                for (int p = 0; p < nb; ++p) {
+                    const int n = __shfl_sync(kFull, held, p), at = __shfl_sync(kFull, found, p);
+                    int32_t *list = a.pair_cache + (it.first + kb + p) * (long long)K + 1 + at;
+                    for (int e = lane; e < min(n, K - 1 - at); e += 32) list[e] = (int)(S.index[p][e] >> 2);
+                }
+                const int n = __shfl_sync(kFull, held, pl), most = __reduce_max_sync(kFull, held);
+                if (cls < CLS) {
+                    if (a.mass) {
+#pragma unroll 4
+                        for (int e = 0; e < most; ++e) {
+                            const unsigned id = S.index[pl][e];
+                            if (e < n && (CLS == 1 || (int)(id & 3u) == cls)) rho = fmaf(__ldg(a.mass + (id >> 2)), S.value[pl][e], rho);
+                        }
+                    } else {  // (adding zero changes no sum: they start at zero and the terms are not negative)
+#pragma unroll 8
+                        for (int e = 0; e < most; ++e) {
+                            const float v = S.value[pl][e];
+                            rho += e < n && (CLS == 1 || (int)(S.index[pl][e] & 3u) == cls) ? v : 0.f;
+                        }
+                    }
+                }
+                found += held;
+                held = 0;
+                __syncwarp();
+            };
+            for (int c0 = 0; c0 < total; c0 += kItemSlots) {
+                const int count = min(kItemSlots, total - c0);
+                if (total > kItemSlots || kb == k0) {  // otherwise the candidates are there already
+                    __syncwarp();
+                    const int group = total > 20 * nr ? 32 : (total > 8 * nr ? 16 : 8);  // lanes per range by the mean length
+                    for (int r = lane / group; r < nr; r += 32 / group) {
+                        const int4 R = S.rng[r];
+                        const int e = min(R.y, c0 + count - R.w);
+                        for (int k = max(0, c0 - R.w) + lane % group; k < e; k += group) {
+                            const int slot = R.w + k - c0;
+                            S.cand[slot].w = __uint_as_float(((unsigned)(R.x + k) << 2) | (unsigned)(k & (CLS - 1)));
+                            if (PER) S.code[slot] = (unsigned char)R.z;
+                        }
+                    }
+                    __syncwarp();
+                    // the positions: the loads of five steps in flight together
+                    bool outside = false;
+#pragma unroll 5
+                    for (int c = lane; c < count; c += 32) {
+                        const Pos<D> p = load_pos<D>(a.x, __float_as_uint(S.cand[c].w) >> 2);
+                        S.cand[c].x = p.x; S.cand[c].y = p.y; S.cand[c].z = p.z;
+                        if (PER) {
+                            const float v[3] = {p.x, p.y, p.z};
+#pragma unroll
+                            for (int d = 0; d < D; ++d)
+                                outside |= !(v[d] >= -(float)g.half[d] * g.h && v[d] <= (float)(g.g[d] - g.half[d]) * g.h);
+                        }
+                    }
+                    if (PER) check |= __any_sync(kFull, outside) != 0;
+                    __syncwarp();
+                }
+                for (int p0 = 0; p0 < nb; p0 += 4) {
+                    Pos<D> pi[4];
+                    int n[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        pi[u] = load_pos<D>(a.x, it.first + kb + min(p0 + u, nb - 1));
+                        n[u] = __shfl_sync(kFull, held, p0 + u);
+                    }
+                    for (int c = 0; c < count; c += 32) {
+                        const bool real = c + lane < count;
+                        const float4 cc = S.cand[real ? c + lane : 0];
+                        const int image = PER && wrapped ? S.code[real ? c + lane : 0] : shift_code(0, 0, 0);
+                        bool full = false;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) {
+                            Origin<D, PER> org;
+                            if (PER && wrapped) {
+                                org = make_origin<D, PER>(g, pi[u].x, pi[u].y, pi[u].z, image);
+                            } else {
+                                org.x[0] = pi[u].x; org.x[1] = pi[u].y; org.x[2] = pi[u].z;
+                                org.c[0] = org.c[1] = org.c[2] = 0.f;
+                            }
+                            float rx = (cc.x - org.x[0]) + org.c[0], ry = (cc.y - org.x[1]) + org.c[1], rz = D == 3 ? (cc.z - org.x[2]) + org.c[2] : 0.f;
+                            if (PER && check) displacement<D, PER, CLS == 4>(g, org, cc.x, cc.y, cc.z, rx, ry, rz);
+                            const float q = CLS == 4 ? sq_norm<D>(rx, ry, rz) : sq_norm_fast<D>(rx, ry, rz);
+                            const bool acc = real && q < g.h2;
+                            const unsigned hits = __ballot_sync(kFull, acc);
+                            if (acc) {
+                                const int e = n[u] + __popc(hits & below);
+                                const float t = fmaxf(g.h2 - q, 0.f);
+                                S.value[p0 + u][e] = t * t * t;
+                                S.index[p0 + u][e] = __float_as_uint(cc.w);
+                            }
+                            n[u] += __popc(hits);
+                            full |= n[u] > kItemRun - 32;
+                        }
+                        if (full) {  // a run may not hold another 32: empty them all
+#pragma unroll
+                            for (int u = 0; u < 4; ++u) {
+                                if (lane == p0 + u && p0 + u < nb) held = n[u];
+                                n[u] = 0;
+                            }
+                            flush();
+                        }
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u)
+                        if (lane == p0 + u && p0 + u < nb) held = n[u];
+                }
+            }
+            flush();
+            // the classes meet as the lanes of the walk (distance 2 first) and the even and odd candidates do
+            if (CLS == 4) rho += __shfl_xor_sync(kFull, rho, 2);
+            if (CLS >= 2) rho += __shfl_xor_sync(kFull, rho, 1);
+            const int listed = __shfl_sync(kFull, found, pl);
+            if (cls == 0 && pl < nb) {
+                const long long i = it.first + kb + pl;
+                a.pair_cache[i * K] = listed <= K - 1 ? listed : -1;
+                const float d = g.c_s * rho;
+                a.rho_out[i] = d;
+                if (a.pv) {
+                    const Pos<D> p = load_pos<D>(a.x, i);
+                    a.pv[i] = make_float4(p.x, p.y, p.z, (a.mass ? __ldg(a.mass + i) : 1.0f) / d);
+                }
+            }
+        }
+    }
+}
+
+template <int D, bool PER, int CLS>
+static int launch_item(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
+    const auto kernel = density_ordered_item_kernel<D, PER, CLS>;
+    const size_t dyn = sizeof(ItemMem) * kItemWarps;
+    int ctas = 0;
+    const int rc = persistent_ctas(kernel, kItemWarps * 32, dyn, &ctas);
+    if (rc != NPA_OK) return rc;
+    // warps sharing an item, four particles of it at least each: enough for two items per resident warp
+    const long long items = (long long)g.B * (g.cells < g.N ? g.cells : g.N);
+    long long split = 2ll * ctas * kItemWarps / items;
+    const int most = (g.mpb < g.N ? g.mpb : g.N) / 4;
+    if (split > most) split = most;
+    if (split > 16) split = 16;
+    if (split < 1) split = 1;
+    const long long needed = ((long long)g.max_blocks * split + kItemWarps - 1) / kItemWarps;
+    kernel<<<(unsigned)(needed < ctas ? needed : ctas), kItemWarps * 32, dyn, st>>>(a, g, (int)split);
+    return check_launch("density_ordered_item_kernel");
+}
+
 int launch_density_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
-    if (g.morton || (g.periodic && g.dim == 3)) return launch_density_walk(g, a, st);
+    if (g.morton || (g.periodic && g.dim == 3)) {
+        if (g.dim == 2) return g.periodic ? launch_item<2, true, 4>(g, a, st) : launch_item<2, false, 4>(g, a, st);
+        return g.periodic ? launch_item<3, true, 4>(g, a, st) : launch_item<3, false, 4>(g, a, st);
+    }
+    // A tile takes as long as the candidates of a lane, whatever the number of particles (2D, 144 candidates: 10 us at 4,096
+    // particles and 19 at 32,768; 370 candidates: 43 and 57); the item kernel's time grows with the particles (10 and 36; 18 and
+    // 96; thin cells in 3D 10 against 15 at 4,000, 28 against 32 at 16,000, 73 against 59 at 64,000).  Crowded cells of otherwise
+    // thin systems make long items.  (Same sums: a row drawn alone is a tile of its own.)
+    const long long particles = (long long)g.B * g.N;
+    const bool few = g.dim == 3 ? particles <= 20000 : particles <= 8192 && g.N >= (particles <= 4096 ? 8 : 20) * g.cells;
+    if (few && ticket_rows(g) == 1) {
+        if (g.dim == 3) return launch_item<3, false, 2>(g, a, st);
+        return g.periodic ? launch_item<2, true, 1>(g, a, st) : launch_item<2, false, 2>(g, a, st);
+    }
     if (g.dim == 3) return launch_ordered<3, false>(g, a, st);
     return g.periodic ? launch_ordered<2, true>(g, a, st) : launch_ordered<2, false>(g, a, st);
 }

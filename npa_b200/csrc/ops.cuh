@@ -158,7 +158,6 @@ int launch_feature_tile_backward(const Geom &g, int mask, const FeatureBwdArgs &
 
 int launch_density_search(const Geom &g, bool count, const ScalarFwdArgs &a, cudaStream_t st);  // density_search.cu
 bool scalar_shared_search();  // scalar_ops.cu: count and density run there
-int launch_density_walk(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st);     // scalar_ops.cu, a sub-group per particle
 int launch_density_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st);  // density_ordered.cu
 int launch_scalar_forward(const Geom &g, int mask, const ScalarFwdArgs &a, cudaStream_t st);
 int launch_scalar_backward(const Geom &g, int mask, const ScalarBwdArgs &a, cudaStream_t st);

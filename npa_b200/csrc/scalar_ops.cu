@@ -309,7 +309,9 @@ void set_scalar_shared_search(bool on) { g_shared_search = on; }
 bool scalar_shared_search() { return g_shared_search; }
 
 template <int MASK>
-static int launch_scalar_walk(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
+static int launch_scalar_fwd_mask(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
+    // the count or the density alone: the search that shares its candidates between particles
+    if ((MASK == S_DENSITY || (MASK == S_COUNT && !g.morton)) && g_shared_search) return launch_density_search(g, MASK == S_COUNT, a, st);
     const char *what = "scalar_forward_kernel";
     if (g.dim == 2) {
         if (g.periodic) return launch_persistent(g, scalar_forward_kernel<2, true, MASK>, a, st, what);
@@ -318,15 +320,6 @@ static int launch_scalar_walk(const Geom &g, const ScalarFwdArgs &a, cudaStream_
     if (g.periodic) return launch_persistent(g, scalar_forward_kernel<3, true, MASK>, a, st, what);
     return launch_persistent(g, scalar_forward_kernel<3, false, MASK>, a, st, what);
 }
-
-template <int MASK>
-static int launch_scalar_fwd_mask(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
-    // the count or the density alone: the search that shares its candidates between particles
-    if ((MASK == S_DENSITY || (MASK == S_COUNT && !g.morton)) && g_shared_search) return launch_density_search(g, MASK == S_COUNT, a, st);
-    return launch_scalar_walk<MASK>(g, a, st);
-}
-
-int launch_density_walk(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) { return launch_scalar_walk<S_DENSITY>(g, a, st); }
 
 int launch_scalar_forward(const Geom &g, int mask, const ScalarFwdArgs &a, cudaStream_t st) {
     switch (mask) {
