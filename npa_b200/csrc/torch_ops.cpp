@@ -584,20 +584,30 @@ py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, con
 constexpr int kHidden = 128;
 
 // Gradients of the MLP's weights and bias from one kernel over the rows.
-void mlp_weight_grads(const Tensor &z, const Tensor &dh, const Tensor &h, const Tensor &dy, const Tensor &w1, const Tensor &w2, Tensor &gw1,
-                      Tensor &gb1, Tensor &gw2, void *st) {
-    const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
-    gw1 = at::empty_strided(w1.sizes(), at::IntArrayRef({k, (int64_t)1}), w1.options().requires_grad(false));
-    gw2 = at::empty_strided(w2.sizes(), at::IntArrayRef({(int64_t)kHidden, (int64_t)1}), w2.options().requires_grad(false));
-    gb1 = floats(z, {kHidden});
-    // the tensor-memory kernel appends a column of ones to z, 176 columns in all
-    const bool tensor = k < 176;
-    const int64_t count = tensor ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o)
-                                 : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
-    Tensor scratch = floats(z, {count});
-    check_status((tensor ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(fptr(z), fptr(dh), fptr(h), fptr(dy), m, (int)k, kHidden, (int)o,
-                                                                              fmut(scratch), count, fmut(gw1), fmut(gw2), fmut(gb1), st));
+// (the tensor-memory kernel appends a column of ones to z, 176 columns in all)
+int64_t weight_grad_scratch_floats(int64_t m, int64_t k, int64_t o) {
+    return k < 176 ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o) : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
 }
+void mlp_weight_grads(const float *z, const float *dh, const float *h, const float *dy, int64_t m, const Tensor &w1, const Tensor &w2,
+                      float *scratch, Tensor &gw1, Tensor &gb1, Tensor &gw2, void *st) {
+    const int64_t k = w1.size(1), o = w2.size(0);
+    gw1 = blank(w1);
+    gw2 = blank(w2);
+    gb1 = floats(w1, {kHidden});
+    check_status((k < 176 ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(z, dh, h, dy, m, (int)k, kHidden, (int)o, scratch,
+                                                                               weight_grad_scratch_floats(m, k, o), fmut(gw1), fmut(gw2), fmut(gb1), st));
+}
+
+// The arrays that a node keeps to itself, in one allocation: offsets in floats, 256-byte aligned.
+struct Slab {
+    int64_t floats = 0;
+    int64_t add(int64_t count) {
+        const int64_t at = floats;
+        floats += (count + 63) & ~(int64_t)63;
+        return at;
+    }
+    Tensor make(const Tensor &like) const { return at::empty({floats}, like.options().dtype(at::kFloat).requires_grad(false)); }
+};
 
 struct MlpNode : Node {
     SavedVariable z_, w1_, w2_;
@@ -619,7 +629,8 @@ struct MlpNode : Node {
         }
         const bool n1 = should_compute_output(1), nb = should_compute_output(2), n2 = should_compute_output(3);
         if (n1 || nb || n2) {
-            mlp_weight_grads(z, dh, h, dy, w1, w2, gw1, gb1, gw2, st);
+            Tensor scratch = floats(z, {weight_grad_scratch_floats(m, k, o)});
+            mlp_weight_grads(fptr(z), fptr(dh), fptr(h), fptr(dy), m, w1, w2, fmut(scratch), gw1, gb1, gw2, st);
         }
         return {gz, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
     }
@@ -661,7 +672,10 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
 struct EulerNode : Node {
     GridPtr grid;
     SavedVariable w1_, w2_;
-    Tensor offs, perm, pairs, x_bin, s_bin, rho, rho_grad, vgrad, packed, z, h, y, dz_image, mask;
+    Tensor offs, perm, slab, mask;
+    const float *x_bin, *s_bin, *rho, *rho_grad, *vgrad, *packed, *z, *h, *y, *dz_image;  // in the slab
+    const int32_t *pairs;
+    int64_t C, columns, dz_bytes;
     float coef, dg_scale, alpha, dt, below;
     bool ln_grad, ln_dg, stop_pos, stop_state;
 
@@ -669,51 +683,59 @@ struct EulerNode : Node {
         const Tensor w1 = w1_.unpack(), w2 = w2_.unpack();  // raise when the graph was released
         const Tensor gx_new = solid(g[0]), gs_new = solid(g[1]);
         if (!gx_new.defined() && !gs_new.defined()) return variable_list(5);
-        c10::cuda::CUDAGuard guard(x_bin.device());
-        void *st = stream_of(x_bin);
-        npa_grid *gd = &grid->g;
-        const int64_t C = s_bin.size(2), k = z.size(-1), m = z.numel() / k, o = w2.size(0);
+        c10::cuda::CUDAGuard guard(slab.device());
+        void *st = stream_of(slab);
+        Grid &gr = *grid;
+        npa_grid *gd = &gr.g;
+        const int64_t k = w1.size(1), m = gr.B * gr.N, o = w2.size(0);
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
         const bool n1 = should_compute_output(2), nb = should_compute_output(3), n2 = should_compute_output(4);
-        const bool back_x = nx && !stop_pos, back_s = ns && !stop_state;
+        const bool back_x = nx && !stop_pos, back_s = ns && !stop_state, back = back_x || back_s, weights = n1 || nb || n2;
+        const int64_t work_bytes = back ? npa_lists_backward_scratch_bytes(gd, (int)C) : 0;
+        if (work_bytes < 0) check_status((int)work_bytes);
+        Slab l;
+        const int64_t o_gy = l.add(m * o), o_dh = l.add(back || weights ? m * kHidden : 0), o_gz = l.add(back ? m * k : 0),
+                      o_work = l.add(work_bytes / 4), o_gs = l.add(back_s ? m * C : 0),
+                      o_scratch = l.add(weights ? weight_grad_scratch_floats(m, k, o) : 0);
+        Tensor temporary = l.make(w1);
+        float *t = fmut(temporary), *gy = t + o_gy, *dh = t + o_dh, *gz = t + o_gz;
         // update
-        Tensor gy = blank(y);
-        check_status(mask.defined() ? npa_step_update_backward_masked(gd, fptr(y), fptr(mask), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fmut(gy), st)
-                                    : npa_step_update_backward(gd, fptr(y), nullptr, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fmut(gy), st));
+        check_status(mask.defined() ? npa_step_update_backward_masked(gd, y, fptr(mask), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), gy, st)
+                                    : npa_step_update_backward(gd, y, nullptr, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), gy, st));
         // MLP
-        Tensor dh, gw1, gb1, gw2;
-        if (back_x || back_s || n1 || nb || n2) {
-            dh = floats(z, {m, kHidden});
-            check_status(npa_mlp_hidden_grad(fptr(gy), fptr(w2), fptr(h), fmut(dh), m, kHidden, (int)o, w2.stride(0), w2.stride(1), st));
-        }
-        if (n1 || nb || n2) mlp_weight_grads(z, dh, h, gy, w1, w2, gw1, gb1, gw2, st);
+        if (back || weights) check_status(npa_mlp_hidden_grad(gy, fptr(w2), h, dh, m, kHidden, (int)o, w2.stride(0), w2.stride(1), st));
+        Tensor gw1, gb1, gw2;
+        if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st);
         // perception, with the update's own gradient of the states added
-        Tensor gx_bin = gx_new, gs_bin = gs_new;
-        if (back_x || back_s) {
-            Tensor gz = blank(z);
-            check_status(npa_linear_tcgen05_prepared(fptr(dh), dz_image.const_data_ptr(), dz_image.numel() * 4, fmut(gz), m, kHidden, (int)k, st));
-            Tensor work = list_scratch(*grid, s_bin, C), gxp = back_x ? blank(x_bin) : Tensor(), gsp = back_s ? blank(s_bin) : Tensor();
-            check_status(npa_perceive_features_backward_lists(gd, (int)C, fptr(x_bin), nullptr, fptr(s_bin), fptr(rho), fptr(rho_grad), fptr(vgrad),
-                                                              fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, fptr(gs_new), fmut(gxp), fmut(gsp),
-                                                              work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs),
-                                                              (int)pairs.size(2), st));
+        Tensor gx_bin = gx_new;
+        const float *gs_bin = fptr(gs_new);
+        if (back) {
+            check_status(npa_linear_tcgen05_prepared(dh, dz_image, dz_bytes, gz, m, kHidden, (int)k, st));
+            Tensor gxp = back_x ? floats(w1, {gr.B, gr.N, gr.P}) : Tensor();
+            float *gsp = back_s ? t + o_gs : nullptr;
+            check_status(npa_perceive_features_backward_lists(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, packed, gz, coef, dg_scale,
+                                                              ln_grad, ln_dg, fptr(gs_new), fmut(gxp), gsp, t + o_work, work_bytes, iptr(offs),
+                                                              pairs, (int)columns, st));
             if (back_s) gs_bin = gsp;
             if (back_x) gx_bin = gx_bin.defined() ? gxp.add_(gx_bin) : gxp;
         }
         // back into the order of the inputs
-        Tensor gx, gs;
-        if (nx && !gx_bin.defined()) gx_bin = at::zeros_like(x_bin);
-        if (ns && !gs_bin.defined()) gs_bin = at::zeros_like(s_bin);
-        if (nx) gx = blank(x_bin);
-        if (ns) gs = blank(s_bin);
+        Tensor gx, gs, none;
+        if (nx && !gx_bin.defined()) gx_bin = at::zeros({gr.B, gr.N, gr.P}, w1.options().requires_grad(false));
+        if (ns && !gs_bin) {
+            none = at::zeros({gr.B, gr.N, C}, w1.options().requires_grad(false));
+            gs_bin = fptr(none);
+        }
+        if (nx) gx = floats(w1, {gr.B, gr.N, gr.P});
+        if (ns) gs = floats(w1, {gr.B, gr.N, C});
         if (nx || ns)
-            check_status(npa_unbin_particles(gd, (int)C, nx ? fptr(gx_bin) : nullptr, ns ? fptr(gs_bin) : nullptr, nullptr, iptr(perm), fmut(gx), fmut(gs),
+            check_status(npa_unbin_particles(gd, (int)C, nx ? fptr(gx_bin) : nullptr, ns ? gs_bin : nullptr, nullptr, iptr(perm), fmut(gx), fmut(gs),
                                              nullptr, st));
         return {gx, gs, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
     }
     void release_variables() override {
         w1_.reset_data(); w2_.reset_data();
-        pairs = x_bin = s_bin = rho = rho_grad = vgrad = packed = z = h = y = dz_image = mask = Tensor();
+        slab = mask = Tensor();
     }
 };
 
@@ -731,28 +753,31 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     const bool back = record && ((wants_grad(x) && !stop_pos) || (wants_grad(s) && !stop_state));  // a backward reaches the perception
     const auto ints = at::TensorOptions().dtype(at::kInt).device(x.device());
     Tensor perm = at::empty({g.B, g.N}, ints), offs = at::empty({g.B * g.cells + 1}, ints), info = at::empty({g.max_blocks, 4}, ints);
-    Tensor x_bin = blank(x), s_bin = blank(s), rho = floats(x, {g.B, g.N}), rho_grad = floats(x, {g.B, g.N, D}), z = floats(s, {g.B, g.N, k});
-    Tensor vgrad = back ? floats(s, {g.B, g.N, C, D}) : Tensor(), pairs = new_lists(g, x, columns), packed = floats(x, {g.B, g.N, 4});
     grid->bin(x, perm, offs, info, st);
-    check_status(npa_bin_particles(&g.g, (int)C, fptr(x), fptr(s), nullptr, iptr(perm), fmut(x_bin), fmut(s_bin), nullptr, st));
-    check_status(npa_perceive_features_forward_lists(&g.g, (int)C, fptr(x_bin), nullptr, fptr(s_bin), (float)coef, (float)dg_scale, (float)inv_tol,
-                                                     ln_grad, ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), fmut(packed), iptr(offs),
-                                                     iptr(info), imut(pairs), (int)columns, st));
     const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), dz_bytes = back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
-    Tensor y = floats(s, {g.B, g.N, o}), h = record ? floats(s, {m, kHidden}) : Tensor(), image = floats(s, {bytes / 4});
-    Tensor dz_image = dz_bytes ? floats(s, {dz_bytes / 4}) : Tensor();
-    check_status(npa_mlp_forward_tcgen05_images(fptr(z), fptr(w1), fptr(b1), fptr(w2), fmut(h), fmut(y), m, (int)k, (int)o, w1.stride(0), w1.stride(1),
-                                                w2.stride(0), w2.stride(1), image.mutable_data_ptr(), bytes, fmut(dz_image), dz_bytes, st));
+    Slab l;
+    const int64_t o_x = l.add(m * g.P), o_s = l.add(m * C), o_rho = l.add(m), o_dg = l.add(m * D), o_z = l.add(m * k), o_v = l.add(back ? m * C * D : 0),
+                  o_packed = l.add(m * 4), o_y = l.add(m * o), o_h = l.add(record ? m * kHidden : 0), o_image = l.add(bytes / 4),
+                  o_dz = l.add(dz_bytes / 4), o_pairs = l.add(m * columns);
+    Tensor slab = l.make(x);
+    float *t = fmut(slab), *x_bin = t + o_x, *s_bin = t + o_s, *rho = t + o_rho, *rho_grad = t + o_dg, *z = t + o_z, *packed = t + o_packed,
+          *y = t + o_y, *vgrad = back ? t + o_v : nullptr, *h = record ? t + o_h : nullptr, *dz_image = dz_bytes ? t + o_dz : nullptr;
+    int32_t *pairs = reinterpret_cast<int32_t *>(t + o_pairs);
+    check_status(npa_bin_particles(&g.g, (int)C, fptr(x), fptr(s), nullptr, iptr(perm), x_bin, s_bin, nullptr, st));
+    check_status(npa_perceive_features_forward_lists(&g.g, (int)C, x_bin, nullptr, s_bin, (float)coef, (float)dg_scale, (float)inv_tol, ln_grad, ln_dg,
+                                                     rho, rho_grad, z, vgrad, packed, iptr(offs), iptr(info), pairs, (int)columns, st));
+    check_status(npa_mlp_forward_tcgen05_images(z, fptr(w1), fptr(b1), fptr(w2), h, y, m, (int)k, (int)o, w1.stride(0), w1.stride(1), w2.stride(0),
+                                                w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
     Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();
     Tensor xo = blank(x), so = blank(s);
-    check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, fptr(y), fptr(x_bin), fptr(s_bin), fptr(mask), (float)update_prob, (int)C,
-                                                                 (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st)
-                                : npa_step_update_forward(&g.g, fptr(y), fptr(x_bin), fptr(s_bin), nullptr, (int)C, (float)alpha, (float)dt, wrap,
-                                                          fmut(xo), fmut(so), st));
+    check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, y, x_bin, s_bin, fptr(mask), (float)update_prob, (int)C, (float)alpha, (float)dt,
+                                                                 wrap, fmut(xo), fmut(so), st)
+                                : npa_step_update_forward(&g.g, y, x_bin, s_bin, nullptr, (int)C, (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st));
     if (record) {
         auto n = node_for<EulerNode>(x, s, w1, b1, w2);
-        n->grid = grid; n->offs = offs; n->perm = perm; n->pairs = pairs; n->x_bin = x_bin; n->s_bin = s_bin; n->rho = rho; n->rho_grad = rho_grad;
-        n->vgrad = vgrad; n->packed = packed; n->z = z; n->h = h; n->y = y; n->dz_image = dz_image; n->mask = mask;
+        n->grid = grid; n->offs = offs; n->perm = perm; n->slab = slab; n->mask = mask;
+        n->x_bin = x_bin; n->s_bin = s_bin; n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad; n->packed = packed; n->z = z; n->h = h; n->y = y;
+        n->dz_image = dz_image; n->pairs = pairs; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
         n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
         n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;

@@ -113,7 +113,7 @@ def supported(module) -> bool:
     CUDA device with ``in <= 176`` and ``out <= 48`` -- the shape of the reference's adaptation MLP."""
     if not (isinstance(module, torch.nn.Sequential) and len(module) == 3):
         return False
-    l1, act, l2 = module[0], module[1], module[2]
+    l1, act, l2 = module
     if not (isinstance(l1, torch.nn.Linear) and isinstance(act, torch.nn.ReLU) and isinstance(l2, torch.nn.Linear)):
         return False
     if l1.bias is None or l2.bias is not None or l1.out_features != HIDDEN or l2.in_features != HIDDEN:

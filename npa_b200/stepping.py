@@ -82,10 +82,12 @@ def _one_node(model, x, s, grid) -> bool:
     """Whether a step of this model is covered by the single autograd node: the adaptation MLP on the default
     engine, gradient features on, rows one warp pass covers, neighbour lists on."""
     C, module = s.shape[-1], model.model
-    return (getattr(model, "state_grad", True) and getattr(model, "density_grad", True) and sph_ops.packable(C)
-            and sph_ops._columns(grid.hashgrid) > 0 and on_tensor_memory(module)
-            and module[0].weight.device == x.device and module[0].in_features == 2 * C + C * grid.dim + grid.dim
-            and module[2].out_features == grid.dim + C)
+    if not (getattr(model, "state_grad", True) and getattr(model, "density_grad", True) and sph_ops.packable(C)
+            and sph_ops._columns(grid.hashgrid) > 0 and on_tensor_memory(module)):
+        return False
+    first, _, last = module
+    return (first.weight.device == x.device and first.in_features == 2 * C + C * grid.dim + grid.dim
+            and last.out_features == grid.dim + C)
 
 
 def step_euler(model, x, s, grid, dt=1.0, update_prob=0.5, intermediate=False, noise_std=0.0, wrap=False):
@@ -98,9 +100,9 @@ def step_euler(model, x, s, grid, dt=1.0, update_prob=0.5, intermediate=False, n
     alpha = _buffer_scalar(model, "alpha")
     stats = None
     if not intermediate and _one_node(model, x, s, grid):
-        mlp = model.model
+        first, _, last = model.model
         x_new, s_new, model.last_snapshot, uniforms = sph_ops.euler_step(
-            grid, x, s, (mlp[0].weight, mlp[0].bias, mlp[2].weight), _buffer_scalar(model, "eps0"), alpha, dt, update_prob, wrap,
+            grid, x, s, (first.weight, first.bias, last.weight), _buffer_scalar(model, "eps0"), alpha, dt, update_prob, wrap,
             getattr(model, "log_norm_grad", True), getattr(model, "log_norm_density_grad", True),
             getattr(model, "stopgrad_pos", True), getattr(model, "stopgrad_state", False))
     else:
