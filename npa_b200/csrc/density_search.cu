@@ -15,7 +15,7 @@
 // also spends as much again on its lists and on setting up an item.
 // Measured, B200, density + lists, us (before: a lane per particle with every list entry written as a word of its own,
 // and a walk per particle on Morton and 3D periodic grids): 262,144 particles 3D, ~240 candidates 140 -> 98;
-// 524,288 particles 3D periodic 542 -> 311; 65,536 particles 3D Morton, thin cells 61 -> 45; 4,096 particles 2D
+// 524,288 particles 3D periodic 542 -> 281; 65,536 particles 3D Morton, thin cells 61 -> 45; 4,096 particles 2D
 // periodic, 370 candidates 45 -> 17; 32,768 particles in 2D 20 -> 14.
 #include "neighbors.cuh"
 #include "ops.cuh"
@@ -233,7 +233,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                 const int at = found + before, take = min(held, K - 1 - at);  // entries that still fit
                 __syncwarp();
                 // eight lanes write a list, four lists at a time
-#pragma unroll 4
+#pragma unroll 1
                 for (int l0 = 0; l0 < 32; l0 += 4) {
                     const int l = l0 + (lane >> 3);
                     const int n = __shfl_sync(kFull, take, l);
@@ -245,92 +245,96 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                 held = 0;
                 __syncwarp();
             };
-            auto batch = [&](auto mode) {
+            // the 32 candidates from slot s0, the first one's bit highest
+            auto test = [&](auto mode, int s0) {
                 constexpr int kMode = decltype(mode)::value;  // 0: plain, 1: with low parts, 2: pair by pair
                 const unsigned long long nx = pack2(-pi.x, -pi.x), ny = pack2(-pi.y, -pi.y), nz = pack2(-pi.z, -pi.z);
                 const unsigned long long nh = pack2(-g.h2, -g.h2);
-                for (int s0 = part * 32; s0 < padded; s0 += 32 * Q) {
-                    unsigned m = 0u;
-                    if (kMode == 2) {
-                        for (int k = 0; k < 32; ++k) {
-                            const int c = s0 + k;
-                            float rx, ry, rz;
-                            Origin<D, PER> org;
-                            if (COUNT) {
-                                org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, S.j[c]);
-                            } else {
-                                org.x[0] = pi.x; org.x[1] = pi.y; org.x[2] = pi.z;
-                                org.c[0] = wrapped ? S.x[kTileSlots / 2 + c] : 0.f;
-                                org.c[1] = wrapped ? S.y[kTileSlots / 2 + c] : 0.f;
-                                org.c[2] = wrapped && D == 3 ? S.z[kTileSlots / 2 + c] : 0.f;
-                            }
-                            const float q = displacement<D, PER, COUNT>(g, org, S.x[c], S.y[c], D == 3 ? S.z[c] : 0.f, rx, ry, rz);
-                            const bool acc = q < g.h2 && c < count;
-                            m = (m << 1) | (acc ? 1u : 0u);
-                            if (!COUNT) {
-                                const float t = acc ? g.h2 - q : 0.f;
-                                rho = fmaf(MASS ? S.m[c] : 1.0f, t * t * t, rho);
-                            }
+                unsigned m = 0u;
+                if (kMode == 2) {
+                    for (int k = 0; k < 32; ++k) {
+                        const int c = s0 + k;
+                        float rx, ry, rz;
+                        Origin<D, PER> org;
+                        if (COUNT) {
+                            org = make_origin<D, PER>(g, pi.x, pi.y, pi.z, S.j[c]);
+                        } else {
+                            org.x[0] = pi.x; org.x[1] = pi.y; org.x[2] = pi.z;
+                            org.c[0] = wrapped ? S.x[kTileSlots / 2 + c] : 0.f;
+                            org.c[1] = wrapped ? S.y[kTileSlots / 2 + c] : 0.f;
+                            org.c[2] = wrapped && D == 3 ? S.z[kTileSlots / 2 + c] : 0.f;
                         }
-                    } else {
-#pragma unroll 4
-                        for (int k = 0; k < 32; k += 4) {
-                            const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(S.x + s0 + k), Y = *reinterpret_cast<const ulonglong2 *>(S.y + s0 + k);
-                            ulonglong2 Z = make_ulonglong2(0ull, 0ull), LX = Z, LY = Z, LZ = Z, M = Z;
-                            if (D == 3) Z = *reinterpret_cast<const ulonglong2 *>(S.z + s0 + k);
-                            if (kMode == 1) {
-                                LX = *reinterpret_cast<const ulonglong2 *>(S.x + kTileSlots / 2 + s0 + k);
-                                LY = *reinterpret_cast<const ulonglong2 *>(S.y + kTileSlots / 2 + s0 + k);
-                                if (D == 3) LZ = *reinterpret_cast<const ulonglong2 *>(S.z + kTileSlots / 2 + s0 + k);
-                            }
-                            if (MASS) M = *reinterpret_cast<const ulonglong2 *>(S.m + s0 + k);
-#pragma unroll
-                            for (int v = 0; v < 2; ++v) {
-                                unsigned long long rx = add2(v ? X.y : X.x, nx), ry = add2(v ? Y.y : Y.x, ny), rz = 0ull;
-                                if (D == 3) rz = add2(v ? Z.y : Z.x, nz);
-                                if (kMode == 1) {
-                                    rx = add2(rx, v ? LX.y : LX.x);
-                                    ry = add2(ry, v ? LY.y : LY.x);
-                                    if (D == 3) rz = add2(rz, v ? LZ.y : LZ.x);
-                                }
-                                unsigned long long q;
-                                if (COUNT) {  // no fused multiply-adds: borderline pairs as in the fp32 oracle
-                                    q = add2(mul2(rx, rx), mul2(ry, ry));
-                                    if (D == 3) q = add2(q, mul2(rz, rz));
-                                } else {
-                                    q = fma2(ry, ry, mul2(rx, rx));
-                                    if (D == 3) q = fma2(rz, rz, q);
-                                }
-                                float d0, d1;
-                                unpack2(add2(q, nh), d0, d1);  // r^2 - h^2, negative inside the cut-off
-                                m = shift_sign(shift_sign(m, d0), d1);
-                                if (!COUNT) {
-                                    const unsigned long long w = pack2(fmaxf(-d0, 0.f), fmaxf(-d1, 0.f));
-                                    const unsigned long long c3 = mul2(mul2(w, w), w);
-                                    sum2 = MASS ? fma2(v ? M.y : M.x, c3, sum2) : add2(sum2, c3);
-                                }
-                            }
+                        const float q = displacement<D, PER, COUNT>(g, org, S.x[c], S.y[c], D == 3 ? S.z[c] : 0.f, rx, ry, rz);
+                        const bool acc = q < g.h2 && c < count;
+                        m = (m << 1) | (acc ? 1u : 0u);
+                        if (!COUNT) {
+                            const float t = acc ? g.h2 - q : 0.f;
+                            rho = fmaf(MASS ? S.m[c] : 1.0f, t * t * t, rho);
                         }
                     }
-                    if (!mine) m = 0u;
-                    if (COUNT) {
-                        found += __popc(m);
-                    } else if (lists) {
-                        // as many rounds as the fullest lane has neighbours here: no divergence
-                        for (int left_over = __reduce_max_sync(kFull, __popc(m)); left_over > 0; --left_over) {
-                            const int b = __clz(m);
-                            if (m) run[held] = (unsigned char)(s0 + b);
-                            held += m != 0u;
-                            m &= ~(0x80000000u >> (b & 31));
+                } else {
+#pragma unroll 4
+                    for (int k = 0; k < 32; k += 4) {
+                        const ulonglong2 X = *reinterpret_cast<const ulonglong2 *>(S.x + s0 + k), Y = *reinterpret_cast<const ulonglong2 *>(S.y + s0 + k);
+                        ulonglong2 Z = make_ulonglong2(0ull, 0ull), LX = Z, LY = Z, LZ = Z, M = Z;
+                        if (D == 3) Z = *reinterpret_cast<const ulonglong2 *>(S.z + s0 + k);
+                        if (kMode == 1) {
+                            LX = *reinterpret_cast<const ulonglong2 *>(S.x + kTileSlots / 2 + s0 + k);
+                            LY = *reinterpret_cast<const ulonglong2 *>(S.y + kTileSlots / 2 + s0 + k);
+                            if (D == 3) LZ = *reinterpret_cast<const ulonglong2 *>(S.z + kTileSlots / 2 + s0 + k);
                         }
-                        if (__any_sync(kFull, held > kTileRun - 4 - 32)) flush();
+                        if (MASS) M = *reinterpret_cast<const ulonglong2 *>(S.m + s0 + k);
+#pragma unroll
+                        for (int v = 0; v < 2; ++v) {
+                            unsigned long long rx = add2(v ? X.y : X.x, nx), ry = add2(v ? Y.y : Y.x, ny), rz = 0ull;
+                            if (D == 3) rz = add2(v ? Z.y : Z.x, nz);
+                            if (kMode == 1) {
+                                rx = add2(rx, v ? LX.y : LX.x);
+                                ry = add2(ry, v ? LY.y : LY.x);
+                                if (D == 3) rz = add2(rz, v ? LZ.y : LZ.x);
+                            }
+                            unsigned long long q;
+                            if (COUNT) {  // no fused multiply-adds: borderline pairs as in the fp32 oracle
+                                q = add2(mul2(rx, rx), mul2(ry, ry));
+                                if (D == 3) q = add2(q, mul2(rz, rz));
+                            } else {
+                                q = fma2(ry, ry, mul2(rx, rx));
+                                if (D == 3) q = fma2(rz, rz, q);
+                            }
+                            float d0, d1;
+                            unpack2(add2(q, nh), d0, d1);  // r^2 - h^2, negative inside the cut-off
+                            m = shift_sign(shift_sign(m, d0), d1);
+                            if (!COUNT) {
+                                const unsigned long long w = pack2(fmaxf(-d0, 0.f), fmaxf(-d1, 0.f));
+                                const unsigned long long c3 = mul2(mul2(w, w), w);
+                                sum2 = MASS ? fma2(v ? M.y : M.x, c3, sum2) : add2(sum2, c3);
+                            }
+                        }
                     }
                 }
+                return mine ? m : 0u;
             };
-            if (PER && (check || (COUNT && wrapped))) batch(Mode<2>());
-            else if (PER && wrapped) batch(Mode<1>());
-            else batch(Mode<0>());
-            if (lists) flush();
+            // One copy of the rest for all ways of testing: with a copy for each, a sixth of the periodic kernel's stalls were
+            // waits for instructions (524,288 particles 311 us, so 281).
+            for (int s0 = part * 32; s0 < padded; s0 += 32 * Q) {
+                unsigned m;
+                if (PER && (check || (COUNT && wrapped))) m = test(Mode<2>(), s0);
+                else if (PER && wrapped) m = test(Mode<1>(), s0);
+                else m = test(Mode<0>(), s0);
+                if (COUNT) {
+                    found += __popc(m);
+                } else if (lists) {
+                    // as many rounds as the fullest lane has neighbours here: no divergence
+                    for (int left_over = __reduce_max_sync(kFull, __popc(m)); left_over > 0; --left_over) {
+                        const int b = __clz(m);
+                        if (m) run[held] = (unsigned char)(s0 + b);
+                        held += m != 0u;
+                        m &= ~(0x80000000u >> (b & 31));
+                    }
+                    // (the lanes of a warp go round equally often: padded is a multiple of 32 Q)
+                    if (s0 + 32 * Q >= padded || __any_sync(kFull, held > kTileRun - 4 - 32)) flush();
+                }
+            }
         }
         float lo, hi;
         unpack2(sum2, lo, hi);

@@ -338,12 +338,16 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
     }
 }
 
-// dW1, db1 and dW2 from the CTAs' partial sums, added in CTA order.
-__global__ void mlp_grad_umma_reduce_kernel(GradArgs a) {
+// dW1, db1 and dW2 from the CTAs' partial sums: 64 outputs per block, the CTAs in eight runs of consecutive ones, each run
+// in order by a thread of its own (one thread for all 148 took 11 us, one round trip for eight of them after another).
+constexpr int kReduceOuts = 64, kReduceRuns = 8;
+__global__ void __launch_bounds__(kReduceOuts * kReduceRuns) mlp_grad_umma_reduce_kernel(GradArgs a) {
+    __shared__ float s_sum[kReduceRuns][kReduceOuts];
     const int K1 = a.in_dim, O = a.out_dim, Wp = a.N1p + a.N2p;
     const int n1 = kGradHidden * K1, total = n1 + kGradHidden + O * kGradHidden;
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= total) return;
+    const int lane = threadIdx.x % kReduceOuts, run = threadIdx.x / kReduceOuts;
+    const bool live = blockIdx.x * kReduceOuts + lane < total;
+    const int e = live ? blockIdx.x * kReduceOuts + lane : total - 1;
     int j, col;
     float *out;
     if (e < n1) {
@@ -362,17 +366,23 @@ __global__ void mlp_grad_umma_reduce_kernel(GradArgs a) {
     }
     const float *p = a.partial + (long long)j * Wp + col;
     const long long step = (long long)kGradHidden * Wp;
+    const int each = (a.ctas + kReduceRuns - 1) / kReduceRuns, end = min((run + 1) * each, a.ctas);
     float sum = 0.f;
-    int c = 0;
-    for (; c + 8 <= a.ctas; c += 8) {  // eight loads in flight, added in CTA order
+    int c = run * each;
+    for (; c + 8 <= end; c += 8) {  // eight loads in flight
         float v[8];
 #pragma unroll
         for (int u = 0; u < 8; ++u) v[u] = __ldg(p + (c + u) * step);
 #pragma unroll
         for (int u = 0; u < 8; ++u) sum += v[u];
     }
-    for (; c < a.ctas; ++c) sum += __ldg(p + c * step);
-    *out = sum;
+    for (; c < end; ++c) sum += __ldg(p + c * step);
+    s_sum[run][lane] = sum;
+    __syncthreads();
+    if (run == 0 && live) {
+        for (int r = 1; r < kReduceRuns; ++r) sum += s_sum[r][lane];
+        *out = sum;
+    }
 }
 
 static int grad_round16(int v) { return (v + 15) / 16 * 16; }
@@ -440,7 +450,7 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
     int rc = check_launch("mlp_grad_umma_kernel");
     if (rc != NPA_OK) return rc;
     const int total = kGradHidden * in_dim + kGradHidden + out_dim * kGradHidden;
-    mlp_grad_umma_reduce_kernel<<<(total + 63) / 64, 64, 0, st>>>(a);
+    mlp_grad_umma_reduce_kernel<<<(total + kReduceOuts - 1) / kReduceOuts, kReduceOuts * kReduceRuns, 0, st>>>(a);
     return check_launch("mlp_grad_umma_reduce_kernel");
 }
 
