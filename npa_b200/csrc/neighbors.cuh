@@ -312,10 +312,15 @@ __device__ inline void scan_candidates(const Geom &g, const float *__restrict__ 
 // shift): on a periodic grid the image is recovered from the raw difference, which lies within
 // half a box of a multiple of the box length, and applied through the same error-free shifted
 // origin the cell walk uses.
+// Most pairs need no image, and then that is the plain difference, bit for bit: a pair nearer than a quarter of the box
+// takes it (the recovery was a third of the pair-scalar stage of the list sweeps).
 template <int D, bool PER>
 __device__ inline void listed_displacement(const Geom &g, const Pos<D> &pi, const Pos<D> &pj, float &rx, float &ry,
                                            float &rz) {
-    if (PER) {
+    rx = pj.x - pi.x;
+    ry = pj.y - pi.y;
+    rz = D == 3 ? pj.z - pi.z : 0.f;
+    if (PER && (fabsf(rx) > 0.25f * g.L[0] || fabsf(ry) > 0.25f * g.L[1] || (D == 3 && fabsf(rz) > 0.25f * g.L[2]))) {
         const float pv[3] = {pi.x, pi.y, pi.z}, jv[3] = {pj.x, pj.y, pj.z};
         float r[3] = {0.f, 0.f, 0.f};
 #pragma unroll
@@ -328,10 +333,6 @@ __device__ inline void listed_displacement(const Geom &g, const Pos<D> &pi, cons
             r[d] = (jv[d] - sum) + __fsub_rn(k * g.Llo[d], err);
         }
         rx = r[0]; ry = r[1]; rz = r[2];
-    } else {
-        rx = pj.x - pi.x;
-        ry = pj.y - pi.y;
-        rz = D == 3 ? pj.z - pi.z : 0.f;
     }
 }
 
