@@ -323,7 +323,7 @@ def fp32_roofline(w, accepted_pairs, launch_ms, clocks):
     sm_mhz = (clocks or {}).get("sm_max_mhz") or 1965.0
     peak = 148 * 128 * 2 * sm_mhz * 1e6 / 1e12
     achieved = accepted_pairs * backward_flops_per_pair(w) / (launch_ms * 1e-3) / 1e12
-    return {"bound": "fp32", "kernel": "feature_backward_kernel", "achieved": achieved, "peak": peak,
+    return {"bound": "fp32", "kernel": "feature_list_backward_kernel", "achieved": achieved, "peak": peak,
             "unit": "TFLOP/s", "frac": achieved / peak, "accepted_pairs": accepted_pairs,
             "flops_per_pair": backward_flops_per_pair(w)}
 
@@ -547,7 +547,7 @@ def run_gpu_arm(args, w):
     flush = torch.empty(256 << 20, dtype=torch.uint8, device=dev)  # > 126 MB of L2
     phases = ["grid_build", "reorder", "density_sweep", "blur_gradient_sweep", "blur_gradient_backward",
               "density_backward"]
-    launches_per_step = 7 + 1 + 1 + 1 + 1 + 1  # grid build (7 kernels), reorder, four sweeps
+    launches_per_step = 6 + 1 + 1 + 1 + 2 + 1  # grid build (6 kernels), reorder, four sweeps (the blur + gradient backward lays its upstream out first)
 
     def step(ev=None):
         mark = (lambda k: ev[k].record()) if ev is not None else (lambda k: None)
@@ -676,7 +676,7 @@ def run_gpu_arm(args, w):
             "parallelism": f"{world} x independent batches of {B} systems (weak scaling)",
             "phase_ms": phase_ms,
             "binning_mpoints_per_s": B * N / ((phase_ms["grid_build"] + phase_ms["reorder"]) * 1e-3) / 1e6,
-            "roofline": {"bound": "hbm", "kernel": "feature_backward_kernel (blur+gradient backward)",
+            "roofline": {"bound": "hbm", "kernel": "feature_list_backward_kernel (blur+gradient backward)",
                          "achieved": achieved, "peak": peak, "peak_kind": peak_kind, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": TRAFFIC_BYTES_PER_LAUNCH.get(w.name),
                          "algorithmic_bytes_per_launch": B * N * bpp[dom], "launch_ms": phase_ms[dom]},
@@ -707,8 +707,8 @@ def run_gpu_arm(args, w):
 
 
 # dram__bytes_read.sum + dram__bytes_write.sum of one launch of the dominant kernel, from an ncu capture of a
-# full launch of the same workload (profiles/ncu_feature_kernels_cfg4_3d_splat.md); other workloads: not captured.
-TRAFFIC_BYTES_PER_LAUNCH = {"cfg4_3d_splat": 273.1e6}
+# full launch of the same workload (profiles/ncu_list_kernels_cfg4_3d_splat.md); other workloads: not captured.
+TRAFFIC_BYTES_PER_LAUNCH = {"cfg4_3d_splat": 284.7e6}
 
 
 def main():

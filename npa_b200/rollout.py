@@ -76,9 +76,9 @@ class PerceptionRollout:
         if grid.boundary == "periodic":
             self.box = torch.tensor([g * grid.eps for g in grid.grid_size[:D]], **f32)
             self.half_box = 0.5 * self.box
-        # kernels of this library per rollout: 7 grid build + reorder + 2 sweeps per step, and for the
-        # last step 2 backward sweeps + the inverse reorder
-        self.launches = self.steps * 10 + 3
+        # kernels of this library per rollout: 6 grid build + reorder + 2 sweeps per step, and for the last step the
+        # layout of the upstream, 2 backward sweeps and the inverse reorder
+        self.launches = self.steps * 9 + 4
 
     def _forward(self, x, s, last):
         hg = self.hg
