@@ -24,8 +24,8 @@
 // of the row sectors come from L2 (prefetching rows into L1 a chunk ahead was slower, 330 -> 340 us; one register
 // set per row refilled early cost spills, 194 -> 234 us; five CTAs of the full backward instead of four 664 -> 758 us).
 // Measured, B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us, kernel with the whole warp per particle
-// -> this one: blur + gradient 328 -> 182 (with the density gradient), packed perception 495 -> 275,
-// features-only backward 499 -> 396, full backward 902 -> 664.
+// -> this one: blur + gradient 328 -> 178 (with the density gradient), features-only backward 499 -> 401, full
+// backward 902 -> 644.
 #pragma once
 #include "neighbors.cuh"
 #include "ops.cuh"
@@ -33,7 +33,10 @@
 namespace npa {
 
 constexpr int kListWarps = 8;      // warps per CTA
-constexpr int kListFullWarps = 4;  // same, backward with position gradients
+// Same, backward; with position gradients it needs more registers than 16 warps per SM leave in 3D (60 bytes of spills):
+// seven CTAs of two warps there (262,144 particles 662 -> 644 us, 524,288 periodic 737 -> 703).
+template <int D, bool FULL>
+constexpr int kListBackwardWarps = FULL ? (D == 3 ? 2 : 4) : kListWarps;
 
 // (x, y, z, m_j / rho_j) of particle j: one 16-byte gather when the density sweep left it packed.
 template <int D>
@@ -434,7 +437,7 @@ __device__ __noinline__ void list_forward_search(const FeatureFwdArgs &a, const 
 }
 
 template <int D, bool PER, int LPP, bool VEC, int MASK>
-__global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 3)
+__global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 4)
 feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
     using S = ListShape<LPP>;
     __shared__ float4 s_k[kListWarps][2][S::kSlots];  // v_j (K.x, K.y, K.z, W)
@@ -464,7 +467,7 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL, bool SEARCH>
 __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
                                               float4 (*s_e)[ListShape<LPP>::kSlots], int4 (*s_j)[ListShape<LPP>::kIndexQuads]) {
-    constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP, WARPS = FULL ? kListFullWarps : kListWarps;
+    constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP, WARPS = kListBackwardWarps<D, FULL>;
     constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
@@ -775,11 +778,13 @@ __device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, c
     list_backward<D, PER, LPP, VEC, MASK, FULL, true>(a, g, s_k, s_e, s_j);
 }
 
+// Features only: four CTAs with up to 16 features -- 32,768 particles are a wave and a seventh of three CTAs, 48 -> 38 us --
+// and three with longer rows, 401 us against 411.
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
-__global__ void __launch_bounds__(FULL ? kListFullWarps * 32 : kListWarps * 32, FULL ? 4 : 3)
+__global__ void __launch_bounds__(kListBackwardWarps<D, FULL> * 32, FULL ? (D == 3 ? 7 : 4) : LPP == 4 ? 4 : 3)
 feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
     using S = ListShape<LPP>;
-    constexpr int WARPS = FULL ? kListFullWarps : kListWarps;
+    constexpr int WARPS = kListBackwardWarps<D, FULL>;
     __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z W
     __shared__ float4 s_e[FULL ? WARPS : 1][2][S::kSlots];  // FULL: phi psi v_j E
     __shared__ int4 s_j[WARPS][2][S::kIndexQuads];
@@ -851,7 +856,7 @@ int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdAr
 
 template <int D, bool PER, int LPP, bool VEC, bool FULL>
 int launch_list_backward_mask(const Geom &g, int mask, const FeatureListBwdArgs &a, cudaStream_t st) {
-    constexpr int PP = 32 / LPP, WARPS = FULL ? kListFullWarps : kListWarps;
+    constexpr int PP = 32 / LPP, WARPS = kListBackwardWarps<D, FULL>;
     const long long particles = (long long)g.B * g.N, per_cta = (long long)WARPS * PP;
     const unsigned blocks = (unsigned)((particles + per_cta - 1) / per_cta);
     switch (mask) {

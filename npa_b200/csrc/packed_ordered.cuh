@@ -16,7 +16,7 @@
 //
 // Bound by instruction issue and latency together (~1,700 warp instructions per two particles with 41 pairs, a third of
 // them the pairs themselves, half of the issue slots at 14.5 warps per SM).  Measured, B200, us, the sweep with the whole
-// warp per particle -> this one: 262,144 particles in 3D, C = 32, ~41 pairs 495 -> 422; 32,768 in 2D, C = 16, ~31 pairs 36.
+// warp per particle -> this one: 262,144 particles in 3D, C = 32, ~41 pairs 495 -> 417; 32,768 in 2D, C = 16, ~31 pairs 36.
 // Not kept: eight lanes per particle with all classes in registers (420, but 42 in 2D), sixteen with every class of one or two
 // features (492), five CTAs per SM in 3D (432, spills).
 #pragma once
@@ -25,7 +25,7 @@
 
 namespace npa {
 
-constexpr int kOrderedWarps = 4;    // warps per CTA
+constexpr int kOrderedWarps = 2;    // warps per CTA
 constexpr int kOrderedPairs = 127;  // longest list that is read in a recorded step
 constexpr int kOrderedRow = 164;    // floats of a packed row: 32 features in 3D
 
@@ -274,7 +274,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
 }
 
 template <int D, bool PER, int VW, int LPR, int CPL>
-__global__ void __launch_bounds__(kOrderedWarps * 32, D == 2 ? 5 : 4)
+__global__ void __launch_bounds__(kOrderedWarps * 32, D == 2 ? 10 : 8)
 packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
     using O = Ordered<D, PER, VW, LPR, CPL>;
     __shared__ OrderedMem s_mem[kOrderedWarps];
