@@ -155,17 +155,19 @@ def _lists_of(snapshot, x_bin):
     return snapshot.lists[1] if snapshot.lists is not None and _same(snapshot.lists[0], x_bin) else None
 
 
-def _lists_for(snapshot, x_bin):
-    """``(lists or None, whether the caller has to record them)``; new lists are left on the snapshot."""
-    pairs = _lists_of(snapshot, x_bin)
-    if pairs is not None:
-        return pairs, False
-    columns = _columns(snapshot.grid)
-    if columns == 0:
-        return None, False
-    pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device)
-    snapshot.lists = (_key(x_bin), pairs)
-    return pairs, True
+def _density(x_bin, mass, snapshot, want_density_gradient):
+    """``(rho, density gradient or None)``.  The lists recorded here serve the backward and every later operator on the
+    same positions; the snapshot gets them when the sweep that fills them has been issued, never before."""
+    pairs, record = _lists_of(snapshot, x_bin), False
+    if pairs is None:
+        columns = _columns(snapshot.grid)
+        record = columns > 0
+        if record:
+            pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device)
+    out = _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, want_density_gradient, record)
+    if record:
+        snapshot.lists = (_key(x_bin), pairs)
+    return out
 
 
 def _sweep_args(snapshot):
@@ -210,8 +212,7 @@ class DensityPair:
 
     @staticmethod
     def apply(x_bin, mass, snapshot):
-        pairs, record = _lists_for(snapshot, x_bin)
-        return _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, True, record)
+        return _density(x_bin, mass, snapshot, True)
 
 
 class BlurGradient:
@@ -255,9 +256,7 @@ def count(x_bin, snapshot):
 class Density:
     @staticmethod
     def apply(x_bin, mass, snapshot):
-        # the lists recorded here serve every later operator on the same positions, and its own backward
-        pairs, record = _lists_for(snapshot, x_bin)
-        return _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, False, record)[0]
+        return _density(x_bin, mass, snapshot, False)[0]
 
 
 def density(x_bin, snapshot, mass=None):
