@@ -156,17 +156,14 @@ def _lists_of(snapshot, x_bin):
 
 
 def _density(x_bin, mass, snapshot, want_density_gradient):
-    """``(rho, density gradient or None)``.  The lists recorded here serve the backward and every later operator on the
-    same positions; the snapshot gets them when the sweep that fills them has been issued, never before."""
-    pairs, record = _lists_of(snapshot, x_bin), False
-    if pairs is None:
-        columns = _columns(snapshot.grid)
-        record = columns > 0
-        if record:
-            pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device)
-    out = _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, want_density_gradient, record)
-    if record:
-        snapshot.lists = (_key(x_bin), pairs)
+    """``(rho, density gradient or None)``, with neighbour lists for the backward and for the later operators on the same
+    positions.  Every call records its own lists: positions can change without a new version (a replayed CUDA graph, a
+    kernel that writes through the pointer, ``.data``), and then the density is computed anew as well.  The snapshot
+    gets the lists when the sweep that fills them has been issued, never before."""
+    columns = _columns(snapshot.grid)
+    pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device) if columns else None
+    out = _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, want_density_gradient, columns > 0)
+    snapshot.lists = (_key(x_bin), pairs) if columns else None
     return out
 
 

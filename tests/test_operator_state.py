@@ -28,3 +28,30 @@ def test_a_refused_density_leaves_no_lists_behind(fused):
     finally:
         sph.enable_fusion(False)
     assert snap.lists is None
+
+
+def test_every_density_records_its_own_lists(monkeypatch):
+    """Positions may change without a new tensor version (a replayed graph, a raw pointer): a second density on the same
+    tensor object must not take the lists of the first."""
+    from npa_b200.sphops import sph as impl
+
+    recorded = []
+
+    class Ops:
+        @staticmethod
+        def density(grid, offs, info, x, mass, pairs, want_rho, want_dg, record):
+            recorded.append((pairs, record))
+            return torch.zeros(x.shape[:2]), None
+
+    monkeypatch.setattr(impl, "_ops", Ops)
+    snap, x = _snapshot(_grid()), torch.zeros(2, 16, 2)
+    for _ in range(2):
+        impl.density(x, snap)
+        assert recorded[-1][1] and snap.lists[1] is recorded[-1][0]
+    assert recorded[0][0] is not recorded[1][0]
+    sph.set_pair_cache(0)
+    try:
+        impl.density(x, snap)          # lists switched off in between: the old ones are not left behind either
+        assert recorded[-1] == (None, False) and snap.lists is None
+    finally:
+        impl._PAIR_CACHE["columns"] = None
