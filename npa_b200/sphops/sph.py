@@ -160,10 +160,11 @@ def _density(x_bin, mass, snapshot, want_density_gradient):
     positions.  Every call records its own lists: positions can change without a new version (a replayed CUDA graph, a
     kernel that writes through the pointer, ``.data``), and then the density is computed anew as well.  The snapshot
     gets the lists when the sweep that fills them has been issued, never before."""
-    columns = _columns(snapshot.grid)
+    key = _key(x_bin)
+    columns = _columns(snapshot.grid) if key is not None else 0
     pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device) if columns else None
     out = _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, want_density_gradient, columns > 0)
-    snapshot.lists = (_key(x_bin), pairs) if columns else None
+    snapshot.lists = (key, pairs) if columns else None
     return out
 
 
@@ -182,7 +183,10 @@ def fusion_enabled():
 
 def _key(*tensors):
     """Identity + version of the input tensor objects (None allowed), held weakly: a parked output never
-    keeps its inputs alive, and an input that has died can never match again."""
+    keeps its inputs alive, and an input that has died can never match again.  None when one of them is an
+    inference tensor: those have no version, a change in place would go unnoticed."""
+    if any(t is not None and t.is_inference() for t in tensors):
+        return None
     return tuple((None if t is None else weakref.ref(t), None if t is None else t._version) for t in tensors)
 
 
@@ -193,7 +197,8 @@ def _same(key, *tensors):
 
 
 def _park(snapshot, name, key, value):
-    snapshot.parked[name] = (key, value)
+    if key is not None:
+        snapshot.parked[name] = (key, value)
 
 
 def _claim(snapshot, name, *tensors):

@@ -30,20 +30,42 @@ def test_a_refused_density_leaves_no_lists_behind(fused):
     assert snap.lists is None
 
 
+class _Ops:
+    """Stands in for the native operators: records the lists a density is given."""
+
+    def __init__(self):
+        self.recorded = []
+
+    def density(self, grid, offs, info, x, mass, pairs, want_rho, want_dg, record):
+        self.recorded.append((pairs, record))
+        return torch.zeros(x.shape[:2]), torch.zeros(*x.shape[:2], 2) if want_dg else None
+
+
+@pytest.mark.parametrize("fused", [False, True])
+def test_density_of_inference_tensors(monkeypatch, fused):
+    """Inference tensors have no version to compare: they are computed with, but nothing is kept for them."""
+    from npa_b200.sphops import sph as impl
+
+    ops = _Ops()
+    monkeypatch.setattr(impl, "_ops", ops)
+    snap = _snapshot(_grid())
+    sph.enable_fusion(fused)
+    try:
+        with torch.inference_mode():
+            assert impl.density(torch.zeros(2, 16, 2), snap).shape == (2, 16)
+    finally:
+        sph.enable_fusion(False)
+    assert ops.recorded == [(None, False)] and snap.lists is None and not snap.parked
+
+
 def test_every_density_records_its_own_lists(monkeypatch):
     """Positions may change without a new tensor version (a replayed graph, a raw pointer): a second density on the same
     tensor object must not take the lists of the first."""
     from npa_b200.sphops import sph as impl
 
-    recorded = []
-
-    class Ops:
-        @staticmethod
-        def density(grid, offs, info, x, mass, pairs, want_rho, want_dg, record):
-            recorded.append((pairs, record))
-            return torch.zeros(x.shape[:2]), None
-
-    monkeypatch.setattr(impl, "_ops", Ops)
+    ops = _Ops()
+    recorded = ops.recorded
+    monkeypatch.setattr(impl, "_ops", ops)
     snap, x = _snapshot(_grid()), torch.zeros(2, 16, 2)
     for _ in range(2):
         impl.density(x, snap)
