@@ -59,8 +59,12 @@ class HashGridSnapshot:
     # outputs computed ahead of their call by a fused sweep (see enable_fusion); not part of the
     # reference's dataclass, defaulted so positional construction still works
     parked: dict = field(default_factory=dict, repr=False, compare=False)
-    # neighbour lists of the positions the first density sweep saw: (key, tensor), see _lists_of
+    # neighbour lists of the positions the last density sweep saw: (key, tensor), see _lists_of
     lists: tuple = field(default=None, repr=False, compare=False)
+
+    def __getstate__(self):
+        # what is kept for tensor objects of this process (by weak reference) is of no use to a copy
+        return {**self.__dict__, "parked": {}, "lists": None}
 
 
 class HashGrid:

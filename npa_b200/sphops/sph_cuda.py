@@ -24,6 +24,7 @@ Differences, all on purpose:
 from __future__ import annotations
 
 import ctypes
+import functools
 
 import torch
 
@@ -81,13 +82,26 @@ class _HashGridBase:
         self._B, self._N, self._P = batch_size, particle_count, (2 if dim == 2 else 4)
         self._eps = eps
         self._mpb = mpb
-        # Columns of a neighbour list (one count + the neighbours): room for 1.6 times the mean number of neighbours
-        # of particles that fill the grid evenly, at least 127 (a particle with more searches the cells again), so
-        # that long-range grids -- 128 neighbours in a 10 x 10 periodic box of 4,096 particles -- fit as well.
-        ball = 3.14159265 if dim == 2 else 4.18879020
-        mean = ball * particle_count / self._cells
-        self.list_columns = 128 if mean <= 79 else min(512, -(-int(1.6 * mean + 1) // 64) * 64)
+        self._bind()
+
+    def _bind(self):
         self.native = N.ops.Grid(ctypes.addressof(self._desc))  # what the autograd nodes take (csrc/torch_ops.cpp)
+
+    # copies and pickles carry the description; the native handle is made anew
+    def __getstate__(self):
+        return {k: v for k, v in self.__dict__.items() if k != "native"}
+
+    def __setstate__(self, state):
+        self.__dict__.update(state)
+        self._bind()
+
+    @functools.cached_property
+    def list_columns(self):
+        """Columns of a neighbour list (one count + the neighbours): room for 1.6 times the mean number of neighbours
+        of particles that fill the grid evenly, at least 127 (a particle with more searches the cells again), so
+        that long-range grids -- 128 neighbours in a 10 x 10 periodic box of 4,096 particles -- fit as well."""
+        mean = (3.14159265 if self._dim == 2 else 4.18879020) * self._N / self._cells
+        return 128 if mean <= 79 else min(512, -(-int(1.6 * mean + 1) // 64) * 64)
 
     # ---- read-only properties of the nanobind classes ----------------------
     grid_size_x = property(lambda self: self._sizes[0])

@@ -1,4 +1,7 @@
 """What the operators keep between calls, on the host: no kernel is launched."""
+import copy
+import pickle
+
 import pytest
 import torch
 
@@ -77,3 +80,20 @@ def test_every_density_records_its_own_lists(monkeypatch):
         assert recorded[-1] == (None, False) and snap.lists is None
     finally:
         impl._PAIR_CACHE["columns"] = None
+
+
+@pytest.mark.parametrize("duplicate", [copy.deepcopy, lambda o: pickle.loads(pickle.dumps(o))], ids=["deepcopy", "pickle"])
+def test_grids_and_snapshots_are_copied_and_pickled(duplicate):
+    """A model that holds a grid or its last snapshot is copied (for a moving average) and saved whole."""
+    from npa_b200.sphops import sph as impl
+
+    grid = _grid(dim=3, N=600)
+    twin = duplicate(grid)
+    assert twin.hashgrid is not grid.hashgrid and twin.hashgrid.max_blocks == grid.hashgrid.max_blocks
+    assert twin.hashgrid.native is not grid.hashgrid.native and twin.hashgrid.list_columns == grid.hashgrid.list_columns
+    snap, x = _snapshot(grid), torch.zeros(2, 600, 4)
+    snap.lists = (impl._key(x), torch.zeros(2, 600, 128, dtype=torch.int32))
+    snap.parked["gradient"] = (impl._key(x), torch.zeros(1))
+    other = duplicate(snap)
+    assert other.lists is None and other.parked == {} and torch.equal(other.bin_offsets, snap.bin_offsets)
+    assert snap.lists is not None and other.grid.cell_count == 512
