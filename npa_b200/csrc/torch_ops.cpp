@@ -63,6 +63,11 @@ void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.devi
 Tensor floats(const Tensor &like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat).requires_grad(false)); }
 Tensor blank(const Tensor &like) { return floats(like, like.sizes()); }
 bool wants_grad(const Tensor &t) { return t.defined() && t.requires_grad(); }
+// No operator here has a forward-mode derivative: a dual number would lose its tangent without a word.
+template <typename... In>
+void refuse_tangents(const char *name, const In &...inputs) {
+    TORCH_CHECK_NOT_IMPLEMENTED(!((inputs.defined() && inputs._fw_grad(0).defined()) || ...), name, " has no forward-mode derivative");
+}
 
 // ---- a grid and the snapshot of one binning pass -------------------------------------------------
 struct Grid {
@@ -184,6 +189,7 @@ struct ReorderNode : Node {
 };
 
 py::tuple reorder(const GridPtr &grid, const Tensor &perm, const Tensor &x, const Tensor &s, const OptTensor &mass_) {
+    refuse_tangents("bin_particles", x, s, or_none(mass_));
     const Tensor mass = or_none(mass_);
     Grid &g = *grid;
     g.positions(x, "input_positions");
@@ -241,6 +247,7 @@ struct DensityNode : SweepNode {
 // with `write` the forward records them first.
 py::tuple density(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const OptTensor &mass, const OptTensor &pairs,
                   bool want_rho, bool want_dg, bool write) {
+    refuse_tangents("density", x, or_none(mass));
     Snap sn(grid, offs, info, mass, pairs);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -296,6 +303,7 @@ struct FeatureNode : SweepNode {
 // lists, valid when `have_lists`, otherwise recorded by this sweep.
 py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const Tensor &s,
                         const OptTensor &mass, const OptTensor &pairs, bool have_lists, bool want_blur, bool want_grad, bool want_moment) {
+    refuse_tangents("blur / gradient", x, rho, s, or_none(mass));
     Snap sn(grid, offs, info, mass, pairs);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -325,6 +333,7 @@ py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &i
 // raw operator.
 Tensor gradient_hybrid(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const Tensor &s,
                        const OptTensor &mass, const Tensor &pairs, double rtol) {
+    refuse_tangents("gradient_hybrid", x, rho, s, or_none(mass));
     Snap sn(grid, offs, info, mass, pairs);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -367,6 +376,7 @@ struct MomentNode : SweepNode {
 };
 
 Tensor moment_matrix(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &rho, const OptTensor &mass) {
+    refuse_tangents("moment_matrix", x, rho, or_none(mass));
     Snap sn(grid, offs, info, mass, std::nullopt);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -389,6 +399,7 @@ struct StraightThroughNode : Node {
 };
 
 Tensor corrected_gradient(const Tensor &raw, const Tensor &moment, double rtol) {
+    refuse_tangents("gradient_hybrid", raw, moment);
     const int64_t B = raw.size(0), N = raw.size(1), C = raw.size(2), D = raw.size(3);
     require(raw, {B, N, C, D}, "gradient");
     require(moment, {B, N, D, D}, "moment_matrix");
@@ -436,6 +447,7 @@ struct PerceptionNode : SweepNode {
 
 py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &s, const OptTensor &mass,
                      bool want_dg, int64_t columns) {
+    refuse_tangents("perceive", x, s, or_none(mass));
     Snap sn(grid, offs, info, mass, std::nullopt);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -506,6 +518,7 @@ struct PackedNode : SweepNode {
 
 Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x, const Tensor &s, const OptTensor &mass,
                          double coef, double dg_scale, double inv_tol, bool ln_grad, bool ln_dg, int64_t columns) {
+    refuse_tangents("perceive_features", x, s, or_none(mass));
     Snap sn(grid, offs, info, mass, std::nullopt);
     Grid &g = *grid;
     g.positions(x, "binned_positions");
@@ -557,6 +570,7 @@ struct StepNode : Node {
 
 py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, const Tensor &s, const OptTensor &mask_, double alpha, double dt, bool wrap,
                       double below) {
+    refuse_tangents("step_update", y, x, s, or_none(mask_));
     Grid &g = *grid;
     const Tensor mask = or_none(mask_);
     g.positions(x, "binned_positions");
@@ -642,6 +656,7 @@ struct MlpNode : Node {
 
 // y = relu(z W1^T + b1) W2^T over the rows of z; the caller has checked the shapes (mlp.supported).
 Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2) {
+    refuse_tangents("the adaptation MLP", z, w1, b1, w2);
     c10::cuda::CUDAGuard guard(z.device());
     const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
     std::vector<int64_t> shape = z.sizes().vec();
@@ -743,6 +758,7 @@ struct EulerNode : Node {
 py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, const Tensor &w1, const Tensor &b1, const Tensor &w2, double coef,
                      double dg_scale, double inv_tol, bool ln_grad, bool ln_dg, bool stop_pos, bool stop_state, double alpha, double dt,
                      double update_prob, bool wrap, int64_t columns) {
+    refuse_tangents("step_euler", x, s, w1, b1, w2);
     Grid &g = *grid;
     g.positions(x, "positions");
     g.features(s, "input_state");
@@ -811,6 +827,7 @@ struct SplatNode : Node {
 };
 
 Tensor splat(const Tensor &x, const Tensor &color, int img, double sigma, int radius, double lo, double hi, bool y_up, bool normalize, double scale) {
+    refuse_tangents("splat_particles", x, color);
     c10::cuda::CUDAGuard guard(x.device());
     const int64_t B = x.size(0), n = x.size(1);
     Tensor out = floats(x, {B, img, img, 4}), scratch = normalize ? floats(x, {B, n}) : Tensor();

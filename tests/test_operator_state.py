@@ -97,3 +97,35 @@ def test_grids_and_snapshots_are_copied_and_pickled(duplicate):
     other = duplicate(snap)
     assert other.lists is None and other.parked == {} and torch.equal(other.bin_offsets, snap.bin_offsets)
     assert snap.lists is not None and other.grid.cell_count == 512
+
+
+def test_forward_mode_derivatives_are_refused():
+    """An operator without a forward-mode derivative must not drop the tangent of a dual number."""
+    from torch.autograd import forward_ad
+    from npa_b200 import _native
+
+    grid, f = _grid(), torch.zeros
+    snap = _snapshot(grid)
+    sweep = (grid.hashgrid.native, snap.bin_offsets, snap.block_info)
+    with forward_ad.dual_level():
+        def dual(*shape):
+            return forward_ad.make_dual(f(*shape), torch.ones(*shape))
+
+        x, s, rho = dual(2, 16, 2), f(2, 16, 4), f(2, 16)
+        calls = {
+            "reorder": (grid.hashgrid.native, f(2, 16, dtype=torch.int32), x, s, None),
+            "density": (*sweep, x, None, None, True, False, False),
+            "blur_gradient": (*sweep, f(2, 16, 2), dual(2, 16), s, None, None, False, True, False, False),
+            "gradient_hybrid": (*sweep, x, rho, s, None, f(2, 16, 128, dtype=torch.int32), 1e-3),
+            "moment_matrix": (*sweep, x, rho, None),
+            "corrected_gradient": (dual(2, 16, 4, 2), f(2, 16, 2, 2), 1e-3),
+            "perception": (*sweep, f(2, 16, 2), dual(2, 16, 4), None, True, 128),
+            "packed_perception": (*sweep, x, s, None, 1.0, 1.0, 1e-3, True, True, 128),
+            "step_update": (grid.hashgrid.native, dual(2, 16, 6), f(2, 16, 2), s, None, 1.0, 1.0, False, -1.0),
+            "mlp": (f(32, 8), dual(128, 8), f(128), f(4, 128)),
+            "euler_step": (grid.hashgrid.native, x, s, f(128, 18), f(128), f(6, 128), 1.0, 1.0, 1e-3, True, True, True, False, 1.0, 1.0,
+                           0.5, False, 128),
+            "splat": (dual(2, 16, 2), f(2, 16, 3), 32, 1.0, 5, -1.0, 1.0, False, False, 1.0)}
+        for name, args in calls.items():
+            with pytest.raises(NotImplementedError, match="forward-mode"):
+                getattr(_native.ops, name)(*args)
