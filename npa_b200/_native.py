@@ -154,7 +154,73 @@ def _load_ops():
     return _torch_ops
 
 
-ops = _load_ops()
+def _traced(native, name, args):
+    """``native(*args)`` as one Python node of the graph that ``torch.jit.trace`` is recording.  A trace sees no C++ node:
+    it would keep the outputs of the traced call as constants."""
+    import torch
+
+    blank = []  # positions of the outputs that are None
+
+    class Call(torch.autograd.Function):
+        @staticmethod
+        def forward(ctx, *args):
+            state = torch._C._get_tracing_state()
+            torch._C._set_tracing_state(None)
+            try:
+                with torch.enable_grad():
+                    inner = [a.detach().requires_grad_(a.requires_grad) if isinstance(a, torch.Tensor) else a for a in args]
+                    outs = native(*inner)
+            finally:
+                torch._C._set_tracing_state(state)
+            ctx.single = isinstance(outs, torch.Tensor)
+            outs = [outs] if ctx.single else list(outs)
+            blank[:] = [k for k, o in enumerate(outs) if o is None]
+            ctx.outs, ctx.inner = [o for o in outs if o is not None], inner
+            plain = tuple(o.detach() for o in ctx.outs)
+            ctx.mark_non_differentiable(*(d for d, o in zip(plain, ctx.outs) if not o.requires_grad))
+            return plain[0] if ctx.single else plain
+
+        @staticmethod
+        def backward(ctx, *grads):
+            wanted = [k for k, need in enumerate(ctx.needs_input_grad) if need]
+            pairs = [(o, g) for o, g in zip(ctx.outs, grads) if o.requires_grad and g is not None]
+            found = torch.autograd.grad([o for o, _ in pairs], [ctx.inner[k] for k in wanted], [g for _, g in pairs],
+                                        retain_graph=True, allow_unused=True)
+            given = dict(zip(wanted, found))
+            return tuple(given.get(k) for k in range(len(ctx.inner)))
+
+    Call.__name__ = f"npa_{name}"
+    out = Call.apply(*args)
+    if isinstance(out, torch.Tensor):
+        return out
+    out = list(out)
+    for k in blank:
+        out.insert(k, None)
+    return tuple(out)
+
+
+class _Ops:
+    """The native operators; while ``torch.jit.trace`` records, each call is a node of its own in the trace."""
+
+    def __init__(self, module):
+        import torch
+
+        tracing = torch._C._get_tracing_state
+
+        def guard(name, native):
+            def call(*args):
+                return native(*args) if tracing() is None else _traced(native, name, args)
+
+            call.__name__ = name
+            return call
+
+        self.Grid = module.Grid
+        for name in dir(module):
+            if callable(getattr(module, name)) and name not in ("Grid",) and not name.startswith("_"):
+                setattr(self, name, guard(name, getattr(module, name)))
+
+
+ops = _Ops(_load_ops())
 
 
 def last_error() -> str:

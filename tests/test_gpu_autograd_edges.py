@@ -33,3 +33,52 @@ def test_operators_in_inference_mode():
     for a, b in zip(got, want):
         # without lists the sweeps search, and sum in another order
         assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max()))
+
+
+def _operators():
+    """Every differentiable operator as a function of positions and features in cell order (odd counts, both directions)."""
+    from npa_b200 import splatting
+    sph, grid, x, s = _inputs()
+    snap = grid.instantiate(x)
+    xb, sb = sph.bin_particles(x, s, snap)
+    rho = sph.density(xb, snap).detach()
+    first = lambda out: out if isinstance(out, tuple) else (out,)
+    ops = {
+        "bin_particles": lambda x, s: sph.bin_particles(x, s, snap),
+        "density": lambda x, s: sph.density(x, snap),
+        "density_gradient": lambda x, s: sph.density_gradient(x, snap),
+        "blur": lambda x, s: sph.blur(x, rho, s, snap),
+        "gradient": lambda x, s: sph.gradient(x, rho, s, snap),
+        "gradient_hybrid": lambda x, s: sph.gradient_hybrid(x, rho, s, snap),
+        "moment_matrix": lambda x, s: sph.moment_matrix(x, rho, snap),
+        "perceive": lambda x, s: sph.perceive(x, s, snap),
+        "perceive_features": lambda x, s: sph.perceive_features(x, s, snap, 0.125),
+        "step_update": lambda x, s: sph.step_update(torch.cat([x, s], -1), x, s, snap, 1.0),
+        "splat": lambda x, s: splatting.splat_particles_batch(x, s[..., :3], img_size=32),
+        "chain": lambda x, s: sph.blur(x, sph.density(x, snap), s, snap)}
+    return xb.detach(), sb.detach(), {k: (lambda f: lambda x, s: first(f(x, s)))(f) for k, f in ops.items()}
+
+
+def _value_and_grads(f, x, s):
+    x, s = x.clone().requires_grad_(True), s.clone().requires_grad_(True)
+    out = f(x, s)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    ups = [torch.randn(o.shape, generator=g, device="cuda") for o in out]
+    return [o.detach() for o in out], torch.autograd.grad(out, [x, s], ups, allow_unused=True)
+
+
+def _assert_same(got, want):
+    for a, b in zip([*got[0], *got[1]], [*want[0], *want[1]]):
+        assert (a is None) == (b is None)
+        if a is not None:  # the same kernels, with or without lists: sums in another order
+            assert torch.allclose(a, b, rtol=1e-4, atol=1e-5 * float(b.abs().max())), float((a - b).abs().max())
+
+
+@pytest.mark.filterwarnings("ignore")
+def test_traces_follow_their_inputs():
+    """torch.jit.trace records an operator as a node that runs, not as the outputs it had while it was traced."""
+    x, s, ops = _operators()
+    moved, other = x + 0.002, s.flip(-1).contiguous()
+    for name, f in ops.items():
+        traced = torch.jit.trace(f, (x, s), check_trace=False)
+        _assert_same(_value_and_grads(lambda x, s: tuple(traced(x, s)), moved, other), _value_and_grads(f, moved, other))
