@@ -6,8 +6,9 @@
 // particles.  Here an operator is one call: checks, output allocation, launch and graph node
 // together are a few microseconds, and backward nodes run in the autograd engine without the
 // interpreter.  Semantics are those of the reference's Functions (sphops/sph.py:127-464): a
-// gradient is produced only for inputs that need it, mass receives one in the reorder only, and
-// kernels run on the current stream of the tensors' device.
+// gradient is produced only for inputs that need it, mass receives one in the reorder only (elsewhere it is an input of
+// the node without a gradient, so that outputs require one wherever any input does), and kernels run on the current
+// stream of the tensors' device.
 #include <torch/extension.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
@@ -228,18 +229,36 @@ py::tuple unreorder(const GridPtr &grid, const Tensor &perm, const Tensor &x, co
     return mass.defined() ? py::make_tuple(xo, so, mo) : py::make_tuple(xo, so);
 }
 
+// ---- neighbour count ------------------------------------------------------------------------------------
+// Piecewise constant in the positions: the node is there because a caller may ask the output for its graph, and gives none.
+struct CountNode : Node {
+    variable_list apply(variable_list &&) override { return {Tensor()}; }
+};
+
+Tensor count(const GridPtr &grid, const Tensor &offs, const Tensor &info, const Tensor &x) {
+    refuse_tangents("count", x);
+    const Grid &g = *grid;
+    g.snapshot(offs, info);
+    g.positions(x, "binned_positions");
+    c10::cuda::CUDAGuard guard(x.device());
+    Tensor out = floats(x, {g.B, g.N});
+    check_status(npa_count_forward(&g.g, fptr(x), fmut(out), iptr(offs), iptr(info), stream_of(x)));
+    if (recording(x)) torch::autograd::set_history(out, node_for<CountNode>(x));
+    return out;
+}
+
 // ---- density and density gradient -------------------------------------------------------------------
 struct DensityNode : SweepNode {
     bool has_rho, has_dg;
     variable_list apply(variable_list &&g) override {
         const Tensor x = x_.unpack(), mass = mass_.unpack();
         const Tensor g_rho = has_rho ? solid(g[0]) : Tensor(), g_dg = has_dg ? solid(g[has_rho ? 1 : 0]) : Tensor();
-        if (!g_rho.defined() && !g_dg.defined()) return {Tensor()};
+        if ((!g_rho.defined() && !g_dg.defined()) || !should_compute_output(0)) return {Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = blank(x);
         check_status(npa_density_chain_backward(&grid->g, fptr(x), fptr(mass), fptr(g_rho), nullptr, fptr(g_dg), fmut(gx), 0, iptr(offs),
                                                 iptr(info), iptr(pairs), list_stride(), stream_of(x)));
-        return {gx};
+        return {gx, Tensor()};
     }
 };
 
@@ -260,8 +279,8 @@ py::tuple density(const GridPtr &grid, const Tensor &offs, const Tensor &info, c
         check_status(npa_density_gradient_forward_lists(&g.g, fptr(x), fptr(sn.mass), fmut(dg), iptr(offs), iptr(sn.pairs), sn.stride(), stream_of(x)));
     else
         check_status(npa_density_gradient_forward(&g.g, fptr(x), fptr(sn.mass), fmut(dg), iptr(offs), iptr(info), stream_of(x)));
-    if (recording(x)) {
-        auto n = node_for<DensityNode>(x);
+    if (recording(x, sn.mass)) {
+        auto n = node_for<DensityNode>(x, sn.mass);
         n->keep(grid, offs, info, sn.pairs, x, sn.mass);
         n->has_rho = want_rho; n->has_dg = want_dg;
         if (want_rho) torch::autograd::set_history(rho, n);
@@ -278,7 +297,7 @@ struct FeatureNode : SweepNode {
         const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(), mass = mass_.unpack();
         const bool nx = should_compute_output(0), ns = should_compute_output(1), nr = should_compute_output(2);
         const Tensor gb = has_blur ? solid(g[0]) : Tensor(), gg = has_grad ? solid(g[has_blur ? 1 : 0]) : Tensor();
-        if ((!gb.defined() && !gg.defined()) || !(nx || ns || nr)) return {Tensor(), Tensor(), Tensor()};
+        if ((!gb.defined() && !gg.defined()) || !(nx || ns || nr)) return variable_list(4);
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nr ? blank(rho) : Tensor();
         const int C = (int)s.size(2);
@@ -291,7 +310,7 @@ struct FeatureNode : SweepNode {
             check_status(npa_blur_gradient_backward(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
                                                     fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
         }
-        return {gx, gs, gr};
+        return {gx, gs, gr, Tensor()};
     }
     void release_variables() override {
         SweepNode::release_variables();
@@ -316,8 +335,8 @@ py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &i
     if (C > 0)
         check_status(npa_blur_gradient_forward(&g.g, (int)C, fptr(x), fptr(rho), fptr(sn.mass), fptr(s), fmut(blur), fmut(grad), fmut(moment),
                                                iptr(offs), iptr(info), imut(sn.pairs), sn.stride(), have_lists ? 1 : 0, stream_of(x)));
-    if (recording(x, s, rho)) {
-        auto n = node_for<FeatureNode>(x, s, rho);
+    if (recording(x, s, rho, sn.mass)) {
+        auto n = node_for<FeatureNode>(x, s, rho, sn.mass);
         n->keep(grid, offs, info, sn.pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
         n->rho_ = SavedVariable(rho, false);
@@ -345,8 +364,8 @@ Tensor gradient_hybrid(const GridPtr &grid, const Tensor &offs, const Tensor &in
     if (C > 0)
         check_status(npa_gradient_hybrid_forward_lists(&g.g, (int)C, fptr(x), fptr(rho), fptr(sn.mass), fptr(s), (float)rtol, fmut(out), iptr(offs),
                                                        iptr(sn.pairs), sn.stride(), stream_of(x)));
-    if (recording(x, s, rho)) {
-        auto n = node_for<FeatureNode>(x, s, rho);
+    if (recording(x, s, rho, sn.mass)) {
+        auto n = node_for<FeatureNode>(x, s, rho, sn.mass);
         n->keep(grid, offs, info, sn.pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
         n->rho_ = SavedVariable(rho, false);
@@ -362,12 +381,12 @@ struct MomentNode : SweepNode {
     variable_list apply(variable_list &&g) override {
         const Tensor x = x_.unpack(), rho = rho_.unpack(), mass = mass_.unpack();
         const bool nx = should_compute_output(0), nr = should_compute_output(1);
-        if (!g[0].defined() || !(nx || nr)) return {Tensor(), Tensor()};
+        if (!g[0].defined() || !(nx || nr)) return variable_list(3);
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = nx ? blank(x) : Tensor(), gr = nr ? blank(rho) : Tensor();
         check_status(npa_moment_matrix_backward(&grid->g, fptr(x), fptr(rho), fptr(mass), fptr(solid(g[0])), fmut(gx), fmut(gr), iptr(offs),
                                                 iptr(info), stream_of(x)));
-        return {gx, gr};
+        return {gx, gr, Tensor()};
     }
     void release_variables() override {
         SweepNode::release_variables();
@@ -384,8 +403,8 @@ Tensor moment_matrix(const GridPtr &grid, const Tensor &offs, const Tensor &info
     c10::cuda::CUDAGuard guard(x.device());
     Tensor out = floats(x, {g.B, g.N, g.D, g.D});
     check_status(npa_moment_matrix_forward(&g.g, fptr(x), fptr(rho), fptr(sn.mass), fmut(out), iptr(offs), iptr(info), stream_of(x)));
-    if (recording(x, rho)) {
-        auto n = node_for<MomentNode>(x, rho);
+    if (recording(x, rho, sn.mass)) {
+        auto n = node_for<MomentNode>(x, rho, sn.mass);
         n->keep(grid, offs, info, Tensor(), x, sn.mass);
         n->rho_ = SavedVariable(rho, false);
         torch::autograd::set_history(out, n);
@@ -422,7 +441,7 @@ struct PerceptionNode : SweepNode {
     variable_list apply(variable_list &&g) override {
         const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(shared_from_this()), mass = mass_.unpack();
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
-        if (!(nx || ns)) return {Tensor(), Tensor()};
+        if (!(nx || ns)) return variable_list(3);
         const Tensor g_rho = nx ? solid(g[0]) : Tensor(), gb = solid(g[1]), gg = solid(g[2]), g_dg = nx && has_dg ? solid(g[3]) : Tensor();
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
@@ -431,12 +450,12 @@ struct PerceptionNode : SweepNode {
             check_status(npa_perception_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(packed), fptr(g_rho),
                                                        fptr(gb), fptr(gg), fptr(g_dg), fmut(gx), fmut(gs), work.mutable_data_ptr(), work.numel() * 4,
                                                        iptr(offs), iptr(pairs), list_stride(), stream_of(x)));
-            return {gx, gs};
+            return {gx, gs, Tensor()};
         }
         Tensor gr = nx ? blank(rho) : Tensor();
         check_status(npa_perception_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(g_rho), fptr(gb), fptr(gg),
                                              fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
-        return {gx, gs};
+        return {gx, gs, Tensor()};
     }
     void release_variables() override {
         SweepNode::release_variables();
@@ -454,7 +473,7 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
     g.features(s, "state_in");
     const int64_t C = s.size(2);
     c10::cuda::CUDAGuard guard(x.device());
-    const bool record = recording(x, s);
+    const bool record = recording(x, s, sn.mass);
     Tensor rho = floats(x, {g.B, g.N}), blur = blank(s), grad = floats(s, {g.B, g.N, C, g.D});
     Tensor dg = want_dg ? floats(x, {g.B, g.N, g.D}) : Tensor(), pairs = new_lists(g, x, columns);
     Tensor packed = columns ? floats(x, {g.B, g.N, 4}) : Tensor();
@@ -465,7 +484,7 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
         check_status(npa_perception_forward(&g.g, (int)C, fptr(x), fptr(sn.mass), fptr(s), fmut(rho), nullptr, fmut(dg), fmut(blur), fmut(grad),
                                             nullptr, iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
     if (record) {
-        auto n = node_for<PerceptionNode>(x, s);
+        auto n = node_for<PerceptionNode>(x, s, sn.mass);
         n->keep(grid, offs, info, pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
         n->has_dg = want_dg;
@@ -488,7 +507,7 @@ struct PackedNode : SweepNode {
     variable_list apply(variable_list &&g) override {
         const Tensor x = x_.unpack(), s = s_.unpack(), mass = mass_.unpack();
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
-        if (!g[0].defined() || !(nx || ns)) return {Tensor(), Tensor()};
+        if (!g[0].defined() || !(nx || ns)) return variable_list(3);
         c10::cuda::CUDAGuard guard(x.device());
         const Tensor gz = g[0].contiguous();
         if (pairs.defined()) {
@@ -497,7 +516,7 @@ struct PackedNode : SweepNode {
                                                               fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, nullptr, fmut(gx), fmut(gs),
                                                               work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
                                                               stream_of(x)));
-            return {gx, gs};
+            return {gx, gs, Tensor()};
         }
         const int64_t n = s.numel(), D = grid->D, rows = rho.numel();
         // dL/dblur and dL/dgradient of the rows, and with position gradients the two per-particle upstreams, in one buffer
@@ -507,7 +526,7 @@ struct PackedNode : SweepNode {
         check_status(npa_perceive_features_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad), fptr(vgrad),
                                                     fptr(gz), coef, dg_scale, ln_grad, ln_dg, gb, gg, g_dg, gr, fmut(gx), fmut(gs), iptr(offs),
                                                     iptr(info), nullptr, 0, stream_of(x)));
-        return {gx, ns ? gs : Tensor()};
+        return {gx, ns ? gs : Tensor(), Tensor()};
     }
     void release_variables() override {
         SweepNode::release_variables();
@@ -525,7 +544,7 @@ Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &
     g.features(s, "state_in");
     const int64_t C = s.size(2), D = g.D;
     c10::cuda::CUDAGuard guard(x.device());
-    const bool record = recording(x, s);
+    const bool record = recording(x, s, sn.mass);
     Tensor rho = floats(x, {g.B, g.N}), rho_grad = floats(x, {g.B, g.N, D}), z = floats(s, {g.B, g.N, 2 * C + C * D + D});
     Tensor vgrad = record ? floats(s, {g.B, g.N, C, D}) : Tensor(), pairs = new_lists(g, x, columns);
     Tensor packed = columns ? floats(x, {g.B, g.N, 4}) : Tensor();
@@ -533,7 +552,7 @@ Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &
                                                      ln_grad, ln_dg, fmut(rho), fmut(rho_grad), fmut(z), fmut(vgrad), fmut(packed), iptr(offs),
                                                      iptr(info), imut(pairs), pairs.defined() ? (int)columns : 0, stream_of(x)));
     if (record) {
-        auto n = node_for<PackedNode>(x, s);
+        auto n = node_for<PackedNode>(x, s, sn.mass);
         n->keep(grid, offs, info, pairs, x, sn.mass);
         n->s_ = SavedVariable(s, false);
         n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad; n->packed = packed;
@@ -560,7 +579,7 @@ struct StepNode : Node {
                              ? npa_step_update_backward_masked(&grid->g, fptr(y), fptr(mask), below, C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y))
                              : npa_step_update_backward(&grid->g, fptr(y), fptr(mask), C, alpha, dt, fptr(gx), fptr(gs), fmut(gy), stream_of(y)));
         }
-        return {gy, should_compute_output(1) ? gx : Tensor(), should_compute_output(2) ? gs : Tensor()};
+        return {gy, should_compute_output(1) ? gx : Tensor(), should_compute_output(2) ? gs : Tensor(), Tensor()};
     }
     void release_variables() override {
         y_.reset_data();
@@ -584,8 +603,8 @@ py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, con
                                                       wrap, fmut(xo), fmut(so), stream_of(x))
                      : npa_step_update_forward(&g.g, fptr(y), fptr(x), fptr(s), fptr(mask), (int)s.size(2), (float)alpha, (float)dt, wrap, fmut(xo),
                                                fmut(so), stream_of(x)));
-    if (recording(y, x, s)) {
-        auto n = node_for<StepNode>(y, x, s);
+    if (recording(y, x, s, mask)) {
+        auto n = node_for<StepNode>(y, x, s, mask);
         n->grid = grid; n->mask = mask; n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)below;
         n->y_ = SavedVariable(y, false);
         torch::autograd::set_history(xo, n);
@@ -850,6 +869,7 @@ PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.def("instantiate", &instantiate);
     m.def("reorder", &reorder);
     m.def("unreorder", &unreorder);
+    m.def("count", &count);
     m.def("density", &density);
     m.def("blur_gradient", &blur_gradient);
     m.def("gradient_hybrid", &gradient_hybrid);

@@ -249,10 +249,8 @@ def unbin_particles(x_bin, s_bin, snapshot, mass_bin=None):
 class Count:
     @staticmethod
     def apply(x_bin, snapshot):
-        # a neighbour count is piecewise constant in the positions: it takes no gradient
-        out = torch.empty(x_bin.shape[:-1], dtype=torch.float32, device=x_bin.device)
-        snapshot.grid.count_forward(x_bin.detach(), out, snapshot.bin_offsets, snapshot.block_info)
-        return out
+        # a neighbour count is piecewise constant in the positions: its node gives no gradient
+        return _ops.count(*_sweep_args(snapshot), x_bin)
 
 
 def count(x_bin, snapshot):

@@ -45,6 +45,7 @@ def _operators():
     first = lambda out: out if isinstance(out, tuple) else (out,)
     ops = {
         "bin_particles": lambda x, s: sph.bin_particles(x, s, snap),
+        "count": lambda x, s: sph.count(x, snap),
         "density": lambda x, s: sph.density(x, snap),
         "density_gradient": lambda x, s: sph.density_gradient(x, snap),
         "blur": lambda x, s: sph.blur(x, rho, s, snap),
@@ -82,3 +83,21 @@ def test_traces_follow_their_inputs():
     for name, f in ops.items():
         traced = torch.jit.trace(f, (x, s), check_trace=False)
         _assert_same(_value_and_grads(lambda x, s: tuple(traced(x, s)), moved, other), _value_and_grads(f, moved, other))
+
+
+def test_outputs_require_a_gradient_wherever_an_input_does():
+    """Also where that input gets none: a count of positions, masses outside the reorder."""
+    sph, grid, x, s = _inputs()
+    snap = grid.instantiate(x)
+    mass = (0.5 + torch.rand(2, 601, device="cuda")).requires_grad_(True)
+    xb, sb, mb = sph.bin_particles(x, s, snap, mass)
+    xb, sb = xb.detach(), sb.detach()
+    rho = sph.density(xb, snap, mb)
+    outs = [rho, sph.density_gradient(xb, snap, mb), sph.blur(xb, rho.detach(), sb, snap, mb), sph.gradient(xb, rho.detach(), sb, snap, mb),
+            sph.gradient_hybrid(xb, rho.detach(), sb, snap, mb), sph.moment_matrix(xb, rho.detach(), snap, mb),
+            *sph.perceive(xb, sb, snap, mb), sph.perceive_features(xb, sb, snap, 0.125, mb),
+            sph.count(xb.clone().requires_grad_(True), snap)]
+    for out in outs:
+        assert out.requires_grad
+        out.sum().backward(retain_graph=True)
+    assert mass.grad is None or not mass.grad.any()

@@ -114,6 +114,7 @@ def test_forward_mode_derivatives_are_refused():
         x, s, rho = dual(2, 16, 2), f(2, 16, 4), f(2, 16)
         calls = {
             "reorder": (grid.hashgrid.native, f(2, 16, dtype=torch.int32), x, s, None),
+            "count": (*sweep, x),
             "density": (*sweep, x, None, None, True, False, False),
             "blur_gradient": (*sweep, f(2, 16, 2), dual(2, 16), s, None, None, False, True, False, False),
             "gradient_hybrid": (*sweep, x, rho, s, None, f(2, 16, 128, dtype=torch.int32), 1e-3),
