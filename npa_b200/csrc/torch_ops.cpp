@@ -121,6 +121,11 @@ bool recording(const In &...inputs) {
     return at::GradMode::is_enabled() && (wants_grad(inputs) || ...);
 }
 
+// What a backward reads of the forward is kept as SavedVariable, so that saved-tensor hooks see it: they move it to the
+// host, or drop and recompute it (checkpointing), and changes in place are noticed.  Outside are the snapshot's arrays and
+// neighbour lists that operators share: whether an operator finds lists may differ between a forward and its recomputation.
+SavedVariable saved(const Tensor &t) { return SavedVariable(t, false); }
+
 // What every node of a neighbour sweep keeps: the grid, the snapshot arrays, the neighbour lists.
 struct SweepNode : Node {
     GridPtr grid;
@@ -128,14 +133,14 @@ struct SweepNode : Node {
     SavedVariable x_, mass_;
     void keep(const GridPtr &g, const Tensor &o, const Tensor &i, const Tensor &p, const Tensor &x, const Tensor &mass) {
         grid = g; offs = o; info = i; pairs = p;
-        x_ = SavedVariable(x, false);
-        mass_ = SavedVariable(mass, false);
+        x_ = saved(x);
+        mass_ = saved(mass);
     }
     void release_variables() override {
         x_.reset_data(); mass_.reset_data();
         pairs = Tensor();
     }
-    int list_stride() const { return pairs.defined() ? (int)pairs.size(2) : 0; }
+    static int list_stride(const Tensor &pairs) { return pairs.defined() ? (int)pairs.size(2) : 0; }
 };
 
 struct Snap {  // arguments every sweep shares, checked
@@ -257,7 +262,7 @@ struct DensityNode : SweepNode {
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = blank(x);
         check_status(npa_density_chain_backward(&grid->g, fptr(x), fptr(mass), fptr(g_rho), nullptr, fptr(g_dg), fmut(gx), 0, iptr(offs),
-                                                iptr(info), iptr(pairs), list_stride(), stream_of(x)));
+                                                iptr(info), iptr(pairs), list_stride(pairs), stream_of(x)));
         return {gx, Tensor()};
     }
 };
@@ -304,7 +309,7 @@ struct FeatureNode : SweepNode {
         if (C > 0 && pairs.defined()) {
             Tensor work = list_scratch(*grid, s, C);
             check_status(npa_blur_gradient_backward_lists(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
-                                                          fmut(gr), work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
+                                                          fmut(gr), work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(pairs),
                                                           stream_of(x)));
         } else if (C > 0) {
             check_status(npa_blur_gradient_backward(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
@@ -338,8 +343,8 @@ py::tuple blur_gradient(const GridPtr &grid, const Tensor &offs, const Tensor &i
     if (recording(x, s, rho, sn.mass)) {
         auto n = node_for<FeatureNode>(x, s, rho, sn.mass);
         n->keep(grid, offs, info, sn.pairs, x, sn.mass);
-        n->s_ = SavedVariable(s, false);
-        n->rho_ = SavedVariable(rho, false);
+        n->s_ = saved(s);
+        n->rho_ = saved(rho);
         n->has_blur = want_blur; n->has_grad = want_grad;
         if (want_blur) torch::autograd::set_history(blur, n);
         if (want_grad) torch::autograd::set_history(grad, n);
@@ -367,8 +372,8 @@ Tensor gradient_hybrid(const GridPtr &grid, const Tensor &offs, const Tensor &in
     if (recording(x, s, rho, sn.mass)) {
         auto n = node_for<FeatureNode>(x, s, rho, sn.mass);
         n->keep(grid, offs, info, sn.pairs, x, sn.mass);
-        n->s_ = SavedVariable(s, false);
-        n->rho_ = SavedVariable(rho, false);
+        n->s_ = saved(s);
+        n->rho_ = saved(rho);
         n->has_blur = false; n->has_grad = true;
         torch::autograd::set_history(out, n);
     }
@@ -406,7 +411,7 @@ Tensor moment_matrix(const GridPtr &grid, const Tensor &offs, const Tensor &info
     if (recording(x, rho, sn.mass)) {
         auto n = node_for<MomentNode>(x, rho, sn.mass);
         n->keep(grid, offs, info, Tensor(), x, sn.mass);
-        n->rho_ = SavedVariable(rho, false);
+        n->rho_ = saved(rho);
         torch::autograd::set_history(out, n);
     }
     return out;
@@ -435,11 +440,11 @@ Tensor corrected_gradient(const Tensor &raw, const Tensor &moment, double rtol) 
 
 // ---- the fused perception step -------------------------------------------------------------------------
 struct PerceptionNode : SweepNode {
-    SavedVariable s_, rho_;
-    Tensor packed;  // (x, y, z, m / rho) records of the density sweep
+    SavedVariable s_, rho_, packed_, pairs_;  // packed: (x, y, z, m / rho) records of the density sweep
     bool has_dg;
     variable_list apply(variable_list &&g) override {
-        const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(shared_from_this()), mass = mass_.unpack();
+        const Tensor x = x_.unpack(), s = s_.unpack(), rho = rho_.unpack(shared_from_this()), mass = mass_.unpack(), packed = packed_.unpack(),
+                     pairs = pairs_.unpack();
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
         if (!(nx || ns)) return variable_list(3);
         const Tensor g_rho = nx ? solid(g[0]) : Tensor(), gb = solid(g[1]), gg = solid(g[2]), g_dg = nx && has_dg ? solid(g[3]) : Tensor();
@@ -449,7 +454,7 @@ struct PerceptionNode : SweepNode {
             Tensor work = list_scratch(*grid, s, s.size(2));
             check_status(npa_perception_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(packed), fptr(g_rho),
                                                        fptr(gb), fptr(gg), fptr(g_dg), fmut(gx), fmut(gs), work.mutable_data_ptr(), work.numel() * 4,
-                                                       iptr(offs), iptr(pairs), list_stride(), stream_of(x)));
+                                                       iptr(offs), iptr(pairs), list_stride(pairs), stream_of(x)));
             return {gx, gs, Tensor()};
         }
         Tensor gr = nx ? blank(rho) : Tensor();
@@ -459,8 +464,7 @@ struct PerceptionNode : SweepNode {
     }
     void release_variables() override {
         SweepNode::release_variables();
-        s_.reset_data(); rho_.reset_data();
-        packed = Tensor();
+        s_.reset_data(); rho_.reset_data(); packed_.reset_data(); pairs_.reset_data();
     }
 };
 
@@ -485,10 +489,11 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
                                             nullptr, iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
     if (record) {
         auto n = node_for<PerceptionNode>(x, s, sn.mass);
-        n->keep(grid, offs, info, pairs, x, sn.mass);
-        n->s_ = SavedVariable(s, false);
+        n->keep(grid, offs, info, Tensor(), x, sn.mass);
+        n->pairs_ = saved(pairs);
+        n->s_ = saved(s);
         n->has_dg = want_dg;
-        n->packed = packed;
+        n->packed_ = saved(packed);
         torch::autograd::set_history(rho, n);
         torch::autograd::set_history(blur, n);
         torch::autograd::set_history(grad, n);
@@ -500,12 +505,12 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
 
 // ---- the packed perception row ---------------------------------------------------------------------------
 struct PackedNode : SweepNode {
-    SavedVariable s_;
-    Tensor rho, rho_grad, vgrad, packed;
+    SavedVariable s_, rho_, rho_grad_, vgrad_, packed_, pairs_;
     float coef, dg_scale;
     bool ln_grad, ln_dg;
     variable_list apply(variable_list &&g) override {
-        const Tensor x = x_.unpack(), s = s_.unpack(), mass = mass_.unpack();
+        const Tensor x = x_.unpack(), s = s_.unpack(), mass = mass_.unpack(), rho = rho_.unpack(), rho_grad = rho_grad_.unpack(), vgrad = vgrad_.unpack(),
+                     packed = packed_.unpack(), pairs = pairs_.unpack();
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
         if (!g[0].defined() || !(nx || ns)) return variable_list(3);
         c10::cuda::CUDAGuard guard(x.device());
@@ -514,7 +519,7 @@ struct PackedNode : SweepNode {
             Tensor work = list_scratch(*grid, s, s.size(2)), gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
             check_status(npa_perceive_features_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad),
                                                               fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, nullptr, fmut(gx), fmut(gs),
-                                                              work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(),
+                                                              work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(pairs),
                                                               stream_of(x)));
             return {gx, gs, Tensor()};
         }
@@ -530,8 +535,7 @@ struct PackedNode : SweepNode {
     }
     void release_variables() override {
         SweepNode::release_variables();
-        s_.reset_data();
-        rho = rho_grad = vgrad = packed = Tensor();
+        s_.reset_data(); rho_.reset_data(); rho_grad_.reset_data(); vgrad_.reset_data(); packed_.reset_data(); pairs_.reset_data();
     }
 };
 
@@ -553,9 +557,10 @@ Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &
                                                      iptr(info), imut(pairs), pairs.defined() ? (int)columns : 0, stream_of(x)));
     if (record) {
         auto n = node_for<PackedNode>(x, s, sn.mass);
-        n->keep(grid, offs, info, pairs, x, sn.mass);
-        n->s_ = SavedVariable(s, false);
-        n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad; n->packed = packed;
+        n->keep(grid, offs, info, Tensor(), x, sn.mass);
+        n->pairs_ = saved(pairs);
+        n->s_ = saved(s);
+        n->rho_ = saved(rho); n->rho_grad_ = saved(rho_grad); n->vgrad_ = saved(vgrad); n->packed_ = saved(packed);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->ln_grad = ln_grad; n->ln_dg = ln_dg;
         torch::autograd::set_history(z, n);
     }
@@ -565,12 +570,11 @@ Tensor packed_perception(const GridPtr &grid, const Tensor &offs, const Tensor &
 // ---- the Euler update --------------------------------------------------------------------------------------
 struct StepNode : Node {
     GridPtr grid;
-    SavedVariable y_;
-    Tensor mask;
+    SavedVariable y_, mask_;
     int C;
     float alpha, dt, below;  // below >= 0: the mask is uniforms, a particle updates where its value is below it
     variable_list apply(variable_list &&g) override {
-        const Tensor y = y_.unpack(), gx = solid(g[0]), gs = solid(g[1]);
+        const Tensor y = y_.unpack(), mask = mask_.unpack(), gx = solid(g[0]), gs = solid(g[1]);
         Tensor gy;
         if (should_compute_output(0) && (gx.defined() || gs.defined())) {
             c10::cuda::CUDAGuard guard(y.device());
@@ -582,8 +586,7 @@ struct StepNode : Node {
         return {gy, should_compute_output(1) ? gx : Tensor(), should_compute_output(2) ? gs : Tensor(), Tensor()};
     }
     void release_variables() override {
-        y_.reset_data();
-        mask = Tensor();
+        y_.reset_data(); mask_.reset_data();
     }
 };
 
@@ -605,8 +608,8 @@ py::tuple step_update(const GridPtr &grid, const Tensor &y, const Tensor &x, con
                                                fmut(so), stream_of(x)));
     if (recording(y, x, s, mask)) {
         auto n = node_for<StepNode>(y, x, s, mask);
-        n->grid = grid; n->mask = mask; n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)below;
-        n->y_ = SavedVariable(y, false);
+        n->grid = grid; n->mask_ = saved(mask); n->C = (int)s.size(2); n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)below;
+        n->y_ = saved(y);
         torch::autograd::set_history(xo, n);
         torch::autograd::set_history(so, n);
     }
@@ -643,11 +646,10 @@ struct Slab {
 };
 
 struct MlpNode : Node {
-    SavedVariable z_, w1_, w2_;
-    Tensor h, dz_image;  // hidden layer; W1 as the tensor cores read it for dz = dh W1
+    SavedVariable z_, w1_, w2_, h_, dz_image_;  // h: hidden layer; dz_image: W1 as the tensor cores read it for dz = dh W1
     std::vector<int64_t> z_shape;
     variable_list apply(variable_list &&g) override {
-        const Tensor z = z_.unpack(), w1 = w1_.unpack(), w2 = w2_.unpack();
+        const Tensor z = z_.unpack(), w1 = w1_.unpack(), w2 = w2_.unpack(), h = h_.unpack(), dz_image = dz_image_.unpack();
         if (!g[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(z.device());
         const Tensor dy = g[0].contiguous();
@@ -668,8 +670,7 @@ struct MlpNode : Node {
         return {gz, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
     }
     void release_variables() override {
-        z_.reset_data(); w1_.reset_data(); w2_.reset_data();
-        h = dz_image = Tensor();
+        z_.reset_data(); w1_.reset_data(); w2_.reset_data(); h_.reset_data(); dz_image_.reset_data();
     }
 };
 
@@ -691,8 +692,8 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
                                                 stream_of(z)));
     if (record) {
         auto n = node_for<MlpNode>(z, w1, b1, w2);
-        n->z_ = SavedVariable(z, false); n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
-        n->h = h; n->dz_image = dz_image; n->z_shape = z.sizes().vec();
+        n->z_ = saved(z); n->w1_ = saved(w1); n->w2_ = saved(w2);
+        n->h_ = saved(h); n->dz_image_ = saved(dz_image); n->z_shape = z.sizes().vec();
         torch::autograd::set_history(y, n);
     }
     return y;
@@ -705,18 +706,20 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
 // the perception's backward).
 struct EulerNode : Node {
     GridPtr grid;
-    SavedVariable w1_, w2_;
-    Tensor offs, perm, slab, mask;
-    const float *x_bin, *s_bin, *rho, *rho_grad, *vgrad, *packed, *z, *h, *y, *dz_image;  // in the slab
-    const int32_t *pairs;
+    SavedVariable w1_, w2_, slab_, mask_;
+    Tensor offs, perm;
+    int64_t o_x, o_s, o_rho, o_dg, o_v, o_packed, o_z, o_h, o_y, o_dz, o_pairs;  // places in the slab, in floats
     int64_t C, columns, dz_bytes;
     float coef, dg_scale, alpha, dt, below;
     bool ln_grad, ln_dg, stop_pos, stop_state;
 
     variable_list apply(variable_list &&g) override {
-        const Tensor w1 = w1_.unpack(), w2 = w2_.unpack();  // raise when the graph was released
+        const Tensor w1 = w1_.unpack(), w2 = w2_.unpack(), slab = slab_.unpack(), mask = mask_.unpack();  // raise when the graph was released
         const Tensor gx_new = solid(g[0]), gs_new = solid(g[1]);
         if (!gx_new.defined() && !gs_new.defined()) return variable_list(5);
+        const float *kept = fptr(slab), *x_bin = kept + o_x, *s_bin = kept + o_s, *rho = kept + o_rho, *rho_grad = kept + o_dg, *vgrad = kept + o_v,
+                    *packed = kept + o_packed, *z = kept + o_z, *h = kept + o_h, *y = kept + o_y, *dz_image = kept + o_dz;
+        const int32_t *pairs = reinterpret_cast<const int32_t *>(kept + o_pairs);
         c10::cuda::CUDAGuard guard(slab.device());
         void *st = stream_of(slab);
         Grid &gr = *grid;
@@ -768,8 +771,7 @@ struct EulerNode : Node {
         return {gx, gs, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};
     }
     void release_variables() override {
-        w1_.reset_data(); w2_.reset_data();
-        slab = mask = Tensor();
+        w1_.reset_data(); w2_.reset_data(); slab_.reset_data(); mask_.reset_data();
     }
 };
 
@@ -810,10 +812,10 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
                                 : npa_step_update_forward(&g.g, y, x_bin, s_bin, nullptr, (int)C, (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st));
     if (record) {
         auto n = node_for<EulerNode>(x, s, w1, b1, w2);
-        n->grid = grid; n->offs = offs; n->perm = perm; n->slab = slab; n->mask = mask;
-        n->x_bin = x_bin; n->s_bin = s_bin; n->rho = rho; n->rho_grad = rho_grad; n->vgrad = vgrad; n->packed = packed; n->z = z; n->h = h; n->y = y;
-        n->dz_image = dz_image; n->pairs = pairs; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
-        n->w1_ = SavedVariable(w1, false); n->w2_ = SavedVariable(w2, false);
+        n->grid = grid; n->offs = offs; n->perm = perm; n->slab_ = saved(slab); n->mask_ = saved(mask);
+        n->o_x = o_x; n->o_s = o_s; n->o_rho = o_rho; n->o_dg = o_dg; n->o_v = o_v; n->o_packed = o_packed; n->o_z = o_z; n->o_h = o_h; n->o_y = o_y;
+        n->o_dz = o_dz; n->o_pairs = o_pairs; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
+        n->w1_ = saved(w1); n->w2_ = saved(w2);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
         n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;
         torch::autograd::set_history(xo, n);
@@ -854,7 +856,7 @@ Tensor splat(const Tensor &x, const Tensor &color, int img, double sigma, int ra
                                    stream_of(x)));
     if (recording(x, color)) {
         auto node = node_for<SplatNode>(x, color);
-        node->x_ = SavedVariable(x, false); node->color_ = SavedVariable(color, false);
+        node->x_ = saved(x); node->color_ = saved(color);
         node->c = SplatConsts{img, radius, y_up ? 1 : 0, normalize ? 1 : 0, sigma, lo, hi, scale};
         torch::autograd::set_history(out, node);
     }

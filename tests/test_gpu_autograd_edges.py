@@ -101,3 +101,83 @@ def test_outputs_require_a_gradient_wherever_an_input_does():
         assert out.requires_grad
         out.sum().backward(retain_graph=True)
     assert mass.grad is None or not mass.grad.any()
+
+
+class _Model(torch.nn.Module):
+    """What step_euler reads of a model, in 2D with 8 channels."""
+
+    def __init__(self, eps, seed=0):
+        super().__init__()
+        torch.manual_seed(seed)
+        self.spatial_dims, self.eps0, self.alpha = 2, eps, 1.0
+        self.state_grad = self.density_grad = self.log_norm_grad = self.log_norm_density_grad = True
+        self.stopgrad_pos, self.stopgrad_state = False, False
+        self.model = torch.nn.Sequential(torch.nn.Linear(34, 128), torch.nn.ReLU(), torch.nn.Linear(128, 10, bias=False)).cuda()
+
+
+def _steps():
+    """The step as one node and as four, as functions of positions and features."""
+    from npa_b200 import stepping
+    _, grid, x, s = _inputs()
+    model = _Model(grid.eps)
+
+    def step(x, s, intermediate):
+        torch.manual_seed(3)
+        return stepping.step_euler(model, x, s, grid, update_prob=0.5, intermediate=intermediate)[:2]
+
+    return x, s, {"step": lambda x, s: step(x, s, False), "four_nodes": lambda x, s: step(x, s, True)}, grid
+
+
+def test_saved_tensor_hooks_see_what_the_backward_reads():
+    """Everything large moves to the host and comes back at another address; the gradients are the same bits."""
+    x, s, ops = _operators()
+    x2, s2, steps, _ = _steps()
+    for name, f in {**ops, **steps}.items():
+        a, b = (x2, s2) if name in steps else (x, s)
+        want = _value_and_grads(f, a, b)
+        packed = []
+
+        def pack(t):
+            packed.append(t.numel() * t.element_size())
+            return t.cpu()
+
+        with torch.autograd.graph.saved_tensors_hooks(pack, lambda t: t.cuda()):
+            got = _value_and_grads(f, a, b)
+        for p, q in zip([*got[0], *got[1]], [*want[0], *want[1]]):
+            assert p is q is None or torch.equal(p, q), name
+        if name in steps:  # the hidden layer alone is 128 floats per particle
+            assert sum(packed) > a.shape[0] * a.shape[1] * 128 * 4
+
+
+@pytest.mark.parametrize("name", ["step", "four_nodes"])
+def test_checkpointed_steps_do_not_keep_what_they_recompute(name):
+    from torch.utils.checkpoint import checkpoint
+    x, s, steps, grid = _steps()
+    f = steps[name]
+
+    def rollout(call):
+        a, b = x.clone().requires_grad_(True), s.clone().requires_grad_(True)
+        p, q = a, b
+        base = torch.cuda.memory_allocated()
+        for _ in range(4):
+            p, q = call(p, q)
+        kept = torch.cuda.memory_allocated() - base
+        return [p.detach(), q.detach()], torch.autograd.grad([p, q], [a, b], [torch.ones_like(p), torch.ones_like(q)]), kept
+
+    plain = rollout(f)
+    again = rollout(lambda p, q: checkpoint(f, p, q, use_reentrant=False))
+    for p, q in zip([*again[0], *again[1]], [*plain[0], *plain[1]]):
+        assert torch.equal(p, q)
+    assert again[2] < plain[2] // 3, (again[2], plain[2])
+
+
+def test_a_mask_changed_in_place_is_noticed():
+    sph, grid, x, s = _inputs()
+    snap = grid.instantiate(x)
+    xb, sb = sph.bin_particles(x, s, snap)
+    y = torch.randn(2, 601, 10, device="cuda", requires_grad=True)
+    mask = torch.ones(2, 601, 1, device="cuda")
+    out = sph.step_update(y, xb, sb, snap, 1.0, 1.0, mask)
+    mask.zero_()
+    with pytest.raises(RuntimeError, match="modified by an inplace operation"):
+        out[1].sum().backward()
