@@ -418,7 +418,7 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
             // (rows of particles without a list are written again by the search that follows)
             const int floats = min(PP, total - first) * Z;
             float *out = a.z + (long long)first * Z;
-            if (PP % 4 == 0) {  // first is a multiple of four rows: 16-byte aligned
+            if (PP % 4 == 0 && a.out_vec) {  // first is a multiple of four rows: 16-byte aligned when z is
                 const int quads = floats / 4;
                 for (int q = lane; q < quads; q += 32) reinterpret_cast<float4 *>(out)[q] = reinterpret_cast<const float4 *>(stage)[q];
                 for (int q = quads * 4 + lane; q < floats; q += 32) out[q] = stage[q];
@@ -841,9 +841,10 @@ int launch_list_forward_mask(const Geom &g, int mask, const FeatureFwdArgs &a, c
     } while (0)
 
 template <int D, bool PER>
-int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st) {
-    const uintptr_t bits = (uintptr_t)a.s | (uintptr_t)a.blur | (uintptr_t)a.grad | (uintptr_t)a.vgrad;
-    if ((mask & F_PACK) && ((uintptr_t)a.z % 16)) return fail(NPA_ERR_INVALID_ARGUMENT, "the packed row tensor must be 16-byte aligned");
+int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdArgs &args, cudaStream_t st) {
+    const uintptr_t bits = (uintptr_t)args.s | (uintptr_t)args.blur | (uintptr_t)args.grad | (uintptr_t)args.vgrad;
+    FeatureFwdArgs a = args;
+    a.out_vec = (uintptr_t)a.z % 16 == 0;
     if (a.C % 4 == 0 && bits % 16 == 0) {
 #define NPA_CALL(L) launch_list_forward_mask<D, PER, L, true>(g, mask, a, st)
         NPA_LIST_LPP(a.C, NPA_CALL);

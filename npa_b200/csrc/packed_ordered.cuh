@@ -57,8 +57,8 @@ struct Ordered {
     unsigned long long nsi[H], acc[CPL][1 + D][H];
     float mom[2][NM], dgs[2][3];
 
-    __device__ inline void begin(const float *__restrict__ row, int f, int C) {
-        load(row, f, C, si);
+    __device__ inline void begin(const float *__restrict__ row, int f, int C, int vec) {
+        load(row, f, C, vec, si);
 #pragma unroll
         for (int h = 0; h < H; ++h) nsi[h] = pack2(-si[2 * h], -si[2 * h + 1]);
 #pragma unroll
@@ -74,9 +74,9 @@ struct Ordered {
             dgs[k][0] = dgs[k][1] = dgs[k][2] = 0.f;
         }
     }
-    // Lanes beyond the last feature read valid neighbours of it (unused).
-    static __device__ inline void load(const float *__restrict__ row, int f, int C, float (&v)[VW]) {
-        if (C % VW == 0) {
+    // Lanes beyond the last feature read valid neighbours of it (unused).  vec: rows are whole vectors at aligned addresses.
+    static __device__ inline void load(const float *__restrict__ row, int f, int C, int vec, float (&v)[VW]) {
+        if (vec) {
             if constexpr (VW == 4) {
                 const float4 t = __ldg(reinterpret_cast<const float4 *>(row + min(f, C - 4)));
                 v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
@@ -116,11 +116,11 @@ struct Ordered {
         return make_float4(kv * rx, kv * ry, kv * rz, w);
     }
     // STEP entries from a position that is a multiple of CLS; this group's are CPL in a row of each block of CLS.
-    __device__ inline void add(const float4 *__restrict__ ent, const int (&js)[U], const float *__restrict__ s, int f, int C) {
+    __device__ inline void add(const float4 *__restrict__ ent, const int (&js)[U], const float *__restrict__ s, int f, int C, int vec) {
         float r[U][VW];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            load(reinterpret_cast<const float *>(reinterpret_cast<const char *>(s) + (unsigned long long)(unsigned)js[u] * ((unsigned)C * 4u)), f, C, r[u]);
+            load(reinterpret_cast<const float *>(reinterpret_cast<const char *>(s) + (unsigned long long)(unsigned)js[u] * ((unsigned)C * 4u)), f, C, vec, r[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const float4 e = ent[u / CPL * CLS + u % CPL];
@@ -201,7 +201,7 @@ struct Ordered {
         }
         if (a.vgrad && valid) {
             float *o = a.vgrad + (i * C + f) * D;
-            if (OWN == 2 && C % 2 == 0) {
+            if (OWN == 2 && C % 2 == 0 && a.out_vec) {
                 if (f < C) {
                     auto at = [&](int e) { return val[e / D][1 + e % D]; };
 #pragma unroll
@@ -242,7 +242,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
     __syncwarp();
     const int nr = build_ranges<D>(g, a.bin_offsets, it, mem.rng);
     O o;
-    o.begin(a.s + (long long)i * C, f, C);
+    o.begin(a.s + (long long)i * C, f, C, a.row_vec);
     collect_pairs<D, PER>(g, a.x, pi, mem.rng, nr, mem.geo, [&](int n) {
         __syncwarp();
         const int filled = (n + O::STEP - 1) / O::STEP * O::STEP;  // kListPerWarp is a multiple of STEP
@@ -263,7 +263,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
             int js[O::U];
 #pragma unroll
             for (int u = 0; u < O::U; ++u) js[u] = __float_as_int(mem.geo[e + u / CPL * O::CLS + u % CPL].w);
-            o.add(mem.ent + e, js, a.s, f, C);
+            o.add(mem.ent + e, js, a.s, f, C, a.row_vec);
         }
         __syncwarp();
     });
@@ -295,7 +295,7 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
     indices(0);
     const Pos<D> pi = load_pos<D>(a.x, i);
     O o;
-    o.begin(a.s + (long long)i * C, f, C);
+    o.begin(a.s + (long long)i * C, f, C, a.row_vec);
     const bool search = count < 0 || count > room;
     const int n = search ? 0 : count, nmax = __reduce_max_sync(kFull, n);
     float4 *ent = mem.ent + sg * 33;
@@ -339,19 +339,19 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
                     js[u] = idx[e + u * O::CLS];
                 }
             }
-            o.add(ent + e, js, a.s, f, C);
+            o.add(ent + e, js, a.s, f, C, a.row_vec);
         }
         __syncwarp();
     }
     const int Z = a.zstride;
     o.template finish<false>(a, g, i, valid && !search, f, sl, mem.rows + sg * Z);
     __syncwarp();
-    // the rows of both particles are one run (8-byte aligned: first is even); the row of a particle that is searched is
-    // written again below
-    const int floats = min(2, total - first) * Z;
+    // the rows of both particles are one run (8-byte aligned when z is: first is even); the row of a particle that is
+    // searched is written again below
+    const int floats = min(2, total - first) * Z, pairs = a.out_vec ? floats / 2 : 0;
     float *out = a.z + (long long)first * Z;
-    for (int q = lane; q < floats / 2; q += 32) reinterpret_cast<float2 *>(out)[q] = reinterpret_cast<const float2 *>(mem.rows)[q];
-    if ((floats & 1) && lane == 0) out[floats - 1] = mem.rows[floats - 1];
+    for (int q = lane; q < pairs; q += 32) reinterpret_cast<float2 *>(out)[q] = reinterpret_cast<const float2 *>(mem.rows)[q];
+    for (int q = 2 * pairs + lane; q < floats; q += 32) out[q] = mem.rows[q];
     const unsigned again = __ballot_sync(kFull, search && valid);
     if (again & 0x0000ffffu) ordered_search<D, PER, VW, LPR, CPL>(a, g, mem, first);
     if (again & 0xffff0000u) ordered_search<D, PER, VW, LPR, CPL>(a, g, mem, first + 1);
@@ -360,12 +360,16 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
 template <int D, bool PER, int VW, int LPR, int CPL>
 int launch_packed_ordered_shape(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
     const long long particles = (long long)g.B * g.N;
-    packed_ordered_kernel<D, PER, VW, LPR, CPL><<<(unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st>>>(a, g);
+    FeatureFwdArgs b = a;
+    b.row_vec = a.C % VW == 0 && (uintptr_t)a.s % (VW * 4) == 0;
+    b.out_vec = ((uintptr_t)a.z | (uintptr_t)a.vgrad) % 8 == 0;
+    packed_ordered_kernel<D, PER, VW, LPR, CPL><<<(unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st>>>(b, g);
     return check_launch("packed_ordered_kernel");
 }
 
-// Up to 32 features.  The classes: 32 / (lanes that cover a row, four features each); without vector loads four for up
-// to eight features and one beyond.
+// Up to 32 features.  The classes: 32 / (lanes that cover a row, four features each); with a count that is not a multiple of
+// four, four for up to eight features and one beyond.  They depend on the count alone: rows at an address that vectors
+// cannot be loaded from are read float by float into the same sums.
 template <int D, bool PER>
 int launch_packed_ordered_geom(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
     if (a.C % 4 == 0) {
