@@ -537,6 +537,8 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     if ((x == nullptr) != (xo == nullptr) || (s == nullptr) != (so == nullptr) || (m == nullptr) != (mo == nullptr))
         return fail(NPA_ERR_INVALID_ARGUMENT, "each input of a permutation needs its output (and vice versa)");
     if (s && C <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "channels must be positive, got %d", C);
+    if (((uintptr_t)x | (uintptr_t)xo) % (g.dim == 2 ? 8 : 16))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "positions to permute must be aligned to one position (%d bytes)", g.dim == 2 ? 8 : 16);
     const bool vec = s && (C % 4 == 0) && ((((uintptr_t)s) | ((uintptr_t)so)) % 16 == 0);
     const int pieces = s ? (vec ? C / 4 : C) : 1;
     const long long total = (long long)g.B * g.N * pieces;

@@ -59,7 +59,12 @@ float *fmut(const Tensor &t) { return t.defined() ? t.mutable_data_ptr<float>() 
 const int32_t *iptr(const Tensor &t) { return t.defined() ? t.const_data_ptr<int32_t>() : nullptr; }
 int32_t *imut(const Tensor &t) { return t.defined() ? t.mutable_data_ptr<int32_t>() : nullptr; }
 Tensor or_none(const OptTensor &t) { return t.has_value() ? *t : Tensor(); }
-Tensor solid(const Tensor &t) { return t.defined() ? t.contiguous() : t; }
+// An upstream gradient as the kernels read it: contiguous, and at an address that any vector load can use.
+Tensor solid(const Tensor &t) {
+    if (!t.defined()) return t;
+    const Tensor c = t.contiguous();
+    return (uintptr_t)c.const_data_ptr() % 16 ? c.clone() : c;
+}
 void *stream_of(const Tensor &t) { return c10::cuda::getCurrentCUDAStream(t.device().index()).stream(); }
 Tensor floats(const Tensor &like, at::IntArrayRef shape) { return at::empty(shape, like.options().dtype(at::kFloat).requires_grad(false)); }
 Tensor blank(const Tensor &like) { return floats(like, like.sizes()); }
@@ -180,7 +185,7 @@ struct ReorderNode : Node {
         c10::cuda::CUDAGuard guard(perm.device());
         auto upstream = [&](const Tensor &t, const std::vector<int64_t> &shape, bool need) {
             if (!need) return Tensor();
-            return t.defined() ? t.contiguous() : at::zeros(shape, opt);
+            return t.defined() ? solid(t) : at::zeros(shape, opt);
         };
         const bool nx = should_compute_output(0), ns = should_compute_output(1), nm = !ms.empty() && should_compute_output(2);
         const Tensor gx = upstream(g[0], xs, nx), gs = upstream(g[1], ss, ns), gm = ms.empty() ? Tensor() : upstream(g[2], ms, nm);
@@ -514,7 +519,7 @@ struct PackedNode : SweepNode {
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
         if (!g[0].defined() || !(nx || ns)) return variable_list(3);
         c10::cuda::CUDAGuard guard(x.device());
-        const Tensor gz = g[0].contiguous();
+        const Tensor gz = solid(g[0]);
         if (pairs.defined()) {
             Tensor work = list_scratch(*grid, s, s.size(2)), gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
             check_status(npa_perceive_features_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad),
@@ -652,7 +657,7 @@ struct MlpNode : Node {
         const Tensor z = z_.unpack(), w1 = w1_.unpack(), w2 = w2_.unpack(), h = h_.unpack(), dz_image = dz_image_.unpack();
         if (!g[0].defined()) return {Tensor(), Tensor(), Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(z.device());
-        const Tensor dy = g[0].contiguous();
+        const Tensor dy = solid(g[0]);
         const int64_t k = z.size(-1), m = z.numel() / k, o = w2.size(0);
         void *st = stream_of(z);
         Tensor dh = floats(z, {m, kHidden});
@@ -838,7 +843,7 @@ struct SplatNode : Node {
         const bool nx = should_compute_output(0), nc = should_compute_output(1);
         if (!g[0].defined() || !(nx || nc)) return {Tensor(), Tensor()};
         c10::cuda::CUDAGuard guard(x.device());
-        const Tensor up = g[0].contiguous();
+        const Tensor up = solid(g[0]);
         Tensor gx = nx ? blank(x) : Tensor(), gc = nc ? blank(color) : Tensor();
         check_status(npa_splat_backward(fptr(x), fptr(color), fptr(up), (int)x.size(0), (int)x.size(1), c.img, c.sigma, c.radius, c.lo, c.hi, c.y_up,
                                         c.normalize, c.scale, fmut(gx), fmut(gc), stream_of(x)));

@@ -52,6 +52,18 @@ def test_geometry_queries_and_errors():
     assert rc == n.NPA_ERR_INVALID_ARGUMENT and "2x2 or 3x3" in n.last_error()
 
 
+def test_misaligned_positions_are_refused_before_any_launch():
+    """The reorder moves a position as one vector; addresses here are never dereferenced (the check comes first)."""
+    from npa_b200 import _native as n
+    for dim, width in ((2, 8), (3, 16)):
+        g = n.make_grid(dim, "clamped", "grid", (8,) * dim, 0.1, 1, 8, 32)
+        ok, off = ctypes.c_void_p(1 << 20), ctypes.c_void_p((1 << 20) + width // 2)
+        for call in (n.lib.npa_bin_particles, n.lib.npa_unbin_particles):
+            for x, xo in ((off, ok), (ok, off)):
+                rc = call(ctypes.byref(g), 4, x, None, None, ok, xo, None, None, None)
+                assert rc == n.NPA_ERR_INVALID_ARGUMENT and "aligned" in n.last_error()
+
+
 def test_hashgrid_host_side_contract():
     from npa_b200 import sphops as sph
     grid = sph.HashGrid(dim=2, boundary="clamped", mode="grid", grid_size=(16, 16), eps=0.1,

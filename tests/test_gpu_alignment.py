@@ -64,3 +64,40 @@ def test_packed_perception_into_outputs_at_any_address(C):
         outs.append((zo, vo, rho, dg))
     for a, b in zip(*outs):
         assert torch.allclose(a, b, rtol=1e-5, atol=1e-6 * float(b.abs().max()))
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_upstream_gradients_at_any_address(dim):
+    from npa_b200 import splatting, stepping
+    sph, grid, snap, xb, sb = _setup(dim, 8)
+    rho = sph.density(xb, snap).detach()
+    y = torch.randn(2, 333, dim + 8, device="cuda")
+    calls = [
+        lambda x, s: sph.bin_particles(x, s, snap), lambda x, s: sph.perceive(x, s, snap),
+        lambda x, s: (sph.density(x, snap), sph.density_gradient(x, snap)), lambda x, s: (sph.blur(x, rho, s, snap),),
+        lambda x, s: (sph.gradient_hybrid(x, rho, s, snap),), lambda x, s: (sph.moment_matrix(x, rho, snap),),
+        lambda x, s: (sph.perceive_features(x, s, snap, 0.2),), lambda x, s: sph.step_update(y, x, s, snap, 1.0)]
+    if dim == 2:
+        calls.append(lambda x, s: (splatting.splat_particles_batch(x, s[..., :3], img_size=32),))
+    for call in calls:
+        g = torch.Generator(device="cuda").manual_seed(2)
+        grads = []
+        ups = None
+        for offset in (0, 1):
+            x, s = xb.detach().requires_grad_(True), sb.detach().requires_grad_(True)
+            out = call(x, s)
+            ups = ups or [torch.randn(o.shape, generator=g, device="cuda") for o in out]
+            grads.append(torch.autograd.grad(out, [x, s], [_at(u, offset) for u in ups], allow_unused=True))
+        for a, b in zip(*grads):
+            assert a is b is None or torch.equal(a, b)
+
+
+def test_euler_step_with_gradients_at_any_address():
+    from test_gpu_autograd_edges import _steps
+    x, s, steps, _ = _steps()
+    grads = []
+    for offset in (0, 1):
+        a, b = x.clone().requires_grad_(True), s.clone().requires_grad_(True)
+        out = steps["step"](a, b)
+        grads.append(torch.autograd.grad(out, [a, b], [_at(torch.ones_like(o), offset) for o in out]))
+    assert all(torch.equal(p, q) for p, q in zip(*grads))
