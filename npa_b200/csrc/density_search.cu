@@ -93,8 +93,10 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     const int i = min(first + lane % PT, total_particles - 1);
     const bool ivalid = first + lane % PT < total_particles;
     const Pos<D> pi = load_pos<D>(a.x, i);
-    const int cx = axis_cell(pi.x, g, 0), cy = axis_cell(pi.y, g, 1), cz = D == 3 ? axis_cell(pi.z, g, 2) : 0;
-    const int sys = i / g.N, key = (sys * g.g[2] + cz) * g.g[1] + cy;
+    const int sys = i / g.N;
+    int cx, cy, cz;  // in cell order, so the particles of a row of cells stand together with cx ascending
+    snapshot_cell_of<D>(g, a.bin_offsets + (size_t)sys * g.cells, i, pi.x, pi.y, pi.z, cx, cy, cz);
+    const int key = (sys * g.g[2] + cz) * g.g[1] + cy;
     // the interval of each axis whose particles sit in the cells their coordinate names, a little narrower
     float box_lo[3], box_hi[3];
 #pragma unroll

@@ -71,8 +71,8 @@ __device__ inline void store_row4(float *__restrict__ row, int f0, int C, const 
     }
 }
 
-// Search of the cells around one particle by the LPP lanes of its sub-group: candidate ranges in the order of
-// the cell walk, LPP candidates per round.
+// Search of the cells around one particle (around the cell it was binned into) by the LPP lanes of its sub-group: candidate
+// ranges in the order of the cell walk, LPP candidates per round.
 template <int D, bool PER, int LPP>
 struct SubgroupSearch {
     int cx, cy, cz, piece, j, end;
@@ -80,10 +80,8 @@ struct SubgroupSearch {
     Origin<D, PER> org;
 
     __device__ inline void begin(const Geom &g, const int32_t *bin_offsets, long long i, const Pos<D> &pi) {
-        cx = axis_cell(pi.x, g, 0);
-        cy = axis_cell(pi.y, g, 1);
-        cz = D == 3 ? axis_cell(pi.z, g, 2) : 0;
         off = bin_offsets + (i / g.N) * (long long)g.cells;
+        snapshot_cell_of<D>(g, off, (int)i, pi.x, pi.y, pi.z, cx, cy, cz);
         piece = -1;
         j = end = 0;
     }

@@ -122,6 +122,33 @@ __device__ inline Origin<D, PER> make_origin(const Geom &g, float px, float py, 
     return o;
 }
 
+// Hash of the cell that particle i (global index) sits in, by the snapshot's cell order: the operators may be given other
+// positions than the ones that were binned, and then candidates are still those around the cell of the binning.
+// `guess`, the cell of the current position, is almost always right and takes two loads to confirm; `off`: bin_offsets of
+// the system.
+__device__ __noinline__ inline uint32_t find_cell(const int32_t *__restrict__ off, int cells, int i) {
+    int lo = 0, hi = cells;  // off[lo] <= i < off[hi]
+    while (hi - lo > 1) {
+        const int mid = (int)(((unsigned)lo + (unsigned)hi) / 2u);
+        if (__ldg(off + mid) <= i) lo = mid;
+        else hi = mid;
+    }
+    return (uint32_t)lo;
+}
+__device__ inline uint32_t snapshot_cell(const Geom &g, const int32_t *__restrict__ off, int i, uint32_t guess) {
+    return __ldg(off + guess) <= i && i < __ldg(off + guess + 1) ? guess : find_cell(off, g.cells, i);
+}
+// The same as cell coordinates, from the particle's position.
+template <int D>
+__device__ inline void snapshot_cell_of(const Geom &g, const int32_t *__restrict__ off, int i, float px, float py, float pz, int &cx,
+                                        int &cy, int &cz) {
+    cx = axis_cell(px, g, 0);
+    cy = axis_cell(py, g, 1);
+    cz = D == 3 ? axis_cell(pz, g, 2) : 0;
+    const uint32_t guess = cell_hash<D>(g, cx, cy, cz), cell = snapshot_cell(g, off, i, guess);
+    if (cell != guess) hash_to_cell<D>(g, cell, cx, cy, cz);
+}
+
 // Number of candidate ranges of a cell: two per neighbour row with the linear hash (the second is the
 // wrapped cell of a periodic row), one per neighbour cell with the Morton hash.
 template <int D>

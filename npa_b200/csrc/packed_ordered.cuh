@@ -238,7 +238,8 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
     const int lane = threadIdx.x & 31, sl = lane & 15, f = sl % LPR * VW, at = sl / LPR * CPL, C = a.C, sys = i / g.N;
     const Pos<D> pi = load_pos<D>(a.x, i);
     WorkItem it = {i, 1, 0, sys};
-    it.cell = sys * g.cells + (int)cell_hash<D>(g, axis_cell(pi.x, g, 0), axis_cell(pi.y, g, 1), D == 3 ? axis_cell(pi.z, g, 2) : 0);
+    it.cell = sys * g.cells + (int)snapshot_cell(g, a.bin_offsets + (size_t)sys * g.cells, i,
+                                                 cell_hash<D>(g, axis_cell(pi.x, g, 0), axis_cell(pi.y, g, 1), D == 3 ? axis_cell(pi.z, g, 2) : 0));
     __syncwarp();
     const int nr = build_ranges<D>(g, a.bin_offsets, it, mem.rng);
     O o;
