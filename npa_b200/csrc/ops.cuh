@@ -74,7 +74,7 @@ struct FeatureFwdArgs {
     int pair_cache_valid;    // 0: this sweep writes the lists; 1: they are valid, read them instead of searching
     unsigned int *tickets;  // row tickets of this launch (set by the launcher)
     const float4 *pv;        // [B*N] (x, y, z, m / rho) written by the density sweep, or NULL (lists only)
-    int row_vec, out_vec;    // the packed sweeps: rows of s can be loaded, and z and vgrad stored, as vectors (set by the launcher)
+    int out_vec;             // packed rows over lists: z can be stored as vectors (set by the launcher)
 };
 
 struct FeatureBwdArgs {

@@ -47,7 +47,7 @@ __device__ inline float spiky_phi_rounded(float q, float h) {
     return quotient_rounded(3.0f * t * t, r);
 }
 
-template <int D, bool PER, int VW, int LPR, int CPL>
+template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
 struct Ordered {
     static constexpr int NM = D * (D + 1) / 2, H = VW / 2;
     static constexpr int G = 16 / LPR, CLS = G * CPL;  // groups of a particle, classes
@@ -57,8 +57,8 @@ struct Ordered {
     unsigned long long nsi[H], acc[CPL][1 + D][H];
     float mom[2][NM], dgs[2][3];
 
-    __device__ inline void begin(const float *__restrict__ row, int f, int C, int vec) {
-        load(row, f, C, vec, si);
+    __device__ inline void begin(const float *__restrict__ row, int f, int C) {
+        load(row, f, C, si);
 #pragma unroll
         for (int h = 0; h < H; ++h) nsi[h] = pack2(-si[2 * h], -si[2 * h + 1]);
 #pragma unroll
@@ -74,9 +74,9 @@ struct Ordered {
             dgs[k][0] = dgs[k][1] = dgs[k][2] = 0.f;
         }
     }
-    // Lanes beyond the last feature read valid neighbours of it (unused).  vec: rows are whole vectors at aligned addresses.
-    static __device__ inline void load(const float *__restrict__ row, int f, int C, int vec, float (&v)[VW]) {
-        if (vec) {
+    // Lanes beyond the last feature read valid neighbours of it (unused).
+    static __device__ inline void load(const float *__restrict__ row, int f, int C, float (&v)[VW]) {
+        if (ALIGNED && C % VW == 0) {
             if constexpr (VW == 4) {
                 const float4 t = __ldg(reinterpret_cast<const float4 *>(row + min(f, C - 4)));
                 v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
@@ -116,11 +116,11 @@ struct Ordered {
         return make_float4(kv * rx, kv * ry, kv * rz, w);
     }
     // STEP entries from a position that is a multiple of CLS; this group's are CPL in a row of each block of CLS.
-    __device__ inline void add(const float4 *__restrict__ ent, const int (&js)[U], const float *__restrict__ s, int f, int C, int vec) {
+    __device__ inline void add(const float4 *__restrict__ ent, const int (&js)[U], const float *__restrict__ s, int f, int C) {
         float r[U][VW];
 #pragma unroll
         for (int u = 0; u < U; ++u)
-            load(reinterpret_cast<const float *>(reinterpret_cast<const char *>(s) + (unsigned long long)(unsigned)js[u] * ((unsigned)C * 4u)), f, C, vec, r[u]);
+            load(reinterpret_cast<const float *>(reinterpret_cast<const char *>(s) + (unsigned long long)(unsigned)js[u] * ((unsigned)C * 4u)), f, C, r[u]);
 #pragma unroll
         for (int u = 0; u < U; ++u) {
             const float4 e = ent[u / CPL * CLS + u % CPL];
@@ -201,7 +201,7 @@ struct Ordered {
         }
         if (a.vgrad && valid) {
             float *o = a.vgrad + (i * C + f) * D;
-            if (OWN == 2 && C % 2 == 0 && a.out_vec) {
+            if (ALIGNED && OWN == 2 && C % 2 == 0) {
                 if (f < C) {
                     auto at = [&](int e) { return val[e / D][1 + e % D]; };
 #pragma unroll
@@ -232,9 +232,9 @@ struct Ordered {
 
 // One particle by the whole warp, through the candidates of its cells (the two halves of the warp sum the features
 // alike).  Out of line, so that it costs the walk over lists no registers.
-template <int D, bool PER, int VW, int LPR, int CPL>
+template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
 __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom &g, OrderedMem &mem, int i) {
-    using O = Ordered<D, PER, VW, LPR, CPL>;
+    using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
     const int lane = threadIdx.x & 31, sl = lane & 15, f = sl % LPR * VW, at = sl / LPR * CPL, C = a.C, sys = i / g.N;
     const Pos<D> pi = load_pos<D>(a.x, i);
     WorkItem it = {i, 1, 0, sys};
@@ -243,7 +243,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
     __syncwarp();
     const int nr = build_ranges<D>(g, a.bin_offsets, it, mem.rng);
     O o;
-    o.begin(a.s + (long long)i * C, f, C, a.row_vec);
+    o.begin(a.s + (long long)i * C, f, C);
     collect_pairs<D, PER>(g, a.x, pi, mem.rng, nr, mem.geo, [&](int n) {
         __syncwarp();
         const int filled = (n + O::STEP - 1) / O::STEP * O::STEP;  // kListPerWarp is a multiple of STEP
@@ -264,7 +264,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
             int js[O::U];
 #pragma unroll
             for (int u = 0; u < O::U; ++u) js[u] = __float_as_int(mem.geo[e + u / CPL * O::CLS + u % CPL].w);
-            o.add(mem.ent + e, js, a.s, f, C, a.row_vec);
+            o.add(mem.ent + e, js, a.s, f, C);
         }
         __syncwarp();
     });
@@ -274,10 +274,10 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
     __syncwarp();
 }
 
-template <int D, bool PER, int VW, int LPR, int CPL>
+template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
 __global__ void __launch_bounds__(kOrderedWarps * 32, D == 2 ? 10 : 8)
 packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
-    using O = Ordered<D, PER, VW, LPR, CPL>;
+    using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
     __shared__ OrderedMem s_mem[kOrderedWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane >> 4, sl = lane & 15;
     const int total = g.B * g.N, first = (blockIdx.x * kOrderedWarps + warp) * 2;
@@ -296,7 +296,7 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
     indices(0);
     const Pos<D> pi = load_pos<D>(a.x, i);
     O o;
-    o.begin(a.s + (long long)i * C, f, C, a.row_vec);
+    o.begin(a.s + (long long)i * C, f, C);
     const bool search = count < 0 || count > room;
     const int n = search ? 0 : count, nmax = __reduce_max_sync(kFull, n);
     float4 *ent = mem.ent + sg * 33;
@@ -340,7 +340,7 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
                     js[u] = idx[e + u * O::CLS];
                 }
             }
-            o.add(ent + e, js, a.s, f, C, a.row_vec);
+            o.add(ent + e, js, a.s, f, C);
         }
         __syncwarp();
     }
@@ -349,22 +349,26 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
     __syncwarp();
     // the rows of both particles are one run (8-byte aligned when z is: first is even); the row of a particle that is
     // searched is written again below
-    const int floats = min(2, total - first) * Z, pairs = a.out_vec ? floats / 2 : 0;
+    const int floats = min(2, total - first) * Z;
     float *out = a.z + (long long)first * Z;
-    for (int q = lane; q < pairs; q += 32) reinterpret_cast<float2 *>(out)[q] = reinterpret_cast<const float2 *>(mem.rows)[q];
-    for (int q = 2 * pairs + lane; q < floats; q += 32) out[q] = mem.rows[q];
+    if (ALIGNED) {
+        for (int q = lane; q < floats / 2; q += 32) reinterpret_cast<float2 *>(out)[q] = reinterpret_cast<const float2 *>(mem.rows)[q];
+        if ((floats & 1) && lane == 0) out[floats - 1] = mem.rows[floats - 1];
+    } else {
+        for (int q = lane; q < floats; q += 32) out[q] = mem.rows[q];
+    }
     const unsigned again = __ballot_sync(kFull, search && valid);
-    if (again & 0x0000ffffu) ordered_search<D, PER, VW, LPR, CPL>(a, g, mem, first);
-    if (again & 0xffff0000u) ordered_search<D, PER, VW, LPR, CPL>(a, g, mem, first + 1);
+    if (again & 0x0000ffffu) ordered_search<D, PER, VW, LPR, CPL, ALIGNED>(a, g, mem, first);
+    if (again & 0xffff0000u) ordered_search<D, PER, VW, LPR, CPL, ALIGNED>(a, g, mem, first + 1);
 }
 
+// ALIGNED: the addresses of the feature rows, of z and of vgrad allow the vector accesses of the shape.
 template <int D, bool PER, int VW, int LPR, int CPL>
 int launch_packed_ordered_shape(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
+    const bool aligned = (a.C % VW != 0 || (uintptr_t)a.s % (VW * 4) == 0) && ((uintptr_t)a.z | (uintptr_t)a.vgrad) % 8 == 0;
+    const auto kernel = aligned ? packed_ordered_kernel<D, PER, VW, LPR, CPL, true> : packed_ordered_kernel<D, PER, VW, LPR, CPL, false>;
     const long long particles = (long long)g.B * g.N;
-    FeatureFwdArgs b = a;
-    b.row_vec = a.C % VW == 0 && (uintptr_t)a.s % (VW * 4) == 0;
-    b.out_vec = ((uintptr_t)a.z | (uintptr_t)a.vgrad) % 8 == 0;
-    packed_ordered_kernel<D, PER, VW, LPR, CPL><<<(unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st>>>(b, g);
+    kernel<<<(unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st>>>(a, g);
     return check_launch("packed_ordered_kernel");
 }
 
