@@ -198,6 +198,10 @@ constexpr int kItemWarps = 4;
 constexpr int kItemSlots = 320;  // candidates staged at a time per warp
 constexpr int kItemRun = 96;     // accepted neighbours of a particle between two flushes
 
+template <bool V> struct Flag {
+    static constexpr bool value = V;
+};
+
 struct ItemMem {
     float4 cand[kItemSlots];            // x, y, z, (index << 2) | class
     unsigned char code[kItemSlots];     // image shift
@@ -242,8 +246,12 @@ density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __gri
         if (len > 0) S.rng[__popc(some & below)] = make_int4(start, len, code, incl - len);
         __syncwarp();
         const bool wrapped = PER && __any_sync(kFull, len > 0 && code != shift_code(0, 0, 0));
-        // an axis too short to know the image of a cell, or a position outside the box: the half-box test decides pair by pair
+        // an axis too short to know the image of a cell, or a position outside its cell: the half-box test decides pair by pair
         bool check = PER && (g.g[0] <= 4 || g.g[1] <= 4 || (D == 3 && g.g[2] <= 4));
+
+        float centre[3];
+#pragma unroll
+        for (int d = 0; d < D; ++d) centre[d] = ((float)((d == 0 ? cx : d == 1 ? cy : cz) - g.half[d]) + 0.5f) * g.h;
 
         for (int kb = k0; kb < k1; kb += 8) {
             const int nb = min(8, k1 - kb);
@@ -291,19 +299,41 @@ density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __gri
                         }
                     }
                     __syncwarp();
-                    // the positions: the loads of five steps in flight together
+                    // the positions: the loads of five steps in flight together.  Periodic: seen from here a candidate's cell may lie
+                    // beyond an edge of the box; three cells around the centre hold it, or its position is not that of its cell
                     bool outside = false;
-#pragma unroll 5
-                    for (int c = lane; c < count; c += 32) {
-                        const Pos<D> p = load_pos<D>(a.x, __float_as_uint(S.cand[c].w) >> 2);
-                        S.cand[c].x = p.x; S.cand[c].y = p.y; S.cand[c].z = p.z;
-                        if (PER) {
-                            const float v[3] = {p.x, p.y, p.z};
+                    auto positions = [&](auto shifted_cells) {
+                        for (int c0 = lane; c0 < count; c0 += 5 * 32) {
+                            Pos<D> p[5];
+                            int code[5];
 #pragma unroll
-                            for (int d = 0; d < D; ++d)
-                                outside |= !(v[d] >= -(float)g.half[d] * g.h && v[d] <= (float)(g.g[d] - g.half[d]) * g.h);
+                            for (int u = 0; u < 5; ++u) {
+                                const int c = min(c0 + 32 * u, count - 1);
+                                p[u] = load_pos<D>(a.x, __float_as_uint(S.cand[c].w) >> 2);
+                                code[u] = PER && decltype(shifted_cells)::value ? S.code[c] : shift_code(0, 0, 0);
+                            }
+#pragma unroll
+                            for (int u = 0; u < 5; ++u) {
+                                const int c = c0 + 32 * u;
+                                if (c >= count) break;
+                                S.cand[c].x = p[u].x; S.cand[c].y = p[u].y; S.cand[c].z = p[u].z;
+                                if (PER) {
+                                    const float v[3] = {p[u].x, p[u].y, p[u].z};
+#pragma unroll
+                                    for (int d = 0; d < D; ++d) {
+                                        float t = v[d] - centre[d];
+                                        if (decltype(shifted_cells)::value) {
+                                            const int k = (code[u] >> (2 * d)) & 3;
+                                            t += k == 1 ? 0.f : (k ? g.L[d] : -g.L[d]);
+                                        }
+                                        outside |= !(fabsf(t) <= 1.5f * g.h + 1e-5f * g.L[d]);
+                                    }
+                                }
+                            }
                         }
-                    }
+                    };
+                    if (PER && wrapped) positions(Flag<true>());
+                    else positions(Flag<false>());
                     if (PER) check |= __any_sync(kFull, outside) != 0;
                     __syncwarp();
                 }
@@ -314,6 +344,10 @@ density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __gri
                     for (int u = 0; u < 4; ++u) {
                         pi[u] = load_pos<D>(a.x, it.first + kb + min(p0 + u, nb - 1));
                         n[u] = __shfl_sync(kFull, held, p0 + u);
+                    }
+                    if (PER && total > kItemSlots && c0 == 0) {  // (a single chunk holds, and tests, the particles themselves as well)
+                        const Pos<D> own = lane & 2 ? (lane & 1 ? pi[3] : pi[2]) : (lane & 1 ? pi[1] : pi[0]);
+                        check |= __any_sync(kFull, outside_cells<D>(g, own, cx, cx, cy, cy, cz, cz)) != 0;
                     }
                     for (int c = 0; c < count; c += 32) {
                         const bool real = c + lane < count;

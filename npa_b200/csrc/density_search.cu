@@ -97,14 +97,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     int cx, cy, cz;  // in cell order, so the particles of a row of cells stand together with cx ascending
     snapshot_cell_of<D>(g, a.bin_offsets + (size_t)sys * g.cells, i, pi.x, pi.y, pi.z, cx, cy, cz);
     const int key = (sys * g.g[2] + cz) * g.g[1] + cy;
-    // the interval of each axis whose particles sit in the cells their coordinate names, a little narrower
-    float box_lo[3], box_hi[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const float margin = 1e-5f * g.L[d];
-        box_lo[d] = margin - (float)g.half[d] * g.h;
-        box_hi[d] = (float)(g.g[d] - g.half[d]) * g.h - margin;
-    }
+    const bool stray = PER && outside_cells<D>(g, pi, cx, cx, cy, cy, cz, cz);
     unsigned left = __ballot_sync(kFull, ivalid) & (Q == 1 ? kFull : ((1u << (PT & 31)) - 1u));  // particles to do
     while (left) {
         // ---- the particles of one x-row of cells, and the candidates of the rows around the cells they span
@@ -115,9 +108,9 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
         left &= ~seg;
         const int last = 31 - __clz(seg);
         const int cx0 = __shfl_sync(kFull, cx, lead), cx1 = __shfl_sync(kFull, cx, last);
+        const int row_y = __shfl_sync(kFull, cy, lead), row_z = __shfl_sync(kFull, cz, lead);
         __syncwarp();
-        const int nr = build_ranges_span<D>(g, a.bin_offsets, __shfl_sync(kFull, sys, lead), cx0, cx1, __shfl_sync(kFull, cy, lead),
-                                            __shfl_sync(kFull, cz, lead), rng);
+        const int nr = build_ranges_span<D>(g, a.bin_offsets, __shfl_sync(kFull, sys, lead), cx0, cx1, row_y, row_z, rng);
         const int4 own = lane < nr ? rng[lane] : make_int4(0, 0, shift_code(0, 0, 0), 0);
         int incl = own.y - own.x;
 #pragma unroll
@@ -129,8 +122,9 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
         const int ordinal = incl - (own.y - own.x);
         if (lane < nr) rng[lane] = make_int4(own.x - ordinal, ordinal, own.z, own.y - own.x);
         const bool wrapped = PER && __any_sync(kFull, own.z != shift_code(0, 0, 0));
-        // an axis too short to know the image of a cell: the half-box test decides pair by pair
+        // an axis too short to know the image of a cell, or a position outside its cell: the half-box test decides pair by pair
         bool check = PER && (g.g[0] <= 3 || g.g[1] <= 2 || (D == 3 && g.g[2] <= 2) || cx1 - cx0 + 3 >= g.g[0]);
+        if (PER) check = check || __any_sync(kFull, mine && stray);
         const int cap = wrapped && !COUNT ? kTileSlots / 2 : kTileSlots;  // the low parts take the other half
         const bool lists = !COUNT && a.pair_cache != nullptr;
 
@@ -185,9 +179,6 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                         for (int k = max(0, c0 - R.y) + lane % group; k < e; k += group) {
                             const int j = R.x + R.y + k, slot = R.y + k - c0;
                             Pos<D> p = load_pos<D>(a.x, j);
-                            const float v[3] = {p.x, p.y, p.z};
-#pragma unroll
-                            for (int d = 0; d < D; ++d) outside |= !(v[d] > box_lo[d] && v[d] < box_hi[d]);
                             if (wrapped && !COUNT) {
                                 float lx, ly, lz = 0.f, hx, hy, hz = 0.f;
                                 shifted(g, 0, p.x, (R.z & 3) - 1, hx, lx);
@@ -197,6 +188,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                                 S.x[kTileSlots / 2 + slot] = lx; S.y[kTileSlots / 2 + slot] = ly;
                                 if (D == 3) S.z[kTileSlots / 2 + slot] = lz;
                             }
+                            if (!COUNT || !wrapped) outside |= outside_cells<D>(g, p, cx0 - 1, cx1 + 1, row_y - 1, row_y + 1, row_z - 1, row_z + 1);
                             S.x[slot] = p.x; S.y[slot] = p.y;
                             if (D == 3) S.z[slot] = p.z;
                             S.j[slot] = COUNT ? R.z : j;
@@ -385,14 +377,6 @@ density_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     float4 *cand = s_mem + warp * (masses ? kSearchSlots + kSearchSlots / 4 : kSearchSlots);
     float *cmass = reinterpret_cast<float *>(cand + kSearchSlots);
     int4 *rng = s_rng[warp];
-    // the interval of each axis whose particles sit in the cells their coordinate names, a little narrower
-    float box_lo[3], box_hi[3];
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const float margin = 1e-5f * g.L[d];
-        box_lo[d] = margin - (float)g.half[d] * g.h;
-        box_hi[d] = (float)(g.g[d] - g.half[d]) * g.h - margin;
-    }
     const unsigned below = (1u << lane) - 1u;
     const int K = a.pair_stride;
     const unsigned long long hh = pack2(g.h2, g.h2), minus = pack2(-1.f, -1.f);
@@ -424,12 +408,16 @@ density_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
         if (len > 0) rng[__popc(some & below)] = make_int4(start, len, code, incl - len);
         __syncwarp();
         const bool wrapped = PER && __any_sync(kFull, len > 0 && code != shift_code(0, 0, 0));
-        // an axis too short to know the image of a cell: the half-box test decides pair by pair
+        // an axis too short to know the image of a cell, or a position outside its cell: the half-box test decides pair by pair
         bool general = PER && (wrapped || g.g[0] <= 3 || g.g[1] <= 2 || (D == 3 && g.g[2] <= 2));
         const int cap = wrapped ? kSearchSlots / 2 : kSearchSlots;  // the low parts take the other half
 
         for (int kb = k0; kb < k1; kb += 32) {
             const int nb = min(32, k1 - kb);
+            // (a particle is one of its own candidates, and within their window on four cells an axis its images stay clear: a
+            // test of its own is needed where it may be staged in a later chunk, or an axis has three)
+            if (PER && !general && (total > cap || g.g[1] == 3 || (D == 3 && g.g[2] == 3)))
+                general = __any_sync(kFull, lane < nb && outside_cells<D>(g, load_pos<D>(a.x, it.first + kb + min(lane, nb - 1)), cx, cx, cy, cy, cz, cz));
             float rho = 0.f;  // of particle kb + lane
             int found = 0;
             for (int c0 = 0; c0 < total; c0 += cap) {
@@ -444,12 +432,8 @@ density_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                             for (int k = max(0, c0 - R.w) + lane % group; k < e; k += group) {
                                 const int j = R.x + k, slot = R.w + k - c0;
                                 Pos<D> p = load_pos<D>(a.x, j);
-                                if (PER) {
-                                    const float v[3] = {p.x, p.y, p.z};
-#pragma unroll
-                                    for (int d = 0; d < D; ++d) outside |= !(v[d] > box_lo[d] && v[d] < box_hi[d]);
-                                }
-                                if (PER && wrapped) {
+                                if (PER && !wrapped) outside |= outside_cells<D>(g, p, cx - 1, cx + 1, cy - 1, cy + 1, cz - 1, cz + 1);
+                                if (PER && wrapped) {  // (these are tested pair by pair in any case)
                                     float4 lo = make_float4(0.f, 0.f, 0.f, 0.f);
                                     float hx, hy, hz = 0.f;
                                     shifted(g, 0, p.x, (R.z & 3) - 1, hx, lo.x);

@@ -122,6 +122,11 @@ __device__ inline Origin<D, PER> make_origin(const Geom &g, float px, float py, 
     return o;
 }
 
+template <int D>
+struct Pos {
+    float x, y, z;
+};
+
 // Hash of the cell that particle i (global index) sits in, by the snapshot's cell order: the operators may be given other
 // positions than the ones that were binned, and then candidates are still those around the cell of the binning.
 // `guess`, the cell of the current position, is almost always right and takes two loads to confirm; `off`: bin_offsets of
@@ -147,6 +152,18 @@ __device__ inline void snapshot_cell_of(const Geom &g, const int32_t *__restrict
     cz = D == 3 ? axis_cell(pz, g, 2) : 0;
     const uint32_t guess = cell_hash<D>(g, cx, cy, cz), cell = snapshot_cell(g, off, i, guess);
     if (cell != guess) hash_to_cell<D>(g, cell, cx, cy, cz);
+}
+
+// Whether coordinate v lies outside the cells [c0, c1] of axis d of the unwrapped grid (with a margin for the rounding of the
+// cell computation).  On a periodic grid the known image shift of a range holds only for positions inside their cell: one
+// beyond the box, on its upper edge (binned into the first cell) or moved since the binning needs the general minimum image.
+__device__ inline bool outside_cells(const Geom &g, int d, float v, int c0, int c1) {
+    const float margin = 1e-5f * g.L[d];
+    return !(v >= (float)(c0 - g.half[d]) * g.h - margin && v <= (float)(c1 + 1 - g.half[d]) * g.h + margin);
+}
+template <int D>
+__device__ inline bool outside_cells(const Geom &g, const Pos<D> &p, int cx0, int cx1, int cy0, int cy1, int cz0, int cz1) {
+    return outside_cells(g, 0, p.x, cx0, cx1) || outside_cells(g, 1, p.y, cy0, cy1) || (D == 3 && outside_cells(g, 2, p.z, cz0, cz1));
 }
 
 // Number of candidate ranges of a cell: two per neighbour row with the linear hash (the second is the
@@ -257,11 +274,6 @@ __device__ inline int build_ranges_span(const Geom &g, const int32_t *__restrict
     __syncwarp();
     return __popc(m);
 }
-
-template <int D>
-struct Pos {
-    float x, y, z;
-};
 
 template <int D>
 __device__ inline Pos<D> load_pos(const float *__restrict__ x, long long idx) {

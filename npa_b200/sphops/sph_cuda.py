@@ -86,6 +86,7 @@ class _HashGridBase:
 
     def _bind(self):
         self.native = N.ops.Grid(ctypes.addressof(self._desc))  # what the autograd nodes take (csrc/torch_ops.cpp)
+        self.list_columns  # here rather than in the first step
 
     # copies and pickles carry the description; the native handle is made anew
     def __getstate__(self):

@@ -1,4 +1,5 @@
-"""Operators given other positions than the ones that were binned: a perturbed copy on the same snapshot."""
+"""Operators given other positions than the ones that were binned (a perturbed copy on the same snapshot), and positions where
+the cell's image is not what the coordinate says: on the edge of a periodic box, and outside it."""
 import numpy as np
 import pytest
 import torch
@@ -66,3 +67,32 @@ def test_candidates_are_those_around_the_binned_cell(dim, boundary, mode, B):
         low, high = _density(q, near, h, dim), _density(q, torch.ones_like(near), h, dim)
         for r in (rho[b], rho2[b], rho3[b].cpu().double()):
             assert (r >= low * (1 - 1e-4)).all() and (r <= high * (1 + 1e-4)).all()
+
+
+@pytest.mark.parametrize("dim,mode", [(2, "grid"), (3, "grid"), (2, "particle"), (3, "particle")])
+@pytest.mark.parametrize("B", [2, 20])
+@pytest.mark.parametrize("where", ["edge", "outside"])
+def test_periodic_images_of_positions_on_the_edge_and_outside(dim, mode, B, where):
+    """A coordinate of exactly half the box is binned into the first cell; one beyond it into the cell of its image."""
+    N, cells = 997, 8
+    sph, grid, h, x, g = _make(dim, "periodic", mode, B, N, cells, seed=4)
+    some = torch.rand(B, N, dim, generator=g)
+    if where == "edge":
+        x = torch.where(some < 0.1, torch.full_like(x, 0.5), torch.where(some > 0.9, torch.full_like(x, -0.5), x))
+    else:
+        x = torch.where(some < 0.1, x + 1.0, torch.where(some > 0.9, x - 2.0, x))
+    snap = grid.instantiate(_padded(x))
+    xb, sb = sph.bin_particles(_padded(x), torch.randn(B, N, 4, generator=g).cuda(), snap)
+    count, rho = sph.count(xb, snap).cpu().double(), sph.density(xb, snap).cpu().double()
+    out = sph.perceive(xb, sb, snap)
+    hat = sph.gradient_hybrid(xb, out[0], sb, snap)
+    z = sph.perceive_features(xb, sb, snap, h, log_norm_grad=False)
+    C = 4
+    assert torch.allclose(z[..., C: 2 * C], out[1], rtol=1e-4, atol=1e-4 * float(out[1].abs().max()))
+    assert torch.allclose(z[..., 2 * C: 2 * C + C * dim].reshape(hat.shape), hat, rtol=1e-3, atol=1e-4 * float(hat.abs().max()))
+    for b in range(B):
+        q, less, more = _pairs(xb[b, :, :dim].cpu().double(), h, True)
+        assert (count[b] >= less.sum(1)).all() and (count[b] <= more.sum(1)).all()
+        want = _density(q, torch.ones_like(less), h, dim)
+        for r in (rho[b], out[0][b].cpu().double()):
+            assert ((r - want).abs() <= 1e-4 * want).all()
