@@ -246,6 +246,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                 const unsigned long long nh = pack2(-g.h2, -g.h2);
                 unsigned m = 0u;
                 if (kMode == 2) {
+#pragma unroll 4
                     for (int k = 0; k < 32; ++k) {
                         const int c = s0 + k;
                         float rx, ry, rz;

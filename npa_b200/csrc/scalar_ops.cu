@@ -308,10 +308,19 @@ static bool g_shared_search = true;  // count / density by density_search.cu
 void set_scalar_shared_search(bool on) { g_shared_search = on; }
 bool scalar_shared_search() { return g_shared_search; }
 
+// The count by the search that shares its candidates: not on Morton grids (its tiles are x-rows of cells), and not for few
+// particles on a 3D periodic grid, where most tiles meet an edge of the box and test every pair with its own shifted origin
+// (walk / search, ~40 neighbours: 4,096 particles 36 / 48 us, 16,384 48 / 57, 65,536 99 / 108, 131,072 139 / 142, 262,144
+// 251 / 217; ~130: 65,536 231 / 201).
+static bool count_by_search(const Geom &g) {
+    return !g.morton && !(g.periodic && g.dim == 3 && (long long)g.B * g.N < 65536);
+}
+
 template <int MASK>
 static int launch_scalar_fwd_mask(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     // the count or the density alone: the search that shares its candidates between particles
-    if ((MASK == S_DENSITY || (MASK == S_COUNT && !g.morton)) && g_shared_search) return launch_density_search(g, MASK == S_COUNT, a, st);
+    if ((MASK == S_DENSITY || (MASK == S_COUNT && count_by_search(g))) && g_shared_search)
+        return launch_density_search(g, MASK == S_COUNT, a, st);
     const char *what = "scalar_forward_kernel";
     if (g.dim == 2) {
         if (g.periodic) return launch_persistent(g, scalar_forward_kernel<2, true, MASK>, a, st, what);

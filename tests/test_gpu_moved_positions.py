@@ -96,3 +96,18 @@ def test_periodic_images_of_positions_on_the_edge_and_outside(dim, mode, B, wher
         want = _density(q, torch.ones_like(less), h, dim)
         for r in (rho[b], out[0][b].cpu().double()):
             assert ((r - want).abs() <= 1e-4 * want).all()
+
+
+@pytest.mark.parametrize("dim,B,N", [(3, 1, 65535), (3, 4, 16384), (2, 1, 3001)])   # either side of the count's dispatch
+def test_counts_on_periodic_grids_against_brute_force(dim, B, N):
+    cells = 16
+    sph, grid, h, x, g = _make(dim, "periodic", "grid", B, N, cells, seed=9)
+    snap = grid.instantiate(_padded(x))
+    xb, _ = sph.bin_particles(_padded(x), torch.zeros(B, N, 1, device="cuda"), snap)
+    count = sph.count(xb, snap)
+    for b in range(B):
+        p = xb[b, :, :dim].double()
+        rows = torch.randint(0, N, (500,), generator=g).cuda()
+        d = p[rows][:, None, :] - p[None, :, :]
+        q = ((d - torch.round(d)) ** 2).sum(-1)
+        assert (count[b][rows] >= (q < h * h * (1 - 1e-5)).sum(1)).all() and (count[b][rows] <= (q < h * h * (1 + 1e-5)).sum(1)).all()
