@@ -430,6 +430,7 @@ static int launch_item(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
 }
 
 int launch_density_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
+    if ((long long)g.B * g.N >= (1ll << 30)) return launch_density_search(g, false, a, st);  // a staged index has 30 bits here
     if (g.morton || (g.periodic && g.dim == 3)) {
         if (g.dim == 2) return g.periodic ? launch_item<2, true, 4>(g, a, st) : launch_item<2, false, 4>(g, a, st);
         return g.periodic ? launch_item<3, true, 4>(g, a, st) : launch_item<3, false, 4>(g, a, st);

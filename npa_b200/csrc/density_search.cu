@@ -88,10 +88,10 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     TileStage<MASS> &S = reinterpret_cast<TileStage<MASS> *>(s_tile)[warp];
     int4 *rng = s_rng[warp];
     const int total_particles = g.B * g.N, K = a.pair_stride;
-    const int first = (blockIdx.x * kTileWarps + warp) * PT;
-    if (first >= total_particles) return;
-    const int i = min(first + lane % PT, total_particles - 1);
-    const bool ivalid = first + lane % PT < total_particles;
+    const unsigned first = (blockIdx.x * kTileWarps + warp) * PT;
+    if (first >= (unsigned)total_particles) return;
+    const int i = (int)min(first + lane % PT, (unsigned)total_particles - 1u);
+    const bool ivalid = first + lane % PT < (unsigned)total_particles;
     const Pos<D> pi = load_pos<D>(a.x, i);
     const int sys = i / g.N;
     int cx, cy, cz;  // in cell order, so the particles of a row of cells stand together with cx ascending

@@ -132,8 +132,8 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
     constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
-    const int first = (blockIdx.x * kListWarps + warp) * PP;
-    bool ivalid = first + sg < total;
+    const int first = (blockIdx.x * kListWarps + warp) * PP;  // (less than total: the kernel has checked)
+    bool ivalid = sg < total - first;
     const int i = ivalid ? first + sg : total - 1;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
@@ -441,12 +441,13 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
     __shared__ float4 s_k[kListWarps][2][S::kSlots];  // v_j (K.x, K.y, K.z, W)
     __shared__ int4 s_j[kListWarps][2][S::kIndexQuads];
     extern __shared__ float4 s_rows[];                 // F_PACK: the rows of z of a warp's particles
-    const int warp = threadIdx.x >> 5, total = g.B * g.N, first = (blockIdx.x * kListWarps + warp) * S::PP;
-    if (first >= total) return;
+    const int warp = threadIdx.x >> 5, total = g.B * g.N;
+    const unsigned first = (blockIdx.x * kListWarps + warp) * S::PP;
+    if (first >= (unsigned)total) return;
     float *stage = reinterpret_cast<float *>(s_rows) + ((MASK & F_PACK) ? (size_t)warp * ((S::PP * a.zstride + 3) & ~3) : 0);
     list_forward<D, PER, LPP, VEC, MASK, false>(a, g, s_k[warp], s_j[warp], stage);
     __syncwarp();
-    const int i = min(first + (int)(threadIdx.x & 31) / LPP, total - 1);
+    const int i = (int)min(first + (threadIdx.x & 31u) / LPP, (unsigned)total - 1u);
     if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
         list_forward_search<D, PER, LPP, VEC, MASK>(a, g, s_k[warp], s_j[warp], stage);
 }
@@ -470,7 +471,7 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
     const int first = (blockIdx.x * WARPS + warp) * PP;
-    bool ivalid = first + sg < total;
+    bool ivalid = sg < total - first;
     const int i = ivalid ? first + sg : total - 1;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
@@ -786,11 +787,12 @@ feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const
     __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z W
     __shared__ float4 s_e[FULL ? WARPS : 1][2][S::kSlots];  // FULL: phi psi v_j E
     __shared__ int4 s_j[WARPS][2][S::kIndexQuads];
-    const int warp = threadIdx.x >> 5, total = g.B * g.N, first = (blockIdx.x * WARPS + warp) * S::PP;
-    if (first >= total) return;
+    const int warp = threadIdx.x >> 5, total = g.B * g.N;
+    const unsigned first = (blockIdx.x * WARPS + warp) * S::PP;
+    if (first >= (unsigned)total) return;
     list_backward<D, PER, LPP, VEC, MASK, FULL, false>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
     __syncwarp();
-    const int i = min(first + (int)(threadIdx.x & 31) / LPP, total - 1);
+    const int i = (int)min(first + (threadIdx.x & 31u) / LPP, (unsigned)total - 1u);
     if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
         list_backward_search<D, PER, LPP, VEC, MASK, FULL>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
 }

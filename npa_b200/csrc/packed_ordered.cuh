@@ -280,11 +280,11 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
     using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
     __shared__ OrderedMem s_mem[kOrderedWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane >> 4, sl = lane & 15;
-    const int total = g.B * g.N, first = (blockIdx.x * kOrderedWarps + warp) * 2;
-    if (first >= total) return;
+    const int total = g.B * g.N, first = (int)((blockIdx.x * kOrderedWarps + warp) * 2u);
+    if ((unsigned)first >= (unsigned)total) return;
     OrderedMem &mem = s_mem[warp];
-    const bool valid = first + sg < total;
-    const int i = min(first + sg, total - 1), C = a.C, f = sl % LPR * VW, at = sl / LPR * CPL;
+    const bool valid = sg < total - first;
+    const int i = valid ? first + sg : total - 1, C = a.C, f = sl % LPR * VW, at = sl / LPR * CPL;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int room = a.vgrad ? min(a.pair_stride - 1, kOrderedPairs) : a.pair_stride - 1;
     const int count = __ldg(list++);

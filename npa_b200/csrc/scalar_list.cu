@@ -15,10 +15,10 @@ scalar_list_backward_kernel(ScalarListArgs a, Geom g) {
     constexpr int LPP = 4;
     const int lane = threadIdx.x & 31, sl = lane % LPP;
     const int total = g.B * g.N;
-    const int at = (blockIdx.x * 256 + threadIdx.x) / LPP;
-    if (at - lane / LPP >= total) return;
-    const bool ivalid = at < total;
-    const int i = ivalid ? at : total - 1;
+    const unsigned at = blockIdx.x * (256u / LPP) + threadIdx.x / LPP;  // below 2^31 + 256 / LPP
+    if (at - lane / LPP >= (unsigned)total) return;
+    const bool ivalid = at < (unsigned)total;
+    const int i = ivalid ? (int)at : total - 1;
     const Pos<D> pi = load_pos<D>(a.x, i);
     const float mi = a.mass ? __ldg(a.mass + i) : 1.0f;
     auto upstream = [&](int j) {
@@ -152,10 +152,10 @@ density_gradient_list_kernel(ScalarListArgs a, Geom g) {
     constexpr int LPP = 8;
     const int lane = threadIdx.x & 31, sl = lane % LPP;
     const int total = g.B * g.N;
-    const int at = (blockIdx.x * 256 + threadIdx.x) / LPP;
-    if (at - lane / LPP >= total) return;
-    const bool ivalid = at < total;
-    const int i = ivalid ? at : total - 1;
+    const unsigned at = blockIdx.x * (256u / LPP) + threadIdx.x / LPP;  // below 2^31 + 256 / LPP
+    if (at - lane / LPP >= (unsigned)total) return;
+    const bool ivalid = at < (unsigned)total;
+    const int i = ivalid ? (int)at : total - 1;
     const Pos<D> pi = load_pos<D>(a.x, i);
     float dg[3] = {0.f, 0.f, 0.f};
     auto visit = [&](int j, float rx, float ry, float rz) {
