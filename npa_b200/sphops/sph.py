@@ -444,6 +444,8 @@ def step_update(y, x_bin, s_bin, snapshot, alpha, dt=1.0, update_mask=None, wrap
 
 def step_update_where(y, x_bin, s_bin, snapshot, alpha, dt, uniforms, update_prob, wrap=False):
     """``step_update`` with ``update_mask = (uniforms < update_prob).float()``, the comparison made in the kernel."""
+    if uniforms.dtype != torch.float32 or not update_prob >= 0.0:  # (the kernel's threshold; negative: the mask itself)
+        return step_update(y, x_bin, s_bin, snapshot, alpha, dt, (uniforms < update_prob).float(), wrap)
     return _ops.step_update(snapshot.grid.native, y.contiguous(), x_bin.contiguous(), s_bin.contiguous(),
                             uniforms.reshape(y.shape[0], y.shape[1]), float(alpha), float(dt), bool(wrap), float(update_prob))
 

@@ -80,10 +80,12 @@ def perceive(model, x, s, grid):
 
 def _one_node(model, x, s, grid) -> bool:
     """Whether a step of this model is covered by the single autograd node: the adaptation MLP on the default
-    engine, gradient features on, rows one warp pass covers, neighbour lists on."""
+    engine, gradient features on, rows one warp pass covers, neighbour lists on, single precision by default."""
     C, module = s.shape[-1], model.model
     if not (getattr(model, "state_grad", True) and getattr(model, "density_grad", True) and sph_ops.packable(C)
             and sph_ops._columns(grid.hashgrid) > 0 and on_tensor_memory(module)):
+        return False
+    if torch.get_default_dtype() != torch.float32:  # the update mask is drawn in the default type
         return False
     first, _, last = module
     return (first.weight.device == x.device and first.in_features == 2 * C + C * grid.dim + grid.dim

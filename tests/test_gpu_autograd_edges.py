@@ -181,3 +181,30 @@ def test_a_mask_changed_in_place_is_noticed():
     mask.zero_()
     with pytest.raises(RuntimeError, match="modified by an inplace operation"):
         out[1].sum().backward()
+
+
+@pytest.mark.parametrize("prob", [-1.0, 0.0, 0.3, 1.0])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+def test_update_masks_below_any_threshold(prob, dtype):
+    """Nothing moves below a probability of zero, and the mask follows the default type."""
+    from npa_b200 import stepping
+    x, s, _, grid = _steps()
+    model = _Model(grid.eps)
+    before = torch.get_default_dtype()
+    torch.set_default_dtype(dtype)
+    try:
+        for intermediate in (False, True):          # one node, and the operators
+            torch.manual_seed(5)
+            x_new, s_new, _ = stepping.step_euler(model, x, s, grid, update_prob=prob, intermediate=intermediate)
+            xb, sb = sph_bin(grid, x, s)
+            moved = (s_new != sb).any(-1)
+            torch.manual_seed(5)
+            want = torch.rand(2, 601, 1, device="cuda").squeeze(-1) < prob if prob < 1.0 else torch.ones(2, 601, dtype=torch.bool, device="cuda")
+            assert torch.equal(moved, want)
+    finally:
+        torch.set_default_dtype(before)
+
+
+def sph_bin(grid, x, s):
+    from npa_b200 import sphops as sph
+    return sph.bin_particles(x, s, grid.instantiate(x))
