@@ -309,8 +309,9 @@ struct FeatureNode : SweepNode {
         const Tensor gb = has_blur ? solid(g[0]) : Tensor(), gg = has_grad ? solid(g[has_blur ? 1 : 0]) : Tensor();
         if ((!gb.defined() && !gg.defined()) || !(nx || ns || nr)) return variable_list(4);
         c10::cuda::CUDAGuard guard(x.device());
-        Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor(), gr = nr ? blank(rho) : Tensor();
         const int C = (int)s.size(2);
+        auto out = [&](const Tensor &t, bool need) { return !need ? Tensor() : C ? blank(t) : at::zeros_like(t); };  // no features: no gradient
+        Tensor gx = out(x, nx), gs = out(s, ns), gr = out(rho, nr);
         if (C > 0 && pairs.defined()) {
             Tensor work = list_scratch(*grid, s, C);
             check_status(npa_blur_gradient_backward_lists(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
@@ -481,6 +482,7 @@ py::tuple perception(const GridPtr &grid, const Tensor &offs, const Tensor &info
     g.positions(x, "binned_positions");
     g.features(s, "state_in");
     const int64_t C = s.size(2);
+    if (C == 0) columns = 0;  // without features the density is all there is
     c10::cuda::CUDAGuard guard(x.device());
     const bool record = recording(x, s, sn.mass);
     Tensor rho = floats(x, {g.B, g.N}), blur = blank(s), grad = floats(s, {g.B, g.N, C, g.D});

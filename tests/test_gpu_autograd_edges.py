@@ -208,3 +208,23 @@ def test_update_masks_below_any_threshold(prob, dtype):
 def sph_bin(grid, x, s):
     from npa_b200 import sphops as sph
     return sph.bin_particles(x, s, grid.instantiate(x))
+
+
+def test_operators_without_features():
+    sph, grid, x, s = _inputs()
+    snap = grid.instantiate(x)
+    empty = torch.empty(2, 601, 0, device="cuda")
+    xb, sb = sph.bin_particles(x, empty, snap)
+    xr, sr = xb.clone().requires_grad_(True), sb.clone().requires_grad_(True)
+    rho, blur, grad, dg = sph.perceive(xr, sr, snap)
+    assert blur.shape == (2, 601, 0) and grad.shape == (2, 601, 0, 2)
+    want = sph.density(xb, snap)
+    assert torch.allclose(rho, want, rtol=1e-6)
+    up = torch.randn_like(rho)
+    got, = torch.autograd.grad(rho, xr, up, retain_graph=True)
+    ref = xb.clone().requires_grad_(True)
+    want, = torch.autograd.grad(sph.density(ref, snap), ref, up)
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-5 * float(want.abs().max()))
+    out = sph.blur(xr, rho.detach(), sr, snap)
+    gx, = torch.autograd.grad(out, xr, torch.empty_like(out))
+    assert not gx.any()
