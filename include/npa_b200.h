@@ -574,6 +574,11 @@ int npa_linear_tcgen05_wait_selftest(int32_t limit_us, int32_t *device_result, v
  * to that many x-adjacent cells share one staged neighbourhood) size the plan, 0 = chosen
  * automatically.  A plan that does not fit in shared memory falls back to the gather kernels.
  *
+ * npa_tile_enabled: 1 when the direction is switched on.  The engine searches for its pairs itself: the forward sweep of
+ * npa_perception_forward_lists takes it when it is on, but the _lists backward entry points are list sweeps by name
+ * and stay so; a caller that wants the engine there asks, and calls the backward without the suffix (the autograd
+ * operators and the grid classes of the Python package do).
+ *
  * npa_tile_status: every wait inside the engine is bounded; a wait that runs out stores a code in a
  * device word (1: a consumer gave up waiting for copies, 2: the producer gave up waiting for a free
  * stage) and the launch drains without finishing its work.  This call copies the word to
@@ -583,6 +588,7 @@ int npa_linear_tcgen05_wait_selftest(int32_t limit_us, int32_t *device_result, v
 int npa_tile_tuning(int32_t backward, int32_t enabled, int32_t rows_per_stage,
                     int32_t particles_per_tile, int32_t stages, int32_t consumer_warps,
                     int32_t cells_per_tile);
+int npa_tile_enabled(int32_t backward);
 int npa_tile_status(int32_t *host_status, int32_t reset);
 /* Health check of the row-ticket words the sweep kernels draw work from (no counterpart in the
  * reference).  Every sweep leaves its two words zero; with no sweep in flight a non-zero word means a

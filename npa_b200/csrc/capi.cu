@@ -428,6 +428,11 @@ int npa_perception_forward_lists(const npa_grid *gd, int32_t channels, const flo
     fa.pair_cache = pair_cache;
     fa.pair_stride = pair_stride;
     fa.pair_cache_valid = 1;
+    if (tile_forward_enabled()) {  // the engine has no density gradient of its own
+        if (rho_grad && (rc = npa_density_gradient_forward_lists(gd, x_bin, mass, rho_grad, bin_offsets, pair_cache, pair_stride, stream)) != NPA_OK)
+            return rc;
+        return launch_feature_forward(g, F_BLUR | F_GRAD, fa, st);
+    }
     return launch_feature_list_forward(g, F_BLUR | F_GRAD | (rho_grad ? F_DGRAD : 0), fa, st);
 }
 

@@ -137,7 +137,7 @@ int npa_perceive_features_forward_lists(const npa_grid *gd, int32_t channels, co
     const bool ordered = pair_cache && in_sweep && channels <= 32;
     ScalarFwdArgs sa = {x_bin, mass, nullptr, nullptr, rho, in_sweep ? nullptr : rho_grad, nullptr, bin_offsets, block_info, pair_cache, pair_stride};
     sa.pv = reinterpret_cast<float4 *>(packed);
-    rc = ordered ? launch_density_ordered(g, sa, st) : launch_scalar_forward(g, in_sweep ? S_DENSITY : (S_DENSITY | S_DGRAD), sa, st);
+    rc = ordered && scalar_shared_search() ? launch_density_ordered(g, sa, st) : launch_scalar_forward(g, in_sweep ? S_DENSITY : (S_DENSITY | S_DGRAD), sa, st);
     if (rc != NPA_OK) return rc;
     FeatureFwdArgs fa = {x_bin, mass, rho, s_bin, nullptr, nullptr, channels, bin_offsets, block_info, nullptr};
     fa.z = z;

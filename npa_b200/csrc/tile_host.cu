@@ -126,6 +126,8 @@ int npa_tile_tuning(int32_t backward, int32_t enabled, int32_t rows_per_stage, i
     return NPA_OK;
 }
 
+int npa_tile_enabled(int32_t backward) { return tile_tuning(backward != 0).enabled; }
+
 int npa_scalar_sweep_tuning(int32_t cells_per_tile) {
     if (cells_per_tile < 0 || (cells_per_tile > 8 && (cells_per_tile < 101 || cells_per_tile > 108)))
         return fail(NPA_ERR_INVALID_ARGUMENT, "scalar_sweep_tuning: cells_per_tile must be in [0, 8] or [101, 108]");

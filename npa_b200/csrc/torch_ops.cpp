@@ -168,6 +168,9 @@ Tensor new_lists(const Grid &g, const Tensor &like, int64_t columns) {
     return columns ? at::empty({g.B, g.N, columns}, like.options().dtype(at::kInt).requires_grad(false)) : Tensor();
 }
 
+// The cell-tile engine, when it is switched on for backward sweeps, searches for its pairs itself.
+bool by_lists(const Tensor &pairs) { return pairs.defined() && !npa_tile_enabled(1); }
+
 // Work memory of a backward over lists.
 Tensor list_scratch(const Grid &g, const Tensor &like, int64_t channels) {
     const int64_t bytes = npa_lists_backward_scratch_bytes(&g.g, (int)channels);
@@ -312,14 +315,14 @@ struct FeatureNode : SweepNode {
         const int C = (int)s.size(2);
         auto out = [&](const Tensor &t, bool need) { return !need ? Tensor() : C ? blank(t) : at::zeros_like(t); };  // no features: no gradient
         Tensor gx = out(x, nx), gs = out(s, ns), gr = out(rho, nr);
-        if (C > 0 && pairs.defined()) {
+        if (C > 0 && by_lists(pairs)) {
             Tensor work = list_scratch(*grid, s, C);
             check_status(npa_blur_gradient_backward_lists(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
                                                           fmut(gr), work.mutable_data_ptr(), work.numel() * 4, iptr(offs), iptr(pairs), list_stride(pairs),
                                                           stream_of(x)));
         } else if (C > 0) {
             check_status(npa_blur_gradient_backward(&grid->g, C, fptr(x), fptr(rho), fptr(mass), fptr(s), fptr(gb), fptr(gg), fmut(gx), fmut(gs),
-                                                    fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
+                                                    fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(pairs), stream_of(x)));
         }
         return {gx, gs, gr, Tensor()};
     }
@@ -456,7 +459,7 @@ struct PerceptionNode : SweepNode {
         const Tensor g_rho = nx ? solid(g[0]) : Tensor(), gb = solid(g[1]), gg = solid(g[2]), g_dg = nx && has_dg ? solid(g[3]) : Tensor();
         c10::cuda::CUDAGuard guard(x.device());
         Tensor gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
-        if (pairs.defined()) {
+        if (by_lists(pairs)) {
             Tensor work = list_scratch(*grid, s, s.size(2));
             check_status(npa_perception_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(packed), fptr(g_rho),
                                                        fptr(gb), fptr(gg), fptr(g_dg), fmut(gx), fmut(gs), work.mutable_data_ptr(), work.numel() * 4,
@@ -465,7 +468,7 @@ struct PerceptionNode : SweepNode {
         }
         Tensor gr = nx ? blank(rho) : Tensor();
         check_status(npa_perception_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(g_rho), fptr(gb), fptr(gg),
-                                             fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), nullptr, 0, stream_of(x)));
+                                             fptr(g_dg), fmut(gx), fmut(gs), fmut(gr), iptr(offs), iptr(info), iptr(pairs), list_stride(pairs), stream_of(x)));
         return {gx, gs, Tensor()};
     }
     void release_variables() override {
@@ -522,7 +525,7 @@ struct PackedNode : SweepNode {
         if (!g[0].defined() || !(nx || ns)) return variable_list(3);
         c10::cuda::CUDAGuard guard(x.device());
         const Tensor gz = solid(g[0]);
-        if (pairs.defined()) {
+        if (by_lists(pairs)) {
             Tensor work = list_scratch(*grid, s, s.size(2)), gx = nx ? blank(x) : Tensor(), gs = ns ? blank(s) : Tensor();
             check_status(npa_perceive_features_backward_lists(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad),
                                                               fptr(vgrad), fptr(packed), fptr(gz), coef, dg_scale, ln_grad, ln_dg, nullptr, fmut(gx), fmut(gs),
@@ -537,7 +540,7 @@ struct PackedNode : SweepNode {
         Tensor gx = nx ? blank(x) : Tensor(), gs = blank(s);
         check_status(npa_perceive_features_backward(&grid->g, (int)s.size(2), fptr(x), fptr(mass), fptr(s), fptr(rho), fptr(rho_grad), fptr(vgrad),
                                                     fptr(gz), coef, dg_scale, ln_grad, ln_dg, gb, gg, g_dg, gr, fmut(gx), fmut(gs), iptr(offs),
-                                                    iptr(info), nullptr, 0, stream_of(x)));
+                                                    iptr(info), iptr(pairs), list_stride(pairs), stream_of(x)));
         return {gx, ns ? gs : Tensor(), Tensor()};
     }
     void release_variables() override {
@@ -714,7 +717,7 @@ Tensor mlp(const Tensor &z, const Tensor &w1, const Tensor &b1, const Tensor &w2
 struct EulerNode : Node {
     GridPtr grid;
     SavedVariable w1_, w2_, slab_, mask_;
-    Tensor offs, perm;
+    Tensor offs, perm, info;
     int64_t o_x, o_s, o_rho, o_dg, o_v, o_packed, o_z, o_h, o_y, o_dz, o_pairs;  // places in the slab, in floats
     int64_t C, columns, dz_bytes;
     float coef, dg_scale, alpha, dt, below;
@@ -751,20 +754,31 @@ struct EulerNode : Node {
         Tensor gw1, gb1, gw2;
         if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st);
         // perception, with the update's own gradient of the states added
-        Tensor gx_bin = gx_new;
+        Tensor gx_bin = gx_new, none;
         const float *gs_bin = fptr(gs_new);
         if (back) {
             check_status(npa_linear_tcgen05_prepared(dh, dz_image, dz_bytes, gz, m, kHidden, (int)k, st));
             Tensor gxp = back_x ? floats(w1, {gr.B, gr.N, gr.P}) : Tensor();
             float *gsp = back_s ? t + o_gs : nullptr;
-            check_status(npa_perceive_features_backward_lists(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, packed, gz, coef, dg_scale,
-                                                              ln_grad, ln_dg, fptr(gs_new), fmut(gxp), gsp, t + o_work, work_bytes, iptr(offs),
-                                                              pairs, (int)columns, st));
+            if (npa_tile_enabled(1)) {
+                Tensor gsf = floats(w1, {gr.B, gr.N, C}), work = floats(w1, {m * (C + 1) * (1 + gr.D)});
+                float *gb = fmut(work), *gg = gb + m * C, *g_dg = gg + m * C * gr.D, *g_rho = g_dg + m * gr.D;
+                check_status(npa_perceive_features_backward(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, gz, coef, dg_scale, ln_grad, ln_dg,
+                                                            gb, gg, back_x ? g_dg : nullptr, back_x ? g_rho : nullptr, fmut(gxp), fmut(gsf), iptr(offs),
+                                                            iptr(info), pairs, (int)columns, st));
+                if (gs_new.defined()) gsf.add_(gs_new.detach());
+                none = gsf;
+                gsp = back_s ? fmut(gsf) : nullptr;
+            } else {
+                check_status(npa_perceive_features_backward_lists(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, packed, gz, coef, dg_scale,
+                                                                  ln_grad, ln_dg, fptr(gs_new), fmut(gxp), gsp, t + o_work, work_bytes, iptr(offs),
+                                                                  pairs, (int)columns, st));
+            }
             if (back_s) gs_bin = gsp;
             if (back_x) gx_bin = gx_bin.defined() ? gxp.add_(gx_bin) : gxp;
         }
         // back into the order of the inputs
-        Tensor gx, gs, none;
+        Tensor gx, gs;
         if (nx && !gx_bin.defined()) gx_bin = at::zeros({gr.B, gr.N, gr.P}, w1.options().requires_grad(false));
         if (ns && !gs_bin) {
             none = at::zeros({gr.B, gr.N, C}, w1.options().requires_grad(false));
@@ -819,7 +833,7 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
                                 : npa_step_update_forward(&g.g, y, x_bin, s_bin, nullptr, (int)C, (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st));
     if (record) {
         auto n = node_for<EulerNode>(x, s, w1, b1, w2);
-        n->grid = grid; n->offs = offs; n->perm = perm; n->slab_ = saved(slab); n->mask_ = saved(mask);
+        n->grid = grid; n->offs = offs; n->perm = perm; n->info = info; n->slab_ = saved(slab); n->mask_ = saved(mask);
         n->o_x = o_x; n->o_s = o_s; n->o_rho = o_rho; n->o_dg = o_dg; n->o_v = o_v; n->o_packed = o_packed; n->o_z = o_z; n->o_h = o_h; n->o_y = o_y;
         n->o_dz = o_dz; n->o_pairs = o_pairs; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
         n->w1_ = saved(w1); n->w2_ = saved(w2);

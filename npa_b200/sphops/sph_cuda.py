@@ -143,6 +143,11 @@ class _HashGridBase:
             raise RuntimeError(f"pair_cache must have between 2 and 513 columns, got {K}")
         return N.ptr(pair_cache), K
 
+    @staticmethod
+    def _by_lists(pair_cache):
+        """Whether a backward with these lists takes the sweeps over lists (the cell-tile engine, when on, searches)."""
+        return pair_cache is not None and not _lib.npa_tile_enabled(1)
+
     def _list_scratch(self, channels, device):
         """Work memory of a backward over neighbour lists, private to the call."""
         n = _lib.npa_lists_backward_scratch_bytes(self._ref(), channels)
@@ -387,7 +392,7 @@ class _HashGridBase:
         self._snap(bin_offsets, block_info)
         if C == 0:
             return
-        if pair_cache is not None:
+        if self._by_lists(pair_cache):
             pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
             self._call(_lib.npa_blur_gradient_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
                        N.ptr(rho), N.ptr(mass), N.ptr(state_in), N.ptr(dL_blur_state_out), N.ptr(dL_grad_state_out),
@@ -462,7 +467,7 @@ class _HashGridBase:
         if grad_s is not None:
             self._bn(grad_s, "grad_s", C)
         self._snap(bin_offsets, block_info)
-        if pair_cache is not None:
+        if self._by_lists(pair_cache):
             pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
             self._call(_lib.npa_perceive_features_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
                        N.ptr(mass), N.ptr(state_in), N.ptr(rho), N.ptr(density_gradient), N.ptr(corrected_gradient), None,
@@ -557,7 +562,7 @@ class _HashGridBase:
             self._bn(grad_s, "grad_s", C)
         if grad_rho_scratch is not None:
             self._bn(grad_rho_scratch, "grad_rho_scratch")
-        if pair_cache is not None and C > 0:
+        if self._by_lists(pair_cache) and C > 0:
             pairs, scratch = self._pairs(pair_cache), self._list_scratch(C, binned_positions.device)
             self._call(_lib.npa_perception_backward_lists, binned_positions, self._ref(), C, N.ptr(binned_positions),
                        N.ptr(mass), N.ptr(state_in), N.ptr(rho), None, N.ptr(dL_rho_out), N.ptr(dL_blur_state_out),

@@ -155,3 +155,58 @@ def test_bounded_wait_gives_up_and_reports():
     torch.cuda.synchronize()
     assert int(res.item()) == 1
     assert float(torch.ones(4, device="cuda").sum().item()) == 4.0
+
+
+@pytest.mark.parametrize("backward", [False, True])
+def test_the_switch_reaches_the_operators(backward):
+    """Each direction of the engine is taken by the autograd operators and the grid classes, lists or not: other bits, equal
+    to rounding."""
+    from npa_b200 import _native as n
+    from npa_b200 import sphops as sph
+    from test_gpu_autograd_edges import _steps
+    w = Workload("t_ops", dim=3, B=2, N=4000, C=32, eps=0.12, grid_size=(10, 10, 10))
+    grid, snap, xb, sb, _, _, ups = _setup(w, with_mass=False, seed=8)
+    x0, s0, steps, _ = _steps()
+
+    def run():
+        out = {}
+        for name in ("perceive", "blur", "features", "grid", "step"):
+            x, s = (t.detach().clone().requires_grad_(True) for t in ((x0, s0) if name == "step" else (xb, sb)))
+            if name == "perceive":
+                res = sph.perceive(x, s, snap)
+            elif name == "blur":
+                rho = sph.density(x, snap)
+                res = (sph.blur(x, rho.detach(), s, snap),)
+            elif name == "features":
+                res = (sph.perceive_features(x, s, snap, 0.1),)
+            elif name == "step":
+                res = steps["step"](x, s)
+            else:
+                pairs = torch.empty(2, 4000, 128, dtype=torch.int32, device="cuda")
+                rho = torch.empty(2, 4000, device="cuda")
+                hg = grid.hashgrid
+                hg.perception_forward(xb, None, None, rho, None, None, None, None, None, snap.bin_offsets, snap.block_info, pair_cache=pairs)
+                gx, gs, gr = torch.empty_like(xb), torch.empty_like(sb), torch.empty_like(rho)
+                hg.blur_gradient_backward(xb, rho, None, sb, ups["g_blur"], ups["g_grad"], gx, gs, gr, snap.bin_offsets, snap.block_info,
+                                          pair_cache=pairs)
+                out[name] = [gx, gs, gr]
+                continue
+            g = torch.Generator(device="cuda").manual_seed(1)
+            u = [torch.randn(r.shape, generator=g, device="cuda") for r in res]
+            out[name] = list(torch.autograd.grad(res, [x, s], u, allow_unused=True)) if backward else [r.detach() for r in res]
+        return out
+
+    want = run()
+    n.tile_tuning(backward, True)
+    got = run()
+    assert n.tile_status() == 0
+    for name in want:
+        differs = False
+        for a, b in zip(got[name], want[name]):
+            if a is None:
+                continue
+            assert torch.allclose(a, b, rtol=1e-4, atol=2e-5 * float(b.abs().max())), name
+            differs = differs or not torch.equal(a, b)
+        # (a step of 601 particles is not a shape of the engine; its forward takes blur and gradient together only)
+        if name != "step" and (backward or name not in ("grid", "blur")):
+            assert differs, f"{name}: identical bits, the engine did not take the call"
