@@ -112,12 +112,14 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
         for (int x = 0; x < 8; ++x) acc[y][x][0] = acc[y][x][1] = 0ull;
 
     // particles off .. off + count - 1 of the list
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
     auto multiply = [&](int off, int count) {
+        bool odd = false;  // a colour that is not finite: zero times it is not zero outside the patch
         const int padded = (count + kSplatParts - 1) / kSplatParts * kSplatParts;
         const int p = tid >> 2, axis = (tid >> 1) & 1, o0 = (tid & 1) * 8;
         if (p < padded) {
             float w[8];
-            float4 c = make_float4(0.f, 0.f, 0.f, 0.f);
+            float4 c = zero;
             int at = 0, lo = 1, hi = 0;
             float frac = 0.f;
             if (p < count) {
@@ -130,6 +132,7 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
                     const float scale = a.normalize ? __ldg(a.wscale + n) : 1.0f;
                     const float *col = a.color + n * 3;
                     c = make_float4(scale * __ldg(col), scale * __ldg(col + 1), scale * __ldg(col + 2), scale);
+                    odd = !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < INFINITY);
                 }
             }
 #pragma unroll
@@ -147,7 +150,22 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
                 for (int k = 0; k < 8; ++k) sh.lists.wy[p][o0 + k] = make_float4(w[k] * c.x, w[k] * c.y, w[k] * c.z, w[k] * c.w);
             }
         }
-        __syncthreads();
+        if (__syncthreads_or(odd)) {
+            for (int q = part; q < padded; q += kSplatParts)
+#pragma unroll
+                for (int y = 0; y < 2; ++y) {
+                    const float4 w = sh.lists.wy[q][py + y];
+#pragma unroll
+                    for (int x = 0; x < 8; ++x) {
+                        const float xs = sh.lists.wx[q][px + x];
+                        if (xs == 0.f || w.w == 0.f) continue;
+                        acc[y][x][0] = fma2(pack2(xs, xs), pack2(w.x, w.y), acc[y][x][0]);
+                        acc[y][x][1] = fma2(pack2(xs, xs), pack2(w.z, w.w), acc[y][x][1]);
+                    }
+                }
+            __syncthreads();
+            return;
+        }
         for (int q = part; q < padded; q += kSplatParts) {
             const float4 x0 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px]), x1 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px + 4]);
             const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};

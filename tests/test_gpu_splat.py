@@ -107,3 +107,24 @@ def test_argument_errors():
         splatting.splat_particles_batch(x, c[:, :4])
     with pytest.raises(ValueError):          # patch radius beyond what the kernels support
         splatting.splat_particles_batch(x, c, img_size=64, sigma=20.0, normalize_color=False)
+
+
+@pytest.mark.parametrize("N", [7, 3000])
+@pytest.mark.parametrize("value", [float("inf"), float("nan")])
+def test_a_colour_that_is_not_finite_stays_in_its_patch(N, value):
+    from npa_b200 import splatting
+    g = torch.Generator().manual_seed(N)
+    x = (torch.rand(1, N, 2, generator=g) - 0.5).cuda()
+    x[0, 0] = 0.0
+    color = torch.rand(1, N, 3, generator=g).cuda()
+    want = splatting.splat_particles_batch(x, color, img_size=128, sigma=1.0)
+    color[0, 0, 1] = value
+    got = splatting.splat_particles_batch(x, color, img_size=128, sigma=1.0)
+    r = 5                                       # ceil(5 sigma) pixels around the pixel of (0, 0)
+    patch = torch.zeros(128, 128, dtype=torch.bool)
+    patch[63 - r: 63 + r + 1, 63 - r: 63 + r + 1] = True
+    bad = ~torch.isfinite(got[0].cpu())
+    assert bool(bad[..., 1][patch].all()) and not bool(bad[..., 1][~patch].any())
+    assert not bool(bad[..., [0, 2, 3]].any())
+    keep = ~bad
+    assert torch.allclose(got[0].cpu()[keep], want[0].cpu()[keep], rtol=1e-6, atol=1e-6)
