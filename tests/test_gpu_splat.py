@@ -128,3 +128,20 @@ def test_a_colour_that_is_not_finite_stays_in_its_patch(N, value):
     assert not bool(bad[..., [0, 2, 3]].any())
     keep = ~bad
     assert torch.allclose(got[0].cpu()[keep], want[0].cpu()[keep], rtol=1e-6, atol=1e-6)
+
+
+@pytest.mark.parametrize("img,sigma", [(128, 2.0), (70, 0.7)])
+def test_forward_on_either_side_of_the_kernel_choice(img, sigma):
+    """Few particles are added pixel by pixel, many multiplied out: the fp64 oracle's image on both sides of the line, and the same
+    bits alone and in a batch."""
+    from npa_b200 import splatting
+    from oracle import splat as splat_oracle
+    radius = splatting._derived(img, sigma, -1.0, 1.0, True, 2.0 / 128.0)[1]
+    reach = min(1.0, (2 * radius + 1 + 16) / img) ** 2
+    for h in (0.0, 26.0, 30.0, 80.0):
+        n = max(1, int(h / reach))
+        g = torch.Generator().manual_seed(n)
+        x, c = (torch.rand(5, n, 2, generator=g) - 0.5) * 2.2, torch.rand(5, n, 3, generator=g)
+        out = splatting.splat_particles_batch(x.cuda(), c.cuda(), img_size=img, sigma=sigma)
+        _close(out[2], splat_oracle.splat_forward(x[2].numpy(), c[2].numpy(), img_size=img, sigma=sigma), f"{n} particles")
+        assert torch.equal(splatting.splat_particles(x[2].cuda(), c[2].cuda(), img_size=img, sigma=sigma), out[2])
