@@ -133,7 +133,7 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
     const int first = (blockIdx.x * kListWarps + warp) * PP;  // (less than total: the kernel has checked)
-    bool ivalid = sg < total - first;
+    bool ivalid = (unsigned)(first + sg) < (unsigned)total;
     const int i = ivalid ? first + sg : total - 1;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
@@ -471,7 +471,7 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
     const int first = (blockIdx.x * WARPS + warp) * PP;
-    bool ivalid = sg < total - first;
+    bool ivalid = (unsigned)(first + sg) < (unsigned)total;
     const int i = ivalid ? first + sg : total - 1;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int count = list_count<LPP>(list, a.pair_stride, ivalid, sl);
