@@ -1,8 +1,8 @@
-// Density and neighbour lists of a recorded step: the order of the sums of the packed perception.
+// Density and neighbour lists of the packed perception, recorded for a backward or not: the order of its sums.
 //
 // A hidden unit of the MLP whose preactivation is within rounding of zero switches with the last bit of the
-// perception vector, and with it a row of the weight gradient.  The forward of a step that will be differentiated
-// therefore keeps one fixed association of its sums, whatever is done to make it faster: here the candidates in the
+// perception vector, and with it a row of the weight gradient.  The packed perception therefore keeps one fixed
+// association of its sums, whatever is done to make it faster: here the candidates in the
 // order of the cell walk, two partial sums (even and odd positions of a row of cells) on a clamped grid; in
 // packed_ordered.cuh the accepted pairs by their position in the list.  Everything else searches in density_search.cu.
 //
@@ -435,12 +435,18 @@ int launch_density_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t s
         if (g.dim == 2) return g.periodic ? launch_item<2, true, 4>(g, a, st) : launch_item<2, false, 4>(g, a, st);
         return g.periodic ? launch_item<3, true, 4>(g, a, st) : launch_item<3, false, 4>(g, a, st);
     }
-    // A tile takes as long as the candidates of a lane, whatever the number of particles (2D, 144 candidates: 10 us at 4,096
-    // particles and 19 at 32,768; 370 candidates: 43 and 57); the item kernel's time grows with the particles (10 and 36; 18 and
-    // 96; thin cells in 3D 10 against 15 at 4,000, 28 against 32 at 16,000, 73 against 59 at 64,000).  Crowded cells of otherwise
-    // thin systems make long items.  (Same sums: a row drawn alone is a tile of its own.)
-    const long long particles = (long long)g.B * g.N;
-    const bool few = g.dim == 3 ? particles <= 20000 : particles <= 8192 && g.N >= (particles <= 4096 ? 8 : 20) * g.cells;
+    // A tile takes as long as the candidates of a lane, whatever the number of particles; the item kernel's time grows with the
+    // particles, and with the candidates of crowded cells, which make long items.  Item / tile (density and packed sweep
+    // together, us): 2D clamped, 16 particles a cell: 2,048 11 / 12, 4,096 17.6 / 17.8, 8,192 28 / 23; 4 a cell: 4,096 13.4 / 11.7;
+    // 2D periodic (whose tiles test pair by pair), 16 a cell: 1,024 11 / 19, 4,096 18 / 28, 8,192 31 / 33, 16,384 44 / 43; 3D clamped,
+    // 2 a cell: 4,096 15 / 16, 16,384 30 / 35, 32,768 51 / 61; 8 a cell: 16,384 44 / 45, 24,000 60 / 57; 16 a cell: 4,096 28 / 35,
+    // 8,192 43 / 38.  Over 289 sizes up to 32,768 particles and 32 a cell these lines are at worst 19 % (2 us) behind the
+    // better kernel and 0.4 % on average.  (Same sums: a row drawn alone is a tile of its own.)
+    const long long particles = (long long)g.B * g.N, cells = g.cells;
+    bool few;
+    if (g.dim == 3) few = particles <= 6000 || (particles <= 20000 && g.N < 12 * cells) || (particles <= 33000 && g.N < 6 * cells);
+    else if (g.periodic) few = particles <= 12000;
+    else few = particles <= 1024 || (particles <= 4608 && g.N >= 14 * cells);
     if (few && ticket_rows(g) == 1) {
         if (g.dim == 3) return launch_item<3, false, 2>(g, a, st);
         return g.periodic ? launch_item<2, true, 1>(g, a, st) : launch_item<2, false, 2>(g, a, st);
