@@ -381,7 +381,24 @@ __host__ __device__ inline int table_at(int c) { return c + (c >> 5); }
 static size_t small_smem(const Geom &g) {
     return (size_t)(table_at(g.cells) + 1) * 4 + (size_t)((g.N + 1) & ~1) * 4 + (size_t)((g.N + 31) / 32) * 8;
 }
-static bool small_system(const Geom &g) { return g.N <= kSmallParticles && g.cells < 65536 && small_smem(g) <= kSmallSmem; }
+
+// Whether one CTA per system is the faster way, from estimates of both in microseconds.  Small: a fixed part; the
+// particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell); the cell table, which a thread walks in
+// consecutive cells -- once in shared memory and, with several systems, again in global memory, where long runs per thread
+// scatter the loads.  General: six launches; the shared histogram; the particles and cells of all systems; ranking, spread
+// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells): the choice is at
+// worst 18 % behind the better way (16 or 16,384 cells, near the line) and within 5 % nearly everywhere.  Some of them, small /
+// general, us, in a graph: 1 system of 2,048 in 16 x 16 6 / 23; 4 of 4,096 12 / 22; 64 of 16,384 in 64 x 64 28 / 61; 1 of 16,384 in
+// 8 x 8 93 / 30; 2 of 4,096 in 32^3 77 / 25; 16 of 12,000 in 128 x 128 43 / 28.
+static bool small_system(const Geom &g) {
+    if (g.N > kSmallParticles || g.cells >= 65536 || small_smem(g) > kSmallSmem) return false;
+    const double n = g.N, c = g.cells, all = n * g.B, per_cell = n / c, ranking = per_cell > kCrowdedCell ? 0.0 : n * per_cell;
+    const double small = 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) +
+                         (g.B > 1 ? 3.0 + c * c / 2.2e7 + c / 4000.0 : c / 2500.0);
+    const double general = 16.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
+                           (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7;
+    return small <= general;
+}
 
 // Exclusive scan over the CTA's cell table: every thread takes `per` consecutive cells.  Calls emit(cell, count, prefix)
 // in cell order; returns the grand total.  prefix and total count (work items << 32 | particles).

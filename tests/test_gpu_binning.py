@@ -150,3 +150,14 @@ def test_cells_are_contiguous_and_sorted():
         counts = np.bincount(ids[b], minlength=cells)
         np.testing.assert_array_equal(np.diff(off[b * cells:(b + 1) * cells + 1]), counts)
     assert off[-1] == w.B * w.N
+
+
+@pytest.mark.parametrize("dim,B,N,cells", [
+    (3, 2, 700, 32), (3, 1, 700, 32), (2, 3, 900, 128), (2, 1, 16384, 8), (2, 1, 8192, 8), (2, 1, 6000, 8), (2, 1, 16384, 64),
+    (2, 1, 5000, 4), (3, 2, 16384, 16), (2, 1, 16385, 64)])
+def test_either_way_of_the_grid_build(dim, B, N, cells):
+    """One CTA per system or the general launches: sizes on both sides of the lines between them."""
+    from npa_b200 import sphops as sph
+    w = Workload("ways", dim=dim, B=B, N=N, C=4, eps=1.0 / cells, grid_size=(cells,) * dim, max_particles_per_block=32)
+    x = (torch.rand(B, N, w.P, generator=torch.Generator().manual_seed(cells)) - 0.5) * 1.05
+    _check(sph, w, x)
