@@ -10,6 +10,7 @@
 // the node without a gradient, so that outputs require one wherever any input does), and kernels run on the current
 // stream of the tensors' device.
 #include <torch/extension.h>
+#include <c10/cuda/CUDACachingAllocator.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <torch/csrc/autograd/function.h>
@@ -159,6 +160,9 @@ struct Snap {  // arguments every sweep shares, checked
             require(pairs, {grid->B, grid->N, pairs.dim() == 3 ? pairs.size(2) : -1}, "pair_cache", at::kInt);
             if (pairs.size(2) < 2 || pairs.size(2) > 513)
                 throw std::runtime_error("pair_cache must have between 2 and 513 columns, got " + std::to_string(pairs.size(2)));
+            // The lists belong to the snapshot, which drops them with the next binning: an operator on another stream than the
+            // one that recorded them may still be reading then (the caller never sees them, and could not do this).
+            c10::cuda::CUDACachingAllocator::recordStream(pairs.storage().data_ptr(), c10::cuda::getCurrentCUDAStream(pairs.device().index()));
         }
     }
     int stride() const { return pairs.defined() ? (int)pairs.size(2) : 0; }

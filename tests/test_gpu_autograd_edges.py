@@ -228,3 +228,24 @@ def test_operators_without_features():
     out = sph.blur(xr, rho.detach(), sr, snap)
     gx, = torch.autograd.grad(out, xr, torch.empty_like(out))
     assert not gx.any()
+
+
+def test_lists_read_on_another_stream_are_not_handed_out_again():
+    """The next binning drops a snapshot's lists; memory that a side stream still reads must stay where it is."""
+    sph, grid, x, s = _inputs(N=4001)
+    snap = grid.instantiate(x)
+    xb, sb = sph.bin_particles(x, s, snap)
+    rho = sph.density(xb, snap)
+    want = sph.gradient_hybrid(xb, rho, sb, snap)
+    shape, where = snap.lists[1].shape, snap.lists[1].data_ptr()
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        torch.cuda._sleep(100_000_000)                  # some 50 ms
+        got = sph.gradient_hybrid(xb, rho, sb, snap)
+    grid.instantiate(x)
+    assert snap.lists is None
+    fresh = [torch.full(shape, -7, dtype=torch.int32, device="cuda") for _ in range(3)]
+    assert all(f.data_ptr() != where for f in fresh)
+    torch.cuda.synchronize()
+    assert torch.equal(got, want)
