@@ -142,9 +142,10 @@ _PAIR_CACHE = {"columns": None}
 
 def set_pair_cache(columns=128):
     """Length of the per-particle neighbour lists that the sweeps of a snapshot share (4 * columns bytes
-    per particle while the snapshot or the autograd graph is alive); 0 disables them."""
-    columns = int(columns)
-    if columns != 0 and not 2 <= columns <= 513:
+    per particle while the snapshot or the autograd graph is alive); 0 disables them, None is the default: by the
+    number of neighbours that the grid's mean density gives."""
+    columns = None if columns is None else int(columns)
+    if columns is not None and columns != 0 and not 2 <= columns <= 513:
         raise ValueError("columns must be 0 or between 2 and 513")
     _PAIR_CACHE["columns"] = columns
 

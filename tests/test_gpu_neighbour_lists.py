@@ -43,7 +43,31 @@ def test_channel_counts_against_oracle(dim, boundary, C):
                 # fp32 sums of up to ~100 terms of both signs: a few 1e-6 of the largest value
                 assert_close(a[..., :dim] if name == "grad_x" else a, b, 1e-5, 5e-6, f"{name}, C={C}, columns={columns}")
     finally:
-        sph.set_pair_cache(128)
+        sph.set_pair_cache(None)
+
+
+def test_default_length_of_the_lists_follows_the_grid():
+    """4,096 particles in 10 x 10 cells have 128 neighbours each: the default lists hold them, and every sweep agrees with shorter
+    lists that overflow."""
+    from npa_b200 import sphops as sph
+    grid = sph.HashGrid(dim=2, boundary="periodic", mode="grid", grid_size=(10, 10), eps=0.1, num_particles=4096, batch_size=1)
+    g = torch.Generator().manual_seed(1)
+    x = (torch.rand(1, 4096, 2, generator=g) - 0.5).cuda()
+    snap = grid.instantiate(x)
+    xb, sb = sph.bin_particles(x, torch.randn(1, 4096, 8, generator=g).cuda(), snap)
+    rho = sph.density(xb, snap)
+    lists = snap.lists[1]
+    assert lists.shape[2] == grid.hashgrid.list_columns == 256 and int(lists[..., 0].min()) > 0 and int(lists[..., 0].max()) > 127
+    assert float((lists[..., 0].float() - sph.count(xb, snap)).abs().max()) <= 1.0     # (a pair on the cut-off itself)
+    want = sph.blur(xb, rho, sb, snap)
+    sph.set_pair_cache(64)
+    try:
+        sph.density(xb, snap)
+        assert int(snap.lists[1][..., 0].max()) == -1
+        got = sph.blur(xb, rho, sb, snap)
+    finally:
+        sph.set_pair_cache(None)
+    assert torch.allclose(got, want, rtol=1e-4, atol=1e-5 * float(want.abs().max()))
 
 
 def _oracle_chain(oracle, w, xb, sb, rho, ups, kw):

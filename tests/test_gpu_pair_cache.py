@@ -125,7 +125,7 @@ def test_public_api_uses_and_sizes_the_cache():
             torch.autograd.backward(list(outs), ups)
             grads.append((xr.grad.clone(), sr.grad.clone()))
     finally:
-        sph.set_pair_cache(64)
+        sph.set_pair_cache(None)
     with pytest.raises(ValueError):
         sph.set_pair_cache(1)
     for gx, gs in grads[1:]:
