@@ -599,9 +599,14 @@ int npa_tile_status(int32_t *host_status, int32_t reset);
 int npa_row_tickets_status(int32_t *host_nonzero_words, int32_t reset);
 /* The count and density forward sweeps let the particles of a work item share the candidates they test (the
  * sharing of a staged cell among the threads of a block in sphops/sph_cuda.cu:1664-1690).  cells_per_tile = 0
- * switches to the per-particle candidate walk, any other accepted value (1..8, 101..108) back; default 3.
- * Process-wide. */
+ * switches to the per-particle candidate walk, any other accepted value (1..8, 101..108) back; default 3.  The
+ * numbers sized the tiles of an earlier search and are accepted for its callers.  Process-wide. */
 int npa_scalar_sweep_tuning(int32_t cells_per_tile);
+/* Self-test of the square root and the quotient of the packed perception (no counterpart in the reference): `count` operands
+ * whose bits are first_bits + k * step, all in [2^-66, 2^66), are compared with CUDA's correctly rounded root, and one quotient by
+ * each root, its numerator drawn from `seed` and k, with the correctly rounded division.  The differences are added to
+ * device_mismatches[0] (roots) and [1] (quotients), int32 in device memory. */
+int npa_rounding_selftest(uint32_t first_bits, int32_t step, int32_t count, uint32_t seed, int32_t *device_mismatches, void *stream);
 /* Self-test of the bounded waits: one CTA waits for an mbarrier phase that is never completed and
  * writes to *device_result (int32, device memory) 1 when the wait gave up after limit_us
  * microseconds (the expected outcome) or 0 had it completed.  Faults nothing; the context stays

@@ -113,6 +113,7 @@ SIGNATURES = {
     "npa_linear_tcgen05_status": (ctypes.c_int, [_P, _I32]),
     "npa_linear_tcgen05_wait_selftest": (ctypes.c_int, [_I32, _P, _P]),
     "npa_step_update_backward": (ctypes.c_int, [_P] * 3 + [_I32, ctypes.c_float, ctypes.c_float, _P, _P, _P, _P]),
+    "npa_rounding_selftest": (ctypes.c_int, [ctypes.c_uint32, _I32, _I32, ctypes.c_uint32, _P, _P]),
     "npa_tile_enabled": (ctypes.c_int, [_I32]),
     "npa_tile_tuning": (ctypes.c_int, [_I32, _I32, _I32, _I32, _I32, _I32, _I32]),
     "npa_tile_status": (ctypes.c_int, [_P, _I32]),

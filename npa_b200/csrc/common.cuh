@@ -200,8 +200,9 @@ __device__ inline Spiky spiky_distance(float q) {
     return Spiky{fmaf(0.5f * y, fmaf(-d, d, Q), d), y};
 }
 // Square root and quotient as IEEE rounds them, without the range checks and branches of the general routines: Newton steps
-// whose residuals are exact by fused multiply-add (P. Markstein, IA-64 and Elementary Functions, ch. 8-9).  Q normal,
-// 2^-66 <= Q < 2^66: over all of them the root equals __fsqrt_rn, and 6e9 quotients of them equal __fdiv_rn.
+// whose residuals are exact by fused multiply-add (P. Markstein, IA-64 and Elementary Functions, ch. 8-9).  For
+// 2^-66 <= Q < 2^66; npa_rounding_selftest compares them with __fsqrt_rn and __fdiv_rn (tests/test_gpu_rounding.py: every root of
+// two binades, 2^17 of each other one, a quotient by each).
 struct Root {
     float d, inv;  // sqrt(Q), and 1 / d to within an ulp
 };

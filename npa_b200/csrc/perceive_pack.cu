@@ -90,6 +90,22 @@ add_direct_kernel(const float *__restrict__ gz, float *__restrict__ grad_s, long
     grad_s[t] += gz[i * Z + (t - i * C)];
 }
 
+// Differences of root_rounded and quotient_rounded from CUDA's rounded intrinsics.
+__global__ void __launch_bounds__(256)
+rounding_selftest_kernel(uint32_t first, int step, int count, uint32_t seed, int32_t *__restrict__ mismatches) {
+    const int k = blockIdx.x * 256 + threadIdx.x;
+    if (k >= count) return;
+    const float Q = __uint_as_float(first + (uint32_t)k * (uint32_t)step);
+    const Root r = root_rounded(Q);
+    const float want = __fsqrt_rn(Q);
+    uint32_t u = ((uint32_t)k + 1u) * 2654435761u + seed * 40503u;  // scrambled: the mantissa and the exponent of the numerator
+    u = (u ^ (u >> 15)) * 0x2c1b3c6du;
+    u ^= u >> 12;
+    const float n = __fmul_rn(__uint_as_float(0x3f800000u | (u >> 9)), ldexpf(want, (int)(u % 81u) - 40));
+    if (r.d != want) atomicAdd(mismatches, 1);
+    else if (quotient_rounded(n, r) != __fdiv_rn(n, want)) atomicAdd(mismatches + 1, 1);
+}
+
 }  // namespace npa
 
 using namespace npa;
@@ -165,6 +181,15 @@ int npa_perceive_features_forward(const npa_grid *gd, int32_t channels, const fl
                                   int32_t *pair_cache, int32_t pair_stride, void *stream) {
     return npa_perceive_features_forward_lists(gd, channels, x_bin, mass, s_bin, coef, dg_scale, inv_tol, log_norm_grad, log_norm_dg, rho,
                                                rho_grad, z, vgrad, nullptr, bin_offsets, block_info, pair_cache, pair_stride, stream);
+}
+
+int npa_rounding_selftest(uint32_t first_bits, int32_t step, int32_t count, uint32_t seed, int32_t *device_mismatches, void *stream) {
+    if (!device_mismatches || step <= 0 || count <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "rounding_selftest: bad arguments");
+    const int64_t last = (int64_t)first_bits + (int64_t)step * (count - 1);
+    if (first_bits < (uint32_t)(127 - 66) << 23 || last >= (int64_t)(127 + 66) << 23)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "rounding_selftest: operands must lie in [2^-66, 2^66)");
+    rounding_selftest_kernel<<<(unsigned)((count + 255) / 256), 256, 0, (cudaStream_t)stream>>>(first_bits, step, count, seed, device_mismatches);
+    return check_launch("rounding_selftest_kernel");
 }
 
 int64_t npa_lists_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
