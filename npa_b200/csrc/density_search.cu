@@ -1,13 +1,13 @@
 // Density and neighbour count by the cell search, and the recording of the neighbour lists: the one
 // search of a snapshot, whose lists every later sweep reads.
 //
-// Linear hash (density_tile_kernel): particles of an x-row of cells are consecutive, so a warp takes 32
-// consecutive particles, a lane each, and tests them against the candidates of the 3 (9) rows of cells
+// Linear hash (density_tile_kernel): particles of an x-row of cells are consecutive, so a warp takes 16
+// consecutive particles, two lanes each, and tests them against the candidates of the 3 (9) rows of cells
 // around the ones they span.  The candidates are staged end to end in shared memory and read as
 // broadcasts, two at a time in packed fp32x2; a lane shifts the sign of every r^2 - h^2 into a word, walks
 // the set bits of each 32 and collects slot numbers (bytes) in shared memory; the lists leave in runs,
-// eight lanes to a list.  No work items, no tickets, no reductions.
-// Morton hash (density_item_kernel): the neighbours of 32 consecutive particles are scattered over many
+// eight lanes to a list.  No work items, no tickets, no reductions but the one between a particle's lanes.
+// Morton hash, and fewer than 16,384 particles (density_item_kernel): the neighbours of 32 consecutive particles are scattered over many
 // short ranges; a warp takes the particles of one cell, lays the candidates of its 3^D cells end to end,
 // one gather per item, and tests 32 candidates, a lane each, against four particles at once; a scan of the
 // accepted bits places the entries.
@@ -53,11 +53,11 @@ __device__ inline void item_cell(const Geom &g, uint32_t hsh, int &cx, int &cy, 
 }
 
 // ---------------------------------------------------------------------------------------------------------
-// Linear hash: a lane per particle.
+// Linear hash: two lanes per particle.
 // ---------------------------------------------------------------------------------------------------------
 constexpr int kTileWarps = 2;
 constexpr int kTileSlots = 256;  // candidates staged at a time per warp; a slot number is a byte
-constexpr int Q = 2;             // lanes per particle, below
+constexpr int kShare = 2;        // lanes per particle, below
 constexpr int kTileRun = 132;    // bytes per lane for the slots accepted since the last flush (33 words: spread over the banks)
 
 // Signs of two differences r^2 - h^2 shifted into a word, the first candidate's bit ending up highest: the bit is set
@@ -75,13 +75,13 @@ template <bool MASS> struct TileStage {
     unsigned char run[32 * kTileRun];
 };
 
-// Q lanes share a particle (each takes every Q-th batch of 32 candidates): 32 / Q consecutive particles per warp.  Fewer
+// kShare lanes share a particle (each takes every kShare-th batch of 32 candidates): 32 / kShare particles per warp.  Fewer
 // particles span fewer cells and meet fewer candidates that none of them accepts, but set up more often: 262,144
-// particles in 3D took 105 / 98 / 126 us with Q = 1 / 2 / 4, 524,288 periodic 340 / 321 / 403, 32,768 in 2D 15.1 / 13.6 / 16.2.
+// particles in 3D took 105 / 98 / 126 us with 1 / 2 / 4 lanes, 524,288 periodic 340 / 321 / 403, 32,768 in 2D 15.1 / 13.6 / 16.2.
 template <int D, bool PER, bool COUNT, bool MASS>
 __global__ void __launch_bounds__(kTileWarps * 32, 12)
 density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g) {
-    constexpr int PT = 32 / Q;
+    constexpr int PT = 32 / kShare;
     extern __shared__ __align__(16) unsigned char s_tile[];
     __shared__ int4 s_rng[kTileWarps][kMaxRanges];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = lane / PT;
@@ -98,7 +98,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
     snapshot_cell_of<D>(g, a.bin_offsets + (size_t)sys * g.cells, i, pi.x, pi.y, pi.z, cx, cy, cz);
     const int key = (sys * g.g[2] + cz) * g.g[1] + cy;
     const bool stray = PER && outside_cells<D>(g, pi, cx, cx, cy, cy, cz, cz);
-    unsigned left = __ballot_sync(kFull, ivalid) & (Q == 1 ? kFull : ((1u << (PT & 31)) - 1u));  // particles to do
+    unsigned left = __ballot_sync(kFull, ivalid) & ((1u << PT) - 1u);  // particles to do
     while (left) {
         // ---- the particles of one x-row of cells, and the candidates of the rows around the cells they span
         const int lead = __ffs(left) - 1;
@@ -129,10 +129,10 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
         const bool lists = !COUNT && a.pair_cache != nullptr;
 
         float rho = 0.f;
-        int found = 0;  // of the particle, the same in its Q lanes
+        int found = 0;  // of the particle, the same in its lanes
         unsigned long long sum2 = 0ull;
         for (int c0 = 0; c0 < total; c0 += cap) {
-            const int count = min(cap, total - c0), padded = (count + 32 * Q - 1) / (32 * Q) * (32 * Q);
+            const int count = min(cap, total - c0), padded = (count + 32 * kShare - 1) / (32 * kShare) * (32 * kShare);
             __syncwarp();
             bool outside = false;
             if (!PER) {
@@ -216,13 +216,11 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
             unsigned char *run = S.run + lane * kTileRun;
             auto flush = [&]() {
                 int before = 0, sum = held;  // entries of the particle's other lanes ahead of this one's, and all of them
-                if (Q > 1) {
 #pragma unroll
-                    for (int q = 1; q < Q; ++q) {
-                        const int v = __shfl_sync(kFull, held, (lane + q * PT) & 31);
-                        sum += v;
-                        if (((lane + q * PT) & 31) / PT < part) before += v;
-                    }
+                for (int q = 1; q < kShare; ++q) {
+                    const int v = __shfl_sync(kFull, held, (lane + q * PT) & 31);
+                    sum += v;
+                    if (((lane + q * PT) & 31) / PT < part) before += v;
                 }
                 const int at = found + before, take = min(held, K - 1 - at);  // entries that still fit
                 __syncwarp();
@@ -311,7 +309,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
             };
             // One copy of the rest for all ways of testing: with a copy for each, a sixth of the periodic kernel's stalls were
             // waits for instructions (524,288 particles 311 us, so 281).
-            for (int s0 = part * 32; s0 < padded; s0 += 32 * Q) {
+            for (int s0 = part * 32; s0 < padded; s0 += 32 * kShare) {
                 unsigned m;
                 if (PER && (check || (COUNT && wrapped))) m = test(Mode<2>(), s0);
                 else if (PER && wrapped) m = test(Mode<1>(), s0);
@@ -326,8 +324,8 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                         held += m != 0u;
                         m &= ~(0x80000000u >> (b & 31));
                     }
-                    // (the lanes of a warp go round equally often: padded is a multiple of 32 Q)
-                    if (s0 + 32 * Q >= padded || __any_sync(kFull, held > kTileRun - 4 - 32)) flush();
+                    // (the lanes of a warp go round equally often: padded is a multiple of 32 kShare)
+                    if (s0 + 32 * kShare >= padded || __any_sync(kFull, held > kTileRun - 4 - 32)) flush();
                 }
             }
         }
@@ -359,7 +357,7 @@ static int launch_tile(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     int unused = 0;
     const int rc = persistent_ctas(kernel, kTileWarps * 32, dyn, &unused);  // raises the shared-memory limit once
     if (rc != NPA_OK) return rc;
-    const long long per_cta = (long long)kTileWarps * (32 / Q), particles = (long long)g.B * g.N;
+    const long long per_cta = (long long)kTileWarps * (32 / kShare), particles = (long long)g.B * g.N;
     kernel<<<(unsigned)((particles + per_cta - 1) / per_cta), kTileWarps * 32, dyn, st>>>(a, g);
     return check_launch("density_tile_kernel");
 }
