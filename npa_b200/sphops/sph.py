@@ -190,9 +190,10 @@ def _key(*tensors):
     """Identity + version of the input tensor objects (None allowed), held weakly: a parked output never
     keeps its inputs alive, and an input that has died can never match again.  None when one of them is an
     inference tensor: those have no version, a change in place would go unnoticed."""
-    if any(t is not None and t.is_inference() for t in tensors):
+    try:
+        return tuple((None if t is None else weakref.ref(t), None if t is None else t._version) for t in tensors)
+    except RuntimeError:  # "Inference tensors do not track version counter"
         return None
-    return tuple((None if t is None else weakref.ref(t), None if t is None else t._version) for t in tensors)
 
 
 def _same(key, *tensors):
