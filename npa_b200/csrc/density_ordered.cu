@@ -308,9 +308,9 @@ density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __gri
                             int code[5];
 #pragma unroll
                             for (int u = 0; u < 5; ++u) {
-                                const int c = min(c0 + 32 * u, count - 1);
-                                p[u] = load_pos<D>(a.x, __float_as_uint(S.cand[c].w) >> 2);
-                                code[u] = PER && decltype(shifted_cells)::value ? S.code[c] : shift_code(0, 0, 0);
+                                const int c = c0 + 32 * u;
+                                if (c < count) p[u] = load_pos<D>(a.x, __float_as_uint(S.cand[c].w) >> 2);
+                                code[u] = PER && decltype(shifted_cells)::value && c < count ? S.code[c] : shift_code(0, 0, 0);
                             }
 #pragma unroll
                             for (int u = 0; u < 5; ++u) {
