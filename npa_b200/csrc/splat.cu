@@ -83,8 +83,8 @@ __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
 // are culled with a pixel to spare (ordered compaction); 64 at a time get their 16 + 16 factors in shared memory (32
 // exponentials per particle and tile instead of 256), eight per thread; every half warp multiplies every 16th particle
 // into 8 x 2 pixels x 4 channels per thread in packed fp32x2; the 16 partial images are added in a fixed order.  Bound
-// by instruction issue (culling, factors and products about a third each).  8 systems of 4,096 particles, 256 x 256,
-// patches of 41 x 41: 201 -> 123 us.
+// by latency (factors read from shared memory, particles, barriers) at two blocks per SM: 38 % of the issue slots.  8 systems
+// of 4,096 particles, 256 x 256, patches of 41 x 41: pixel by pixel 201 us, this 119.
 constexpr int kSplatThreads = 256, kSplatCull = 4, kSplatChunk = 64, kSplatParts = 16, kSplatWarps = kSplatThreads / 32;
 
 struct SplatLists {
