@@ -723,12 +723,15 @@ struct EulerNode : Node {
     SavedVariable w1_, w2_, slab_, mask_;
     Tensor offs, perm, info;
     int64_t o_x, o_s, o_rho, o_dg, o_v, o_packed, o_z, o_h, o_y, o_dz, o_pairs;  // places in the slab, in floats
-    int64_t C, columns, dz_bytes;
+    int64_t C, columns, dz_bytes, slab_floats;
     float coef, dg_scale, alpha, dt, below;
     bool ln_grad, ln_dg, stop_pos, stop_state;
 
     variable_list apply(variable_list &&g) override {
-        const Tensor w1 = w1_.unpack(), w2 = w2_.unpack(), slab = slab_.unpack(), mask = mask_.unpack();  // raise when the graph was released
+        const Tensor w1 = w1_.unpack(), w2 = w2_.unpack(), slab = solid(slab_.unpack()), mask = mask_.unpack();  // raise when the graph was released
+        // (a hook may have had it elsewhere: the places below are only good in a block of the same size)
+        TORCH_CHECK(slab.numel() == slab_floats && slab.scalar_type() == at::kFloat && slab.device() == w1.device(),
+                    "a saved-tensor hook returned another tensor than the step had saved");
         const Tensor gx_new = solid(g[0]), gs_new = solid(g[1]);
         if (!gx_new.defined() && !gs_new.defined()) return variable_list(5);
         const float *kept = fptr(slab), *x_bin = kept + o_x, *s_bin = kept + o_s, *rho = kept + o_rho, *rho_grad = kept + o_dg, *vgrad = kept + o_v,
@@ -839,7 +842,7 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
         auto n = node_for<EulerNode>(x, s, w1, b1, w2);
         n->grid = grid; n->offs = offs; n->perm = perm; n->info = info; n->slab_ = saved(slab); n->mask_ = saved(mask);
         n->o_x = o_x; n->o_s = o_s; n->o_rho = o_rho; n->o_dg = o_dg; n->o_v = o_v; n->o_packed = o_packed; n->o_z = o_z; n->o_h = o_h; n->o_y = o_y;
-        n->o_dz = o_dz; n->o_pairs = o_pairs; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
+        n->o_dz = o_dz; n->o_pairs = o_pairs; n->slab_floats = l.floats; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
         n->w1_ = saved(w1); n->w2_ = saved(w2);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
         n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;

@@ -249,3 +249,29 @@ def test_lists_read_on_another_stream_are_not_handed_out_again():
     assert all(f.data_ptr() != where for f in fresh)
     torch.cuda.synchronize()
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("change", ["short", "half", "offset"])
+def test_what_a_hook_returns_for_a_step_is_checked(change):
+    """The node of a step reads its saved block by offsets: another size or type is refused, another address is not."""
+    x, s, steps, _ = _steps()
+    want = _value_and_grads(steps["step"], x, s)
+
+    def unpack(t):
+        if t.numel() < 100_000:              # weights and mask
+            return t
+        if change == "short":
+            return t[:-64]
+        if change == "half":
+            return t.half()
+        flat = torch.empty(t.numel() + 1, device="cuda")
+        flat[1:].copy_(t)
+        return flat[1:]
+
+    with torch.autograd.graph.saved_tensors_hooks(lambda t: t, unpack):
+        if change == "offset":
+            got = _value_and_grads(steps["step"], x, s)
+            assert all(torch.equal(p, q) for p, q in zip([*got[0], *got[1]], [*want[0], *want[1]]))
+        else:
+            with pytest.raises(RuntimeError, match="saved-tensor hook"):
+                _value_and_grads(steps["step"], x, s)
