@@ -437,16 +437,16 @@ int launch_density_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t s
     }
     // A tile takes as long as the candidates of a lane, whatever the number of particles; the item kernel's time grows with the
     // particles, and with the candidates of crowded cells, which make long items.  Item / tile (density and packed sweep
-    // together, us): 2D clamped, 16 particles a cell: 2,048 11 / 12, 4,096 17.6 / 17.8, 8,192 28 / 23; 4 a cell: 4,096 13.4 / 11.7;
+    // together, us): 2D clamped, 16 particles a cell: 2,048 15.6 / 17.3, 4,096 17.6 / 17.8, 8,192 28 / 23; 4 a cell: 1,024 10.0 / 10.6, 4,096 13.4 / 11.7;
     // 2D periodic (whose tiles test pair by pair), 16 a cell: 1,024 11 / 19, 4,096 18 / 28, 8,192 31 / 33, 16,384 44 / 43; 3D clamped,
     // 2 a cell: 4,096 15 / 16, 16,384 30 / 35, 32,768 51 / 61; 8 a cell: 16,384 44 / 45, 24,000 60 / 57; 16 a cell: 4,096 28 / 35,
-    // 8,192 43 / 38.  Over 289 sizes up to 32,768 particles and 32 a cell these lines are at worst 19 % (2 us) behind the
-    // better kernel and 0.4 % on average.  (Same sums: a row drawn alone is a tile of its own.)
+    // 8,192 43 / 38.  Over 289 sizes up to 32,768 particles and 32 a cell these lines are at worst 12 % (3 us) behind the
+    // better kernel and 0.3 % on average.  (Same sums: a row drawn alone is a tile of its own.)
     const long long particles = (long long)g.B * g.N, cells = g.cells;
     bool few;
     if (g.dim == 3) few = particles <= 6000 || (particles <= 20000 && g.N < 12 * cells) || (particles <= 33000 && g.N < 6 * cells);
     else if (g.periodic) few = particles <= 12000;
-    else few = particles <= 1024 || (particles <= 4608 && g.N >= 14 * cells);
+    else few = particles <= 4608 && 320ll * g.N >= particles * cells;
     if (few && ticket_rows(g) == 1) {
         if (g.dim == 3) return launch_item<3, false, 2>(g, a, st);
         return g.periodic ? launch_item<2, true, 1>(g, a, st) : launch_item<2, false, 2>(g, a, st);
