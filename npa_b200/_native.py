@@ -156,11 +156,12 @@ def _load_ops():
     return _torch_ops
 
 
-def _traced(native, name, args):
-    """``native(*args)`` as one Python node of the graph that ``torch.jit.trace`` is recording.  A trace sees no C++ node:
-    it would keep the outputs of the traced call as constants."""
+def _traced(name, *args):
+    """The native operator ``name`` as one Python node of the graph that ``torch.jit.trace`` is recording (called by the
+    operator itself): a trace sees no C++ node and would keep the outputs of the traced call as constants."""
     import torch
 
+    native = getattr(ops, name)
     blank = []  # positions of the outputs that are None
 
     class Call(torch.autograd.Function):
@@ -201,28 +202,7 @@ def _traced(native, name, args):
     return tuple(out)
 
 
-class _Ops:
-    """The native operators; while ``torch.jit.trace`` records, each call is a node of its own in the trace."""
-
-    def __init__(self, module):
-        import torch
-
-        tracing = torch._C._get_tracing_state
-
-        def guard(name, native):
-            def call(*args):
-                return native(*args) if tracing() is None else _traced(native, name, args)
-
-            call.__name__ = name
-            return call
-
-        self.Grid = module.Grid
-        for name in dir(module):
-            if callable(getattr(module, name)) and name not in ("Grid",) and not name.startswith("_"):
-                setattr(self, name, guard(name, getattr(module, name)))
-
-
-ops = _Ops(_load_ops())
+ops = _load_ops()
 
 
 def last_error() -> str:

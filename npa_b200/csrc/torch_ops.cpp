@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/function.h>
 #include <torch/csrc/autograd/functions/utils.h>
 #include <torch/csrc/autograd/saved_variable.h>
+#include <torch/csrc/jit/frontend/tracer.h>
 
 #include "../../include/npa_b200.h"
 
@@ -891,24 +892,35 @@ Tensor splat(const Tensor &x, const Tensor &color, int img, double sigma, int ra
     return out;
 }
 
+// `fn` as Python calls it.  torch.jit.trace sees no C++ node and would keep the outputs of the traced call as constants: while
+// it records, the call is handed to Python, which makes it one node of the trace (npa_b200/_native.py).
+template <typename R, typename... A>
+auto op(const char *name, R (*fn)(A...)) {
+    return [name, fn](A... a) -> py::object {
+        if (torch::jit::tracer::isTracing()) return py::module_::import("npa_b200._native").attr("_traced")(name, a...);
+        if constexpr (std::is_base_of_v<py::object, R>) return fn(a...);
+        else return py::cast(fn(a...));
+    };
+}
+
 }  // namespace
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
     m.attr("abi_version") = NPA_B200_ABI_VERSION;
     py::class_<Grid, GridPtr>(m, "Grid").def(py::init<uintptr_t>());
-    m.def("instantiate", &instantiate);
-    m.def("reorder", &reorder);
-    m.def("unreorder", &unreorder);
-    m.def("count", &count);
-    m.def("density", &density);
-    m.def("blur_gradient", &blur_gradient);
-    m.def("gradient_hybrid", &gradient_hybrid);
-    m.def("moment_matrix", &moment_matrix);
-    m.def("corrected_gradient", &corrected_gradient);
-    m.def("perception", &perception);
-    m.def("packed_perception", &packed_perception);
-    m.def("step_update", &step_update);
-    m.def("mlp", &mlp);
-    m.def("euler_step", &euler_step);
-    m.def("splat", &splat);
+    m.def("instantiate", op("instantiate", &instantiate));
+    m.def("reorder", op("reorder", &reorder));
+    m.def("unreorder", op("unreorder", &unreorder));
+    m.def("count", op("count", &count));
+    m.def("density", op("density", &density));
+    m.def("blur_gradient", op("blur_gradient", &blur_gradient));
+    m.def("gradient_hybrid", op("gradient_hybrid", &gradient_hybrid));
+    m.def("moment_matrix", op("moment_matrix", &moment_matrix));
+    m.def("corrected_gradient", op("corrected_gradient", &corrected_gradient));
+    m.def("perception", op("perception", &perception));
+    m.def("packed_perception", op("packed_perception", &packed_perception));
+    m.def("step_update", op("step_update", &step_update));
+    m.def("mlp", op("mlp", &mlp));
+    m.def("euler_step", op("euler_step", &euler_step));
+    m.def("splat", op("splat", &splat));
 }
