@@ -385,9 +385,10 @@ static size_t small_smem(const Geom &g) {
 // Whether one CTA per system is the faster way, from estimates of both in microseconds.  Small: a fixed part; the
 // particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell); the cell table, which a thread walks in
 // consecutive cells -- once in shared memory and, with several systems, again in global memory, where long runs per thread
-// scatter the loads.  General: six launches; the shared histogram; the particles and cells of all systems; ranking, spread
-// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells): the choice is at
-// worst 18 % behind the better way (16 or 16,384 cells, near the line) and within 5 % nearly everywhere.  Some of them, small /
+// scatter the loads.  General: six launches and their gaps; the shared histogram; the particles and cells of all systems; ranking, spread
+// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells) in a graph; back to
+// back on a stream the general way takes 8 us more, in the gaps between its launches, and that is counted (8 systems of
+// 16,384 in 40 x 40: kernels 35 / 28, but a pass that bins them is 8 us shorter with the small way).  Some sizes, small /
 // general, us, in a graph: 1 system of 2,048 in 16 x 16 6 / 23; 4 of 4,096 12 / 22; 64 of 16,384 in 64 x 64 28 / 61; 1 of 16,384 in
 // 8 x 8 93 / 30; 2 of 4,096 in 32^3 77 / 25; 16 of 12,000 in 128 x 128 43 / 28.
 static bool small_system(const Geom &g) {
@@ -395,7 +396,7 @@ static bool small_system(const Geom &g) {
     const double n = g.N, c = g.cells, all = n * g.B, per_cell = n / c, ranking = per_cell > kCrowdedCell ? 0.0 : n * per_cell;
     const double small = 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) +
                          (g.B > 1 ? 3.0 + c * c / 2.2e7 + c / 4000.0 : c / 2500.0);
-    const double general = 16.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
+    const double general = 24.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
                            (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7;
     return small <= general;
 }
