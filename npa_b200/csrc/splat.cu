@@ -13,9 +13,12 @@
 // frac = p - base; weight of pixel base + (dx, dy): g = exp(-((dx - frac_x)^2 + (dy - frac_y)^2) / (2 sigma^2)),
 // with normalisation w = g / (1e-8 + sum of g over the whole patch) * norm_scale; out = [sum c w | sum w].
 // The patch sum factorises into two 1D sums (the weight is separable).
+#include <cooperative_groups.h>
 #include "common.cuh"
 
 namespace npa {
+
+namespace cg = cooperative_groups;
 
 constexpr int kSplatTile = 16;
 constexpr int kSplatMaxRadius = 64;
@@ -37,20 +40,22 @@ struct SplatPoint {
     float fx, fy;
 };
 
+// Pixel of a coordinate along one axis, and the fraction beyond it.  Far-away or non-finite positions touch no pixel: they
+// are parked outside every tile.
+__device__ inline int splat_axis(const SplatArgs &a, float v, int axis, float &frac) {
+    const float top = (float)(a.img - 1);
+    float p = __fmul_rn(__fdiv_rn(v - a.lo, a.span), top);
+    if (axis && a.y_up) p = top - p;
+    const float base = floorf(p), lim = 1.0e8f;
+    frac = p - base;
+    return (base > -lim && base < lim) ? (int)base : -(1 << 30);
+}
+
 __device__ inline SplatPoint splat_point(const SplatArgs &a, long long n) {
     const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + n);
-    const float top = (float)(a.img - 1);
-    float px = __fmul_rn(__fdiv_rn(v.x - a.lo, a.span), top);
-    float py = __fmul_rn(__fdiv_rn(v.y - a.lo, a.span), top);
-    if (a.y_up) py = top - py;
-    const float bx = floorf(px), by = floorf(py);
     SplatPoint p;
-    // far-away or non-finite positions touch no pixel: park them outside every tile
-    const float lim = 1.0e8f;
-    p.cx = (bx > -lim && bx < lim) ? (int)bx : -(1 << 30);
-    p.cy = (by > -lim && by < lim) ? (int)by : -(1 << 30);
-    p.fx = px - bx;
-    p.fy = py - by;
+    p.cx = splat_axis(a, v.x, 0, p.fx);
+    p.cy = splat_axis(a, v.y, 1, p.fy);
     return p;
 }
 
@@ -79,18 +84,28 @@ __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
 }
 
 // A CTA per 16 x 16 pixel tile.  The weight of a particle is a product of a row and a column factor, so a tile's image is
-// a product of small matrices over the particles that touch it: sum_n wx_n[px] (wy_n[py] c_n).  1,024 particles at a time
-// are culled with a pixel to spare (ordered compaction); 64 at a time get their 16 + 16 factors in shared memory (32
-// exponentials per particle and tile instead of 256), eight per thread; every half warp multiplies every 16th particle
-// into 8 x 2 pixels x 4 channels per thread in packed fp32x2; the 16 partial images are added in a fixed order.  Bound
-// by latency (factors read from shared memory, particles, barriers) at two blocks per SM: 38 % of the issue slots.  8 systems
-// of 4,096 particles, 256 x 256, patches of 41 x 41: pixel by pixel 201 us, this 119.
-constexpr int kSplatThreads = 256, kSplatCull = 4, kSplatChunk = 64, kSplatParts = 16, kSplatWarps = kSplatThreads / 32;
+// a product of small matrices over the particles that touch it: sum_n wx_n[px] (wy_n[py] c_n).  4,096 particles at a time are
+// culled with a pixel to spare into a list (a thread's hits in a row, threads in order); 64 at a time get their 16 + 16
+// factors in shared memory (32 exponentials per particle and tile instead of 256; eight per thread) while the 64 before are
+// multiplied; every half warp multiplies every 16th particle into 8 x 2 pixels x 4 channels per thread in packed fp32x2, two
+// neighbouring pixels to a pair; the 16 partial images are added in a fixed order.  SLICED: the CTAs of a cluster share the tile,
+// each with a slice of the particles, and add their images through distributed shared memory, slices in order.
+// Bound by latency (fill of the list, first factors, sum of the partial images) at two blocks per SM: 45 % of the issue slots,
+// fp32 pipe 22 %.  8 systems of 4,096 particles, 256 x 256, patches of 41 x 41, us: pixel by pixel 201; list of 1,024
+// particles at a time, factors and products between barriers, channels packed (wants every column factor twice) 113; this 86.  64 x 64,
+// one system of 8,192: 92 -> 19 (eight slices).  More warps do not fit: 64 sums per thread.
+constexpr int kSplatThreads = 256, kSplatCull = 16, kSplatWindow = kSplatThreads * kSplatCull, kSplatChunk = 64, kSplatParts = 16,
+              kSplatWarps = kSplatThreads / 32;
 
-struct SplatLists {
-    int n[kSplatThreads * kSplatCull + kSplatChunk];
+struct SplatFactors {
     float wx[kSplatChunk][kSplatTile];
-    float4 wy[kSplatChunk][kSplatTile];  // row factor times scale times (r, g, b, 1)
+    float pad[4];                       // the row and the column factors that one instruction stores lie on different banks
+    float wy[kSplatChunk][kSplatTile];
+    float4 c[kSplatChunk];              // scale times (r, g, b, 1)
+};
+struct SplatLists {
+    SplatFactors f[2];
+    unsigned short n[kSplatWindow];
 };
 union SplatShared {
     SplatLists lists;
@@ -101,163 +116,185 @@ union SplatShared {
 // layout (4,096 tiles with a few particles each: 67 us, so 48).
 __device__ inline int part_at(int pixel) { return pixel ^ ((pixel >> 5) & 7); }
 
+template <bool SLICED>
 __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatArgs a) {
     __shared__ SplatShared sh;
-    __shared__ int s_count[kSplatCull * kSplatWarps];
+    __shared__ int s_count[kSplatWarps];
     const int tiles = (a.img + kSplatTile - 1) / kSplatTile;
-    const int tx0 = (blockIdx.x % tiles) * kSplatTile, ty0 = (blockIdx.x / tiles) * kSplatTile;
+    const int slices = SLICED ? (int)cg::this_cluster().num_blocks() : 1, slice = SLICED ? blockIdx.x % slices : 0, tile = blockIdx.x / slices;
+    const int tx0 = (tile % tiles) * kSplatTile, ty0 = (tile / tiles) * kSplatTile;
     const int b = blockIdx.y, r = a.radius;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int part = tid >> 4, cell = tid & 15, px = (cell & 1) * 8, py = (cell >> 1) * 2;  // pixels px..px+7, py..py+1
     const float inv2s2 = 1.0f / (2.0f * a.sigma * a.sigma);
-    unsigned long long acc[2][8][2];  // [row][pixel][(r, g), (b, density)]
+    unsigned long long acc[2][4][4];  // [row][channel][two pixels]
 #pragma unroll
     for (int y = 0; y < 2; ++y)
 #pragma unroll
-        for (int x = 0; x < 8; ++x) acc[y][x][0] = acc[y][x][1] = 0ull;
+        for (int c = 0; c < 4; ++c)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) acc[y][c][x] = 0ull;
 
-    // particles off .. off + count - 1 of the list
-    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto multiply = [&](int off, int count) {
-        bool odd = false;  // a colour that is not finite: zero times it is not zero outside the patch
-        const int padded = (count + kSplatParts - 1) / kSplatParts * kSplatParts;
-        const int p = tid >> 2, axis = (tid >> 1) & 1, o0 = (tid & 1) * 8;
-        if (p < padded) {
-            float w[8];
-            float4 c = zero;
-            int at = 0, lo = 1, hi = 0;
-            float frac = 0.f;
-            if (p < count) {
-                const long long n = (long long)b * a.N + sh.lists.n[off + p];
-                const SplatPoint pt = splat_point(a, n);
-                at = (axis ? ty0 - pt.cy : tx0 - pt.cx) + o0;  // offset of the first of the eight from the particle's pixel
-                frac = axis ? pt.fy : pt.fx;
-                lo = -r; hi = r;
-                if (axis) {
-                    const float scale = a.normalize ? __ldg(a.wscale + n) : 1.0f;
-                    const float *col = a.color + n * 3;
-                    c = make_float4(scale * __ldg(col), scale * __ldg(col + 1), scale * __ldg(col + 2), scale);
-                    odd = !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < INFINITY);
-                }
-            }
-#pragma unroll
-            for (int k = 0; k < 8; ++k) {
-                const int d = at + k;
-                const float t = (float)d - frac;
-                w[k] = d >= lo && d <= hi ? expf(-(t * t) * inv2s2) : 0.f;
-            }
-            if (!axis) {
-                float4 *o = reinterpret_cast<float4 *>(&sh.lists.wx[p][o0]);
-                o[0] = make_float4(w[0], w[1], w[2], w[3]);
-                o[1] = make_float4(w[4], w[5], w[6], w[7]);
-            } else {
-#pragma unroll
-                for (int k = 0; k < 8; ++k) sh.lists.wy[p][o0 + k] = make_float4(w[k] * c.x, w[k] * c.y, w[k] * c.z, w[k] * c.w);
-            }
+    // What a thread needs to make eight factors of one axis of a particle: loaded a chunk ahead.
+    const int sp = tid >> 2, axis = (tid >> 1) & 1, o0 = (tid & 1) * 8;
+    const bool colours = (tid & 3) == 3;
+    float pos = 0.f;
+    float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
+    auto fetch = [&](int window, int off, int count) {
+        if (off + sp >= count) return;
+        const long long n = (long long)b * a.N + window + sh.lists.n[off + sp];
+        pos = __ldg(a.x + n * 2 + axis);
+        if (colours) {
+            const float *c = a.color + n * 3;
+            col = make_float4(__ldg(c), __ldg(c + 1), __ldg(c + 2), a.normalize ? __ldg(a.wscale + n) : 1.0f);
         }
-        if (__syncthreads_or(odd)) {
-            for (int q = part; q < padded; q += kSplatParts)
+    };
+    // Eight factors into buffer f; whether the particle's colour is finite (zero times one that is not is not zero outside the patch).
+    auto factors = [&](SplatFactors &f, int off, int count) {
+        if (off + sp >= (count + kSplatParts - 1) / kSplatParts * kSplatParts) return false;
+        const bool valid = off + sp < count;
+        float w[8], frac;
+        int at = splat_axis(a, pos, axis, frac);
+        at = (axis ? ty0 : tx0) - at + o0;  // offset of the first of the eight from the particle's pixel
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+            const int d = at + k;
+            const float t = (float)d - frac;
+            w[k] = valid && d >= -r && d <= r ? expf(-(t * t) * inv2s2) : 0.f;
+        }
+        float4 *o = reinterpret_cast<float4 *>(axis ? &f.wy[sp][o0] : &f.wx[sp][o0]);
+        o[0] = make_float4(w[0], w[1], w[2], w[3]);
+        o[1] = make_float4(w[4], w[5], w[6], w[7]);
+        if (!colours) return false;
+        const float4 c = valid ? make_float4(col.w * col.x, col.w * col.y, col.w * col.z, col.w) : make_float4(0.f, 0.f, 0.f, 0.f);
+        f.c[sp] = c;
+        return !(fabsf(c.x) + fabsf(c.y) + fabsf(c.z) < INFINITY);
+    };
+    auto multiply = [&](const SplatFactors &f, int padded, bool odd) {
+#pragma unroll 1
+        for (int q = part; q < padded; q += kSplatParts) {
+            const float4 x0 = *reinterpret_cast<const float4 *>(&f.wx[q][px]), x1 = *reinterpret_cast<const float4 *>(&f.wx[q][px + 4]);
+            const float2 wy = *reinterpret_cast<const float2 *>(&f.wy[q][py]);
+            const float4 c = f.c[q];
+            const float cs[4] = {c.x, c.y, c.z, c.w};
+            if (odd) {
+                const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
 #pragma unroll
                 for (int y = 0; y < 2; ++y) {
-                    const float4 w = sh.lists.wy[q][py + y];
+                    const float w = y ? wy.y : wy.x;
 #pragma unroll
-                    for (int x = 0; x < 8; ++x) {
-                        const float xs = sh.lists.wx[q][px + x];
-                        if (xs == 0.f || w.w == 0.f) continue;
-                        acc[y][x][0] = fma2(pack2(xs, xs), pack2(w.x, w.y), acc[y][x][0]);
-                        acc[y][x][1] = fma2(pack2(xs, xs), pack2(w.z, w.w), acc[y][x][1]);
-                    }
+                    for (int k = 0; k < 4; ++k)
+#pragma unroll
+                        for (int x = 0; x < 4; ++x) {
+                            float lo, hi;
+                            unpack2(acc[y][k][x], lo, hi);
+                            if (w != 0.f && xs[2 * x] != 0.f) lo = fmaf(xs[2 * x], w * cs[k], lo);
+                            if (w != 0.f && xs[2 * x + 1] != 0.f) hi = fmaf(xs[2 * x + 1], w * cs[k], hi);
+                            acc[y][k][x] = pack2(lo, hi);
+                        }
                 }
-            __syncthreads();
-            return;
-        }
-        for (int q = part; q < padded; q += kSplatParts) {
-            const float4 x0 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px]), x1 = *reinterpret_cast<const float4 *>(&sh.lists.wx[q][px + 4]);
-            const float xs[8] = {x0.x, x0.y, x0.z, x0.w, x1.x, x1.y, x1.z, x1.w};
+                continue;
+            }
+            const unsigned long long xx[4] = {pack2(x0.x, x0.y), pack2(x0.z, x0.w), pack2(x1.x, x1.y), pack2(x1.z, x1.w)};
 #pragma unroll
             for (int y = 0; y < 2; ++y) {
-                const float4 w = sh.lists.wy[q][py + y];
-                const unsigned long long rg = pack2(w.x, w.y), bd = pack2(w.z, w.w);
+                const float w = y ? wy.y : wy.x;
 #pragma unroll
-                for (int x = 0; x < 8; ++x) {
-                    const unsigned long long xx = pack2(xs[x], xs[x]);
-                    acc[y][x][0] = fma2(xx, rg, acc[y][x][0]);
-                    acc[y][x][1] = fma2(xx, bd, acc[y][x][1]);
+                for (int k = 0; k < 4; ++k) {
+                    const float v = w * cs[k];
+                    const unsigned long long vv = pack2(v, v);
+#pragma unroll
+                    for (int x = 0; x < 4; ++x) acc[y][k][x] = fma2(xx[x], vv, acc[y][k][x]);
                 }
             }
         }
-        __syncthreads();
     };
 
     const float top = (float)(a.img - 1), per = top / a.span, reach = (float)r + 9.25f;  // patch radius, half a tile, a pixel, rounding
     const float mx = (float)tx0 + 7.5f, my = (float)ty0 + 7.5f;
-    int pending = 0;
-    for (int n0 = 0; n0 < a.N; n0 += kSplatThreads * kSplatCull) {
-        unsigned ballots[kSplatCull];
-#pragma unroll
+    const int share = (a.N + slices - 1) / slices, end = min(a.N, (slice + 1) * share);
+    for (int n0 = slice * share; n0 < end; n0 += kSplatWindow) {
+        unsigned hits = 0;
+#pragma unroll 8
         for (int q = 0; q < kSplatCull; ++q) {
             const int n = n0 + q * kSplatThreads + tid;
-            bool hit = false;
-            if (n < a.N) {
+            if (n < end) {
                 const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + (long long)b * a.N + n);
                 const float x = (v.x - a.lo) * per;
                 float y = (v.y - a.lo) * per;
                 if (a.y_up) y = top - y;
-                hit = fabsf(x - mx) <= reach && fabsf(y - my) <= reach;
+                if (fabsf(x - mx) <= reach && fabsf(y - my) <= reach) hits |= 1u << q;
             }
-            ballots[q] = __ballot_sync(0xffffffffu, hit);
-            if (lane == 0) s_count[q * kSplatWarps + warp] = __popc(ballots[q]);
         }
-        __syncthreads();
-        int incl = s_count[lane];  // kSplatCull * kSplatWarps == 32 counts in list order
+        int incl = __popc(hits);
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int v = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += v;
         }
-        const int total = pending + __shfl_sync(0xffffffffu, incl, 31);
+        if (lane == 31) s_count[warp] = incl;
+        __syncthreads();  // (also: the window before has read its list and factors)
+        int at = incl - __popc(hits), count = 0;
 #pragma unroll
-        for (int q = 0; q < kSplatCull; ++q) {
-            const int before = q * kSplatWarps + warp - 1;
-            const int base = __shfl_sync(0xffffffffu, incl, before & 31);
-            if ((ballots[q] >> lane) & 1u)
-                sh.lists.n[pending + (before < 0 ? 0 : base) + __popc(ballots[q] & ((1u << lane) - 1u))] = n0 + q * kSplatThreads + tid;
+        for (int w = 0; w < kSplatWarps; ++w) {
+            const int c = s_count[w];
+            if (w < warp) at += c;
+            count += c;
         }
+        for (; hits; hits &= hits - 1) sh.lists.n[at++] = (unsigned short)((__ffs(hits) - 1) * kSplatThreads + tid);
         __syncthreads();
-        pending = total;
-        int done = 0;
-        for (; pending - done >= kSplatChunk; done += kSplatChunk) multiply(done, kSplatChunk);
-        // the rest of the list moves to its front
-        const int keep = tid < pending - done ? sh.lists.n[done + tid] : 0;
-        __syncthreads();
-        if (tid < pending - done) sh.lists.n[tid] = keep;
-        __syncthreads();
-        pending -= done;
+        fetch(n0, 0, count);
+        for (int off = 0, buf = 0; off < count; off += kSplatChunk, buf ^= 1) {
+            const bool odd = factors(sh.lists.f[buf], off, count);
+            fetch(n0, off + kSplatChunk, count);
+            const bool any_odd = __syncthreads_or(odd);  // (also: the chunk before the last has left its buffer)
+            multiply(sh.lists.f[buf], min(kSplatChunk, (count - off + kSplatParts - 1) / kSplatParts * kSplatParts), any_odd);
+        }
     }
-    if (pending > 0) multiply(0, pending);
     __syncthreads();
     // the two halves of a warp meet by shuffles, the eight warps in shared memory
 #pragma unroll
     for (int y = 0; y < 2; ++y)
 #pragma unroll
-        for (int x = 0; x < 8; ++x) {
-            float4 v;
-            unpack2(acc[y][x][0], v.x, v.y);
-            unpack2(acc[y][x][1], v.z, v.w);
-            v.x += __shfl_xor_sync(0xffffffffu, v.x, 16);
-            v.y += __shfl_xor_sync(0xffffffffu, v.y, 16);
-            v.z += __shfl_xor_sync(0xffffffffu, v.z, 16);
-            v.w += __shfl_xor_sync(0xffffffffu, v.w, 16);
-            if (lane < 16) sh.part[warp][part_at((py + y) * kSplatTile + px + x)] = v;
+        for (int x = 0; x < 4; ++x) {
+            float v[2][4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {
+                unpack2(acc[y][k][x], v[0][k], v[1][k]);
+                v[0][k] += __shfl_xor_sync(0xffffffffu, v[0][k], 16);
+                v[1][k] += __shfl_xor_sync(0xffffffffu, v[1][k], 16);
+            }
+            // each half stores one of the two pixels
+            const int h = lane >> 4;
+            sh.part[warp][part_at((py + y) * kSplatTile + px + 2 * x + h)] =
+                make_float4(h ? v[1][0] : v[0][0], h ? v[1][1] : v[0][1], h ? v[1][2] : v[0][2], h ? v[1][3] : v[0][3]);
         }
     __syncthreads();
-    const int ox = tx0 + (tid % kSplatTile), oy = ty0 + (tid / kSplatTile);
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
     for (int w = 0; w < kSplatWarps; ++w) {
         const float4 q = sh.part[w][part_at(tid)];
         v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
     }
+    int pixel = tid;
+    if (SLICED) {
+        // every CTA of the cluster adds up its share of the pixels, over the slices in order
+        cg::cluster_group cluster = cg::this_cluster();
+        sh.part[0][part_at(tid)] = v;  // (only this thread reads this place of the first warp's image)
+        cluster.sync();
+        const int each = kSplatTile * kSplatTile / slices;
+        pixel = slice * each + tid;
+        if (tid < each) {
+            v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int k = 0; k < slices; ++k) {
+                const float4 q = cluster.map_shared_rank(&sh.part[0][0], k)[part_at(pixel)];
+                v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
+            }
+        }
+        cluster.sync();
+        if (tid >= each) return;
+    }
+    const int ox = tx0 + (pixel % kSplatTile), oy = ty0 + (pixel / kSplatTile);
     if (ox < a.img && oy < a.img) reinterpret_cast<float4 *>(a.out)[((long long)b * a.img + oy) * a.img + ox] = v;
 }
 
@@ -334,8 +371,10 @@ __device__ inline float warp_sum(float v) {
 // the whole patch axis; t_x = dx - frac_x.  floor() passes no gradient, so dL/dp = dL/dfrac.
 // The weight is separable: a lane keeps one column of the patch, runs down its rows with the row factors from shared
 // memory and applies the column factor once at the end (2 (2r+1) exponentials per particle instead of (2r+1)^2).  The
-// last, narrow group of columns is dealt to the lanes several rows at a time.  Bound by the reads of the upstream image
-// (16 bytes per pixel of the patch, from L1 and L2).  8 x 4,096 particles, patches of 41 x 41: 158 -> 75 us.
+// last, narrow group of columns is dealt to the lanes several rows at a time.  Bound by the latency of the reads of the upstream
+// image (16 bytes per pixel of the patch, from L1 and L2) at 32 warps per SM: with a third of the instructions less (packed sums, three
+// columns per lane and two rows at a time) 80-102 us instead of 74, with particles sorted by place (L1 hits 81 %) 83.
+// 8 x 4,096 particles, patches of 41 x 41: 158 -> 74 us.
 __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
     constexpr int kMost = 2 * kSplatMaxRadius + 1;
     __shared__ float2 s_y[8][kMost];  // row factor, row factor times t_y
@@ -413,9 +452,22 @@ __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
 // systems), sparse / product kernel, us: 16 systems, 256 x 256, patch 21: h = 1.3 12.8 / 48, 11 31 / 57, 21 54 / 65; 1 system, 256 x
 // 256, patch 41: h = 13 8.7 / 9.0, 25 11.6 / 9.9, 51 17.3 / 12.7.  The line is at worst 19 % behind the better kernel, 0.7 % on
 // average.
-static bool sparse_tiles(const SplatArgs &a) {
+static double particles_of_a_tile(const SplatArgs &a) {
     const double reach = (2.0 * a.radius + 1.0 + kSplatTile) / a.img, part = reach < 1.0 ? reach * reach : 1.0;
-    return a.N * part < 28.0;
+    return a.N * part;
+}
+static bool sparse_tiles(const SplatArgs &a) { return particles_of_a_tile(a) < 28.0; }
+
+// CTAs that share a tile, each with a slice of the particles: an image of few tiles leaves most of the 148 SMs idle, a second CTA
+// per tile costs the fixed part of one.  By the tiles of an image and the particles of a tile (h above), again not by the batch.
+// Measured over images of 64 to 256 pixels, 64 to 8,192 particles and 1 to 16 systems, us with one / two / four / eight slices: 64
+// pixels, h = 1458, 1 system 76 / 43 / 27 / 19, 4 systems 76 / 45 / 33 / 35; h = 729, 1 system 43 / 27 / 19 / 15, 8 systems 43 / 31 /
+// 32 / 39; h = 364, 16 systems 31 / 32 / 37; 192 pixels, h = 491, 1 system 37 / 27, 4 systems 71 / 71; h = 245, 8 systems 66 / 84; 224
+// pixels, h = 440, 1 system 35 / 33, 4 systems 83 / 85.
+static int splat_slices(const SplatArgs &a, int tiles) {
+    const double h = particles_of_a_tile(a);
+    if (tiles <= 64) return h >= 1400.0 ? 8 : h >= 680.0 ? 4 : h >= 340.0 ? 2 : 1;
+    return tiles <= 144 && h >= 340.0 ? 2 : 1;
 }
 
 static int check_splat(const char *name, const SplatArgs &a) {
@@ -456,7 +508,22 @@ int npa_splat_forward(const float *x, const float *color, int32_t batch, int32_t
         splat_forward_sparse_kernel<<<dim3(tiles * tiles, batch), kSplatTile * kSplatTile, 0, st>>>(a);
         return check_launch("splat_forward_sparse_kernel");
     }
-    splat_forward_kernel<<<dim3(tiles * tiles, batch), kSplatThreads, 0, st>>>(a);
+    const int slices = splat_slices(a, tiles * tiles);
+    if (slices == 1) {
+        splat_forward_kernel<false><<<dim3(tiles * tiles, batch), kSplatThreads, 0, st>>>(a);
+        return check_launch("splat_forward_kernel");
+    }
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(slices * tiles * tiles, batch);
+    cfg.blockDim = dim3(kSplatThreads);
+    cfg.stream = st;
+    cudaLaunchAttribute cluster;
+    cluster.id = cudaLaunchAttributeClusterDimension;
+    cluster.val.clusterDim.x = slices;
+    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
+    cfg.attrs = &cluster;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, splat_forward_kernel<true>, a);
     return check_launch("splat_forward_kernel");
 }
 

@@ -145,3 +145,22 @@ def test_forward_on_either_side_of_the_kernel_choice(img, sigma):
         out = splatting.splat_particles_batch(x.cuda(), c.cuda(), img_size=img, sigma=sigma)
         _close(out[2], splat_oracle.splat_forward(x[2].numpy(), c[2].numpy(), img_size=img, sigma=sigma), f"{n} particles")
         assert torch.equal(splatting.splat_particles(x[2].cuda(), c[2].cuda(), img_size=img, sigma=sigma), out[2])
+
+
+@pytest.mark.parametrize("img,n", [(64, 1900), (64, 1950), (70, 4100), (64, 8200), (150, 5000), (160, 9001)])
+def test_tiles_shared_by_a_cluster(img, n):
+    """One, two, four and eight slices of the particles per tile (the last size: three windows of the list, two slices), particles
+    outside the image and a colour that is not finite: the fp64 oracle's image, and the same bits alone and in a batch."""
+    from npa_b200 import splatting
+    from oracle import splat as splat_oracle
+    g = torch.Generator().manual_seed(n)
+    x, c = (torch.rand(2, n, 2, generator=g) - 0.5) * 2.2, torch.rand(2, n, 3, generator=g)
+    out = splatting.splat_particles_batch(x.cuda(), c.cuda(), img_size=img)
+    _close(out[1], splat_oracle.splat_forward(x[1].numpy(), c[1].numpy(), img_size=img), f"{n} particles")
+    assert torch.equal(splatting.splat_particles(x[1].cuda(), c[1].cuda(), img_size=img), out[1])
+    x[1, n - 1], c[1, n - 1, 0] = 0.0, float("inf")
+    bad = ~torch.isfinite(splatting.splat_particles(x[1].cuda(), c[1].cuda(), img_size=img)).cpu()
+    r, mid = splatting._derived(img, 2.0, -1.0, 1.0, True, 2.0 / 128.0)[1], (img - 1) // 2
+    patch = torch.zeros(img, img, dtype=torch.bool)
+    patch[mid - r: mid + r + 1, mid - r: mid + r + 1] = True
+    assert torch.equal(bad[..., 0], patch) and not bool(bad[..., 1:].any())
