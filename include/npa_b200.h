@@ -465,6 +465,13 @@ int npa_splat_backward(const float *x, const float *color, const float *g_out, i
                        int32_t img_size, double sigma_pixels, int32_t radius, double lo, double hi, int32_t y_up,
                        int32_t normalize, double norm_scale, float *g_x, float *g_color, void *stream);
 
+/* ---- move between the steps of a rollout ------------------------------------------ *
+ * x_out = wrap(x + dt amp^T sin(k^T x + phase)) for positions x [B,N,P]; k [dim, modes], phase [modes],
+ * amp [modes, dim], 1 <= modes <= 64.  Periodic grids wrap into the box (HashGrid.wrap_positions,
+ * sphops/sph.py:107-123).  The padding column of x_out is not written; x_out may be x. */
+int npa_rollout_move(const npa_grid *grid, const float *x, const float *k, const float *phase, const float *amp,
+                     int32_t modes, float dt, float *x_out, void *stream);
+
 /* ---- weight gradients of the per-particle MLP ------------------------------------ *
  * The adaptation MLP of an NPA model (models/npa.py:63-75) is Linear(in, 128) -> ReLU ->
  * Linear(128, out, bias = False), applied to every particle.  One pass over the rows gives

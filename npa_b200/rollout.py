@@ -17,6 +17,7 @@ import math
 
 import torch
 
+from . import _native as N
 from . import sphops as sph
 
 
@@ -37,6 +38,12 @@ class VelocityField:
     def __call__(self, x: torch.Tensor) -> torch.Tensor:
         arg = x[..., : self.dim] @ self.k_t + self.phase
         return torch.sin(arg) @ self.amp
+
+
+def _written(t):
+    """Autograd's note of a change in place, as a torch operation would leave it."""
+    if not t.is_inference():
+        torch.autograd.graph.increment_version(t)
 
 
 class PerceptionRollout:
@@ -76,38 +83,57 @@ class PerceptionRollout:
         if grid.boundary == "periodic":
             self.box = torch.tensor([g * grid.eps for g in grid.grid_size[:D]], **f32)
             self.half_box = 0.5 * self.box
-        # kernels of this library per rollout: 6 grid build + reorder + 2 sweeps per step, and for the last step the
-        # layout of the upstream, 2 backward sweeps and the inverse reorder
-        self.launches = self.steps * 9 + 4
+        # kernels of this library per rollout: 6 grid build + reorder + 2 sweeps per step, a move between steps, and for the
+        # last step the layout of the upstream, 2 backward sweeps and the inverse reorder
+        self.launches = self.steps * 9 + 4 + (self.steps - 1 if self._native_move() else 0)
 
-    def _forward(self, x, s, last):
+    def _native_move(self):
+        v = self.velocity
+        return (type(v) is VelocityField and v.dim == self.grid.dim and 1 <= v.phase.numel() <= 64
+                and all(t.dtype == torch.float32 and t.is_contiguous() and t.device == self.x_bin.device for t in (v.k_t, v.phase, v.amp)))
+
+    def _forward(self, x, s, s_bin):
         hg = self.hg
         hg.initialize(x, self.perm, self.offs, self.info)
-        hg.bin_particles(x, s, None, self.perm, self.x_bin, self.s_bin, None)
+        hg.bin_particles(x, s, None, self.perm, self.x_bin, s_bin, None)
         # the density sweep records the neighbour lists in every step: writing them costs 15 % of that sweep, and
         # the blur + gradient sweep that reads them takes less than half the time of one that searches the cells
         # itself (cfg5's shape, 3D periodic: 1.05 + 1.09 ms against 0.91 + 2.42 ms per million particles)
         hg.perception_forward(self.x_bin, None, None, self.rho, None, None, None, None, None, self.offs, self.info,
                               pair_cache=self.pairs)
-        hg.blur_gradient_forward(self.x_bin, self.rho, None, self.s_bin, self.blur, self.grad, self.offs, self.info,
+        hg.blur_gradient_forward(self.x_bin, self.rho, None, s_bin, self.blur, self.grad, self.offs, self.info,
                                  pair_cache=self.pairs, pair_cache_valid=True)
 
-    def _move(self, x, s):
-        """x <- wrap(x_bin + dt * v(x_bin)), s <- s_bin: the particles continue in cell order."""
-        D = self.grid.dim
-        xn = self.x_bin[..., :D] + self.dt * self.velocity(self.x_bin)
+    def _move(self, x):
+        """x <- wrap(x_bin + dt * v(x_bin)): the particles continue in cell order."""
+        D, v = self.grid.dim, self.velocity
+        if self._native_move() and not x.requires_grad:
+            self.hg._call(N.lib.npa_rollout_move, x, self.hg._ref(), N.ptr(self.x_bin), N.ptr(v.k_t), N.ptr(v.phase), N.ptr(v.amp),
+                          v.phase.numel(), self.dt, N.ptr(x))
+            _written(x)
+            return
+        xn = self.x_bin[..., :D] + self.dt * v(self.x_bin)
         if self.half_box is not None:
             xn = torch.remainder(xn + self.half_box, self.box) - self.half_box
         x[..., :D] = xn
-        s.copy_(self.s_bin)
 
     def run(self, x, s, upstream):
         """One rollout; returns ``(grad_x, grad_s)`` with respect to the inputs of the final step."""
+        # the states are reordered from s into s_bin and from s_bin back into s in turn; the last step reads s and writes
+        # s_bin, so that with an even number of steps one copy remains
+        source, target = s, self.s_bin
         for k in range(self.steps):
             last = k == self.steps - 1
-            self._forward(x, s, last)
-            if not last:
-                self._move(x, s)
+            self._forward(x, source, target)
+            if target is s:
+                _written(s)
+            if last:
+                break
+            self._move(x)
+            if s.requires_grad or s.data_ptr() == self.s_bin.data_ptr() or (k == 0 and self.steps % 2 == 0):
+                s.copy_(self.s_bin)
+            else:
+                source, target = target, source
         hg = self.hg
         hg.blur_gradient_backward(self.x_bin, self.rho, None, self.s_bin, upstream["g_blur"], upstream["g_grad"],
                                   self.grad_x, self.grad_s, self.grad_rho, self.offs, self.info, pair_cache=self.pairs)

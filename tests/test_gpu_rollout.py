@@ -52,3 +52,33 @@ def test_rollout_matches_the_public_api_loop(w):
     torch.autograd.backward([r, bl, gr], [ups["g_rho"], ups["g_blur"], ups["g_grad"]])
     assert torch.equal(gx, xr.grad), "gradient with respect to the positions of the last step differs"
     assert torch.equal(gs, sr.grad)
+
+
+@pytest.mark.parametrize("steps", [1, 2, 3])
+@pytest.mark.parametrize("dim,N,boundary,modes", [(3, 20011, "periodic", 8), (2, 1001, "periodic", 64), (3, 515, "clamped", 8)])
+def test_the_native_move_gives_the_bits_of_the_tensor_operations(dim, N, boundary, modes, steps):
+    """A rollout whose velocity field is not the built-in type moves by tensor operations and copies the states: the same positions
+    (bit for bit, or particles would change cells), states, outputs and gradients, with an odd and an even number of steps."""
+    from npa_b200 import sphops as sph
+    from npa_b200.rollout import PerceptionRollout, VelocityField
+
+    class Another(VelocityField):
+        pass
+
+    cells = 8
+    grid = sph.HashGrid(dim=dim, boundary=boundary, mode="grid", grid_size=(cells,) * dim, eps=0.125, num_particles=N, batch_size=2)
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x0 = torch.rand(2, N, 2 if dim == 2 else 4, generator=g, device="cuda") - 0.5
+    s0 = torch.randn(2, N, 8, generator=g, device="cuda")
+    ups = {"g_rho": torch.randn(2, N, generator=g, device="cuda"), "g_blur": torch.randn(2, N, 8, generator=g, device="cuda"),
+           "g_grad": torch.randn(2, N, 8, dim, generator=g, device="cuda")}
+    got = []
+    for field in (VelocityField, Another):
+        roll = PerceptionRollout(grid, 8, steps, 0.3, field(dim, x0.device, seed=1, modes=modes))
+        x, s = x0.clone(), s0.clone()
+        versions = x._version, s._version
+        grads = roll.run(x, s, ups)
+        assert steps == 1 or (x._version > versions[0] and s._version > versions[1])
+        got.append([t.clone() for t in (x, s, roll.x_bin, roll.s_bin, roll.rho, roll.blur, roll.grad, *grads)])
+    for a, b in zip(*got):
+        assert torch.equal(a, b)
