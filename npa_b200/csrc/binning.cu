@@ -113,6 +113,7 @@ template <int D, bool SMEM>
 __global__ void __launch_bounds__(kBinThreads)
 hash_count_kernel(const float *__restrict__ x, uint32_t *__restrict__ cellid, uint32_t *__restrict__ arrive,
                   uint32_t *__restrict__ counts, Geom g) {
+    after_previous_kernel();
     extern __shared__ uint32_t hist[];
     const int b = blockIdx.y;
     const int base = blockIdx.x * kBinChunk;
@@ -194,6 +195,7 @@ __device__ inline unsigned long long block_exclusive(unsigned long long v, unsig
 __global__ void __launch_bounds__(kScanThreads)
 scan_tile_sums_kernel(const uint32_t *__restrict__ counts, unsigned long long *__restrict__ partials,
                       int n, int mpb) {
+    after_previous_kernel();
     __shared__ unsigned long long tot;
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanPerThread;
     unsigned long long v = 0;
@@ -207,6 +209,7 @@ scan_tile_sums_kernel(const uint32_t *__restrict__ counts, unsigned long long *_
 
 __global__ void __launch_bounds__(1024)
 scan_partials_kernel(unsigned long long *partials, int tiles) {
+    after_previous_kernel();
     __shared__ unsigned long long tot;
     __shared__ unsigned long long carry_s;
     if (threadIdx.x == 0) carry_s = 0;
@@ -230,6 +233,7 @@ __global__ void __launch_bounds__(kScanThreads)
 scan_apply_kernel(const uint32_t *__restrict__ counts, const unsigned long long *__restrict__ partials,
                   int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, uint32_t *__restrict__ crowded,
                   uint32_t *__restrict__ crowded_count, int n, Geom g) {
+    after_previous_kernel();
     __shared__ unsigned long long tot;
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanPerThread;
     uint32_t c[kScanPerThread];
@@ -269,6 +273,7 @@ scan_apply_kernel(const uint32_t *__restrict__ counts, const unsigned long long 
 __global__ void __launch_bounds__(kBinThreads)
 scatter_kernel(const uint32_t *__restrict__ cellid, const uint32_t *__restrict__ arrive,
                const int32_t *__restrict__ bin_offsets, uint32_t *__restrict__ order, Geom g) {
+    after_previous_kernel();
     const int b = blockIdx.y;
     const int i = blockIdx.x * kBinThreads + threadIdx.x;
     if (i >= g.N) return;
@@ -345,6 +350,7 @@ __global__ void __launch_bounds__(kBinThreads)
 rank_kernel(const uint32_t *__restrict__ cellid, const int32_t *__restrict__ bin_offsets, const uint32_t *__restrict__ order,
             int32_t *__restrict__ permutation, const uint32_t *__restrict__ crowded, const uint32_t *__restrict__ crowded_count, Geom g,
             int rank_columns) {
+    after_previous_kernel();
     if ((int)blockIdx.x >= rank_columns) {
         if (blockIdx.y == 0)
             rank_crowded(bin_offsets, order, permutation, crowded, crowded_count, g, blockIdx.x - rank_columns, gridDim.x - rank_columns);
@@ -429,6 +435,7 @@ template <int D>
 __global__ void __launch_bounds__(kSmallThreads)
 bin_small_kernel(const float *__restrict__ x, int32_t *__restrict__ permutation, int32_t *__restrict__ bin_offsets,
                  int4 *__restrict__ block_info, uint32_t *__restrict__ rows_of_system, Geom g) {
+    after_previous_kernel();
     extern __shared__ uint32_t small_mem[];
     __shared__ uint32_t crowded_n, s_crowded[kSmallParticles / kCrowdedCell];
     uint32_t *table = small_mem;                                     // per cell: count, then next free slot, then end
@@ -496,6 +503,7 @@ bin_small_kernel(const float *__restrict__ x, int32_t *__restrict__ permutation,
 // Work list of several small systems: the rows of a system start behind those of the systems before it.
 __global__ void __launch_bounds__(kSmallThreads)
 rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, const uint32_t *__restrict__ rows_of_system, Geom g) {
+    after_previous_kernel();
     __shared__ unsigned long long before_s;
     const int b = blockIdx.x, tid = threadIdx.x;
     unsigned long long before = 0, all = 0;  // rows of the systems before this one, rows in all
@@ -524,6 +532,7 @@ __global__ void __launch_bounds__(256)
 permute_kernel(const float *__restrict__ x, const float *__restrict__ s, const float *__restrict__ m,
                const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
                float *__restrict__ mo, int pieces, long long total, int N) {
+    after_previous_kernel();
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     if (t >= total) return;
     const long long particle = t / pieces;
@@ -562,7 +571,7 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     const long long total = (long long)g.B * g.N * pieces;
     const unsigned blocks = (unsigned)((total + 255) / 256);
 #define NPA_PERMUTE(DD, VEC) \
-    permute_kernel<DD, FORWARD, VEC><<<blocks, 256, 0, st>>>(x, s, m, perm, xo, so, mo, pieces, total, g.N)
+    launch_early(permute_kernel<DD, FORWARD, VEC>, blocks, 256, 0, st, x, s, m, perm, xo, so, mo, pieces, total, g.N)
     if (g.dim == 2) {
         if (vec) NPA_PERMUTE(2, float4); else NPA_PERMUTE(2, float);
     } else {
@@ -619,6 +628,7 @@ template <int D>
 __global__ void __launch_bounds__(256)
 corrected_gradient_kernel(const float *__restrict__ raw, const float *__restrict__ moment, float *__restrict__ out, long long total, int C,
                           float tol) {
+    after_previous_kernel();
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     if (t >= total) return;
     const float *mp = moment + (t / C) * (D * D);
@@ -672,13 +682,13 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
         int unused = 0;
         if (g.dim == 2) {
             if ((rc = persistent_ctas(bin_small_kernel<2>, kSmallThreads, bytes, &unused)) != NPA_OK) return rc;  // shared-memory limit
-            bin_small_kernel<2><<<g.B, kSmallThreads, bytes, st>>>(x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+            launch_early(bin_small_kernel<2>, g.B, kSmallThreads, bytes, st, x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         } else {
             if ((rc = persistent_ctas(bin_small_kernel<3>, kSmallThreads, bytes, &unused)) != NPA_OK) return rc;
-            bin_small_kernel<3><<<g.B, kSmallThreads, bytes, st>>>(x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+            launch_early(bin_small_kernel<3>, g.B, kSmallThreads, bytes, st, x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         }
         if ((rc = check_launch("bin_small_kernel")) != NPA_OK || g.B == 1) return rc;
-        rows_small_kernel<<<g.B, kSmallThreads, 0, st>>>(bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         return check_launch("rows_small_kernel");
     }
     cudaError_t e = cudaMemsetAsync(s.counts, 0, s.zero_bytes, st);
@@ -688,30 +698,30 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     const bool smem = g.cells <= kSmemHistCells;
     const size_t smem_bytes = smem ? (size_t)g.cells * 4 : 0;
     if (g.dim == 2) {
-        if (smem) hash_count_kernel<2, true><<<pgrid, kBinThreads, smem_bytes, st>>>(x, s.cellid, s.arrive, s.counts, g);
-        else hash_count_kernel<2, false><<<pgrid, kBinThreads, 0, st>>>(x, s.cellid, s.arrive, s.counts, g);
+        if (smem) launch_early(hash_count_kernel<2, true>, pgrid, kBinThreads, smem_bytes, st, x, s.cellid, s.arrive, s.counts, g);
+        else launch_early(hash_count_kernel<2, false>, pgrid, kBinThreads, 0, st, x, s.cellid, s.arrive, s.counts, g);
     } else {
-        if (smem) hash_count_kernel<3, true><<<pgrid, kBinThreads, smem_bytes, st>>>(x, s.cellid, s.arrive, s.counts, g);
-        else hash_count_kernel<3, false><<<pgrid, kBinThreads, 0, st>>>(x, s.cellid, s.arrive, s.counts, g);
+        if (smem) launch_early(hash_count_kernel<3, true>, pgrid, kBinThreads, smem_bytes, st, x, s.cellid, s.arrive, s.counts, g);
+        else launch_early(hash_count_kernel<3, false>, pgrid, kBinThreads, 0, st, x, s.cellid, s.arrive, s.counts, g);
     }
     if ((rc = check_launch("hash_count_kernel")) != NPA_OK) return rc;
 
     const int n = g.B * g.cells;
-    scan_tile_sums_kernel<<<s.tiles, kScanThreads, 0, st>>>(s.counts, s.partials, n, g.mpb);
+    launch_early(scan_tile_sums_kernel, s.tiles, kScanThreads, 0, st, s.counts, s.partials, n, g.mpb);
     if ((rc = check_launch("scan_tile_sums_kernel")) != NPA_OK) return rc;
-    scan_partials_kernel<<<1, 1024, 0, st>>>(s.partials, s.tiles);
+    launch_early(scan_partials_kernel, 1, 1024, 0, st, s.partials, s.tiles);
     if ((rc = check_launch("scan_partials_kernel")) != NPA_OK) return rc;
     uint32_t *crowded_count = s.counts + (size_t)n + 1;
-    scan_apply_kernel<<<s.tiles, kScanThreads, 0, st>>>(s.counts, s.partials, bin_offsets,
+    launch_early(scan_apply_kernel, s.tiles, kScanThreads, 0, st, s.counts, s.partials, bin_offsets,
                                                         reinterpret_cast<int4 *>(block_info), s.crowded, crowded_count, n, g);
     if ((rc = check_launch("scan_apply_kernel")) != NPA_OK) return rc;
 
     const dim3 tgrid((g.N + kBinThreads - 1) / kBinThreads, g.B);
-    scatter_kernel<<<tgrid, kBinThreads, 0, st>>>(s.cellid, s.arrive, bin_offsets, s.order, g);
+    launch_early(scatter_kernel, tgrid, kBinThreads, 0, st, s.cellid, s.arrive, bin_offsets, s.order, g);
     if ((rc = check_launch("scatter_kernel")) != NPA_OK) return rc;
     const int win = g.N < kRankWindow ? g.N : kRankWindow;
     const dim3 rgrid(tgrid.x + kRankCtas, g.B);
-    rank_kernel<<<rgrid, kBinThreads, (size_t)((win + 31) / 32) * 8, st>>>(s.cellid, bin_offsets, s.order, permutation, s.crowded, crowded_count, g,
+    launch_early(rank_kernel, rgrid, kBinThreads, (size_t)((win + 31) / 32) * 8, st, s.cellid, bin_offsets, s.order, permutation, s.crowded, crowded_count, g,
                                                                          (int)tgrid.x);
     return check_launch("rank_kernel");
 }
@@ -804,8 +814,8 @@ int npa_corrected_gradient(int32_t dim, int64_t n, int32_t channels, const float
     if (n == 0) return NPA_OK;
     const long long total = (long long)n * channels;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (dim == 2) corrected_gradient_kernel<2><<<blocks, 256, 0, (cudaStream_t)stream>>>(raw, moment, out, total, channels, tol);
-    else corrected_gradient_kernel<3><<<blocks, 256, 0, (cudaStream_t)stream>>>(raw, moment, out, total, channels, tol);
+    if (dim == 2) launch_early(corrected_gradient_kernel<2>, blocks, 256, 0, (cudaStream_t)stream, raw, moment, out, total, channels, tol);
+    else launch_early(corrected_gradient_kernel<3>, blocks, 256, 0, (cudaStream_t)stream, raw, moment, out, total, channels, tol);
     return check_launch("corrected_gradient_kernel");
 }
 

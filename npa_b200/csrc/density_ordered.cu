@@ -22,6 +22,7 @@ constexpr int kTicketRows = 8; // most work-list rows a warp draws per ticket
 template <int D, bool PER>
 __global__ void __launch_bounds__(kWarpsPerCta * 32)
 density_ordered_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g, int batch) {
+    after_previous_kernel();
     __shared__ int4 s_ranges[kWarpsPerCta][kMaxRanges];
     __shared__ float4 s_cand[kWarpsPerCta][2][32];  // x, y, z, mass of the staged candidates (two batches)
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -182,7 +183,7 @@ static int launch_ordered(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st
     const int needed = (g.max_blocks + batch * kWarpsPerCta - 1) / (batch * kWarpsPerCta);
     ScalarFwdArgs b = a;
     if ((rc = acquire_row_tickets(st, &b.tickets)) != NPA_OK) return rc;
-    density_ordered_kernel<D, PER><<<needed < ctas ? needed : ctas, kWarpsPerCta * 32, 0, st>>>(b, g, batch);
+    launch_early(density_ordered_kernel<D, PER>, needed < ctas ? needed : ctas, kWarpsPerCta * 32, 0, st, b, g, batch);
     return check_launch("density_ordered_kernel");
 }
 
@@ -213,6 +214,7 @@ struct ItemMem {
 template <int D, bool PER, int CLS>
 __global__ void __launch_bounds__(kItemWarps * 32, 4)
 density_ordered_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g, int split) {
+    after_previous_kernel();
     extern __shared__ __align__(16) unsigned char s_item[];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, K = a.pair_stride;
     ItemMem &S = reinterpret_cast<ItemMem *>(s_item)[warp];
@@ -425,7 +427,7 @@ static int launch_item(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     if (split > 16) split = 16;
     if (split < 1) split = 1;
     const long long needed = ((long long)g.max_blocks * split + kItemWarps - 1) / kItemWarps;
-    kernel<<<(unsigned)(needed < ctas ? needed : ctas), kItemWarps * 32, dyn, st>>>(a, g, (int)split);
+    launch_early(kernel, (unsigned)(needed < ctas ? needed : ctas), kItemWarps * 32, dyn, st, a, g, (int)split);
     return check_launch("density_ordered_item_kernel");
 }
 

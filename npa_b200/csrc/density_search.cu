@@ -81,6 +81,7 @@ template <bool MASS> struct TileStage {
 template <int D, bool PER, bool COUNT, bool MASS>
 __global__ void __launch_bounds__(kTileWarps * 32, 12)
 density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g) {
+    after_previous_kernel();
     constexpr int PT = 32 / kShare;
     extern __shared__ __align__(16) unsigned char s_tile[];
     __shared__ int4 s_rng[kTileWarps][kMaxRanges];
@@ -358,7 +359,7 @@ static int launch_tile(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     const int rc = persistent_ctas(kernel, kTileWarps * 32, dyn, &unused);  // raises the shared-memory limit once
     if (rc != NPA_OK) return rc;
     const long long per_cta = (long long)kTileWarps * (32 / kShare), particles = (long long)g.B * g.N;
-    kernel<<<(unsigned)((particles + per_cta - 1) / per_cta), kTileWarps * 32, dyn, st>>>(a, g);
+    launch_early(kernel, (unsigned)((particles + per_cta - 1) / per_cta), kTileWarps * 32, dyn, st, a, g);
     return check_launch("density_tile_kernel");
 }
 
@@ -368,6 +369,7 @@ static int launch_tile(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
 template <int D, bool PER>
 __global__ void __launch_bounds__(kSearchWarps * 32, 8)
 density_item_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_constant__ Geom g, int split) {
+    after_previous_kernel();
     extern __shared__ float4 s_mem[];  // per warp: candidates (x, y, z, index), then their masses when there are any
     __shared__ int4 s_rng[kSearchWarps][32];
     __shared__ int s_run[kSearchWarps][4][kSearchRun];
@@ -603,7 +605,7 @@ static int launch_item(const Geom &g, const ScalarFwdArgs &a, cudaStream_t st) {
     if (split > 16) split = 16;
     if (split < 1) split = 1;
     const long long needed = ((long long)g.max_blocks * split + kSearchWarps - 1) / kSearchWarps;
-    kernel<<<(unsigned)(needed < ctas ? needed : ctas), kSearchWarps * 32, dyn, st>>>(a, g, (int)split);
+    launch_early(kernel, (unsigned)(needed < ctas ? needed : ctas), kSearchWarps * 32, dyn, st, a, g, (int)split);
     return check_launch("density_item_kernel");
 }
 

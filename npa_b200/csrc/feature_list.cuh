@@ -437,6 +437,7 @@ __device__ __noinline__ void list_forward_search(const FeatureFwdArgs &a, const 
 template <int D, bool PER, int LPP, bool VEC, int MASK>
 __global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 4)
 feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
+    after_previous_kernel();
     using S = ListShape<LPP>;
     __shared__ float4 s_k[kListWarps][2][S::kSlots];  // v_j (K.x, K.y, K.z, W)
     __shared__ int4 s_j[kListWarps][2][S::kIndexQuads];
@@ -782,6 +783,7 @@ __device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, c
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
 __global__ void __launch_bounds__(kListBackwardWarps<D, FULL> * 32, FULL ? (D == 3 ? 7 : 4) : LPP == 4 ? 4 : 3)
 feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
+    after_previous_kernel();
     using S = ListShape<LPP>;
     constexpr int WARPS = kListBackwardWarps<D, FULL>;
     __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z W

@@ -73,6 +73,7 @@ struct GradArgs {
 unsigned *umma_status_word();  // mlp_tcgen05.cu: device address of the status word on the current device
 
 __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __grid_constant__ GradArgs args) {
+    after_previous_kernel();
     const float *__restrict__ Z = args.z;
     const float *__restrict__ DH = args.dh;
     const float *__restrict__ H = args.h;
@@ -342,6 +343,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
 // in order by a thread of its own (one thread for all 148 took 11 us, one round trip for eight of them after another).
 constexpr int kReduceOuts = 64, kReduceRuns = 8;
 __global__ void __launch_bounds__(kReduceOuts * kReduceRuns) mlp_grad_umma_reduce_kernel(GradArgs a) {
+    after_previous_kernel();
     __shared__ float s_sum[kReduceRuns][kReduceOuts];
     const int K1 = a.in_dim, O = a.out_dim, Wp = a.N1p + a.N2p;
     const int n1 = kGradHidden * K1, total = n1 + kGradHidden + O * kGradHidden;
@@ -446,7 +448,7 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
         a.status = d.status;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    mlp_grad_umma_kernel<<<a.ctas, kGradThreads, kGradSmemBytes, st>>>(a);
+    launch_early(mlp_grad_umma_kernel, a.ctas, kGradThreads, kGradSmemBytes, st, a);
     int rc = check_launch("mlp_grad_umma_kernel");
     if (rc != NPA_OK) return rc;
     const int total = kGradHidden * in_dim + kGradHidden + out_dim * kGradHidden;

@@ -30,6 +30,7 @@ struct HiddenGradArgs {
 };
 
 __global__ void __launch_bounds__(kHgThreads, 3) mlp_hidden_grad_kernel(HiddenGradArgs a) {
+    after_previous_kernel();
     __shared__ __align__(16) float w2s[kHgMaxOut][kHgHidden];
     __shared__ __align__(16) float dys[kHgWarps][kHgRows][kHgMaxOut];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;

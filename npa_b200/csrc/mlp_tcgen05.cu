@@ -99,6 +99,7 @@ struct ImageJobs {
     int count;
 };
 __global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
+    after_previous_kernel();
     int at = blockIdx.x * blockDim.x + threadIdx.x;
     for (int q = 0; q < jobs.count; ++q) {
         const ImageJob &j = jobs.job[q];
@@ -121,6 +122,7 @@ __global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
 
 template <bool FUSE>
 __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __grid_constant__ UmmaArgs args) {
+    after_previous_kernel();
     // every field is read into a register once: the role loops below must not go back to the parameter block
     const float *__restrict__ A = args.A;
     const float *__restrict__ Wimg = args.Wimg;
@@ -566,7 +568,7 @@ static ImageJob image_job(const float *W, int64_t stride_out, int64_t stride_in,
 static int launch_images(const ImageJobs &jobs, cudaStream_t st) {
     int total = 0;
     for (int q = 0; q < jobs.count; ++q) total += jobs.job[q].total();
-    weight_image_kernel<<<(total + 255) / 256, 256, 0, st>>>(jobs);
+    launch_early(weight_image_kernel, (total + 255) / 256, 256, 0, st, jobs);
     return check_launch("weight_image_kernel");
 }
 
@@ -615,7 +617,7 @@ static int linear_tcgen05(const float *A, const float *W, const float *bias, con
     }
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
-    linear_umma_kernel<false><<<ctas, kUmmaThreads, smem, (cudaStream_t)stream>>>(a);
+    launch_early(linear_umma_kernel<false>, ctas, kUmmaThreads, smem, (cudaStream_t)stream, a);
     return check_launch("linear_umma_kernel");
 }
 
@@ -677,7 +679,7 @@ int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float 
     if ((rc = launch_images(jobs, st)) != NPA_OK) return rc;
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
-    linear_umma_kernel<true><<<ctas, kUmmaThreads, smem, st>>>(a);
+    launch_early(linear_umma_kernel<true>, ctas, kUmmaThreads, smem, st, a);
     return check_launch("linear_umma_kernel (two layers)");
 }
 

@@ -277,6 +277,7 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
 template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
 __global__ void __launch_bounds__(kOrderedWarps * 32, D == 2 ? 10 : 8)
 packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
+    after_previous_kernel();
     using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
     __shared__ OrderedMem s_mem[kOrderedWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane >> 4, sl = lane & 15;
@@ -368,7 +369,7 @@ int launch_packed_ordered_shape(const Geom &g, const FeatureFwdArgs &a, cudaStre
     const bool aligned = (a.C % VW != 0 || (uintptr_t)a.s % (VW * 4) == 0) && ((uintptr_t)a.z | (uintptr_t)a.vgrad) % 8 == 0;
     const auto kernel = aligned ? packed_ordered_kernel<D, PER, VW, LPR, CPL, true> : packed_ordered_kernel<D, PER, VW, LPR, CPL, false>;
     const long long particles = (long long)g.B * g.N;
-    kernel<<<(unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st>>>(a, g);
+    launch_early(kernel, (unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st, a, g);
     return check_launch("packed_ordered_kernel");
 }
 

@@ -42,6 +42,7 @@ __global__ void __launch_bounds__(256)
 pack_backward_kernel(const float *__restrict__ gz, const float *__restrict__ vgrad, const float *__restrict__ rho_grad,
                      float *__restrict__ g_blur, float *__restrict__ g_grad, float *__restrict__ g_rho_grad,
                      long long particles, int C, float coef, float dg_scale, int log_norm_grad, int log_norm_dg) {
+    after_previous_kernel();
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     const int cp = ROWS ? (C + 3) & ~3 : C;
     if (t >= particles * cp) return;
@@ -228,10 +229,10 @@ int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, c
     float4 *pg = reinterpret_cast<float4 *>(g_dg + n * 4);
     const unsigned blocks = (unsigned)((n * cp + 255) / 256);
     if (g.dim == 2)
-        pack_backward_kernel<2, true><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+        launch_early(pack_backward_kernel<2, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
                                                               dg_scale, log_norm_grad, log_norm_dg);
     else
-        pack_backward_kernel<3, true><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+        launch_early(pack_backward_kernel<3, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
                                                               dg_scale, log_norm_grad, log_norm_dg);
     if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
     FeatureListBwdArgs a = {};
@@ -271,10 +272,10 @@ int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const f
     const unsigned blocks = (unsigned)((particles * channels + 255) / 256);
     float *grg = grad_x ? g_rho_grad_scratch : nullptr;
     if (g.dim == 2)
-        pack_backward_kernel<2, false><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
+        launch_early(pack_backward_kernel<2, false>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
                                                         particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
     else
-        pack_backward_kernel<3, false><<<blocks, 256, 0, st>>>(dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
+        launch_early(pack_backward_kernel<3, false>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
                                                         particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
     if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
     rc = npa_perception_backward(gd, channels, x_bin, mass, s_bin, rho, nullptr, g_blur_scratch, g_grad_scratch, grg,

@@ -25,6 +25,7 @@ struct MoveArgs {
 
 template <int D>
 __global__ void __launch_bounds__(256) rollout_move_kernel(const __grid_constant__ MoveArgs a, const __grid_constant__ Geom g) {
+    after_previous_kernel();
     constexpr int P = D == 2 ? 2 : 4;
     __shared__ float s_k[D * kMoveModes], s_phase[kMoveModes], s_amp[D * kMoveModes];
     for (int q = threadIdx.x; q < D * a.modes; q += blockDim.x) {
@@ -76,6 +77,6 @@ extern "C" int npa_rollout_move(const npa_grid *grid, const float *x, const floa
     if ((uintptr_t)x % (g.dim == 2 ? 8 : 16)) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_rollout_move: x must be aligned to one position");
     const MoveArgs a = {x, k, phase, amp, x_out, modes, dt};
     const unsigned blocks = (unsigned)(((long long)g.B * g.N + 255) / 256);
-    (g.dim == 2 ? rollout_move_kernel<2> : rollout_move_kernel<3>)<<<blocks, 256, 0, (cudaStream_t)stream>>>(a, g);
+    launch_early(g.dim == 2 ? rollout_move_kernel<2> : rollout_move_kernel<3>, blocks, 256, 0, (cudaStream_t)stream, a, g);
     return check_launch("rollout_move_kernel");
 }

@@ -12,6 +12,7 @@ namespace npa {
 template <int D, bool PER, int MASK>
 __global__ void __launch_bounds__(256)
 scalar_list_backward_kernel(ScalarListArgs a, Geom g) {
+    after_previous_kernel();
     constexpr int LPP = 4;
     const int lane = threadIdx.x & 31, sl = lane % LPP;
     const int total = g.B * g.N;
@@ -129,9 +130,9 @@ static int launch_scalar_list_geom(const Geom &g, const ScalarListArgs &a, cudaS
     const long long threads = 4ll * g.B * g.N;
     const unsigned blocks = (unsigned)((threads + 255) / 256);
     switch (mask) {
-        case S_DENSITY: scalar_list_backward_kernel<D, PER, S_DENSITY><<<blocks, 256, 0, st>>>(a, g); break;
-        case S_DGRAD: scalar_list_backward_kernel<D, PER, S_DGRAD><<<blocks, 256, 0, st>>>(a, g); break;
-        default: scalar_list_backward_kernel<D, PER, S_DENSITY | S_DGRAD><<<blocks, 256, 0, st>>>(a, g); break;
+        case S_DENSITY: launch_early(scalar_list_backward_kernel<D, PER, S_DENSITY>, blocks, 256, 0, st, a, g); break;
+        case S_DGRAD: launch_early(scalar_list_backward_kernel<D, PER, S_DGRAD>, blocks, 256, 0, st, a, g); break;
+        default: launch_early(scalar_list_backward_kernel<D, PER, S_DENSITY | S_DGRAD>, blocks, 256, 0, st, a, g); break;
     }
     return check_launch("scalar_list_backward_kernel");
 }
@@ -149,6 +150,7 @@ int launch_scalar_list_backward(const Geom &g, const ScalarListArgs &a, cudaStre
 template <int D, bool PER>
 __global__ void __launch_bounds__(256)
 density_gradient_list_kernel(ScalarListArgs a, Geom g) {
+    after_previous_kernel();
     constexpr int LPP = 8;
     const int lane = threadIdx.x & 31, sl = lane % LPP;
     const int total = g.B * g.N;
@@ -200,11 +202,11 @@ density_gradient_list_kernel(ScalarListArgs a, Geom g) {
 int launch_density_gradient_list(const Geom &g, const ScalarListArgs &a, cudaStream_t st) {
     const unsigned blocks = (unsigned)((8ll * g.B * g.N + 255) / 256);
     if (g.dim == 2) {
-        if (g.periodic) density_gradient_list_kernel<2, true><<<blocks, 256, 0, st>>>(a, g);
-        else density_gradient_list_kernel<2, false><<<blocks, 256, 0, st>>>(a, g);
+        if (g.periodic) launch_early(density_gradient_list_kernel<2, true>, blocks, 256, 0, st, a, g);
+        else launch_early(density_gradient_list_kernel<2, false>, blocks, 256, 0, st, a, g);
     } else {
-        if (g.periodic) density_gradient_list_kernel<3, true><<<blocks, 256, 0, st>>>(a, g);
-        else density_gradient_list_kernel<3, false><<<blocks, 256, 0, st>>>(a, g);
+        if (g.periodic) launch_early(density_gradient_list_kernel<3, true>, blocks, 256, 0, st, a, g);
+        else launch_early(density_gradient_list_kernel<3, false>, blocks, 256, 0, st, a, g);
     }
     return check_launch("density_gradient_list_kernel");
 }
@@ -217,6 +219,7 @@ template <int D, bool VEC>
 __global__ void __launch_bounds__(256)
 upstream_rows_kernel(const float *__restrict__ g_blur, const float *__restrict__ g_grad, float *__restrict__ rows, long long total, int C, int cp,
                      int with_blur) {
+    after_previous_kernel();
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     const int quads = cp / 4;
     if (t >= total * quads) return;
@@ -262,11 +265,11 @@ int launch_upstream_rows(const Geom &g, int C, const float *g_blur, const float 
     const bool vec = C % 4 == 0 && (((uintptr_t)g_grad | (with_blur ? (uintptr_t)g_blur : 0)) % 16) == 0;
     const int wb = with_blur ? 1 : 0;
     if (g.dim == 2) {
-        if (vec) upstream_rows_kernel<2, true><<<blocks, 256, 0, st>>>(g_blur, g_grad, rows, total, C, cp, wb);
-        else upstream_rows_kernel<2, false><<<blocks, 256, 0, st>>>(g_blur, g_grad, rows, total, C, cp, wb);
+        if (vec) launch_early(upstream_rows_kernel<2, true>, blocks, 256, 0, st, g_blur, g_grad, rows, total, C, cp, wb);
+        else launch_early(upstream_rows_kernel<2, false>, blocks, 256, 0, st, g_blur, g_grad, rows, total, C, cp, wb);
     } else {
-        if (vec) upstream_rows_kernel<3, true><<<blocks, 256, 0, st>>>(g_blur, g_grad, rows, total, C, cp, wb);
-        else upstream_rows_kernel<3, false><<<blocks, 256, 0, st>>>(g_blur, g_grad, rows, total, C, cp, wb);
+        if (vec) launch_early(upstream_rows_kernel<3, true>, blocks, 256, 0, st, g_blur, g_grad, rows, total, C, cp, wb);
+        else launch_early(upstream_rows_kernel<3, false>, blocks, 256, 0, st, g_blur, g_grad, rows, total, C, cp, wb);
     }
     return check_launch("upstream_rows_kernel");
 }

@@ -73,6 +73,7 @@ __device__ inline void axis_sums(int r, float f, float inv2s2, float &s0, float 
 // Normalised mode: the scale of every particle, once (the forward tiles would otherwise redo the
 // 2 (2r+1) exponentials for every tile a particle touches).
 __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
+    after_previous_kernel();
     const long long n = blockIdx.x * (long long)blockDim.x + threadIdx.x;
     if (n >= (long long)a.B * a.N) return;
     const SplatPoint p = splat_point(a, n);
@@ -118,6 +119,7 @@ __device__ inline int part_at(int pixel) { return pixel ^ ((pixel >> 5) & 7); }
 
 template <bool SLICED>
 __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatArgs a) {
+    after_previous_kernel();
     __shared__ SplatShared sh;
     __shared__ int s_count[kSplatWarps];
     const int tiles = (a.img + kSplatTile - 1) / kSplatTile;
@@ -301,6 +303,7 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
 // Few particles to a tile: a thread per pixel adds the particles that touch the tile in particle order.  Most of the
 // kernel above is fixed cost then (sixteen partial images, two blocks per SM); this one keeps eight blocks per SM.
 __global__ void __launch_bounds__(kSplatTile *kSplatTile) splat_forward_sparse_kernel(SplatArgs a) {
+    after_previous_kernel();
     constexpr int T = kSplatTile * kSplatTile;
     __shared__ int s_cx[T], s_cy[T];
     __shared__ float s_fx[T], s_fy[T], s_w[T], s_r[T], s_g[T], s_b[T];
@@ -376,6 +379,7 @@ __device__ inline float warp_sum(float v) {
 // columns per lane and two rows at a time) 80-102 us instead of 74, with particles sorted by place (L1 hits 81 %) 83.
 // 8 x 4,096 particles, patches of 41 x 41: 158 -> 74 us.
 __global__ void __launch_bounds__(256) splat_backward_kernel(SplatArgs a) {
+    after_previous_kernel();
     constexpr int kMost = 2 * kSplatMaxRadius + 1;
     __shared__ float2 s_y[8][kMost];  // row factor, row factor times t_y
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -500,17 +504,17 @@ int npa_splat_forward(const float *x, const float *color, int32_t batch, int32_t
     if (normalize) {
         if (!scale_scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_splat_forward: scale_scratch [B*N] is needed when normalize != 0");
         const long long n = (long long)batch * particles;
-        splat_scale_kernel<<<(unsigned)((n + 255) / 256), 256, 0, st>>>(a);
+        launch_early(splat_scale_kernel, (unsigned)((n + 255) / 256), 256, 0, st, a);
         if ((rc = check_launch("splat_scale_kernel")) != NPA_OK) return rc;
     }
     const int tiles = (img_size + kSplatTile - 1) / kSplatTile;
     if (sparse_tiles(a)) {
-        splat_forward_sparse_kernel<<<dim3(tiles * tiles, batch), kSplatTile * kSplatTile, 0, st>>>(a);
+        launch_early(splat_forward_sparse_kernel, dim3(tiles * tiles, batch), kSplatTile * kSplatTile, 0, st, a);
         return check_launch("splat_forward_sparse_kernel");
     }
     const int slices = splat_slices(a, tiles * tiles);
     if (slices == 1) {
-        splat_forward_kernel<false><<<dim3(tiles * tiles, batch), kSplatThreads, 0, st>>>(a);
+        launch_early(splat_forward_kernel<false>, dim3(tiles * tiles, batch), kSplatThreads, 0, st, a);
         return check_launch("splat_forward_kernel");
     }
     cudaLaunchConfig_t cfg = {};
@@ -541,7 +545,7 @@ int npa_splat_backward(const float *x, const float *color, const float *g_out, i
     const long long warps = (long long)batch * particles;
     const long long ctas = (warps * 32 + 255) / 256;
     if (ctas >= (1ll << 31)) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_splat_backward: too many particles");
-    splat_backward_kernel<<<(unsigned)ctas, 256, 0, (cudaStream_t)stream>>>(a);
+    launch_early(splat_backward_kernel, (unsigned)ctas, 256, 0, (cudaStream_t)stream, a);
     return check_launch("splat_backward_kernel");
 }
 

@@ -98,6 +98,7 @@ __device__ inline float step_backward_element(const StepArgs &a, long long i, in
 // has fewer than 2^31 elements.
 template <int D, typename Index, bool BACKWARD>
 __global__ void __launch_bounds__(256) step_update_kernel(StepArgs a, Geom g) {
+    after_previous_kernel();
     const Index W = (Index)(D + a.C);
     const Index total = (Index)a.particles * W;
     const Index quads = (total + 3) / 4;
@@ -146,6 +147,7 @@ __device__ inline void tile_copy_async(float *smem_dst, const float *gmem_src, i
 
 template <int D, bool BACKWARD>
 __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom g) {
+    after_previous_kernel();
     extern __shared__ __align__(16) float tile_mem[];  // forward: two tiles [kStepRows][D + C]; backward: one
     const int W = D + a.C, C4 = a.C / 4;
     const long long tiles = (a.particles + kStepRows - 1) / kStepRows;
@@ -258,8 +260,8 @@ static int launch_step(const Geom &g, const StepArgs &a, cudaStream_t st) {
         const long long tiles = (a.particles + kStepRows - 1) / kStepRows;
         const long long cap = 148ll * 8;
         const int ctas = (int)(tiles < cap ? (tiles > 0 ? tiles : 1) : cap);
-        if (g.dim == 2) step_update_tiled_kernel<2, BACKWARD><<<ctas, 256, tile_bytes, st>>>(a, g);
-        else step_update_tiled_kernel<3, BACKWARD><<<ctas, 256, tile_bytes, st>>>(a, g);
+        if (g.dim == 2) launch_early(step_update_tiled_kernel<2, BACKWARD>, ctas, 256, tile_bytes, st, a, g);
+        else launch_early(step_update_tiled_kernel<3, BACKWARD>, ctas, 256, tile_bytes, st, a, g);
         return check_launch(BACKWARD ? "step_update_tiled_kernel (backward)" : "step_update_tiled_kernel (forward)");
     }
     const long long total = a.particles * (g.dim + a.C);
@@ -269,11 +271,11 @@ static int launch_step(const Geom &g, const StepArgs &a, cudaStream_t st) {
     const int ctas = (int)(want < cap ? (want > 0 ? want : 1) : cap);
     const bool small = total < (1ll << 31) - 4;
     if (g.dim == 2) {
-        if (small) step_update_kernel<2, unsigned, BACKWARD><<<ctas, 256, 0, st>>>(a, g);
-        else step_update_kernel<2, long long, BACKWARD><<<ctas, 256, 0, st>>>(a, g);
+        if (small) launch_early(step_update_kernel<2, unsigned, BACKWARD>, ctas, 256, 0, st, a, g);
+        else launch_early(step_update_kernel<2, long long, BACKWARD>, ctas, 256, 0, st, a, g);
     } else {
-        if (small) step_update_kernel<3, unsigned, BACKWARD><<<ctas, 256, 0, st>>>(a, g);
-        else step_update_kernel<3, long long, BACKWARD><<<ctas, 256, 0, st>>>(a, g);
+        if (small) launch_early(step_update_kernel<3, unsigned, BACKWARD>, ctas, 256, 0, st, a, g);
+        else launch_early(step_update_kernel<3, long long, BACKWARD>, ctas, 256, 0, st, a, g);
     }
     return check_launch(BACKWARD ? "step_update_kernel (backward)" : "step_update_kernel (forward)");
 }
