@@ -25,7 +25,8 @@
 // set per row refilled early cost spills, 194 -> 234 us; five CTAs of the full backward instead of four 664 -> 758 us).
 // Measured, B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us, kernel with the whole warp per particle
 // -> this one: blur + gradient 328 -> 178 (with the density gradient), features-only backward 499 -> 401, full
-// backward 902 -> 644.
+// backward 902 -> 575 (644 with one sum per term and 14 warps per SM; 524,288 periodic, C = 16: 700 -> 632, with two list entries per
+// lane and chunk and the registers of these 790).  In 2D the one sum is level (8 x 16,384, C = 32: 446 -> 441; 8 x 4,096, C = 16: 43.8 -> 44.7).
 #pragma once
 #include "neighbors.cuh"
 #include "ops.cuh"
@@ -33,8 +34,7 @@
 namespace npa {
 
 constexpr int kListWarps = 8;      // warps per CTA
-// Same, backward; with position gradients it needs more registers than 16 warps per SM leave in 3D (60 bytes of spills):
-// seven CTAs of two warps there (262,144 particles 662 -> 644 us, 524,288 periodic 737 -> 703).
+// Same, backward; with position gradients sixteen warps per SM either way (128 registers), in 3D as eight CTAs of two.
 template <int D, bool FULL>
 constexpr int kListBackwardWarps = FULL ? (D == 3 ? 2 : 4) : kListWarps;
 
@@ -110,9 +110,9 @@ __device__ inline int compact_slot(bool acc, int sg, int sl, int &m) {
 
 // Shared memory of one warp: the entries of two chunks per sub-group (one entry of padding keeps the sub-groups'
 // broadcasts on different banks).
-template <int LPP>
+template <int LPP, bool ONE = false>  // ONE: an entry per lane in any case (registers)
 struct ListShape {
-    static constexpr int EPL = LPP == 4 ? 2 : 1;  // list entries per lane and chunk
+    static constexpr int EPL = LPP == 4 && !ONE ? 2 : 1;  // list entries per lane and chunk
     static constexpr int CH = LPP * EPL, PP = 32 / LPP;
     static constexpr int kSlots = PP * (CH + 1), kIndexQuads = PP * (CH / 4 + 1);
 };
@@ -461,13 +461,15 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
 //   u_d    = v_j (s_i - s_j).gG_i[d] + v_i (s_i - s_j).gG_j[d],   t = v_j gB_i.s_j + v_i gB_j.s_i
 //   dx_i   = sum_j (E t - psi r.u) r + phi u      (E, phi, psi with their constants)
 //   drho_i = (v_i / m_i) v_i sum_j [ phi r.((s_i - s_j) gG_j) - c_s W gB_j.s_i ]
+// With position gradients the scalars of a pair carry v_i, and v_j / v_i stands in for v_j: u_d / v_i = (s_i - s_j).(v_j / v_i gG_i[d] +
+// gG_j[d]) is one sum over the features instead of two, and sum_d K_d gG_j[d] serves ds and, times s_i - s_j, drho.
 // Sums over features stay lane-partial (packed pairs) until the particle is done.  The density gradient's own
 // backward, dx_i += sum_j J (m_i g_j - m_j g_i), uses the same pair scalars and rides stage B.
 // ---------------------------------------------------------------------------------------------------------
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL, bool SEARCH>
-__device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
-                                              float4 (*s_e)[ListShape<LPP>::kSlots], int4 (*s_j)[ListShape<LPP>::kIndexQuads]) {
-    constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP, WARPS = kListBackwardWarps<D, FULL>;
+__device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP, FULL && D == 3>::kSlots],
+                                              float4 (*s_e)[ListShape<LPP, FULL && D == 3>::kSlots], int4 (*s_j)[ListShape<LPP, FULL && D == 3>::kIndexQuads]) {
+    constexpr int EPL = ListShape<LPP, FULL && D == 3>::EPL, CH = ListShape<LPP, FULL && D == 3>::CH, PP = ListShape<LPP, FULL && D == 3>::PP, WARPS = kListBackwardWarps<D, FULL>;
     constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
     const int total = g.B * g.N, C = a.C;
@@ -484,33 +486,29 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
     const float mi = a.mass ? __ldg(a.mass + i) : 1.0f;
     const float rhoi = __ldg(a.rho + i);
     const float vi = mi / rhoi;
+    // v_i as the pair scalars carry it: a particle without volume has only its neighbours' terms, which v_j / v_i must be able to hold
+    const float vs = fabsf(vi) < 1e-25f ? 1e-25f : vi, inv_vs = 1.0f / vs;
     const unsigned spitch = (unsigned)C * 4u, bpitch = (unsigned)a.gb_pitch * 4u, gpitch = (unsigned)a.gg_pitch * 4u;
     const int Cp = a.cp;
     float dx[3] = {0.f, 0.f, 0.f};           // lane-partial over features and pairs
-    float dxd[3] = {0.f, 0.f, 0.f};          // density-gradient part, lane-partial over pairs
     unsigned long long drp = 0ull;           // minus the sum in drho, lane-partial
-    float gdi[3] = {0.f, 0.f, 0.f};
-    if (FULL && a.g_dg) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) gdi[d] = __ldg(a.g_dg + (long long)i * D + d);
-    }
 
     for (int fbase = 0; fbase < C; fbase += LPP * 4) {
         __syncwarp();
         const int f0 = fbase + sl * 4, fv = min(f0, Cp - 4);
-        // the i side: s_i, v_i s_i, gB_i, gG_i and v_i in packed pairs; a lane beyond the last feature contributes zeros
-        unsigned long long si[2] = {0ull, 0ull}, svi[2] = {0ull, 0ull}, gbi[2] = {0ull, 0ull}, vi2[2] = {0ull, 0ull}, ggi[2 * D];
+        // the i side: s_i, gB_i, gG_i in packed pairs; a lane beyond the last feature contributes zeros (minus1: -1 where it has features)
+        unsigned long long si[2] = {0ull, 0ull}, gbi[2] = {0ull, 0ull}, minus1[2] = {0ull, 0ull}, ggi[2 * D];
 #pragma unroll
         for (int q = 0; q < 2 * D; ++q) ggi[q] = 0ull;
         if (FULL) {
             float t[4];
             load_row4<VEC>(a.s + (long long)i * C, f0, C, t);
-            const bool live[4] = {f0 < C, f0 + 1 < C, f0 + 2 < C, f0 + 3 < C};
+            const bool live[4] = {f0 < C, VEC ? f0 < C : f0 + 1 < C, VEC ? f0 < C : f0 + 2 < C, VEC ? f0 < C : f0 + 3 < C};
 #pragma unroll
             for (int q = 0; q < 4; ++q) t[q] = live[q] ? t[q] : 0.f;
             si[0] = pack2(t[0], t[1]); si[1] = pack2(t[2], t[3]);
-            vi2[0] = pack2(live[0] ? vi : 0.f, live[1] ? vi : 0.f); vi2[1] = pack2(live[2] ? vi : 0.f, live[3] ? vi : 0.f);
-            svi[0] = pack2(vi * t[0], vi * t[1]); svi[1] = pack2(vi * t[2], vi * t[3]);
+            minus1[0] = pack2(live[0] ? -1.f : 0.f, live[1] ? -1.f : 0.f);
+            minus1[1] = VEC ? minus1[0] : pack2(live[2] ? -1.f : 0.f, live[3] ? -1.f : 0.f);
             if (kBlur && f0 < C) {
                 const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gb + (long long)i * a.gb_pitch + f0));
                 gbi[0] = pack2(b.x, live[1] ? b.y : 0.f);
@@ -525,7 +523,6 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
                 }
             }
         }
-        const unsigned long long minus1 = pack2(-1.f, -1.f);
         unsigned long long ds[2] = {0ull, 0ull};
         float tsum[3] = {0.f, 0.f, 0.f};  // T, lane-partial over the pairs
 
@@ -545,21 +542,21 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
             tsum[1] = fmaf(vj, ky, tsum[1]);
             if (D == 3) tsum[2] = fmaf(vj, kz, tsum[2]);
             const int at = sg * (CH + 1) + slot;
-            s_k[buf][at] = FULL ? make_float4(rx, ry, rz, w) : make_float4(-kx, -ky, -kz, w);
+            s_k[buf][at] = FULL ? make_float4(rx, ry, rz, vs * w) : make_float4(-kx, -ky, -kz, w);
             if (FULL) {
-                s_e[buf][at] = make_float4(phi, psi, vj, pair ? g.c_s * 6.0f * t * t : 0.f);
+                s_e[buf][at] = make_float4(vs * phi, vs * psi, vj * inv_vs, pair ? vs * (g.c_s * 6.0f * t * t) : 0.f);
                 if (a.g_dg && fbase == 0 && q > 0.f) {
                     const float mj = a.mass ? __ldg(a.mass + j) : 1.0f;
                     const float rv[3] = {rx, ry, rz};
                     float u[3] = {0.f, 0.f, 0.f}, ru = 0.f;
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
-                        u[d] = mi * __ldg(a.g_dg + (long long)j * D + d) - mj * gdi[d];
+                        u[d] = mi * __ldg(a.g_dg + (long long)j * D + d) - mj * __ldg(a.g_dg + (long long)i * D + d);
                         ru = fmaf(rv[d], u[d], ru);
                     }
                     const float sc = psi * ru;
 #pragma unroll
-                    for (int d = 0; d < D; ++d) dxd[d] += phi * u[d] - sc * rv[d];
+                    for (int d = 0; d < D; ++d) dx[d] += phi * u[d] - sc * rv[d];
                 }
             }
             reinterpret_cast<int *>(&s_j[buf][sg * (CH / 4 + 1)])[slot] = j;
@@ -586,7 +583,7 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
             const float4 ke = s_k[buf][at];
             const float4 ex = FULL ? s_e[buf][at] : make_float4(-1.f, 0.f, 0.f, 0.f);
             const unsigned long long w = pack2(ke.w, ke.w);
-            unsigned long long b01, b23, k[D];
+            unsigned long long b01, b23, k01 = 0ull, k23 = 0ull;  // k: minus sum_d K_d gG_j[d]
             if (kBlur) {
                 b01 = pack2(r.b[0], r.b[1]); b23 = pack2(r.b[2], r.b[3]);
                 ds[0] = fma2(w, b01, ds[0]);
@@ -597,9 +594,21 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
                     const float m = FULL ? -(ex.x * kv[d]) : kv[d];  // -K
-                    k[d] = pack2(m, m);
-                    ds[0] = fma2(k[d], pack2(r.g[d][0], r.g[d][1]), ds[0]);
-                    ds[1] = fma2(k[d], pack2(r.g[d][2], r.g[d][3]), ds[1]);
+                    const unsigned long long kd = pack2(m, m);
+                    if (!FULL) {
+                        ds[0] = fma2(kd, pack2(r.g[d][0], r.g[d][1]), ds[0]);
+                        ds[1] = fma2(kd, pack2(r.g[d][2], r.g[d][3]), ds[1]);
+                    } else if (d == 0) {
+                        k01 = mul2(kd, pack2(r.g[d][0], r.g[d][1]));
+                        k23 = mul2(kd, pack2(r.g[d][2], r.g[d][3]));
+                    } else {
+                        k01 = fma2(kd, pack2(r.g[d][0], r.g[d][1]), k01);
+                        k23 = fma2(kd, pack2(r.g[d][2], r.g[d][3]), k23);
+                    }
+                }
+                if (FULL) {
+                    ds[0] = add2(ds[0], k01);
+                    ds[1] = add2(ds[1], k23);
                 }
             }
             if (FULL) {
@@ -608,23 +617,23 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
                 float coef = 0.f;
                 if (kBlur) {
                     const unsigned long long A = fma2(gbi[1], s23, mul2(gbi[0], s01));
-                    const unsigned long long Bp = fma2(svi[1], b23, mul2(svi[0], b01));
+                    const unsigned long long Bp = fma2(si[1], b23, mul2(si[0], b01));
                     float lo, hi;
                     unpack2(fma2(vj, A, Bp), lo, hi);
                     coef = ex.w * (lo + hi);
                     drp = fma2(w, Bp, drp);
                 }
                 if (kGrad) {
-                    const unsigned long long e01 = fma2(s01, minus1, si[0]), e23 = fma2(s23, minus1, si[1]);  // s_i - s_j
-                    const unsigned long long f01 = mul2(vi2[0], e01), f23 = mul2(vi2[1], e23);
+                    const unsigned long long e01 = fma2(s01, minus1[0], si[0]), e23 = fma2(s23, minus1[1], si[1]);  // s_i - s_j
+                    drp = fma2(e01, k01, drp);
+                    drp = fma2(e23, k23, drp);
                     float u[3] = {0.f, 0.f, 0.f};
 #pragma unroll
                     for (int d = 0; d < D; ++d) {
-                        const unsigned long long A = fma2(ggi[2 * d + 1], e23, mul2(ggi[2 * d], e01));
-                        const unsigned long long Bv = fma2(pack2(r.g[d][2], r.g[d][3]), f23, mul2(pack2(r.g[d][0], r.g[d][1]), f01));
-                        drp = fma2(k[d], Bv, drp);
+                        const unsigned long long h01 = fma2(vj, ggi[2 * d], pack2(r.g[d][0], r.g[d][1]));
+                        const unsigned long long h23 = fma2(vj, ggi[2 * d + 1], pack2(r.g[d][2], r.g[d][3]));
                         float lo, hi;
-                        unpack2(fma2(vj, A, Bv), lo, hi);
+                        unpack2(fma2(h23, e23, mul2(h01, e01)), lo, hi);
                         u[d] = lo + hi;
                     }
                     float ru = rv[0] * u[0] + rv[1] * u[1];
@@ -728,8 +737,10 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
             float o[4];
             unpack2(ds[0], o[0], o[1]);
             unpack2(ds[1], o[2], o[3]);
+            if (!FULL) {
 #pragma unroll
-            for (int q = 0; q < 4; ++q) o[q] *= vi;
+                for (int q = 0; q < 4; ++q) o[q] *= vi;
+            }
             if (kGrad) {
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
@@ -759,7 +770,7 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
         const float dr = -subgroup_sum<LPP>(lo + hi) / rhoi;
         float out[3] = {0.f, 0.f, 0.f};
 #pragma unroll
-        for (int d = 0; d < D; ++d) out[d] = subgroup_sum<LPP>(dx[d] + dxd[d]);
+        for (int d = 0; d < D; ++d) out[d] = subgroup_sum<LPP>(dx[d]);
         if (ivalid && sl == 0) {
             if (a.grad_x) {
                 if (D == 2) reinterpret_cast<float2 *>(a.grad_x)[i] = make_float2(out[0], out[1]);
@@ -773,21 +784,21 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
 }
 
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
-__device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
-                                                  float4 (*s_e)[ListShape<LPP>::kSlots], int4 (*s_j)[ListShape<LPP>::kIndexQuads]) {
+__device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP, FULL && D == 3>::kSlots],
+                                                  float4 (*s_e)[ListShape<LPP, FULL && D == 3>::kSlots], int4 (*s_j)[ListShape<LPP, FULL && D == 3>::kIndexQuads]) {
     list_backward<D, PER, LPP, VEC, MASK, FULL, true>(a, g, s_k, s_e, s_j);
 }
 
 // Features only: four CTAs with up to 16 features -- 32,768 particles are a wave and a seventh of three CTAs, 48 -> 38 us --
 // and three with longer rows, 401 us against 411.
 template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
-__global__ void __launch_bounds__(kListBackwardWarps<D, FULL> * 32, FULL ? (D == 3 ? 7 : 4) : LPP == 4 ? 4 : 3)
+__global__ void __launch_bounds__(kListBackwardWarps<D, FULL> * 32, FULL ? (D == 3 ? 8 : 4) : LPP == 4 ? 4 : 3)
 feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
     after_previous_kernel();
-    using S = ListShape<LPP>;
+    using S = ListShape<LPP, FULL && D == 3>;
     constexpr int WARPS = kListBackwardWarps<D, FULL>;
-    __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z W
-    __shared__ float4 s_e[FULL ? WARPS : 1][2][S::kSlots];  // FULL: phi psi v_j E
+    __shared__ float4 s_k[WARPS][2][S::kSlots];             // -K.x -K.y -K.z W; FULL: r.x r.y r.z v_i W
+    __shared__ float4 s_e[FULL ? WARPS : 1][2][S::kSlots];  // FULL: v_i (phi, psi, ., E), v_j / v_i
     __shared__ int4 s_j[WARPS][2][S::kIndexQuads];
     const int warp = threadIdx.x >> 5, total = g.B * g.N;
     const unsigned first = (blockIdx.x * WARPS + warp) * S::PP;
