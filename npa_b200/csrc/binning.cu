@@ -11,6 +11,8 @@
 //  * cell counts and work-item counts are scanned together in one three-phase
 //    scan, and the work list is written by the scan's last phase.
 // All kernels are HBM-bound integer work; nothing here is GEMM shaped.
+#include <cooperative_groups.h>
+
 #include <mutex>
 
 #include "ops.cuh"
@@ -378,7 +380,7 @@ rank_kernel(const uint32_t *__restrict__ cellid, const int32_t *__restrict__ bin
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallParticles = 16384;
-constexpr size_t kSmallSmem = 200 * 1024;
+constexpr size_t kSmallSmem = 200 * 1024, kClusterSmem = 220 * 1024;
 
 // Place of a cell in the shared table: one word of padding per 32, so that threads that walk consecutive cells each do not
 // meet on one bank.
@@ -388,23 +390,37 @@ static size_t small_smem(const Geom &g) {
     return (size_t)(table_at(g.cells) + 1) * 4 + (size_t)((g.N + 1) & ~1) * 4 + (size_t)((g.N + 31) / 32) * 8;
 }
 
-// Whether one CTA per system is the faster way, from estimates of both in microseconds.  Small: a fixed part; the
-// particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell); the cell table, which a thread walks in
+// Which way to build a grid, from estimates of all in microseconds.  Small (one CTA per system): a fixed part; the particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell); the cell table, which a thread walks in
 // consecutive cells -- once in shared memory and, with several systems, again in global memory, where long runs per thread
 // scatter the loads.  General: six launches and their gaps; the shared histogram; the particles and cells of all systems; ranking, spread
-// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells) in a graph; back to
-// back on a stream the general way takes 8 us more, in the gaps between its launches, and that is counted (8 systems of
-// 16,384 in 40 x 40: kernels 35 / 28, but a pass that bins them is 8 us shorter with the small way).  Some sizes, small /
+// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells) in a graph; what
+// the general way takes more back to back on a stream, in the gaps between its launches, is counted.  Some sizes, small /
 // general, us, in a graph: 1 system of 2,048 in 16 x 16 6 / 23; 4 of 4,096 12 / 22; 64 of 16,384 in 64 x 64 28 / 61; 1 of 16,384 in
 // 8 x 8 93 / 30; 2 of 4,096 in 32^3 77 / 25; 16 of 12,000 in 128 x 128 43 / 28.
-static bool small_system(const Geom &g) {
-    if (g.N > kSmallParticles || g.cells >= 65536 || small_smem(g) > kSmallSmem) return false;
+enum class GridBuild { kSmall, kCluster, kGeneral };
+
+static double rows_estimate(const Geom &g) {
+    const double c = g.cells;
+    return g.B > 1 ? 3.0 + c * c / 2.2e7 + c / 4000.0 : c / 2500.0;
+}
+
+// One cluster per system (bin_cluster_kernel): a fixed part, the share of a CTA, the CTAs (eight per system on 148 SMs), the cells and
+// rows.  Measured against the others over 33 sizes: with the better way of the two others 1 % behind at worst where it is chosen, 12 %
+// where it is not (16 systems of 4,096).  Since the general launches overlap they take 4 us less on a stream than when they were fitted.
+constexpr int kClusterCtas = 8;
+static size_t cluster_smem(const Geom &g, int ctas);
+
+static GridBuild grid_build(const Geom &g) {
     const double n = g.N, c = g.cells, all = n * g.B, per_cell = n / c, ranking = per_cell > kCrowdedCell ? 0.0 : n * per_cell;
-    const double small = 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) +
-                         (g.B > 1 ? 3.0 + c * c / 2.2e7 + c / 4000.0 : c / 2500.0);
-    const double general = 24.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
+    const double none = 1e30;
+    const bool fits = g.N <= kSmallParticles && g.cells < 65536 && small_smem(g) <= kSmallSmem;
+    const double small = fits ? 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) + rows_estimate(g) : none;
+    const double general = 20.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
                            (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7;
-    return small <= general;
+    const bool shares = g.N > 2048 && g.N <= 65536 && g.cells < 65536 && cluster_smem(g, kClusterCtas) <= kClusterSmem;
+    const double cluster = shares ? 7.0 + n / 4400.0 + g.B / 8.0 + rows_estimate(g) : none;
+    if (cluster < small && cluster < general) return GridBuild::kCluster;
+    return small <= general ? GridBuild::kSmall : GridBuild::kGeneral;
 }
 
 // Exclusive scan over the CTA's cell table: every thread takes `per` consecutive cells.  Calls emit(cell, count, prefix)
@@ -498,6 +514,166 @@ bin_small_kernel(const float *__restrict__ x, int32_t *__restrict__ permutation,
             permutation[sys + i] = (int32_t)(s + pre[i >> 5] + (uint32_t)__popc(bits[i >> 5] & ((1u << (i & 31)) - 1u)));
         }
     }
+}
+
+// ---------------------------------------------------------------------------
+// Systems of up to 65,536 particles by one cluster of CTAs each.  A CTA counts and orders its share of the particles (consecutive
+// indices) in shared memory; the CTAs then share the cells: the owner of a slice of them reads the counts of all CTAs through
+// distributed shared memory, scans them and leaves every CTA the slot of its first particle in each cell.  Stable: the particles of a
+// cell lie CTA by CTA, and inside a CTA in index order.  Counts and slots are 16 bits, two to a word (shares of at most 8,192).
+// Bound by latency: four passes over the share and three meetings of the cluster.  Back to back on a stream, work list included,
+// us: 8 systems of 16,384 in 40 x 40 25 (one CTA per system) -> 13, 1 of 16,384 in 64 x 64 21 -> 11, 1 of 4,096 in 10 x 10 9.6 -> 7.4, 8 of
+// 4,096 in 16 x 16 11.2 -> 10; 1 of 65,536 in 64 x 64 32 (general launches) -> 20, 2 of 32,768 in 20^3 37 -> 26.
+// ---------------------------------------------------------------------------
+constexpr int kClusterThreads = 512, kClusterMost = 8, kClusterShare = 8192;
+
+static size_t cluster_smem(const Geom &g, int ctas) {
+    const int words = (g.cells + 1) / 2, slice = (words + ctas - 1) / ctas, share = (g.N + ctas - 1) / ctas;
+    return (size_t)(table_at(words) + 1) * 8 + (size_t)slice * 8 + (size_t)((share + 31) / 32) * 8 + (size_t)((share + 1) & ~1) * 4;
+}
+
+__device__ inline uint32_t half_of(const uint32_t *words, uint32_t c) { return (words[table_at((int)(c >> 1))] >> (16 * (c & 1))) & 0xffffu; }
+
+template <int D>
+__global__ void __launch_bounds__(kClusterThreads)
+bin_cluster_kernel(const float *__restrict__ x, int32_t *__restrict__ permutation, int32_t *__restrict__ bin_offsets,
+                   int4 *__restrict__ block_info, uint32_t *__restrict__ rows_of_system, Geom g) {
+    after_previous_kernel();
+    constexpr int T = kClusterThreads;
+    extern __shared__ uint32_t cluster_mem[];
+    __shared__ uint32_t s_bound[kClusterMost], s_items, crowded_n, s_crowded[kClusterShare / kCrowdedCell];
+    __shared__ unsigned long long scan_total;
+    cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+    const int K = (int)cluster.num_blocks(), r = (int)cluster.block_rank(), b = blockIdx.x / K, tid = threadIdx.x;
+    const int words = (g.cells + 1) / 2, slice = (words + K - 1) / K, share = (g.N + K - 1) / K;
+    const int i0 = min(r * share, g.N), mine = min(share, g.N - i0), marks = (share + 31) / 32;
+    uint32_t *first = cluster_mem;                            // per cell: particles of this CTA, then the slot of the first of them
+    uint32_t *next = first + table_at(words) + 1;             // per cell: next place in this CTA's order, then their end
+    uint32_t *total = next + table_at(words) + 1;             // per cell of this CTA's slice: particles of the system
+    uint32_t *bits = total + 2 * slice, *pre = bits + marks;  // crowded cells only
+    uint16_t *key = reinterpret_cast<uint16_t *>(pre + marks), *order = key + ((share + 1) & ~1);
+    const size_t sys = (size_t)b * g.N;
+    for (int w = tid; w <= table_at(words); w += T) first[w] = 0u;
+    if (tid < K) s_bound[tid] = (uint32_t)mine;
+    if (tid == 0) crowded_n = 0u;
+    __syncthreads();
+    for (int i = tid; i < mine; i += T) {
+        const uint32_t c = particle_cell<D>(x, sys + i0 + i, g);
+        key[i] = (uint16_t)c;
+        atomicAdd(&first[table_at((int)(c >> 1))], 1u << (16 * (c & 1)));
+    }
+    __syncthreads();
+    {   // places in this CTA's order, and how many of its particles lie before each slice of the cells
+        const int per = (words + T - 1) / T, w0 = tid * per, w1 = min(w0 + per, words);
+        unsigned long long v = 0;
+        for (int w = w0; w < w1; ++w) {
+            const uint32_t n = first[table_at(w)];
+            v += (n & 0xffffu) + (n >> 16);
+        }
+        uint32_t run = (uint32_t)block_exclusive<T>(v, scan_total);
+        for (int w = w0; w < w1; ++w) {
+            const uint32_t n = first[table_at(w)], lo = n & 0xffffu, hi = n >> 16;
+            if (w % slice == 0) s_bound[w / slice] = run;
+            if (lo > (uint32_t)kCrowdedCell) s_crowded[atomicAdd(&crowded_n, 1u)] = (uint32_t)(2 * w);
+            if (hi > (uint32_t)kCrowdedCell) s_crowded[atomicAdd(&crowded_n, 1u)] = (uint32_t)(2 * w + 1);
+            next[table_at(w)] = run | ((run + lo) << 16);
+            run += lo + hi;
+        }
+    }
+    cluster.sync();
+    // this CTA's slice of the cells
+    unsigned long long before = 0;  // work items of the slice << 32 | particles of the system, up to here
+    for (int q = 0; q < K; ++q) before += cluster.map_shared_rank(s_bound, q)[r];
+    for (int base = 0; base < slice; base += T) {
+        const int w = r * slice + base + tid;
+        const bool valid = base + tid < slice && w < words;
+        uint32_t n[kClusterMost], lo = 0, hi = 0;
+#pragma unroll
+        for (int q = 0; q < kClusterMost; ++q) {
+            n[q] = valid && q < K ? cluster.map_shared_rank(first, q)[table_at(w)] : 0u;
+            lo += n[q] & 0xffffu;
+            hi += n[q] >> 16;
+        }
+        const unsigned long long at = before + block_exclusive<T>(pack_cell(lo, g.mpb) + pack_cell(hi, g.mpb), scan_total);
+        if (valid) {
+            uint32_t slot_lo = (uint32_t)at, slot_hi = slot_lo + lo;
+            int32_t *o = bin_offsets + (size_t)b * g.cells + 2 * w;
+            o[0] = (int32_t)((uint32_t)sys + slot_lo);
+            if (2 * w + 1 < g.cells) o[1] = (int32_t)((uint32_t)sys + slot_hi);
+            if (g.B == 1) {
+                total[2 * (base + tid)] = lo;
+                total[2 * (base + tid) + 1] = hi;
+            }
+#pragma unroll
+            for (int q = 0; q < kClusterMost; ++q) {
+                if (q >= K) break;
+                cluster.map_shared_rank(first, q)[table_at(w)] = (slot_lo & 0xffffu) | (slot_hi << 16);
+                slot_lo += n[q] & 0xffffu;
+                slot_hi += n[q] >> 16;
+            }
+        }
+        before += scan_total;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        s_items = (uint32_t)(before >> 32);
+        if (b == g.B - 1 && r == 0) bin_offsets[(size_t)g.B * g.cells] = (int32_t)((size_t)g.B * g.N);
+    }
+    for (int i = tid; i < mine; i += T) {
+        const uint32_t c = key[i], shift = 16 * (c & 1);
+        order[(atomicAdd(&next[table_at((int)(c >> 1))], 1u << shift) >> shift) & 0xffffu] = (uint16_t)i;
+    }
+    cluster.sync();
+    // every place of a cell is taken: its entry is now its end, the entry before it its start
+    auto cell_start = [&](uint32_t c) { return c ? half_of(next, c - 1) : 0u; };
+    for (int p = tid; p < mine; p += T) {
+        const uint32_t i = order[p], c = key[i], s = cell_start(c), e = half_of(next, c);
+        if (e - s > (uint32_t)kCrowdedCell) continue;
+        uint32_t rank = 0;
+        for (uint32_t q = s; q < e; ++q) rank += order[q] < i ? 1u : 0u;
+        permutation[sys + i0 + i] = (int32_t)(half_of(first, c) + rank);
+    }
+    // crowded cells: a bitmap over the particle indices and its prefix popcounts, as above
+    for (uint32_t k = 0; k < crowded_n; ++k) {
+        const uint32_t c = s_crowded[k], s = cell_start(c), e = half_of(next, c);
+        __syncthreads();
+        for (int w = tid; w < marks; w += T) bits[w] = 0u;
+        __syncthreads();
+        for (uint32_t q = s + tid; q < e; q += T) atomicOr(&bits[order[q] >> 5], 1u << (order[q] & 31));
+        __syncthreads();
+        const unsigned long long here = tid < marks ? (unsigned long long)__popc(bits[tid]) : 0ull;  // marks <= 256
+        const unsigned long long earlier = block_exclusive<T>(here, scan_total);
+        if (tid < marks) pre[tid] = (uint32_t)earlier;
+        __syncthreads();
+        for (uint32_t q = s + tid; q < e; q += T) {
+            const uint32_t i = order[q];
+            permutation[sys + i0 + i] = (int32_t)(half_of(first, c) + pre[i >> 5] + (uint32_t)__popc(bits[i >> 5] & ((1u << (i & 31)) - 1u)));
+        }
+    }
+    // rows: their number for rows_small_kernel, or with a single system the work list itself
+    uint32_t row = 0, rows = 0;
+    for (int q = 0; q < K; ++q) {
+        const uint32_t n = *cluster.map_shared_rank(&s_items, q);
+        if (q < r) row += n;
+        rows += n;
+    }
+    if (g.B > 1) {
+        if (r == 0 && tid == 0) rows_of_system[b] = rows;
+    } else {
+        for (int base = 0; base < slice; base += T) {
+            const int w = r * slice + base + tid;
+            const bool valid = base + tid < slice && w < words;
+            const uint32_t lo = valid ? total[2 * (base + tid)] : 0u, hi = valid ? total[2 * (base + tid) + 1] : 0u;
+            const unsigned long long n_lo = pack_cell(lo, g.mpb) >> 32, n_hi = pack_cell(hi, g.mpb) >> 32;
+            __syncthreads();
+            const uint32_t at = row + (uint32_t)block_exclusive<T>(n_lo + n_hi, scan_total);
+            write_rows(block_info, g, 0, 2 * w, lo, at);
+            write_rows(block_info, g, 0, 2 * w + 1, hi, at + (uint32_t)n_lo);
+            row += (uint32_t)scan_total;
+        }
+        for (int k = (int)rows + r * T + tid; k < g.max_blocks; k += K * T) block_info[k] = make_int4(0, 0, 0, 0);
+    }
+    cluster.sync();  // a CTA's shared memory stays until all have read it
 }
 
 // Work list of several small systems: the rows of a system start behind those of the systems before it.
@@ -677,7 +853,19 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     if (scratch_bytes < (int64_t)need)
         return fail(NPA_ERR_SCRATCH_TOO_SMALL, "npa_grid_build: scratch has %lld bytes, %zu needed", (long long)scratch_bytes, need);
     cudaStream_t st = (cudaStream_t)stream;
-    if (small_system(g)) {
+    const GridBuild way = grid_build(g);
+    if (way == GridBuild::kCluster) {
+        const int ctas = kClusterCtas;
+        const auto kernel = g.dim == 2 ? bin_cluster_kernel<2> : bin_cluster_kernel<3>;
+        const size_t bytes = cluster_smem(g, ctas);
+        int unused = 0;
+        if ((rc = persistent_ctas(kernel, kClusterThreads, bytes, &unused)) != NPA_OK) return rc;  // shared-memory limit
+        launch_cluster(ctas, kernel, g.B * ctas, kClusterThreads, bytes, st, x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        if ((rc = check_launch("bin_cluster_kernel")) != NPA_OK || g.B == 1) return rc;
+        launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
+        return check_launch("rows_small_kernel");
+    }
+    if (way == GridBuild::kSmall) {
         const size_t bytes = small_smem(g);
         int unused = 0;
         if (g.dim == 2) {

@@ -8,6 +8,9 @@
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <utility>
+
 #include "../../include/npa_b200.h"
 
 namespace npa {
@@ -62,17 +65,29 @@ __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
+// The same with clusters of `cluster` blocks.
+template <typename... P, typename... A>
+inline void launch_cluster(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    cudaLaunchAttribute attrs[2];
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream; cfg.attrs = attrs;
+    if (cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
+        attrs[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attrs[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (cluster > 1) {
+        attrs[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+        attrs[cfg.numAttrs].val.clusterDim.x = cluster;
+        attrs[cfg.numAttrs].val.clusterDim.y = attrs[cfg.numAttrs].val.clusterDim.z = 1;
+        ++cfg.numAttrs;
+    }
+    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // an error is check_launch's
+}
+
 template <typename... P, typename... A>
 inline void launch_early(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    const bool early = cudaStreamIsCapturing(stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone;
-    cudaLaunchAttribute attr;
-    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    attr.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = grid; cfg.blockDim = block; cfg.dynamicSmemBytes = smem; cfg.stream = stream;
-    cfg.attrs = &attr; cfg.numAttrs = early ? 1 : 0;
-    (void)cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);  // an error is check_launch's
+    launch_cluster(1, kernel, grid, block, smem, stream, std::forward<A>(args)...);
 }
 
 // ---- cell hashing (sphops/utils.cuh:394-524) -------------------------------

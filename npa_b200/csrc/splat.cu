@@ -517,17 +517,7 @@ int npa_splat_forward(const float *x, const float *color, int32_t batch, int32_t
         launch_early(splat_forward_kernel<false>, dim3(tiles * tiles, batch), kSplatThreads, 0, st, a);
         return check_launch("splat_forward_kernel");
     }
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(slices * tiles * tiles, batch);
-    cfg.blockDim = dim3(kSplatThreads);
-    cfg.stream = st;
-    cudaLaunchAttribute cluster;
-    cluster.id = cudaLaunchAttributeClusterDimension;
-    cluster.val.clusterDim.x = slices;
-    cluster.val.clusterDim.y = cluster.val.clusterDim.z = 1;
-    cfg.attrs = &cluster;
-    cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, splat_forward_kernel<true>, a);
+    launch_cluster(slices, splat_forward_kernel<true>, dim3(slices * tiles * tiles, batch), kSplatThreads, 0, st, a);
     return check_launch("splat_forward_kernel");
 }
 

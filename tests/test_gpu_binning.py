@@ -161,3 +161,17 @@ def test_either_way_of_the_grid_build(dim, B, N, cells):
     w = Workload("ways", dim=dim, B=B, N=N, C=4, eps=1.0 / cells, grid_size=(cells,) * dim, max_particles_per_block=32)
     x = (torch.rand(B, N, w.P, generator=torch.Generator().manual_seed(cells)) - 0.5) * 1.05
     _check(sph, w, x)
+
+
+@pytest.mark.parametrize("dim,B,N,cells,hash_mode,boundary", [
+    (2, 1, 4096, 10, "grid", "periodic"), (2, 3, 4097, 5, "grid", "clamped"), (2, 1, 65536, 64, "grid", "clamped"), (2, 2, 65535, 33, "grid", "periodic"),
+    (3, 1, 16384, 32, "particle", "clamped"), (3, 2, 20001, 16, "particle", "periodic"), (3, 5, 2501, 3, "grid", "clamped")])
+@pytest.mark.parametrize("spread", [1.05, 0.02])
+def test_one_cluster_per_system(dim, B, N, cells, hash_mode, boundary, spread):
+    """A cluster of CTAs per system: shares that do not divide evenly, odd numbers of cells, one and several systems, and particles
+    in a handful of cells, thousands to each."""
+    from npa_b200 import sphops as sph
+    w = Workload("cluster", dim=dim, B=B, N=N, C=4, eps=1.0 / cells, grid_size=(cells,) * dim, boundary=boundary, mode=hash_mode,
+                 max_particles_per_block=32)
+    x = (torch.rand(B, N, w.P, generator=torch.Generator().manual_seed(cells)) - 0.5) * spread
+    _check(sph, w, x)
