@@ -89,7 +89,7 @@ def _link_ops(obj: Path) -> None:
 
     dirs = [arg for p in library_paths() for arg in (f"-L{p}", f"-Wl,-rpath,{p}")]
     cmd = ["g++", "-shared", "-o", str(OPS_PATH), str(obj), f"-L{PKG_DIR}", "-l:libnpa_b200.so", "-Wl,-rpath,$ORIGIN", *dirs,
-           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch", "-ltorch_python"]
+           "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch", "-ltorch_python"]
     res = subprocess.run(cmd, capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"link of {OPS_PATH.name} failed:\n{res.stdout}\n{res.stderr}")
