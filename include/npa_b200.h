@@ -472,6 +472,9 @@ int npa_splat_backward(const float *x, const float *color, const float *g_out, i
 int npa_rollout_move(const npa_grid *grid, const float *x, const float *k, const float *phase, const float *amp,
                      int32_t modes, float dt, float *x_out, void *stream);
 
+/* a_out = a [na floats] and b_out = b [nb floats] in one launch; 16-byte aligned arrays that do not overlap. */
+int npa_copy_pair(const float *a, float *a_out, int64_t na, const float *b, float *b_out, int64_t nb, void *stream);
+
 /* ---- weight gradients of the per-particle MLP ------------------------------------ *
  * The adaptation MLP of an NPA model (models/npa.py:63-75) is Linear(in, 128) -> ReLU ->
  * Linear(128, out, bias = False), applied to every particle.  One pass over the rows gives

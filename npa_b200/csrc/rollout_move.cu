@@ -63,9 +63,32 @@ __global__ void __launch_bounds__(256) rollout_move_kernel(const __grid_constant
     }
 }
 
+// Two arrays in one launch: the inputs of a recorded step are copied into its buffers before every replay, and two copies of
+// a few hundred kilobytes are mostly the gap between them (2.5 us of a step of 42).
+__global__ void __launch_bounds__(256) copy_pair_kernel(const float *__restrict__ a, float *__restrict__ a_out, long long na,
+                                                        const float *__restrict__ b, float *__restrict__ b_out, long long nb) {
+    const long long qa = na / 4, qb = nb / 4, step = (long long)gridDim.x * blockDim.x, t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
+    for (long long q = t; q < qa + qb; q += step) {
+        const bool second = q >= qa;
+        const long long at = second ? q - qa : q;
+        reinterpret_cast<float4 *>(second ? b_out : a_out)[at] = __ldg(reinterpret_cast<const float4 *>(second ? b : a) + at);
+    }
+    if (t < na % 4) a_out[qa * 4 + t] = a[qa * 4 + t];
+    if (t < nb % 4) b_out[qb * 4 + t] = b[qb * 4 + t];
+}
+
 }  // namespace npa
 
 using namespace npa;
+
+extern "C" int npa_copy_pair(const float *a, float *a_out, int64_t na, const float *b, float *b_out, int64_t nb, void *stream) {
+    if (!a || !a_out || !b || !b_out || na < 0 || nb < 0) return fail(NPA_ERR_INVALID_ARGUMENT, "npa_copy_pair: arrays must be non-NULL");
+    if (((uintptr_t)a | (uintptr_t)a_out | (uintptr_t)b | (uintptr_t)b_out) % 16)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "npa_copy_pair: arrays must be 16-byte aligned");
+    const long long blocks = (na / 4 + nb / 4 + 255) / 256;
+    copy_pair_kernel<<<(unsigned)(blocks < 1 ? 1 : blocks < 148 * 8 ? blocks : 148 * 8), 256, 0, (cudaStream_t)stream>>>(a, a_out, na, b, b_out, nb);
+    return check_launch("copy_pair_kernel");
+}
 
 extern "C" int npa_rollout_move(const npa_grid *grid, const float *x, const float *k, const float *phase, const float *amp, int32_t modes, float dt,
                                 float *x_out, void *stream) {

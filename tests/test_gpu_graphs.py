@@ -50,3 +50,20 @@ def test_graphed_euler_rollout_equals_eager():
             xe, se, _ = step_euler(model, xe, se, grid, dt=1.0, update_prob=1.0, wrap=True)
     assert torch.allclose(xg, xe, rtol=0, atol=1e-6) and torch.allclose(sg, se, rtol=1e-5, atol=1e-5)
     assert float(xg.abs().max()) <= 0.5 * 16 * 0.06 + 1e-6  # wrapped into the box
+
+
+@pytest.mark.parametrize("N,C", [(501, 3), (2500, 16), (1027, 8)])
+def test_inputs_of_a_recorded_step_by_one_launch_or_by_copies(N, C):
+    """Contiguous, unaligned, strided, double and host inputs end in the same buffers."""
+    from npa_b200.graphs import _load
+    g = torch.Generator(device="cuda").manual_seed(N)
+    x, s = torch.randn(1, N, 2, generator=g, device="cuda"), torch.randn(1, N, C, generator=g, device="cuda")
+    wide, shifted = torch.zeros(1, N, C + 1, device="cuda"), torch.zeros(N * C + 1, device="cuda")
+    wide[..., :C] = s
+    shifted[1:] = s.flatten()
+    for other in (s, wide[..., :C], shifted[1:].view(1, N, C), s.double(), s.cpu()):
+        x_in, s_in = torch.full_like(x, 7.0), torch.full_like(s, 7.0)
+        _load(x_in, x, s_in, other)
+        assert torch.equal(x_in, x) and torch.equal(s_in, s)
+        _load(x_in, x_in, s_in, s_in)
+        assert torch.equal(x_in, x) and torch.equal(s_in, s)
