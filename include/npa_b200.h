@@ -558,6 +558,15 @@ int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float 
                                    int64_t rows, int32_t in_dim, int32_t out_dim, int64_t w1_stride_out,
                                    int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,
                                    int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, void *stream);
+
+/* The same in two calls: the images of the weights (scratch as above, and dz_image unless NULL) made by the launch that reorders
+ * positions and states into cell order (npa_bin_particles without masses), and the two layers on images that are there. */
+int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation,
+                                 float *x_out, float *s_out, const float *W1, const float *W2, int32_t in_dim, int32_t out_dim,
+                                 int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in,
+                                 void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, void *stream);
+int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim,
+                                     int32_t out_dim, const void *scratch, int64_t scratch_bytes, void *stream);
 int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image_bytes, float *C, int64_t rows,
                                 int32_t in_dim, int32_t out_dim, void *stream);
 /* Self-test of those bounded waits: a two-warp kernel in which warp 0 waits `limit_us` (1..1,000,000)

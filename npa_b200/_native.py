@@ -93,6 +93,8 @@ SIGNATURES = {
                                           ctypes.c_double, _I32, _I32, ctypes.c_double, _P, _P, _P]),
     "npa_rollout_move": (ctypes.c_int, [_P, _P, _P, _P, _P, _I32, ctypes.c_float, _P, _P]),
     "npa_copy_pair": (ctypes.c_int, [_P, _P, _I64, _P, _P, _I64, _P]),
+    "npa_bin_particles_mlp_images": (ctypes.c_int, [_P, _I32, _P, _P, _P, _P, _P, _P, _P, _I32, _I32, _I64, _I64, _I64, _I64, _P, _I64, _P, _I64, _P]),
+    "npa_mlp_forward_tcgen05_prepared": (ctypes.c_int, [_P, _P, _P, _P, _I64, _I32, _I32, _P, _I64, _P]),
     "npa_mlp_weight_grad_scratch_floats": (ctypes.c_int64, [ctypes.c_int64, _I32, _I32]),
     "npa_mlp_weight_grad": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int64, _I32, _I32, _I32, _P, ctypes.c_int64,
                                            _P, _P, _P, _P]),

@@ -16,6 +16,7 @@
 #include <mutex>
 
 #include "ops.cuh"
+#include "weight_image.cuh"
 
 namespace npa {
 
@@ -704,11 +705,9 @@ rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ bl
 // position and the mass.  FORWARD: out[perm[i]] = in[i]; else out[i] = in[perm[i]].
 // ---------------------------------------------------------------------------
 template <int D, bool FORWARD, typename VEC>
-__global__ void __launch_bounds__(256)
-permute_kernel(const float *__restrict__ x, const float *__restrict__ s, const float *__restrict__ m,
-               const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
-               float *__restrict__ mo, int pieces, long long total, int N) {
-    after_previous_kernel();
+__device__ inline void permute_piece(const float *__restrict__ x, const float *__restrict__ s, const float *__restrict__ m,
+                                     const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
+                                     float *__restrict__ mo, int pieces, long long total, int N) {
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     if (t >= total) return;
     const long long particle = t / pieces;
@@ -733,9 +732,29 @@ permute_kernel(const float *__restrict__ x, const float *__restrict__ s, const f
     }
 }
 
+template <int D, bool FORWARD, typename VEC>
+__global__ void __launch_bounds__(256)
+permute_kernel(const float *__restrict__ x, const float *__restrict__ s, const float *__restrict__ m,
+               const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
+               float *__restrict__ mo, int pieces, long long total, int N) {
+    after_previous_kernel();
+    permute_piece<D, FORWARD, VEC>(x, s, m, perm, xo, so, mo, pieces, total, N);
+}
+
+// The reorder of a step, with the images of the MLP's weights made by blocks behind those of the particles: they have no launch of
+// their own then (2 us of a small step, and 5 us of the host).
+template <int D, typename VEC>
+__global__ void __launch_bounds__(256)
+permute_images_kernel(const float *__restrict__ x, const float *__restrict__ s, const int32_t *__restrict__ perm, float *__restrict__ xo,
+                      float *__restrict__ so, int pieces, long long total, int N, unsigned blocks, const __grid_constant__ ImageJobs jobs) {
+    after_previous_kernel();
+    if (blockIdx.x < blocks) permute_piece<D, true, VEC>(x, s, nullptr, perm, xo, so, nullptr, pieces, total, N);
+    else write_image_element(jobs, (int)(blockIdx.x - blocks) * 256 + threadIdx.x);
+}
+
 template <bool FORWARD>
 static int launch_permute(const Geom &g, int C, const float *x, const float *s, const float *m,
-                          const int32_t *perm, float *xo, float *so, float *mo, cudaStream_t st) {
+                          const int32_t *perm, float *xo, float *so, float *mo, cudaStream_t st, const ImageJobs *jobs = nullptr) {
     if (!perm) return fail(NPA_ERR_INVALID_ARGUMENT, "permutation is NULL");
     if ((x == nullptr) != (xo == nullptr) || (s == nullptr) != (so == nullptr) || (m == nullptr) != (mo == nullptr))
         return fail(NPA_ERR_INVALID_ARGUMENT, "each input of a permutation needs its output (and vice versa)");
@@ -746,6 +765,18 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     const int pieces = s ? (vec ? C / 4 : C) : 1;
     const long long total = (long long)g.B * g.N * pieces;
     const unsigned blocks = (unsigned)((total + 255) / 256);
+    if (jobs) {
+        const unsigned all = blocks + (unsigned)(jobs->total() + 255) / 256;
+#define NPA_PERMUTE(DD, VEC) \
+    launch_early(permute_images_kernel<DD, VEC>, all, 256, 0, st, x, s, perm, xo, so, pieces, total, g.N, blocks, *jobs)
+        if (g.dim == 2) {
+            if (vec) NPA_PERMUTE(2, float4); else NPA_PERMUTE(2, float);
+        } else {
+            if (vec) NPA_PERMUTE(3, float4); else NPA_PERMUTE(3, float);
+        }
+#undef NPA_PERMUTE
+        return check_launch("permute_images_kernel");
+    }
 #define NPA_PERMUTE(DD, VEC) \
     launch_early(permute_kernel<DD, FORWARD, VEC>, blocks, 256, 0, st, x, s, m, perm, xo, so, mo, pieces, total, g.N)
     if (g.dim == 2) {
@@ -755,6 +786,13 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     }
 #undef NPA_PERMUTE
     return check_launch(FORWARD ? "permute_kernel(forward)" : "permute_kernel(inverse)");
+}
+
+int bin_particles_and_images(const npa_grid *grid, int channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
+                             float *s_out, const ImageJobs &jobs, cudaStream_t stream) {
+    Geom g;
+    const int rc = make_geom(grid, &g);
+    return rc != NPA_OK ? rc : launch_permute<true>(g, channels, x, s, nullptr, permutation, x_out, s_out, nullptr, stream, &jobs);
 }
 
 // ---------------------------------------------------------------------------

@@ -28,11 +28,12 @@
 #include <mutex>
 
 #include "umma.cuh"
+#include "weight_image.cuh"
 
 namespace npa {
 
 constexpr int kUmmaRows = 128;
-constexpr int kUmmaChunk = 32;            // floats of K per stage
+constexpr int kUmmaChunk = kImageChunk;   // floats of K per stage
 constexpr int kUmmaProducerWarps = 16;
 constexpr int kUmmaEpilogueWarps = 8;     // two per quarter of the accumulator's lanes
 constexpr int kUmmaWarpMma = 8, kUmmaWarpWeights = 9, kUmmaWarpProducer0 = 10;
@@ -83,41 +84,9 @@ struct UmmaArgs {
 
 __device__ unsigned g_umma_status;
 
-// Head and tail images of one or more weight matrices, chunk by chunk, in the layout the MMA reads.  The jobs share one
-// launch: a step of a small system waits for its launches, and both layers' images (and the one the backward will
-// want) are a few microseconds of work together.
-struct ImageJob {
-    const float *W;
-    long long stride_n, stride_k;
-    int K, N, Np, nchunks;
-    float *img;
-    __host__ __device__ int total() const { return nchunks * Np * kUmmaChunk; }
-};
-constexpr int kImageJobs = 3;
-struct ImageJobs {
-    ImageJob job[kImageJobs];
-    int count;
-};
 __global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
     after_previous_kernel();
-    int at = blockIdx.x * blockDim.x + threadIdx.x;
-    for (int q = 0; q < jobs.count; ++q) {
-        const ImageJob &j = jobs.job[q];
-        const int total = j.total();
-        if (at < total) {
-            const int Np = j.Np, c = at / (Np * kUmmaChunk), rem = at - c * Np * kUmmaChunk;
-            const int n = rem / kUmmaChunk, kk = rem - n * kUmmaChunk;
-            const int k = c * kUmmaChunk + kk;
-            const float v = (n < j.N && k < j.K) ? __ldg(j.W + n * j.stride_n + k * j.stride_k) : 0.f;
-            const float head = __uint_as_float(tf32_head_bits(v));
-            float *chunk = j.img + (size_t)c * 2 * Np * kUmmaChunk;
-            const int to = umma_swizzled(n, kk);
-            chunk[to] = head;
-            chunk[Np * kUmmaChunk + to] = v - head;
-            return;
-        }
-        at -= total;
-    }
+    write_image_element(jobs, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
 template <bool FUSE>
@@ -566,10 +535,30 @@ static ImageJob image_job(const float *W, int64_t stride_out, int64_t stride_in,
     return ImageJob{W, stride_out, stride_in, in_dim, out_dim, umma_round16(out_dim), umma_chunks(in_dim), static_cast<float *>(img)};
 }
 static int launch_images(const ImageJobs &jobs, cudaStream_t st) {
-    int total = 0;
-    for (int q = 0; q < jobs.count; ++q) total += jobs.job[q].total();
-    launch_early(weight_image_kernel, (total + 255) / 256, 256, 0, st, jobs);
+    launch_early(weight_image_kernel, (jobs.total() + 255) / 256, 256, 0, st, jobs);
     return check_launch("weight_image_kernel");
+}
+
+// The images of both layers, and of W1 as the backward wants it.
+static int mlp_images(const char *me, const float *W1, const float *W2, int in_dim, int out_dim, int64_t w1_stride_out, int64_t w1_stride_in,
+                      int64_t w2_stride_out, int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes,
+                      ImageJobs *jobs) {
+    if (dz_image && ((uintptr_t)dz_image % 16 || dz_image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim)))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: dz_image must be 16-byte aligned and hold %lld bytes", me,
+                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim));
+    if (in_dim <= 0 || out_dim <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
+    if (in_dim > 1024 || out_dim > 64)
+        return fail(NPA_ERR_UNSUPPORTED, "%s: supports in_dim <= 1024 and out_dim <= 64 (hidden width 128), got %d and %d", me, in_dim, out_dim);
+    if (!W1 || !W2 || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
+    if ((uintptr_t)scratch % 16) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, h and y must be float aligned, scratch 16-byte aligned", me);
+    if (scratch_bytes < npa_mlp_forward_tcgen05_scratch_bytes(in_dim, out_dim))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: scratch holds %lld bytes, %lld needed", me, (long long)scratch_bytes,
+                    (long long)npa_mlp_forward_tcgen05_scratch_bytes(in_dim, out_dim));
+    void *w2 = (char *)scratch + npa_linear_tcgen05_scratch_bytes(in_dim, kUmmaRows);
+    *jobs = {{image_job(W1, w1_stride_out, w1_stride_in, in_dim, kUmmaRows, scratch),
+              image_job(W2, w2_stride_out, w2_stride_in, kUmmaRows, out_dim, w2)}, 2};
+    if (dz_image) jobs->job[jobs->count++] = image_job(W1, w1_stride_in, w1_stride_out, kUmmaRows, in_dim, dz_image);
+    return NPA_OK;
 }
 
 }  // namespace npa
@@ -643,13 +632,36 @@ int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float 
                                    int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes,
                                    void *stream) {
     const char *me = "npa_mlp_forward_tcgen05";
-    if (dz_image && ((uintptr_t)dz_image % 16 || dz_image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim)))
-        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: dz_image must be 16-byte aligned and hold %lld bytes", me,
-                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim));
+    ImageJobs jobs;
+    int rc = mlp_images(me, W1, W2, in_dim, out_dim, w1_stride_out, w1_stride_in, w2_stride_out, w2_stride_in, scratch, scratch_bytes, dz_image,
+                        dz_image_bytes, &jobs);
+    if (rc != NPA_OK) return rc;
+    if (rows <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
+    if (!z || !y) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
+    if ((uintptr_t)z % 4 || (uintptr_t)h % 4 || (uintptr_t)y % 4)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, h and y must be float aligned, scratch 16-byte aligned", me);
+    if ((rc = launch_images(jobs, (cudaStream_t)stream)) != NPA_OK) return rc;
+    return npa_mlp_forward_tcgen05_prepared(z, b1, h, y, rows, in_dim, out_dim, scratch, scratch_bytes, stream);
+}
+
+int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
+                                 float *s_out, const float *W1, const float *W2, int32_t in_dim, int32_t out_dim, int64_t w1_stride_out,
+                                 int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch, int64_t scratch_bytes,
+                                 void *dz_image, int64_t dz_image_bytes, void *stream) {
+    ImageJobs jobs;
+    const int rc = mlp_images("npa_bin_particles_mlp_images", W1, W2, in_dim, out_dim, w1_stride_out, w1_stride_in, w2_stride_out, w2_stride_in,
+                              scratch, scratch_bytes, dz_image, dz_image_bytes, &jobs);
+    if (rc != NPA_OK) return rc;
+    return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream);
+}
+
+int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim, int32_t out_dim,
+                                     const void *scratch, int64_t scratch_bytes, void *stream) {
+    const char *me = "npa_mlp_forward_tcgen05";
     if (rows <= 0 || in_dim <= 0 || out_dim <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
     if (in_dim > 1024 || out_dim > 64)
         return fail(NPA_ERR_UNSUPPORTED, "%s: supports in_dim <= 1024 and out_dim <= 64 (hidden width 128), got %d and %d", me, in_dim, out_dim);
-    if (!z || !W1 || !W2 || !y || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
+    if (!z || !y || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
     if ((uintptr_t)z % 4 || (uintptr_t)h % 4 || (uintptr_t)y % 4 || (uintptr_t)scratch % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, h and y must be float aligned, scratch 16-byte aligned", me);
     if (scratch_bytes < npa_mlp_forward_tcgen05_scratch_bytes(in_dim, out_dim))
@@ -670,13 +682,9 @@ int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float 
     if (a.stages > kUmmaMaxStages) a.stages = kUmmaMaxStages;
     if (a.stages < 2) return fail(NPA_ERR_UNSUPPORTED, "%s: no room for two stages", me);
     const size_t smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
-    int rc = umma_device_setup((int)smem, true, &a.status);
+    const int rc = umma_device_setup((int)smem, true, &a.status);
     if (rc != NPA_OK) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    ImageJobs jobs = {{image_job(W1, w1_stride_out, w1_stride_in, in_dim, kUmmaRows, scratch),
-                       image_job(W2, w2_stride_out, w2_stride_in, kUmmaRows, out_dim, (void *)a.W2img)}, 2};
-    if (dz_image) jobs.job[jobs.count++] = image_job(W1, w1_stride_in, w1_stride_out, kUmmaRows, in_dim, dz_image);
-    if ((rc = launch_images(jobs, st)) != NPA_OK) return rc;
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
     launch_early(linear_umma_kernel<true>, ctas, kUmmaThreads, smem, st, a);

@@ -834,11 +834,11 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     float *t = fmut(slab), *x_bin = t + o_x, *s_bin = t + o_s, *rho = t + o_rho, *rho_grad = t + o_dg, *z = t + o_z, *packed = t + o_packed,
           *y = t + o_y, *vgrad = back ? t + o_v : nullptr, *h = record ? t + o_h : nullptr, *dz_image = dz_bytes ? t + o_dz : nullptr;
     int32_t *pairs = reinterpret_cast<int32_t *>(t + o_pairs);
-    check_status(npa_bin_particles(&g.g, (int)C, fptr(x), fptr(s), nullptr, iptr(perm), x_bin, s_bin, nullptr, st));
+    check_status(npa_bin_particles_mlp_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), (int)k, (int)o, w1.stride(0),
+                                              w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
     check_status(npa_perceive_features_forward_lists(&g.g, (int)C, x_bin, nullptr, s_bin, (float)coef, (float)dg_scale, (float)inv_tol, ln_grad, ln_dg,
                                                      rho, rho_grad, z, vgrad, packed, iptr(offs), iptr(info), pairs, (int)columns, st));
-    check_status(npa_mlp_forward_tcgen05_images(z, fptr(w1), fptr(b1), fptr(w2), h, y, m, (int)k, (int)o, w1.stride(0), w1.stride(1), w2.stride(0),
-                                                w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
+    check_status(npa_mlp_forward_tcgen05_prepared(z, fptr(b1), h, y, m, (int)k, (int)o, t + o_image, bytes, st));
     Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();
     Tensor xo = blank(x), so = blank(s);
     check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, y, x_bin, s_bin, fptr(mask), (float)update_prob, (int)C, (float)alpha, (float)dt,

@@ -1,0 +1,57 @@
+// Images of weight matrices as the tensor-memory kernels of the MLP read them (mlp_tcgen05.cu).
+#pragma once
+#include "common.cuh"
+#include "umma.cuh"
+
+namespace npa {
+
+constexpr int kImageChunk = 32;  // floats of K per chunk
+
+// Head and tail images of one or more weight matrices, chunk by chunk, in the layout the MMA reads.  The jobs share one
+// launch: a step of a small system waits for its launches, and both layers' images (and the one the backward will
+// want) are a few microseconds of work together.  A whole step lets the reorder of its particles make them
+// (bin_particles_and_images).
+struct ImageJob {
+    const float *W;
+    long long stride_n, stride_k;
+    int K, N, Np, nchunks;
+    float *img;
+    __host__ __device__ int total() const { return nchunks * Np * kImageChunk; }
+};
+constexpr int kImageJobs = 3;
+struct ImageJobs {
+    ImageJob job[kImageJobs];
+    int count;
+    int total() const {
+        int n = 0;
+        for (int q = 0; q < count; ++q) n += job[q].total();
+        return n;
+    }
+};
+
+// Element `at` of all jobs together; nothing beyond the last.
+__device__ inline void write_image_element(const ImageJobs &jobs, int at) {
+    for (int q = 0; q < jobs.count; ++q) {
+        const ImageJob &j = jobs.job[q];
+        const int total = j.total();
+        if (at < total) {
+            const int Np = j.Np, c = at / (Np * kImageChunk), rem = at - c * Np * kImageChunk;
+            const int n = rem / kImageChunk, kk = rem - n * kImageChunk;
+            const int k = c * kImageChunk + kk;
+            const float v = (n < j.N && k < j.K) ? __ldg(j.W + n * j.stride_n + k * j.stride_k) : 0.f;
+            const float head = __uint_as_float(tf32_head_bits(v));
+            float *chunk = j.img + (size_t)c * 2 * Np * kImageChunk;
+            const int to = umma_swizzled(n, kk);
+            chunk[to] = head;
+            chunk[Np * kImageChunk + to] = v - head;
+            return;
+        }
+        at -= total;
+    }
+}
+
+// binning.cu: npa_bin_particles (without masses) whose launch also makes the images.
+int bin_particles_and_images(const npa_grid *grid, int channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
+                             float *s_out, const ImageJobs &jobs, cudaStream_t stream);
+
+}  // namespace npa
