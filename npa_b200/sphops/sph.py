@@ -155,6 +155,11 @@ def _columns(grid):
     return grid.list_columns if set_by_user is None else set_by_user
 
 
+def _roomy_columns(grid):
+    set_by_user = _PAIR_CACHE["columns"]
+    return grid.roomy_list_columns if set_by_user is None else set_by_user
+
+
 def _lists_of(snapshot, x_bin):
     """Neighbour lists recorded on this snapshot for the very same positions object, or None."""
     return snapshot.lists[1] if snapshot.lists is not None and _same(snapshot.lists[0], x_bin) else None
@@ -166,7 +171,7 @@ def _density(x_bin, mass, snapshot, want_density_gradient):
     kernel that writes through the pointer, ``.data``), and then the density is computed anew as well.  The snapshot
     gets the lists when the sweep that fills them has been issued, never before."""
     key = _key(x_bin)
-    columns = _columns(snapshot.grid) if key is not None else 0
+    columns = _roomy_columns(snapshot.grid) if key is not None else 0
     pairs = torch.empty(*x_bin.shape[:2], columns, dtype=torch.int32, device=x_bin.device) if columns else None
     out = _ops.density(*_sweep_args(snapshot), x_bin, mass, pairs, True, want_density_gradient, columns > 0)
     snapshot.lists = (key, pairs) if columns else None
@@ -361,7 +366,7 @@ class Perception:
 
     @staticmethod
     def apply(x_bin, s_bin, mass, snapshot, want_density_gradient):
-        return _ops.perception(*_sweep_args(snapshot), x_bin, s_bin, mass, want_density_gradient, _columns(snapshot.grid))
+        return _ops.perception(*_sweep_args(snapshot), x_bin, s_bin, mass, want_density_gradient, _roomy_columns(snapshot.grid))
 
 
 def perceive(x_bin, s_bin, snapshot, mass=None, with_density_gradient=True):

@@ -86,7 +86,7 @@ class _HashGridBase:
 
     def _bind(self):
         self.native = N.ops.Grid(ctypes.addressof(self._desc))  # what the autograd nodes take (csrc/torch_ops.cpp)
-        self.list_columns  # here rather than in the first step
+        self.list_columns, self.roomy_list_columns  # here rather than in the first step
 
     # copies and pickles carry the description; the native handle is made anew
     def __getstate__(self):
@@ -103,6 +103,16 @@ class _HashGridBase:
         that long-range grids -- 128 neighbours in a 10 x 10 periodic box of 4,096 particles -- fit as well."""
         mean = (3.14159265 if self._dim == 2 else 4.18879020) * self._N / self._cells
         return 128 if mean <= 79 else min(512, -(-int(1.6 * mean + 1) // 64) * 64)
+
+    @functools.cached_property
+    def roomy_list_columns(self):
+        """Columns for sweeps whose order of sums does not depend on the length of the lists: where 128 is the rule, as many
+        more as 128 MiB of lists leave, at most 512.  A particle that does not fit searches its cells at several times the cost of a
+        list: 8 x 16,384 particles in 2D clusters, one in forty of them with 128 to 188 neighbours where the mean is 56, forward 163
+        -> 113 us and full backward 446 -> 344; without such particles the longer rows cost nothing (177 and 640 us in 3D either way)."""
+        if self.list_columns > 128:
+            return self.list_columns
+        return max(128, min(512, (128 << 20) // (4 * self._B * self._N) // 64 * 64))
 
     # ---- read-only properties of the nanobind classes ----------------------
     grid_size_x = property(lambda self: self._sizes[0])

@@ -100,3 +100,35 @@ def test_spiky_kernel_of_single_pairs():
     # relative: rounding of q and d (2^-24 each, doubled by the square and amplified by d / (h - d)) and of six operations
     bound = 2.0 ** -24 * (8.0 + 4.0 * d / (hf - d))
     assert (np.abs(got - want) <= bound[:, None] * np.abs(want).max(axis=1, keepdims=True)).all()
+
+
+@pytest.mark.parametrize("dim,C", [(3, 32), (3, 16), (2, 13), (3, 20)])
+def test_full_backward_with_particles_of_no_mass_and_crowded_lists(dim, C):
+    """Lists of the default length (longer than 128 where memory allows) against sweeps that search: gradients of particles without
+    mass, whose volume is zero, and of clusters with more than 127 neighbours.  The searching backward divides by the mass: there the
+    particles weigh 1e-20, which changes no sum."""
+    from npa_b200 import sphops as sph
+    N = 3000
+    grid = sph.HashGrid(dim=dim, boundary="clamped", mode="grid", grid_size=(8,) * dim, eps=0.125, num_particles=N, batch_size=1)
+    assert grid.hashgrid.roomy_list_columns == (512 if grid.hashgrid.list_columns == 128 else grid.hashgrid.list_columns)
+    g = torch.Generator().manual_seed(C)
+    x = torch.rand(1, N, 2 if dim == 2 else 4, generator=g) - 0.5
+    x[:, : N // 4, :dim] *= 0.3
+    mass = 0.5 + torch.rand(1, N, generator=g)
+    mass[:, ::7] = 0.0
+    s = torch.randn(1, N, C, generator=g)
+    ups = [torch.randn(1, N, *t, generator=g).cuda() for t in ((), (C,), (C, dim), (dim,))]
+    got = []
+    for columns in (None, 0):
+        sph.set_pair_cache(columns)
+        try:
+            xr, sr = x.cuda().requires_grad_(True), s.cuda().requires_grad_(True)
+            snap = grid.instantiate(xr)
+            xb, sb, mb = sph.bin_particles(xr, sr, snap, mass.clamp(min=0.0 if columns is None else 1e-20).cuda())
+            out = sph.perceive(xb, sb, snap, mb)
+            got.append([*(t.detach() for t in out), *torch.autograd.grad(out, [xr, sr], ups)])
+        finally:
+            sph.set_pair_cache(None)
+    # two fp32 sums of up to a few hundred terms in different orders: 2e-5 of the largest value
+    for a, b in zip(*got):
+        assert torch.isfinite(a).all() and float((a - b).abs().max()) <= 2e-5 * float(b.abs().max())
