@@ -40,6 +40,13 @@ class VelocityField:
         return torch.sin(arg) @ self.amp
 
 
+def _writable(t):
+    """Whether a kernel may write ``t`` where autograd knows nothing of it: a leaf or a view that requires a gradient, and
+    an inference tensor outside inference mode, are left to the operations of torch, which refuse what is not allowed."""
+    recorded = t.requires_grad or (t._base is not None and t._base.requires_grad)
+    return not recorded and (torch.is_inference_mode_enabled() or not t.is_inference())
+
+
 def _written(t):
     """Autograd's note of a change in place, as a torch operation would leave it."""
     if not t.is_inference():
@@ -88,9 +95,14 @@ class PerceptionRollout:
         self.launches = self.steps * 9 + 4 + (self.steps - 1 if self._native_move() else 0)
 
     def _native_move(self):
-        v = self.velocity
-        return (type(v) is VelocityField and v.dim == self.grid.dim and 1 <= v.phase.numel() <= 64
-                and all(t.dtype == torch.float32 and t.is_contiguous() and t.device == self.x_bin.device for t in (v.k_t, v.phase, v.amp)))
+        """Whether the move kernel computes this field: parameters of the shapes that it reads, as plain memory, and without a
+        gradient (the tensor operations raise on other shapes, and record what requires one)."""
+        v, D = self.velocity, self.grid.dim
+        if type(v) is not VelocityField or v.dim != D or v.phase.dim() != 1 or not 1 <= v.phase.numel() <= 64:
+            return False
+        shapes = ((D, v.phase.numel()), v.phase.shape, (v.phase.numel(), D))
+        return all(t.shape == shape and t.dtype == torch.float32 and t.is_contiguous() and t.device == self.x_bin.device
+                   and not t.requires_grad and not t.is_neg() for t, shape in zip((v.k_t, v.phase, v.amp), shapes))
 
     def _forward(self, x, s, s_bin):
         hg = self.hg
@@ -107,7 +119,7 @@ class PerceptionRollout:
     def _move(self, x):
         """x <- wrap(x_bin + dt * v(x_bin)): the particles continue in cell order."""
         D, v = self.grid.dim, self.velocity
-        if self._native_move() and not x.requires_grad:
+        if self._native_move() and _writable(x):
             self.hg._call(N.lib.npa_rollout_move, x, self.hg._ref(), N.ptr(self.x_bin), N.ptr(v.k_t), N.ptr(v.phase), N.ptr(v.amp),
                           v.phase.numel(), self.dt, N.ptr(x))
             _written(x)
@@ -130,7 +142,7 @@ class PerceptionRollout:
             if last:
                 break
             self._move(x)
-            if s.requires_grad or s.data_ptr() == self.s_bin.data_ptr() or (k == 0 and self.steps % 2 == 0):
+            if not _writable(s) or s.data_ptr() == self.s_bin.data_ptr() or (k == 0 and self.steps % 2 == 0):
                 s.copy_(self.s_bin)
             else:
                 source, target = target, source

@@ -55,26 +55,28 @@ def test_rollout_matches_the_public_api_loop(w):
 
 
 @pytest.mark.parametrize("steps", [1, 2, 3])
-@pytest.mark.parametrize("dim,N,boundary,modes", [(3, 20011, "periodic", 8), (2, 1001, "periodic", 64), (3, 515, "clamped", 8)])
-def test_the_native_move_gives_the_bits_of_the_tensor_operations(dim, N, boundary, modes, steps):
+@pytest.mark.parametrize("dim,N,boundary,modes,cells,eps,dt", [
+    (3, 20011, "periodic", 8, 8, 0.125, 0.3), (2, 1001, "periodic", 64, 8, 0.125, 0.3), (3, 515, "clamped", 8, 8, 0.125, 0.3),
+    (2, 1501, "periodic", 8, 9, 0.1, 5.0), (3, 3001, "periodic", 8, 24, 0.0879, 20.0)])
+def test_the_native_move_gives_the_bits_of_the_tensor_operations(dim, N, boundary, modes, cells, eps, dt, steps):
     """A rollout whose velocity field is not the built-in type moves by tensor operations and copies the states: the same positions
-    (bit for bit, or particles would change cells), states, outputs and gradients, with an odd and an even number of steps."""
+    (bit for bit, or particles would change cells), states, outputs and gradients, with an odd and an even number of steps.  The last
+    two boxes have lengths that are rounded, and moves of several lengths."""
     from npa_b200 import sphops as sph
     from npa_b200.rollout import PerceptionRollout, VelocityField
 
     class Another(VelocityField):
         pass
 
-    cells = 8
-    grid = sph.HashGrid(dim=dim, boundary=boundary, mode="grid", grid_size=(cells,) * dim, eps=0.125, num_particles=N, batch_size=2)
+    grid = sph.HashGrid(dim=dim, boundary=boundary, mode="grid", grid_size=(cells,) * dim, eps=eps, num_particles=N, batch_size=2)
     g = torch.Generator(device="cuda").manual_seed(N)
-    x0 = torch.rand(2, N, 2 if dim == 2 else 4, generator=g, device="cuda") - 0.5
+    x0 = (torch.rand(2, N, 2 if dim == 2 else 4, generator=g, device="cuda") - 0.5) * (cells * eps)
     s0 = torch.randn(2, N, 8, generator=g, device="cuda")
     ups = {"g_rho": torch.randn(2, N, generator=g, device="cuda"), "g_blur": torch.randn(2, N, 8, generator=g, device="cuda"),
            "g_grad": torch.randn(2, N, 8, dim, generator=g, device="cuda")}
     got = []
     for field in (VelocityField, Another):
-        roll = PerceptionRollout(grid, 8, steps, 0.3, field(dim, x0.device, seed=1, modes=modes))
+        roll = PerceptionRollout(grid, 8, steps, dt, field(dim, x0.device, seed=1, modes=modes))
         x, s = x0.clone(), s0.clone()
         versions = x._version, s._version
         grads = roll.run(x, s, ups)
@@ -82,3 +84,36 @@ def test_the_native_move_gives_the_bits_of_the_tensor_operations(dim, N, boundar
         got.append([t.clone() for t in (x, s, roll.x_bin, roll.s_bin, roll.rho, roll.blur, roll.grad, *grads)])
     for a, b in zip(*got):
         assert torch.equal(a, b)
+
+
+def test_fields_and_tensors_that_the_move_kernel_does_not_take():
+    """A phase that torch broadcasts over the modes moves as torch moves it, parameters of other shapes raise as in torch, and
+    positions that may not be written in place are refused."""
+    from npa_b200 import sphops as sph
+    from npa_b200.rollout import PerceptionRollout, VelocityField
+
+    class Another(VelocityField):
+        pass
+
+    grid = sph.HashGrid(dim=2, boundary="periodic", mode="grid", grid_size=(8, 8), eps=0.125, num_particles=300, batch_size=1)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    x0, s0 = torch.rand(1, 300, 2, generator=g, device="cuda") - 0.5, torch.randn(1, 300, 4, generator=g, device="cuda")
+    ups = {"g_rho": torch.randn(1, 300, generator=g, device="cuda"), "g_blur": torch.randn(1, 300, 4, generator=g, device="cuda"),
+           "g_grad": torch.randn(1, 300, 4, 2, generator=g, device="cuda")}
+    moved = []
+    for kind in (VelocityField, Another):
+        field = kind(2, x0.device, seed=1)
+        field.phase = field.phase[:1].clone()
+        x = x0.clone()
+        PerceptionRollout(grid, 4, 2, 0.3, field).run(x, s0.clone(), ups)
+        moved.append(x)
+    assert torch.equal(*moved)
+    for name, shape in (("phase", (9,)), ("k_t", (2, 7)), ("amp", (7, 2))):
+        field = VelocityField(2, x0.device, seed=1)
+        setattr(field, name, torch.zeros(shape, device="cuda"))
+        with pytest.raises(RuntimeError):
+            PerceptionRollout(grid, 4, 2, 0.3, field).run(x0.clone(), s0.clone(), ups)
+    with torch.inference_mode():
+        frozen = x0.clone()
+    with pytest.raises(RuntimeError, match="[Ii]nference"):
+        PerceptionRollout(grid, 4, 2, 0.3, VelocityField(2, x0.device, seed=1)).run(frozen, s0.clone(), ups)

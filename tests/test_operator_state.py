@@ -130,3 +130,40 @@ def test_forward_mode_derivatives_are_refused():
         for name, args in calls.items():
             with pytest.raises(NotImplementedError, match="forward-mode"):
                 getattr(_native.ops, name)(*args)
+
+
+def test_the_move_kernel_takes_only_fields_of_the_shapes_it_reads():
+    """The kernel reads dim x modes products and phases by pointer: parameters that torch would broadcast, refuse or record stay
+    with the tensor operations."""
+    from npa_b200.rollout import PerceptionRollout, VelocityField, _writable
+
+    class Another(VelocityField):
+        pass
+
+    def native(change=lambda field: None, kind=VelocityField, modes=8):
+        field = kind(2, torch.device("cpu"), modes=modes)
+        roll = PerceptionRollout(_grid(), 4, 2, 0.1, field)
+        change(field)
+        return roll._native_move()
+
+    assert native() and native(modes=64)
+    assert not native(modes=65) and not native(kind=Another)
+    assert not native(lambda f: setattr(f, "phase", f.phase[:1]))            # broadcast over the modes
+    assert not native(lambda f: setattr(f, "phase", torch.zeros(9)))
+    assert not native(lambda f: setattr(f, "phase", f.phase.view(2, 4)))
+    assert not native(lambda f: setattr(f, "k_t", f.k_t[:, :7].contiguous()))
+    assert not native(lambda f: setattr(f, "k_t", torch.zeros(3, 8)))
+    assert not native(lambda f: setattr(f, "amp", torch.zeros(7, 2)))
+    assert not native(lambda f: setattr(f, "amp", f.amp.t().contiguous()))
+    assert not native(lambda f: setattr(f, "amp", f.amp.double()))
+    assert not native(lambda f: f.amp.requires_grad_(True))
+    assert not native(lambda f: setattr(f, "amp", torch._neg_view(f.amp)))
+    # positions and states
+    x = torch.zeros(2, 3)
+    with torch.inference_mode():
+        inference = torch.zeros(2, 3)
+        assert _writable(inference)
+    leaf = torch.zeros(2, 3, requires_grad=True)
+    with torch.no_grad():
+        view = leaf[:1]
+    assert _writable(x) and _writable(x[:1]) and not _writable(inference) and not _writable(leaf) and not _writable(view)
