@@ -15,11 +15,24 @@ from . import _native as N
 from . import sphops as sph
 
 
+def _plain(t, buf):
+    """Whether ``buf <- t`` is a copy of memory that a kernel can make by pointer: no conversion, no view that negates, no subclass
+    without memory of its own."""
+    return ((type(t) is torch.Tensor or type(t) is torch.nn.Parameter) and t.dtype == torch.float32 and t.device == buf.device
+            and t.shape == buf.shape and t.is_contiguous() and not t.is_neg() and t.data_ptr() % 16 == 0)
+
+
+def _apart(*tensors):
+    """Whether no two of these contiguous float tensors share memory."""
+    ends = sorted((t.data_ptr(), t.data_ptr() + 4 * t.numel()) for t in tensors)
+    return ends[0][0] != 0 and all(a[1] <= b[0] for a, b in zip(ends, ends[1:]))
+
+
 def _load(x_in, x, s_in, s):
-    """``x_in <- x, s_in <- s``: one launch where both are plain copies on the current device, else ``copy_``."""
-    plain = all(t.dtype == torch.float32 and t.is_contiguous() and t.device == buf.device and t.shape == buf.shape and t.data_ptr() % 16 == 0
-                and t.data_ptr() != buf.data_ptr() for t, buf in ((x, x_in), (s, s_in)))
-    if plain and x_in.device.index == torch.cuda.current_device() and s.numel() > 0:
+    """``x_in <- x, s_in <- s``: one launch where both are plain copies on the current device, else ``copy_``, one after the other
+    (what overlaps the buffers, such as the buffers themselves in each other's place, has an order then)."""
+    if (_plain(x, x_in) and _plain(s, s_in) and s.numel() > 0 and x_in.device.index == torch.cuda.current_device()
+            and _apart(x_in, s_in, x) and _apart(x_in, s_in, s)):
         N.check(N.lib.npa_copy_pair(N.ptr(x), N.ptr(x_in), x.numel(), N.ptr(s), N.ptr(s_in), s.numel(), N.current_stream()))
         return
     x_in.copy_(x, non_blocking=True)

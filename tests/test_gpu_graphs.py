@@ -67,3 +67,19 @@ def test_inputs_of_a_recorded_step_by_one_launch_or_by_copies(N, C):
         assert torch.equal(x_in, x) and torch.equal(s_in, s)
         _load(x_in, x_in, s_in, s_in)
         assert torch.equal(x_in, x) and torch.equal(s_in, s)
+
+
+def test_inputs_of_a_recorded_step_that_are_not_plain_memory():
+    """Negated views and inputs that lie in the buffers are copied as torch copies them, one after the other."""
+    from npa_b200.graphs import _load
+    g = torch.Generator(device="cuda").manual_seed(9)
+    x, s = torch.randn(1, 4096, 2, generator=g, device="cuda"), torch.randn(1, 4096, 2, generator=g, device="cuda")
+    x_in, s_in = torch.zeros_like(x), torch.zeros_like(s)
+    _load(x_in, torch._neg_view(x), s_in, torch._neg_view(s))
+    assert torch.equal(x_in, -x) and torch.equal(s_in, -s)
+    _load(x_in, x, s_in, s)
+    for _ in range(20):  # the buffers in each other's place: the first is written before the second is read
+        x_in.copy_(x)
+        s_in.copy_(s)
+        _load(x_in, s_in, s_in, x_in)
+        assert torch.equal(x_in, s) and torch.equal(s_in, s)
