@@ -89,8 +89,9 @@ __global__ void __launch_bounds__(256) splat_scale_kernel(SplatArgs a) {
 // culled with a pixel to spare into a list (a thread's hits in a row, threads in order); 64 at a time get their 16 + 16
 // factors in shared memory (32 exponentials per particle and tile instead of 256; eight per thread) while the 64 before are
 // multiplied; every half warp multiplies every 16th particle into 8 x 2 pixels x 4 channels per thread in packed fp32x2, two
-// neighbouring pixels to a pair; the 16 partial images are added in a fixed order.  SLICED: the CTAs of a cluster share the tile,
-// each with a slice of the particles, and add their images through distributed shared memory, slices in order.
+// neighbouring pixels to a pair; the 16 partial images are added in a fixed order.  kCluster: the CTAs of a cluster share the tile,
+// each with a slice of the particles, and add their images through distributed shared memory, slices in order.  kTurns: one CTA takes
+// the slices one after the other and adds in the same order, so that either gives the same bits.
 // Bound by latency (fill of the list, first factors, sum of the partial images) at two blocks per SM: 45 % of the issue slots,
 // fp32 pipe 22 %.  8 systems of 4,096 particles, 256 x 256, patches of 41 x 41, us: pixel by pixel 201; list of 1,024
 // particles at a time, factors and products between barriers, channels packed (wants every column factor twice) 113; this 86.  64 x 64,
@@ -117,25 +118,24 @@ union SplatShared {
 // layout (4,096 tiles with a few particles each: 67 us, so 48).
 __device__ inline int part_at(int pixel) { return pixel ^ ((pixel >> 5) & 7); }
 
-template <bool SLICED>
-__global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatArgs a) {
+enum class SplatSlices { kOne, kCluster, kTurns };
+
+template <SplatSlices SLICES>
+__global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatArgs a, int slices) {
     after_previous_kernel();
+    constexpr bool CLUSTER = SLICES == SplatSlices::kCluster, TURNS = SLICES == SplatSlices::kTurns;
     __shared__ SplatShared sh;
     __shared__ int s_count[kSplatWarps];
+    __shared__ float4 s_sum[TURNS ? kSplatThreads : 1];  // a pixel's sum over the slices so far (registers are all taken)
     const int tiles = (a.img + kSplatTile - 1) / kSplatTile;
-    const int slices = SLICED ? (int)cg::this_cluster().num_blocks() : 1, slice = SLICED ? blockIdx.x % slices : 0, tile = blockIdx.x / slices;
+    if (SLICES == SplatSlices::kOne) slices = 1;
+    const int mine = CLUSTER ? blockIdx.x % slices : 0, tile = CLUSTER ? blockIdx.x / slices : blockIdx.x;
     const int tx0 = (tile % tiles) * kSplatTile, ty0 = (tile / tiles) * kSplatTile;
     const int b = blockIdx.y, r = a.radius;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     const int part = tid >> 4, cell = tid & 15, px = (cell & 1) * 8, py = (cell >> 1) * 2;  // pixels px..px+7, py..py+1
     const float inv2s2 = 1.0f / (2.0f * a.sigma * a.sigma);
     unsigned long long acc[2][4][4];  // [row][channel][two pixels]
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int c = 0; c < 4; ++c)
-#pragma unroll
-            for (int x = 0; x < 4; ++x) acc[y][c][x] = 0ull;
 
     // What a thread needs to make eight factors of one axis of a particle: loaded a chunk ahead.
     const int sp = tid >> 2, axis = (tid >> 1) & 1, o0 = (tid & 1) * 8;
@@ -214,78 +214,94 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
 
     const float top = (float)(a.img - 1), per = top / a.span, reach = (float)r + 9.25f;  // patch radius, half a tile, a pixel, rounding
     const float mx = (float)tx0 + 7.5f, my = (float)ty0 + 7.5f;
-    const int share = (a.N + slices - 1) / slices, end = min(a.N, (slice + 1) * share);
-    for (int n0 = slice * share; n0 < end; n0 += kSplatWindow) {
-        unsigned hits = 0;
+    const int share = (a.N + slices - 1) / slices;
+    float4 v;
+    for (int slice = mine; slice < (TURNS ? slices : mine + 1); ++slice) {
+#pragma unroll
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int c = 0; c < 4; ++c)
+#pragma unroll
+                for (int x = 0; x < 4; ++x) acc[y][c][x] = 0ull;
+        const int end = min(a.N, (slice + 1) * share);
+        for (int n0 = slice * share; n0 < end; n0 += kSplatWindow) {
+            unsigned hits = 0;
 #pragma unroll 8
-        for (int q = 0; q < kSplatCull; ++q) {
-            const int n = n0 + q * kSplatThreads + tid;
-            if (n < end) {
-                const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + (long long)b * a.N + n);
-                const float x = (v.x - a.lo) * per;
-                float y = (v.y - a.lo) * per;
-                if (a.y_up) y = top - y;
-                if (fabsf(x - mx) <= reach && fabsf(y - my) <= reach) hits |= 1u << q;
+            for (int q = 0; q < kSplatCull; ++q) {
+                const int n = n0 + q * kSplatThreads + tid;
+                if (n < end) {
+                    const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + (long long)b * a.N + n);
+                    const float x = (v.x - a.lo) * per;
+                    float y = (v.y - a.lo) * per;
+                    if (a.y_up) y = top - y;
+                    if (fabsf(x - mx) <= reach && fabsf(y - my) <= reach) hits |= 1u << q;
+                }
+            }
+            int incl = __popc(hits);
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const int v = __shfl_up_sync(0xffffffffu, incl, o);
+                if (lane >= o) incl += v;
+            }
+            if (lane == 31) s_count[warp] = incl;
+            __syncthreads();  // (also: the window before has read its list and factors)
+            int at = incl - __popc(hits), count = 0;
+#pragma unroll
+            for (int w = 0; w < kSplatWarps; ++w) {
+                const int c = s_count[w];
+                if (w < warp) at += c;
+                count += c;
+            }
+            for (; hits; hits &= hits - 1) sh.lists.n[at++] = (unsigned short)((__ffs(hits) - 1) * kSplatThreads + tid);
+            __syncthreads();
+            fetch(n0, 0, count);
+            for (int off = 0, buf = 0; off < count; off += kSplatChunk, buf ^= 1) {
+                const bool odd = factors(sh.lists.f[buf], off, count);
+                fetch(n0, off + kSplatChunk, count);
+                const bool any_odd = __syncthreads_or(odd);  // (also: the chunk before the last has left its buffer)
+                multiply(sh.lists.f[buf], min(kSplatChunk, (count - off + kSplatParts - 1) / kSplatParts * kSplatParts), any_odd);
             }
         }
-        int incl = __popc(hits);
+        __syncthreads();
+        // the two halves of a warp meet by shuffles, the eight warps in shared memory
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int v = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += v;
-        }
-        if (lane == 31) s_count[warp] = incl;
-        __syncthreads();  // (also: the window before has read its list and factors)
-        int at = incl - __popc(hits), count = 0;
+        for (int y = 0; y < 2; ++y)
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {
+                float v[2][4];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    unpack2(acc[y][k][x], v[0][k], v[1][k]);
+                    v[0][k] += __shfl_xor_sync(0xffffffffu, v[0][k], 16);
+                    v[1][k] += __shfl_xor_sync(0xffffffffu, v[1][k], 16);
+                }
+                // each half stores one of the two pixels
+                const int h = lane >> 4;
+                sh.part[warp][part_at((py + y) * kSplatTile + px + 2 * x + h)] =
+                    make_float4(h ? v[1][0] : v[0][0], h ? v[1][1] : v[0][1], h ? v[1][2] : v[0][2], h ? v[1][3] : v[0][3]);
+            }
+        __syncthreads();
+        v = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll
         for (int w = 0; w < kSplatWarps; ++w) {
-            const int c = s_count[w];
-            if (w < warp) at += c;
-            count += c;
+            const float4 q = sh.part[w][part_at(tid)];
+            v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
         }
-        for (; hits; hits &= hits - 1) sh.lists.n[at++] = (unsigned short)((__ffs(hits) - 1) * kSplatThreads + tid);
-        __syncthreads();
-        fetch(n0, 0, count);
-        for (int off = 0, buf = 0; off < count; off += kSplatChunk, buf ^= 1) {
-            const bool odd = factors(sh.lists.f[buf], off, count);
-            fetch(n0, off + kSplatChunk, count);
-            const bool any_odd = __syncthreads_or(odd);  // (also: the chunk before the last has left its buffer)
-            multiply(sh.lists.f[buf], min(kSplatChunk, (count - off + kSplatParts - 1) / kSplatParts * kSplatParts), any_odd);
+        // (the next turn's list overwrites the partial images only behind a barrier that follows these reads)
+        if (TURNS) {
+            const float4 before = slice ? s_sum[tid] : make_float4(0.f, 0.f, 0.f, 0.f);
+            v = make_float4(before.x + v.x, before.y + v.y, before.z + v.z, before.w + v.w);
+            s_sum[tid] = v;
         }
-    }
-    __syncthreads();
-    // the two halves of a warp meet by shuffles, the eight warps in shared memory
-#pragma unroll
-    for (int y = 0; y < 2; ++y)
-#pragma unroll
-        for (int x = 0; x < 4; ++x) {
-            float v[2][4];
-#pragma unroll
-            for (int k = 0; k < 4; ++k) {
-                unpack2(acc[y][k][x], v[0][k], v[1][k]);
-                v[0][k] += __shfl_xor_sync(0xffffffffu, v[0][k], 16);
-                v[1][k] += __shfl_xor_sync(0xffffffffu, v[1][k], 16);
-            }
-            // each half stores one of the two pixels
-            const int h = lane >> 4;
-            sh.part[warp][part_at((py + y) * kSplatTile + px + 2 * x + h)] =
-                make_float4(h ? v[1][0] : v[0][0], h ? v[1][1] : v[0][1], h ? v[1][2] : v[0][2], h ? v[1][3] : v[0][3]);
-        }
-    __syncthreads();
-    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll
-    for (int w = 0; w < kSplatWarps; ++w) {
-        const float4 q = sh.part[w][part_at(tid)];
-        v.x += q.x; v.y += q.y; v.z += q.z; v.w += q.w;
     }
     int pixel = tid;
-    if (SLICED) {
+    if (CLUSTER) {
         // every CTA of the cluster adds up its share of the pixels, over the slices in order
         cg::cluster_group cluster = cg::this_cluster();
         sh.part[0][part_at(tid)] = v;  // (only this thread reads this place of the first warp's image)
         cluster.sync();
         const int each = kSplatTile * kSplatTile / slices;
-        pixel = slice * each + tid;
+        pixel = mine * each + tid;
         if (tid < each) {
             v = make_float4(0.f, 0.f, 0.f, 0.f);
             for (int k = 0; k < slices; ++k) {
@@ -468,11 +484,18 @@ static bool sparse_tiles(const SplatArgs &a) { return particles_of_a_tile(a) < 2
 // pixels, h = 1458, 1 system 76 / 43 / 27 / 19, 4 systems 76 / 45 / 33 / 35; h = 729, 1 system 43 / 27 / 19 / 15, 8 systems 43 / 31 /
 // 32 / 39; h = 364, 16 systems 31 / 32 / 37; 192 pixels, h = 491, 1 system 37 / 27, 4 systems 71 / 71; h = 245, 8 systems 66 / 84; 224
 // pixels, h = 440, 1 system 35 / 33, 4 systems 83 / 85.
+// What the batch decides is whether a cluster takes the slices or one CTA in turn, with the same bits: once all tiles of the batch
+// fill the chip the clusters only repeat the fixed part, up to 45 % of the kernel with eight slices.  us, cluster / in turn: 64 pixels,
+// eight slices of 8,192, 16 systems (256 tiles) 97 / 112, 32 181 / 178, 64 353 / 308; 128 pixels, four slices of 8,192, 8 systems (512) 94 / 99,
+// 16 174 / 160, 32 334 / 286; 192 pixels, two slices of 8,192, 4 systems (576) 73 / 74, 8 132 / 128, 16 245 / 227.  Images of four
+// tiles, which are all as full, fill the chip evenly and earlier: 32 pixels, eight slices of 4,096, 32 systems 52 / 84, 64 98 / 85.
 static int splat_slices(const SplatArgs &a, int tiles) {
     const double h = particles_of_a_tile(a);
     if (tiles <= 64) return h >= 1400.0 ? 8 : h >= 680.0 ? 4 : h >= 340.0 ? 2 : 1;
     return tiles <= 144 && h >= 340.0 ? 2 : 1;
 }
+
+static bool slices_in_turn(const SplatArgs &a, int tiles) { return (long long)a.B * tiles >= (tiles <= 4 ? 256 : 1024); }
 
 static int check_splat(const char *name, const SplatArgs &a) {
     if (a.B <= 0 || a.N <= 0 || a.img <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: batch, particles and img_size must be positive", name);
@@ -514,10 +537,14 @@ int npa_splat_forward(const float *x, const float *color, int32_t batch, int32_t
     }
     const int slices = splat_slices(a, tiles * tiles);
     if (slices == 1) {
-        launch_early(splat_forward_kernel<false>, dim3(tiles * tiles, batch), kSplatThreads, 0, st, a);
+        launch_early(splat_forward_kernel<SplatSlices::kOne>, dim3(tiles * tiles, batch), kSplatThreads, 0, st, a, 1);
         return check_launch("splat_forward_kernel");
     }
-    launch_cluster(slices, splat_forward_kernel<true>, dim3(slices * tiles * tiles, batch), kSplatThreads, 0, st, a);
+    if (slices_in_turn(a, tiles * tiles)) {
+        launch_early(splat_forward_kernel<SplatSlices::kTurns>, dim3(tiles * tiles, batch), kSplatThreads, 0, st, a, slices);
+        return check_launch("splat_forward_kernel (slices in turn)");
+    }
+    launch_cluster(slices, splat_forward_kernel<SplatSlices::kCluster>, dim3(slices * tiles * tiles, batch), kSplatThreads, 0, st, a, slices);
     return check_launch("splat_forward_kernel");
 }
 

@@ -147,10 +147,11 @@ def test_forward_on_either_side_of_the_kernel_choice(img, sigma):
         assert torch.equal(splatting.splat_particles(x[2].cuda(), c[2].cuda(), img_size=img, sigma=sigma), out[2])
 
 
-@pytest.mark.parametrize("img,n", [(64, 1900), (64, 1950), (70, 4100), (64, 8200), (150, 5000), (160, 9001)])
+@pytest.mark.parametrize("img,n", [(64, 1900), (64, 1950), (70, 4100), (64, 8200), (150, 5000), (160, 9001), (208, 4097), (200, 8200)])
 def test_tiles_shared_by_a_cluster(img, n):
-    """One, two, four and eight slices of the particles per tile (the last size: three windows of the list, two slices), particles
-    outside the image and a colour that is not finite: the fp64 oracle's image, and the same bits alone and in a batch."""
+    """One, two, four and eight slices of the particles per tile (160 pixels: two windows of the list in each of two slices; 208 and 200: one
+    slice with two and three windows), particles outside the image and a colour that is not finite, in the last window: the
+    fp64 oracle's image, and the same bits alone and in a batch."""
     from npa_b200 import splatting
     from oracle import splat as splat_oracle
     g = torch.Generator().manual_seed(n)
@@ -164,3 +165,25 @@ def test_tiles_shared_by_a_cluster(img, n):
     patch = torch.zeros(img, img, dtype=torch.bool)
     patch[mid - r: mid + r + 1, mid - r: mid + r + 1] = True
     assert torch.equal(bad[..., 0], patch) and not bool(bad[..., 1:].any())
+
+
+@pytest.mark.parametrize("img,n,batch", [(64, 1950, 64), (64, 4100, 65), (64, 8200, 64), (144, 9001, 13), (32, 2048, 64), (32, 4099, 64)])
+def test_slices_by_a_cluster_or_in_turn(img, n, batch):
+    """Two, four and eight slices of a tile (the fourth size: two windows in each), by a cluster for single images and by one CTA in turn
+    for large batches: the same bits, the fp64 oracle's image, and a colour that is not finite stays in its patch."""
+    from npa_b200 import splatting
+    from oracle import splat as splat_oracle
+    g = torch.Generator().manual_seed(n)
+    x, c = (torch.rand(batch, n, 2, generator=g) - 0.5) * 2.2, torch.rand(batch, n, 3, generator=g)
+    x[1, n - 1], c[1, n - 1, 0] = 0.0, float("inf")
+    x, c = x.cuda(), c.cuda()
+    out = splatting.splat_particles_batch(x, c, img_size=img)
+    for b in (0, 1, batch - 1):
+        alone = splatting.splat_particles(x[b], c[b], img_size=img)
+        assert torch.equal(torch.nan_to_num(alone, nan=-7.0), torch.nan_to_num(out[b], nan=-7.0))
+    _close(out[0], splat_oracle.splat_forward(x[0].cpu().numpy(), c[0].cpu().numpy(), img_size=img), f"{n} particles")
+    assert not torch.isfinite(out[1, ..., 0]).all() and torch.isfinite(out[1, ..., 1:]).all()
+    r, mid = splatting._derived(img, 2.0, -1.0, 1.0, True, 2.0 / 128.0)[1], (img - 1) // 2
+    patch = torch.zeros(img, img, dtype=torch.bool)
+    patch[max(0, mid - r): mid + r + 1, max(0, mid - r): mid + r + 1] = True
+    assert torch.equal(~torch.isfinite(out[1, ..., 0]).cpu(), patch)
