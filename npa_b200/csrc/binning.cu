@@ -391,13 +391,18 @@ static size_t small_smem(const Geom &g) {
     return (size_t)(table_at(g.cells) + 1) * 4 + (size_t)((g.N + 1) & ~1) * 4 + (size_t)((g.N + 31) / 32) * 8;
 }
 
-// Which way to build a grid, from estimates of all in microseconds.  Small (one CTA per system): a fixed part; the particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell); the cell table, which a thread walks in
-// consecutive cells -- once in shared memory and, with several systems, again in global memory, where long runs per thread
-// scatter the loads.  General: six launches and their gaps; the shared histogram; the particles and cells of all systems; ranking, spread
-// over the chip.  Fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells) in a graph; what
-// the general way takes more back to back on a stream, in the gaps between its launches, is counted.  Some sizes, small /
-// general, us, in a graph: 1 system of 2,048 in 16 x 16 6 / 23; 4 of 4,096 12 / 22; 64 of 16,384 in 64 x 64 28 / 61; 1 of 16,384 in
-// 8 x 8 93 / 30; 2 of 4,096 in 32^3 77 / 25; 16 of 12,000 in 128 x 128 43 / 28.
+// Which way to build a grid, from estimates of all in microseconds.
+//  * Small, one CTA per system: a fixed part; the particles; ranking inside cells (pairs of a cell, or a bitmap beyond kCrowdedCell);
+//    the cell table, which a thread walks in consecutive cells -- once in shared memory and, with several systems, again in
+//    global memory, where long runs per thread scatter the loads.
+//  * Cluster, eight CTAs per system: a fixed part; the share of a CTA; ranking among the share's particles of a cell; the systems, and
+//    the cells where there are more CTAs than SMs; the rows as above.
+//  * General: six launches; the shared histogram; the particles and cells of all systems; ranking, spread over the chip; crowded cells.
+// Small and general were fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells), cluster, crowded
+// cells and the launches of the general way, which overlap on a stream, to 600 sizes (2,500 to 65,536 particles, 1 to 32 systems, 9 to
+// 32,768 cells) on a stream and in a graph: 0.2 % behind the best way on average, 14 % at worst.  Some sizes, small / cluster /
+// general, us, in a graph: 1 system of 2,500 in 10 x 10 7.6 / 8.4 / 23; 1 of 16,384 in 3^3 48 / 19 / 35; 32 of 8,192 in 100 x 100
+// 24 / 26 / 32; 1 of 65,536 in 6 x 6 - / 63 / 43, in 3 x 3 - / 54 / 102; 1 of 30,000 in 32^3 - / 28 / 25; 2 of 4,096 in 32^3 77 / 76 / 24.
 enum class GridBuild { kSmall, kCluster, kGeneral };
 
 static double rows_estimate(const Geom &g) {
@@ -405,9 +410,6 @@ static double rows_estimate(const Geom &g) {
     return g.B > 1 ? 3.0 + c * c / 2.2e7 + c / 4000.0 : c / 2500.0;
 }
 
-// One cluster per system (bin_cluster_kernel): a fixed part, the share of a CTA, the CTAs (eight per system on 148 SMs), the cells and
-// rows.  Measured against the others over 33 sizes: with the better way of the two others 1 % behind at worst where it is chosen, 12 %
-// where it is not (16 systems of 4,096).  Since the general launches overlap they take 4 us less on a stream than when they were fitted.
 constexpr int kClusterCtas = 8;
 static size_t cluster_smem(const Geom &g, int ctas);
 
@@ -416,10 +418,13 @@ static GridBuild grid_build(const Geom &g) {
     const double none = 1e30;
     const bool fits = g.N <= kSmallParticles && g.cells < 65536 && small_smem(g) <= kSmallSmem;
     const double small = fits ? 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) + rows_estimate(g) : none;
-    const double general = 20.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
-                           (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7;
+    const double crowded = per_cell > kCrowdedCell ? 4.0 + per_cell * 0.008 + all * 5e-5 + per_cell * g.B * 8e-4 : 0.0;
+    const double general = 19.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
+                           (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7 + crowded;
     const bool shares = g.N > 2048 && g.N <= 65536 && g.cells < 65536 && cluster_smem(g, kClusterCtas) <= kClusterSmem;
-    const double cluster = shares ? 7.0 + n / 4400.0 + g.B / 8.0 + rows_estimate(g) : none;
+    const double share_ranking = per_cell > kCrowdedCell * kClusterCtas ? 19.0 : n * per_cell / 2.6e6;
+    const double beyond = kClusterCtas * g.B > 148 ? c * (kClusterCtas * g.B - 148) / 160000.0 : 0.0;  // CTAs beyond one per SM
+    const double cluster = shares ? 7.5 + n / 4800.0 + share_ranking + g.B / 24.0 + beyond + rows_estimate(g) : none;
     if (cluster < small && cluster < general) return GridBuild::kCluster;
     return small <= general ? GridBuild::kSmall : GridBuild::kGeneral;
 }

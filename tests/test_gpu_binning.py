@@ -154,7 +154,7 @@ def test_cells_are_contiguous_and_sorted():
 
 @pytest.mark.parametrize("dim,B,N,cells", [
     (3, 2, 700, 32), (3, 1, 700, 32), (2, 3, 900, 128), (2, 1, 16384, 8), (2, 1, 8192, 8), (2, 1, 6000, 8), (2, 1, 16384, 64),
-    (2, 1, 5000, 4), (3, 2, 16384, 16), (2, 1, 16385, 64)])
+    (2, 1, 5000, 4), (3, 2, 16384, 16), (2, 1, 16385, 64), (2, 1, 65536, 6), (2, 32, 8192, 100), (3, 1, 30000, 32)])
 def test_either_way_of_the_grid_build(dim, B, N, cells):
     """One CTA per system or the general launches: sizes on both sides of the lines between them."""
     from npa_b200 import sphops as sph
