@@ -143,7 +143,9 @@ _PAIR_CACHE = {"columns": None}
 def set_pair_cache(columns=128):
     """Length of the per-particle neighbour lists that the sweeps of a snapshot share (4 * columns bytes
     per particle while the snapshot or the autograd graph is alive); 0 disables them, None is the default: by the
-    number of neighbours that the grid's mean density gives."""
+    number of neighbours that the grid's mean density gives, and for the density, ``perceive`` and the single operators up to 512
+    as long as the lists of a call take at most 128 MiB.  A backward through many recorded steps of those keeps the lists of all of
+    them: ``set_pair_cache(128)`` bounds them at 512 bytes per particle and step, for more time where particles have more neighbours."""
     columns = None if columns is None else int(columns)
     if columns is not None and columns != 0 and not 2 <= columns <= 513:
         raise ValueError("columns must be 0 or between 2 and 513")

@@ -106,10 +106,14 @@ class _HashGridBase:
 
     @functools.cached_property
     def roomy_list_columns(self):
-        """Columns for sweeps whose order of sums does not depend on the length of the lists: where 128 is the rule, as many
-        more as 128 MiB of lists leave, at most 512.  A particle that does not fit searches its cells at several times the cost of a
-        list: 8 x 16,384 particles in 2D clusters, one in forty of them with 128 to 188 neighbours where the mean is 56, forward 163
-        -> 113 us and full backward 446 -> 344; without such particles the longer rows cost nothing (177 and 640 us in 3D either way)."""
+        """Columns for the density, ``perceive`` and the single operators: where 128 is the rule, as many more as 128 MiB of lists
+        leave, at most 512.  A particle that does not fit searches its cells at several times the cost of a list, and adds up in another
+        order (the packed perception, whose MLP switches hidden units with the last bit, keeps ``list_columns``).  8 x 16,384 particles in
+        2D clusters, one in forty of them with 128 to 188 neighbours where the mean is 56, 128 / 256 columns: forward 161 -> 113 us, full
+        backward 440 -> 342; 65,536 in clusters, 128 / 256 / 512: pass 764 / 568 / 452 us; 2 x 16,384 along lines 498 / 469 / 290.  Rows that
+        are not used cost no time (8 x 4,096 uniform 101.2 / 101.1 / 101.6 us), but memory as long as the lists live -- with an autograd
+        graph until its backward: 64 MiB instead of 16 for each recorded step of 8 x 4,096 particles (the step keeps 83 MiB instead of
+        35 at C = 16), at most 96 MiB more for a step of any size.  ``set_pair_cache(128)`` goes back to 128 columns."""
         if self.list_columns > 128:
             return self.list_columns
         return max(128, min(512, (128 << 20) // (4 * self._B * self._N) // 64 * 64))

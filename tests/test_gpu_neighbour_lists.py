@@ -132,3 +132,37 @@ def test_full_backward_with_particles_of_no_mass_and_crowded_lists(dim, C):
     # two fp32 sums of up to a few hundred terms in different orders: 2e-5 of the largest value
     for a, b in zip(*got):
         assert torch.isfinite(a).all() and float((a - b).abs().max()) <= 2e-5 * float(b.abs().max())
+
+
+def test_memory_that_recorded_steps_keep():
+    """A chain of steps through ``perceive``: what every further step keeps until the backward is its tensors and its lists, at the
+    default length and at 128 columns."""
+    from npa_b200 import sphops as sph
+    B, N, C = 8, 4096, 16
+    grid = sph.HashGrid(dim=2, boundary="clamped", mode="grid", grid_size=(16, 16), eps=0.0625, num_particles=N, batch_size=B)
+    g = torch.Generator(device="cuda").manual_seed(2)
+    x0, s0 = torch.rand(B, N, 2, generator=g, device="cuda") - 0.5, torch.randn(B, N, C, generator=g, device="cuda")
+
+    def kept(steps):
+        """Bytes that are alive after ``steps`` recorded steps."""
+        torch.cuda.synchronize()
+        before = torch.cuda.memory_allocated()
+        x, s = x0.clone().requires_grad_(True), s0.clone().requires_grad_(True)
+        for _ in range(steps):
+            snap = grid.instantiate(x)
+            xb, sb = sph.bin_particles(x, s, snap)
+            rho, blur, grad, dg = sph.perceive(xb, sb, snap)
+            x, s = xb + 1e-4 * dg, blur
+        return torch.cuda.memory_allocated() - before
+
+    per_step = {}
+    for columns in (None, 128):
+        sph.set_pair_cache(columns)
+        try:
+            kept(2)
+            per_step[columns] = (kept(5) - kept(2)) / 3
+        finally:
+            sph.set_pair_cache(None)
+    lists = {None: 4 * grid.hashgrid.roomy_list_columns * B * N, 128: 4 * 128 * B * N}
+    assert abs((per_step[None] - per_step[128]) - (lists[None] - lists[128])) <= 2 << 20
+    assert per_step[128] <= lists[128] + (32 << 20)  # tensors of a step: positions, features, blur, gradient, density: 12 MiB

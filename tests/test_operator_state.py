@@ -167,3 +167,25 @@ def test_the_move_kernel_takes_only_fields_of_the_shapes_it_reads():
     with torch.no_grad():
         view = leaf[:1]
     assert _writable(x) and _writable(x[:1]) and not _writable(inference) and not _writable(leaf) and not _writable(view)
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+def test_memory_of_the_default_lists(dim):
+    """Longer lists than 128 columns stay below 128 MiB for a call, so that a recorded step never keeps over 96 MiB more than with 128;
+    a setting of the user's is taken as it is."""
+    from npa_b200.sphops import sph as impl
+    for B, N in ((1, 16), (64, 512), (8, 4096), (3, 5001), (1, 65536), (8, 16384), (1, 131073), (4, 65536), (16, 65536), (2, 1 << 20)):
+        cells = max(3, round((N / (16 if dim == 2 else 8)) ** (1.0 / dim)))
+        grid = sph.HashGrid(dim=dim, boundary="clamped", mode="grid", grid_size=(cells,) * dim, eps=1.0 / cells, num_particles=N, batch_size=B).hashgrid
+        if grid.list_columns > 128:
+            assert grid.roomy_list_columns == grid.list_columns
+            continue
+        columns, narrow = grid.roomy_list_columns, 4 * 128 * B * N
+        assert 128 <= columns <= 512 and (columns == 128 or 4 * columns * B * N <= 128 << 20)
+        assert 4 * columns * B * N - narrow <= 96 << 20
+        try:
+            sph.set_pair_cache(128)
+            assert impl._roomy_columns(grid) == impl._columns(grid) == 128
+        finally:
+            sph.set_pair_cache(None)
+        assert impl._roomy_columns(grid) == columns and impl._columns(grid) == 128
