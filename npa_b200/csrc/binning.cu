@@ -757,9 +757,11 @@ permute_images_kernel(const float *__restrict__ x, const float *__restrict__ s, 
     else write_image_element(jobs, (int)(blockIdx.x - blocks) * 256 + threadIdx.x);
 }
 
-template <bool FORWARD>
+// `images`: with those blocks, which only the forward reorder of a step has.
+template <bool FORWARD, typename... Images>
 static int launch_permute(const Geom &g, int C, const float *x, const float *s, const float *m,
-                          const int32_t *perm, float *xo, float *so, float *mo, cudaStream_t st, const ImageJobs *jobs = nullptr) {
+                          const int32_t *perm, float *xo, float *so, float *mo, cudaStream_t st, const Images &...images) {
+    static_assert(sizeof...(Images) == 0 || FORWARD, "the images are made by the forward reorder");
     if (!perm) return fail(NPA_ERR_INVALID_ARGUMENT, "permutation is NULL");
     if ((x == nullptr) != (xo == nullptr) || (s == nullptr) != (so == nullptr) || (m == nullptr) != (mo == nullptr))
         return fail(NPA_ERR_INVALID_ARGUMENT, "each input of a permutation needs its output (and vice versa)");
@@ -770,10 +772,10 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     const int pieces = s ? (vec ? C / 4 : C) : 1;
     const long long total = (long long)g.B * g.N * pieces;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if (jobs) {
-        const unsigned all = blocks + (unsigned)(jobs->total() + 255) / 256;
+    if constexpr (sizeof...(Images) == 1) {
+        const unsigned all = blocks + (unsigned)((images.total() + ...) + 255) / 256;
 #define NPA_PERMUTE(DD, VEC) \
-    launch_early(permute_images_kernel<DD, VEC>, all, 256, 0, st, x, s, perm, xo, so, pieces, total, g.N, blocks, *jobs)
+    launch_early(permute_images_kernel<DD, VEC>, all, 256, 0, st, x, s, perm, xo, so, pieces, total, g.N, blocks, images...)
         if (g.dim == 2) {
             if (vec) NPA_PERMUTE(2, float4); else NPA_PERMUTE(2, float);
         } else {
@@ -797,7 +799,7 @@ int bin_particles_and_images(const npa_grid *grid, int channels, const float *x,
                              float *s_out, const ImageJobs &jobs, cudaStream_t stream) {
     Geom g;
     const int rc = make_geom(grid, &g);
-    return rc != NPA_OK ? rc : launch_permute<true>(g, channels, x, s, nullptr, permutation, x_out, s_out, nullptr, stream, &jobs);
+    return rc != NPA_OK ? rc : launch_permute<true>(g, channels, x, s, nullptr, permutation, x_out, s_out, nullptr, stream, jobs);
 }
 
 // ---------------------------------------------------------------------------

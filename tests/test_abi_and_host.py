@@ -273,3 +273,47 @@ def test_tcgen05_entry_points_reject_bad_arguments_before_any_launch():
     assert lib.npa_linear_tcgen05_status(null, 0) == n.NPA_ERR_INVALID_ARGUMENT
     assert lib.npa_linear_tcgen05_wait_selftest(0, buf, null) == n.NPA_ERR_INVALID_ARGUMENT
     assert lib.npa_linear_tcgen05_wait_selftest(2000, null, null) == n.NPA_ERR_INVALID_ARGUMENT
+
+
+def test_move_copy_and_image_entries_reject_bad_arguments_before_any_launch():
+    """The move of a rollout, the paired copy and the reorder that lays out the MLP's weights: refusals come from the host, with addresses
+    that are never dereferenced."""
+    from npa_b200 import _native as n
+    lib = n.lib
+    buf, odd, null, big = ctypes.c_void_p(1 << 20), ctypes.c_void_p((1 << 20) + 4), ctypes.c_void_p(0), 1 << 40
+    for dim in (2, 3):
+        g = n.make_grid(dim, "periodic", "grid", (8,) * dim, 0.1, 1, 8, 32)
+        move = lambda modes=8, x=buf, k=buf, phase=buf, amp=buf, out=buf: lib.npa_rollout_move(ctypes.byref(g), x, k, phase, amp, modes, 0.1, out, null)
+        assert move(modes=0) == n.NPA_ERR_UNSUPPORTED and "modes" in n.last_error()
+        assert move(modes=65) == n.NPA_ERR_UNSUPPORTED
+        assert move(x=odd) == n.NPA_ERR_INVALID_ARGUMENT and "aligned" in n.last_error()
+        for missing in ("x", "k", "phase", "amp", "out"):
+            assert move(**{missing: null}) == n.NPA_ERR_INVALID_ARGUMENT and "non-NULL" in n.last_error()
+    assert lib.npa_rollout_move(ctypes.byref(n.make_grid(2, "periodic", "grid", (8, 8), 0.0, 1, 8, 32)), buf, buf, buf, buf, 8, 0.1, buf, null) < 0
+    copy = lambda a=buf, ao=buf, na=4, b=buf, bo=buf, nb=4: lib.npa_copy_pair(a, ao, na, b, bo, nb, null)
+    for name in ("a", "ao", "b", "bo"):
+        assert copy(**{name: odd}) == n.NPA_ERR_INVALID_ARGUMENT and "aligned" in n.last_error()
+        assert copy(**{name: null}) == n.NPA_ERR_INVALID_ARGUMENT
+    assert copy(na=-1) == n.NPA_ERR_INVALID_ARGUMENT and copy(nb=-1) == n.NPA_ERR_INVALID_ARGUMENT
+    # reorder with the images of the weights
+    g = n.make_grid(2, "clamped", "grid", (8, 8), 0.1, 1, 8, 32)
+    need, need_dz = lib.npa_mlp_forward_tcgen05_scratch_bytes(66, 18), lib.npa_linear_tcgen05_scratch_bytes(128, 66)
+
+    def images(C=16, x=buf, s=buf, perm=buf, xo=buf, so=buf, w1=buf, w2=buf, k=66, o=18, scratch=buf, nbytes=need, dz=buf, dz_bytes=need_dz):
+        return lib.npa_bin_particles_mlp_images(ctypes.byref(g), C, x, s, perm, xo, so, w1, w2, k, o, k, 1, 128, 1, scratch, nbytes, dz, dz_bytes, null)
+
+    assert images(k=1025, dz=null) == n.NPA_ERR_UNSUPPORTED and images(o=65) == n.NPA_ERR_UNSUPPORTED
+    assert images(k=0) == n.NPA_ERR_INVALID_ARGUMENT and images(o=-1) == n.NPA_ERR_INVALID_ARGUMENT
+    assert images(nbytes=need - 1) == n.NPA_ERR_INVALID_ARGUMENT and "scratch" in n.last_error()
+    assert images(dz_bytes=need_dz - 1) == n.NPA_ERR_INVALID_ARGUMENT and "dz_image" in n.last_error()
+    assert images(scratch=odd) == n.NPA_ERR_INVALID_ARGUMENT and images(dz=odd) == n.NPA_ERR_INVALID_ARGUMENT
+    for bad in (dict(w1=null), dict(w2=null), dict(scratch=null), dict(perm=null), dict(x=null), dict(xo=null), dict(s=null), dict(so=null),
+                dict(C=0), dict(x=odd), dict(xo=odd)):
+        assert images(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
+    # both layers on images that are there
+    two = lambda rows=1000, k=66, o=18, z=buf, y=buf, scratch=buf, nbytes=need: lib.npa_mlp_forward_tcgen05_prepared(
+        z, null, null, y, rows, k, o, scratch, nbytes, null)
+    assert two(k=1025) == n.NPA_ERR_UNSUPPORTED and two(o=65) == n.NPA_ERR_UNSUPPORTED
+    assert two(nbytes=need - 1) == n.NPA_ERR_INVALID_ARGUMENT and two(scratch=odd) == n.NPA_ERR_INVALID_ARGUMENT
+    for bad in (dict(rows=0), dict(k=0), dict(o=0), dict(z=null), dict(y=null), dict(scratch=null), dict(z=ctypes.c_void_p((1 << 20) + 2))):
+        assert two(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
