@@ -88,6 +88,8 @@ int64_t npa_grid_max_blocks(const npa_grid *g);
  * cell ids, unsorted slots, scan partials); replaces the cudaMalloc'ed members
  * of the reference's HashGrid (sph_cuda.cu:1881-1895). */
 int64_t npa_grid_scratch_bytes(const npa_grid *g);
+/* Kernels that one npa_grid_build() launches: 1 or 2 where a CTA or a cluster of them bins a system, else 6. */
+int npa_grid_build_kernels(const npa_grid *g);
 
 /*
  * Uniform-grid binning; replaces HashGrid::initialize (sph_cuda.cu:1926-1992:

@@ -49,6 +49,7 @@ SIGNATURES = {
     "npa_abi_version": (ctypes.c_int, []),
     "npa_grid_num_cells": (_I64, [_P]),
     "npa_grid_max_blocks": (_I64, [_P]),
+    "npa_grid_build_kernels": (ctypes.c_int, [_P]),
     "npa_grid_scratch_bytes": (_I64, [_P]),
     "npa_grid_build": (ctypes.c_int, [_P, _P, _P, _P, _P, _P, _I64, _P]),
     "npa_grid_build_static": (ctypes.c_int, [_P, _P, _P, _P, _P, _P]),

@@ -884,6 +884,13 @@ int64_t npa_grid_scratch_bytes(const npa_grid *gd) {
     return (int64_t)layout_scratch(g, nullptr, nullptr);
 }
 
+int npa_grid_build_kernels(const npa_grid *gd) {
+    Geom g;
+    const int rc = make_geom(gd, &g);
+    if (rc != NPA_OK) return rc;
+    return grid_build(g) == GridBuild::kGeneral ? 6 : g.B == 1 ? 1 : 2;
+}
+
 int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int32_t *bin_offsets,
                    int32_t *block_info, void *scratch, int64_t scratch_bytes, void *stream) {
     Geom g;

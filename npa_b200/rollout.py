@@ -90,9 +90,9 @@ class PerceptionRollout:
         if grid.boundary == "periodic":
             self.box = torch.tensor([g * grid.eps for g in grid.grid_size[:D]], **f32)
             self.half_box = 0.5 * self.box
-        # kernels of this library per rollout: 6 grid build + reorder + 2 sweeps per step, a move between steps, and for the
+        # kernels of this library per rollout: grid build, reorder and 2 sweeps per step, a move between steps, and for the
         # last step the layout of the upstream, 2 backward sweeps and the inverse reorder
-        self.launches = self.steps * 9 + 4 + (self.steps - 1 if self._native_move() else 0)
+        self.launches = self.steps * (self.hg.build_kernels + 3) + 4 + (self.steps - 1 if self._native_move() else 0)
 
     def _native_move(self):
         """Whether the move kernel computes this field: parameters of the shapes that it reads, as plain memory, and without a

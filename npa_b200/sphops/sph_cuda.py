@@ -127,6 +127,7 @@ class _HashGridBase:
     max_blocks = property(lambda self: self._max_blocks)
     max_particles_per_block = property(lambda self: self._mpb)
     cell_count = property(lambda self: self._cells)
+    build_kernels = property(lambda self: int(_lib.npa_grid_build_kernels(self._ref())))  # kernels that one binning launches
 
     # ---- helpers -------------------------------------------------------------
     def _ref(self):

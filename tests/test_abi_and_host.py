@@ -52,6 +52,19 @@ def test_geometry_queries_and_errors():
     assert rc == n.NPA_ERR_INVALID_ARGUMENT and "2x2 or 3x3" in n.last_error()
 
 
+def test_kernels_of_a_grid_build():
+    """One CTA or one cluster per system is a kernel, with several systems a second one; the general way is six.  A rollout counts them."""
+    from npa_b200 import _native as n, sphops as sph
+    from npa_b200.rollout import PerceptionRollout, VelocityField
+    for (cells, B, N), want in {(16, 1, 2500): 1, (10, 1, 4096): 1, (16, 64, 512): 2, (40, 8, 16384): 2, (6, 1, 65536): 6, (64, 4, 1 << 20): 6}.items():
+        grid = sph.HashGrid(dim=2, boundary="clamped", mode="grid", grid_size=(cells, cells), eps=1.0 / cells, num_particles=N, batch_size=B)
+        assert grid.hashgrid.build_kernels == want, (cells, B, N)
+        if N < 10000:
+            roll = PerceptionRollout(grid, 4, 3, 0.1, VelocityField(2, torch.device("cpu")))
+            assert roll.launches == 3 * (want + 3) + 4 + 2
+    assert n.lib.npa_grid_build_kernels(ctypes.byref(n.make_grid(2, "clamped", "grid", (8, 8), -1.0, 1, 8, 32))) == n.NPA_ERR_INVALID_ARGUMENT
+
+
 def test_misaligned_positions_are_refused_before_any_launch():
     """The reorder moves a position as one vector; addresses here are never dereferenced (the check comes first)."""
     from npa_b200 import _native as n
