@@ -54,18 +54,24 @@ int check_launch(const char *what);
 // come before it: a kernel launched this way that does not call it would not wait for its inputs at all.  Every kernel waits for the
 // one before, so a chain is in order as a whole.  Kernels of others, copies and events wait for complete kernels, as ever.
 // Training step of 8 x 4,096 particles in 2D 234 -> 207 us, of 4 x 16,384 in 3D 374 -> 336, inference step of 4,096 72 -> 60.
-// Not launched this way: the sweeps over neighbour lists, which live off L1 and got slower (full backward and forward of 2 x
-// 262,144 particles 3,116 -> 3,344 us for the rollout: a CTA that takes its place early finds the SM divided between L1 and shared
-// memory as the kernel before wanted it); the kernels after the weight gradients and after the update's backward (training step in 2D
-// 207 -> 252 us with the former, in 3D 1,615 -> 1,643 with the latter; not explained); the kernels that search, not measured.  While
-// a graph is recorded launches are plain ones: its nodes are close already (41.3 us instead of 41.9), and the edges would make it
-// 10 % slower to build.
+// Plain launches, because they were slower this way:
+//  * feature_list.cuh, forward and backward (rollout of 2 x 262,144 particles 3,116 -> 3,344 us): they live off L1, and a CTA that takes
+//    its place early finds the SM divided between L1 and shared memory as the kernel before wanted it;
+//  * the reduction of the weight gradients (training step in 2D 207 -> 252 us): early, its 170 CTAs are placed three to an SM on the
+//    sixty SMs that the gradient kernel leaves first, and those that read dW2's partial sums across rows, neighbours in the grid,
+//    take 16-40 us there instead of 3-7 (measured per CTA with the global timer);
+//  * the hidden gradient of the MLP (3D step 1,615 -> 1,643 us, not explained).
+// Plain and not measured otherwise: the searching sweeps of feature_kernels.cuh and scalar_ops.cu, the cell-tile engine, the paths of
+// mlp_gemm.cu and mlp_grad.cu, small conversions.  The density searches, the packed sweep and the sweeps of scalar_list.cu are launched
+// early; they were measured within the chains above only.
+// While a graph is recorded all launches are plain: its nodes are close already (41.3 us instead of 41.9), and the edges would make
+// it 10 % slower to build.
 __device__ __forceinline__ void after_previous_kernel() {
     asm volatile("griddepcontrol.wait;" ::: "memory");
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
-// The same with clusters of `cluster` blocks.
+// Such a launch; in clusters of `cluster` blocks where that is more than one.
 template <typename... P, typename... A>
 inline void launch_cluster(int cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A &&...args) {
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;

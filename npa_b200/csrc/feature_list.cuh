@@ -26,7 +26,9 @@
 // Measured, B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us, kernel with the whole warp per particle
 // -> this one: blur + gradient 328 -> 178 (with the density gradient), features-only backward 499 -> 401, full
 // backward 902 -> 575 (644 with one sum per term and 14 warps per SM; 524,288 periodic, C = 16: 700 -> 632, with two list entries per
-// lane and chunk and the registers of these 790).  In 2D the one sum is level (8 x 16,384, C = 32: 446 -> 441; 8 x 4,096, C = 16: 43.8 -> 44.7).
+// lane and chunk and the registers of these 790).  In 2D the one sum gains little or loses
+// little (blur and gradient together, 8 x 16,384, C = 32: 446 -> 441; 4 x 65,536, C = 64 723 -> 711; 8 x 4,096, C = 16 56.3 -> 56.4, C = 13 58.4
+// -> 59.2; one operator alone, C = 16: gradient 43.5 -> 44.6, blur 30.7 -> 31.2, where the preparation of a particle shows).
 #pragma once
 #include "neighbors.cuh"
 #include "ops.cuh"
