@@ -142,7 +142,7 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
     const bool colours = (tid & 3) == 3;
     float pos = 0.f;
     float4 col = make_float4(0.f, 0.f, 0.f, 0.f);
-    auto fetch = [&](int window, int off, int count) {
+    auto fetch = [&](unsigned window, int off, int count) {
         if (off + sp >= count) return;
         const long long n = (long long)b * a.N + window + sh.lists.n[off + sp];
         pos = __ldg(a.x + n * 2 + axis);
@@ -214,7 +214,7 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
 
     const float top = (float)(a.img - 1), per = top / a.span, reach = (float)r + 9.25f;  // patch radius, half a tile, a pixel, rounding
     const float mx = (float)tx0 + 7.5f, my = (float)ty0 + 7.5f;
-    const int share = (a.N + slices - 1) / slices;
+    const unsigned share = ((unsigned)a.N + slices - 1) / slices;  // (unsigned: a window may end beyond 2^31 particles)
     float4 v;
     for (int slice = mine; slice < (TURNS ? slices : mine + 1); ++slice) {
 #pragma unroll
@@ -223,12 +223,12 @@ __global__ void __launch_bounds__(kSplatThreads, 2) splat_forward_kernel(SplatAr
             for (int c = 0; c < 4; ++c)
 #pragma unroll
                 for (int x = 0; x < 4; ++x) acc[y][c][x] = 0ull;
-        const int end = min(a.N, (slice + 1) * share);
-        for (int n0 = slice * share; n0 < end; n0 += kSplatWindow) {
+        const unsigned from = slice * share, end = min((unsigned)a.N, from + share);
+        for (unsigned n0 = from; n0 < end; n0 += kSplatWindow) {
             unsigned hits = 0;
 #pragma unroll 8
             for (int q = 0; q < kSplatCull; ++q) {
-                const int n = n0 + q * kSplatThreads + tid;
+                const unsigned n = n0 + q * kSplatThreads + tid;
                 if (n < end) {
                     const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x) + (long long)b * a.N + n);
                     const float x = (v.x - a.lo) * per;
@@ -333,11 +333,11 @@ __global__ void __launch_bounds__(kSplatTile *kSplatTile) splat_forward_sparse_k
     const float inv2s2 = 1.0f / (2.0f * a.sigma * a.sigma);
     float acc[4] = {0.f, 0.f, 0.f, 0.f};
 
-    for (int n0 = 0; n0 < a.N; n0 += T) {
-        const int n = n0 + tid;
+    for (unsigned n0 = 0; n0 < (unsigned)a.N; n0 += T) {
+        const unsigned n = n0 + tid;
         bool hit = false;
         SplatPoint p = {0, 0, 0.f, 0.f};
-        if (n < a.N) {
+        if (n < (unsigned)a.N) {
             p = splat_point(a, (long long)b * a.N + n);
             hit = p.cx + r >= tx0 && p.cx - r < tx0 + kSplatTile && p.cy + r >= ty0 && p.cy - r < ty0 + kSplatTile;
         }
@@ -487,15 +487,16 @@ static bool sparse_tiles(const SplatArgs &a) { return particles_of_a_tile(a) < 2
 // What the batch decides is whether a cluster takes the slices or one CTA in turn, with the same bits: once all tiles of the batch
 // fill the chip the clusters only repeat the fixed part, up to 45 % of the kernel with eight slices.  us, cluster / in turn: 64 pixels,
 // eight slices of 8,192, 16 systems (256 tiles) 97 / 112, 32 181 / 178, 64 353 / 308; 128 pixels, four slices of 8,192, 8 systems (512) 94 / 99,
-// 16 174 / 160, 32 334 / 286; 192 pixels, two slices of 8,192, 4 systems (576) 73 / 74, 8 132 / 128, 16 245 / 227.  Images of four
-// tiles, which are all as full, fill the chip evenly and earlier: 32 pixels, eight slices of 4,096, 32 systems 52 / 84, 64 98 / 85.
+// 16 174 / 160, 32 334 / 286; 192 pixels, two slices of 8,192, 8 systems (1,152) 132 / 128, 16 245 / 227, of 16,384,
+// 8 systems 224 / 232.  Images of four tiles, which are all as full, fill the chip evenly and earlier: 32 pixels, eight slices of 4,096,
+// 32 systems 52 / 84, 64 98 / 85.
 static int splat_slices(const SplatArgs &a, int tiles) {
     const double h = particles_of_a_tile(a);
     if (tiles <= 64) return h >= 1400.0 ? 8 : h >= 680.0 ? 4 : h >= 340.0 ? 2 : 1;
     return tiles <= 144 && h >= 340.0 ? 2 : 1;
 }
 
-static bool slices_in_turn(const SplatArgs &a, int tiles) { return (long long)a.B * tiles >= (tiles <= 4 ? 256 : 1024); }
+static bool slices_in_turn(const SplatArgs &a, int tiles) { return (long long)a.B * tiles >= (tiles <= 4 ? 256 : tiles <= 64 ? 1024 : 1600); }
 
 static int check_splat(const char *name, const SplatArgs &a) {
     if (a.B <= 0 || a.N <= 0 || a.img <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: batch, particles and img_size must be positive", name);
