@@ -24,8 +24,8 @@
 // of the row sectors come from L2 (prefetching rows into L1 a chunk ahead was slower, 330 -> 340 us; one register
 // set per row refilled early cost spills, 194 -> 234 us; five CTAs of the full backward instead of four 664 -> 758 us).
 // Measured, B200, 262,144 particles in 3D, C = 32, ~41 neighbours, us, kernel with the whole warp per particle
-// -> this one: blur + gradient 328 -> 178 (with the density gradient), features-only backward 499 -> 401, full
-// backward 902 -> 575 (644 with one sum per term and 14 warps per SM; 524,288 periodic, C = 16: 700 -> 632, with two list entries per
+// -> this one: blur + gradient 328 -> 164 (with the density gradient), features-only backward 499 -> 383, full
+// backward 902 -> 560 (575 before rows were filled, 644 before that with one sum per term and 14 warps per SM; 524,288 periodic, C = 16: 700 -> 632 -> 596, with two list entries per
 // lane and chunk and the registers of these 790).  In 2D the one sum gains little or loses
 // little (blur and gradient together, 8 x 16,384, C = 32: 446 -> 441; 4 x 65,536, C = 64 723 -> 711; 8 x 4,096, C = 16 56.3 -> 56.4, C = 13 58.4
 // -> 59.2; one operator alone, C = 16: gradient 43.5 -> 44.6, blur 30.7 -> 31.2, where the preparation of a particle shows).
@@ -36,6 +36,14 @@
 namespace npa {
 
 constexpr int kListWarps = 8;      // warps per CTA
+
+// How a kernel addresses rows of C floats: float by float; four at a time (C a multiple of four, 16-byte aligned); or the same with
+// C = 4 LPP known to the compiler: the rows fill the lanes, no lane lies beyond the last feature, there is one slice, and the rows of a
+// neighbour lie at constant distances from one address.  Same sums.  Measured, B200, us, four at a time -> filled: 262,144 particles
+// in 3D, C = 32, forward 176 -> 164, full backward 574 -> 560, features only 402 -> 383, packed sweep (packed_ordered.cuh) 418 -> 371;
+// 2 x 262,144 periodic, C = 16, forward 236 -> 223, full backward 633 -> 596; 8 x 16,384 clustered in 2D, C = 32, 112 -> 107 and
+// 339 -> 321; 8 x 4,096 in 2D, C = 16, packed sweep 35 -> 33, full backward 44.5 -> 43.5.
+enum ListRows : int { kRowsAny = 0, kRowsVec = 1, kRowsFilled = 2 };
 // Same, backward; with position gradients sixteen warps per SM either way (128 registers), in 3D as eight CTAs of two.
 template <int D, bool FULL>
 constexpr int kListBackwardWarps = FULL ? (D == 3 ? 2 : 4) : kListWarps;
@@ -51,10 +59,10 @@ __device__ inline float4 fetch_particle(const float *__restrict__ x, const float
 }
 
 // Four features f0..f0+3 of a row; lanes beyond the last feature read valid neighbours of it (unused).
-template <bool VEC>
+template <int ROWS>
 __device__ inline void load_row4(const float *__restrict__ row, int f0, int C, float (&v)[4]) {
-    if (VEC) {
-        const float4 t = __ldg(reinterpret_cast<const float4 *>(row + min(f0, C - 4)));
+    if (ROWS != kRowsAny) {
+        const float4 t = __ldg(reinterpret_cast<const float4 *>(row + (ROWS == kRowsFilled ? f0 : min(f0, C - 4))));
         v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
     } else {
 #pragma unroll
@@ -62,10 +70,10 @@ __device__ inline void load_row4(const float *__restrict__ row, int f0, int C, f
     }
 }
 
-template <bool VEC>
+template <int ROWS>
 __device__ inline void store_row4(float *__restrict__ row, int f0, int C, const float (&v)[4]) {
-    if (VEC) {
-        if (f0 < C) *reinterpret_cast<float4 *>(row + f0) = make_float4(v[0], v[1], v[2], v[3]);
+    if (ROWS != kRowsAny) {
+        if (ROWS == kRowsFilled || f0 < C) *reinterpret_cast<float4 *>(row + f0) = make_float4(v[0], v[1], v[2], v[3]);
     } else {
 #pragma unroll
         for (int q = 0; q < 4; ++q)
@@ -128,12 +136,13 @@ __device__ inline int list_count(const int32_t *list, int stride, bool valid, in
 }
 
 // The particles first .. first + PP - 1 of a warp: those with a list (SEARCH false) or those whose list overflowed.
-template <int D, bool PER, int LPP, bool VEC, int MASK, bool SEARCH>
+template <int D, bool PER, int LPP, int ROWS, int MASK, bool SEARCH>
 __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
                                              int4 (*s_j)[ListShape<LPP>::kIndexQuads], float *stage) {
     constexpr int EPL = ListShape<LPP>::EPL, CH = ListShape<LPP>::CH, PP = ListShape<LPP>::PP;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
-    const int total = g.B * g.N, C = a.C;
+    constexpr bool kFilled = ROWS == kRowsFilled, kVec = ROWS != kRowsAny;
+    const int total = g.B * g.N, C = kFilled ? LPP * 4 : a.C;
     const int first = (blockIdx.x * kListWarps + warp) * PP;  // (less than total: the kernel has checked)
     bool ivalid = (unsigned)(first + sg) < (unsigned)total;
     const int i = ivalid ? first + sg : total - 1;
@@ -153,7 +162,7 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
         __syncwarp();  // the slice before has drained its buffers
         const int f0 = fbase + sl * 4;
         float si[4];
-        load_row4<VEC>(a.s + (long long)i * C, f0, C, si);
+        load_row4<ROWS>(a.s + (long long)i * C, f0, C, si);
         const unsigned long long nsi01 = pack2(-si[0], -si[1]), nsi23 = pack2(-si[2], -si[3]);
         // packed sums of the features (0, 1) and (2, 3): blur, then the gradient axis by axis
         unsigned long long acc[2 + 2 * D];
@@ -212,7 +221,7 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
                 float r[4][4];
 #pragma unroll
                 for (int u = 0; u < 4; ++u)
-                    load_row4<VEC>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + (unsigned long long)(unsigned)js[u] * pitch),
+                    load_row4<ROWS>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + (unsigned long long)(unsigned)js[u] * pitch),
                                    f0, C, r[u]);
 #pragma unroll
                 for (int u = 0; u < 4; ++u) {
@@ -332,7 +341,7 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
 #pragma unroll
             for (int q = 0; q < D * (D + 1) / 2; ++q) mom[q] = g.c_g * subgroup_sum<LPP>(mom[q]);
         }
-        if (kBlur && a.blur && ivalid) store_row4<VEC>(a.blur + (long long)i * C, f0, C, blur);
+        if (kBlur && a.blur && ivalid) store_row4<ROWS>(a.blur + (long long)i * C, f0, C, blur);
         float L[D * D];
         if (MASK & (F_PACK | F_CORRECTED)) {
             safe_inverse_sym<D>(mom, a.inv_tol, L);
@@ -353,8 +362,8 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
         float *gout = (MASK & F_PACK) ? a.vgrad : a.grad;
         if (kGrad && gout && ivalid) {
             float *o = gout + ((long long)i * C + f0) * D;
-            if (VEC) {
-                if (f0 < C) {
+            if (kVec) {
+                if (kFilled || f0 < C) {
                     const float *v = &gr[0][0];
 #pragma unroll
                     for (int k = 0; k < D; ++k) reinterpret_cast<float4 *>(o)[k] = make_float4(v[4 * k], v[4 * k + 1], v[4 * k + 2], v[4 * k + 3]);
@@ -430,13 +439,13 @@ __device__ __forceinline__ void list_forward(const FeatureFwdArgs &a, const Geom
 }
 
 // Out of line, so that the search does not cost the walk over lists registers.
-template <int D, bool PER, int LPP, bool VEC, int MASK>
+template <int D, bool PER, int LPP, int ROWS, int MASK>
 __device__ __noinline__ void list_forward_search(const FeatureFwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP>::kSlots],
                                                  int4 (*s_j)[ListShape<LPP>::kIndexQuads], float *stage) {
-    list_forward<D, PER, LPP, VEC, MASK, true>(a, g, s_k, s_j, stage);
+    list_forward<D, PER, LPP, ROWS, MASK, true>(a, g, s_k, s_j, stage);
 }
 
-template <int D, bool PER, int LPP, bool VEC, int MASK>
+template <int D, bool PER, int LPP, int ROWS, int MASK>
 __global__ void __launch_bounds__(kListWarps * 32, (MASK & F_MOMENT) ? 2 : 4)
 feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
     after_previous_kernel();
@@ -448,11 +457,11 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
     const unsigned first = (blockIdx.x * kListWarps + warp) * S::PP;
     if (first >= (unsigned)total) return;
     float *stage = reinterpret_cast<float *>(s_rows) + ((MASK & F_PACK) ? (size_t)warp * ((S::PP * a.zstride + 3) & ~3) : 0);
-    list_forward<D, PER, LPP, VEC, MASK, false>(a, g, s_k[warp], s_j[warp], stage);
+    list_forward<D, PER, LPP, ROWS, MASK, false>(a, g, s_k[warp], s_j[warp], stage);
     __syncwarp();
     const int i = (int)min(first + (threadIdx.x & 31u) / LPP, (unsigned)total - 1u);
     if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
-        list_forward_search<D, PER, LPP, VEC, MASK>(a, g, s_k[warp], s_j[warp], stage);
+        list_forward_search<D, PER, LPP, ROWS, MASK>(a, g, s_k[warp], s_j[warp], stage);
 }
 
 // ---------------------------------------------------------------------------------------------------------
@@ -468,13 +477,14 @@ feature_list_forward_kernel(const __grid_constant__ FeatureFwdArgs a, const __gr
 // Sums over features stay lane-partial (packed pairs) until the particle is done.  The density gradient's own
 // backward, dx_i += sum_j J (m_i g_j - m_j g_i), uses the same pair scalars and rides stage B.
 // ---------------------------------------------------------------------------------------------------------
-template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL, bool SEARCH>
+template <int D, bool PER, int LPP, int ROWS, int MASK, bool FULL, bool SEARCH>
 __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP, FULL && D == 3>::kSlots],
                                               float4 (*s_e)[ListShape<LPP, FULL && D == 3>::kSlots], int4 (*s_j)[ListShape<LPP, FULL && D == 3>::kIndexQuads]) {
     constexpr int EPL = ListShape<LPP, FULL && D == 3>::EPL, CH = ListShape<LPP, FULL && D == 3>::CH, PP = ListShape<LPP, FULL && D == 3>::PP, WARPS = kListBackwardWarps<D, FULL>;
     constexpr bool kGrad = (MASK & F_GRAD) != 0, kBlur = (MASK & F_BLUR) != 0;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane / LPP, sl = lane % LPP;
-    const int total = g.B * g.N, C = a.C;
+    constexpr bool kFilled = ROWS == kRowsFilled, kVec = ROWS != kRowsAny;
+    const int total = g.B * g.N, C = kFilled ? LPP * 4 : a.C;
     const int first = (blockIdx.x * WARPS + warp) * PP;
     bool ivalid = (unsigned)(first + sg) < (unsigned)total;
     const int i = ivalid ? first + sg : total - 1;
@@ -491,32 +501,32 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
     // v_i as the pair scalars carry it: a particle without volume has only its neighbours' terms, which v_j / v_i must be able to hold
     const float vs = fabsf(vi) < 1e-25f ? 1e-25f : vi, inv_vs = 1.0f / vs;
     const unsigned spitch = (unsigned)C * 4u, bpitch = (unsigned)a.gb_pitch * 4u, gpitch = (unsigned)a.gg_pitch * 4u;
-    const int Cp = a.cp;
+    const int Cp = kFilled ? C : a.cp;
     float dx[3] = {0.f, 0.f, 0.f};           // lane-partial over features and pairs
     unsigned long long drp = 0ull;           // minus the sum in drho, lane-partial
 
     for (int fbase = 0; fbase < C; fbase += LPP * 4) {
         __syncwarp();
-        const int f0 = fbase + sl * 4, fv = min(f0, Cp - 4);
+        const int f0 = fbase + sl * 4, fv = kFilled ? f0 : min(f0, Cp - 4);
         // the i side: s_i, gB_i, gG_i in packed pairs; a lane beyond the last feature contributes zeros (minus1: -1 where it has features)
         unsigned long long si[2] = {0ull, 0ull}, gbi[2] = {0ull, 0ull}, minus1[2] = {0ull, 0ull}, ggi[2 * D];
 #pragma unroll
         for (int q = 0; q < 2 * D; ++q) ggi[q] = 0ull;
         if (FULL) {
             float t[4];
-            load_row4<VEC>(a.s + (long long)i * C, f0, C, t);
-            const bool live[4] = {f0 < C, VEC ? f0 < C : f0 + 1 < C, VEC ? f0 < C : f0 + 2 < C, VEC ? f0 < C : f0 + 3 < C};
+            load_row4<ROWS>(a.s + (long long)i * C, f0, C, t);
+            const bool in = kFilled || f0 < C, live[4] = {in, kVec ? in : f0 + 1 < C, kVec ? in : f0 + 2 < C, kVec ? in : f0 + 3 < C};
 #pragma unroll
             for (int q = 0; q < 4; ++q) t[q] = live[q] ? t[q] : 0.f;
             si[0] = pack2(t[0], t[1]); si[1] = pack2(t[2], t[3]);
             minus1[0] = pack2(live[0] ? -1.f : 0.f, live[1] ? -1.f : 0.f);
-            minus1[1] = VEC ? minus1[0] : pack2(live[2] ? -1.f : 0.f, live[3] ? -1.f : 0.f);
-            if (kBlur && f0 < C) {
+            minus1[1] = kVec ? minus1[0] : pack2(live[2] ? -1.f : 0.f, live[3] ? -1.f : 0.f);
+            if (kBlur && in) {
                 const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gb + (long long)i * a.gb_pitch + f0));
                 gbi[0] = pack2(b.x, live[1] ? b.y : 0.f);
                 gbi[1] = pack2(live[2] ? b.z : 0.f, live[3] ? b.w : 0.f);
             }
-            if (kGrad && f0 < C) {
+            if (kGrad && in) {
 #pragma unroll
                 for (int d = 0; d < D; ++d) {
                     const float4 b = __ldg(reinterpret_cast<const float4 *>(a.gg + (long long)i * a.gg_pitch + d * Cp + f0));
@@ -567,7 +577,7 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
         struct Rows { float s[4], b[4], g[D][4]; };
         auto load = [&](int j, Rows &r) {
             const unsigned long long u = (unsigned)j;
-            if (FULL) load_row4<VEC>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + u * spitch), f0, C, r.s);
+            if (FULL) load_row4<ROWS>(reinterpret_cast<const float *>(reinterpret_cast<const char *>(a.s) + u * spitch), f0, C, r.s);
             if (kBlur) {
                 const float4 t = __ldg(reinterpret_cast<const float4 *>(reinterpret_cast<const char *>(a.gb + fv) + u * bpitch));
                 r.b[0] = t.x; r.b[1] = t.y; r.b[2] = t.z; r.b[3] = t.w;
@@ -756,14 +766,14 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
                 const float *z = a.direct + (long long)i * a.direct_pitch;
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (f0 + q < C) o[q] += __ldg(z + f0 + q);
+                    if (kFilled || f0 + q < C) o[q] += __ldg(z + f0 + q);
             }
             if (a.add && ivalid) {
 #pragma unroll
                 for (int q = 0; q < 4; ++q)
-                    if (f0 + q < C) o[q] += __ldg(a.add + (long long)i * C + f0 + q);
+                    if (kFilled || f0 + q < C) o[q] += __ldg(a.add + (long long)i * C + f0 + q);
             }
-            if (ivalid) store_row4<VEC>(a.grad_s + (long long)i * C, f0, C, o);
+            if (ivalid) store_row4<ROWS>(a.grad_s + (long long)i * C, f0, C, o);
         }
     }
     if (FULL) {
@@ -785,15 +795,15 @@ __device__ __forceinline__ void list_backward(const FeatureListBwdArgs &a, const
     }
 }
 
-template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
+template <int D, bool PER, int LPP, int ROWS, int MASK, bool FULL>
 __device__ __noinline__ void list_backward_search(const FeatureListBwdArgs &a, const Geom &g, float4 (*s_k)[ListShape<LPP, FULL && D == 3>::kSlots],
                                                   float4 (*s_e)[ListShape<LPP, FULL && D == 3>::kSlots], int4 (*s_j)[ListShape<LPP, FULL && D == 3>::kIndexQuads]) {
-    list_backward<D, PER, LPP, VEC, MASK, FULL, true>(a, g, s_k, s_e, s_j);
+    list_backward<D, PER, LPP, ROWS, MASK, FULL, true>(a, g, s_k, s_e, s_j);
 }
 
 // Features only: four CTAs with up to 16 features -- 32,768 particles are a wave and a seventh of three CTAs, 48 -> 38 us --
 // and three with longer rows, 401 us against 411.
-template <int D, bool PER, int LPP, bool VEC, int MASK, bool FULL>
+template <int D, bool PER, int LPP, int ROWS, int MASK, bool FULL>
 __global__ void __launch_bounds__(kListBackwardWarps<D, FULL> * 32, FULL ? (D == 3 ? 8 : 4) : LPP == 4 ? 4 : 3)
 feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
     after_previous_kernel();
@@ -805,20 +815,20 @@ feature_list_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const
     const int warp = threadIdx.x >> 5, total = g.B * g.N;
     const unsigned first = (blockIdx.x * WARPS + warp) * S::PP;
     if (first >= (unsigned)total) return;
-    list_backward<D, PER, LPP, VEC, MASK, FULL, false>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
+    list_backward<D, PER, LPP, ROWS, MASK, FULL, false>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
     __syncwarp();
     const int i = (int)min(first + (threadIdx.x & 31u) / LPP, (unsigned)total - 1u);
     if (__any_sync(kFull, __ldg(a.pair_cache + (long long)i * a.pair_stride) < 0))
-        list_backward_search<D, PER, LPP, VEC, MASK, FULL>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
+        list_backward_search<D, PER, LPP, ROWS, MASK, FULL>(a, g, s_k[warp], s_e[FULL ? warp : 0], s_j[warp]);
 }
 
 // ---------------------------------------------------------------------------------------------------------
 // dispatch
 // ---------------------------------------------------------------------------------------------------------
-template <int D, bool PER, int LPP, bool VEC, int MASK>
+template <int D, bool PER, int LPP, int ROWS, int MASK>
 int launch_list_forward(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
     constexpr int PP = 32 / LPP;
-    const auto kernel = feature_list_forward_kernel<D, PER, LPP, VEC, MASK>;
+    const auto kernel = feature_list_forward_kernel<D, PER, LPP, ROWS, MASK>;
     const size_t dyn = (MASK & F_PACK) ? (size_t)kListWarps * ((PP * a.zstride + 3) & ~3) * sizeof(float) : 0;
     if (dyn > 0) {
         int rc, unused = 0;
@@ -829,18 +839,18 @@ int launch_list_forward(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st)
     return check_launch("feature_list_forward_kernel");
 }
 
-template <int D, bool PER, int LPP, bool VEC>
+template <int D, bool PER, int LPP, int ROWS>
 int launch_list_forward_mask(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st) {
     switch (mask) {
-        case F_BLUR: return launch_list_forward<D, PER, LPP, VEC, F_BLUR>(g, a, st);
-        case F_GRAD: return launch_list_forward<D, PER, LPP, VEC, F_GRAD>(g, a, st);
-        case F_BLUR | F_GRAD: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD>(g, a, st);
-        case F_BLUR | F_GRAD | F_DGRAD: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_DGRAD>(g, a, st);
-        case F_BLUR | F_GRAD | F_MOMENT: return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_MOMENT>(g, a, st);
-        case F_GRAD | F_MOMENT | F_CORRECTED: return launch_list_forward<D, PER, LPP, VEC, F_GRAD | F_MOMENT | F_CORRECTED>(g, a, st);
+        case F_BLUR: return launch_list_forward<D, PER, LPP, ROWS, F_BLUR>(g, a, st);
+        case F_GRAD: return launch_list_forward<D, PER, LPP, ROWS, F_GRAD>(g, a, st);
+        case F_BLUR | F_GRAD: return launch_list_forward<D, PER, LPP, ROWS, F_BLUR | F_GRAD>(g, a, st);
+        case F_BLUR | F_GRAD | F_DGRAD: return launch_list_forward<D, PER, LPP, ROWS, F_BLUR | F_GRAD | F_DGRAD>(g, a, st);
+        case F_BLUR | F_GRAD | F_MOMENT: return launch_list_forward<D, PER, LPP, ROWS, F_BLUR | F_GRAD | F_MOMENT>(g, a, st);
+        case F_GRAD | F_MOMENT | F_CORRECTED: return launch_list_forward<D, PER, LPP, ROWS, F_GRAD | F_MOMENT | F_CORRECTED>(g, a, st);
         case F_BLUR | F_GRAD | F_MOMENT | F_PACK:
             if (a.C > LPP * 4) return fail(NPA_ERR_UNSUPPORTED, "the packed perception sweep supports up to %d features here", LPP * 4);
-            return launch_list_forward<D, PER, LPP, VEC, F_BLUR | F_GRAD | F_MOMENT | F_PACK | F_DGRAD>(g, a, st);
+            return launch_list_forward<D, PER, LPP, ROWS, F_BLUR | F_GRAD | F_MOMENT | F_PACK | F_DGRAD>(g, a, st);
         default: return fail(NPA_ERR_INVALID_ARGUMENT, "unsupported feature forward mask %d", mask);
     }
 }
@@ -854,6 +864,8 @@ int launch_list_forward_mask(const Geom &g, int mask, const FeatureFwdArgs &a, c
         if ((C) <= 64) return CALL(16);                       \
         return CALL(32);                                      \
     } while (0)
+// The counts whose rows fill the lanes of their particle.
+__host__ inline bool rows_filled(int C) { return C == 16 || C == 32 || C == 64 || C == 128; }
 
 template <int D, bool PER>
 int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdArgs &args, cudaStream_t st) {
@@ -861,24 +873,27 @@ int launch_feature_list_forward_geom(const Geom &g, int mask, const FeatureFwdAr
     FeatureFwdArgs a = args;
     a.out_vec = (uintptr_t)a.z % 16 == 0;
     if (a.C % 4 == 0 && bits % 16 == 0) {
-#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, true>(g, mask, a, st)
+#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, kRowsFilled>(g, mask, a, st)
+        if (rows_filled(a.C)) NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, kRowsVec>(g, mask, a, st)
         NPA_LIST_LPP(a.C, NPA_CALL);
 #undef NPA_CALL
     }
-#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, false>(g, mask, a, st)
+#define NPA_CALL(L) launch_list_forward_mask<D, PER, L, kRowsAny>(g, mask, a, st)
     NPA_LIST_LPP(a.C, NPA_CALL);
 #undef NPA_CALL
 }
 
-template <int D, bool PER, int LPP, bool VEC, bool FULL>
+template <int D, bool PER, int LPP, int ROWS, bool FULL>
 int launch_list_backward_mask(const Geom &g, int mask, const FeatureListBwdArgs &a, cudaStream_t st) {
     constexpr int PP = 32 / LPP, WARPS = kListBackwardWarps<D, FULL>;
     const long long particles = (long long)g.B * g.N, per_cta = (long long)WARPS * PP;
     const unsigned blocks = (unsigned)((particles + per_cta - 1) / per_cta);
     switch (mask) {
-        case F_BLUR: feature_list_backward_kernel<D, PER, LPP, VEC, F_BLUR, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
-        case F_GRAD: feature_list_backward_kernel<D, PER, LPP, VEC, F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
-        case F_BLUR | F_GRAD: feature_list_backward_kernel<D, PER, LPP, VEC, F_BLUR | F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        case F_BLUR: feature_list_backward_kernel<D, PER, LPP, ROWS, F_BLUR, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        case F_GRAD: feature_list_backward_kernel<D, PER, LPP, ROWS, F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
+        case F_BLUR | F_GRAD: feature_list_backward_kernel<D, PER, LPP, ROWS, F_BLUR | F_GRAD, FULL><<<blocks, WARPS * 32, 0, st>>>(a, g); break;
         default: return fail(NPA_ERR_INVALID_ARGUMENT, "unsupported feature backward mask %d", mask);
     }
     return check_launch("feature_list_backward_kernel");
@@ -889,11 +904,14 @@ int launch_feature_list_backward_geom(const Geom &g, int mask, const FeatureList
     // the features-only pass reads no feature row, only its output has the caller's layout
     const uintptr_t bits = (FULL ? (uintptr_t)a.s : 0) | (uintptr_t)a.grad_s;
     if (a.C % 4 == 0 && bits % 16 == 0) {
-#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, true, FULL>(g, mask, a, st)
+#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, kRowsFilled, FULL>(g, mask, a, st)
+        if (rows_filled(a.C) && a.cp == a.C) NPA_LIST_LPP(a.C, NPA_CALL);
+#undef NPA_CALL
+#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, kRowsVec, FULL>(g, mask, a, st)
         NPA_LIST_LPP(a.C, NPA_CALL);
 #undef NPA_CALL
     }
-#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, false, FULL>(g, mask, a, st)
+#define NPA_CALL(L) launch_list_backward_mask<D, PER, L, kRowsAny, FULL>(g, mask, a, st)
     NPA_LIST_LPP(a.C, NPA_CALL);
 #undef NPA_CALL
 }

@@ -16,7 +16,8 @@
 //
 // Bound by instruction issue and latency together (~1,700 warp instructions per two particles with 41 pairs, a third of
 // them the pairs themselves, half of the issue slots at 14.5 warps per SM).  Measured, B200, us, the sweep with the whole
-// warp per particle -> this one: 262,144 particles in 3D, C = 32, ~41 pairs 495 -> 417; 32,768 in 2D, C = 16, ~31 pairs 36.
+// warp per particle -> this one: 262,144 particles in 3D, C = 32, ~41 pairs 495 -> 417, with rows that
+// fill their lanes (feature_list.cuh) 371; 32,768 in 2D, C = 16, ~31 pairs 36 -> 33.
 // Not kept: eight lanes per particle with all classes in registers (420, but 42 in 2D), sixteen with every class of one or two
 // features (492), five CTAs per SM in 3D (432, spills).
 #pragma once
@@ -47,12 +48,14 @@ __device__ inline float spiky_phi_rounded(float q, float h) {
     return quotient_rounded(3.0f * t * t, r);
 }
 
-template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
+template <int D, bool PER, int VW, int LPR, int CPL, int ROWS>
 struct Ordered {
     static constexpr int NM = D * (D + 1) / 2, H = VW / 2;
     static constexpr int G = 16 / LPR, CLS = G * CPL;  // groups of a particle, classes
     static constexpr int U = 4, STEP = U / CPL * CLS;  // rows in flight per lane, entries they stand for
     static constexpr int OWN = VW > G ? VW / G : 1;    // features a lane ends with
+    static constexpr bool ALIGNED = ROWS != kRowsAny, FILLED = ROWS == kRowsFilled;
+    static __device__ inline int features(const FeatureFwdArgs &a) { return FILLED ? VW * LPR : a.C; }
     float si[VW];
     unsigned long long nsi[H], acc[CPL][1 + D][H];
     float mom[2][NM], dgs[2][3];
@@ -76,12 +79,12 @@ struct Ordered {
     }
     // Lanes beyond the last feature read valid neighbours of it (unused).
     static __device__ inline void load(const float *__restrict__ row, int f, int C, float (&v)[VW]) {
-        if (ALIGNED && C % VW == 0) {
+        if (FILLED || (ALIGNED && C % VW == 0)) {
             if constexpr (VW == 4) {
-                const float4 t = __ldg(reinterpret_cast<const float4 *>(row + min(f, C - 4)));
+                const float4 t = __ldg(reinterpret_cast<const float4 *>(row + (FILLED ? f : min(f, C - 4))));
                 v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
             } else {
-                const float2 t = __ldg(reinterpret_cast<const float2 *>(row + min(f, C - 2)));
+                const float2 t = __ldg(reinterpret_cast<const float2 *>(row + (FILLED ? f : min(f, C - 2))));
                 v[0] = t.x; v[1] = t.y;
             }
         } else {
@@ -138,7 +141,7 @@ struct Ordered {
     template <bool WIDE>
     __device__ inline void finish(const FeatureFwdArgs &a, const Geom &g, long long i, bool valid, int f, int sl, float *zs) {
         constexpr int L = WIDE ? 32 : 16;
-        const int C = a.C;
+        const int C = features(a);
         float m[NM], dg[3] = {0.f, 0.f, 0.f}, inv[D * D];
 #pragma unroll
         for (int q = 0; q < NM; ++q) m[q] = g.c_g * subgroup_sum<L>(WIDE ? mom[0][q] : mom[0][q] + mom[1][q]);
@@ -192,7 +195,7 @@ struct Ordered {
 #pragma unroll
             for (int d = 0; d < D; ++d) w[d] *= a.coef;
             if (a.log_norm_grad) log_normalize<D>(w);
-            if (f + v < C) {
+            if (FILLED || f + v < C) {
                 zs[f + v] = si[v];
                 zs[C + f + v] = g.c_s * val[v][0];
 #pragma unroll
@@ -202,7 +205,7 @@ struct Ordered {
         if (a.vgrad && valid) {
             float *o = a.vgrad + (i * C + f) * D;
             if (ALIGNED && OWN == 2 && C % 2 == 0) {
-                if (f < C) {
+                if (FILLED || f < C) {
                     auto at = [&](int e) { return val[e / D][1 + e % D]; };
 #pragma unroll
                     for (int k = 0; k < D; ++k) reinterpret_cast<float2 *>(o)[k] = make_float2(at(2 * k), at(2 * k + 1));
@@ -232,10 +235,10 @@ struct Ordered {
 
 // One particle by the whole warp, through the candidates of its cells (the two halves of the warp sum the features
 // alike).  Out of line, so that it costs the walk over lists no registers.
-template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
+template <int D, bool PER, int VW, int LPR, int CPL, int ROWS>
 __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom &g, OrderedMem &mem, int i) {
-    using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
-    const int lane = threadIdx.x & 31, sl = lane & 15, f = sl % LPR * VW, at = sl / LPR * CPL, C = a.C, sys = i / g.N;
+    using O = Ordered<D, PER, VW, LPR, CPL, ROWS>;
+    const int lane = threadIdx.x & 31, sl = lane & 15, f = sl % LPR * VW, at = sl / LPR * CPL, C = Ordered<D, PER, VW, LPR, CPL, ROWS>::features(a), sys = i / g.N;
     const Pos<D> pi = load_pos<D>(a.x, i);
     WorkItem it = {i, 1, 0, sys};
     it.cell = sys * g.cells + (int)snapshot_cell(g, a.bin_offsets + (size_t)sys * g.cells, i,
@@ -274,18 +277,18 @@ __device__ __noinline__ void ordered_search(const FeatureFwdArgs &a, const Geom 
     __syncwarp();
 }
 
-template <int D, bool PER, int VW, int LPR, int CPL, bool ALIGNED>
+template <int D, bool PER, int VW, int LPR, int CPL, int ROWS>
 __global__ void __launch_bounds__(kOrderedWarps * 32, D == 2 ? 10 : 8)
 packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_constant__ Geom g) {
     after_previous_kernel();
-    using O = Ordered<D, PER, VW, LPR, CPL, ALIGNED>;
+    using O = Ordered<D, PER, VW, LPR, CPL, ROWS>;
     __shared__ OrderedMem s_mem[kOrderedWarps];
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, sg = lane >> 4, sl = lane & 15;
     const int total = g.B * g.N, first = (int)((blockIdx.x * kOrderedWarps + warp) * 2u);
     if ((unsigned)first >= (unsigned)total) return;
     OrderedMem &mem = s_mem[warp];
     const bool valid = sg < total - first;
-    const int i = valid ? first + sg : total - 1, C = a.C, f = sl % LPR * VW, at = sl / LPR * CPL;
+    const int i = valid ? first + sg : total - 1, C = O::features(a), f = sl % LPR * VW, at = sl / LPR * CPL;
     const int32_t *list = a.pair_cache + (long long)i * a.pair_stride;
     const int room = a.vgrad ? min(a.pair_stride - 1, kOrderedPairs) : a.pair_stride - 1;
     const int count = __ldg(list++);
@@ -345,29 +348,34 @@ packed_ordered_kernel(const __grid_constant__ FeatureFwdArgs a, const __grid_con
         }
         __syncwarp();
     }
-    const int Z = a.zstride;
+    const int Z = O::FILLED ? (2 + D) * C + D : a.zstride;
     o.template finish<false>(a, g, i, valid && !search, f, sl, mem.rows + sg * Z);
     __syncwarp();
     // the rows of both particles are one run (8-byte aligned when z is: first is even); the row of a particle that is
     // searched is written again below
     const int floats = min(2, total - first) * Z;
     float *out = a.z + (long long)first * Z;
-    if (ALIGNED) {
+    if (O::ALIGNED) {
         for (int q = lane; q < floats / 2; q += 32) reinterpret_cast<float2 *>(out)[q] = reinterpret_cast<const float2 *>(mem.rows)[q];
         if ((floats & 1) && lane == 0) out[floats - 1] = mem.rows[floats - 1];
     } else {
         for (int q = lane; q < floats; q += 32) out[q] = mem.rows[q];
     }
     const unsigned again = __ballot_sync(kFull, search && valid);
-    if (again & 0x0000ffffu) ordered_search<D, PER, VW, LPR, CPL, ALIGNED>(a, g, mem, first);
-    if (again & 0xffff0000u) ordered_search<D, PER, VW, LPR, CPL, ALIGNED>(a, g, mem, first + 1);
+    if (again & 0x0000ffffu) ordered_search<D, PER, VW, LPR, CPL, ROWS>(a, g, mem, first);
+    if (again & 0xffff0000u) ordered_search<D, PER, VW, LPR, CPL, ROWS>(a, g, mem, first + 1);
 }
 
-// ALIGNED: the addresses of the feature rows, of z and of vgrad allow the vector accesses of the shape.
+// ROWS (feature_list.cuh): kRowsAny where the addresses of the feature rows, of z or of vgrad do not allow the vector accesses of the
+// shape, kRowsFilled where the lanes of a row cover it exactly.
 template <int D, bool PER, int VW, int LPR, int CPL>
 int launch_packed_ordered_shape(const Geom &g, const FeatureFwdArgs &a, cudaStream_t st) {
     const bool aligned = (a.C % VW != 0 || (uintptr_t)a.s % (VW * 4) == 0) && ((uintptr_t)a.z | (uintptr_t)a.vgrad) % 8 == 0;
-    const auto kernel = aligned ? packed_ordered_kernel<D, PER, VW, LPR, CPL, true> : packed_ordered_kernel<D, PER, VW, LPR, CPL, false>;
+    auto kernel = packed_ordered_kernel<D, PER, VW, LPR, CPL, kRowsAny>;
+    if (aligned) kernel = packed_ordered_kernel<D, PER, VW, LPR, CPL, kRowsVec>;
+    if constexpr (VW == 4) {
+        if (aligned && a.C == VW * LPR) kernel = packed_ordered_kernel<D, PER, VW, LPR, CPL, kRowsFilled>;
+    }
     const long long particles = (long long)g.B * g.N;
     launch_early(kernel, (unsigned)((particles + 2 * kOrderedWarps - 1) / (2 * kOrderedWarps)), kOrderedWarps * 32, 0, st, a, g);
     return check_launch("packed_ordered_kernel");

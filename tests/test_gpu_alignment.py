@@ -50,6 +50,29 @@ def test_packed_perception_of_features_at_any_address(dim, C, offset):
         impl._PAIR_CACHE["columns"] = before
 
 
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("C", [16, 32, 64, 128])        # rows that fill the lanes of their particle
+def test_perception_of_features_at_any_address(dim, C):
+    """The kernels that know the feature count and those that read float by float add the same products in the same order."""
+    from npa_b200.sphops import sph as impl
+    sph, grid, snap, xb, sb = _setup(dim, C, "periodic")
+    before = impl._PAIR_CACHE["columns"]
+    try:
+        for columns in (128, 16):                       # 16: particles with more neighbours are searched for
+            impl._PAIR_CACHE["columns"] = columns
+            res, ups = [], None
+            for offset in (0, 1):
+                x, s = xb.detach().requires_grad_(True), _at(sb, offset).requires_grad_(True)
+                out = sph.perceive(x, s, snap)
+                ups = ups or [torch.randn_like(o) for o in out]
+                res.append([*out, *torch.autograd.grad(out, [x, s], ups, retain_graph=True), torch.autograd.grad(out[1:3], s, ups[1:3])[0]])
+            for a, b in zip(*res):
+                assert torch.allclose(a, b, rtol=1e-5, atol=1e-6 * float(a.abs().max()))
+            assert all(torch.equal(a, b) for a, b in zip(res[0][:4], res[1][:4]))
+    finally:
+        impl._PAIR_CACHE["columns"] = before
+
+
 @pytest.mark.parametrize("C", [8, 16, 64])
 def test_packed_perception_into_outputs_at_any_address(C):
     sph, grid, snap, xb, sb = _setup(2, C)
