@@ -8,8 +8,8 @@
 //  * histograms use warp-aggregated atomics, held in shared memory when the
 //    per-system cell table fits, so a cell-coherent input (every step after the
 //    first of a rollout) does not serialise on one address;
-//  * cell counts and work-item counts are scanned together in one three-phase
-//    scan, and the work list is written by the scan's last phase.
+//  * cell counts and work-item counts are scanned together, and the work list
+//    is written by the scan's last phase.
 // All kernels are HBM-bound integer work; nothing here is GEMM shaped.
 #include <cooperative_groups.h>
 
@@ -21,12 +21,17 @@
 namespace npa {
 
 constexpr int kBinThreads = 256;
-constexpr int kBinPerThread = 8;                       // particles per thread in the hash pass
-constexpr int kBinChunk = kBinThreads * kBinPerThread;  // particles per CTA
+// Particles per thread in the hash pass: as many as share a shared-memory histogram well, and one where the atomics go to global memory:
+// each is a round trip that the next waits for, and eight after another were all of the pass (65,536 and 524,288 particles in 3D 14.5 and
+// 15 us,
+// now 4.2 and 6.6).
+template <bool SMEM>
+constexpr int kBinPerThread = SMEM ? 8 : 1;
 constexpr int kSmemHistCells = 8192;                   // 32 KB of shared histogram at most
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = 8;
 constexpr int kScanTile = kScanThreads * kScanPerThread;
+constexpr int kScanPartials = 4096;  // up to so many tiles every CTA of scan_apply_kernel adds up the tiles before its own by itself
 // Cells with more particles than this are ranked by rank_crowded_kernel (linear in the population)
 // instead of the per-particle scan of rank_kernel (quadratic in it).
 constexpr int kCrowdedCell = 256;
@@ -112,6 +117,13 @@ __device__ inline uint32_t warp_aggregated_take(uint32_t *hist, uint32_t key, bo
     return base + (uint32_t)__popc(peers & ((1u << lane) - 1));
 }
 
+// The counts of a build start at zero.  A kernel and not a memset, so that its launch and that of the next overlap.
+__global__ void __launch_bounds__(kBinThreads) zero_counts_kernel(uint4 *__restrict__ counts, size_t quads) {
+    after_previous_kernel();
+    for (size_t q = blockIdx.x * (size_t)kBinThreads + threadIdx.x; q < quads; q += (size_t)gridDim.x * kBinThreads)
+        counts[q] = make_uint4(0u, 0u, 0u, 0u);
+}
+
 template <int D, bool SMEM>
 __global__ void __launch_bounds__(kBinThreads)
 hash_count_kernel(const float *__restrict__ x, uint32_t *__restrict__ cellid, uint32_t *__restrict__ arrive,
@@ -119,46 +131,54 @@ hash_count_kernel(const float *__restrict__ x, uint32_t *__restrict__ cellid, ui
     after_previous_kernel();
     extern __shared__ uint32_t hist[];
     const int b = blockIdx.y;
-    const int base = blockIdx.x * kBinChunk;
+    constexpr int PT = kBinPerThread<SMEM>;
+    const int base = blockIdx.x * kBinThreads * PT;
     if (SMEM) {
         for (int c = threadIdx.x; c < g.cells; c += kBinThreads) hist[c] = 0;
         __syncthreads();
     }
     uint32_t *gl = counts + (size_t)b * g.cells;
-    uint32_t keys[kBinPerThread], arr[kBinPerThread];
+    uint32_t keys[PT], arr[PT];
 #pragma unroll
-    for (int k = 0; k < kBinPerThread; ++k) {
+    for (int k = 0; k < PT; ++k) {
         const int i = base + k * kBinThreads + threadIdx.x;
-        const bool valid = i < g.N;
-        uint32_t key = 0;
-        if (valid) {
-            const size_t idx = (size_t)b * g.N + i;
-            key = particle_cell<D>(x, idx, g);
-            cellid[idx] = key;
-        }
-        keys[k] = key;
-        arr[k] = warp_aggregated_take(SMEM ? hist : gl, key, valid);
+        keys[k] = i < g.N ? particle_cell<D>(x, (size_t)b * g.N + i, g) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < PT; ++k) {
+        const int i = base + k * kBinThreads + threadIdx.x;
+        if (i < g.N) cellid[(size_t)b * g.N + i] = keys[k];
+        arr[k] = warp_aggregated_take(SMEM ? hist : gl, keys[k], i < g.N);
     }
     if (SMEM) {
         // the CTA's populations go to the global counters in one atomic per cell; the old values
         // (where this CTA's particles start in the cell) replace the local counts
         __syncthreads();
-        for (int c = threadIdx.x; c < g.cells; c += kBinThreads) {
-            const uint32_t v = hist[c];
-            hist[c] = v ? atomicAdd(&gl[c], v) : 0u;
+        for (int c0 = threadIdx.x; c0 < g.cells; c0 += kBinThreads * 8) {  // eight round trips at a time
+            uint32_t v[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) {
+                const int c = c0 + u * kBinThreads;
+                v[u] = c < g.cells ? hist[c] : 0u;
+                if (v[u]) v[u] = atomicAdd(&gl[c], v[u]);
+            }
+#pragma unroll
+            for (int u = 0; u < 8; ++u)
+                if (c0 + u * kBinThreads < g.cells) hist[c0 + u * kBinThreads] = v[u];
         }
         __syncthreads();
     }
 #pragma unroll
-    for (int k = 0; k < kBinPerThread; ++k) {
+    for (int k = 0; k < PT; ++k) {
         const int i = base + k * kBinThreads + threadIdx.x;
         if (i < g.N) arrive[(size_t)b * g.N + i] = arr[k] + (SMEM ? hist[keys[k]] : 0u);
     }
 }
 
 // ---------------------------------------------------------------------------
-// Three-phase exclusive scan of (particles per cell, work items per cell),
-// packed as one 64-bit word so both prefix sums ride the same shuffles.
+// Exclusive scan of (particles per cell, work items per cell), packed as one 64-bit word so both prefix sums ride the same shuffles:
+// the sums of tiles of cells, then in each tile the sum of the tiles before it and the cells' own prefixes (of more than
+// kScanPartials tiles the sums are scanned in a launch between).
 // ---------------------------------------------------------------------------
 __device__ inline unsigned long long pack_cell(uint32_t count, int mpb) {
     uint32_t blocks = (count + (uint32_t)mpb - 1) / (uint32_t)mpb;
@@ -231,13 +251,41 @@ scan_partials_kernel(unsigned long long *partials, int tiles) {
 }
 
 // Writes bin_offsets, the work list rows of every non-empty cell, and zeroes
-// the unused tail of the work list (rows [total_items, max_blocks)).
+// the unused tail of the work list (rows [total_items, max_blocks)).  SCANNED: the partial sums are prefixes already, the grand total last.
+template <bool SCANNED>
 __global__ void __launch_bounds__(kScanThreads)
 scan_apply_kernel(const uint32_t *__restrict__ counts, const unsigned long long *__restrict__ partials,
                   int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, uint32_t *__restrict__ crowded,
                   uint32_t *__restrict__ crowded_count, int n, Geom g) {
     after_previous_kernel();
-    __shared__ unsigned long long tot;
+    __shared__ unsigned long long tot, sums[2][kScanThreads / 32];
+    unsigned long long before = 0, grand = 0;  // the tiles before this one, all tiles
+    if (SCANNED) {
+        before = partials[blockIdx.x];
+        grand = partials[gridDim.x];
+    } else {
+        for (int t = threadIdx.x; t < (int)gridDim.x; t += kScanThreads) {
+            const unsigned long long v = partials[t];
+            grand += v;
+            if (t < (int)blockIdx.x) before += v;
+        }
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            before += __shfl_xor_sync(kFull, before, o);
+            grand += __shfl_xor_sync(kFull, grand, o);
+        }
+        if ((threadIdx.x & 31) == 0) {
+            sums[0][threadIdx.x >> 5] = before;
+            sums[1][threadIdx.x >> 5] = grand;
+        }
+        __syncthreads();
+        before = grand = 0;
+#pragma unroll
+        for (int w = 0; w < kScanThreads / 32; ++w) {
+            before += sums[0][w];
+            grand += sums[1][w];
+        }
+    }
     const int base = blockIdx.x * kScanTile + threadIdx.x * kScanPerThread;
     uint32_t c[kScanPerThread];
     unsigned long long v = 0;
@@ -246,7 +294,7 @@ scan_apply_kernel(const uint32_t *__restrict__ counts, const unsigned long long 
         c[k] = base + k < n ? counts[base + k] : 0u;
         v += pack_cell(c[k], g.mpb);
     }
-    unsigned long long run = partials[blockIdx.x] + block_exclusive<kScanThreads>(v, tot);
+    unsigned long long run = before + block_exclusive<kScanThreads>(v, tot);
 #pragma unroll
     for (int k = 0; k < kScanPerThread; ++k) {
         const int cell = base + k;
@@ -261,7 +309,6 @@ scan_apply_kernel(const uint32_t *__restrict__ counts, const unsigned long long 
         }
         run += pack_cell(c[k], g.mpb);
     }
-    const unsigned long long grand = partials[gridDim.x];
     if (blockIdx.x == 0 && threadIdx.x == 0) bin_offsets[n] = (int32_t)(uint32_t)grand;
     const int total_items = (int)(grand >> 32);
     for (int r = total_items + blockIdx.x * kScanThreads + threadIdx.x; r < g.max_blocks;
@@ -375,9 +422,8 @@ rank_kernel(const uint32_t *__restrict__ cellid, const int32_t *__restrict__ bin
 
 // ---------------------------------------------------------------------------
 // Small systems: everything but the work list in one launch, a CTA per system with the cell table, the cell ids and the
-// slots in shared memory.  The general path is seven dependent launches of 1.5-11 us each for 8 x 4,096 particles
-// (31 us, and a host that needs 35-40 us to issue them): what bounds it there is launch latency and the serial atomics
-// of few CTAs, not memory.  With the work list's launch this takes 13 us (9.2 + 3.7), 6.5 for one system of 2,500.
+// slots in shared memory.  The general path is six dependent launches of 1.5-8 us each for 8 x 4,096 particles
+// (21 us): what bounds it there is launch latency, not memory.  With the work list's launch this takes 13 us (9.2 + 3.7), 6.5 for one system of 2,500.
 // ---------------------------------------------------------------------------
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallParticles = 16384;
@@ -397,12 +443,12 @@ static size_t small_smem(const Geom &g) {
 //    global memory, where long runs per thread scatter the loads.
 //  * Cluster, eight CTAs per system: a fixed part; the share of a CTA; ranking among the share's particles of a cell; the systems, and
 //    the cells where there are more CTAs than SMs; the rows as above.
-//  * General: six launches; the shared histogram; the particles and cells of all systems; ranking, spread over the chip; crowded cells.
-// Small and general were fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells), cluster, crowded
-// cells and the launches of the general way, which overlap on a stream, to 600 sizes (2,500 to 65,536 particles, 1 to 32 systems, 9 to
-// 32,768 cells) on a stream and in a graph: 0.2 % behind the best way on average, 14 % at worst.  Some sizes, small / cluster /
-// general, us, in a graph: 1 system of 2,500 in 10 x 10 7.6 / 8.4 / 23; 1 of 16,384 in 3^3 48 / 19 / 35; 32 of 8,192 in 100 x 100
-// 24 / 26 / 32; 1 of 65,536 in 6 x 6 - / 63 / 43, in 3 x 3 - / 54 / 102; 1 of 30,000 in 32^3 - / 28 / 25; 2 of 4,096 in 32^3 77 / 76 / 24.
+//  * General: six launches (seven beyond kScanPartials tiles of cells); the shared histogram; the particles and cells of all systems; ranking, spread over the chip; crowded cells.
+// Small was fitted to 560 sizes (2D and 3D, 256 to 16,384 particles, 1 to 64 systems, 16 to 32,768 cells), cluster and general, whose
+// launches overlap on a stream, to 777 sizes (2,500 to 65,536 particles, 1 to 32 systems, 9 to 32,768 cells) on a stream and in a graph:
+// 0.3 % behind the best way on average, 16 % at worst.  Some sizes, small / cluster / general, us, in a graph: 1 system of 2,500 in
+// 10 x 10 7.7 / 8.1 / 20; 8 of 4,096 in 16 x 16 13 / 11 / 22; 8 of 16,384 in 40 x 40 27 / 14 / 25; 4 of 16,384 in 32^3 - / 86 / 17;
+// 2 of 30,000 in 24^3 - / 33 / 17; 1 of 65,536 in 64 x 64 - / 20 / 25, in 16 x 16 - / 24 / 39.
 enum class GridBuild { kSmall, kCluster, kGeneral };
 
 static double rows_estimate(const Geom &g) {
@@ -418,9 +464,9 @@ static GridBuild grid_build(const Geom &g) {
     const double none = 1e30;
     const bool fits = g.N <= kSmallParticles && g.cells < 65536 && small_smem(g) <= kSmallSmem;
     const double small = fits ? 4.0 + n / 900.0 + (per_cell > kCrowdedCell ? 10.0 : ranking / 54000.0) + rows_estimate(g) : none;
-    const double crowded = per_cell > kCrowdedCell ? 4.0 + per_cell * 0.008 + all * 5e-5 + per_cell * g.B * 8e-4 : 0.0;
-    const double general = 19.0 + (n < 2048.0 ? n / 256.0 : 8.0) + (g.cells <= kSmemHistCells ? c / 800.0 : 0.0) +
-                           (all > 1e5 ? (all - 1e5) / 30000.0 : 0.0) + c * g.B / 150000.0 + ranking * g.B * 3.3e-7 + crowded;
+    const double crowded = per_cell > 0.9 * kCrowdedCell ? 1.6 + per_cell * 0.0078 + all * 8.3e-5 : 0.0;  // (half of the cells, at the mean)
+    const double general = 14.5 + (g.cells <= kSmemHistCells ? 6.6 + c / 8400.0 : 0.0) + all / 35000.0 + c * g.B / 123000.0 +
+                           ranking * g.B * 3.05e-7 + crowded;
     const bool shares = g.N > 2048 && g.N <= 65536 && g.cells < 65536 && cluster_smem(g, kClusterCtas) <= kClusterSmem;
     const double share_ranking = per_cell > kCrowdedCell * kClusterCtas ? 19.0 : n * per_cell / 2.6e6;
     const double beyond = kClusterCtas * g.B > 148 ? c * (kClusterCtas * g.B - 148) / 160000.0 : 0.0;  // CTAs beyond one per SM
@@ -888,7 +934,8 @@ int npa_grid_build_kernels(const npa_grid *gd) {
     Geom g;
     const int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
-    return grid_build(g) == GridBuild::kGeneral ? 6 : g.B == 1 ? 1 : 2;
+    if (grid_build(g) != GridBuild::kGeneral) return g.B == 1 ? 1 : 2;
+    return ((long long)g.B * g.cells + kScanTile - 1) / kScanTile > kScanPartials ? 7 : 6;
 }
 
 int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int32_t *bin_offsets,
@@ -931,11 +978,14 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
         launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         return check_launch("rows_small_kernel");
     }
-    cudaError_t e = cudaMemsetAsync(s.counts, 0, s.zero_bytes, st);
-    if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "cudaMemsetAsync(scratch): %s", cudaGetErrorString(e));
+    const size_t quads = s.zero_bytes / 16;  // (a multiple of 256 bytes)
+    const size_t zero_ctas = (quads + kBinThreads - 1) / kBinThreads;
+    launch_early(zero_counts_kernel, (unsigned)(zero_ctas < 148 * 8 ? zero_ctas : 148 * 8), kBinThreads, 0, st, reinterpret_cast<uint4 *>(s.counts), quads);
+    if ((rc = check_launch("zero_counts_kernel")) != NPA_OK) return rc;
 
-    const dim3 pgrid((g.N + kBinChunk - 1) / kBinChunk, g.B);
     const bool smem = g.cells <= kSmemHistCells;
+    const int per_cta = kBinThreads * (smem ? kBinPerThread<true> : kBinPerThread<false>);
+    const dim3 pgrid((g.N + per_cta - 1) / per_cta, g.B);
     const size_t smem_bytes = smem ? (size_t)g.cells * 4 : 0;
     if (g.dim == 2) {
         if (smem) launch_early(hash_count_kernel<2, true>, pgrid, kBinThreads, smem_bytes, st, x, s.cellid, s.arrive, s.counts, g);
@@ -949,11 +999,14 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     const int n = g.B * g.cells;
     launch_early(scan_tile_sums_kernel, s.tiles, kScanThreads, 0, st, s.counts, s.partials, n, g.mpb);
     if ((rc = check_launch("scan_tile_sums_kernel")) != NPA_OK) return rc;
-    launch_early(scan_partials_kernel, 1, 1024, 0, st, s.partials, s.tiles);
-    if ((rc = check_launch("scan_partials_kernel")) != NPA_OK) return rc;
+    const bool scanned = s.tiles > kScanPartials;
+    if (scanned) {
+        launch_early(scan_partials_kernel, 1, 1024, 0, st, s.partials, s.tiles);
+        if ((rc = check_launch("scan_partials_kernel")) != NPA_OK) return rc;
+    }
     uint32_t *crowded_count = s.counts + (size_t)n + 1;
-    launch_early(scan_apply_kernel, s.tiles, kScanThreads, 0, st, s.counts, s.partials, bin_offsets,
-                                                        reinterpret_cast<int4 *>(block_info), s.crowded, crowded_count, n, g);
+    launch_early(scanned ? scan_apply_kernel<true> : scan_apply_kernel<false>, s.tiles, kScanThreads, 0, st, s.counts, s.partials, bin_offsets,
+                 reinterpret_cast<int4 *>(block_info), s.crowded, crowded_count, n, g);
     if ((rc = check_launch("scan_apply_kernel")) != NPA_OK) return rc;
 
     const dim3 tgrid((g.N + kBinThreads - 1) / kBinThreads, g.B);

@@ -163,6 +163,19 @@ def test_either_way_of_the_grid_build(dim, B, N, cells):
     _check(sph, w, x)
 
 
+@pytest.mark.parametrize("dim,B,N,cells", [
+    (3, 1, 131073, 8), (2, 1, 70001, 90), (3, 2, 65537, 20),    # histogram in shared memory, two sizes; in global memory
+    (3, 5, 300, 128)])                                          # 5,120 tiles of cells: their sums scanned by a launch of their own
+@pytest.mark.parametrize("spread", [1.05, 0.02])
+def test_general_launches(dim, B, N, cells, spread):
+    from npa_b200 import sphops as sph
+    w = Workload("general", dim=dim, B=B, N=N, C=4, eps=1.0 / cells, grid_size=(cells,) * dim, max_particles_per_block=32)
+    assert make_grid(sph, w).hashgrid.build_kernels == (7 if cells == 128 else 6)
+    x = (torch.rand(B, N, w.P, generator=torch.Generator().manual_seed(cells)) - 0.5) * spread
+    _check(sph, w, x)
+    _check(sph, w, x.flip(1).contiguous())      # the same sizes again: memory that has been counted in
+
+
 @pytest.mark.parametrize("dim,B,N,cells,hash_mode,boundary", [
     (2, 1, 4096, 10, "grid", "periodic"), (2, 3, 4097, 5, "grid", "clamped"), (2, 1, 65536, 64, "grid", "clamped"), (2, 2, 65535, 33, "grid", "periodic"),
     (3, 1, 16384, 32, "particle", "clamped"), (3, 2, 20001, 16, "particle", "periodic"), (3, 5, 2501, 3, "grid", "clamped")])
