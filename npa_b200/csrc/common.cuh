@@ -57,9 +57,8 @@ int check_launch(const char *what);
 // Plain launches, because they were slower this way:
 //  * feature_list.cuh, forward and backward (rollout of 2 x 262,144 particles 3,116 -> 3,344 us): they live off L1, and a CTA that takes
 //    its place early finds the SM divided between L1 and shared memory as the kernel before wanted it;
-//  * the reduction of the weight gradients (training step in 2D 207 -> 252 us): early, its 170 CTAs are placed three to an SM on the
-//    sixty SMs that the gradient kernel leaves first, and those that read dW2's partial sums across rows, neighbours in the grid,
-//    take 16-40 us there instead of 3-7 (measured per CTA with the global timer);
+//  * the reduction of the weight gradients (3D step of 262,144 particles 1,544 -> 1,552 us, its kernel and the one behind it together: it
+//    takes room beside the gradient kernel's CTAs that the next kernel would have had);
 //  * the hidden gradient of the MLP (3D step 1,615 -> 1,643 us, not explained).
 // Plain and not measured otherwise: the searching sweeps of feature_kernels.cuh and scalar_ops.cu, the cell-tile engine, the paths of
 // mlp_gemm.cu and mlp_grad.cu, small conversions.  The density searches, the packed sweep and the sweeps of scalar_list.cu are launched
