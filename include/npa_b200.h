@@ -498,6 +498,14 @@ int npa_mlp_weight_grad(const float *z, const float *dh, const float *h, const f
 int npa_mlp_hidden_grad(const float *dy, const float *W2, const float *h, float *dh, int64_t rows,
                         int32_t hidden, int32_t out_dim, int64_t w_stride_out, int64_t w_stride_in, void *stream);
 
+/* npa_step_update_backward (mask: 0 / 1 per particle, or with `uniforms` set values that update where they are below
+ * update_below; NULL = all) and npa_mlp_hidden_grad of its result in one pass: g_y [B*N, D + C] and dh [B*N, 128] from the
+ * upstream gradients of the updated positions and states (either may be NULL = zero).  D + C <= 48. */
+int npa_step_hidden_grad(const npa_grid *g, const float *y, const float *mask, int32_t uniforms, float update_below,
+                         int32_t channels, float alpha, float dt, const float *g_x_out, const float *g_s_out, const float *W2,
+                         const float *h, float *g_y, float *dh, int32_t hidden, int64_t w_stride_out, int64_t w_stride_in,
+                         void *stream);
+
 /* The same three reductions on the fifth-generation tensor cores (tcgen05.mma, TF32 head / tail
  * products, accumulators in tensor memory drained into fp32 partial sums every 128 rows so that no
  * accumulation chain of the tensor cores is longer than 48 MMAs).  Same arguments and results as

@@ -6,34 +6,11 @@
 // torch kernels over [B,N,D+C] -- and optionally HashGrid.wrap_positions (sphops/sph.py:107-123).
 // `y` is the MLP output in cell order, [B*N, D + C]: the first D columns are the raw displacement,
 // the rest the state update.  One thread per four elements of y; HBM bound (every tensor is read or
-// written once: 4(D+C) + 8P + 8C + 4 bytes per particle).
-#include "ops.cuh"
+// written once: 4(D+C) + 8P + 8C + 4 bytes per particle).  In a whole step the backward is part of the MLP's
+// hidden gradient (mlp_hidden_grad.cu).
+#include "step_update.cuh"
 
 namespace npa {
-
-struct StepArgs {
-    const float *y;       // [BN, D + C]
-    const float *x_bin;   // [BN, P]
-    const float *s_bin;   // [BN, C]
-    const float *mask;    // [BN] (0 / 1, or uniforms) or NULL = every particle updates
-    int uniforms;         // mask holds uniforms: a particle updates where its value is below `below`
-    float below;
-    float *x_out;         // [BN, P]
-    float *s_out;         // [BN, C]
-    const float *g_x_out; // backward: upstream of x_out [BN, P]
-    const float *g_s_out; // backward: upstream of s_out [BN, C]
-    float *g_y;           // backward: [BN, D + C]
-    long long particles;
-    int C;
-    float alpha, eps, dt;
-    int wrap;
-};
-
-__device__ inline float mask_of(const StepArgs &a, long long i) {
-    if (!a.mask) return 1.0f;
-    const float m = __ldg(a.mask + i);
-    return a.uniforms ? (m < a.below ? 1.0f : 0.0f) : m;
-}
 
 // remainder(x + L/2, L) - L/2 with torch's sign convention (result of remainder in [0, L)).
 __device__ inline float wrap_axis(float x, float L) {
@@ -66,31 +43,6 @@ __device__ inline void step_forward_element(const StepArgs &a, const Geom &g, lo
         a.x_out[i * P + c] = xo;
         if (D == 3 && c == 0) a.x_out[i * P + 3] = __ldg(a.x_bin + i * P + 3);  // padding column
     }
-}
-
-// dL/dy of one element.  The limiter f(u) = k u / (1 + |u|), k = alpha * eps, has the Jacobian
-//   df_a/du_b = k [ delta_ab / (1 + n) - u_a u_b / (n (1 + n)^2) ],  n = |u|  (second term 0 at n = 0,
-// as torch's norm backward); the wrap and the additions are the identity for gradients.
-template <int D>
-__device__ inline float step_backward_element(const StepArgs &a, long long i, int c) {
-    constexpr int P = D == 2 ? 2 : 4;
-    const float m = mask_of(a, i);
-    if (c >= D) return a.g_s_out ? (a.dt * m) * __ldg(a.g_s_out + i * a.C + (c - D)) : 0.f;
-    if (!a.g_x_out) return 0.f;
-    const float *row = a.y + i * (D + a.C);
-    float n2 = 0.f, gu = 0.f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) {
-        const float t = __ldg(row + d);
-        n2 = fmaf(t, t, n2);
-        gu = fmaf(t, __ldg(a.g_x_out + i * P + d), gu);
-    }
-    const float n = sqrtf(n2);
-    const float k = a.alpha * a.eps * a.dt * m;
-    const float inv = 1.0f / (1.0f + n);
-    float out = __ldg(a.g_x_out + i * P + c) * inv;
-    if (n > 0.f) out -= __ldg(row + c) * gu * inv * inv / n;
-    return k * out;
 }
 
 // A thread takes four consecutive elements of the flat y (a 16-byte load / store whatever the row

@@ -760,11 +760,10 @@ struct EulerNode : Node {
                       o_scratch = l.add(weights ? weight_grad_scratch_floats(m, k, o) : 0);
         Tensor temporary = l.make(w1);
         float *t = fmut(temporary), *gy = t + o_gy, *dh = t + o_dh, *gz = t + o_gz;
-        // update
-        check_status(mask.defined() ? npa_step_update_backward_masked(gd, y, fptr(mask), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), gy, st)
-                                    : npa_step_update_backward(gd, y, nullptr, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), gy, st));
-        // MLP
-        if (back || weights) check_status(npa_mlp_hidden_grad(gy, fptr(w2), h, dh, m, kHidden, (int)o, w2.stride(0), w2.stride(1), st));
+        // update, and the MLP's output layer
+        if (back || weights)
+            check_status(npa_step_hidden_grad(gd, y, fptr(mask), mask.defined(), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fptr(w2), h, gy,
+                                              dh, kHidden, w2.stride(0), w2.stride(1), st));
         Tensor gw1, gb1, gw2;
         if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st);
         // perception, with the update's own gradient of the states added

@@ -282,6 +282,11 @@ def test_tcgen05_entry_points_reject_bad_arguments_before_any_launch():
     assert hg(1000, 128, 49) == n.NPA_ERR_UNSUPPORTED
     assert hg(0, 128, 18) == n.NPA_ERR_INVALID_ARGUMENT
     assert hg(1000, 128, 18, dh=odd) == n.NPA_ERR_INVALID_ARGUMENT
+    grid = n.make_grid(3, "clamped", "grid", (8, 8, 8), 0.1, 1, 128, 32)
+    shg = lambda C, y=buf, dh=buf, hidden=128: lib.npa_step_hidden_grad(ctypes.byref(grid), y, null, 0, 0.5, C, 1.0, 1.0, buf, buf, buf, buf, buf, dh, hidden,
+                                                                        128, 1, null)
+    assert shg(46) == shg(16, hidden=64) == n.NPA_ERR_UNSUPPORTED
+    assert shg(0) == shg(16, y=null) == shg(16, dh=odd) == n.NPA_ERR_INVALID_ARGUMENT
     # status and self-test arguments
     assert lib.npa_linear_tcgen05_status(null, 0) == n.NPA_ERR_INVALID_ARGUMENT
     assert lib.npa_linear_tcgen05_wait_selftest(0, buf, null) == n.NPA_ERR_INVALID_ARGUMENT

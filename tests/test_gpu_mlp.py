@@ -130,3 +130,34 @@ def test_a_wait_that_runs_out_ends_the_tcgen05_kernel_roles_cleanly(engine):
     torch.cuda.synchronize()
     assert res.tolist() == [1, 1]
     assert float(torch.ones(4, device="cuda").sum().item()) == 4.0
+
+
+@pytest.mark.parametrize("dim", [2, 3])
+@pytest.mark.parametrize("C,N", [(4, 1), (13, 15), (16, 16), (16, 4097), (32, 17), (32, 40000), (45, 333)])   # sixteen rows per warp, up to 48 columns
+@pytest.mark.parametrize("mask", [None, "weights", "uniforms"])
+def test_hidden_gradient_of_a_step(dim, C, N, mask):
+    """The update's backward and the hidden gradient in one pass: g_y to the bit as by the update's own kernel, dh to the bit as from that
+    g_y, and dh against float64."""
+    import ctypes
+    from npa_b200 import _native as n
+    gen = torch.Generator(device="cuda").manual_seed(C + N)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    P, O = (2 if dim == 2 else 4), dim + C
+    grid = n.make_grid(dim, "clamped", "grid", (8,) * dim, 0.1, 1, N, 32)
+    y, gx, gs, W2, h = randn(N, O), randn(N, P), randn(N, C), randn(O, 128), randn(N, 128).relu()
+    y[0, :dim] = 0                                          # the limiter's corner
+    m = None if mask is None else torch.rand(N, generator=gen, device="cuda") if mask == "uniforms" else (randn(N) > 0).float()
+    st, ref = n.current_stream(), ctypes.byref(grid)
+    for up_x, up_s in ((gx, gs), (None, gs), (gx, None)):
+        gy, gy_one, dh, dh_one = (torch.full(s, float("nan"), device="cuda") for s in ((N, O), (N, O), (N, 128), (N, 128)))
+        if mask == "uniforms":
+            n.check(n.lib.npa_step_update_backward_masked(ref, n.ptr(y), n.ptr(m), 0.5, C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(gy), st))
+        else:
+            n.check(n.lib.npa_step_update_backward(ref, n.ptr(y), n.ptr(m), C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(gy), st))
+        n.check(n.lib.npa_mlp_hidden_grad(n.ptr(gy), n.ptr(W2), n.ptr(h), n.ptr(dh), N, 128, O, 128, 1, st))
+        n.check(n.lib.npa_step_hidden_grad(ref, n.ptr(y), n.ptr(m), mask == "uniforms", 0.5, C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(W2),
+                                           n.ptr(h), n.ptr(gy_one), n.ptr(dh_one), 128, 128, 1, st))
+        assert torch.equal(gy_one, gy) and torch.equal(dh_one, dh)
+        want = (gy.double() @ W2.double()) * (h > 0)
+        bound = 2.0 ** -24 * O * (gy.double().abs() @ W2.double().abs())    # a rounding per product of the chain
+        assert ((dh.double() - want).abs() <= bound).all()
