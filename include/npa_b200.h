@@ -500,8 +500,9 @@ int npa_mlp_hidden_grad(const float *dy, const float *W2, const float *h, float 
 
 /* npa_step_update_backward (mask: 0 / 1 per particle, or with `uniforms` set values that update where they are below
  * update_below; NULL = all) and npa_mlp_hidden_grad of its result in one pass: g_y [B*N, D + C] and dh [B*N, 128] from the
- * upstream gradients of the updated positions and states (either may be NULL = zero).  D + C <= 48. */
-int npa_step_hidden_grad(const npa_grid *g, const float *y, const float *mask, int32_t uniforms, float update_below,
+ * upstream gradients of the updated positions and states (either may be NULL = zero).  Of y only the raw displacements are read, the
+ * first D floats of rows of y_pitch.  D + C <= 48. */
+int npa_step_hidden_grad(const npa_grid *g, const float *y, int32_t y_pitch, const float *mask, int32_t uniforms, float update_below,
                          int32_t channels, float alpha, float dt, const float *g_x_out, const float *g_s_out, const float *W2,
                          const float *h, float *g_y, float *dh, int32_t hidden, int64_t w_stride_out, int64_t w_stride_in,
                          void *stream);
@@ -577,6 +578,15 @@ int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const f
                                  void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, void *stream);
 int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim,
                                      int32_t out_dim, const void *scratch, int64_t scratch_bytes, void *stream);
+
+/* The same with the Euler update of npa_step_update_forward in the kernel's epilogue: instead of y [B*N, D + C] the updated positions
+ * and states leave, and the raw displacements when `displacement` [B*N, 2 or 4] is not NULL (what the backward reads of y).  mask,
+ * uniforms and update_below as in npa_step_hidden_grad; h may be NULL.  Multiples of four up to 32 features; x_bin, s_bin,
+ * displacement, x_out and s_out 16-byte aligned. */
+int npa_mlp_step_forward(const npa_grid *g, const float *z, const float *b1, float *h, int32_t in_dim, const void *scratch,
+                         int64_t scratch_bytes, const float *x_bin, const float *s_bin, const float *mask, int32_t uniforms,
+                         float update_below, int32_t channels, float alpha, float dt, int32_t wrap, float *displacement, float *x_out,
+                         float *s_out, void *stream);
 int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image_bytes, float *C, int64_t rows,
                                 int32_t in_dim, int32_t out_dim, void *stream);
 /* Self-test of those bounded waits: a two-warp kernel in which warp 0 waits `limit_us` (1..1,000,000)

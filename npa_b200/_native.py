@@ -100,7 +100,9 @@ SIGNATURES = {
     "npa_mlp_weight_grad": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int64, _I32, _I32, _I32, _P, ctypes.c_int64,
                                            _P, _P, _P, _P]),
     "npa_mlp_hidden_grad": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int64, _I32, _I32, ctypes.c_int64, ctypes.c_int64, _P]),
-    "npa_step_hidden_grad": (ctypes.c_int, [_P, _P, _P, _I32, ctypes.c_float, _I32, ctypes.c_float, ctypes.c_float] + [_P] * 6
+    "npa_mlp_step_forward": (ctypes.c_int, [_P] * 4 + [_I32, _P, _I64, _P, _P, _P, _I32, ctypes.c_float, _I32, ctypes.c_float, ctypes.c_float, _I32]
+                             + [_P] * 4),
+    "npa_step_hidden_grad": (ctypes.c_int, [_P, _P, _I32, _P, _I32, ctypes.c_float, _I32, ctypes.c_float, ctypes.c_float] + [_P] * 6
                              + [_I32, ctypes.c_int64, ctypes.c_int64, _P]),
     "npa_mlp_weight_grad_tcgen05": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int64, _I32, _I32, _I32, _P, ctypes.c_int64,
                                                    _P, _P, _P, _P]),

@@ -80,7 +80,7 @@ __global__ void __launch_bounds__(kHgThreads, 4) mlp_hidden_grad_kernel(const __
                 for (int q = lane; q < n * (S / 4); q += 32) copy(raw + 4 * q, step.g_s_out + i0 * S + 4 * q, Int<16>());
             if (r < n) {  // four lanes to a row: a component each, the last one the mask
                 if (part < D && step.g_x_out) copy(small + 4 * r + part, step.g_x_out + (i0 + r) * P + part, Int<4>());
-                if (part < D) copy(small + kHgRows * 4 + 4 * r + part, step.y + (i0 + r) * O + part, Int<4>());
+                if (part < D) copy(small + kHgRows * 4 + 4 * r + part, step.y + (i0 + r) * step.y_pitch + part, Int<4>());
                 if (part == 3 && step.mask) copy(small + kHgRows * 8 + r, step.mask + i0 + r, Int<4>());
             }
         }
@@ -235,7 +235,7 @@ int npa_mlp_hidden_grad(const float *dy, const float *W2, const float *h, float 
     return launch_hidden_grad<0, false>(a, StepArgs{}, (cudaStream_t)stream);
 }
 
-int npa_step_hidden_grad(const npa_grid *gd, const float *y, const float *mask, int32_t uniforms, float update_below, int32_t channels, float alpha,
+int npa_step_hidden_grad(const npa_grid *gd, const float *y, int32_t y_pitch, const float *mask, int32_t uniforms, float update_below, int32_t channels, float alpha,
                          float dt, const float *g_x_out, const float *g_s_out, const float *W2, const float *h, float *g_y, float *dh,
                          int32_t hidden, int64_t w_stride_out, int64_t w_stride_in, void *stream) {
     const char *me = "npa_step_hidden_grad";
@@ -246,8 +246,9 @@ int npa_step_hidden_grad(const npa_grid *gd, const float *y, const float *mask, 
     const int out_dim = g.dim + channels;
     if ((rc = check_hidden_grad(me, W2, h, dh, (int64_t)g.B * g.N, hidden, out_dim)) != NPA_OK) return rc;
     if (!y || !g_y) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: y and g_y must be non-NULL", me);
+    if (y_pitch < g.dim) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows of %d floats do not hold a displacement", me, y_pitch);
     StepArgs s = {};
-    s.y = y; s.mask = mask; s.uniforms = uniforms; s.below = update_below; s.g_x_out = g_x_out; s.g_s_out = g_s_out; s.g_y = g_y;
+    s.y = y; s.y_pitch = y_pitch; s.mask = mask; s.uniforms = uniforms; s.below = update_below; s.g_x_out = g_x_out; s.g_s_out = g_s_out; s.g_y = g_y;
     s.particles = (long long)g.B * g.N; s.C = channels; s.alpha = alpha; s.eps = g.h; s.dt = dt;
     const HiddenGradArgs a = {nullptr, W2, h, dh, s.particles, w_stride_out, w_stride_in, out_dim};
     cudaStream_t st = (cudaStream_t)stream;

@@ -23,10 +23,15 @@
 //     turn the blocks through shared memory and store rows with bias, ReLU and the optional gate
 //     applied (float4 when out_dim is a multiple of 4).
 //
+// The forward of a step ends with the Euler update (step_update.cuh): the epilogue has y's tile in shared memory and writes the updated
+// positions and states instead of y, of which the backward only needs the raw displacements.  Measured, B200, us, two kernels -> one:
+// 262,144 particles in 3D, C = 32, 142 + 25.5 -> 159; pass of an inference step of 4,096 in 2D 54.2 -> 52.7, of 2,500 in a graph 37.8 -> 35.8.
+//
 // Every wait on an mbarrier is bounded in time; a wait that gives up raises a flag that ends all
 // roles, the CTA frees its tensor memory and the host reads the reason from a status word.
 #include <mutex>
 
+#include "step_update.cuh"
 #include "umma.cuh"
 #include "weight_image.cuh"
 
@@ -80,7 +85,13 @@ struct UmmaArgs {
     const float *W2img;
     float *Y;
     int N2, N2p;
+    // with the Euler update (D > 0): instead of the rows of the second layer the updated positions and states leave, and
+    // into step.y (NULL: nobody wants them) rows of step.y_pitch floats that begin with the raw displacements
+    int D;
+    StepArgs step;
+    Geom g;
 };
+constexpr int kUmmaStepQuads = 4;  // float4 of the states per epilogue thread and tile: up to 32 features
 
 __device__ unsigned g_umma_status;
 
@@ -89,7 +100,50 @@ __global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
     write_image_element(jobs, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-template <bool FUSE>
+enum : int { kUmmaOneLayer = 0, kUmmaTwoLayers = 1, kUmmaStep = 2 };
+
+// The tile of the second layer as the Euler update: the epilogue's threads move four states at a time, the first 128 of them a position.
+template <int D>
+__device__ __forceinline__ void umma_store_step(const UmmaArgs &a, const float *tile, long long row0, int rows, int e, const float4 (&s_bin)[kUmmaStepQuads],
+                                                const float (&m)[kUmmaStepQuads], float m_x, const float4 &x_bin) {
+    const StepArgs &st = a.step;
+    const int C4 = st.C / 4, W = D + st.C;
+#pragma unroll
+    for (int k = 0; k < kUmmaStepQuads; ++k) {
+        const int q = e + k * kUmmaEpilogueWarps * 32;
+        if (q < rows * C4) {
+            const int row = q / C4;
+            reinterpret_cast<float4 *>(st.s_out)[row0 * C4 + q] = step_forward_states(st, m[k], s_bin[k], tile + row * W + D + 4 * (q - row * C4));
+        }
+    }
+    if (e < rows) {
+        const float *u = tile + e * W;
+        float x[4] = {x_bin.x, x_bin.y, x_bin.z, x_bin.w};
+        step_forward_position<D>(st, a.g, m_x, u, x);
+        if (D == 2) {
+            reinterpret_cast<float2 *>(st.x_out)[row0 + e] = make_float2(x[0], x[1]);
+            if (st.y) reinterpret_cast<float2 *>(const_cast<float *>(st.y))[row0 + e] = make_float2(u[0], u[1]);
+        } else {
+            reinterpret_cast<float4 *>(st.x_out)[row0 + e] = make_float4(x[0], x[1], x[2], x[3]);
+            if (st.y) reinterpret_cast<float4 *>(const_cast<float *>(st.y))[row0 + e] = make_float4(u[0], u[1], u[2], 0.f);
+        }
+    }
+}
+
+// What the update will read of a tile's particles towards L2: the states, positions and mask were last touched before the perception, whose
+// rows of z may have taken their place (the kernel for 262,144 particles in 3D: 159 us with it, 167 without; loading them into registers
+// ahead of the last pass instead 178, spills).
+__device__ __forceinline__ void umma_prefetch_step(const UmmaArgs &a, long long tile, int e) {
+    const long long row0 = tile * kUmmaRows;
+    const int rows = a.M - row0 < kUmmaRows ? (int)(a.M - row0) : kUmmaRows, P = a.D == 2 ? 2 : 4;
+    auto fetch = [](const float *p) { asm volatile("prefetch.global.L2 [%0];" ::"l"(p)); };
+    if (e * 32 < rows * a.step.C) fetch(a.step.s_bin + row0 * a.step.C + e * 32);  // 256 threads: up to 64 features
+    const int f = kUmmaEpilogueWarps * 32 - 1 - e;
+    if (f * 32 < rows * P) fetch(a.step.x_bin + row0 * P + f * 32);
+    else if (f >= 16 && f < 20 && a.step.mask && (f - 16) * 32 < rows) fetch(a.step.mask + row0 + (f - 16) * 32);
+}
+
+template <int MODE>
 __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __grid_constant__ UmmaArgs args) {
     after_previous_kernel();
     // every field is read into a register once: the role loops below must not go back to the parameter block
@@ -102,7 +156,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
     const int K = args.K, N = args.N, Np = args.Np, nchunks = args.nchunks, last_ksteps = args.last_ksteps;
     const int stages = args.stages, stage_bytes = args.stage_bytes;
     const bool relu = args.relu != 0;
-    constexpr bool fuse = FUSE;  // two-layer mode
+    constexpr bool fuse = MODE != kUmmaOneLayer;  // two-layer mode
     const int N2 = args.N2, N2p = args.N2p;
     const int acc_stride = fuse ? 128 : kUmmaAccStride;
     extern __shared__ uint8_t umma_smem_raw[];
@@ -317,6 +371,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
             const int acc = it & 1;
             const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * kUmmaRows + quarter * 32;
             const int nrows = M - row0 < 32 ? (int)(M - row0) : 32;  // may be <= 0 in the last tile
+            if constexpr (MODE == kUmmaStep) umma_prefetch_step(args, (long long)blockIdx.x + (long long)it * gridDim.x, warp * 32 + lane);
 #pragma unroll 1
             for (int pass = fuse ? 0 : 1; pass < (fuse ? 3 : 2); ++pass) {
                 // what this pass reads and where it goes
@@ -438,15 +493,44 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
                     __syncwarp();
                 }
                 if (fuse && pass == 2) {
+                    const int e = warp * 32 + lane;
+                    [[maybe_unused]] float4 s_bin[kUmmaStepQuads], x_bin = make_float4(0.f, 0.f, 0.f, 0.f);
+                    [[maybe_unused]] float m[kUmmaStepQuads], m_x = 1.f;
+                    if constexpr (MODE == kUmmaStep) {  // what the update reads of the tile's particles, while the other warps finish
+                        const long long r0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * kUmmaRows;
+                        const int here = M - r0 < kUmmaRows ? (int)(M - r0) : kUmmaRows, C4 = args.step.C / 4;
+#pragma unroll
+                        for (int k = 0; k < kUmmaStepQuads; ++k) {
+                            const int q = e + k * kUmmaEpilogueWarps * 32;
+                            s_bin[k] = make_float4(0.f, 0.f, 0.f, 0.f);
+                            m[k] = 1.f;
+                            if (q < here * C4) {
+                                s_bin[k] = __ldg(reinterpret_cast<const float4 *>(args.step.s_bin) + r0 * C4 + q);
+                                m[k] = mask_of(args.step, r0 + q / C4);
+                            }
+                        }
+                        if (e < here) {
+                            m_x = mask_of(args.step, r0 + e);
+                            if (args.D == 2) {
+                                const float2 v = __ldg(reinterpret_cast<const float2 *>(args.step.x_bin) + r0 + e);
+                                x_bin.x = v.x; x_bin.y = v.y;
+                            } else {
+                                x_bin = __ldg(reinterpret_cast<const float4 *>(args.step.x_bin) + r0 + e);
+                            }
+                        }
+                    }
                     __syncwarp();
                     if (lane == 0) mbar_arrive(&sh->y_written);
                     if (!(ok = umma_wait(&sh->y_written, it & 1, &sh->abort))) break;
                     // all eight warps copy the tile: (rows that exist) x N2 floats, contiguous and 16-byte aligned in global memory
                     const long long tile_row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * kUmmaRows;
                     const int rows_here = M - tile_row0 < kUmmaRows ? (int)(M - tile_row0) : kUmmaRows;
-                    const int total = rows_here * ncol, e = warp * 32 + lane;
+                    const int total = rows_here * ncol;
                     float *dst = out + tile_row0 * ncol;
-                    if (((uintptr_t)out & 15) == 0) {
+                    if constexpr (MODE == kUmmaStep) {
+                        if (args.D == 2) umma_store_step<2>(args, ytile, tile_row0, rows_here, e, s_bin, m, m_x, x_bin);
+                        else umma_store_step<3>(args, ytile, tile_row0, rows_here, e, s_bin, m, m_x, x_bin);
+                    } else if (((uintptr_t)out & 15) == 0) {
                         for (int q = e; q < total / 4; q += kUmmaEpilogueWarps * 32) ((float4 *)dst)[q] = ((const float4 *)ytile)[q];
                         for (int q = (total & ~3) + e; q < total; q += kUmmaEpilogueWarps * 32) dst[q] = ytile[q];
                     } else {
@@ -497,12 +581,12 @@ __global__ void umma_wait_selftest_kernel(unsigned long long limit_ns, int *resu
 // Per-device set-up done once: the address of the status word and the shared-memory limit of the kernel.
 struct UmmaDevice {
     unsigned *status = nullptr;
-    int smem_limit[2] = {0, 0};  // per kernel instantiation
+    int smem_limit[3] = {0, 0, 0};  // per kernel instantiation
 };
 static std::mutex g_umma_mutex;
 static UmmaDevice g_umma_device[64];
 
-static int umma_device_setup(int smem, bool fuse, unsigned **status) {
+static int umma_device_setup(int smem, int mode, unsigned **status) {
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return fail(NPA_ERR_CUDA, "npa_linear_tcgen05: cudaGetDevice: %s", cudaGetErrorString(e));
@@ -512,11 +596,11 @@ static int umma_device_setup(int smem, bool fuse, unsigned **status) {
         e = cudaGetSymbolAddress((void **)&d.status, g_umma_status);
         if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "npa_linear_tcgen05: status word: %s", cudaGetErrorString(e));
     }
-    if (smem > d.smem_limit[fuse]) {
-        e = fuse ? cudaFuncSetAttribute(linear_umma_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem)
-                 : cudaFuncSetAttribute(linear_umma_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (smem > d.smem_limit[mode]) {
+        const auto kernel = mode == kUmmaStep ? linear_umma_kernel<kUmmaStep> : mode == kUmmaTwoLayers ? linear_umma_kernel<kUmmaTwoLayers> : linear_umma_kernel<kUmmaOneLayer>;
+        e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "npa_linear_tcgen05: raising the shared-memory limit: %s", cudaGetErrorString(e));
-        d.smem_limit[fuse] = smem;
+        d.smem_limit[mode] = smem;
     }
     *status = d.status;
     return NPA_OK;
@@ -598,7 +682,7 @@ static int linear_tcgen05(const float *A, const float *W, const float *bias, con
     if (a.stages > kUmmaMaxStages) a.stages = kUmmaMaxStages;
     if (a.stages < 2) return fail(NPA_ERR_UNSUPPORTED, "npa_linear_tcgen05: out_dim %d leaves room for fewer than two stages", out_dim);
     const size_t smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
-    int rc = umma_device_setup((int)smem, false, &a.status);
+    int rc = umma_device_setup((int)smem, kUmmaOneLayer, &a.status);
     if (rc != NPA_OK) return rc;
     if (W) {
         ImageJobs jobs = {{image_job(W, w_stride_out, w_stride_in, in_dim, out_dim, scratch)}, 1};
@@ -606,7 +690,7 @@ static int linear_tcgen05(const float *A, const float *W, const float *bias, con
     }
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
-    launch_early(linear_umma_kernel<false>, ctas, kUmmaThreads, smem, (cudaStream_t)stream, a);
+    launch_early(linear_umma_kernel<kUmmaOneLayer>, ctas, kUmmaThreads, smem, (cudaStream_t)stream, a);
     return check_launch("linear_umma_kernel");
 }
 
@@ -655,13 +739,13 @@ int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const f
     return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream);
 }
 
-int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim, int32_t out_dim,
-                                     const void *scratch, int64_t scratch_bytes, void *stream) {
-    const char *me = "npa_mlp_forward_tcgen05";
+// step != NULL: with the Euler update of D-dimensional positions on the geometry g.
+static int mlp_forward(const char *me, const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim, int32_t out_dim,
+                       const void *scratch, int64_t scratch_bytes, const StepArgs *step, const Geom *g, cudaStream_t st) {
     if (rows <= 0 || in_dim <= 0 || out_dim <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
     if (in_dim > 1024 || out_dim > 64)
         return fail(NPA_ERR_UNSUPPORTED, "%s: supports in_dim <= 1024 and out_dim <= 64 (hidden width 128), got %d and %d", me, in_dim, out_dim);
-    if (!z || !y || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
+    if (!z || (!y && !step) || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, W1, W2, y and scratch must be non-NULL", me);
     if ((uintptr_t)z % 4 || (uintptr_t)h % 4 || (uintptr_t)y % 4 || (uintptr_t)scratch % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, h and y must be float aligned, scratch 16-byte aligned", me);
     if (scratch_bytes < npa_mlp_forward_tcgen05_scratch_bytes(in_dim, out_dim))
@@ -682,13 +766,43 @@ int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, 
     if (a.stages > kUmmaMaxStages) a.stages = kUmmaMaxStages;
     if (a.stages < 2) return fail(NPA_ERR_UNSUPPORTED, "%s: no room for two stages", me);
     const size_t smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
-    const int rc = umma_device_setup((int)smem, true, &a.status);
+    const int mode = step ? kUmmaStep : kUmmaTwoLayers;
+    if (step) {
+        a.D = g->dim;
+        a.step = *step;
+        a.g = *g;
+    }
+    const int rc = umma_device_setup((int)smem, mode, &a.status);
     if (rc != NPA_OK) return rc;
-    cudaStream_t st = (cudaStream_t)stream;
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
-    launch_early(linear_umma_kernel<true>, ctas, kUmmaThreads, smem, st, a);
+    launch_early(step ? linear_umma_kernel<kUmmaStep> : linear_umma_kernel<kUmmaTwoLayers>, ctas, kUmmaThreads, smem, st, a);
     return check_launch("linear_umma_kernel (two layers)");
+}
+
+int npa_mlp_forward_tcgen05_prepared(const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim, int32_t out_dim,
+                                     const void *scratch, int64_t scratch_bytes, void *stream) {
+    return mlp_forward("npa_mlp_forward_tcgen05", z, b1, h, y, rows, in_dim, out_dim, scratch, scratch_bytes, nullptr, nullptr, (cudaStream_t)stream);
+}
+
+int npa_mlp_step_forward(const npa_grid *gd, const float *z, const float *b1, float *h, int32_t in_dim, const void *scratch, int64_t scratch_bytes,
+                         const float *x_bin, const float *s_bin, const float *mask, int32_t uniforms, float update_below, int32_t channels,
+                         float alpha, float dt, int32_t wrap, float *displacement, float *x_out, float *s_out, void *stream) {
+    const char *me = "npa_mlp_step_forward";
+    Geom g;
+    const int rc = make_geom(gd, &g);
+    if (rc != NPA_OK) return rc;
+    if (channels <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: channels must be positive, got %d", me, channels);
+    if (channels % 4 != 0 || channels > 4 * 2 * kUmmaStepQuads)
+        return fail(NPA_ERR_UNSUPPORTED, "%s: supports multiples of four up to %d features, got %d", me, 4 * 2 * kUmmaStepQuads, channels);
+    if (!x_bin || !s_bin || !x_out || !s_out) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: x_bin, s_bin, x_out and s_out must be non-NULL", me);
+    if (((uintptr_t)x_bin | (uintptr_t)s_bin | (uintptr_t)x_out | (uintptr_t)s_out | (uintptr_t)displacement) % 16)
+        return fail(NPA_ERR_INVALID_ARGUMENT, "%s: x_bin, s_bin, displacement, x_out and s_out must be 16-byte aligned", me);
+    StepArgs s = {};
+    s.y = displacement; s.y_pitch = g.dim == 2 ? 2 : 4; s.x_bin = x_bin; s.s_bin = s_bin; s.mask = mask; s.uniforms = uniforms;
+    s.below = update_below; s.x_out = x_out; s.s_out = s_out; s.particles = (long long)g.B * g.N; s.C = channels; s.alpha = alpha; s.eps = g.h;
+    s.dt = dt; s.wrap = wrap;
+    return mlp_forward(me, z, b1, h, nullptr, s.particles, in_dim, g.dim + channels, scratch, scratch_bytes, &s, &g, (cudaStream_t)stream);
 }
 
 int npa_mlp_forward_tcgen05(const float *z, const float *W1, const float *b1, const float *W2, float *h, float *y, int64_t rows,

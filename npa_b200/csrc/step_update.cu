@@ -12,14 +12,6 @@
 
 namespace npa {
 
-// remainder(x + L/2, L) - L/2 with torch's sign convention (result of remainder in [0, L)).
-__device__ inline float wrap_axis(float x, float L) {
-    const float half = 0.5f * L;
-    float r = fmodf(x + half, L);
-    if (r < 0.f) r += L;
-    return r - half;
-}
-
 // One element of y: column c of particle i.
 template <int D>
 __device__ inline void step_forward_element(const StepArgs &a, const Geom &g, long long i, int c, float v) {
@@ -132,18 +124,12 @@ __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom
                 const float m = mask_of(a, i);
                 const float4 sv = __ldg(reinterpret_cast<const float4 *>(a.s_bin) + i * C4 + c4);
                 const float *yr = tile + row * W + D + 4 * c4;
-                reinterpret_cast<float4 *>(a.s_out)[i * C4 + c4] =
-                    make_float4(sv.x + (a.dt * yr[0]) * m, sv.y + (a.dt * yr[1]) * m, sv.z + (a.dt * yr[2]) * m,
-                                sv.w + (a.dt * yr[3]) * m);
+                reinterpret_cast<float4 *>(a.s_out)[i * C4 + c4] = step_forward_states(a, m, sv, yr);
             }
             for (int row = threadIdx.x; row < rows; row += blockDim.x) {
                 const long long i = r0 + row;
                 const float m = mask_of(a, i);
                 const float *yr = tile + row * W;
-                float n2 = 0.f;
-#pragma unroll
-                for (int d = 0; d < D; ++d) n2 = fmaf(yr[d], yr[d], n2);
-                const float den = 1.0f + sqrtf(n2);
                 float xi[4] = {0.f, 0.f, 0.f, 0.f};
                 if (D == 2) {
                     const float2 v = __ldg(reinterpret_cast<const float2 *>(a.x_bin) + i);
@@ -152,12 +138,7 @@ __global__ void __launch_bounds__(256) step_update_tiled_kernel(StepArgs a, Geom
                     const float4 v = __ldg(reinterpret_cast<const float4 *>(a.x_bin) + i);
                     xi[0] = v.x; xi[1] = v.y; xi[2] = v.z; xi[3] = v.w;
                 }
-#pragma unroll
-                for (int d = 0; d < D; ++d) {
-                    const float lim = ((a.alpha * yr[d]) * a.eps) / den;
-                    xi[d] = xi[d] + (a.dt * lim) * m;
-                    if (a.wrap && g.periodic) xi[d] = wrap_axis(xi[d], g.L[d]);
-                }
+                step_forward_position<D>(a, g, m, yr, xi);
                 if (D == 2) reinterpret_cast<float2 *>(a.x_out)[i] = make_float2(xi[0], xi[1]);
                 else reinterpret_cast<float4 *>(a.x_out)[i] = make_float4(xi[0], xi[1], xi[2], xi[3]);
             }

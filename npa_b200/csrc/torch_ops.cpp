@@ -730,7 +730,7 @@ struct EulerNode : Node {
     SavedVariable w1_, w2_, slab_, mask_;
     Tensor offs, perm, info;
     int64_t o_x, o_s, o_rho, o_dg, o_v, o_packed, o_z, o_h, o_y, o_dz, o_pairs;  // places in the slab, in floats
-    int64_t C, columns, dz_bytes, slab_floats;
+    int64_t C, columns, dz_bytes, slab_floats, y_pitch;  // y: rows that begin with the raw displacements
     float coef, dg_scale, alpha, dt, below;
     bool ln_grad, ln_dg, stop_pos, stop_state;
 
@@ -762,7 +762,7 @@ struct EulerNode : Node {
         float *t = fmut(temporary), *gy = t + o_gy, *dh = t + o_dh, *gz = t + o_gz;
         // update, and the MLP's output layer
         if (back || weights)
-            check_status(npa_step_hidden_grad(gd, y, fptr(mask), mask.defined(), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fptr(w2), h, gy,
+            check_status(npa_step_hidden_grad(gd, y, (int)y_pitch, fptr(mask), mask.defined(), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fptr(w2), h, gy,
                                               dh, kHidden, w2.stride(0), w2.stride(1), st));
         Tensor gw1, gb1, gw2;
         if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st);
@@ -825,9 +825,10 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     Tensor perm = ints(x, {g.B, g.N}), offs = ints(x, {g.B * g.cells + 1}), info = ints(x, {g.max_blocks, 4});
     grid->bin(x, perm, offs, info, st);
     const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), dz_bytes = back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
+    const bool in_mlp = C % 4 == 0 && C <= 32;  // the update in the MLP's epilogue, which of y keeps only what the backward reads
     Slab l;
     const int64_t o_x = l.add(m * g.P), o_s = l.add(m * C), o_rho = l.add(m), o_dg = l.add(m * D), o_z = l.add(m * k), o_v = l.add(back ? m * C * D : 0),
-                  o_packed = l.add(m * 4), o_y = l.add(m * o), o_h = l.add(record ? m * kHidden : 0), o_image = l.add(bytes / 4),
+                  o_packed = l.add(m * 4), o_y = l.add(!in_mlp ? m * o : record ? m * g.P : 0), o_h = l.add(record ? m * kHidden : 0), o_image = l.add(bytes / 4),
                   o_dz = l.add(dz_bytes / 4), o_pairs = l.add(m * columns);
     Tensor slab = l.make(x);
     float *t = fmut(slab), *x_bin = t + o_x, *s_bin = t + o_s, *rho = t + o_rho, *rho_grad = t + o_dg, *z = t + o_z, *packed = t + o_packed,
@@ -837,17 +838,22 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
                                               w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
     check_status(npa_perceive_features_forward_lists(&g.g, (int)C, x_bin, nullptr, s_bin, (float)coef, (float)dg_scale, (float)inv_tol, ln_grad, ln_dg,
                                                      rho, rho_grad, z, vgrad, packed, iptr(offs), iptr(info), pairs, (int)columns, st));
-    check_status(npa_mlp_forward_tcgen05_prepared(z, fptr(b1), h, y, m, (int)k, (int)o, t + o_image, bytes, st));
     Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();
     Tensor xo = blank(x), so = blank(s);
-    check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, y, x_bin, s_bin, fptr(mask), (float)update_prob, (int)C, (float)alpha, (float)dt,
-                                                                 wrap, fmut(xo), fmut(so), st)
-                                : npa_step_update_forward(&g.g, y, x_bin, s_bin, nullptr, (int)C, (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st));
+    if (in_mlp) {
+        check_status(npa_mlp_step_forward(&g.g, z, fptr(b1), h, (int)k, t + o_image, bytes, x_bin, s_bin, fptr(mask), mask.defined(), (float)update_prob,
+                                          (int)C, (float)alpha, (float)dt, wrap, record ? y : nullptr, fmut(xo), fmut(so), st));
+    } else {
+        check_status(npa_mlp_forward_tcgen05_prepared(z, fptr(b1), h, y, m, (int)k, (int)o, t + o_image, bytes, st));
+        check_status(mask.defined() ? npa_step_update_forward_masked(&g.g, y, x_bin, s_bin, fptr(mask), (float)update_prob, (int)C, (float)alpha, (float)dt,
+                                                                     wrap, fmut(xo), fmut(so), st)
+                                    : npa_step_update_forward(&g.g, y, x_bin, s_bin, nullptr, (int)C, (float)alpha, (float)dt, wrap, fmut(xo), fmut(so), st));
+    }
     if (record) {
         auto n = node_for<EulerNode>(x, s, w1, b1, w2);
         n->grid = grid; n->offs = offs; n->perm = perm; n->info = info; n->slab_ = saved(slab); n->mask_ = saved(mask);
         n->o_x = o_x; n->o_s = o_s; n->o_rho = o_rho; n->o_dg = o_dg; n->o_v = o_v; n->o_packed = o_packed; n->o_z = o_z; n->o_h = o_h; n->o_y = o_y;
-        n->o_dz = o_dz; n->o_pairs = o_pairs; n->slab_floats = l.floats; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
+        n->o_dz = o_dz; n->o_pairs = o_pairs; n->slab_floats = l.floats; n->y_pitch = in_mlp ? g.P : o; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
         n->w1_ = saved(w1); n->w2_ = saved(w2);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
         n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;

@@ -283,10 +283,15 @@ def test_tcgen05_entry_points_reject_bad_arguments_before_any_launch():
     assert hg(0, 128, 18) == n.NPA_ERR_INVALID_ARGUMENT
     assert hg(1000, 128, 18, dh=odd) == n.NPA_ERR_INVALID_ARGUMENT
     grid = n.make_grid(3, "clamped", "grid", (8, 8, 8), 0.1, 1, 128, 32)
-    shg = lambda C, y=buf, dh=buf, hidden=128: lib.npa_step_hidden_grad(ctypes.byref(grid), y, null, 0, 0.5, C, 1.0, 1.0, buf, buf, buf, buf, buf, dh, hidden,
+    shg = lambda C, y=buf, dh=buf, hidden=128: lib.npa_step_hidden_grad(ctypes.byref(grid), y, 3 + C, null, 0, 0.5, C, 1.0, 1.0, buf, buf, buf, buf, buf, dh, hidden,
                                                                         128, 1, null)
     assert shg(46) == shg(16, hidden=64) == n.NPA_ERR_UNSUPPORTED
     assert shg(0) == shg(16, y=null) == shg(16, dh=odd) == n.NPA_ERR_INVALID_ARGUMENT
+    # the forward with the update
+    fs = lambda C, x=buf, u=buf, floats=big: lib.npa_mlp_step_forward(ctypes.byref(grid), buf, buf, buf, 3 + 5 * max(C, 1), buf, floats, x, buf, null, 0, 0.5,
+                                                                      C, 1.0, 1.0, 0, u, buf, buf, null)
+    assert fs(13) == fs(36) == n.NPA_ERR_UNSUPPORTED and "features" in n.last_error()
+    assert fs(0) == fs(16, x=null) == fs(16, x=odd) == fs(16, u=odd) == fs(16, floats=10) == n.NPA_ERR_INVALID_ARGUMENT
     # status and self-test arguments
     assert lib.npa_linear_tcgen05_status(null, 0) == n.NPA_ERR_INVALID_ARGUMENT
     assert lib.npa_linear_tcgen05_wait_selftest(0, buf, null) == n.NPA_ERR_INVALID_ARGUMENT

@@ -155,9 +155,39 @@ def test_hidden_gradient_of_a_step(dim, C, N, mask):
         else:
             n.check(n.lib.npa_step_update_backward(ref, n.ptr(y), n.ptr(m), C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(gy), st))
         n.check(n.lib.npa_mlp_hidden_grad(n.ptr(gy), n.ptr(W2), n.ptr(h), n.ptr(dh), N, 128, O, 128, 1, st))
-        n.check(n.lib.npa_step_hidden_grad(ref, n.ptr(y), n.ptr(m), mask == "uniforms", 0.5, C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(W2),
+        n.check(n.lib.npa_step_hidden_grad(ref, n.ptr(y), O, n.ptr(m), mask == "uniforms", 0.5, C, 0.7, 0.9, n.ptr(up_x), n.ptr(up_s), n.ptr(W2),
                                            n.ptr(h), n.ptr(gy_one), n.ptr(dh_one), 128, 128, 1, st))
         assert torch.equal(gy_one, gy) and torch.equal(dh_one, dh)
         want = (gy.double() @ W2.double()) * (h > 0)
         bound = 2.0 ** -24 * O * (gy.double().abs() @ W2.double().abs())    # a rounding per product of the chain
         assert ((dh.double() - want).abs() <= bound).all()
+
+
+@pytest.mark.parametrize("dim,C,N", [(2, 4, 1), (2, 16, 127), (3, 12, 129), (3, 32, 128), (3, 32, 20001), (2, 28, 40000)])  # tiles of 128 rows, 148 at a time
+@pytest.mark.parametrize("mask", [None, "weights", "uniforms"])
+def test_forward_with_the_update(dim, C, N, mask):
+    """The update in the MLP's epilogue: positions, states, hidden layer and raw displacements to the bit as by the two kernels."""
+    import ctypes
+    from npa_b200 import _native as n
+    gen = torch.Generator(device="cuda").manual_seed(C + N)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    P, O, K = (2 if dim == 2 else 4), dim + C, 2 * C + C * dim + dim
+    z, W1, b1, W2, x, s = randn(N, K), randn(128, K) / K ** 0.5, randn(128), randn(O, 128) / 11, randn(N, P) * 0.3, randn(N, C)
+    m = None if mask is None else torch.rand(N, generator=gen, device="cuda") if mask == "uniforms" else (randn(N) > 0).float()
+    nan = lambda *s: torch.full(s, float("nan"), device="cuda")
+    h, y, xo, so, h1, u1, x1, s1 = nan(N, 128), nan(N, O), nan(N, P), nan(N, C), nan(N, 128), nan(N, P), nan(N, P), nan(N, C)
+    st, nbytes = n.current_stream(), n.lib.npa_mlp_forward_tcgen05_scratch_bytes(K, O)
+    image = torch.empty(nbytes // 4, device="cuda")
+    n.check(n.lib.npa_mlp_forward_tcgen05(n.ptr(z), n.ptr(W1), n.ptr(b1), n.ptr(W2), n.ptr(h), n.ptr(y), N, K, O, K, 1, 128, 1, n.ptr(image), nbytes, st))
+    for boundary, wrap in (("clamped", 0), ("periodic", 1)):
+        grid = ctypes.byref(n.make_grid(dim, boundary, "grid", (8,) * dim, 0.1, 1, N, 32))
+        if mask == "uniforms":
+            n.check(n.lib.npa_step_update_forward_masked(grid, n.ptr(y), n.ptr(x), n.ptr(s), n.ptr(m), 0.5, C, 0.7, 0.9, wrap, n.ptr(xo), n.ptr(so), st))
+        else:
+            n.check(n.lib.npa_step_update_forward(grid, n.ptr(y), n.ptr(x), n.ptr(s), n.ptr(m), C, 0.7, 0.9, wrap, n.ptr(xo), n.ptr(so), st))
+        for hidden, u in ((h1, u1), (None, None)):
+            x1.fill_(float("nan"))
+            n.check(n.lib.npa_mlp_step_forward(grid, n.ptr(z), n.ptr(b1), n.ptr(hidden), K, n.ptr(image), nbytes, n.ptr(x), n.ptr(s), n.ptr(m),
+                                               mask == "uniforms", 0.5, C, 0.7, 0.9, wrap, n.ptr(u), n.ptr(x1), n.ptr(s1), st))
+            assert torch.equal(x1, xo) and torch.equal(s1, so)
+        assert torch.equal(h1, h) and torch.equal(u1[:, :dim], y[:, :dim])
