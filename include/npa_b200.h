@@ -415,6 +415,16 @@ int npa_perceive_features_backward_lists(const npa_grid *g, int32_t channels, co
                                          void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
                                          const int32_t *pair_cache, int32_t pair_stride, void *stream);
 
+/* The same for positions that are those that were binned, bit for bit, as a step has them between its reorder and its update:
+ * with grad_x = NULL it may then find the neighbours among the cells instead of reading the lists. */
+int npa_perceive_features_backward_binned(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
+                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                         const float *packed, const float *dL_dz, float coef, float dg_scale,
+                                         int32_t log_norm_grad, int32_t log_norm_dg, const float *grad_s_add,
+                                         float *grad_x, float *grad_s,
+                                         void *scratch, int64_t scratch_bytes, const int32_t *bin_offsets,
+                                         const int32_t *pair_cache, int32_t pair_stride, void *stream);
+
 /* ---- the Euler update after perception and the per-particle MLP ----------------- *
  * Replaces the elementwise torch code of NPA.forward (models/npa.py:145-153, the
  * displacement limiter) and of step_euler (models/npa.py:183-203) and, with

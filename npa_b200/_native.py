@@ -85,6 +85,8 @@ SIGNATURES = {
                                                            _I32, _I32] + [_P] * 8 + [_I32, _P]),
     "npa_perceive_features_backward_lists": (ctypes.c_int, [_P, _I32] + [_P] * 8 + [ctypes.c_float, ctypes.c_float, _I32, _I32]
                                              + [_P] * 4 + [_I64, _P, _P, _I32, _P]),
+    "npa_perceive_features_backward_binned": (ctypes.c_int, [_P, _I32] + [_P] * 8 + [ctypes.c_float, ctypes.c_float, _I32, _I32]
+                                             + [_P] * 4 + [_I64, _P, _P, _I32, _P]),
     "npa_perception_forward": (ctypes.c_int, [_P, _I32] + [_P] * 11 + [_P, _I32, _P]),
     "npa_perception_backward": (ctypes.c_int, [_P, _I32] + [_P] * 13 + [_P, _I32, _P]),
     "npa_step_update_forward": (ctypes.c_int, [_P] * 5 + [_I32, ctypes.c_float, ctypes.c_float, _I32, _P, _P, _P]),

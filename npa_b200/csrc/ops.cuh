@@ -105,6 +105,7 @@ struct FeatureListBwdArgs {
     const float *direct;      // rows of direct_pitch floats added to grad_s, or NULL
     int direct_pitch;
     const float *add;         // [B,N,C] added to grad_s, or NULL
+    int out_vec;              // feature_dense.cu: grad_s and add can be moved in vectors
     const float *g_dg;        // upstream of the density gradient [B,N,D] (its part of grad_x is added), or NULL
     const float *g_rho;       // upstream of the density [B,N], or NULL: only goes into pg
     float *grad_x, *grad_s, *grad_rho;
@@ -130,6 +131,10 @@ int launch_scalar_list_backward(const Geom &g, const ScalarListArgs &a, cudaStre
 int launch_density_gradient_list(const Geom &g, const ScalarListArgs &a, cudaStream_t st);
 int launch_feature_list_forward(const Geom &g, int mask, const FeatureFwdArgs &a, cudaStream_t st);
 int launch_feature_list_backward(const Geom &g, int mask, bool full, const FeatureListBwdArgs &a, cudaStream_t st);
+// Features only, blur and gradient, for positions that are those that were binned (feature_dense.cu); what it covers and is faster at.
+bool feature_dense_covers(const Geom &g, int C);
+int feature_dense_pitch(int dim, int cp);  // floats from particle to particle of the rows (gb and gg in one)
+int launch_feature_dense_backward(const Geom &g, const FeatureListBwdArgs &a, cudaStream_t st);
 // [N, C(, D)] upstreams -> rows [N, (1 +) D, cp] of `rows` (blur part only when with_blur).
 int launch_upstream_rows(const Geom &g, int C, const float *g_blur, const float *g_grad, bool with_blur, float *rows, cudaStream_t st);
 

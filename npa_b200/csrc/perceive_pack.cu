@@ -35,13 +35,13 @@ __device__ inline void log_normalize_backward(const float *w, const float *gin, 
 
 // One thread per (particle, feature): dL/dz -> dL/dblur, dL/dgrad; the thread of feature 0 also
 // handles the density-gradient part.  ROWS: the rows the backward over neighbour lists reads, blur and the D
-// axes of the gradient as cp floats each (g_blur = the rows, g_grad unused, columns C..cp-1 zero); otherwise the
+// axes of the gradient as cp floats each, `pitch` floats per particle (g_blur = the rows, g_grad unused, columns C..cp-1 zero); otherwise the
 // operators' own layouts.
 template <int D, bool ROWS>
 __global__ void __launch_bounds__(256)
 pack_backward_kernel(const float *__restrict__ gz, const float *__restrict__ vgrad, const float *__restrict__ rho_grad,
                      float *__restrict__ g_blur, float *__restrict__ g_grad, float *__restrict__ g_rho_grad,
-                     long long particles, int C, float coef, float dg_scale, int log_norm_grad, int log_norm_dg) {
+                     long long particles, int C, int pitch, float coef, float dg_scale, int log_norm_grad, int log_norm_dg) {
     after_previous_kernel();
     const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
     const int cp = ROWS ? (C + 3) & ~3 : C;
@@ -50,7 +50,7 @@ pack_backward_kernel(const float *__restrict__ gz, const float *__restrict__ vgr
     const int f = (int)(t - i * cp);
     const int Z = 2 * C + C * D + D;
     const float *gr = gz + i * Z;
-    float *row = ROWS ? g_blur + i * ((1 + D) * cp) + f : nullptr;
+    float *row = ROWS ? g_blur + i * pitch + f : nullptr;
     if (ROWS && f >= C) {
 #pragma unroll
         for (int d = 0; d <= D; ++d) row[d * cp] = 0.f;
@@ -200,14 +200,16 @@ int64_t npa_lists_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
     if (channels < 0) return fail(NPA_ERR_INVALID_ARGUMENT, "lists_backward_scratch_bytes: channels must not be negative");
     // upstream rows, the density gradient's upstream (rounded up to whole 16-byte records), position + upstream records
     const int64_t n = (int64_t)g.B * g.N, cp = (channels + 3) & ~3;
-    return n * (1 + g.dim) * cp * 4 + n * 16 + n * 16;
+    const int64_t lists = (1 + g.dim) * cp * 4 + 32, dense = feature_dense_pitch(g.dim, (int)cp) * 4;
+    return n * (lists > dense ? lists : dense);
 }
 
-int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
-                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
-                                         const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
-                                         int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
-                                         int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+static int features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                   const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                   const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
+                                   int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
+                                   int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, bool binned,
+                                   void *stream) {
     const char *me = "perceive_features_backward_lists";
     Geom g;
     int rc = make_geom(gd, &g);
@@ -224,15 +226,17 @@ int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, c
     if (!grad_x && !grad_s) return NPA_OK;
     cudaStream_t st = (cudaStream_t)stream;
     const long long n = (long long)g.B * g.N;
-    const int cp = (channels + 3) & ~3, pitch = (1 + g.dim) * cp;
+    const int cp = (channels + 3) & ~3;
+    const bool dense = binned && packed && !grad_x && feature_dense_covers(g, channels);
+    const int pitch = dense ? feature_dense_pitch(g.dim, cp) : (1 + g.dim) * cp;
     float *rows = static_cast<float *>(scratch), *g_dg = rows + n * pitch;
     float4 *pg = reinterpret_cast<float4 *>(g_dg + n * 4);
     const unsigned blocks = (unsigned)((n * cp + 255) / 256);
     if (g.dim == 2)
-        launch_early(pack_backward_kernel<2, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+        launch_early(pack_backward_kernel<2, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, pitch, coef,
                                                               dg_scale, log_norm_grad, log_norm_dg);
     else
-        launch_early(pack_backward_kernel<3, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, coef,
+        launch_early(pack_backward_kernel<3, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, pitch, coef,
                                                               dg_scale, log_norm_grad, log_norm_dg);
     if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
     FeatureListBwdArgs a = {};
@@ -243,11 +247,32 @@ int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, c
     a.g_dg = grad_x ? g_dg : nullptr;
     a.grad_x = grad_x; a.grad_s = grad_s; a.pg = grad_x ? pg : nullptr; a.C = channels;
     a.bin_offsets = bin_offsets; a.pair_cache = pair_cache; a.pair_stride = pair_stride;
+    if (dense) return launch_feature_dense_backward(g, a, st);
     if ((rc = launch_feature_list_backward(g, F_BLUR | F_GRAD, grad_x != nullptr, a, st)) != NPA_OK || !grad_x) return rc;
     ScalarListArgs d = {};
     d.x = x_bin; d.mass = mass; d.pg = pg; d.grad_x = grad_x; d.accumulate_x = 1;
     d.bin_offsets = bin_offsets; d.pair_cache = pair_cache; d.pair_stride = pair_stride;
     return launch_scalar_list_backward(g, d, st);
+}
+
+int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                         const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
+                                         int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
+                                         int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "perceive_features_backward_lists";
+    return features_backward_lists(gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
+                                   scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, false, stream);
+}
+
+int npa_perceive_features_backward_binned(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+                                         const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
+                                         const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
+                                         int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
+                                         int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "perceive_features_backward_lists";
+    return features_backward_lists(gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
+                                   scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, true, stream);
 }
 
 int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
@@ -273,10 +298,10 @@ int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const f
     float *grg = grad_x ? g_rho_grad_scratch : nullptr;
     if (g.dim == 2)
         launch_early(pack_backward_kernel<2, false>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
-                                                        particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
+                                                        particles, channels, 0, coef, dg_scale, log_norm_grad, log_norm_dg);
     else
         launch_early(pack_backward_kernel<3, false>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, g_blur_scratch, g_grad_scratch, grg,
-                                                        particles, channels, coef, dg_scale, log_norm_grad, log_norm_dg);
+                                                        particles, channels, 0, coef, dg_scale, log_norm_grad, log_norm_dg);
     if ((rc = check_launch("pack_backward_kernel")) != NPA_OK) return rc;
     rc = npa_perception_backward(gd, channels, x_bin, mass, s_bin, rho, nullptr, g_blur_scratch, g_grad_scratch, grg,
                                  grad_x, grad_s, grad_rho_scratch, bin_offsets, block_info, pair_cache, pair_stride, stream);

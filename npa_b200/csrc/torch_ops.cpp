@@ -783,7 +783,7 @@ struct EulerNode : Node {
                 none = gsf;
                 gsp = back_s ? fmut(gsf) : nullptr;
             } else {
-                check_status(npa_perceive_features_backward_lists(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, packed, gz, coef, dg_scale,
+                check_status(npa_perceive_features_backward_binned(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, packed, gz, coef, dg_scale,
                                                                   ln_grad, ln_dg, fptr(gs_new), fmut(gxp), gsp, t + o_work, work_bytes, iptr(offs),
                                                                   pairs, (int)columns, st));
             }

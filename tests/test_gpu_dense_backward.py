@@ -1,0 +1,113 @@
+"""Feature gradients of a step as dense products on the tensor cores (positions as binned), against float64 and the sums over lists."""
+import ctypes
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+class Call:
+    """The backward of the packed perception for given rows of dL/dz, by lists or as a step calls it."""
+
+    def __init__(self, x, cells, eps, boundary, C):
+        from npa_b200 import _native as n, sphops as sph
+        from npa_b200.sphops import sph as impl
+        self.n, self.C, self.eps, self.boundary = n, C, eps, boundary
+        self.B, self.N = x.shape[:2]
+        self.dim = 2 if x.shape[2] == 2 else 3
+        grid = sph.HashGrid(dim=self.dim, boundary=boundary, mode="grid", grid_size=(cells,) * self.dim, eps=eps, num_particles=self.N,
+                            batch_size=self.B, max_particles_per_block=32)
+        self.gd = n.make_grid(self.dim, boundary, "grid", (cells,) * self.dim, eps, self.B, self.N, 32)
+        self.box = cells * eps
+        s = torch.randn(self.B, self.N, C, device="cuda")
+        self.snap = grid.instantiate(x)
+        self.x, self.s = sph.bin_particles(x, s, self.snap)
+        Z, self.K = 2 * C + C * self.dim + self.dim, impl._columns(grid.hashgrid)
+        e = lambda *shape, **kw: torch.empty(self.B, self.N, *shape, device="cuda", **kw)
+        self.rho, self.dg, self.z, self.v, self.packed, self.pairs = e(), e(self.dim), e(Z), e(C, self.dim), e(4), e(self.K, dtype=torch.int32)
+        self.st, p = n.current_stream(), n.ptr
+        n.check(n.lib.npa_perceive_features_forward_lists(ctypes.byref(self.gd), C, p(self.x), None, p(self.s), 1.0, 1.0, 1e-3, 0, 0, p(self.rho), p(self.dg),
+                                                          p(self.z), p(self.v), p(self.packed), p(self.snap.bin_offsets), p(self.snap.block_info),
+                                                          p(self.pairs), self.K, self.st))
+        self.dz = torch.randn(self.B, self.N, Z, device="cuda")
+        self.add = torch.randn(self.B, self.N, C, device="cuda")
+
+    def __call__(self, binned, add=None):
+        n, p = self.n, self.n.ptr
+        f = n.lib.npa_perceive_features_backward_binned if binned else n.lib.npa_perceive_features_backward_lists
+        nbytes = n.lib.npa_lists_backward_scratch_bytes(ctypes.byref(self.gd), self.C)
+        work, out = torch.empty(nbytes // 4, device="cuda"), torch.full((self.B, self.N, self.C), float("nan"), device="cuda")
+        n.check(f(ctypes.byref(self.gd), self.C, p(self.x), None, p(self.s), p(self.rho), p(self.dg), p(self.v), p(self.packed), p(self.dz), 1.0, 1.0, 0, 0,
+                  p(add), None, p(out), p(work), nbytes, p(self.snap.bin_offsets), p(self.pairs), self.K, self.st))
+        return out
+
+    def exact(self, b, idx):
+        """Float64 value for particles ``idx`` of system ``b``, and the sum of the magnitudes of its terms with weights that bound how
+        the rounding of a distance moves them: (h^2 - q)^3 by 3 (h^2 - q)^2 h^2, (h - d)^2 by 2 (h - d) h."""
+        C, D = self.C, self.dim
+        X, V, dz = self.x[b, :, :D].double(), 1.0 / self.rho[b].double(), self.dz[b].double()
+        gB, gG = dz[:, C:2 * C], dz[:, 2 * C:2 * C + C * D].reshape(-1, C, D)
+        f32 = lambda v: float(torch.tensor(v, dtype=torch.float32))
+        h, h2 = f32(self.eps), f32(self.eps ** 2)
+        cs = f32(4 / (math.pi * self.eps ** 8) if D == 2 else 315 / (64 * math.pi * self.eps ** 9))
+        cg = f32(10 / (math.pi * self.eps ** 5) if D == 2 else 15 / (math.pi * self.eps ** 6))
+        r = X[None] - X[idx][:, None]
+        if self.boundary == "periodic":
+            r = r - self.box * torch.round(r / self.box)
+        q = (r * r).sum(-1)
+        t, d = (h2 - q).clamp_min(0), (q + 1e-12).sqrt()
+        near = (q > 0) & (q < h2)
+        phi = torch.where(near, cg * 3 * (h - d).clamp_min(0) ** 2 / d, 0.0)
+        wide = torch.where(near, cg * 6 * (h - d).clamp_min(0) * h / d, 0.0)
+        K, Kw = phi[..., None] * r, wide[..., None] * r.abs()
+        value = cs * t ** 3 @ gB - torch.einsum("ijd,jfd->if", K, gG)
+        size = cs * 3 * h2 * t ** 2 @ gB.abs() + torch.einsum("ijd,jfd->if", Kw, gG.abs())
+        T, Tw = torch.einsum("j,ijd->id", V, K), torch.einsum("j,ijd->id", V, Kw)
+        own = lambda T, g: torch.einsum("id,ifd->if", T, g)
+        return (value * V[idx, None] - own(T, gG[idx]) + dz[idx, :C], size * V[idx, None] + own(Tw, gG[idx].abs()) + dz[idx, :C].abs())
+
+
+def _positions(dim, B, N, side, spread="uniform"):
+    x = (torch.rand(B, N, dim, device="cuda") - 0.5) * side
+    if spread == "lines":                                   # crowded cells beside empty ones
+        x[..., 1:] = torch.round(x[..., 1:] * 4 / side) * side / 4 + 0.002 * torch.randn_like(x[..., 1:])
+    if dim == 3:
+        x = torch.cat([x, torch.zeros_like(x[..., :1])], -1)
+    return x.contiguous()
+
+
+# tiles of eight particles, blocks of sixteen features; a tile over the end of a row of cells and of a system; one particle, one tile and one more
+@pytest.mark.parametrize("dim,B,N,cells,boundary,spread", [
+    (2, 1, 9, 1, "clamped", "uniform"), (2, 3, 701, 6, "clamped", "uniform"), (2, 2, 4096, 16, "clamped", "lines"), (2, 3, 1003, 7, "periodic", "uniform"),
+    (2, 1, 200, 4, "periodic", "uniform"), (3, 3, 6700, 9, "clamped", "uniform"), (3, 1, 20001, 11, "clamped", "lines")])
+@pytest.mark.parametrize("C", [1, 4, 13, 16, 17, 32])
+def test_against_float64(dim, B, N, cells, boundary, spread, C):
+    torch.manual_seed(C)
+    side = 1.0 if boundary == "periodic" else 0.97
+    call = Call(_positions(dim, B, N, side, spread), cells, 1.0 / cells, boundary, C)
+    got, lists = call(True), call(False)
+    assert not torch.equal(got, lists)                      # two kernels
+    assert torch.equal(call(True), got)                     # the same bits every time
+    assert torch.allclose(call(True, call.add), got + call.add, rtol=1e-6, atol=0)
+    for b in range(B):
+        for idx in torch.arange(0, N, max(1, N // 300), device="cuda").split(64):
+            want, size = call.exact(b, idx)
+            # four roundings of a weight's distance, 2^-22 of the split operands, and of the sums
+            assert ((got[b, idx].double() - want).abs() <= 16 * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("value", [float("inf"), float("-inf"), float("nan"), 3.0e38])
+def test_rows_that_are_not_finite_reach_their_neighbours_only(value):
+    torch.manual_seed(3)
+    call = Call(_positions(2, 2, 700, 0.97), 6, 1 / 6, "clamped", 16)
+    clean = call(True)
+    call.dz[0, 100, 20] = call.dz[1, 350, 40] = value       # of the blur and of the gradient
+    got, want = call(True), call(False)
+    fine = torch.isfinite(want)
+    assert torch.equal(torch.isfinite(got), fine)
+    assert torch.allclose(got[fine], want[fine], rtol=2e-5, atol=1e-4) and (~fine).any() and fine.float().mean() > 0.9
+    touched = (got != clean).any(-1)
+    assert touched.float().mean() < 0.5
+
