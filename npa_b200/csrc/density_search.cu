@@ -6,7 +6,7 @@
 // around the ones they span.  The candidates are staged end to end in shared memory and read as
 // broadcasts, two at a time in packed fp32x2; a lane shifts the sign of every r^2 - h^2 into a word, walks
 // the set bits of each 32 and collects slot numbers (bytes) in shared memory; the lists leave in runs,
-// eight lanes to a list.  No work items, no tickets, no reductions but the one between a particle's lanes.
+// four lanes to a list.  No work items, no tickets, no reductions but the one between a particle's lanes.
 // Morton hash, and fewer than 16,384 particles (density_item_kernel): the neighbours of 32 consecutive particles are scattered over many
 // short ranges; a warp takes the particles of one cell, lays the candidates of its 3^D cells end to end,
 // one gather per item, and tests 32 candidates, a lane each, against four particles at once; a scan of the
@@ -14,9 +14,10 @@
 // Both are bound by instruction issue: about 8 warp instructions per 32 tests in the first, 11 in the second, which
 // also spends as much again on its lists and on setting up an item.
 // Measured, B200, density + lists, us (before: a lane per particle with every list entry written as a word of its own,
-// and a walk per particle on Morton and 3D periodic grids): 262,144 particles 3D, ~240 candidates 140 -> 98;
-// 524,288 particles 3D periodic 542 -> 281; 65,536 particles 3D Morton, thin cells 61 -> 45; 4,096 particles 2D
-// periodic, 370 candidates 45 -> 17; 32,768 particles in 2D 20 -> 14.
+// and a walk per particle on Morton and 3D periodic grids): 262,144 particles 3D, ~240 candidates 140 -> 93;
+// 524,288 particles 3D periodic 542 -> 213 (265 while its candidates were staged range by range); 65,536 particles 3D Morton, thin cells 61 -> 45; 4,096 particles 2D
+// periodic, 370 candidates 45 -> 17; 32,768 particles in 2D 20 -> 13.  Of the 93 us staging takes 25, the tests 30, the collecting of
+// the entries 25 and their way out a dozen (kernels without one part).
 #include "neighbors.cuh"
 #include "ops.cuh"
 
@@ -171,42 +172,51 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                     S.j[k] = COUNT ? shift_code(0, 0, 0) : from[u];
                     if (MASS) S.m[k] = mass[u];
                 }
-            } else {  // up to 27 ranges, with image shifts: range by range, `group` lanes each
-                auto stage = [&](int group) {
-                    for (int r = lane / group; r < nr; r += 32 / group) {
-                        const int4 R = rng[r];
-                        const int e = min(R.w, c0 + count - R.y);
-#pragma unroll 2
-                        for (int k = max(0, c0 - R.y) + lane % group; k < e; k += group) {
-                            const int j = R.x + R.y + k, slot = R.y + k - c0;
-                            Pos<D> p = load_pos<D>(a.x, j);
-                            if (wrapped && !COUNT) {
-                                float lx, ly, lz = 0.f, hx, hy, hz = 0.f;
-                                shifted(g, 0, p.x, (R.z & 3) - 1, hx, lx);
-                                shifted(g, 1, p.y, ((R.z >> 2) & 3) - 1, hy, ly);
-                                if (D == 3) shifted(g, 2, p.z, ((R.z >> 4) & 3) - 1, hz, lz);
-                                p = Pos<D>{hx, hy, hz};
-                                S.x[kTileSlots / 2 + slot] = lx; S.y[kTileSlots / 2 + slot] = ly;
-                                if (D == 3) S.z[kTileSlots / 2 + slot] = lz;
-                            }
-                            if (!COUNT || !wrapped) outside |= outside_cells<D>(g, p, cx0 - 1, cx1 + 1, row_y - 1, row_y + 1, row_z - 1, row_z + 1);
-                            S.x[slot] = p.x; S.y[slot] = p.y;
-                            if (D == 3) S.z[slot] = p.z;
-                            S.j[slot] = COUNT ? R.z : j;
-                            if (MASS) S.m[slot] = __ldg(a.mass + j);
-                        }
+            } else {  // up to 27 ranges, with image shifts: the same, four slots a lane at a time
+                const bool low = wrapped && !COUNT;
+                for (int base = 0; base < padded; base += 4 * 32) {
+                    int which[4];  // range of the slot
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) which[u] = 0;
+                    for (int r = 1; r < nr; ++r) {
+                        const int at = rng[r].y - c0 - base - lane;
+#pragma unroll
+                        for (int u = 0; u < 4; ++u) which[u] += u * 32 >= at ? 1 : 0;
                     }
-                };
-                if (total > 20 * nr) stage(32);  // by the mean length of the ranges
-                else stage(8);
-                for (int k = count + lane; k < padded; k += 32) {
-                    S.x[k] = S.y[k] = kFarAway;
-                    if (D == 3) S.z[k] = kFarAway;
-                    S.j[k] = COUNT ? shift_code(0, 0, 0) : 0;
-                    if (MASS) S.m[k] = 0.f;
-                    if (wrapped && !COUNT) {
-                        S.x[kTileSlots / 2 + k] = S.y[kTileSlots / 2 + k] = 0.f;
-                        if (D == 3) S.z[kTileSlots / 2 + k] = 0.f;
+                    Pos<D> p[4];
+                    int code[4], from[4];
+                    float mass[4];
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int k = base + u * 32 + lane;
+                        const int4 R = rng[which[u]];
+                        const bool real = k < count;
+                        p[u] = Pos<D>{kFarAway, kFarAway, kFarAway};
+                        from[u] = real ? R.x + c0 + k : 0;
+                        code[u] = real ? R.z : shift_code(0, 0, 0);
+                        if (real) p[u] = load_pos<D>(a.x, from[u]);
+                        mass[u] = MASS && real ? __ldg(a.mass + from[u]) : 0.f;
+                    }
+#pragma unroll
+                    for (int u = 0; u < 4; ++u) {
+                        const int k = base + u * 32 + lane;
+                        if (k >= padded) break;
+                        if (low) {
+                            float lx = 0.f, ly = 0.f, lz = 0.f, hx = p[u].x, hy = p[u].y, hz = p[u].z;
+                            if (k < count) {
+                                shifted(g, 0, p[u].x, (code[u] & 3) - 1, hx, lx);
+                                shifted(g, 1, p[u].y, ((code[u] >> 2) & 3) - 1, hy, ly);
+                                if (D == 3) shifted(g, 2, p[u].z, ((code[u] >> 4) & 3) - 1, hz, lz);
+                            }
+                            p[u] = Pos<D>{hx, hy, hz};
+                            S.x[kTileSlots / 2 + k] = lx; S.y[kTileSlots / 2 + k] = ly;
+                            if (D == 3) S.z[kTileSlots / 2 + k] = lz;
+                        }
+                        if (k < count && (!COUNT || !wrapped)) outside |= outside_cells<D>(g, p[u], cx0 - 1, cx1 + 1, row_y - 1, row_y + 1, row_z - 1, row_z + 1);
+                        S.x[k] = p[u].x; S.y[k] = p[u].y;
+                        if (D == 3) S.z[k] = p[u].z;
+                        S.j[k] = COUNT ? code[u] : from[u];
+                        if (MASS) S.m[k] = mass[u];
                     }
                 }
             }
@@ -225,14 +235,21 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                 }
                 const int at = found + before, take = min(held, K - 1 - at);  // entries that still fit
                 __syncwarp();
-                // eight lanes write a list, four lists at a time
+                // four lanes write a list, two entries each at a time, eight lists at once (eight lanes and one entry: 262,144 particles in
+                // 3D 100 us instead of 93, 524,288 periodic 231 instead of 213; two lanes 94 and 214, but 40 instead of 37 in 2D)
 #pragma unroll 1
-                for (int l0 = 0; l0 < 32; l0 += 4) {
-                    const int l = l0 + (lane >> 3);
+                for (int l0 = 0; l0 < 32; l0 += 8) {
+                    const int l = l0 + (lane >> 2);
                     const int n = __shfl_sync(kFull, take, l);
                     int32_t *list = a.pair_cache + (long long)__shfl_sync(kFull, i, l) * K + 1 + __shfl_sync(kFull, at, l);
                     const unsigned char *from = S.run + l * kTileRun;
-                    for (int e = lane & 7; e < n; e += 8) list[e] = S.j[from[e]];
+                    int e = lane & 3;
+                    for (; e + 4 < n; e += 8) {
+                        const int j0 = S.j[from[e]], j1 = S.j[from[e + 4]];
+                        list[e] = j0;
+                        list[e + 4] = j1;
+                    }
+                    if (e < n) list[e] = S.j[from[e]];
                 }
                 found += sum;
                 held = 0;
@@ -309,7 +326,7 @@ density_tile_kernel(const __grid_constant__ ScalarFwdArgs a, const __grid_consta
                 return mine ? m : 0u;
             };
             // One copy of the rest for all ways of testing: with a copy for each, a sixth of the periodic kernel's stalls were
-            // waits for instructions (524,288 particles 311 us, so 281).
+            // waits for instructions (524,288 particles 311 us, so 281, when that was tried).
             for (int s0 = part * 32; s0 < padded; s0 += 32 * kShare) {
                 unsigned m;
                 if (PER && (check || (COUNT && wrapped))) m = test(Mode<2>(), s0);
