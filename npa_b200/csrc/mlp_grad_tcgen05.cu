@@ -40,23 +40,32 @@ constexpr int kGradEpilogueWarps = 8;
 constexpr int kGradWarpMma = 8, kGradWarpCopy = 9, kGradWarpProducer0 = 10;
 constexpr int kGradThreads = (kGradWarpProducer0 + kGradProducerWarps) * 32;
 constexpr int kGradAtomBytes = 512;                // 4 rows x 128 bytes (32 columns)
-constexpr int kGradAtomsH = 4, kGradAtomsZ = 6, kGradAtomsY = 2;  // atoms of 32 columns: dh / h, [z | 1], dy
-// byte offsets inside a stage: [k-group of 8 rows][4-row half][atom] per operand part
-constexpr int kGradOffDhHi = 0, kGradOffDhLo = 8192, kGradOffHHi = 16384, kGradOffHLo = 24576;
-constexpr int kGradOffZHi = 32768, kGradOffZLo = 45056, kGradOffYHi = 57344, kGradOffYLo = 61440;
-constexpr int kGradStageBytes = 65536;
-constexpr int kGradStages = 2;                     // operand stages
-constexpr int kGradRawStages = 3;                  // raw input rows, as the bulk copies deliver them
-// a raw stage: 16 rows of dh | h | z | dy, each block contiguous as in global memory
-constexpr int kGradRawDh = 0, kGradRawH = 8192, kGradRawZ = 16384, kGradRawY = 16384 + 11264, kGradRawBytes = 16384 + 11264 + 3072;
+constexpr int kGradAtomsH = 4;                     // atoms of 32 columns: dh / h
+// The rest of the shape: atoms of [z | 1] and of dy, operand stages, raw stages.  Byte offsets inside a stage: [k-group of 8 rows][4-row
+// half][atom] per operand part; a raw stage holds 16 rows of dh | h | z | dy, each block contiguous as in global memory.
+template <int ATOMS_Z, int ATOMS_Y, int STAGES, int RAW_STAGES>
+struct GradShape {
+    static constexpr int kAtomsZ = ATOMS_Z, kAtomsY = ATOMS_Y, kStages = STAGES, kRawStages = RAW_STAGES;
+    static constexpr int kOffDhHi = 0, kOffDhLo = 8192, kOffHHi = 16384, kOffHLo = 24576, kOffZHi = 32768;
+    static constexpr int kOffZLo = kOffZHi + 4 * ATOMS_Z * kGradAtomBytes, kOffYHi = kOffZLo + 4 * ATOMS_Z * kGradAtomBytes;
+    static constexpr int kOffYLo = kOffYHi + 4 * ATOMS_Y * kGradAtomBytes, kStageBytes = kOffYLo + 4 * ATOMS_Y * kGradAtomBytes;
+    // in + 1 columns of D1 fit the atoms, out of D2
+    static constexpr int kMaxIn = ATOMS_Z == 6 ? 175 : 32 * ATOMS_Z - 1, kMaxOut = ATOMS_Y == 2 ? 48 : 32 * ATOMS_Y;
+    static constexpr int kRawDh = 0, kRawH = 8192, kRawZ = 16384, kRawY = kRawZ + (kGradStageRows * kMaxIn * 4 + 127) / 128 * 128;
+    static constexpr int kRawBytes = (kRawY + kGradStageRows * kMaxOut * 4 + 127) / 128 * 128;
+    static_assert(kStageBytes % 1024 == 0 && STAGES <= 4 && RAW_STAGES <= 4, "stages are aligned to the swizzle, and have barriers");
+};
+using GradWide = GradShape<6, 2, 2, 3>;    // up to 175 columns of z and 48 of dy: 64 KB per stage
+using GradNarrow = GradShape<3, 1, 3, 3>;  // up to 95 and 32: 48 KB, a stage more and a quarter fewer stores
+// (B200, us, wide -> narrow: 32,768 rows of 66 and 18 20.9 -> 19.6, 65,536 rows of 83 and 19 40.1 -> 37.6.)
 constexpr int kGradTmemCols = 512, kGradSumCol = 256, kGradD2Col = 192;  // accumulators at 0 / 192, running sums 256 columns up
-constexpr int kGradMaxIn = 175, kGradMaxOut = 48;  // in + 1 <= 192 columns of D1 (six atoms), out <= 64 of D2
+constexpr int kGradMaxIn = GradWide::kMaxIn, kGradMaxOut = GradWide::kMaxOut;
 
 enum { GRAD_STATUS_MMA = 16, GRAD_STATUS_PRODUCER = 32, GRAD_STATUS_EPILOGUE = 64 };
 
 struct GradShared {
-    uint64_t full[kGradStages], empty[kGradStages], acc_full, acc_empty;
-    uint64_t raw_full[kGradRawStages], raw_empty[kGradRawStages];
+    uint64_t full[4], empty[4], acc_full, acc_empty;
+    uint64_t raw_full[4], raw_empty[4];
     uint32_t tmem_base;
     int abort;
 };
@@ -72,6 +81,7 @@ struct GradArgs {
 
 unsigned *umma_status_word();  // mlp_tcgen05.cu: device address of the status word on the current device
 
+template <typename S>
 __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __grid_constant__ GradArgs args) {
     after_previous_kernel();
     const float *__restrict__ Z = args.z;
@@ -83,16 +93,16 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
     unsigned *status = args.status;
     extern __shared__ uint8_t grad_smem_raw[];
     uint8_t *base = grad_smem_raw + ((1024u - (smem_u32(grad_smem_raw) & 1023u)) & 1023u);
-    uint8_t *raw = base + kGradStages * kGradStageBytes;
-    GradShared *sh = (GradShared *)(raw + kGradRawStages * kGradRawBytes);
+    uint8_t *raw = base + S::kStages * S::kStageBytes;
+    GradShared *sh = (GradShared *)(raw + S::kRawStages * S::kRawBytes);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kGradStages; ++s) {
+        for (int s = 0; s < S::kStages; ++s) {
             mbar_init(&sh->full[s], kGradProducerWarps);
             mbar_init(&sh->empty[s], 1);
         }
-        for (int s = 0; s < kGradRawStages; ++s) {
+        for (int s = 0; s < S::kRawStages; ++s) {
             mbar_init(&sh->raw_full[s], 1);                    // the copy lane's arrival + the bytes of four copies
             mbar_init(&sh->raw_empty[s], kGradProducerWarps);  // every producer warp has read its row
         }
@@ -140,19 +150,19 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
                 for (int st = 0; st < nst; ++st) {
                     if (!(ok = umma_wait(&sh->full[s], ph, &sh->abort))) break;
                     tc_fence_after();
-                    const unsigned sa = sbase + s * kGradStageBytes;
+                    const unsigned sa = sbase + s * S::kStageBytes;
 #pragma unroll
                     for (int kk = 0; kk < 2; ++kk) {
-                        const unsigned oh = kk * 2 * kGradAtomsH * kGradAtomBytes, oz = kk * 2 * kGradAtomsZ * kGradAtomBytes;
-                        const unsigned oy = kk * 2 * kGradAtomsY * kGradAtomBytes;
-                        const uint64_t a1h = umma_desc_mn32(sa + kGradOffDhHi + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
-                        const uint64_t a1l = umma_desc_mn32(sa + kGradOffDhLo + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
-                        const uint64_t b1h = umma_desc_mn32(sa + kGradOffZHi + oz, kGradAtomBytes, kGradAtomsZ * kGradAtomBytes);
-                        const uint64_t b1l = umma_desc_mn32(sa + kGradOffZLo + oz, kGradAtomBytes, kGradAtomsZ * kGradAtomBytes);
-                        const uint64_t a2h = umma_desc_mn32(sa + kGradOffHHi + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
-                        const uint64_t a2l = umma_desc_mn32(sa + kGradOffHLo + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
-                        const uint64_t b2h = umma_desc_mn32(sa + kGradOffYHi + oy, kGradAtomBytes, kGradAtomsY * kGradAtomBytes);
-                        const uint64_t b2l = umma_desc_mn32(sa + kGradOffYLo + oy, kGradAtomBytes, kGradAtomsY * kGradAtomBytes);
+                        const unsigned oh = kk * 2 * kGradAtomsH * kGradAtomBytes, oz = kk * 2 * S::kAtomsZ * kGradAtomBytes;
+                        const unsigned oy = kk * 2 * S::kAtomsY * kGradAtomBytes;
+                        const uint64_t a1h = umma_desc_mn32(sa + S::kOffDhHi + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
+                        const uint64_t a1l = umma_desc_mn32(sa + S::kOffDhLo + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
+                        const uint64_t b1h = umma_desc_mn32(sa + S::kOffZHi + oz, kGradAtomBytes, S::kAtomsZ * kGradAtomBytes);
+                        const uint64_t b1l = umma_desc_mn32(sa + S::kOffZLo + oz, kGradAtomBytes, S::kAtomsZ * kGradAtomBytes);
+                        const uint64_t a2h = umma_desc_mn32(sa + S::kOffHHi + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
+                        const uint64_t a2l = umma_desc_mn32(sa + S::kOffHLo + oh, kGradAtomBytes, kGradAtomsH * kGradAtomBytes);
+                        const uint64_t b2h = umma_desc_mn32(sa + S::kOffYHi + oy, kGradAtomBytes, S::kAtomsY * kGradAtomBytes);
+                        const uint64_t b2l = umma_desc_mn32(sa + S::kOffYLo + oy, kGradAtomBytes, S::kAtomsY * kGradAtomBytes);
                         const int acc = (st | kk) != 0;
                         umma_tf32(d1, a1l, b1h, idesc1, acc);
                         umma_tf32(d1, a1h, b1l, idesc1, 1);
@@ -162,7 +172,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
                         umma_tf32(d2, a2h, b2h, idesc2, 1);
                     }
                     umma_commit(&sh->empty[s]);
-                    if (++s == kGradStages) {
+                    if (++s == S::kStages) {
                         s = 0;
                         ph ^= 1;
                     }
@@ -184,13 +194,13 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
             for (int q = 0; q < nraw; ++q) {
                 if (!(ok = umma_wait(&sh->raw_empty[rs], rphase, &sh->abort))) break;
                 const long long row = (first_stage + q) * kGradStageRows;
-                uint8_t *dst = raw + rs * kGradRawBytes;
+                uint8_t *dst = raw + rs * S::kRawBytes;
                 mbar_arrive_expect(&sh->raw_full[rs], 2u * 8192u + bz + by);
-                bulk_copy_g2s(dst + kGradRawDh, DH + row * kGradHidden, 8192u, &sh->raw_full[rs]);
-                bulk_copy_g2s(dst + kGradRawH, H + row * kGradHidden, 8192u, &sh->raw_full[rs]);
-                bulk_copy_g2s(dst + kGradRawZ, Z + row * K1, bz, &sh->raw_full[rs]);
-                bulk_copy_g2s(dst + kGradRawY, DY + row * O, by, &sh->raw_full[rs]);
-                if (++rs == kGradRawStages) {
+                bulk_copy_g2s(dst + S::kRawDh, DH + row * kGradHidden, 8192u, &sh->raw_full[rs]);
+                bulk_copy_g2s(dst + S::kRawH, H + row * kGradHidden, 8192u, &sh->raw_full[rs]);
+                bulk_copy_g2s(dst + S::kRawZ, Z + row * K1, bz, &sh->raw_full[rs]);
+                bulk_copy_g2s(dst + S::kRawY, DY + row * O, by, &sh->raw_full[rs]);
+                if (++rs == S::kRawStages) {
                     rs = 0;
                     rphase ^= 1;
                 }
@@ -213,21 +223,21 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
             float v[16];
             if (q < nraw) {
                 if (!(ok = umma_wait(&sh->raw_full[rs], rphase, &sh->abort))) break;
-                const float *r = (const float *)(raw + rs * kGradRawBytes);
+                const float *r = (const float *)(raw + rs * S::kRawBytes);
 #pragma unroll
                 for (int t = 0; t < 4; ++t) {
-                    v[t] = r[kGradRawDh / 4 + pw * kGradHidden + 32 * t + lane];
-                    v[4 + t] = r[kGradRawH / 4 + pw * kGradHidden + 32 * t + lane];
+                    v[t] = r[S::kRawDh / 4 + pw * kGradHidden + 32 * t + lane];
+                    v[4 + t] = r[S::kRawH / 4 + pw * kGradHidden + 32 * t + lane];
                 }
 #pragma unroll
-                for (int t = 0; t < 6; ++t) {
+                for (int t = 0; t < S::kAtomsZ; ++t) {
                     const int col = 32 * t + lane;
-                    v[8 + t] = col < K1 ? r[kGradRawZ / 4 + pw * K1 + col] : (col == K1 ? 1.f : 0.f);  // the ones column gives db1
+                    v[8 + t] = col < K1 ? r[S::kRawZ / 4 + pw * K1 + col] : (col == K1 ? 1.f : 0.f);  // the ones column gives db1
                 }
 #pragma unroll
-                for (int t = 0; t < 2; ++t) {
+                for (int t = 0; t < S::kAtomsY; ++t) {
                     const int col = 32 * t + lane;
-                    v[14 + t] = col < O ? r[kGradRawY / 4 + pw * O + col] : 0.f;
+                    v[14 + t] = col < O ? r[S::kRawY / 4 + pw * O + col] : 0.f;
                 }
             } else {
                 const long long row = (first_stage + q) * kGradStageRows + pw;
@@ -238,12 +248,12 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
                         v[4 + t] = __ldg(H + row * kGradHidden + 32 * t + lane);
                     }
 #pragma unroll
-                    for (int t = 0; t < 6; ++t) {
+                    for (int t = 0; t < S::kAtomsZ; ++t) {
                         const int col = 32 * t + lane;
                         v[8 + t] = col < K1 ? __ldg(Z + row * K1 + col) : (col == K1 ? 1.f : 0.f);
                     }
 #pragma unroll
-                    for (int t = 0; t < 2; ++t) {
+                    for (int t = 0; t < S::kAtomsY; ++t) {
                         const int col = 32 * t + lane;
                         v[14 + t] = col < O ? __ldg(DY + row * O + col) : 0.f;
                     }
@@ -253,7 +263,7 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
                 }
             }
             if (!(ok = umma_wait(&sh->empty[s], phase, &sh->abort))) break;
-            float *stage = (float *)(base + s * kGradStageBytes);
+            float *stage = (float *)(base + s * S::kStageBytes);
             auto put = [&](int off_hi, int off_lo, int natoms, int atom, float x) {
                 const int f = ((kk * 2 + half4) * natoms + atom) * (kGradAtomBytes / 4) + at;
                 const float head = __uint_as_float(tf32_head_bits(x));
@@ -262,24 +272,24 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
             };
 #pragma unroll
             for (int t = 0; t < 4; ++t) {
-                put(kGradOffDhHi, kGradOffDhLo, kGradAtomsH, t, v[t]);
-                put(kGradOffHHi, kGradOffHLo, kGradAtomsH, t, v[4 + t]);
+                put(S::kOffDhHi, S::kOffDhLo, kGradAtomsH, t, v[t]);
+                put(S::kOffHHi, S::kOffHLo, kGradAtomsH, t, v[4 + t]);
             }
 #pragma unroll
-            for (int t = 0; t < 6; ++t) put(kGradOffZHi, kGradOffZLo, kGradAtomsZ, t, v[8 + t]);
+            for (int t = 0; t < S::kAtomsZ; ++t) put(S::kOffZHi, S::kOffZLo, S::kAtomsZ, t, v[8 + t]);
 #pragma unroll
-            for (int t = 0; t < 2; ++t) put(kGradOffYHi, kGradOffYLo, kGradAtomsY, t, v[14 + t]);
+            for (int t = 0; t < S::kAtomsY; ++t) put(S::kOffYHi, S::kOffYLo, S::kAtomsY, t, v[14 + t]);
             fence_proxy_async();  // the MMA reads these through the async proxy
             __syncwarp();
             if (lane == 0) {
                 mbar_arrive(&sh->full[s]);
                 if (q < nraw) mbar_arrive(&sh->raw_empty[rs]);  // the raw row has been consumed
             }
-            if (q < nraw && ++rs == kGradRawStages) {
+            if (q < nraw && ++rs == S::kRawStages) {
                 rs = 0;
                 rphase ^= 1;
             }
-            if (++s == kGradStages) {
+            if (++s == S::kStages) {
                 s = 0;
                 phase ^= 1;
             }
@@ -389,11 +399,13 @@ static int grad_round16(int v) { return (v + 15) / 16 * 16; }
 
 struct GradDevice {
     unsigned *status = nullptr;
-    bool smem_set = false;
+    bool smem_set[2] = {false, false};  // per shape
 };
 static std::mutex g_grad_mutex;
 static GradDevice g_grad_device[64];
-constexpr int kGradSmemBytes = 1024 + kGradStages * kGradStageBytes + kGradRawStages * kGradRawBytes + (int)sizeof(GradShared);
+template <typename S>
+constexpr int kGradSmemBytes = 1024 + S::kStages * S::kStageBytes + S::kRawStages * S::kRawBytes + (int)sizeof(GradShared);
+static_assert(kGradSmemBytes<GradWide> <= 227 * 1024 && kGradSmemBytes<GradNarrow> <= 227 * 1024, "shared memory of a CTA");
 
 }  // namespace npa
 
@@ -431,6 +443,9 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
     a.stages_per_cta = (int)((stages_total + ctas - 1) / ctas);
     a.ctas = (int)((stages_total + a.stages_per_cta - 1) / a.stages_per_cta);
 
+    const bool narrow = in_dim <= GradNarrow::kMaxIn && out_dim <= GradNarrow::kMaxOut;
+    const auto kernel = narrow ? mlp_grad_umma_kernel<GradNarrow> : mlp_grad_umma_kernel<GradWide>;
+    const int smem = narrow ? kGradSmemBytes<GradNarrow> : kGradSmemBytes<GradWide>;
     int dev = 0;
     cudaError_t e = cudaGetDevice(&dev);
     if (e != cudaSuccess || dev < 0 || dev >= 64) return fail(NPA_ERR_CUDA, "%s: cudaGetDevice: %s", me, cudaGetErrorString(e));
@@ -438,15 +453,15 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
         std::lock_guard<std::mutex> lock(g_grad_mutex);
         GradDevice &d = g_grad_device[dev];
         if (!d.status && !(d.status = umma_status_word())) return fail(NPA_ERR_CUDA, "%s: no status word", me);
-        if (!d.smem_set) {
-            e = cudaFuncSetAttribute(mlp_grad_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmemBytes);
+        if (!d.smem_set[narrow]) {
+            e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
             if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "%s: raising the shared-memory limit: %s", me, cudaGetErrorString(e));
-            d.smem_set = true;
+            d.smem_set[narrow] = true;
         }
         a.status = d.status;
     }
     cudaStream_t st = (cudaStream_t)stream;
-    launch_early(mlp_grad_umma_kernel, a.ctas, kGradThreads, kGradSmemBytes, st, a);
+    launch_early(kernel, a.ctas, kGradThreads, smem, st, a);
     int rc = check_launch("mlp_grad_umma_kernel");
     if (rc != NPA_OK) return rc;
     const int quads = kGradHidden * ((in_dim + 4) / 4 + (out_dim + 3) / 4);

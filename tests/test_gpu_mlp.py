@@ -191,3 +191,22 @@ def test_forward_with_the_update(dim, C, N, mask):
                                                mask == "uniforms", 0.5, C, 0.7, 0.9, wrap, n.ptr(u), n.ptr(x1), n.ptr(s1), st))
             assert torch.equal(x1, xo) and torch.equal(s1, so)
         assert torch.equal(h1, h) and torch.equal(u1[:, :dim], y[:, :dim])
+
+
+@pytest.mark.parametrize("k,o", [(95, 32), (96, 32), (95, 33), (94, 31), (175, 48)])   # both shapes of the kernel, on the lines between them
+@pytest.mark.parametrize("rows", [1, 16, 17, 129, 40001])                               # a stage of rows, a segment, more than a segment per CTA
+def test_weight_gradients_of_either_shape(engine, k, o, rows):
+    from npa_b200 import _native as n
+    if engine != "tcgen05":
+        pytest.skip("the kernel of the tensor-memory engine")
+    gen = torch.Generator(device="cuda").manual_seed(rows + k)
+    randn = lambda *s: torch.randn(*s, generator=gen, device="cuda")
+    z, dh, h, dy = randn(rows, k), randn(rows, 128), randn(rows, 128), randn(rows, o)
+    floats = n.lib.npa_mlp_weight_grad_tcgen05_scratch_floats(rows, k, o)
+    scratch, gw1, gw2, gb1 = (torch.full(s, float("nan"), device="cuda") for s in ((floats,), (128, k), (o, 128), (128,)))
+    n.check(n.lib.npa_mlp_weight_grad_tcgen05(n.ptr(z), n.ptr(dh), n.ptr(h), n.ptr(dy), rows, k, 128, o, n.ptr(scratch), floats, n.ptr(gw1), n.ptr(gw2),
+                                              n.ptr(gb1), n.current_stream()))
+    for got, a, b in ((gw1, dh, z), (gw2, dy, h), (gb1[:, None], dh, torch.ones_like(z[:, :1]))):
+        a, b = a.double(), b.double()
+        # heads and tails drop 2^-22 per product, a chain of 48 accumulations truncates by 2^-23 of its sum each
+        assert ((got.double() - a.T @ b).abs() <= (2.0 ** -21 + 48 * 2.0 ** -23) * (a.abs().T @ b.abs())).all()
