@@ -599,6 +599,22 @@ int npa_mlp_step_forward(const npa_grid *g, const float *z, const float *b1, flo
                          float *s_out, void *stream);
 int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image_bytes, float *C, int64_t rows,
                                 int32_t in_dim, int32_t out_dim, void *stream);
+/* The backward of a step's perception without dL/dz in memory, for steps whose positions want no gradient: the product dL/dz = dh W1
+ * (dh [B*N, 128]) takes its rows apart as they leave the tensor cores, and the sweep of npa_perceive_features_backward_binned follows.
+ * rows_image holds npa_step_rows_image_bytes() bytes (0: this number of features is not taken; multiples of four up to 32 are) and is
+ * made by npa_bin_particles_step_images, which is npa_bin_particles_mlp_images otherwise (in_dim = 2C + C D + D, out_dim = D + C).
+ * vgrad, rows_image and scratch 16-byte aligned; grad_s [B*N, C] as grad_s_add (may be NULL). */
+int64_t npa_step_rows_image_bytes(const npa_grid *g, int32_t channels);
+int npa_bin_particles_step_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation,
+                                  float *x_out, float *s_out, const float *W1, const float *W2, int64_t w1_stride_out,
+                                  int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,
+                                  int64_t scratch_bytes, void *rows_image, int64_t rows_image_bytes, void *stream);
+int64_t npa_step_perceive_backward_scratch_bytes(const npa_grid *g, int32_t channels);
+int npa_step_perceive_backward(const npa_grid *g, int32_t channels, const float *dh, const void *rows_image, int64_t rows_image_bytes,
+                               const float *x_bin, const float *s_bin, const float *rho, const float *vgrad, const float *packed,
+                               float coef, int32_t log_norm_grad, const float *grad_s_add, float *grad_s, void *scratch,
+                               int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride,
+                               void *stream);
 /* Self-test of those bounded waits: a two-warp kernel in which warp 0 waits `limit_us` (1..1,000,000)
  * on an mbarrier that nothing completes, gives up and raises the kernel's leave flag, and warp 1,
  * waiting on a second such mbarrier with the full limit, leaves through the flag.  device_result[0]

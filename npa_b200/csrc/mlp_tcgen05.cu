@@ -27,10 +27,17 @@
 // positions and states instead of y, of which the backward only needs the raw displacements.  Measured, B200, us, two kernels -> one:
 // 262,144 particles in 3D, C = 32, 142 + 25.5 -> 159; pass of an inference step of 4,096 in 2D 54.2 -> 52.7, of 2,500 in a graph 37.8 -> 35.8.
 //
+// The backward of a step whose positions want no gradient takes dL/dz = dh W1 apart in the epilogue (umma_store_parts): the weights' columns
+// stand in the order of StepColumns, so that an axis of the gradient is a run of columns, and the rows that the feature sweep reads leave
+// instead of dL/dz, which went to memory (rows of an odd number of floats) and came back.  Measured, B200, us, with the kernel that took it
+// apart before -> this one: 262,144 particles in 3D, C = 32, 97 + 85 -> 124; 65,536, C = 16, 27 + 16 -> 30; 32,768 in 2D 17 + 11 -> 17.5 (a
+// training step 1,466 -> 1,422, 304 -> 296, 183 -> 175).  Same products and expressions: the same bits.
+//
 // Every wait on an mbarrier is bounded in time; a wait that gives up raises a flag that ends all
 // roles, the CTA frees its tensor memory and the host reads the reason from a status word.
 #include <mutex>
 
+#include "perceive_backward.cuh"
 #include "step_update.cuh"
 #include "umma.cuh"
 #include "weight_image.cuh"
@@ -90,6 +97,7 @@ struct UmmaArgs {
     int D;
     StepArgs step;
     Geom g;
+    StepRows parts;  // kUmmaParts: where the rows go instead of C
 };
 constexpr int kUmmaStepQuads = 4;  // float4 of the states per epilogue thread and tile: up to 32 features
 
@@ -100,7 +108,11 @@ __global__ void weight_image_kernel(const __grid_constant__ ImageJobs jobs) {
     write_image_element(jobs, blockIdx.x * blockDim.x + threadIdx.x);
 }
 
-enum : int { kUmmaOneLayer = 0, kUmmaTwoLayers = 1, kUmmaStep = 2 };
+enum : int { kUmmaOneLayer = 0, kUmmaTwoLayers = 1, kUmmaStep = 2, kUmmaParts2 = 3, kUmmaParts3 = 4, kUmmaModes = 5 };
+constexpr int kUmmaPartPitch = 12;  // floats per staged row of 8 features: float4 writes of eight lanes cover all banks
+__host__ __device__ constexpr int umma_epilogue_floats(int mode) {
+    return mode == kUmmaParts2 || mode == kUmmaParts3 ? kUmmaEpilogueWarps * 32 * kUmmaPartPitch * (mode == kUmmaParts2 ? 4 : 5) : kUmmaEpiFloats;
+}
 
 // The tile of the second layer as the Euler update: the epilogue's threads move four states at a time, the first 128 of them a position.
 template <int D>
@@ -143,6 +155,84 @@ __device__ __forceinline__ void umma_prefetch_step(const UmmaArgs &a, long long 
     else if (f >= 16 && f < 20 && a.step.mask && (f - 16) * 32 < rows) fetch(a.step.mask + row0 + (f - 16) * 32);
 }
 
+// One warp's 32 rows of a tile of dL/dz, columns in the order of StepColumns, as the upstream rows of the perception's backward: eight features
+// at a time, every second eight (`first`: 0 or 1); lane = row, four features' gradients through the log-normalisation together, then
+// through shared memory so that 32-byte sectors leave whole.  `release` hands the accumulator back.
+template <int D, typename Release>
+__device__ __forceinline__ void umma_store_parts(const StepRows &p, unsigned taddr, float *stg, long long row0, int nrows, int first, int lane, Release release) {
+    const int C = p.C, S = StepColumns::section(C), units = (C + 7) / 8;
+    const float *vg = p.vgrad + (row0 + lane) * C * D;
+    float v[4 * D];
+    auto fetch = [&](int f) {
+#pragma unroll
+        for (int q = 0; q < D; ++q) {
+            const float4 t = lane < nrows ? __ldg(reinterpret_cast<const float4 *>(vg + f * D) + q) : make_float4(0.f, 0.f, 0.f, 0.f);
+            v[4 * q] = t.x; v[4 * q + 1] = t.y; v[4 * q + 2] = t.z; v[4 * q + 3] = t.w;
+        }
+    };
+    if (first >= units) {
+        release();
+        return;
+    }
+    fetch(8 * first);
+    float *mine = stg + lane * kUmmaPartPitch;
+#pragma unroll 1
+    for (int u = first; u < units; u += 2) {
+        const int f0 = 8 * u, width = min(8, C - f0);
+#pragma unroll
+        for (int sec = 0; sec < 2; ++sec) {
+            unsigned r[8];
+            tmem_ld8(taddr + sec * S + f0, r);
+            tc_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 2; ++q)
+                *reinterpret_cast<float4 *>(mine + sec * 32 * kUmmaPartPitch + 4 * q) =
+                    make_float4(__uint_as_float(r[4 * q]), __uint_as_float(r[4 * q + 1]), __uint_as_float(r[4 * q + 2]), __uint_as_float(r[4 * q + 3]));
+        }
+#pragma unroll 1
+        for (int h = 0; h < width; h += 4) {
+            unsigned r[D][4];
+            float out[D][4], w[4 * D];
+#pragma unroll
+            for (int d = 0; d < D; ++d) tmem_ld4(taddr + (2 + d) * S + f0 + h, r[d]);
+#pragma unroll
+            for (int q = 0; q < 4 * D; ++q) w[q] = v[q] * p.coef;
+            const int next = h + 4 < width ? f0 + h + 4 : f0 + 16;
+            if (next < C) fetch(next);
+            tc_wait_ld();
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                float gin[D], gout[D];
+#pragma unroll
+                for (int d = 0; d < D; ++d) gin[d] = __uint_as_float(r[d][q]);
+                log_normalize_backward<D>(w + q * D, gin, p.log_norm, p.coef, gout);
+#pragma unroll
+                for (int d = 0; d < D; ++d) out[d][q] = gout[d];
+            }
+#pragma unroll
+            for (int d = 0; d < D; ++d)
+                *reinterpret_cast<float4 *>(mine + (2 + d) * 32 * kUmmaPartPitch + h) = make_float4(out[d][0], out[d][1], out[d][2], out[d][3]);
+        }
+        if (u + 2 >= units) release();
+        __syncwarp();
+        const int half = 4 * (lane & 1);
+        if (half < width) {
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int row = (lane >> 1) + 16 * i;
+                if (row >= nrows) continue;
+                const float *from = stg + row * kUmmaPartPitch + half;
+                *reinterpret_cast<float4 *>(p.direct + (row0 + row) * C + f0 + half) = *reinterpret_cast<const float4 *>(from);
+                float *to = p.rows + (row0 + row) * p.pitch + f0 + half;
+#pragma unroll
+                for (int sec = 0; sec <= D; ++sec)
+                    *reinterpret_cast<float4 *>(to + sec * C) = *reinterpret_cast<const float4 *>(from + (1 + sec) * 32 * kUmmaPartPitch);
+            }
+        }
+        __syncwarp();
+    }
+}
+
 template <int MODE>
 __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __grid_constant__ UmmaArgs args) {
     after_previous_kernel();
@@ -156,7 +246,8 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
     const int K = args.K, N = args.N, Np = args.Np, nchunks = args.nchunks, last_ksteps = args.last_ksteps;
     const int stages = args.stages, stage_bytes = args.stage_bytes;
     const bool relu = args.relu != 0;
-    constexpr bool fuse = MODE != kUmmaOneLayer;  // two-layer mode
+    constexpr bool fuse = MODE == kUmmaTwoLayers || MODE == kUmmaStep;  // two-layer mode
+    constexpr int kParts = MODE == kUmmaParts2 ? 2 : MODE == kUmmaParts3 ? 3 : 0;
     const int N2 = args.N2, N2p = args.N2p;
     const int acc_stride = fuse ? 128 : kUmmaAccStride;
     extern __shared__ uint8_t umma_smem_raw[];
@@ -164,7 +255,7 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
     uint8_t *w2s = base + (size_t)stages * stage_bytes;   // two-layer mode: the whole image of W2, resident
     const int w2_bytes = fuse ? 4 * 2 * N2p * 128 : 0;
     float *epi = (float *)(w2s + w2_bytes);
-    float *ytile = epi + kUmmaEpiFloats;                  // two-layer mode: the second layer's tile, rows of N2 floats as in global memory
+    float *ytile = epi + umma_epilogue_floats(MODE);                  // two-layer mode: the second layer's tile, rows of N2 floats as in global memory
     UmmaShared *sh = (UmmaShared *)(ytile + (fuse ? ((kUmmaRows * N2 + 3) & ~3) : 0));
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -371,6 +462,19 @@ __global__ void __launch_bounds__(kUmmaThreads, 1) linear_umma_kernel(const __gr
             const int acc = it & 1;
             const long long row0 = ((long long)blockIdx.x + (long long)it * gridDim.x) * kUmmaRows + quarter * 32;
             const int nrows = M - row0 < 32 ? (int)(M - row0) : 32;  // may be <= 0 in the last tile
+            if constexpr (kParts > 0) {
+                const int rows_here = M - (row0 - quarter * 32) < kUmmaRows ? (int)(M - (row0 - quarter * 32)) : kUmmaRows;
+                for (int q = (warp * 32 + lane) * 32; q < rows_here * args.parts.C * kParts; q += kUmmaEpilogueWarps * 32 * 32)
+                    asm volatile("prefetch.global.L2 [%0];" ::"l"(args.parts.vgrad + (row0 - quarter * 32) * args.parts.C * kParts + q));
+                if (!(ok = umma_wait(&sh->acc_full[acc], (it >> 1) & 1, &sh->abort))) break;
+                tc_fence_after();
+                umma_store_parts<kParts>(args.parts, tlane + acc * acc_stride, epi + warp * 32 * kUmmaPartPitch * (2 + kParts), row0, nrows, first_block, lane, [&]() {
+                    tc_fence_before();
+                    __syncwarp();
+                    if (lane == 0) mbar_arrive(&sh->acc_empty[acc]);
+                });
+                continue;
+            }
             if constexpr (MODE == kUmmaStep) umma_prefetch_step(args, (long long)blockIdx.x + (long long)it * gridDim.x, warp * 32 + lane);
 #pragma unroll 1
             for (int pass = fuse ? 0 : 1; pass < (fuse ? 3 : 2); ++pass) {
@@ -578,10 +682,20 @@ __global__ void umma_wait_selftest_kernel(unsigned long long limit_ns, int *resu
     if ((threadIdx.x & 31) == 0) result[warp] = completed ? 0 : (warp == 0 || by_flag ? 1 : 2);
 }
 
+static void (*umma_kernel(int mode))(UmmaArgs) {
+    switch (mode) {
+        case kUmmaStep: return linear_umma_kernel<kUmmaStep>;
+        case kUmmaTwoLayers: return linear_umma_kernel<kUmmaTwoLayers>;
+        case kUmmaParts2: return linear_umma_kernel<kUmmaParts2>;
+        case kUmmaParts3: return linear_umma_kernel<kUmmaParts3>;
+        default: return linear_umma_kernel<kUmmaOneLayer>;
+    }
+}
+
 // Per-device set-up done once: the address of the status word and the shared-memory limit of the kernel.
 struct UmmaDevice {
     unsigned *status = nullptr;
-    int smem_limit[3] = {0, 0, 0};  // per kernel instantiation
+    int smem_limit[kUmmaModes] = {};  // per kernel instantiation
 };
 static std::mutex g_umma_mutex;
 static UmmaDevice g_umma_device[64];
@@ -597,7 +711,7 @@ static int umma_device_setup(int smem, int mode, unsigned **status) {
         if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "npa_linear_tcgen05: status word: %s", cudaGetErrorString(e));
     }
     if (smem > d.smem_limit[mode]) {
-        const auto kernel = mode == kUmmaStep ? linear_umma_kernel<kUmmaStep> : mode == kUmmaTwoLayers ? linear_umma_kernel<kUmmaTwoLayers> : linear_umma_kernel<kUmmaOneLayer>;
+        const auto kernel = umma_kernel(mode);
         e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
         if (e != cudaSuccess) return fail(NPA_ERR_CUDA, "npa_linear_tcgen05: raising the shared-memory limit: %s", cudaGetErrorString(e));
         d.smem_limit[mode] = smem;
@@ -626,10 +740,11 @@ static int launch_images(const ImageJobs &jobs, cudaStream_t st) {
 // The images of both layers, and of W1 as the backward wants it.
 static int mlp_images(const char *me, const float *W1, const float *W2, int in_dim, int out_dim, int64_t w1_stride_out, int64_t w1_stride_in,
                       int64_t w2_stride_out, int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes,
-                      ImageJobs *jobs) {
-    if (dz_image && ((uintptr_t)dz_image % 16 || dz_image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim)))
+                      ImageJobs *jobs, int features = 0, int dim = 0) {
+    const int dz_columns = features > 0 ? StepColumns::total(features, dim) : in_dim;
+    if (dz_image && ((uintptr_t)dz_image % 16 || dz_image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, dz_columns)))
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: dz_image must be 16-byte aligned and hold %lld bytes", me,
-                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, in_dim));
+                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, dz_columns));
     if (in_dim <= 0 || out_dim <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows, in_dim and out_dim must be positive", me);
     if (in_dim > 1024 || out_dim > 64)
         return fail(NPA_ERR_UNSUPPORTED, "%s: supports in_dim <= 1024 and out_dim <= 64 (hidden width 128), got %d and %d", me, in_dim, out_dim);
@@ -641,8 +756,46 @@ static int mlp_images(const char *me, const float *W1, const float *W2, int in_d
     void *w2 = (char *)scratch + npa_linear_tcgen05_scratch_bytes(in_dim, kUmmaRows);
     *jobs = {{image_job(W1, w1_stride_out, w1_stride_in, in_dim, kUmmaRows, scratch),
               image_job(W2, w2_stride_out, w2_stride_in, kUmmaRows, out_dim, w2)}, 2};
-    if (dz_image) jobs->job[jobs->count++] = image_job(W1, w1_stride_in, w1_stride_out, kUmmaRows, in_dim, dz_image);
+    if (dz_image) {
+        ImageJob j = image_job(W1, w1_stride_in, w1_stride_out, kUmmaRows, dz_columns, dz_image);
+        j.features = features;
+        j.dim = dim;
+        jobs->job[jobs->count++] = j;
+    }
     return NPA_OK;
+}
+
+// Stages and shared memory of a single layer whose A, K and N are set.
+static int plan_one_layer(UmmaArgs &a, int mode, size_t *smem) {
+    a.Np = umma_round16(a.N);
+    a.nchunks = umma_chunks(a.K);
+    a.last_ksteps = (a.K - (a.nchunks - 1) * kUmmaChunk + 7) / 8;
+    a.stage_bytes = 2 * kUmmaTileABytes + 2 * a.Np * 128;
+    const int fixed = 1024 + umma_epilogue_floats(mode) * 4 + (int)sizeof(UmmaShared);
+    a.stages = (227 * 1024 - fixed) / a.stage_bytes;
+    if (a.stages > kUmmaMaxStages) a.stages = kUmmaMaxStages;
+    if (a.stages < 2) return fail(NPA_ERR_UNSUPPORTED, "npa_linear_tcgen05: out_dim %d leaves room for fewer than two stages", a.N);
+    *smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
+    return umma_device_setup((int)*smem, mode, &a.status);
+}
+static int launch_one_layer(const UmmaArgs &a, int mode, size_t smem, cudaStream_t st) {
+    const long long tiles = (a.M + kUmmaRows - 1) / kUmmaRows;
+    launch_early(umma_kernel(mode), (int)(tiles < 148 ? tiles : 148), kUmmaThreads, smem, st, a);
+    return check_launch("linear_umma_kernel");
+}
+
+int launch_step_rows(const StepRows &rows, const float *dh, long long particles, const void *image, int64_t image_bytes, cudaStream_t st) {
+    const int columns = StepColumns::total(rows.C, rows.dim);
+    if (!dh || !image || !rows.vgrad || (uintptr_t)dh % 4 || ((uintptr_t)image | (uintptr_t)rows.vgrad | (uintptr_t)rows.direct | (uintptr_t)rows.rows) % 16 ||
+        image_bytes < npa_linear_tcgen05_scratch_bytes(kUmmaRows, columns))
+        return fail(NPA_ERR_INVALID_ARGUMENT, "step_perceive_backward: dh, vgrad and an image of %lld bytes must be there, 16-byte aligned",
+                    (long long)npa_linear_tcgen05_scratch_bytes(kUmmaRows, columns));
+    UmmaArgs a = {};
+    a.A = dh; a.Wimg = static_cast<const float *>(image); a.M = particles; a.K = kUmmaRows; a.N = columns; a.parts = rows;
+    const int mode = rows.dim == 2 ? kUmmaParts2 : kUmmaParts3;
+    size_t smem = 0;
+    const int rc = plan_one_layer(a, mode, &smem);
+    return rc != NPA_OK ? rc : launch_one_layer(a, mode, smem, st);
 }
 
 }  // namespace npa
@@ -672,26 +825,15 @@ static int linear_tcgen05(const float *A, const float *W, const float *bias, con
                     (long long)npa_linear_tcgen05_scratch_bytes(in_dim, out_dim));
     UmmaArgs a = {};
     a.A = A; a.Wimg = (const float *)scratch; a.bias = bias; a.gate = gate; a.C = C; a.M = rows; a.K = in_dim; a.N = out_dim;
-    a.Np = umma_round16(out_dim);
-    a.nchunks = umma_chunks(in_dim);
-    a.last_ksteps = (in_dim - (a.nchunks - 1) * kUmmaChunk + 7) / 8;
-    a.stage_bytes = 2 * kUmmaTileABytes + 2 * a.Np * 128;
     a.relu = relu;
-    const int fixed = 1024 + kUmmaEpiFloats * 4 + (int)sizeof(UmmaShared);
-    a.stages = (227 * 1024 - fixed) / a.stage_bytes;
-    if (a.stages > kUmmaMaxStages) a.stages = kUmmaMaxStages;
-    if (a.stages < 2) return fail(NPA_ERR_UNSUPPORTED, "npa_linear_tcgen05: out_dim %d leaves room for fewer than two stages", out_dim);
-    const size_t smem = (size_t)fixed + (size_t)a.stages * a.stage_bytes;
-    int rc = umma_device_setup((int)smem, kUmmaOneLayer, &a.status);
+    size_t smem = 0;
+    int rc = plan_one_layer(a, kUmmaOneLayer, &smem);
     if (rc != NPA_OK) return rc;
     if (W) {
         ImageJobs jobs = {{image_job(W, w_stride_out, w_stride_in, in_dim, out_dim, scratch)}, 1};
         if ((rc = launch_images(jobs, (cudaStream_t)stream)) != NPA_OK) return rc;
     }
-    const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
-    const int ctas = (int)(tiles < 148 ? tiles : 148);
-    launch_early(linear_umma_kernel<kUmmaOneLayer>, ctas, kUmmaThreads, smem, (cudaStream_t)stream, a);
-    return check_launch("linear_umma_kernel");
+    return launch_one_layer(a, kUmmaOneLayer, smem, (cudaStream_t)stream);
 }
 
 int npa_linear_tcgen05(const float *A, const float *W, const float *bias, const float *gate, float *C, int64_t rows,
@@ -739,6 +881,29 @@ int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const f
     return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream);
 }
 
+int64_t npa_step_rows_image_bytes(const npa_grid *gd, int32_t channels) {
+    Geom g;
+    const int rc = make_geom(gd, &g);
+    if (rc != NPA_OK) return rc;
+    return step_rows_cover(channels) ? npa_linear_tcgen05_scratch_bytes(kUmmaRows, StepColumns::total(channels, g.dim)) : 0;
+}
+
+int npa_bin_particles_step_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
+                                  float *s_out, const float *W1, const float *W2, int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out,
+                                  int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *rows_image, int64_t rows_image_bytes, void *stream) {
+    const char *me = "npa_bin_particles_step_images";
+    Geom g;
+    int rc = make_geom(grid, &g);
+    if (rc != NPA_OK) return rc;
+    if (!rows_image) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows_image must be non-NULL", me);
+    if (!step_rows_cover(channels)) return fail(NPA_ERR_UNSUPPORTED, "%s: supports multiples of four up to 32 features, got %d", me, channels);
+    ImageJobs jobs;
+    rc = mlp_images(me, W1, W2, 2 * channels + channels * g.dim + g.dim, g.dim + channels, w1_stride_out, w1_stride_in, w2_stride_out, w2_stride_in, scratch,
+                    scratch_bytes, rows_image, rows_image_bytes, &jobs, channels, g.dim);
+    if (rc != NPA_OK) return rc;
+    return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream);
+}
+
 // step != NULL: with the Euler update of D-dimensional positions on the geometry g.
 static int mlp_forward(const char *me, const float *z, const float *b1, float *h, float *y, int64_t rows, int32_t in_dim, int32_t out_dim,
                        const void *scratch, int64_t scratch_bytes, const StepArgs *step, const Geom *g, cudaStream_t st) {
@@ -776,7 +941,7 @@ static int mlp_forward(const char *me, const float *z, const float *b1, float *h
     if (rc != NPA_OK) return rc;
     const long long tiles = (rows + kUmmaRows - 1) / kUmmaRows;
     const int ctas = (int)(tiles < 148 ? tiles : 148);
-    launch_early(step ? linear_umma_kernel<kUmmaStep> : linear_umma_kernel<kUmmaTwoLayers>, ctas, kUmmaThreads, smem, st, a);
+    launch_early(umma_kernel(mode), ctas, kUmmaThreads, smem, st, a);
     return check_launch("linear_umma_kernel (two layers)");
 }
 

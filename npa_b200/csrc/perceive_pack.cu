@@ -8,30 +8,11 @@
 // re-read the [B,N,C,D] gradient tensor.  Here sweep 2 applies that per-particle epilogue while
 // the sums are still in registers (feature_kernels.cuh, F_PACK) and writes z once; backward turns
 // dL/dz into the upstream gradients of blur / gradient / density gradient with one elementwise
-// kernel and then runs the ordinary fused backward sweeps.
-#include "ops.cuh"
+// kernel and then runs the ordinary fused backward sweeps.  (In a step whose positions want no gradient
+// the product that makes dL/dz writes them: launch_step_rows.)
+#include "perceive_backward.cuh"
 
 namespace npa {
-
-// Gradient of  f(w) = log(1 + |w|) w / |w|  (symmetric Jacobian) applied to g, times `scale`;
-// without log-normalisation f is the identity.
-template <int D>
-__device__ inline void log_normalize_backward(const float *w, const float *gin, int log_norm, float scale, float *gout) {
-    if (!log_norm) {
-#pragma unroll
-        for (int d = 0; d < D; ++d) gout[d] = scale * gin[d];
-        return;
-    }
-    float n2 = w[0] * w[0] + w[1] * w[1];
-    float wg = w[0] * gin[0] + w[1] * gin[1];
-    if (D == 3) { n2 += w[2] * w[2]; wg += w[2] * gin[2]; }
-    const float n = sqrtf(n2);
-    const float l = logf(1.0f + n);
-    const float a = l / fmaxf(n, 1e-12f);
-    const float b = n > 1e-12f ? (1.0f / ((1.0f + n) * n2) - l / (n2 * n)) : 0.0f;
-#pragma unroll
-    for (int d = 0; d < D; ++d) gout[d] = scale * (a * gin[d] + b * wg * w[d]);
-}
 
 // One thread per (particle, feature): dL/dz -> dL/dblur, dL/dgrad; the thread of feature 0 also
 // handles the density-gradient part.  ROWS: the rows the backward over neighbour lists reads, blur and the D
@@ -209,12 +190,12 @@ static int features_backward_lists(const npa_grid *gd, int32_t channels, const f
                                    const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
                                    int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
                                    int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, bool binned,
-                                   void *stream) {
-    const char *me = "perceive_features_backward_lists";
+                                   void *stream, const float *dh = nullptr, const void *image = nullptr, int64_t image_bytes = 0) {
+    const char *me = dh ? "step_perceive_backward" : "perceive_features_backward_lists";
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
-    if (!x_bin || !s_bin || !rho || !rho_grad || !vgrad || !dL_dz || !scratch || !bin_offsets || !pair_cache)
+    if (!x_bin || !s_bin || !rho || (!rho_grad && !dh) || !vgrad || (!dL_dz && !dh) || !scratch || !bin_offsets || !pair_cache)
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: a required pointer is NULL", me);
     if (channels <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: channels must be positive", me);
     if (((uintptr_t)x_bin | (uintptr_t)grad_x) % (g.dim == 2 ? 8 : 16) || ((uintptr_t)scratch | (uintptr_t)packed) % 16)
@@ -232,7 +213,12 @@ static int features_backward_lists(const npa_grid *gd, int32_t channels, const f
     float *rows = static_cast<float *>(scratch), *g_dg = rows + n * pitch;
     float4 *pg = reinterpret_cast<float4 *>(g_dg + n * 4);
     const unsigned blocks = (unsigned)((n * cp + 255) / 256);
-    if (g.dim == 2)
+    // dh: dL/dz has not been formed; its product's epilogue writes the rows (and the features' own part where the density gradient's
+    // upstream and the records would lie)
+    if (dh) {
+        const StepRows out = {vgrad, g_dg, rows, pitch, channels, g.dim, coef, log_norm_grad};
+        if ((rc = launch_step_rows(out, dh, n, image, image_bytes, st)) != NPA_OK) return rc;
+    } else if (g.dim == 2)
         launch_early(pack_backward_kernel<2, true>, blocks, 256, 0, st, dL_dz, vgrad, rho_grad, rows, nullptr, grad_x ? g_dg : nullptr, n, channels, pitch, coef,
                                                               dg_scale, log_norm_grad, log_norm_dg);
     else
@@ -242,7 +228,7 @@ static int features_backward_lists(const npa_grid *gd, int32_t channels, const f
     FeatureListBwdArgs a = {};
     a.x = x_bin; a.mass = mass; a.rho = rho; a.s = s_bin; a.pv = reinterpret_cast<const float4 *>(packed);
     a.gb = rows; a.gg = rows + cp; a.gb_pitch = a.gg_pitch = pitch; a.cp = cp;
-    a.direct = dL_dz; a.direct_pitch = 2 * channels + channels * g.dim + g.dim;  // the features enter z unchanged as its first columns
+    a.direct = dh ? g_dg : dL_dz; a.direct_pitch = dh ? channels : 2 * channels + channels * g.dim + g.dim;  // the features enter z unchanged as its first columns
     a.add = grad_s_add;
     a.g_dg = grad_x ? g_dg : nullptr;
     a.grad_x = grad_x; a.grad_s = grad_s; a.pg = grad_x ? pg : nullptr; a.C = channels;
@@ -273,6 +259,26 @@ int npa_perceive_features_backward_binned(const npa_grid *gd, int32_t channels, 
     const char *me = "perceive_features_backward_lists";
     return features_backward_lists(gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
                                    scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, true, stream);
+}
+
+int64_t npa_step_perceive_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
+    const int64_t bytes = npa_lists_backward_scratch_bytes(gd, channels);
+    return bytes < 0 ? bytes : bytes + (int64_t)gd->batch * gd->particles * channels * 4;
+}
+
+int npa_step_perceive_backward(const npa_grid *gd, int32_t channels, const float *dh, const void *rows_image, int64_t rows_image_bytes,
+                               const float *x_bin, const float *s_bin, const float *rho, const float *vgrad, const float *packed, float coef,
+                               int32_t log_norm_grad, const float *grad_s_add, float *grad_s, void *scratch, int64_t scratch_bytes,
+                               const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
+    const char *me = "step_perceive_backward";
+    if (!step_rows_cover(channels)) return fail(NPA_ERR_UNSUPPORTED, "%s: supports multiples of four up to 32 features, got %d", me, channels);
+    if (!dh || !rows_image || !grad_s) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: a required pointer is NULL", me);
+    const int64_t need = npa_step_perceive_backward_scratch_bytes(gd, channels);
+    if (need < 0) return (int)need;
+    if (scratch_bytes < need)
+        return fail(NPA_ERR_SCRATCH_TOO_SMALL, "%s: scratch holds %lld bytes, %lld needed", me, (long long)scratch_bytes, (long long)need);
+    return features_backward_lists(gd, channels, x_bin, nullptr, s_bin, rho, nullptr, vgrad, packed, nullptr, coef, 0.f, log_norm_grad, 0, grad_s_add, nullptr,
+                                   grad_s, scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, true, stream, dh, rows_image, rows_image_bytes);
 }
 
 int npa_perceive_features_backward(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,

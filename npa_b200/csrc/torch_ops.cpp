@@ -733,6 +733,7 @@ struct EulerNode : Node {
     int64_t C, columns, dz_bytes, slab_floats, y_pitch;  // y: rows that begin with the raw displacements
     float coef, dg_scale, alpha, dt, below;
     bool ln_grad, ln_dg, stop_pos, stop_state;
+    bool rows;  // the image of W1 is in the order of npa_step_perceive_backward
 
     variable_list apply(variable_list &&g) override {
         const Tensor w1 = w1_.unpack(), w2 = w2_.unpack(), slab = solid(slab_.unpack()), mask = mask_.unpack();  // raise when the graph was released
@@ -752,10 +753,10 @@ struct EulerNode : Node {
         const bool nx = should_compute_output(0), ns = should_compute_output(1);
         const bool n1 = should_compute_output(2), nb = should_compute_output(3), n2 = should_compute_output(4);
         const bool back_x = nx && !stop_pos, back_s = ns && !stop_state, back = back_x || back_s, weights = n1 || nb || n2;
-        const int64_t work_bytes = back ? npa_lists_backward_scratch_bytes(gd, (int)C) : 0;
+        const int64_t work_bytes = !back ? 0 : rows ? npa_step_perceive_backward_scratch_bytes(gd, (int)C) : npa_lists_backward_scratch_bytes(gd, (int)C);
         if (work_bytes < 0) check_status((int)work_bytes);
         Slab l;
-        const int64_t o_gy = l.add(m * o), o_dh = l.add(back || weights ? m * kHidden : 0), o_gz = l.add(back ? m * k : 0),
+        const int64_t o_gy = l.add(m * o), o_dh = l.add(back || weights ? m * kHidden : 0), o_gz = l.add(back && !rows ? m * k : 0),
                       o_work = l.add(work_bytes / 4), o_gs = l.add(back_s ? m * C : 0),
                       o_scratch = l.add(weights ? weight_grad_scratch_floats(m, k, o) : 0);
         Tensor temporary = l.make(w1);
@@ -770,10 +771,13 @@ struct EulerNode : Node {
         Tensor gx_bin = gx_new, none;
         const float *gs_bin = fptr(gs_new);
         if (back) {
-            check_status(npa_linear_tcgen05_prepared(dh, dz_image, dz_bytes, gz, m, kHidden, (int)k, st));
+            if (!rows) check_status(npa_linear_tcgen05_prepared(dh, dz_image, dz_bytes, gz, m, kHidden, (int)k, st));
             Tensor gxp = back_x ? floats(w1, {gr.B, gr.N, gr.P}) : Tensor();
             float *gsp = back_s ? t + o_gs : nullptr;
-            if (npa_tile_enabled(1)) {
+            if (rows) {  // (the positions want none)
+                check_status(npa_step_perceive_backward(gd, (int)C, dh, dz_image, dz_bytes, x_bin, s_bin, rho, vgrad, packed, coef, ln_grad, fptr(gs_new), gsp,
+                                                        t + o_work, work_bytes, iptr(offs), pairs, (int)columns, st));
+            } else if (npa_tile_enabled(1)) {
                 Tensor gsf = floats(w1, {gr.B, gr.N, C}), work = floats(w1, {m * (C + 1) * (1 + gr.D)});
                 float *gb = fmut(work), *gg = gb + m * C, *g_dg = gg + m * C * gr.D, *g_rho = g_dg + m * gr.D;
                 check_status(npa_perceive_features_backward(gd, (int)C, x_bin, nullptr, s_bin, rho, rho_grad, vgrad, gz, coef, dg_scale, ln_grad, ln_dg,
@@ -824,7 +828,9 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     const bool back = record && ((wants_grad(x) && !stop_pos) || (wants_grad(s) && !stop_state));  // a backward reaches the perception
     Tensor perm = ints(x, {g.B, g.N}), offs = ints(x, {g.B * g.cells + 1}), info = ints(x, {g.max_blocks, 4});
     grid->bin(x, perm, offs, info, st);
-    const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), dz_bytes = back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
+    const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), rows_bytes = back && !npa_tile_enabled(1) && !(wants_grad(x) && !stop_pos) ? npa_step_rows_image_bytes(&g.g, (int)C) : 0;
+    const bool rows = rows_bytes > 0;  // the backward takes dL/dz apart as it forms it
+    const int64_t dz_bytes = rows ? rows_bytes : back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
     const bool in_mlp = C % 4 == 0 && C <= 32;  // the update in the MLP's epilogue, which of y keeps only what the backward reads
     Slab l;
     const int64_t o_x = l.add(m * g.P), o_s = l.add(m * C), o_rho = l.add(m), o_dg = l.add(m * D), o_z = l.add(m * k), o_v = l.add(back ? m * C * D : 0),
@@ -834,8 +840,12 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     float *t = fmut(slab), *x_bin = t + o_x, *s_bin = t + o_s, *rho = t + o_rho, *rho_grad = t + o_dg, *z = t + o_z, *packed = t + o_packed,
           *y = t + o_y, *vgrad = back ? t + o_v : nullptr, *h = record ? t + o_h : nullptr, *dz_image = dz_bytes ? t + o_dz : nullptr;
     int32_t *pairs = reinterpret_cast<int32_t *>(t + o_pairs);
-    check_status(npa_bin_particles_mlp_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), (int)k, (int)o, w1.stride(0),
-                                              w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
+    if (rows)
+        check_status(npa_bin_particles_step_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), w1.stride(0), w1.stride(1),
+                                                   w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
+    else
+        check_status(npa_bin_particles_mlp_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), (int)k, (int)o, w1.stride(0),
+                                                  w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
     check_status(npa_perceive_features_forward_lists(&g.g, (int)C, x_bin, nullptr, s_bin, (float)coef, (float)dg_scale, (float)inv_tol, ln_grad, ln_dg,
                                                      rho, rho_grad, z, vgrad, packed, iptr(offs), iptr(info), pairs, (int)columns, st));
     Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();
@@ -856,7 +866,7 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
         n->o_dz = o_dz; n->o_pairs = o_pairs; n->slab_floats = l.floats; n->y_pitch = in_mlp ? g.P : o; n->C = C; n->columns = columns; n->dz_bytes = dz_bytes;
         n->w1_ = saved(w1); n->w2_ = saved(w2);
         n->coef = (float)coef; n->dg_scale = (float)dg_scale; n->alpha = (float)alpha; n->dt = (float)dt; n->below = (float)update_prob;
-        n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state;
+        n->ln_grad = ln_grad; n->ln_dg = ln_dg; n->stop_pos = stop_pos; n->stop_state = stop_state; n->rows = rows;
         torch::autograd::set_history(xo, n);
         torch::autograd::set_history(so, n);
     }

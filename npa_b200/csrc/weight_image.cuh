@@ -16,7 +16,19 @@ struct ImageJob {
     long long stride_n, stride_k;
     int K, N, Np, nchunks;
     float *img;
+    int features, dim;  // > 0: rows n in the order of StepColumns (below)
     __host__ __device__ int total() const { return nchunks * Np * kImageChunk; }
+};
+// The columns of z in the order in which the gradient of a step wants them: the features themselves, their blur, then axis by axis the
+// gradient, each section rounded up to 16 columns; the density gradient's columns are left out (nothing of a step reads them).
+struct StepColumns {
+    __host__ __device__ static int section(int features) { return (features + 15) & ~15; }
+    __host__ __device__ static int total(int features, int dim) { return (2 + dim) * section(features); }
+    // column of z, or -1 for padding
+    __host__ __device__ static int column(int n, int features, int dim) {
+        const int sec = n / section(features), f = n - sec * section(features);
+        return f >= features ? -1 : sec < 2 ? sec * features + f : 2 * features + f * dim + sec - 2;
+    }
 };
 constexpr int kImageJobs = 3;
 struct ImageJobs {
@@ -38,7 +50,8 @@ __device__ inline void write_image_element(const ImageJobs &jobs, int at) {
             const int Np = j.Np, c = at / (Np * kImageChunk), rem = at - c * Np * kImageChunk;
             const int n = rem / kImageChunk, kk = rem - n * kImageChunk;
             const int k = c * kImageChunk + kk;
-            const float v = (n < j.N && k < j.K) ? __ldg(j.W + n * j.stride_n + k * j.stride_k) : 0.f;
+            const int row = j.features > 0 ? StepColumns::column(n, j.features, j.dim) : n;
+            const float v = (n < j.N && row >= 0 && k < j.K) ? __ldg(j.W + row * j.stride_n + k * j.stride_k) : 0.f;
             const float head = __uint_as_float(tf32_head_bits(v));
             float *chunk = j.img + (size_t)c * 2 * Np * kImageChunk;
             const int to = umma_swizzled(n, kk);

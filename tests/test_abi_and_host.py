@@ -340,3 +340,37 @@ def test_move_copy_and_image_entries_reject_bad_arguments_before_any_launch():
     assert two(nbytes=need - 1) == n.NPA_ERR_INVALID_ARGUMENT and two(scratch=odd) == n.NPA_ERR_INVALID_ARGUMENT
     for bad in (dict(rows=0), dict(k=0), dict(o=0), dict(z=null), dict(y=null), dict(scratch=null), dict(z=ctypes.c_void_p((1 << 20) + 2))):
         assert two(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
+
+
+def test_step_rows_entries_reject_bad_arguments_before_any_launch():
+    """The backward of a step without dL/dz in memory: refusals come from the host, with addresses that are never dereferenced."""
+    from npa_b200 import _native as n
+    lib = n.lib
+    buf, odd, null, big = ctypes.c_void_p(1 << 20), ctypes.c_void_p((1 << 20) + 4), ctypes.c_void_p(0), 1 << 40
+    for dim in (2, 3):
+        g = n.make_grid(dim, "clamped", "grid", (8,) * dim, 0.1, 1, 8, 32)
+        ref = ctypes.byref(g)
+        for C in (1, 2, 13, 30, 36, 128):
+            assert lib.npa_step_rows_image_bytes(ref, C) == 0
+        for C in (4, 12, 16, 20, 32):
+            section = (C + 15) // 16 * 16
+            assert lib.npa_step_rows_image_bytes(ref, C) == lib.npa_linear_tcgen05_scratch_bytes(128, (2 + dim) * section)
+            assert lib.npa_step_perceive_backward_scratch_bytes(ref, C) == lib.npa_lists_backward_scratch_bytes(ref, C) + 8 * C * 4
+        need = lib.npa_mlp_forward_tcgen05_scratch_bytes(32 + 17 * dim, 16 + dim)
+        size, work = lib.npa_step_rows_image_bytes(ref, 16), lib.npa_step_perceive_backward_scratch_bytes(ref, 16)
+
+        def images(C=16, x=buf, w1=buf, nbytes=need, image=buf, image_bytes=size):
+            return lib.npa_bin_particles_step_images(ref, C, x, buf, buf, buf, buf, w1, buf, 82, 1, 128, 1, buf, nbytes, image, image_bytes, null)
+
+        def backward(C=16, dh=buf, image=buf, image_bytes=size, x=buf, v=buf, out=buf, scratch=buf, nbytes=work, stride=128):
+            return lib.npa_step_perceive_backward(ref, C, dh, image, image_bytes, x, buf, buf, v, buf, 1.0, 1, null, out, scratch, nbytes, buf, buf, stride, null)
+
+        assert images(C=13) == n.NPA_ERR_UNSUPPORTED and images(C=36) == n.NPA_ERR_UNSUPPORTED
+        for bad in (dict(image=null), dict(image=odd), dict(image_bytes=size - 1), dict(nbytes=need - 1), dict(w1=null), dict(x=null)):
+            assert images(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
+        assert backward(C=13) == n.NPA_ERR_UNSUPPORTED and backward(C=36) == n.NPA_ERR_UNSUPPORTED
+        assert backward(nbytes=work - 1) == n.NPA_ERR_SCRATCH_TOO_SMALL
+        for bad in (dict(dh=null), dict(image=null), dict(image=odd), dict(image_bytes=size - 1), dict(v=null), dict(v=odd), dict(out=null), dict(scratch=null),
+                    dict(scratch=odd), dict(x=null), dict(x=odd), dict(stride=1), dict(stride=514)):
+            assert backward(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
+    assert lib.npa_step_rows_image_bytes(ctypes.byref(n.make_grid(2, "clamped", "grid", (8, 8), 0.0, 1, 8, 32)), 16) < 0

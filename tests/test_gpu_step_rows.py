@@ -1,0 +1,63 @@
+"""dL/dz of a step taken apart as it leaves the tensor cores, against the product and the rows made one after the other."""
+import ctypes
+
+import pytest
+import torch
+
+from test_gpu_dense_backward import Call, _positions
+
+pytestmark = pytest.mark.gpu
+
+
+def _images(call, W1, W2, rows):
+    """The image of W1 for the backward, in the order of the rows or in W1's own, made by the reorder's launch."""
+    n, p, C, D = call.n, call.n.ptr, call.C, call.dim
+    K, O = 2 * C + C * D + D, D + C
+    nbytes = n.lib.npa_mlp_forward_tcgen05_scratch_bytes(K, O)
+    size = n.lib.npa_step_rows_image_bytes(ctypes.byref(call.gd), C) if rows else n.lib.npa_linear_tcgen05_scratch_bytes(128, K)
+    work, image = torch.empty(nbytes // 4, device="cuda"), torch.full((size // 4,), float("nan"), device="cuda")
+    xo, so = torch.empty_like(call.x), torch.empty_like(call.s)
+    head = (ctypes.byref(call.gd), C, p(call.x), p(call.s), p(call.snap.permutation), p(xo), p(so), p(W1), p(W2))
+    tail = (W1.stride(0), W1.stride(1), W2.stride(0), W2.stride(1), p(work), nbytes, p(image), size, call.st)
+    n.check(n.lib.npa_bin_particles_step_images(*head, *tail) if rows else n.lib.npa_bin_particles_mlp_images(*head, K, O, *tail))
+    return image, size
+
+
+# tiles of 128 rows: one row, one short of a tile, one more, a full round of 148 tiles and beyond; sections of 16 columns filled or not
+@pytest.mark.parametrize("dim,boundary,B,N,C", [(2, "clamped", 1, 1, 16), (2, "periodic", 1, 127, 12), (2, "clamped", 3, 43, 20), (2, "clamped", 2, 9600, 32),
+                                                (3, "clamped", 1, 129, 28), (3, "periodic", 2, 64, 24), (3, "clamped", 1, 19073, 16), (3, "clamped", 1, 2000, 12),
+                                                (2, "clamped", 1, 300, 4), (3, "periodic", 1, 130, 8),
+                                                (3, "clamped", 2, 10001, 32)])
+@pytest.mark.parametrize("log_norm", [0, 1])
+def test_rows_as_the_separate_kernels_make_them(dim, boundary, B, N, C, log_norm):
+    """The same products and the same expression for each element: equal bits, also of rows that begin in another system."""
+    torch.manual_seed(N + C)
+    eps = 0.05 if dim == 2 else 0.1
+    cells = max(4, round((N / 8) ** (1 / dim)))
+    call = Call(_positions(dim, B, N, cells * eps), cells, eps, boundary, C)
+    n, p, D = call.n, call.n.ptr, dim
+    K = 2 * C + C * D + D
+    W1, W2 = torch.randn(128, K, device="cuda"), torch.randn(D + C, 128, device="cuda")
+    if log_norm:
+        W1 = W1.t().contiguous().t()                        # strides of a transposed weight
+    dh = torch.randn(B, N, 128, device="cuda") * (torch.rand(B, N, 128, device="cuda") < 0.5)
+    call.v[0, 0] = 0.0                                      # a gradient of zero: the normalisation's own case
+    plain, plain_bytes = _images(call, W1, W2, False)
+    dz = torch.empty(B, N, K, device="cuda")
+    n.check(n.lib.npa_linear_tcgen05_prepared(p(dh), p(plain), plain_bytes, p(dz), B * N, 128, K, call.st))
+    ref = ctypes.byref(call.gd)
+    nbytes = n.lib.npa_lists_backward_scratch_bytes(ref, C)
+    work, want = torch.empty(nbytes // 4, device="cuda"), torch.empty(B, N, C, device="cuda")
+    n.check(n.lib.npa_perceive_features_backward_binned(ref, C, p(call.x), None, p(call.s), p(call.rho), p(call.dg), p(call.v), p(call.packed), p(dz), 0.8, 0.3,
+                                                        log_norm, 1, p(call.add), None, p(want), p(work), nbytes, p(call.snap.bin_offsets), p(call.pairs), call.K,
+                                                        call.st))
+    image, image_bytes = _images(call, W1, W2, True)
+    nbytes = n.lib.npa_step_perceive_backward_scratch_bytes(ref, C)
+    work, got = torch.full((nbytes // 4 + 64,), float("nan"), device="cuda"), torch.full((B, N, C), float("nan"), device="cuda")
+    n.check(n.lib.npa_step_perceive_backward(ref, C, p(dh), p(image), image_bytes, p(call.x), p(call.s), p(call.rho), p(call.v), p(call.packed), 0.8, log_norm,
+                                             p(call.add), p(got), p(work), nbytes, p(call.snap.bin_offsets), p(call.pairs), call.K, call.st))
+    assert torch.equal(got, want)
+    assert bool(torch.isnan(work[nbytes // 4:]).all())      # nothing beyond the scratch that was asked for
+    status = ctypes.c_uint32(1)
+    n.check(n.lib.npa_linear_tcgen05_status(ctypes.byref(status), 0))
+    assert status.value == 0
