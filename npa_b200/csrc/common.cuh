@@ -59,7 +59,8 @@ int check_launch(const char *what);
 //    its place early finds the SM divided between L1 and shared memory as the kernel before wanted it;
 //  * the reduction of the weight gradients (3D step of 262,144 particles 1,544 -> 1,552 us, its kernel and the one behind it together: it
 //    takes room beside the gradient kernel's CTAs that the next kernel would have had);
-//  * the hidden gradient of the MLP (3D step 1,615 -> 1,643 us, not explained).
+//  * the hidden gradient of the MLP (3D steps 298 -> 301, 1,428 -> 1,432 us, not explained);
+//  * feature_dense.cu (1,428 -> 1,454, not explained further: its rows come through L1 as well).
 // Plain and not measured otherwise: the searching sweeps of feature_kernels.cuh and scalar_ops.cu, the cell-tile engine, the paths of
 // mlp_gemm.cu and mlp_grad.cu, small conversions.  The density searches, the packed sweep and the sweeps of scalar_list.cu are launched
 // early; they were measured within the chains above only.
