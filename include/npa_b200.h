@@ -605,6 +605,13 @@ int npa_linear_tcgen05_prepared(const float *A, const void *image, int64_t image
  * made by npa_bin_particles_step_images, which is npa_bin_particles_mlp_images otherwise (in_dim = 2C + C D + D, out_dim = D + C).
  * vgrad, rows_image and scratch 16-byte aligned; grad_s [B*N, C] as grad_s_add (may be NULL). */
 int64_t npa_step_rows_image_bytes(const npa_grid *g, int32_t channels);
+/* The beginning of a step: npa_grid_build followed by npa_bin_particles_mlp_images (rows = 0; in_dim = 2C + C D + D, out_dim = D + C) or
+ * npa_bin_particles_step_images (rows = 1), with the work list of several small systems written by the second one's launch.  Arguments as
+ * there; grid_scratch is npa_grid_build's scratch; dz_image may be NULL. */
+int npa_step_bin(const npa_grid *g, int32_t channels, const float *x, const float *s, int32_t *permutation, int32_t *bin_offsets,
+                 int32_t *block_info, void *grid_scratch, int64_t grid_scratch_bytes, float *x_out, float *s_out, const float *W1,
+                 const float *W2, int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,
+                 int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, int32_t rows, void *stream);
 int npa_bin_particles_step_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation,
                                   float *x_out, float *s_out, const float *W1, const float *W2, int64_t w1_stride_out,
                                   int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch,

@@ -96,6 +96,7 @@ SIGNATURES = {
                                           ctypes.c_double, _I32, _I32, ctypes.c_double, _P, _P, _P]),
     "npa_rollout_move": (ctypes.c_int, [_P, _P, _P, _P, _P, _I32, ctypes.c_float, _P, _P]),
     "npa_copy_pair": (ctypes.c_int, [_P, _P, _I64, _P, _P, _I64, _P]),
+    "npa_step_bin": (ctypes.c_int, [_P, _I32] + [_P] * 6 + [_I64] + [_P] * 4 + [_I64] * 4 + [_P, _I64, _P, _I64, _I32, _P]),
     "npa_step_rows_image_bytes": (_I64, [_P, _I32]),
     "npa_bin_particles_step_images": (ctypes.c_int, [_P, _I32] + [_P] * 7 + [_I64] * 4 + [_P, _I64, _P, _I64, _P]),
     "npa_step_perceive_backward_scratch_bytes": (_I64, [_P, _I32]),

@@ -477,13 +477,13 @@ static GridBuild grid_build(const Geom &g) {
 
 // Exclusive scan over the CTA's cell table: every thread takes `per` consecutive cells.  Calls emit(cell, count, prefix)
 // in cell order; returns the grand total.  prefix and total count (work items << 32 | particles).
-template <typename Count, typename Emit>
+template <int THREADS = kSmallThreads, typename Count, typename Emit>
 __device__ inline unsigned long long scan_cells(const Geom &g, Count &&count, Emit &&emit) {
     __shared__ unsigned long long tot;
-    const int per = (g.cells + kSmallThreads - 1) / kSmallThreads, c0 = threadIdx.x * per, c1 = min(c0 + per, g.cells);
+    const int per = (g.cells + THREADS - 1) / THREADS, c0 = threadIdx.x * per, c1 = min(c0 + per, g.cells);
     unsigned long long v = 0;
     for (int c = c0; c < c1; ++c) v += pack_cell(count(c), g.mpb);
-    unsigned long long run = block_exclusive<kSmallThreads>(v, tot);
+    unsigned long long run = block_exclusive<THREADS>(v, tot);
     for (int c = c0; c < c1; ++c) {
         const uint32_t n = count(c);
         emit(c, n, run);
@@ -728,26 +728,37 @@ bin_cluster_kernel(const float *__restrict__ x, int32_t *__restrict__ permutatio
     cluster.sync();  // a CTA's shared memory stays until all have read it
 }
 
-// Work list of several small systems: the rows of a system start behind those of the systems before it.
-__global__ void __launch_bounds__(kSmallThreads)
-rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, const uint32_t *__restrict__ rows_of_system, Geom g) {
-    after_previous_kernel();
+// Cells of a system up to which its work list is written beside the reorder, by a block of 256 threads, instead of by a launch of its own with 1,024.
+// Grid build and reorder, launch / beside, us: 8 x 4,096 particles in 2D, 256 cells 12.9 / 9.9, 1,024 13.2 / 11.0, 4,096 16.2 / 16.1; 64 x 512, 64 cells
+// 9.5 / 6.5, 4,096 12.3 / 12.0; 8 x 4,096 in 3D, 4,096 cells 16.5 / 16.6; 300 x 100, 36 cells 13.4 / 9.0.
+constexpr int kRowsBesideCells = 2048;
+
+// Work list of several small systems, a CTA each: the rows of a system start behind those of the systems before it.
+template <int THREADS>
+__device__ inline void write_system_rows(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info,
+                                         const uint32_t *__restrict__ rows_of_system, const Geom &g, int b) {
     __shared__ unsigned long long before_s;
-    const int b = blockIdx.x, tid = threadIdx.x;
+    const int tid = threadIdx.x;
     unsigned long long before = 0, all = 0;  // rows of the systems before this one, rows in all
-    for (int k = tid; k < g.B; k += kSmallThreads) {
+    for (int k = tid; k < g.B; k += THREADS) {
         const uint32_t r = rows_of_system[k];
         all += r;
         if (k < b) before += r;
     }
-    block_exclusive<kSmallThreads>(before | (all << 32), before_s);  // both totals below 2^29
+    block_exclusive<THREADS>(before | (all << 32), before_s);  // both totals below 2^29
     __syncthreads();
     const uint32_t row0 = (uint32_t)before_s, grand = (uint32_t)(before_s >> 32);
     const int32_t *off = bin_offsets + (size_t)b * g.cells;
-    scan_cells(g, [&](int c) { return (uint32_t)(off[c + 1] - off[c]); },
-               [&](int c, uint32_t n, unsigned long long run) { write_rows(block_info, g, b, c, n, row0 + (uint32_t)(run >> 32)); });
-    for (long long r = (long long)grand + (long long)b * kSmallThreads + tid; r < g.max_blocks; r += (long long)g.B * kSmallThreads)
+    scan_cells<THREADS>(g, [&](int c) { return (uint32_t)(off[c + 1] - off[c]); },
+                        [&](int c, uint32_t n, unsigned long long run) { write_rows(block_info, g, b, c, n, row0 + (uint32_t)(run >> 32)); });
+    for (long long r = (long long)grand + (long long)b * THREADS + tid; r < g.max_blocks; r += (long long)g.B * THREADS)
         block_info[r] = make_int4(0, 0, 0, 0);
+}
+
+__global__ void __launch_bounds__(kSmallThreads)
+rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ block_info, const uint32_t *__restrict__ rows_of_system, Geom g) {
+    after_previous_kernel();
+    write_system_rows<kSmallThreads>(bin_offsets, block_info, rows_of_system, g, blockIdx.x);
 }
 
 // ---------------------------------------------------------------------------
@@ -758,8 +769,8 @@ rows_small_kernel(const int32_t *__restrict__ bin_offsets, int4 *__restrict__ bl
 template <int D, bool FORWARD, typename VEC>
 __device__ inline void permute_piece(const float *__restrict__ x, const float *__restrict__ s, const float *__restrict__ m,
                                      const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
-                                     float *__restrict__ mo, int pieces, long long total, int N) {
-    const long long t = (long long)blockIdx.x * 256 + threadIdx.x;
+                                     float *__restrict__ mo, int pieces, long long total, int N, unsigned block) {
+    const long long t = (long long)block * 256 + threadIdx.x;
     if (t >= total) return;
     const long long particle = t / pieces;
     const int piece = (int)(t - particle * pieces);
@@ -789,21 +800,29 @@ permute_kernel(const float *__restrict__ x, const float *__restrict__ s, const f
                const int32_t *__restrict__ perm, float *__restrict__ xo, float *__restrict__ so,
                float *__restrict__ mo, int pieces, long long total, int N) {
     after_previous_kernel();
-    permute_piece<D, FORWARD, VEC>(x, s, m, perm, xo, so, mo, pieces, total, N);
+    permute_piece<D, FORWARD, VEC>(x, s, m, perm, xo, so, mo, pieces, total, N, blockIdx.x);
 }
 
-// The reorder of a step, with the images of the MLP's weights made by blocks behind those of the particles: they have no launch of
-// their own then (2 us of a small step, and 5 us of the host).
+// The reorder of a step, with the images of the MLP's weights made by blocks behind those of the particles, and the work list of several
+// small systems by blocks before them: they have no launch of their own then (2 us of a small step each, and 5 us of the host).
 template <int D, typename VEC>
 __global__ void __launch_bounds__(256)
 permute_images_kernel(const float *__restrict__ x, const float *__restrict__ s, const int32_t *__restrict__ perm, float *__restrict__ xo,
-                      float *__restrict__ so, int pieces, long long total, int N, unsigned blocks, const __grid_constant__ ImageJobs jobs) {
+                      float *__restrict__ so, int pieces, long long total, int N, unsigned blocks, const __grid_constant__ ImageJobs jobs,
+                      const __grid_constant__ RowsJob rest) {
     after_previous_kernel();
-    if (blockIdx.x < blocks) permute_piece<D, true, VEC>(x, s, nullptr, perm, xo, so, nullptr, pieces, total, N);
-    else write_image_element(jobs, (int)(blockIdx.x - blocks) * 256 + threadIdx.x);
+    if (blockIdx.x < (unsigned)rest.systems) {
+        write_system_rows<256>(rest.bin_offsets, rest.block_info, rest.rows_of_system, rest.g, (int)blockIdx.x);
+        return;
+    }
+    const unsigned block = blockIdx.x - rest.systems;
+    if (block < blocks) permute_piece<D, true, VEC>(x, s, nullptr, perm, xo, so, nullptr, pieces, total, N, block);
+    else write_image_element(jobs, (int)(block - blocks) * 256 + threadIdx.x);
 }
 
-// `images`: with those blocks, which only the forward reorder of a step has.
+static unsigned blocks_beside(const ImageJobs &jobs, const RowsJob &rest) { return (unsigned)(jobs.total() + 255) / 256 + (unsigned)rest.systems; }
+
+// `images`: with those blocks (ImageJobs, RowsJob), which only the forward reorder of a step has.
 template <bool FORWARD, typename... Images>
 static int launch_permute(const Geom &g, int C, const float *x, const float *s, const float *m,
                           const int32_t *perm, float *xo, float *so, float *mo, cudaStream_t st, const Images &...images) {
@@ -818,8 +837,8 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
     const int pieces = s ? (vec ? C / 4 : C) : 1;
     const long long total = (long long)g.B * g.N * pieces;
     const unsigned blocks = (unsigned)((total + 255) / 256);
-    if constexpr (sizeof...(Images) == 1) {
-        const unsigned all = blocks + (unsigned)((images.total() + ...) + 255) / 256;
+    if constexpr (sizeof...(Images) == 2) {
+        const unsigned all = blocks + blocks_beside(images...);
 #define NPA_PERMUTE(DD, VEC) \
     launch_early(permute_images_kernel<DD, VEC>, all, 256, 0, st, x, s, perm, xo, so, pieces, total, g.N, blocks, images...)
         if (g.dim == 2) {
@@ -842,10 +861,10 @@ static int launch_permute(const Geom &g, int C, const float *x, const float *s, 
 }
 
 int bin_particles_and_images(const npa_grid *grid, int channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
-                             float *s_out, const ImageJobs &jobs, cudaStream_t stream) {
+                             float *s_out, const ImageJobs &jobs, cudaStream_t stream, const RowsJob &rest) {
     Geom g;
     const int rc = make_geom(grid, &g);
-    return rc != NPA_OK ? rc : launch_permute<true>(g, channels, x, s, nullptr, permutation, x_out, s_out, nullptr, stream, jobs);
+    return rc != NPA_OK ? rc : launch_permute<true>(g, channels, x, s, nullptr, permutation, x_out, s_out, nullptr, stream, jobs, rest);
 }
 
 // ---------------------------------------------------------------------------
@@ -940,6 +959,25 @@ int npa_grid_build_kernels(const npa_grid *gd) {
 
 int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int32_t *bin_offsets,
                    int32_t *block_info, void *scratch, int64_t scratch_bytes, void *stream) {
+    return grid_build_leaving(gd, x, permutation, bin_offsets, block_info, scratch, scratch_bytes, (cudaStream_t)stream, nullptr);
+}
+
+}  // extern "C"
+
+namespace npa {
+
+static int build_rows(const Geom &g, const int32_t *bin_offsets, int32_t *block_info, const uint32_t *rows_of_system, cudaStream_t st, RowsJob *rest) {
+    const RowsJob job = {bin_offsets, reinterpret_cast<int4 *>(block_info), rows_of_system, g, g.B};
+    if (rest && g.cells <= kRowsBesideCells) {
+        *rest = job;
+        return NPA_OK;
+    }
+    launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, job.block_info, rows_of_system, g);
+    return check_launch("rows_small_kernel");
+}
+
+int grid_build_leaving(const npa_grid *gd, const float *x, int32_t *permutation, int32_t *bin_offsets, int32_t *block_info, void *scratch,
+                       int64_t scratch_bytes, cudaStream_t st, RowsJob *rest) {
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
@@ -951,7 +989,6 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
     const size_t need = layout_scratch(g, scratch, &s);
     if (scratch_bytes < (int64_t)need)
         return fail(NPA_ERR_SCRATCH_TOO_SMALL, "npa_grid_build: scratch has %lld bytes, %zu needed", (long long)scratch_bytes, need);
-    cudaStream_t st = (cudaStream_t)stream;
     const GridBuild way = grid_build(g);
     if (way == GridBuild::kCluster) {
         const int ctas = kClusterCtas;
@@ -961,8 +998,7 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
         if ((rc = persistent_ctas(kernel, kClusterThreads, bytes, &unused)) != NPA_OK) return rc;  // shared-memory limit
         launch_cluster(ctas, kernel, g.B * ctas, kClusterThreads, bytes, st, x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         if ((rc = check_launch("bin_cluster_kernel")) != NPA_OK || g.B == 1) return rc;
-        launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
-        return check_launch("rows_small_kernel");
+        return build_rows(g, bin_offsets, block_info, s.counts, st, rest);
     }
     if (way == GridBuild::kSmall) {
         const size_t bytes = small_smem(g);
@@ -975,8 +1011,7 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
             launch_early(bin_small_kernel<3>, g.B, kSmallThreads, bytes, st, x, permutation, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
         }
         if ((rc = check_launch("bin_small_kernel")) != NPA_OK || g.B == 1) return rc;
-        launch_early(rows_small_kernel, g.B, kSmallThreads, 0, st, bin_offsets, reinterpret_cast<int4 *>(block_info), s.counts, g);
-        return check_launch("rows_small_kernel");
+        return build_rows(g, bin_offsets, block_info, s.counts, st, rest);
     }
     const size_t quads = s.zero_bytes / 16;  // (a multiple of 256 bytes)
     const size_t zero_ctas = (quads + kBinThreads - 1) / kBinThreads;
@@ -1018,6 +1053,10 @@ int npa_grid_build(const npa_grid *gd, const float *x, int32_t *permutation, int
                                                                          (int)tgrid.x);
     return check_launch("rank_kernel");
 }
+
+}  // namespace npa
+
+extern "C" {
 
 }  // extern "C"
 

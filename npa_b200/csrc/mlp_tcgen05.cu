@@ -881,6 +881,26 @@ int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const f
     return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream);
 }
 
+int npa_step_bin(const npa_grid *grid, int32_t channels, const float *x, const float *s, int32_t *permutation, int32_t *bin_offsets, int32_t *block_info,
+                 void *grid_scratch, int64_t grid_scratch_bytes, float *x_out, float *s_out, const float *W1, const float *W2, int64_t w1_stride_out,
+                 int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in, void *scratch, int64_t scratch_bytes, void *dz_image,
+                 int64_t dz_image_bytes, int32_t rows, void *stream) {
+    const char *me = "npa_step_bin";
+    Geom g;
+    int rc = make_geom(grid, &g);
+    if (rc != NPA_OK) return rc;
+    if (rows && !step_rows_cover(channels)) return fail(NPA_ERR_UNSUPPORTED, "%s: rows of multiples of four up to 32 features, got %d", me, channels);
+    if (!x || !s || !x_out || !s_out) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: x, s and their outputs must be non-NULL", me);
+    ImageJobs jobs;
+    rc = mlp_images(me, W1, W2, 2 * channels + channels * g.dim + g.dim, g.dim + channels, w1_stride_out, w1_stride_in, w2_stride_out, w2_stride_in, scratch,
+                    scratch_bytes, dz_image, dz_image_bytes, &jobs, rows ? channels : 0, g.dim);
+    if (rc != NPA_OK) return rc;
+    RowsJob rest = {};
+    rc = grid_build_leaving(grid, x, permutation, bin_offsets, block_info, grid_scratch, grid_scratch_bytes, (cudaStream_t)stream, &rest);
+    if (rc != NPA_OK) return rc;
+    return bin_particles_and_images(grid, channels, x, s, permutation, x_out, s_out, jobs, (cudaStream_t)stream, rest);
+}
+
 int64_t npa_step_rows_image_bytes(const npa_grid *gd, int32_t channels) {
     Geom g;
     const int rc = make_geom(gd, &g);

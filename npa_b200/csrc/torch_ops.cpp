@@ -105,9 +105,12 @@ struct Grid {
         require(info, {max_blocks, 4}, "block_info", at::kInt);
     }
     void bin(const Tensor &x, const Tensor &perm, const Tensor &offs, const Tensor &info, void *st) {
+        check_status(npa_grid_build(&g, fptr(x), imut(perm), imut(offs), imut(info), scratch_for(x), scratch_bytes, st));
+    }
+    void *scratch_for(const Tensor &x) {
         if (!scratch.defined() || scratch.device() != x.device())
             scratch = at::empty({scratch_bytes}, at::TensorOptions().dtype(at::kByte).device(x.device()));
-        check_status(npa_grid_build(&g, fptr(x), imut(perm), imut(offs), imut(info), scratch.mutable_data_ptr(), scratch_bytes, st));
+        return scratch.mutable_data_ptr();
     }
     void features(const Tensor &s, const char *name) const { require(s, {B, N, s.dim() == 3 ? s.size(2) : -1}, name); }
 };
@@ -827,7 +830,6 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     const bool record = recording(x, s, w1, b1, w2);
     const bool back = record && ((wants_grad(x) && !stop_pos) || (wants_grad(s) && !stop_state));  // a backward reaches the perception
     Tensor perm = ints(x, {g.B, g.N}), offs = ints(x, {g.B * g.cells + 1}), info = ints(x, {g.max_blocks, 4});
-    grid->bin(x, perm, offs, info, st);
     const int64_t bytes = npa_mlp_forward_tcgen05_scratch_bytes((int)k, (int)o), rows_bytes = back && !npa_tile_enabled(1) && !(wants_grad(x) && !stop_pos) ? npa_step_rows_image_bytes(&g.g, (int)C) : 0;
     const bool rows = rows_bytes > 0;  // the backward takes dL/dz apart as it forms it
     const int64_t dz_bytes = rows ? rows_bytes : back ? npa_linear_tcgen05_scratch_bytes(kHidden, (int)k) : 0;
@@ -840,12 +842,8 @@ py::tuple euler_step(const GridPtr &grid, const Tensor &x, const Tensor &s, cons
     float *t = fmut(slab), *x_bin = t + o_x, *s_bin = t + o_s, *rho = t + o_rho, *rho_grad = t + o_dg, *z = t + o_z, *packed = t + o_packed,
           *y = t + o_y, *vgrad = back ? t + o_v : nullptr, *h = record ? t + o_h : nullptr, *dz_image = dz_bytes ? t + o_dz : nullptr;
     int32_t *pairs = reinterpret_cast<int32_t *>(t + o_pairs);
-    if (rows)
-        check_status(npa_bin_particles_step_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), w1.stride(0), w1.stride(1),
-                                                   w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
-    else
-        check_status(npa_bin_particles_mlp_images(&g.g, (int)C, fptr(x), fptr(s), iptr(perm), x_bin, s_bin, fptr(w1), fptr(w2), (int)k, (int)o, w1.stride(0),
-                                                  w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, st));
+    check_status(npa_step_bin(&g.g, (int)C, fptr(x), fptr(s), imut(perm), imut(offs), imut(info), g.scratch_for(x), g.scratch_bytes, x_bin, s_bin, fptr(w1),
+                              fptr(w2), w1.stride(0), w1.stride(1), w2.stride(0), w2.stride(1), t + o_image, bytes, dz_image, dz_bytes, rows, st));
     check_status(npa_perceive_features_forward_lists(&g.g, (int)C, x_bin, nullptr, s_bin, (float)coef, (float)dg_scale, (float)inv_tol, ln_grad, ln_dg,
                                                      rho, rho_grad, z, vgrad, packed, iptr(offs), iptr(info), pairs, (int)columns, st));
     Tensor mask = update_prob < 1.0 ? at::rand({g.B, g.N, 1}, s.options().requires_grad(false)) : Tensor();

@@ -63,8 +63,19 @@ __device__ inline void write_image_element(const ImageJobs &jobs, int at) {
     }
 }
 
-// binning.cu: npa_bin_particles (without masses) whose launch also makes the images.
+// Work list of several small systems that a grid build has left to the launch behind it.
+struct RowsJob {
+    const int32_t *bin_offsets;
+    int4 *block_info;
+    const uint32_t *rows_of_system;
+    Geom g;
+    int systems;  // 0: nothing is left
+};
+// binning.cu: npa_grid_build; with `rest`, the work list of several systems is left to bin_particles_and_images where it has a launch of its own.
+int grid_build_leaving(const npa_grid *grid, const float *x, int32_t *permutation, int32_t *bin_offsets, int32_t *block_info, void *scratch,
+                       int64_t scratch_bytes, cudaStream_t stream, RowsJob *rest);
+// binning.cu: npa_bin_particles (without masses) whose launch also makes the images, and the work list that `rest` names.
 int bin_particles_and_images(const npa_grid *grid, int channels, const float *x, const float *s, const int32_t *permutation, float *x_out,
-                             float *s_out, const ImageJobs &jobs, cudaStream_t stream);
+                             float *s_out, const ImageJobs &jobs, cudaStream_t stream, const RowsJob &rest = {});
 
 }  // namespace npa

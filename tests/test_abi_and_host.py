@@ -365,6 +365,15 @@ def test_step_rows_entries_reject_bad_arguments_before_any_launch():
         def backward(C=16, dh=buf, image=buf, image_bytes=size, x=buf, v=buf, out=buf, scratch=buf, nbytes=work, stride=128):
             return lib.npa_step_perceive_backward(ref, C, dh, image, image_bytes, x, buf, buf, v, buf, 1.0, 1, null, out, scratch, nbytes, buf, buf, stride, null)
 
+        build = lib.npa_grid_scratch_bytes(ref)
+
+        def begin(C=16, x=buf, s=buf, perm=buf, scratch=buf, build_bytes=build, xo=buf, w1=buf, nbytes=need, image=buf, image_bytes=size, rows=1):
+            return lib.npa_step_bin(ref, C, x, s, perm, buf, buf, scratch, build_bytes, xo, buf, w1, buf, 82, 1, 128, 1, buf, nbytes, image, image_bytes, rows, null)
+
+        assert begin(C=13) == n.NPA_ERR_UNSUPPORTED and begin(build_bytes=build - 1) == n.NPA_ERR_SCRATCH_TOO_SMALL
+        for bad in (dict(x=null), dict(s=null), dict(perm=null), dict(scratch=null), dict(scratch=odd), dict(xo=null), dict(w1=null), dict(nbytes=need - 1),
+                    dict(image=odd), dict(image_bytes=size - 1), dict(x=odd if dim == 3 else ctypes.c_void_p((1 << 20) + 2))):
+            assert begin(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
         assert images(C=13) == n.NPA_ERR_UNSUPPORTED and images(C=36) == n.NPA_ERR_UNSUPPORTED
         for bad in (dict(image=null), dict(image=odd), dict(image_bytes=size - 1), dict(nbytes=need - 1), dict(w1=null), dict(x=null)):
             assert images(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad

@@ -61,3 +61,35 @@ def test_rows_as_the_separate_kernels_make_them(dim, boundary, B, N, C, log_norm
     status = ctypes.c_uint32(1)
     n.check(n.lib.npa_linear_tcgen05_status(ctypes.byref(status), 0))
     assert status.value == 0
+
+
+# one system and several, binned by a CTA, a cluster or the general way; cells up to the line beyond which the work list has its own launch
+@pytest.mark.parametrize("dim,B,N,cells,C", [(2, 1, 300, 16, 16), (2, 5, 1, 4, 12), (2, 64, 512, 9, 16), (2, 300, 33, 5, 8), (2, 3, 4096, 45, 16), (2, 3, 4096, 46, 16),
+                                             (2, 7, 20000, 20, 13), (3, 4, 9000, 12, 32), (3, 2, 70000, 20, 16), (3, 3, 2000, 13, 16)])
+def test_beginning_of_a_step_in_one_call(dim, B, N, cells, C):
+    """Grid build, work list, reorder and images: the bytes of the separate calls."""
+    from npa_b200 import _native as n, sphops as sph
+    torch.manual_seed(N)
+    p, st, eps = n.ptr, n.current_stream(), 0.05
+    x, s = _positions(dim, B, N, cells * eps), torch.randn(B, N, C, device="cuda")
+    grid = sph.HashGrid(dim=dim, boundary="clamped", mode="grid", grid_size=(cells,) * dim, eps=eps, num_particles=N, batch_size=B, max_particles_per_block=16)
+    gd = n.make_grid(dim, "clamped", "grid", (cells,) * dim, eps, B, N, 16)
+    ref, snap = ctypes.byref(gd), grid.instantiate(x)
+    K, O = 2 * C + C * dim + dim, dim + C
+    W1, W2 = torch.randn(128, K, device="cuda"), torch.randn(O, 128, device="cuda")
+    strides = (K, 1, 128, 1)
+    nbytes, build_bytes = n.lib.npa_mlp_forward_tcgen05_scratch_bytes(K, O), n.lib.npa_grid_scratch_bytes(ref)
+    for rows in (0, 1) if C % 4 == 0 else (0,):
+        size = n.lib.npa_step_rows_image_bytes(ref, C) if rows else n.lib.npa_linear_tcgen05_scratch_bytes(128, K)
+        new = lambda: [torch.full((nbytes // 4,), -1.0, device="cuda"), torch.full((size // 4,), -1.0, device="cuda"), torch.empty_like(x), torch.empty_like(s)]
+        want, got = new(), new()
+        head, tail = (ref, C, p(x), p(s)), (*strides, p(want[0]), nbytes, p(want[1]), size)
+        out = (p(want[2]), p(want[3]), p(W1), p(W2))
+        n.check(n.lib.npa_bin_particles_step_images(*head, p(snap.permutation), *out, *tail, st) if rows
+                else n.lib.npa_bin_particles_mlp_images(*head, p(snap.permutation), *out, K, O, *tail, st))
+        lists = [torch.full_like(t, -7) for t in (snap.permutation, snap.bin_offsets, snap.block_info)]
+        scratch = torch.empty(build_bytes, dtype=torch.uint8, device="cuda")
+        n.check(n.lib.npa_step_bin(*head, *map(p, lists), p(scratch), build_bytes, p(got[2]), p(got[3]), p(W1), p(W2), *strides, p(got[0]), nbytes, p(got[1]), size,
+                                   rows, st))
+        for a, b in zip(got + lists, want + [snap.permutation, snap.bin_offsets, snap.block_info]):
+            assert torch.equal(a, b)
