@@ -524,6 +524,14 @@ int npa_step_hidden_grad(const npa_grid *g, const float *y, int32_t y_pitch, con
  * scratch with npa_mlp_weight_grad_tcgen05_scratch_floats() floats.  Bounded waits report through
  * npa_linear_tcgen05_status (bits 16, 32, 64: MMA lane, producers, epilogue of this kernel). */
 int64_t npa_mlp_weight_grad_tcgen05_scratch_floats(int64_t rows, int32_t in_dim, int32_t out_dim);
+/* The same in two calls: the partial sums (in scratch), and their sum beside the inverse reorder of a step's gradients (npa_unbin_particles
+ * without masses) on a grid of B*N = rows particles.  `partial` is the scratch of the first call. */
+int npa_mlp_weight_grad_tcgen05_partial(const float *z, const float *dh, const float *h, const float *dy, int64_t rows,
+                                        int32_t in_dim, int32_t hidden, int32_t out_dim, float *scratch, int64_t scratch_floats,
+                                        void *stream);
+int npa_step_unbin(const npa_grid *g, int32_t channels, const float *x_bin, const float *s_bin, const int32_t *permutation,
+                   float *x_out, float *s_out, int32_t in_dim, int32_t out_dim, const float *partial, int64_t partial_floats,
+                   float *dW1, float *dW2, float *db1, void *stream);
 int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h, const float *dy, int64_t rows,
                                 int32_t in_dim, int32_t hidden, int32_t out_dim, float *scratch,
                                 int64_t scratch_floats, float *dW1, float *dW2, float *db1, void *stream);

@@ -113,6 +113,8 @@ SIGNATURES = {
                              + [_I32, ctypes.c_int64, ctypes.c_int64, _P]),
     "npa_mlp_weight_grad_tcgen05": (ctypes.c_int, [_P, _P, _P, _P, ctypes.c_int64, _I32, _I32, _I32, _P, ctypes.c_int64,
                                                    _P, _P, _P, _P]),
+    "npa_mlp_weight_grad_tcgen05_partial": (ctypes.c_int, [_P] * 4 + [_I64, _I32, _I32, _I32, _P, _I64, _P]),
+    "npa_step_unbin": (ctypes.c_int, [_P, _I32] + [_P] * 5 + [_I32, _I32, _P, _I64, _P, _P, _P, _P]),
     "npa_mlp_weight_grad_tcgen05_scratch_floats": (ctypes.c_int64, [ctypes.c_int64, _I32, _I32]),
     "npa_linear_tf32x3": (ctypes.c_int, [_P, _P, _P, _P, _P, ctypes.c_int64, _I32, _I32, ctypes.c_int64, ctypes.c_int64,
                                          _I32, _P]),

@@ -14,7 +14,8 @@
 // segment of 128 rows (48 accumulations): after each segment the epilogue warps add the accumulators,
 // rounding to nearest, into running sums kept in a second region of tensor memory, and the MMAs
 // start the next segment from zero.  At the end each CTA writes its sums to global memory and a
-// second kernel adds the CTAs' partial sums in a fixed order: results are deterministic.
+// second kernel (in a step the launch of the inverse reorder: mlp_grad_reduce.cuh) adds the CTAs' partial sums in a fixed order: results are
+// deterministic.
 //
 // One persistent CTA per SM with a contiguous slab of rows; stages of 16 rows:
 //   * one lane brings the 16 rows of dh, h, z and dy of a stage into a ring of raw stages with four bulk
@@ -28,12 +29,11 @@
 // npa_linear_tcgen05_status (bits 16, 32, 64: MMA lane, producers, epilogue of this kernel).
 #include <mutex>
 
+#include "mlp_grad_reduce.cuh"
 #include "umma.cuh"
 
 namespace npa {
 
-constexpr int kGradHidden = 128;
-constexpr int kGradStageRows = 16;                 // two k-groups of eight rows
 constexpr int kGradSegmentStages = 8;              // 128 rows per accumulation chain
 constexpr int kGradProducerWarps = 16;
 constexpr int kGradEpilogueWarps = 8;
@@ -73,7 +73,6 @@ struct GradShared {
 struct GradArgs {
     const float *z, *dh, *h, *dy;
     float *partial;          // [ctas][128][N1p + N2p]
-    float *dW1, *dW2, *db1;
     long long M;
     int in_dim, out_dim, N1p, N2p, stages_per_cta, ctas;
     unsigned *status;
@@ -349,53 +348,11 @@ __global__ void __launch_bounds__(kGradThreads, 1) mlp_grad_umma_kernel(const __
     }
 }
 
-// dW1, db1 and dW2 from the CTAs' partial sums.  A thread takes four neighbouring columns of a hidden unit, as they lie in the partial
-// sums, of one run of CTAs: all its loads are in flight at once, and a warp reads 512 bytes in a row of each CTA (by output instead,
-// dW2's columns lay a row apart).  The runs meet in shared memory, in order.  Latency bound: 7.6 MB (in = 66, out = 18) or 17 MB (163, 35)
-// from L2 in one round trip: 8.4 -> 5.2 us and 9.1 -> 5.7.
-constexpr int kReduceQuads = 32, kReduceRuns = 16, kReduceMost = (148 + kReduceRuns - 1) / kReduceRuns;
-__global__ void __launch_bounds__(kReduceQuads * kReduceRuns) mlp_grad_umma_reduce_kernel(const __grid_constant__ GradArgs a) {
+__global__ void __launch_bounds__(kReduceQuads * kReduceRuns) mlp_grad_umma_reduce_kernel(const __grid_constant__ GradReduce a) {
     after_previous_kernel();
-    __shared__ float4 s_sum[kReduceRuns][kReduceQuads];
-    const int K1 = a.in_dim, O = a.out_dim, Wp = a.N1p + a.N2p;
-    const int q1 = (K1 + 4) / 4, per_unit = q1 + (O + 3) / 4, total = kGradHidden * per_unit;  // quads that hold results
-    const int lane = threadIdx.x % kReduceQuads, run = threadIdx.x / kReduceQuads;
-    auto column = [&](int q) {  // of the first float of quad q, in the partial sums
-        const int u = q % per_unit;
-        return (long long)(q / per_unit) * Wp + (u < q1 ? 4 * u : a.N1p + 4 * (u - q1));
-    };
-    const int quad = min((int)blockIdx.x * kReduceQuads + lane, total - 1);
-    const float *p = a.partial + column(quad);
-    const long long step = (long long)kGradHidden * Wp;
-    const int each = (a.ctas + kReduceRuns - 1) / kReduceRuns, c0 = run * each, end = min(c0 + each, a.ctas);
-    float4 v[kReduceMost];
-#pragma unroll
-    for (int u = 0; u < kReduceMost; ++u)
-        v[u] = u < each && c0 + u < end ? __ldg(reinterpret_cast<const float4 *>(p + (c0 + u) * step)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 sum = v[0];
-#pragma unroll
-    for (int u = 1; u < kReduceMost; ++u) {
-        sum.x += v[u].x; sum.y += v[u].y; sum.z += v[u].z; sum.w += v[u].w;
-    }
-    s_sum[run][lane] = sum;
-    __syncthreads();
-    if (threadIdx.x >= 4 * kReduceQuads) return;
-    const int q = blockIdx.x * kReduceQuads + threadIdx.x / 4, part = threadIdx.x % 4;
-    if (q >= total) return;
-    float out = 0.f;
-#pragma unroll
-    for (int r = 0; r < kReduceRuns; ++r) out += reinterpret_cast<const float *>(&s_sum[r][threadIdx.x / 4])[part];
-    const int j = q / per_unit, u = q - j * per_unit, col = u < q1 ? 4 * u + part : 4 * (u - q1) + part;
-    if (u >= q1) {
-        if (col < O) a.dW2[(long long)col * kGradHidden + j] = out;
-    } else if (col < K1) {
-        a.dW1[(long long)j * K1 + col] = out;
-    } else if (col == K1) {
-        a.db1[j] = out;  // the ones column
-    }
+    reduce_weight_grads<kReduceQuads>(a, (int)blockIdx.x);
 }
 
-static int grad_round16(int v) { return (v + 15) / 16 * 16; }
 
 struct GradDevice {
     unsigned *status = nullptr;
@@ -413,6 +370,9 @@ using namespace npa;
 
 extern "C" {
 
+static int weight_grad_partial(const char *me, const float *z, const float *dh, const float *h, const float *dy, int64_t rows, int32_t in_dim, int32_t hidden,
+                               int32_t out_dim, float *scratch, int64_t scratch_floats, void *stream);
+
 int64_t npa_mlp_weight_grad_tcgen05_scratch_floats(int64_t rows, int32_t in_dim, int32_t out_dim) {
     if (rows <= 0 || in_dim <= 0 || out_dim <= 0) return 0;
     return (int64_t)148 * kGradHidden * (grad_round16(in_dim + 1) + grad_round16(out_dim));
@@ -422,11 +382,27 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
                                 int32_t hidden, int32_t out_dim, float *scratch, int64_t scratch_floats, float *dW1,
                                 float *dW2, float *db1, void *stream) {
     const char *me = "npa_mlp_weight_grad_tcgen05";
+    if (!dW1 || !dW2 || !db1) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: every pointer must be non-NULL", me);
+    const int rc = weight_grad_partial(me, z, dh, h, dy, rows, in_dim, hidden, out_dim, scratch, scratch_floats, stream);
+    if (rc != NPA_OK) return rc;
+    GradReduce a = grad_plan(rows, in_dim, out_dim);
+    a.partial = scratch; a.dW1 = dW1; a.dW2 = dW2; a.db1 = db1;
+    mlp_grad_umma_reduce_kernel<<<a.blocks(kReduceQuads), kReduceQuads * kReduceRuns, 0, (cudaStream_t)stream>>>(a);
+    return check_launch("mlp_grad_umma_reduce_kernel");
+}
+
+int npa_mlp_weight_grad_tcgen05_partial(const float *z, const float *dh, const float *h, const float *dy, int64_t rows, int32_t in_dim,
+                                        int32_t hidden, int32_t out_dim, float *scratch, int64_t scratch_floats, void *stream) {
+    return weight_grad_partial("npa_mlp_weight_grad_tcgen05_partial", z, dh, h, dy, rows, in_dim, hidden, out_dim, scratch, scratch_floats, stream);
+}
+
+static int weight_grad_partial(const char *me, const float *z, const float *dh, const float *h, const float *dy, int64_t rows, int32_t in_dim, int32_t hidden,
+                               int32_t out_dim, float *scratch, int64_t scratch_floats, void *stream) {
     if (hidden != kGradHidden) return fail(NPA_ERR_UNSUPPORTED, "%s: hidden width must be %d, got %d", me, kGradHidden, hidden);
     if (in_dim <= 0 || in_dim > kGradMaxIn || out_dim <= 0 || out_dim > kGradMaxOut)
         return fail(NPA_ERR_UNSUPPORTED, "%s: supports in <= %d and out <= %d, got %d and %d", me, kGradMaxIn, kGradMaxOut, in_dim, out_dim);
     if (rows <= 0) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: rows must be positive", me);
-    if (!z || !dh || !h || !dy || !scratch || !dW1 || !dW2 || !db1) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: every pointer must be non-NULL", me);
+    if (!z || !dh || !h || !dy || !scratch) return fail(NPA_ERR_INVALID_ARGUMENT, "%s: every pointer must be non-NULL", me);
     if (((uintptr_t)z | (uintptr_t)dh | (uintptr_t)h | (uintptr_t)dy | (uintptr_t)scratch) % 16)
         return fail(NPA_ERR_INVALID_ARGUMENT, "%s: z, dh, h, dy and scratch must be 16-byte aligned", me);
     const int64_t need = npa_mlp_weight_grad_tcgen05_scratch_floats(rows, in_dim, out_dim);
@@ -434,14 +410,10 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
         return fail(NPA_ERR_SCRATCH_TOO_SMALL, "%s: scratch has %lld floats, %lld needed", me, (long long)scratch_floats, (long long)need);
 
     GradArgs a = {};
-    a.z = z; a.dh = dh; a.h = h; a.dy = dy; a.partial = scratch; a.dW1 = dW1; a.dW2 = dW2; a.db1 = db1;
+    a.z = z; a.dh = dh; a.h = h; a.dy = dy; a.partial = scratch;
     a.M = rows; a.in_dim = in_dim; a.out_dim = out_dim;
-    a.N1p = grad_round16(in_dim + 1);
-    a.N2p = grad_round16(out_dim);
-    const long long stages_total = (rows + kGradStageRows - 1) / kGradStageRows;
-    int ctas = (int)(stages_total < 148 ? stages_total : 148);
-    a.stages_per_cta = (int)((stages_total + ctas - 1) / ctas);
-    a.ctas = (int)((stages_total + a.stages_per_cta - 1) / a.stages_per_cta);
+    const GradReduce plan = grad_plan(rows, in_dim, out_dim);
+    a.N1p = plan.N1p; a.N2p = plan.N2p; a.ctas = plan.ctas; a.stages_per_cta = plan.stages_per_cta;
 
     const bool narrow = in_dim <= GradNarrow::kMaxIn && out_dim <= GradNarrow::kMaxOut;
     const auto kernel = narrow ? mlp_grad_umma_kernel<GradNarrow> : mlp_grad_umma_kernel<GradWide>;
@@ -462,11 +434,7 @@ int npa_mlp_weight_grad_tcgen05(const float *z, const float *dh, const float *h,
     }
     cudaStream_t st = (cudaStream_t)stream;
     launch_early(kernel, a.ctas, kGradThreads, smem, st, a);
-    int rc = check_launch("mlp_grad_umma_kernel");
-    if (rc != NPA_OK) return rc;
-    const int quads = kGradHidden * ((in_dim + 4) / 4 + (out_dim + 3) / 4);
-    mlp_grad_umma_reduce_kernel<<<(quads + kReduceQuads - 1) / kReduceQuads, kReduceQuads * kReduceRuns, 0, st>>>(a);
-    return check_launch("mlp_grad_umma_reduce_kernel");
+    return check_launch("mlp_grad_umma_kernel");
 }
 
 }  // extern "C"

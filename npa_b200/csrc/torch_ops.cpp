@@ -649,11 +649,15 @@ int64_t weight_grad_scratch_floats(int64_t m, int64_t k, int64_t o) {
     return k < 176 ? npa_mlp_weight_grad_tcgen05_scratch_floats(m, (int)k, (int)o) : npa_mlp_weight_grad_scratch_floats(m, (int)k, (int)o);
 }
 void mlp_weight_grads(const float *z, const float *dh, const float *h, const float *dy, int64_t m, const Tensor &w1, const Tensor &w2,
-                      float *scratch, Tensor &gw1, Tensor &gb1, Tensor &gw2, void *st) {
+                      float *scratch, Tensor &gw1, Tensor &gb1, Tensor &gw2, void *st, bool partial = false) {
     const int64_t k = w1.size(1), o = w2.size(0);
     gw1 = blank(w1);
     gw2 = blank(w2);
     gb1 = floats(w1, {kHidden});
+    if (partial) {  // added up by npa_step_unbin
+        check_status(npa_mlp_weight_grad_tcgen05_partial(z, dh, h, dy, m, (int)k, kHidden, (int)o, scratch, weight_grad_scratch_floats(m, k, o), st));
+        return;
+    }
     check_status((k < 176 ? npa_mlp_weight_grad_tcgen05 : npa_mlp_weight_grad)(z, dh, h, dy, m, (int)k, kHidden, (int)o, scratch,
                                                                                weight_grad_scratch_floats(m, k, o), fmut(gw1), fmut(gw2), fmut(gb1), st));
 }
@@ -769,7 +773,8 @@ struct EulerNode : Node {
             check_status(npa_step_hidden_grad(gd, y, (int)y_pitch, fptr(mask), mask.defined(), below, (int)C, alpha, dt, fptr(gx_new), fptr(gs_new), fptr(w2), h, gy,
                                               dh, kHidden, w2.stride(0), w2.stride(1), st));
         Tensor gw1, gb1, gw2;
-        if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st);
+        const bool sum_later = weights && k < 176 && (nx || ns);  // the launch of the inverse reorder adds the partial sums up
+        if (weights) mlp_weight_grads(z, dh, h, gy, m, w1, w2, t + o_scratch, gw1, gb1, gw2, st, sum_later);
         // perception, with the update's own gradient of the states added
         Tensor gx_bin = gx_new, none;
         const float *gs_bin = fptr(gs_new);
@@ -806,7 +811,10 @@ struct EulerNode : Node {
         }
         if (nx) gx = floats(w1, {gr.B, gr.N, gr.P});
         if (ns) gs = floats(w1, {gr.B, gr.N, C});
-        if (nx || ns)
+        if (sum_later)
+            check_status(npa_step_unbin(gd, (int)C, nx ? fptr(gx_bin) : nullptr, ns ? gs_bin : nullptr, iptr(perm), fmut(gx), fmut(gs), (int)k, (int)o,
+                                        t + o_scratch, weight_grad_scratch_floats(m, k, o), fmut(gw1), fmut(gw2), fmut(gb1), st));
+        else if (nx || ns)
             check_status(npa_unbin_particles(gd, (int)C, nx ? fptr(gx_bin) : nullptr, ns ? gs_bin : nullptr, nullptr, iptr(perm), fmut(gx), fmut(gs),
                                              nullptr, st));
         return {gx, gs, n1 ? gw1 : Tensor(), nb ? gb1 : Tensor(), n2 ? gw2 : Tensor()};

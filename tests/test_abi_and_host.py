@@ -374,6 +374,14 @@ def test_step_rows_entries_reject_bad_arguments_before_any_launch():
         for bad in (dict(x=null), dict(s=null), dict(perm=null), dict(scratch=null), dict(scratch=odd), dict(xo=null), dict(w1=null), dict(nbytes=need - 1),
                     dict(image=odd), dict(image_bytes=size - 1), dict(x=odd if dim == 3 else ctypes.c_void_p((1 << 20) + 2))):
             assert begin(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
+        floats = lib.npa_mlp_weight_grad_tcgen05_scratch_floats(8, 32 + 17 * dim, 16 + dim)
+
+        def unbin(x=buf, s=buf, perm=buf, xo=buf, partial=buf, size=floats, k=32 + 17 * dim, w1=buf, w2=buf, b1=buf):
+            return lib.npa_step_unbin(ref, 16, x, s, perm, xo, buf, k, 16 + dim, partial, size, w1, w2, b1, null)
+
+        assert unbin(size=floats - 1) == n.NPA_ERR_SCRATCH_TOO_SMALL
+        for bad in (dict(x=null, s=null), dict(perm=null), dict(xo=null), dict(partial=null), dict(partial=odd), dict(k=0), dict(w1=null), dict(w2=null), dict(b1=null)):
+            assert unbin(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
         assert images(C=13) == n.NPA_ERR_UNSUPPORTED and images(C=36) == n.NPA_ERR_UNSUPPORTED
         for bad in (dict(image=null), dict(image=odd), dict(image_bytes=size - 1), dict(nbytes=need - 1), dict(w1=null), dict(x=null)):
             assert images(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad

@@ -93,3 +93,32 @@ def test_beginning_of_a_step_in_one_call(dim, B, N, cells, C):
                                    rows, st))
         for a, b in zip(got + lists, want + [snap.permutation, snap.bin_offsets, snap.block_info]):
             assert torch.equal(a, b)
+
+
+@pytest.mark.parametrize("dim,B,N,C", [(2, 1, 5, 1), (2, 3, 43, 16), (2, 8, 4096, 16), (3, 1, 9001, 13), (3, 2, 700, 32)])
+@pytest.mark.parametrize("which", ["both", "features", "positions"])
+def test_weight_gradients_added_beside_the_inverse_reorder(dim, B, N, C, which):
+    """The bits of the two separate calls: the runs and the order of the sums are the same."""
+    from npa_b200 import _native as n
+    torch.manual_seed(N)
+    p, st, K, O, M = n.ptr, n.current_stream(), 2 * C + C * dim + dim, dim + C, B * N
+    gd = n.make_grid(dim, "clamped", "grid", (4,) * dim, 0.1, B, N, 16)
+    e = lambda *shape: torch.randn(*shape, device="cuda")
+    z, dh, h, dy, x, s = e(M, K), e(M, 128), e(M, 128), e(M, O), e(B, N, 2 if dim == 2 else 4), e(B, N, C)
+    perm = torch.stack([torch.randperm(N, device="cuda") for _ in range(B)]).to(torch.int32)
+    size = n.lib.npa_mlp_weight_grad_tcgen05_scratch_floats(M, K, O)
+    x_in, s_in = (x if which != "features" else None), (s if which != "positions" else None)
+
+    def outputs():
+        return [torch.full_like(t, float("nan")) for t in (x, s)] + [torch.full(q, float("nan"), device="cuda") for q in ((128, K), (O, 128), (128,))]
+
+    want, got, work = outputs(), outputs(), torch.empty(size, device="cuda")
+    of = lambda t, given: p(t) if given is not None else None
+    rows = (p(z), p(dh), p(h), p(dy), M, K, 128, O, p(work), size)
+    n.check(n.lib.npa_mlp_weight_grad_tcgen05(*rows, *map(p, want[2:]), st))
+    n.check(n.lib.npa_unbin_particles(ctypes.byref(gd), C, p(x_in), p(s_in), None, p(perm), of(want[0], x_in), of(want[1], s_in), None, st))
+    n.check(n.lib.npa_mlp_weight_grad_tcgen05_partial(*rows, st))
+    n.check(n.lib.npa_step_unbin(ctypes.byref(gd), C, p(x_in), p(s_in), p(perm), of(got[0], x_in), of(got[1], s_in), K, O, p(work), size, *map(p, got[2:]), st))
+    for a, b in zip(got, want):
+        assert torch.equal(a.nan_to_num(7.0), b.nan_to_num(7.0))
+    assert not bool(torch.isnan(got[2]).any() | torch.isnan(got[3]).any() | torch.isnan(got[4]).any())
