@@ -14,8 +14,8 @@
 // Single precision: every operand is split into a TF32 head, rounded to nearest, and a tail of at most twelve bits; three MMAs per product
 // (tail . head + head . tail + head . head).  The tensor cores truncate when they accumulate, so a chain is one group of eight neighbours
 // (heads 1 + D MMAs, the others apart) and is added to the running sums in single precision.  A product with a zero weight spreads a row
-// that is not finite to particles that are no neighbours of it; a warp whose sums are not finite therefore computes its particles again,
-// pair by pair.
+// or a volume that is not finite to particles that are no neighbours of it; a warp whose sums, of the rows or of T, are not finite therefore
+// computes its particles again, pair by pair.
 //
 // Measured, B200, us, lists -> this: 8 x 4,096 particles in 2D, C = 16, 50 neighbours 32 -> 24; 64 x 512 along lines 34 -> 20; 4 x 65,536 in 3D,
 // C = 32, 41 neighbours 372 -> 334 (of these the search 121; instructions 210 M, 60 % of the slots, MMAs a quarter of the tensor pipe's time).
@@ -333,6 +333,8 @@ feature_dense_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, cons
             acc[m][q] += others[m][q];
             probe = fmaf(0.f, acc[m][q], probe);
         }
+#pragma unroll
+    for (int d = 0; d < D; ++d) probe = fmaf(0.f, tsum[d], probe);
     if (__any_sync(kFull, !(probe == 0.f))) {
         dense_pairwise<D, PER>(a, g, mem, first, here);
         return;

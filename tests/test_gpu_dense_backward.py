@@ -11,7 +11,7 @@ pytestmark = pytest.mark.gpu
 class Call:
     """The backward of the packed perception for given rows of dL/dz, by lists or as a step calls it."""
 
-    def __init__(self, x, cells, eps, boundary, C):
+    def __init__(self, x, cells, eps, boundary, C, mass=None):
         from npa_b200 import _native as n, sphops as sph
         from npa_b200.sphops import sph as impl
         self.n, self.C, self.eps, self.boundary = n, C, eps, boundary
@@ -23,12 +23,13 @@ class Call:
         self.box = cells * eps
         s = torch.randn(self.B, self.N, C, device="cuda")
         self.snap = grid.instantiate(x)
-        self.x, self.s = sph.bin_particles(x, s, self.snap)
+        self.x, self.s, *m = sph.bin_particles(x, s, self.snap, *(() if mass is None else (mass,)))
+        self.mass = m[0] if m else None
         Z, self.K = 2 * C + C * self.dim + self.dim, impl._columns(grid.hashgrid)
         e = lambda *shape, **kw: torch.empty(self.B, self.N, *shape, device="cuda", **kw)
         self.rho, self.dg, self.z, self.v, self.packed, self.pairs = e(), e(self.dim), e(Z), e(C, self.dim), e(4), e(self.K, dtype=torch.int32)
         self.st, p = n.current_stream(), n.ptr
-        n.check(n.lib.npa_perceive_features_forward_lists(ctypes.byref(self.gd), C, p(self.x), None, p(self.s), 1.0, 1.0, 1e-3, 0, 0, p(self.rho), p(self.dg),
+        n.check(n.lib.npa_perceive_features_forward_lists(ctypes.byref(self.gd), C, p(self.x), p(self.mass), p(self.s), 1.0, 1.0, 1e-3, 0, 0, p(self.rho), p(self.dg),
                                                           p(self.z), p(self.v), p(self.packed), p(self.snap.bin_offsets), p(self.snap.block_info),
                                                           p(self.pairs), self.K, self.st))
         self.dz = torch.randn(self.B, self.N, Z, device="cuda")
@@ -39,7 +40,7 @@ class Call:
         f = n.lib.npa_perceive_features_backward_binned if binned else n.lib.npa_perceive_features_backward_lists
         nbytes = n.lib.npa_lists_backward_scratch_bytes(ctypes.byref(self.gd), self.C)
         work, out = torch.empty(nbytes // 4, device="cuda"), torch.full((self.B, self.N, self.C), float("nan"), device="cuda")
-        n.check(f(ctypes.byref(self.gd), self.C, p(self.x), None, p(self.s), p(self.rho), p(self.dg), p(self.v), p(self.packed), p(self.dz), 1.0, 1.0, 0, 0,
+        n.check(f(ctypes.byref(self.gd), self.C, p(self.x), p(self.mass), p(self.s), p(self.rho), p(self.dg), p(self.v), p(self.packed), p(self.dz), 1.0, 1.0, 0, 0,
                   p(add), None, p(out), p(work), nbytes, p(self.snap.bin_offsets), p(self.pairs), self.K, self.st))
         return out
 
@@ -111,3 +112,25 @@ def test_rows_that_are_not_finite_reach_their_neighbours_only(value):
     touched = (got != clean).any(-1)
     assert touched.float().mean() < 0.5
 
+
+@pytest.mark.parametrize("dim,B,N,cells", [(2, 2, 700, 6), (3, 1, 20003, 12)])
+@pytest.mark.parametrize("volume", [None, float("inf"), float("nan")])
+def test_volumes_that_are_not_finite_reach_their_neighbours_only(dim, B, N, cells, volume):
+    """A particle of no mass and no neighbour has the volume 0 / 0: particles beside it in memory that have no pair with it keep their sums,
+    as over the lists."""
+    torch.manual_seed(7)
+    x = _positions(dim, B, N, 0.97)
+    eps = 1 / cells
+    alone = torch.tensor([0.49] * dim, device="cuda")
+    x[(x[..., :dim] - alone).norm(dim=-1) < 1.01 * eps] *= 0.5                  # nobody in reach of the corner
+    x[:, 5, :dim] = alone
+    mass = 0.5 + torch.rand(B, N, device="cuda")
+    mass[:, 5] = 0.0
+    call = Call(x, cells, eps, "clamped", 16, mass)
+    lone = (call.x[..., :dim] == alone).all(-1)
+    assert int(lone.sum()) == B and bool(torch.isnan(call.packed[lone][:, 3]).all())
+    if volume is not None:
+        call.packed[..., 3][lone] = volume
+    got, want = call(True), call(False)
+    assert not torch.isfinite(got[lone]).any() and torch.isfinite(want[~lone]).all()
+    assert torch.allclose(got[~lone], want[~lone], rtol=2e-5, atol=1e-4)
