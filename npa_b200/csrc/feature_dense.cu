@@ -12,14 +12,17 @@
 // cut-off are zero; two fifths of the products are of pairs.
 //
 // Single precision: every operand is split into a TF32 head, rounded to nearest, and a tail of at most twelve bits; three MMAs per product
-// (tail . head + head . tail + head . head).  The tensor cores truncate when they accumulate, so a chain is one group of eight neighbours
+// (tail . head + head . tail + head . head), four in 2D (tail . tail), where few neighbours' roundings do not outweigh it.  The tensor cores truncate when they accumulate, so a chain is one group of eight neighbours
 // (heads 1 + D MMAs, the others apart) and is added to the running sums in single precision.  A product with a zero weight spreads a row
 // or a volume that is not finite to particles that are no neighbours of it; a warp whose sums, of the rows or of T, are not finite therefore
 // computes its particles again, pair by pair.
 //
 // Measured, B200, us, lists -> this: 8 x 4,096 particles in 2D, C = 16, 50 neighbours 32 -> 24; 64 x 512 along lines 34 -> 20; 4 x 65,536 in 3D,
 // C = 32, 41 neighbours 372 -> 334 (of these the search 121; instructions 210 M, 60 % of the slots, MMAs a quarter of the tensor pipe's time).
-// Error against 64 bits (2-norm) 1.3e-7 to 1.75e-7 where the lists' sums have 1.5e-7 to 2.5e-7.  Not kept: sixteen particles per warp (411,
+// Error against 64 bits (2-norm, 1e-7), lists / this, rows N(0, 1): 2D, 14 neighbours 1.47 / 1.44 (1.48 with three MMAs), 25 1.70 / 1.47, 77
+// 2.52 / 1.67; 3D 16 1.66 / 1.62, 39 2.09 / 1.65, 76 2.58 / 1.73; over 80 drawn training cases of 12 and more neighbours at most 0.99 of
+// the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 26 -> 27 us with 16 features, 36 -> 39
+// with 32.  Not kept: sixteen particles per warp (411,
 // larger unions and fewer warps); a queue per residue of the neighbour's index, for rows in banks of their own (515); the head by
 // cvt.rna (452).
 //
@@ -249,6 +252,7 @@ feature_dense_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, cons
                     const Tf32 a0 = split_tf32(v0[c][2 * m]), a1 = split_tf32(v0[c][2 * m + 1]);
                     const Tf32 a2 = split_tf32(v1[c][2 * m]), a3 = split_tf32(v1[c][2 * m + 1]);
                     const unsigned ah[4] = {a0.head, a1.head, a2.head, a3.head}, at[4] = {a0.tail, a1.tail, a2.tail, a3.tail};
+                    if constexpr (D == 2) mma_m16n8k8(others[m], at, b0.tail, b1.tail);
                     mma_m16n8k8(others[m], at, b0.head, b1.head);
                     if (c == 0) mma_m16n8k8_from_zero(heads[m], ah, b0.head, b1.head);
                     else mma_m16n8k8(heads[m], ah, b0.head, b1.head);

@@ -134,3 +134,20 @@ def test_volumes_that_are_not_finite_reach_their_neighbours_only(dim, B, N, cell
     got, want = call(True), call(False)
     assert not torch.isfinite(got[lone]).any() and torch.isfinite(want[~lone]).all()
     assert torch.allclose(got[~lone], want[~lone], rtol=2e-5, atol=1e-4)
+
+
+@pytest.mark.parametrize("dim,N,cells,boundary,C,most", [
+    (2, 6144, 39, "clamped", 16, 1.0), (2, 6144, 39, "clamped", 32, 1.0), (2, 6144, 24, "periodic", 8, 1.0), (2, 6144, 16, "clamped", 13, 1.0),
+    (3, 20480, 17, "clamped", 16, 1.0), (3, 20480, 13, "clamped", 32, 1.0),                          # 13 to 35 neighbours
+    (2, 6144, 55, "clamped", 16, 1.05)])                                                             # 7
+def test_error_is_not_larger_than_that_of_the_lists(dim, N, cells, boundary, C, most):
+    """2-norm against float64: operands in two pieces and sums that the tensor cores truncate have to be as good as single precision."""
+    torch.manual_seed(N + C)
+    call = Call(_positions(dim, 1, N, 1.0), cells, 1.0 / cells, boundary, C)
+    dense, lists = call(True), call(False)
+    error = [0.0, 0.0]
+    for idx in torch.arange(0, N, N // 6144, device="cuda").split(64):
+        want, _ = call.exact(0, idx)
+        for k, out in enumerate((dense, lists)):
+            error[k] += float((out[0, idx].double() - want).square().sum())
+    assert 0 < error[0] ** 0.5 <= most * error[1] ** 0.5
