@@ -393,19 +393,38 @@ int feature_dense_pitch(int dim, int cp) {
 }
 
 // Where it is the faster one, by the mean number of particles per cell of the grid (a tile costs its candidates and the union of its
-// neighbours, a list its length).  Lists / this, us, with the preparation of the rows: 65,536 particles in 2D, C = 16, 16 a cell 71 / 52, 7 a cell
-// 42 / 35, 2 a cell 24.8 / 25.0, 1 a cell 20.7 / 23; periodic, whose candidates are tested image by image, 10 a cell 53 / 51, 7 a cell 43.0 / 42.6,
-// 4 a cell 33 / 35; C = 32 4 a cell 51.7 / 49.5, 2 a cell 42 / 43; clustered particles (8 x 4,096 along lines in 16 x 16 cells) 213 / 68.
-// 65,536 in 3D, C = 16, 8 a cell 73 / 62, 4 a cell 48 / 47.5, 2.4 a cell 37 / 41; C = 32, 19 a cell 191 / 166, 8 a cell 104 / 102, 4 a cell 74 / 80,
-// where the particles fill the grid, and 4 a cell 100 / 101, 4.7 a cell (262,144) 441 / 405 in a ball, where they are twice as dense; 3D periodic
-// 64 a cell 428 / 463, 8 a cell 76 / 89.  Few particles in 3D are a long chain for few warps (8 a cell, C = 32): 8,192 18.7 / 26.7, 16,384 35 / 33,
-// 24,000 44 / 43.
+// neighbours, a list its length) and by the particles in all: a tile is a longer chain than a list, which shows while either kernel is a
+// wave or two.  Particles that leave cells empty have more neighbours than the mean tells, and lists that overflow are searched, so that clustered ones gain
+// earlier and more; the lines are where uniform ones lose nothing or little.  The kernels alone, lists / this, us, uniform unless said otherwise:
+//  * 2D, C = 16: 65,536 particles 2 a cell 17.7 / 18.9, 3 21.3 / 20.5, 4 24.5 / 22.7, 8 37 / 31; along lines 2 a cell 52 / 39, 4 160 / 61; in blobs
+//    29 / 25, 86 / 32; 8,192 2 a cell 6.3 / 7.6, 4 8.5 / 8.5, 8 11.6 / 10.5, along lines 16.4 / 13.7, 67 / 19.  The line at 2 costs uniform particles
+//    up to 1.3 us below 4 a cell, where the clustered ones, which are what is that thin (12 neighbours of uniform particles are 3.8 a cell), gain 2 to 50.
+//  * C = 32: 65,536 2 a cell 26.9 / 27.3, 4 36 / 32; 16,384 9.9 / 9.8, 13.8 / 11.9; 24,000, beyond a wave, 11.0 / 13.5, 14.9 / 14.0; 12,000 2 a cell
+//    6.7 / 9.2, 8 12.8 / 14.3; 8,192 5.8 / 8.7, 10.0 / 12.2; along lines 8,192 2 a cell 14.4 / 15.9, 8 66 / 32, in blobs 8.0 / 10.6, 20.5 / 20.2, 12 a cell
+//    58 / 25: for few particles from 8 a cell, where lists of clustered ones overflow.
+//  * 2D periodic, whose candidates are tested image by image: C = 16, 65,536 7 a cell 34.8 / 35.1, 10 45 / 42; C = 8 33.3 / 35.4, 42.4 / 43.2; C = 32 4 a cell 36.6 /
+//    35.7; 48,000 C = 16 8 a cell 32.6 / 30.9, C = 32 4 a cell 28.3 / 27.9; 33,000 20.3 / 22.7, 8 a cell 30.1 / 30.6; 24,000 C = 16 10 a cell 19.8 / 24.0, 12
+//    22.4 / 25.6.  Fewer particles than 44,000 lose at any uniform density (8,192 12 a cell 14.1 / 18.7, C = 32 13.0 / 19.7): beyond 12 a cell that is left so
+//    for clustered ones.
+//  * 3D, C = 16: 65,536 4 a cell 39.6 / 38.8, 6 52 / 47; 262,144 4 a cell 134 / 136, 5 154 / 150; 32,768 5 a cell 25.2 / 27.7, 8 35.9 / 33.7.  C = 12, whose rows are
+//    padded to 16: 65,536 4 a cell 37.7 / 39.6, 6 50.5 / 47.8.
+//  * 3D, C = 32: 98,304 5 a cell 88.5 / 94.7, 6 96.5 / 98.1, 7 110 / 108; C = 20 6 a cell 94.8 / 99.2, 8 118 / 120.  One wave (20,500) C = 32 7 a cell 30.6 / 30.8, 8
+//    34.9 / 32.4; little more (28,000) 8 a cell 36.4 / 43.4, 14 72.2 / 71.1.  In a ball, where the particles are twice as dense: 98,304 5 a cell
+//    137 / 135, 8 199 / 188.  262,144 uniform 4.5 a cell 215 / 227, 5 218 / 225, 6 250 / 249, in a ball 333 / 323, 341 / 325, 399 / 365, 4 x 65,536 with a radius of
+//    1.05 cells 378 / 343: there the line at 4.5 costs the ones 12 us and gives the others 10 to 35.
+//  * 3D periodic: lists (64 a cell 428 / 463, 8 a cell 76 / 89).
 bool feature_dense_covers(const Geom &g, int C) {
     const long long particles = (long long)g.B * g.N;
     if (g.morton || C > 32 || particles * feature_dense_pitch(g.dim, (C + 3) & ~3) >= (1ll << 30)) return false;
     const double per_cell = (double)g.N / g.cells;
-    if (g.dim == 2) return per_cell >= (!g.periodic ? 2.0 : C > 16 ? 4.0 : 7.0);
-    return !g.periodic && particles >= 20000 && per_cell >= (C > 16 ? 4.5 : 4.0);
+    const bool wide = C > 16;  // two blocks of features
+    if (g.dim == 2 && !g.periodic) return per_cell >= (wide && particles < 14000 ? 8.0 : 2.0);
+    if (g.dim == 2) return per_cell >= (particles < 44000 ? 12.0 : wide ? 4.0 : 10.0);
+    if (g.periodic || particles < 20000) return false;
+    if (!wide) return per_cell >= (particles < 40000 ? 8.0 : C > 12 ? 4.0 : 5.0);
+    if (particles < 60000) return per_cell >= (particles <= 148 * 5 * kDenseWarps * kDenseTile ? 8.0 : 14.0);
+    const bool many = particles >= 200000;
+    return per_cell >= (C > 28 ? (many ? 4.5 : 6.0) : many ? 6.0 : 8.0);
 }
 
 int launch_feature_dense_backward(const Geom &g, const FeatureListBwdArgs &args, cudaStream_t st) {
