@@ -32,7 +32,11 @@ constexpr int kSmemHistCells = 8192;                   // 32 KB of shared histog
 constexpr int kScanThreads = 256;
 constexpr int kScanPerThread = 8;
 constexpr int kScanTile = kScanThreads * kScanPerThread;
-constexpr int kScanPartials = 4096;  // up to so many tiles every CTA of scan_apply_kernel adds up the tiles before its own by itself
+// Up to so many tiles every CTA of scan_apply_kernel adds up the tiles before its own by itself, tiles^2 x 8 bytes from L2 in all; beyond, a
+// launch of one CTA makes prefixes of their sums.  The whole build by prefixes / by itself, us, on a stream: 256 tiles (2 x 64^3 cells) 26.9 / 25.4,
+// 512 (1,024^2) 24.9 / 23.1, 1,024 (128^3) 36.4 / 37.1, 2,048 57.7 / 58.6, 4,096 95 / 100; in a graph 26.1 / 24.8, 22.8 / 22.1, 33.2 / 33.0, 52.4 / 52.1,
+// 93 / 92.
+constexpr int kScanPartials = 512;
 // Cells with more particles than this are ranked by rank_crowded_kernel (linear in the population)
 // instead of the per-particle scan of rank_kernel (quadratic in it).
 constexpr int kCrowdedCell = 256;

@@ -391,3 +391,11 @@ def test_step_rows_entries_reject_bad_arguments_before_any_launch():
                     dict(scratch=odd), dict(x=null), dict(x=odd), dict(stride=1), dict(stride=514)):
             assert backward(**bad) == n.NPA_ERR_INVALID_ARGUMENT, bad
     assert lib.npa_step_rows_image_bytes(ctypes.byref(n.make_grid(2, "clamped", "grid", (8, 8), 0.0, 1, 8, 32)), 16) < 0
+
+
+def test_kernels_of_a_grid_build_general_way():
+    """The sums of up to 512 tiles of 2,048 cells are added up where they are needed, more are scanned by a launch of their own."""
+    from npa_b200 import _native as n
+    for dim, cells, batch, kernels in ((2, (1024, 1024), 1, 6), (2, (1025, 1024), 1, 7), (3, (64, 64, 64), 4, 6), (3, (64, 64, 64), 5, 7), (3, (128,) * 3, 2, 7)):
+        grid = n.make_grid(dim, "clamped", "grid", cells, 0.01, batch, 100000, 32)
+        assert n.lib.npa_grid_build_kernels(ctypes.byref(grid)) == kernels
