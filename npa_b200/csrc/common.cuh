@@ -247,8 +247,7 @@ struct Spiky {
 };
 __device__ inline Spiky spiky_distance(float q) {
     const float Q = q + 1e-12f;
-    float y;  // (Q is a normal number: the general routine scales subnormal ones first, four instructions a pair)
-    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Q));
+    float y = rsqrtf(Q);
     y = fmaf(0.5f * y, fmaf(-(Q * y), y, 1.0f), y);
     const float d = Q * y;
     return Spiky{fmaf(0.5f * y, fmaf(-d, d, Q), d), y};
