@@ -1086,10 +1086,6 @@ int grid_build_leaving(const npa_grid *gd, const float *x, int32_t *permutation,
 
 }  // namespace npa
 
-extern "C" {
-
-}  // extern "C"
-
 // Work arrays of npa_grid_build_static(): a fixed device array owned by the library, so that the
 // call needs no scratch from the caller and allocates nothing.  In host code the symbol is only a
 // handle; its device address is looked up once per device and cached below.

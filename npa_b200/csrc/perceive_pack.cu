@@ -185,13 +185,12 @@ int64_t npa_lists_backward_scratch_bytes(const npa_grid *gd, int32_t channels) {
     return n * (lists > dense ? lists : dense);
 }
 
-static int features_backward_lists(const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
+static int features_backward_lists(const char *me, const npa_grid *gd, int32_t channels, const float *x_bin, const float *mass,
                                    const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
                                    const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
                                    int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
                                    int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, bool binned,
                                    void *stream, const float *dh = nullptr, const void *image = nullptr, int64_t image_bytes = 0) {
-    const char *me = dh ? "step_perceive_backward" : "perceive_features_backward_lists";
     Geom g;
     int rc = make_geom(gd, &g);
     if (rc != NPA_OK) return rc;
@@ -247,7 +246,7 @@ int npa_perceive_features_backward_lists(const npa_grid *gd, int32_t channels, c
                                          int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
                                          int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
     const char *me = "perceive_features_backward_lists";
-    return features_backward_lists(gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
+    return features_backward_lists(me, gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
                                    scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, false, stream);
 }
 
@@ -256,8 +255,8 @@ int npa_perceive_features_backward_binned(const npa_grid *gd, int32_t channels, 
                                          const float *packed, const float *dL_dz, float coef, float dg_scale, int32_t log_norm_grad,
                                          int32_t log_norm_dg, const float *grad_s_add, float *grad_x, float *grad_s, void *scratch,
                                          int64_t scratch_bytes, const int32_t *bin_offsets, const int32_t *pair_cache, int32_t pair_stride, void *stream) {
-    const char *me = "perceive_features_backward_lists";
-    return features_backward_lists(gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
+    const char *me = "perceive_features_backward_binned";
+    return features_backward_lists(me, gd, channels, x_bin, mass, s_bin, rho, rho_grad, vgrad, packed, dL_dz, coef, dg_scale, log_norm_grad, log_norm_dg, grad_s_add, grad_x, grad_s,
                                    scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, true, stream);
 }
 
@@ -277,7 +276,7 @@ int npa_step_perceive_backward(const npa_grid *gd, int32_t channels, const float
     if (need < 0) return (int)need;
     if (scratch_bytes < need)
         return fail(NPA_ERR_SCRATCH_TOO_SMALL, "%s: scratch holds %lld bytes, %lld needed", me, (long long)scratch_bytes, (long long)need);
-    return features_backward_lists(gd, channels, x_bin, nullptr, s_bin, rho, nullptr, vgrad, packed, nullptr, coef, 0.f, log_norm_grad, 0, grad_s_add, nullptr,
+    return features_backward_lists(me, gd, channels, x_bin, nullptr, s_bin, rho, nullptr, vgrad, packed, nullptr, coef, 0.f, log_norm_grad, 0, grad_s_add, nullptr,
                                    grad_s, scratch, scratch_bytes, bin_offsets, pair_cache, pair_stride, true, stream, dh, rows_image, rows_image_bytes);
 }
 

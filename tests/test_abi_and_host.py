@@ -399,3 +399,11 @@ def test_kernels_of_a_grid_build_general_way():
     for dim, cells, batch, kernels in ((2, (1024, 1024), 1, 6), (2, (1025, 1024), 1, 7), (3, (64, 64, 64), 4, 6), (3, (64, 64, 64), 5, 7), (3, (128,) * 3, 2, 7)):
         grid = n.make_grid(dim, "clamped", "grid", cells, 0.01, batch, 100000, 32)
         assert n.lib.npa_grid_build_kernels(ctypes.byref(grid)) == kernels
+
+
+@pytest.mark.parametrize("entry", ["perceive_features_backward_lists", "perceive_features_backward_binned"])
+def test_entries_name_themselves_in_their_errors(entry):
+    from npa_b200 import _native as n
+    grid, null = n.make_grid(2, "clamped", "grid", (8, 8), 0.1, 1, 8, 32), ctypes.c_void_p(0)
+    assert getattr(n.lib, "npa_" + entry)(ctypes.byref(grid), 16, *[null] * 8, 1.0, 1.0, 0, 0, *[null] * 4, 0, null, null, 128, null) == n.NPA_ERR_INVALID_ARGUMENT
+    assert n.last_error().startswith(entry + ":")
