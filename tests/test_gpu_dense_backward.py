@@ -167,3 +167,43 @@ def test_lines_between_the_two_sweeps(dim, boundary, cells, N, C, dense):
     got, lists = call(True), call(False)
     assert torch.equal(got, lists) != dense
     assert torch.allclose(got, lists, rtol=2e-5, atol=2e-5 * float(lists.abs().max()))
+
+
+# boxes of one, two and three cells, whose rows of cells are each other's neighbours on both sides; positions boxes away; positions beyond the cells,
+# which are binned into those at the edge
+@pytest.mark.parametrize("dim,B,N,cells,boundary,away", [
+    (2, 2, 61, 1, "periodic", 0), (2, 3, 133, 2, "periodic", 0), (2, 1, 403, 3, "periodic", 0), (2, 2, 133, 2, "periodic", 3), (2, 2, 1003, 7, "periodic", 3),
+    (2, 1, 48000, 61, "periodic", 100), (2, 2, 4097, 16, "clamped", 0.5), (3, 1, 20011, 11, "clamped", 0.3)])
+@pytest.mark.parametrize("C", [8, 16, 32])
+def test_small_boxes_and_positions_beyond_them(dim, B, N, cells, boundary, away, C):
+    torch.manual_seed(cells + C)
+    x = _positions(dim, B, N, 1.0)
+    if boundary == "periodic":
+        x += torch.randint(-away, away + 1, x.shape, device="cuda")
+    else:
+        x *= 1 + away
+    call = Call(x, cells, 1.0 / cells, boundary, C)
+    got, lists = call(True), call(False)
+    assert not torch.equal(got, lists)
+    for b in range(B):
+        for idx in torch.arange(0, N, max(1, N // 300), device="cuda").split(64):
+            want, size = call.exact(b, idx)
+            for out in (got, lists):
+                assert ((out[b, idx].double() - want).abs() <= 16 * 2.0 ** -24 * size).all()
+
+
+@pytest.mark.parametrize("dim,B,N,cells,C", [(2, 5, 701, 6, 16), (2, 5, 1003, 8, 32), (3, 3, 6701, 9, 13)])
+def test_a_system_alone_and_in_a_batch(dim, B, N, cells, C):
+    """Tiles of eight particles begin elsewhere, and the batch decides between the sweeps: the sums agree within their rounding, not to the bit."""
+    torch.manual_seed(N)
+    batch = Call(_positions(dim, B, N, 0.97), cells, 1.0 / cells, "clamped", C)
+    together = batch(True, batch.add)
+    for b in (1, B - 1):
+        alone = Call(batch.x[b:b + 1].clone(), cells, 1.0 / cells, "clamped", C)
+        assert torch.equal(alone.x[0], batch.x[b]) and torch.equal(alone.rho[0], batch.rho[b])
+        alone.dz, add = batch.dz[b:b + 1].clone(), batch.add[b:b + 1].clone()
+        got = alone(True, add)[0]
+        idx = torch.arange(0, N, max(1, N // 256), device="cuda")
+        for part in idx.split(64):
+            _, size = batch.exact(b, part)
+            assert ((got[part] - together[b, part]).abs() <= 2 * 16 * 2.0 ** -24 * (size + add[0, part].abs())).all()
