@@ -245,12 +245,14 @@ __device__ __forceinline__ unsigned long long add2(unsigned long long a, unsigne
 struct Spiky {
     float d, inv;  // distance and its reciprocal
 };
-__device__ inline Spiky spiky_distance(float q) {
-    const float Q = q + 1e-12f;
-    float y = rsqrtf(Q);
+__device__ inline Spiky spiky_refined(float Q, float y) {  // y: 1 / sqrt(Q) to a few ulps
     y = fmaf(0.5f * y, fmaf(-(Q * y), y, 1.0f), y);
     const float d = Q * y;
     return Spiky{fmaf(0.5f * y, fmaf(-d, d, Q), d), y};
+}
+__device__ inline Spiky spiky_distance(float q) {
+    const float Q = q + 1e-12f;
+    return spiky_refined(Q, rsqrtf(Q));
 }
 // Square root and quotient as IEEE rounds them, without the range checks and branches of the general routines: Newton steps
 // whose residuals are exact by fused multiply-add (P. Markstein, IA-64 and Elementary Functions, ch. 8-9).  For

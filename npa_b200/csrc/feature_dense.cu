@@ -21,7 +21,7 @@
 // C = 32, 41 neighbours 372 -> 334 (of these the search 121; instructions 210 M, 60 % of the slots, MMAs a quarter of the tensor pipe's time).
 // Error against 64 bits (2-norm, 1e-7), lists / this, rows N(0, 1): 2D, 14 neighbours 1.47 / 1.44 (1.48 with three MMAs), 25 1.70 / 1.47, 77
 // 2.52 / 1.67; 3D 16 1.66 / 1.62, 39 2.09 / 1.65, 76 2.58 / 1.73; over 80 drawn training cases of 12 and more neighbours at most 0.99 of
-// the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 26 -> 27 us with 16 features, 36 -> 39
+// the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 26 -> 27 us with 16 features, 36 -> 38
 // with 32.  Not kept: sixteen particles per warp (411,
 // larger unions and fewer warps); a queue per residue of the neighbour's index, for rows in banks of their own (515); the head by
 // cvt.rna (452).
@@ -62,6 +62,17 @@ __device__ __forceinline__ void mma_m16n8k8_from_zero(float (&d)[4], const unsig
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1), "f"(0.f));
 }
 
+// spiky_distance; in 2D with the instruction for the reciprocal square root of a normal number, which Q >= 1e-12 is.  With it / with rsqrtf, us:
+// 8 x 4,096 particles in 2D, C = 16, 26.7 / 28.4, 64 x 512 along lines 23.6 / 24.4, C = 32 38.1 / 40.4; 4 x 65,536 in 3D, C = 32, 344 / 330, C = 16 228 / 234.
+template <int D>
+__device__ __forceinline__ Spiky dense_distance(float q) {
+    if constexpr (D == 3) return spiky_distance(q);
+    const float Q = q + 1e-12f;
+    float y;
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(Q));
+    return spiky_refined(Q, y);
+}
+
 // Weights of one pair: c_s W and -K, zero unless `live`; K itself times the neighbour's volume goes into T.
 template <int D, bool PER>
 __device__ __forceinline__ void dense_weights(const Geom &g, const Pos<D> &pi, const float4 &c, bool live, float (&w)[1 + D], float (&tsum)[3]) {
@@ -69,7 +80,7 @@ __device__ __forceinline__ void dense_weights(const Geom &g, const Pos<D> &pi, c
     listed_displacement<D, PER>(g, pi, Pos<D>{c.x, c.y, c.z}, r[0], r[1], r[2]);
     const float q = live ? sq_norm_fast<D>(r[0], r[1], r[2]) : 1.0e30f, t = fmaxf(g.h2 - q, 0.f);
     w[0] = g.c_s * (t * t * t);
-    const float phi = q > 0.f ? g.c_g * spiky_phi(spiky_distance(q), g.h) : 0.f;
+    const float phi = q > 0.f ? g.c_g * spiky_phi(dense_distance<D>(q), g.h) : 0.f;
 #pragma unroll
     for (int d = 0; d < D; ++d) {
         const float k = phi * r[d];
