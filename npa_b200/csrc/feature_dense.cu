@@ -405,24 +405,24 @@ int feature_dense_pitch(int dim, int cp) {
 
 // Where it is the faster one, by the mean number of particles per cell of the grid (a tile costs its candidates and the union of its
 // neighbours, a list its length) and by the particles in all: a tile is a longer chain than a list, which shows while either kernel is a
-// wave or two.  Particles that leave cells empty have more neighbours than the mean tells, and lists that overflow are searched, so that clustered ones gain
-// earlier and more; the lines are where uniform ones lose nothing or little.  The kernels alone, lists / this, us, uniform unless said otherwise:
-//  * 2D, C = 16: 65,536 particles 2 a cell 17.7 / 18.9, 3 21.3 / 20.5, 4 24.5 / 22.7, 8 37 / 31; along lines 2 a cell 52 / 39, 4 160 / 61; in blobs
-//    29 / 25, 86 / 32; 8,192 2 a cell 6.3 / 7.6, 4 8.5 / 8.5, 8 11.6 / 10.5, along lines 16.4 / 13.7, 67 / 19.  The line at 2 costs uniform particles
-//    up to 1.3 us below 4 a cell, where the clustered ones, which are what is that thin (12 neighbours of uniform particles are 3.8 a cell), gain 2 to 50.
-//  * C = 32: 65,536 2 a cell 26.9 / 27.3, 4 36 / 32; 16,384 9.9 / 9.8, 13.8 / 11.9; 24,000, beyond a wave, 11.0 / 13.5, 14.9 / 14.0; 12,000 2 a cell
-//    6.7 / 9.2, 8 12.8 / 14.3; 8,192 5.8 / 8.7, 10.0 / 12.2; along lines 8,192 2 a cell 14.4 / 15.9, 8 66 / 32, in blobs 8.0 / 10.6, 20.5 / 20.2, 12 a cell
-//    58 / 25: for few particles from 8 a cell, where lists of clustered ones overflow.
-//  * 2D periodic, whose candidates are tested image by image: C = 16, 65,536 7 a cell 34.8 / 35.1, 10 45 / 42; C = 8 33.3 / 35.4, 42.4 / 43.2; C = 32 4 a cell 36.6 /
-//    35.7; 48,000 C = 16 8 a cell 32.6 / 30.9, C = 32 4 a cell 28.3 / 27.9; 33,000 20.3 / 22.7, 8 a cell 30.1 / 30.6; 24,000 C = 16 10 a cell 19.8 / 24.0, 12
-//    22.4 / 25.6.  Fewer particles than 44,000 lose at any uniform density (8,192 12 a cell 14.1 / 18.7, C = 32 13.0 / 19.7): beyond 12 a cell that is left so
-//    for clustered ones.
-//  * 3D, C = 16: 65,536 4 a cell 39.6 / 38.8, 6 52 / 47; 262,144 4 a cell 134 / 136, 5 154 / 150; 32,768 5 a cell 25.2 / 27.7, 8 35.9 / 33.7.  C = 12, whose rows are
-//    padded to 16: 65,536 4 a cell 37.7 / 39.6, 6 50.5 / 47.8.
-//  * 3D, C = 32: 98,304 5 a cell 88.5 / 94.7, 6 96.5 / 98.1, 7 110 / 108; C = 20 6 a cell 94.8 / 99.2, 8 118 / 120.  One wave (20,500) C = 32 7 a cell 30.6 / 30.8, 8
-//    34.9 / 32.4; little more (28,000) 8 a cell 36.4 / 43.4, 14 72.2 / 71.1.  In a ball, where the particles are twice as dense: 98,304 5 a cell
-//    137 / 135, 8 199 / 188.  262,144 uniform 4.5 a cell 215 / 227, 5 218 / 225, 6 250 / 249, in a ball 333 / 323, 341 / 325, 399 / 365, 4 x 65,536 with a radius of
-//    1.05 cells 378 / 343: there the line at 4.5 costs the ones 12 us and gives the others 10 to 35.
+// wave or two.  Particles that leave cells empty have more neighbours than the mean tells, and lists that overflow are searched, so that clustered
+// ones gain earlier and more; the lines are where uniform ones lose nothing or little.  The kernels alone, lists / this, us, uniform unless said otherwise:
+//  * 2D, C = 16: 65,536 particles 2 a cell 17.8 / 19.0, 3 21.2 / 20.8, 4 24.4 / 22.5, 8 38 / 31; along lines 2 a cell 51 / 37, 4 166 / 59; in blobs
+//    29 / 24, 87 / 32; 8,192 2 a cell 6.2 / 7.6, 4 8.5 / 8.4, 8 11.7 / 10.8, along lines 16.2 / 13.5, 67 / 19.  The line at 2 costs uniform particles
+//    up to 1.4 us below 4 a cell, where the clustered ones, which are what is that thin (12 neighbours of uniform particles are 3.8 a cell), gain 2 to 50.
+//  * C = 32: 65,536 2 a cell 27.4 / 27.5, 4 36 / 32; 16,384 9.9 / 9.9, 13.4 / 11.5; 24,000, beyond a wave, 11.1 / 13.4, 14.9 / 14.0; 12,000 2 a cell
+//    6.7 / 8.9, 8 12.7 / 13.9; 8,192 5.7 / 8.5, 10.0 / 11.9; along lines 8,192 2 a cell 14.1 / 15.8, 8 68 / 31, in blobs 8.0 / 10.3, 20.4 / 19.9, 12 a cell
+//    60 / 25: for few particles from 8 a cell, where lists of clustered ones overflow.
+//  * 2D periodic, whose candidates are tested image by image: C = 16, 65,536 7 a cell 34.7 / 34.5, 10 45 / 43; C = 8 8 a cell 36.3 / 38.0, 10 42.4 / 42.8; C = 32 4 a cell
+//    36.7 / 35.7; 48,000 C = 16 8 a cell 34.7 / 30.7, C = 32 4 a cell 28.4 / 27.7; 33,000 20.3 / 22.7, 8 a cell 30.0 / 30.3; 24,000 C = 16 10 a cell 19.5 / 23.9,
+//    12 22.4 / 25.5.  Fewer particles than 44,000 lose at any uniform density (8,192 12 a cell 13.7 / 18.6, C = 32 12.8 / 19.8): from 12 a cell on that is
+//    left so for clustered ones.
+//  * 3D, C = 16: 65,536 4 a cell 39.7 / 39.0, 6 52 / 48; 262,144 4 a cell 134 / 138, 5 154 / 152; 32,768 6 a cell 28.5 / 31.7, 8 35.7 / 34.2.  C = 12, whose rows are
+//    padded to 16: 65,536 5 a cell 45.3 / 47.7, 6 51.0 / 49.1; 262,144 147 / 157, 169 / 174.
+//  * 3D, C = 32: 98,304 4 a cell 77.5 / 83.2, 5 89.1 / 89.6, 6 96.4 / 92.7; C = 20 5 a cell 87.1 / 91.8, 6 95.4 / 94.9.  262,144 C = 32 4 a cell 194 / 195, 4.5
+//    215 / 216, C = 20 5 220 / 223.  One wave (20,500) C = 32 6 a cell 27.8 / 26.4, C = 20 7 30.4 / 30.8, 8 35.0 / 32.2; little more (28,000) 8 a cell
+//    35.9 / 40.6, 10 43.1 / 45.8; 41,000 8 53.0 / 52.6, 10 63.1 / 60.4, C = 20 52.5 / 54.9, 61.8 / 61.9.  In a ball, where the particles are twice as dense, C = 32: 98,304
+//    5 a cell 138 / 128, 262,144 342 / 309, 4 x 65,536 with a radius of 1.05 cells, 4.7 a cell, 380 / 329.
 //  * 3D periodic: lists (64 a cell 428 / 463, 8 a cell 76 / 89).
 bool feature_dense_covers(const Geom &g, int C) {
     const long long particles = (long long)g.B * g.N;
@@ -432,10 +432,10 @@ bool feature_dense_covers(const Geom &g, int C) {
     if (g.dim == 2 && !g.periodic) return per_cell >= (wide && particles < 14000 ? 8.0 : 2.0);
     if (g.dim == 2) return per_cell >= (particles < 44000 ? 12.0 : wide ? 4.0 : 10.0);
     if (g.periodic || particles < 20000) return false;
-    if (!wide) return per_cell >= (particles < 40000 ? 8.0 : C > 12 ? 4.0 : 5.0);
-    if (particles < 60000) return per_cell >= (particles <= 148 * 5 * kDenseWarps * kDenseTile ? 8.0 : 14.0);
-    const bool many = particles >= 200000;
-    return per_cell >= (C > 28 ? (many ? 4.5 : 6.0) : many ? 6.0 : 8.0);
+    if (!wide) return per_cell >= (particles < 40000 ? 8.0 : C > 12 ? 4.0 : 6.0);
+    if (particles < 60000) return per_cell >= (particles <= 148 * 5 * kDenseWarps * kDenseTile ? 8.0 : 10.0);
+    if (particles < 200000) return per_cell >= (C > 28 ? 5.0 : 6.0);
+    return per_cell >= (C > 28 ? 4.5 : 5.0);
 }
 
 int launch_feature_dense_backward(const Geom &g, const FeatureListBwdArgs &args, cudaStream_t st) {
