@@ -416,7 +416,8 @@ int npa_perceive_features_backward_lists(const npa_grid *g, int32_t channels, co
                                          const int32_t *pair_cache, int32_t pair_stride, void *stream);
 
 /* The same for positions that are those that were binned, bit for bit, as a step has them between its reorder and its update:
- * with grad_x = NULL it may then find the neighbours among the cells instead of reading the lists. */
+ * with grad_x = NULL it may then find the neighbours among the cells instead of reading the lists.  The number of particles in all is one of the
+ * things that decide, and tiles of eight particles may straddle systems: a system's sums inside another batch agree within rounding. */
 int npa_perceive_features_backward_binned(const npa_grid *g, int32_t channels, const float *x_bin, const float *mass,
                                          const float *s_bin, const float *rho, const float *rho_grad, const float *vgrad,
                                          const float *packed, const float *dL_dz, float coef, float dg_scale,
@@ -589,7 +590,8 @@ int npa_mlp_forward_tcgen05_images(const float *z, const float *W1, const float 
                                    int64_t scratch_bytes, void *dz_image, int64_t dz_image_bytes, void *stream);
 
 /* The same in two calls: the images of the weights (scratch as above, and dz_image unless NULL) made by the launch that reorders
- * positions and states into cell order (npa_bin_particles without masses), and the two layers on images that are there. */
+ * positions and states into cell order (npa_bin_particles without masses), and the two layers on images that are there.  (The first, and
+ * npa_bin_particles_step_images below, are for callers that build their grids by themselves; a step of this package begins with npa_step_bin.) */
 int npa_bin_particles_mlp_images(const npa_grid *grid, int32_t channels, const float *x, const float *s, const int32_t *permutation,
                                  float *x_out, float *s_out, const float *W1, const float *W2, int32_t in_dim, int32_t out_dim,
                                  int64_t w1_stride_out, int64_t w1_stride_in, int64_t w2_stride_out, int64_t w2_stride_in,

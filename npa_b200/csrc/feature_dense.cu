@@ -17,12 +17,12 @@
 // or a volume that is not finite to particles that are no neighbours of it; a warp whose sums, of the rows or of T, are not finite therefore
 // computes its particles again, pair by pair.
 //
-// Measured, B200, us, lists -> this: 8 x 4,096 particles in 2D, C = 16, 50 neighbours 32 -> 24; 64 x 512 along lines 34 -> 20; 4 x 65,536 in 3D,
-// C = 32, 41 neighbours 372 -> 334 (of these the search 121; instructions 210 M, 60 % of the slots, MMAs a quarter of the tensor pipe's time).
+// Measured, B200, us, lists -> this: 8 x 4,096 particles in 2D, C = 16, 49 neighbours 35 -> 27; 64 x 512 along lines 35 -> 24; 4 x 65,536 in 3D,
+// C = 32, 41 neighbours 380 -> 330 (of these the search 121; instructions 220 M, 64 % of the slots, MMAs a quarter of the tensor pipe's time).
 // Error against 64 bits (2-norm, 1e-7), lists / this, rows N(0, 1): 2D, 14 neighbours 1.47 / 1.44 (1.48 with three MMAs), 25 1.70 / 1.47, 77
 // 2.52 / 1.67; 3D 16 1.66 / 1.62, 39 2.09 / 1.65, 76 2.58 / 1.73; over 80 drawn training cases of 12 and more neighbours at most 0.99 of
 // the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 26 -> 27 us with 16 features, 36 -> 38
-// with 32.  Not kept: sixteen particles per warp (411,
+// with 32.  Not kept (3D, against 334 then): sixteen particles per warp (411,
 // larger unions and fewer warps); a queue per residue of the neighbour's index, for rows in banks of their own (515); the head by
 // cvt.rna (452).
 //

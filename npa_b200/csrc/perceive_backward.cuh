@@ -34,7 +34,7 @@ struct StepRows {
     int log_norm;
 };
 // Rows of whole float4, up to the features of the packed sweep.  dL/dz stored and taken apart by a kernel of its own / as it leaves, with the
-// sweep that follows, us: 32,768 particles in 2D, C = 4 / 16 / 20 / 32: 32.9 / 30.8, 36.9 / 32.8, 47.0 / 43.1, 49.7 / 45.2; 65,536 in 3D
+// sweep that followed then, us: 32,768 particles in 2D, C = 4 / 16 / 20 / 32: 32.9 / 30.8, 36.9 / 32.8, 47.0 / 43.1, 49.7 / 45.2; 65,536 in 3D
 // 81.7 / 78.1, 91.8 / 83.0, 126.0 / 118.9, 137.2 / 126.7 (sections that fill half of their columns gain least).
 inline bool step_rows_cover(int channels) { return channels % 4 == 0 && channels > 0 && channels <= 32; }
 int launch_step_rows(const StepRows &rows, const float *dh, long long particles, const void *image, int64_t image_bytes, cudaStream_t st);

@@ -133,7 +133,7 @@ def test_a_wait_that_runs_out_ends_the_tcgen05_kernel_roles_cleanly(engine):
 
 
 @pytest.mark.parametrize("dim", [2, 3])
-@pytest.mark.parametrize("C,N", [(4, 1), (13, 15), (16, 16), (16, 4097), (32, 17), (32, 40000), (45, 333)])   # sixteen rows per warp, up to 48 columns
+@pytest.mark.parametrize("C,N", [(4, 1), (13, 15), (16, 16), (16, 4097), (32, 17), (32, 40000), (45, 333)])   # eight rows per warp, up to 48 columns
 @pytest.mark.parametrize("mask", [None, "weights", "uniforms"])
 def test_hidden_gradient_of_a_step(dim, C, N, mask):
     """The update's backward and the hidden gradient in one pass: g_y to the bit as by the update's own kernel, dh to the bit as from that
