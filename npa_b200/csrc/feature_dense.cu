@@ -12,7 +12,7 @@
 // cut-off are zero; two fifths of the products are of pairs.
 //
 // Single precision: every operand is split into a TF32 head, rounded to nearest, and a tail of at most twelve bits; three MMAs per product
-// (tail . head + head . tail + head . head), four in 2D (tail . tail), where few neighbours' roundings do not outweigh it.  The tensor cores truncate when they accumulate, so a chain is one group of eight neighbours
+// (tail . head + head . tail + head . head), four (tail . tail) where the roundings of few neighbours do not outweigh it.  The tensor cores truncate when they accumulate, so a chain is one group of eight neighbours
 // (heads 1 + D MMAs, the others apart) and is added to the running sums in single precision.  A product with a zero weight spreads a row
 // or a volume that is not finite to particles that are no neighbours of it; a warp whose sums, of the rows or of T, are not finite therefore
 // computes its particles again, pair by pair.
@@ -21,7 +21,7 @@
 // C = 32, 41 neighbours 380 -> 330 (of these the search 121; instructions 220 M, 64 % of the slots, MMAs a quarter of the tensor pipe's time).
 // Error against 64 bits (2-norm, 1e-7), lists / this, rows N(0, 1): 2D, 14 neighbours 1.47 / 1.44 (1.48 with three MMAs), 25 1.70 / 1.47, 77
 // 2.52 / 1.67; 3D 16 1.66 / 1.62, 39 2.09 / 1.65, 76 2.58 / 1.73; over 80 drawn training cases of 12 and more neighbours at most 0.99 of
-// the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 26 -> 27 us with 16 features, 36 -> 38
+// the lists'.  Below ten neighbours up to 1.03 of it (2D, 7: 1.35 / 1.39).  The fourth MMA costs 2D 25.5 -> 26.7 us with 16 features, 36 -> 38
 // with 32.  Not kept (3D, against 334 then): sixteen particles per warp (411,
 // larger unions and fewer warps); a queue per residue of the neighbour's index, for rows in banks of their own (515); the head by
 // cvt.rna (452).
@@ -35,6 +35,10 @@ namespace npa {
 constexpr int kDenseWarps = 4;
 constexpr int kDenseTile = 8;    // particles per warp
 constexpr int kDenseRing = 64;   // neighbours found and not yet multiplied
+// Particles per cell in 2D below which the tails are multiplied as well: uniform particles have 16 neighbours there, clustered ones more.
+// Error against the lists', three / four products: 7 neighbours 1.06 / 1.03, 10 1.04 / 1.01, 12 1.01 / 0.99, 14 1.01 / 0.98, 16 0.96 / 0.94, 19 0.94 / 0.92.
+// In 3D the sweep begins at 16 (0.97).
+constexpr double kDenseTailsBelow = 5.0;
 
 struct DenseMem {  // of one warp
     float4 at[kDenseRing];  // position and volume of a neighbour
@@ -171,8 +175,8 @@ __device__ __forceinline__ unsigned long long nearest_image2(unsigned long long 
     return fma2(k, pack2(-L, -L), r);
 }
 
-// Rows are [1 + D][cp] (gb and gg in one).  MT: blocks of sixteen features; FILLED: cp = 16 MT.
-template <int D, bool PER, int MT, bool FILLED>
+// Rows are [1 + D][cp] (gb and gg in one).  MT: blocks of sixteen features; FILLED: cp = 16 MT; TAILS: with the products of the tails.
+template <int D, bool PER, int MT, bool FILLED, bool TAILS>
 __global__ void __launch_bounds__(kDenseWarps * 32, MT == 2 ? 5 : D == 3 ? 6 : 7)
 feature_dense_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, const __grid_constant__ Geom g) {
     after_previous_kernel();
@@ -263,7 +267,7 @@ feature_dense_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, cons
                     const Tf32 a0 = split_tf32(v0[c][2 * m]), a1 = split_tf32(v0[c][2 * m + 1]);
                     const Tf32 a2 = split_tf32(v1[c][2 * m]), a3 = split_tf32(v1[c][2 * m + 1]);
                     const unsigned ah[4] = {a0.head, a1.head, a2.head, a3.head}, at[4] = {a0.tail, a1.tail, a2.tail, a3.tail};
-                    if constexpr (D == 2) mma_m16n8k8(others[m], at, b0.tail, b1.tail);
+                    if constexpr (TAILS) mma_m16n8k8(others[m], at, b0.tail, b1.tail);
                     mma_m16n8k8(others[m], at, b0.head, b1.head);
                     if (c == 0) mma_m16n8k8_from_zero(heads[m], ah, b0.head, b1.head);
                     else mma_m16n8k8(heads[m], ah, b0.head, b1.head);
@@ -384,14 +388,14 @@ feature_dense_backward_kernel(const __grid_constant__ FeatureListBwdArgs a, cons
     }
 }
 
-template <int D, bool PER>
+template <int D, bool PER, bool TAILS>
 static int launch_dense(const Geom &g, const FeatureListBwdArgs &a, cudaStream_t st) {
     const long long tiles = ((long long)g.B * g.N + kDenseTile - 1) / kDenseTile;
     const unsigned blocks = (unsigned)((tiles + kDenseWarps - 1) / kDenseWarps);
-    auto kernel = feature_dense_backward_kernel<D, PER, 2, false>;
-    if (a.cp == 32) kernel = feature_dense_backward_kernel<D, PER, 2, true>;
-    else if (a.cp == 16) kernel = feature_dense_backward_kernel<D, PER, 1, true>;
-    else if (a.cp < 16) kernel = feature_dense_backward_kernel<D, PER, 1, false>;
+    auto kernel = feature_dense_backward_kernel<D, PER, 2, false, TAILS>;
+    if (a.cp == 32) kernel = feature_dense_backward_kernel<D, PER, 2, true, TAILS>;
+    else if (a.cp == 16) kernel = feature_dense_backward_kernel<D, PER, 1, true, TAILS>;
+    else if (a.cp < 16) kernel = feature_dense_backward_kernel<D, PER, 1, false, TAILS>;
     kernel<<<blocks, kDenseWarps * 32, 0, st>>>(a, g);
     return check_launch("feature_dense_backward_kernel");
 }
@@ -407,15 +411,15 @@ int feature_dense_pitch(int dim, int cp) {
 // neighbours, a list its length) and by the particles in all: a tile is a longer chain than a list, which shows while either kernel is a
 // wave or two.  Particles that leave cells empty have more neighbours than the mean tells, and lists that overflow are searched, so that clustered
 // ones gain earlier and more; the lines are where uniform ones lose nothing or little.  The kernels alone, lists / this, us, uniform unless said otherwise:
-//  * 2D, C = 16: 65,536 particles 2 a cell 17.8 / 19.0, 3 21.2 / 20.8, 4 24.4 / 22.5, 8 38 / 31; along lines 2 a cell 51 / 37, 4 166 / 59; in blobs
-//    29 / 24, 87 / 32; 8,192 2 a cell 6.2 / 7.6, 4 8.5 / 8.4, 8 11.7 / 10.8, along lines 16.2 / 13.5, 67 / 19.  The line at 2 costs uniform particles
-//    up to 1.4 us below 4 a cell, where the clustered ones, which are what is that thin (12 neighbours of uniform particles are 3.8 a cell), gain 2 to 50.
-//  * C = 32: 65,536 2 a cell 27.4 / 27.5, 4 36 / 32; 16,384 9.9 / 9.9, 13.4 / 11.5; 24,000, beyond a wave, 11.1 / 13.4, 14.9 / 14.0; 12,000 2 a cell
-//    6.7 / 8.9, 8 12.7 / 13.9; 8,192 5.7 / 8.5, 10.0 / 11.9; along lines 8,192 2 a cell 14.1 / 15.8, 8 68 / 31, in blobs 8.0 / 10.3, 20.4 / 19.9, 12 a cell
-//    60 / 25: for few particles from 8 a cell, where lists of clustered ones overflow.
-//  * 2D periodic, whose candidates are tested image by image: C = 16, 65,536 7 a cell 34.7 / 34.5, 10 45 / 43; C = 8 8 a cell 36.3 / 38.0, 10 42.4 / 42.8; C = 32 4 a cell
-//    36.7 / 35.7; 48,000 C = 16 8 a cell 34.7 / 30.7, C = 32 4 a cell 28.4 / 27.7; 33,000 20.3 / 22.7, 8 a cell 30.0 / 30.3; 24,000 C = 16 10 a cell 19.5 / 23.9,
-//    12 22.4 / 25.5.  Fewer particles than 44,000 lose at any uniform density (8,192 12 a cell 13.7 / 18.6, C = 32 12.8 / 19.8): from 12 a cell on that is
+//  * 2D, C = 16: 65,536 particles 2 a cell 17.8 / 18.9, 3 21.3 / 20.6, 4 24.6 / 22.3, 8 37 / 29; along lines 2 a cell 52 / 38, 4 161 / 60; in blobs
+//    29 / 24, 86 / 31; 8,192 2 a cell 6.1 / 7.6, 4 8.5 / 8.4, 8 11.1 / 10.0, along lines 16.8 / 13.4, 70 / 19.  The line at 2 costs uniform particles
+//    up to 1.5 us below 4 a cell, where the clustered ones, which are what is that thin (12 neighbours of uniform particles are 3.8 a cell), gain 2 to 50.
+//  * C = 32: 65,536 2 a cell 27.3 / 27.2, 4 36 / 32; 16,384 10.2 / 9.7, 13.5 / 11.3; 24,000, beyond a wave, 11.1 / 13.3, 15.1 / 13.6; 12,000 2 a cell
+//    6.6 / 9.1, 8 12.6 / 13.1; 8,192 5.6 / 8.6, 9.9 / 11.2; along lines 8,192 2 a cell 14.1 / 15.9, 8 68 / 28, in blobs 8.0 / 10.8, 20.7 / 18.4, 12 a cell
+//    60 / 23: for few particles from 8 a cell, where lists of clustered ones overflow.
+//  * 2D periodic, whose candidates are tested image by image: C = 16, 65,536 7 a cell 34.8 / 34.0, 10 45 / 41; C = 8 8 a cell 35.7 / 36.6, 10 42.3 / 41.0; C = 32 4 a cell
+//    37.0 / 35.8; 48,000 C = 16 7 a cell 30.6 / 28.2, C = 32 4 a cell 28.0 / 27.9; 33,000 20.4 / 22.4, 8 a cell 29.7 / 29.1; 24,000 C = 16 10 a cell 19.9 / 22.7,
+//    12 22.7 / 24.4.  Fewer particles than 44,000 lose at any uniform density (8,192 12 a cell 14.6 / 17.8, C = 32 12.7 / 18.4): from 12 a cell on that is
 //    left so for clustered ones.
 //  * 3D, C = 16: 65,536 4 a cell 39.7 / 39.0, 6 52 / 48; 262,144 4 a cell 134 / 138, 5 154 / 152; 32,768 6 a cell 28.5 / 31.7, 8 35.7 / 34.2.  C = 12, whose rows are
 //    padded to 16: 65,536 5 a cell 45.3 / 47.7, 6 51.0 / 49.1; 262,144 147 / 157, 169 / 174.
@@ -430,7 +434,7 @@ bool feature_dense_covers(const Geom &g, int C) {
     const double per_cell = (double)g.N / g.cells;
     const bool wide = C > 16;  // two blocks of features
     if (g.dim == 2 && !g.periodic) return per_cell >= (wide && particles < 14000 ? 8.0 : 2.0);
-    if (g.dim == 2) return per_cell >= (particles < 44000 ? 12.0 : wide ? 4.0 : 10.0);
+    if (g.dim == 2) return per_cell >= (particles < 44000 ? 12.0 : wide ? 4.0 : C > 12 ? 7.0 : 8.0);
     if (g.periodic || particles < 20000) return false;
     if (!wide) return per_cell >= (particles < 40000 ? 8.0 : C > 12 ? 4.0 : 6.0);
     if (particles < 60000) return per_cell >= (particles <= 148 * 5 * kDenseWarps * kDenseTile ? 8.0 : 10.0);
@@ -441,8 +445,9 @@ bool feature_dense_covers(const Geom &g, int C) {
 int launch_feature_dense_backward(const Geom &g, const FeatureListBwdArgs &args, cudaStream_t st) {
     FeatureListBwdArgs a = args;
     a.out_vec = a.C == a.cp && ((uintptr_t)a.grad_s | (uintptr_t)a.add) % 16 == 0;
-    if (g.dim == 3) return launch_dense<3, false>(g, a, st);
-    return g.periodic ? launch_dense<2, true>(g, a, st) : launch_dense<2, false>(g, a, st);
+    if (g.dim == 3) return launch_dense<3, false, false>(g, a, st);
+    if ((double)g.N / g.cells < kDenseTailsBelow) return g.periodic ? launch_dense<2, true, true>(g, a, st) : launch_dense<2, false, true>(g, a, st);
+    return g.periodic ? launch_dense<2, true, false>(g, a, st) : launch_dense<2, false, false>(g, a, st);
 }
 
 }  // namespace npa
