@@ -157,16 +157,21 @@ def test_error_is_not_larger_than_that_of_the_lists(dim, N, cells, boundary, C, 
 @pytest.mark.parametrize("dim,boundary,cells,N,C,dense", [
     (2, "clamped", 40, 3200, 16, True), (2, "clamped", 40, 3199, 16, False), (2, "clamped", 80, 13999, 17, False), (2, "clamped", 80, 14000, 17, True),
     (2, "clamped", 20, 3200, 32, True), (2, "periodic", 79, 44000, 16, True), (2, "periodic", 79, 43999, 16, False),
-    (2, "periodic", 80, 44000, 16, False),     (2, "periodic", 74, 44000, 12, True), (2, "periodic", 75, 44000, 12, False),
+    (2, "periodic", 80, 44000, 16, False),
+    (2, "periodic", 74, 44000, 12, True), (2, "periodic", 75, 44000, 12, False),
     (2, "periodic", 104, 44000, 32, True), (2, "periodic", 20, 4799, 8, False), (3, "clamped", 14, 21952, 16, True),
-    (3, "clamped", 14, 21951, 16, False),     (3, "clamped", 21, 40000, 13, True),
-    (3, "clamped", 21, 40000, 12, False),     (3, "clamped", 18, 40000, 12, True), (3, "clamped", 14, 23680, 32, True),
-    (3, "clamped", 14, 23681, 32, False), (3, "clamped", 14, 27440, 32, True),     (3, "clamped", 14, 27439, 32, False),
+    (3, "clamped", 14, 21951, 16, False),
+    (3, "clamped", 21, 40000, 13, True),
+    (3, "clamped", 21, 40000, 12, False),
+    (3, "clamped", 18, 40000, 12, True), (3, "clamped", 14, 23680, 32, True),
+    (3, "clamped", 14, 23681, 32, False), (3, "clamped", 14, 27440, 32, True),
+    (3, "clamped", 14, 27439, 32, False),
     (3, "clamped", 22, 60000, 29, True), (3, "clamped", 22, 59999, 29, False),
-    (3, "clamped", 24, 69119, 32, False),     (3, "clamped", 24, 69120, 28, False), (3, "clamped", 21, 60000, 28, True),
-    (3, "clamped", 35, 200000, 32, True), (3, "clamped", 35, 199999, 32, False),     (3, "clamped", 34, 200000, 20, True),
-    (3, "clamped", 34, 199999, 20, False),
-    (3, "periodic", 12, 40000, 16, False)])
+    (3, "clamped", 24, 69119, 32, False),
+    (3, "clamped", 24, 69120, 28, False), (3, "clamped", 21, 60000, 28, True),
+    (3, "clamped", 35, 200000, 32, True), (3, "clamped", 35, 199999, 32, False),
+    (3, "clamped", 34, 200000, 20, True),
+    (3, "clamped", 34, 199999, 20, False), (3, "periodic", 12, 40000, 16, False)])
 def test_lines_between_the_two_sweeps(dim, boundary, cells, N, C, dense):
     torch.manual_seed(C)
     call = Call(_positions(dim, 1, N, 1.0), cells, 1.0 / cells, boundary, C)
